@@ -139,6 +139,9 @@ _sig = {
     "bsrl_qkv_attention": (C.c_int, [_P, _P, _P, _P, C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P, _P]),
     "bsrl_attention": (C.c_int, [_P, _P, C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P, _P]),
     "bsrl_apply_updates_pack": (C.c_int, [_CFG, C.POINTER(_P), C.POINTER(_P), C.c_int32, _P, _P, C.c_int64, _P]),
+    "bsrl_muon_workspace_bytes": (C.c_int64, [_CFG, C.POINTER(C.c_int32), C.c_int32]),
+    "bsrl_muon_step": (C.c_int, [_CFG, C.POINTER(_P), C.POINTER(_P), C.POINTER(_P), C.c_int32, C.POINTER(C.c_float),
+                                 C.c_float, C.c_float, _P, _P, C.c_int64, _P, C.c_int64, _P]),
     "bsrl_linear_ln": (C.c_int, [_P, _P, _P, _P, _P, _P, C.c_float, C.c_int64, C.c_int32, C.c_int32, _P, _P, _P]),
     "bsrl_qkv_attention_body": (C.c_int, [_P, _P, _P, _P, _P, C.c_int64, C.c_int32, C.c_int32, C.c_int32, _P, _P]),
     "bsrl_attention_tokens": (C.c_int, [_P, _P, C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_int32, _P, _P]),

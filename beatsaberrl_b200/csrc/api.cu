@@ -546,8 +546,9 @@ int64_t bsrl_weights_bytes(const bsrl_config* cfg) {
 int bsrl_pack_weights(const bsrl_config* cfg, const float* const* params, int32_t n_params, void* arena,
                       int64_t arena_bytes, void* stream) {
   BSRL_TRY(validate_config(cfg));
-  Layout l = make_layout(*cfg);
-  std::vector<ParamSlot> s = make_param_slots(*cfg, l);
+  const Plan& plan = plan_of(*cfg);
+  const Layout& l = plan.l;
+  const std::vector<ParamSlot>& s = plan.slots;
   if (!params || !arena) {
     set_error("pack_weights: NULL argument");
     return BSRL_ERR_NULL;
@@ -582,8 +583,9 @@ int bsrl_adam_step_pack(const bsrl_config* cfg, float* const* params, const floa
                         const float* inv_scale, const float* found_inf, void* arena, int64_t arena_bytes,
                         void* stream) {
   BSRL_TRY(validate_config(cfg));
-  Layout l = make_layout(*cfg);
-  const int32_t want = (int32_t)make_param_slots(*cfg, l).size();
+  const Plan& plan = plan_of(*cfg);
+  const Layout& l = plan.l;
+  const int32_t want = (int32_t)plan.slots.size();
   if (!params || !grads || !exp_avg || !exp_avg_sq || !lr || !arena) {
     set_error("adam_step_pack: NULL argument");
     return BSRL_ERR_NULL;
@@ -616,8 +618,9 @@ int bsrl_adam_step_pack(const bsrl_config* cfg, float* const* params, const floa
 int bsrl_apply_updates_pack(const bsrl_config* cfg, float* const* params, const float* const* updates, int32_t n_params,
                             const float* found_inf, void* arena, int64_t arena_bytes, void* stream) {
   BSRL_TRY(validate_config(cfg));
-  Layout l = make_layout(*cfg);
-  const int32_t want = (int32_t)make_param_slots(*cfg, l).size();
+  const Plan& plan = plan_of(*cfg);
+  const Layout& l = plan.l;
+  const int32_t want = (int32_t)plan.slots.size();
   if (!params || !updates || !arena) {
     set_error("apply_updates_pack: NULL argument");
     return BSRL_ERR_NULL;

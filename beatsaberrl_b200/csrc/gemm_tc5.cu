@@ -439,9 +439,7 @@ bool make_tmap_env3d(CUtensorMap* map, const void* base, int64_t n_envs, int tok
   return true;
 }
 
-// (k_rows, cols) fp16 row-major matrix seen as {64 columns, k rows, cols / 64 blocks}: one load of a
-// {64, box_k, box_blocks} box brings box_blocks tiles of box_k x 128 bytes, each with the 128-byte swizzle
-static bool make_tmap_mn(CUtensorMap* map, const void* base, int64_t k_rows, int64_t cols, int64_t ld_elems, int box_k,
+bool make_tmap_mn(CUtensorMap* map, const void* base, int64_t k_rows, int64_t cols, int64_t ld_elems, int box_k,
                          int box_blocks) {
   EncodeTiledFn fn = encode_fn();
   if (!fn) {

@@ -285,15 +285,12 @@ std::vector<CopySlot> make_copy_slots(const bsrl_config& c, const Layout& l, con
     return -1;
   };
   if (l.attn_G == 0) return out;
-  const int d = l.d, gd = l.attn_G * (d / l.H), n_groups = d / gd;
+  const int gd = l.attn_G * (l.d / l.H);
   auto regroup = [&](const Mat& m, const std::string names[3]) {
     for (int sct = 0; sct < 3; ++sct) {
       const int pw = find(names[sct] + ".weight"), pb = find(names[sct] + ".bias");
-      for (int g = 0; g < n_groups; ++g) {
-        const int64_t row = (int64_t)g * 3 * gd + sct * gd;
-        out.push_back({pw, (int64_t)g * gd, gd, d, m.w + row * m.pitch * 2, m.pitch, true});
-        out.push_back({pb, (int64_t)g * gd, gd, 1, m.b + row * 4, 0, false});
-      }
+      out.push_back({pw, gd, 3 * gd, m.w + (int64_t)sct * gd * m.pitch * 2, m.pitch, true});
+      out.push_back({pb, gd, 3 * gd, m.b + (int64_t)sct * gd * 4, 0, false});
     }
   };
   for (int i = 0; i < l.L; ++i) {
@@ -304,6 +301,21 @@ std::vector<CopySlot> make_copy_slots(const bsrl_config& c, const Layout& l, con
   const std::string cn[3] = {"critic_q", "critic_k", "critic_v"};
   regroup(l.critic_qkv_g, cn);
   return out;
+}
+
+const Plan& plan_of(const bsrl_config& c) {
+  static thread_local Plan plan;
+  static thread_local bsrl_config key;
+  static thread_local bool have = false;
+  if (!have || memcmp(&key, &c, sizeof(c)) != 0) {     // every field is four bytes: no padding to compare
+    have = false;
+    plan.l = make_layout(c);
+    plan.slots = make_param_slots(c, plan.l);
+    plan.copies = make_copy_slots(c, plan.l, plan.slots);
+    key = c;
+    have = true;
+  }
+  return plan;
 }
 
 // ------------------------------------------------------------------ workspace

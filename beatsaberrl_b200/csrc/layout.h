@@ -58,10 +58,11 @@ struct ParamSlot {
   bool half;
 };
 
-// A second destination for (a row range of) a master parameter: the regrouped q|k|v copies.
+// A second destination of a master parameter: its regrouped q|k|v copy.  Rows move in groups of group_rows: row r goes
+// to row (r / group_rows) * group_stride + r % group_rows of the matrix (or vector) at dst.
 struct CopySlot {
   int param;               // index into make_param_slots()
-  int64_t src_row0, n_rows, cols;
+  int group_rows, group_stride;
   int64_t dst, dst_pitch;
   bool half;
 };
@@ -71,6 +72,15 @@ int multi_pack_slots(const std::vector<ParamSlot>& slots, const std::vector<Copy
                      const float* const* grads, float* const* exp_avg, float* const* exp_avg_sq, const float* lr,
                      const float* wd, float beta1, float beta2, float eps, int step, const float* inv_scale,
                      const float* found_inf, void* arena, cudaStream_t stream);
+
+// Layout and parameter tables of a configuration, built once per host thread and kept for its next call with the same
+// configuration (building them takes tens of microseconds of string work, as long as an optimizer step's kernels).
+struct Plan {
+  Layout l;
+  std::vector<ParamSlot> slots;
+  std::vector<CopySlot> copies;
+};
+const Plan& plan_of(const bsrl_config& c);
 
 int validate_config(const bsrl_config* c);
 Layout make_layout(const bsrl_config& c);

@@ -165,18 +165,15 @@ std::vector<CopySlot> g_copy_slots(const GLayout& l, const std::vector<ParamSlot
       if (params[i].name == name) return (int)i;
     return -1;
   };
-  const int d = l.d, gd = 64, n_groups = d / gd;
+  const int gd = 64;
   for (int i = 0; i < l.L; ++i) {
     const std::string p = "blocks." + std::to_string(i);
     const std::string names[3] = {p + ".q_proj", p + ".k_proj", p + ".v_proj"};
     const Mat& m = l.blocks[i].qkv_g;
     for (int sct = 0; sct < 3; ++sct) {
       const int pw = find(names[sct] + ".weight"), pb = find(names[sct] + ".bias");
-      for (int g = 0; g < n_groups; ++g) {
-        const int64_t row = (int64_t)g * 3 * gd + sct * gd;
-        out.push_back({pw, (int64_t)g * gd, gd, d, m.w + row * m.pitch * 2, m.pitch, true});
-        out.push_back({pb, (int64_t)g * gd, gd, 1, m.b + row * 4, 0, false});
-      }
+      out.push_back({pw, gd, 3 * gd, m.w + (int64_t)sct * gd * m.pitch * 2, m.pitch, true});
+      out.push_back({pb, gd, 3 * gd, m.b + (int64_t)sct * gd * 4, 0, false});
     }
   }
   return out;

@@ -14,74 +14,136 @@
 //   p -= (lr / (1 - b1^t)) m / (sqrt(v) / sqrt(1 - b2^t) + eps)        (torch.optim.AdamW)
 //
 // so the fp16 arena is produced by the optimizer kernel itself and no separate refresh pass runs.  In additive
-// mode (step = 0 with gradients given) the "gradient" is a finished update and the step is p += u: the last
+// mode (step = 0 with gradients given) the "gradient" is an update direction and the step is p = p (1 - lr wd) + lr u: the last
 // stage of an optimizer whose direction is computed elsewhere (the Muon half of the reference's hybrid optimizer
-// orthogonalises its momentum with a chain of small matrix products first, python/train_batch.py:818-931).
+// orthogonalises its momentum with a chain of small matrix products first, python/train_batch.py:818-931; muon.cu).
+#include <string.h>
+
 #include "kernels.cuh"
 #include "layout.h"
 
 namespace bsrl {
 namespace {
 
-constexpr int kMaxSegs = 20, kMaxCopies = 64;
+// Segments of one launch: the table is a kernel parameter (32,764 bytes at most), so that nearly every model's refresh
+// is ONE launch (130-200 masters; it was nine launches of 20 masters, 94 us, at d = 256 and four blocks).
+constexpr int kMaxSegs = 240;
+constexpr int kBlockElems = 2048;     // elements per block: 256 threads, two 16-byte pieces each
 
 struct Seg {
   float* p;                // master (rows, cols) f32
   const float* g;          // gradient, or nullptr: no update, scatter only
   float* m;                // exp_avg
   float* v;                // exp_avg_sq
-  int64_t dst;             // primary destination in the arena (bytes)
-  int rows, cols, pitch;   // pitch: elements per destination row (fp16 matrices); 0: dense fp32 vector
-  int half;
+  int64_t dst, dst2;       // primary and second (regrouped) destination in the arena (bytes)
+  int n, cols;             // elements, elements per row (vectors: one row)
+  int pitch, pitch2;       // fp16 matrices: elements per destination row; fp32 vectors: 0
+  int group, gstride;      // second destination: row r -> (r / group) * gstride + r % group; group 0: none
   float lr, wd;
-  int copy_first, copy_n;  // its row ranges with a second destination
-};
-struct Copy {
-  int row0, n_rows, pitch, half;
-  int64_t dst;
+  int blk0;                // first block of this segment
+  int vec;                 // 16-byte accesses are possible throughout
 };
 struct Table {
   Seg seg[kMaxSegs];
-  Copy copy[kMaxCopies];
   int n_seg;
   float beta1, beta2, eps, bc1, rsqrt_bc2;   // bias corrections 1 - b1^t and 1 / sqrt(1 - b2^t)
   const float* inv_scale;                    // device scalar multiplying every gradient, or nullptr
   const float* found_inf;                    // device scalar: non-zero = skip every update (scatter still runs)
-  int additive;                              // the gradients are finished updates: p += g
+  int additive;                              // the gradients are update directions: p = p (1 - lr wd) + lr g
+};
+static_assert(sizeof(Table) + 16 <= 32764, "kernel parameter limit");
+
+// one element's update; true when the master changes
+struct Updater {
+  float beta1, beta2, eps, rsqrt_bc2, inv_scale, step, decay, lr;
+  bool additive;
+  __device__ __forceinline__ float adam(float p, float g_in, float& m, float& v) const {
+    const float g = g_in * inv_scale;
+    m = beta1 * m + (1.f - beta1) * g;
+    v = beta2 * v + (1.f - beta2) * g * g;
+    return p * decay - step * m / (sqrtf(v) * rsqrt_bc2 + eps);
+  }
+  __device__ __forceinline__ float add(float p, float u) const { return fmaf(lr, u, p * decay); }
 };
 
-__device__ __forceinline__ void put(uint8_t* arena, int64_t dst, int pitch, int half, int r, int c, int cols, float val) {
-  if (half) reinterpret_cast<__half*>(arena + dst)[(int64_t)r * pitch + c] = __float2half_rn(val);
-  else reinterpret_cast<float*>(arena + dst)[(int64_t)r * cols + c] = val;
+__device__ __forceinline__ void put(const Seg& s, uint8_t* arena, int r, int c, float val) {
+  if (s.pitch) reinterpret_cast<__half*>(arena + s.dst)[(int64_t)r * s.pitch + c] = __float2half_rn(val);
+  else reinterpret_cast<float*>(arena + s.dst)[c] = val;
+  if (s.group) {
+    const int row = s.pitch ? r : c;       // a vector's elements are its rows
+    const int row2 = (row / s.group) * s.gstride + row % s.group;
+    if (s.pitch) reinterpret_cast<__half*>(arena + s.dst2)[(int64_t)row2 * s.pitch2 + c] = __float2half_rn(val);
+    else reinterpret_cast<float*>(arena + s.dst2)[row2] = val;
+  }
 }
 
-// blockIdx.y = segment; blockIdx.x strides over its elements
+// Bound by the masters', gradients' and moments' traffic once the launch is large enough to fill the GPU: every block
+// takes kBlockElems consecutive elements of one segment (found by bisection over the segments' first blocks), so small
+// vectors cost one block each and a large matrix is spread over as many as it has pieces.
 __global__ void __launch_bounds__(256) multi_pack_kernel(const __grid_constant__ Table t, uint8_t* __restrict__ arena) {
-  const Seg& s = t.seg[blockIdx.y];
-  const int64_t n = (int64_t)s.rows * s.cols;
+  int lo = 0, hi = t.n_seg - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (t.seg[mid].blk0 <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+  }
+  const Seg& s = t.seg[lo];
   const bool update = s.g != nullptr && !(t.found_inf && *t.found_inf != 0.f);
-  const float inv_scale = (update && t.inv_scale) ? *t.inv_scale : 1.f;
-  const float step = s.lr / t.bc1, decay = 1.f - s.lr * s.wd;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+  Updater u;
+  u.beta1 = t.beta1; u.beta2 = t.beta2; u.eps = t.eps; u.rsqrt_bc2 = t.rsqrt_bc2;
+  u.inv_scale = (update && t.inv_scale) ? *t.inv_scale : 1.f;
+  u.step = s.lr / t.bc1; u.decay = 1.f - s.lr * s.wd; u.lr = s.lr;
+  u.additive = t.additive != 0;
+  const int i0 = ((int)blockIdx.x - s.blk0) * kBlockElems, i1 = min(s.n, i0 + kBlockElems);
+  if (s.vec) {
+#pragma unroll
+    for (int k = 0; k < kBlockElems / 1024; ++k) {
+      const int i = i0 + k * 1024 + threadIdx.x * 4;
+      if (i >= i1) break;
+      float4 p = *reinterpret_cast<const float4*>(s.p + i);
+      if (update) {
+        const float4 g = *reinterpret_cast<const float4*>(s.g + i);
+        if (u.additive) {
+          p = make_float4(u.add(p.x, g.x), u.add(p.y, g.y), u.add(p.z, g.z), u.add(p.w, g.w));
+        } else {
+          float4 m = *reinterpret_cast<const float4*>(s.m + i), v = *reinterpret_cast<const float4*>(s.v + i);
+          p = make_float4(u.adam(p.x, g.x, m.x, v.x), u.adam(p.y, g.y, m.y, v.y), u.adam(p.z, g.z, m.z, v.z),
+                          u.adam(p.w, g.w, m.w, v.w));
+          *reinterpret_cast<float4*>(s.m + i) = m;
+          *reinterpret_cast<float4*>(s.v + i) = v;
+        }
+        *reinterpret_cast<float4*>(s.p + i) = p;
+      }
+      if (s.pitch) {                         // matrix: cols, pitches and offsets are multiples of four
+        const int r = i / s.cols, c = i - r * s.cols;
+        const uint2 h = make_uint2(pack_half2(p.x, p.y), pack_half2(p.z, p.w));
+        *reinterpret_cast<uint2*>(arena + s.dst + ((int64_t)r * s.pitch + c) * 2) = h;
+        if (s.group) {
+          const int row2 = (r / s.group) * s.gstride + r % s.group;
+          *reinterpret_cast<uint2*>(arena + s.dst2 + ((int64_t)row2 * s.pitch2 + c) * 2) = h;
+        }
+      } else {
+        const float e[4] = {p.x, p.y, p.z, p.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) put(s, arena, 0, i + j, e[j]);
+      }
+    }
+    return;
+  }
+  for (int i = i0 + threadIdx.x; i < i1; i += 256) {
     float p = s.p[i];
-    if (update && t.additive) {
-      p += s.g[i];
-      s.p[i] = p;
-    } else if (update) {
-      const float g = s.g[i] * inv_scale;
-      const float m = t.beta1 * s.m[i] + (1.f - t.beta1) * g;
-      const float v = t.beta2 * s.v[i] + (1.f - t.beta2) * g * g;
-      s.m[i] = m;
-      s.v[i] = v;
-      p = p * decay - step * m / (sqrtf(v) * t.rsqrt_bc2 + t.eps);
+    if (update) {
+      if (u.additive) {
+        p = u.add(p, s.g[i]);
+      } else {
+        float m = s.m[i], v = s.v[i];
+        p = u.adam(p, s.g[i], m, v);
+        s.m[i] = m;
+        s.v[i] = v;
+      }
       s.p[i] = p;
     }
-    const int r = (int)(i / s.cols), c = (int)(i % s.cols);
-    put(arena, s.dst, s.pitch, s.half, r, c, s.cols, p);
-    for (int k = 0; k < s.copy_n; ++k) {
-      const Copy& cp = t.copy[s.copy_first + k];
-      if (r >= cp.row0 && r < cp.row0 + cp.n_rows) put(arena, cp.dst, cp.pitch, cp.half, r - cp.row0, c, s.cols, p);
-    }
+    const int r = i / s.cols;
+    put(s, arena, r, i - r * s.cols, p);
   }
 }
 
@@ -91,10 +153,9 @@ int multi_pack(const bsrl_config& cfg, const Layout& l, float* const* params, co
                float* const* exp_avg, float* const* exp_avg_sq, const float* lr, const float* wd, float beta1,
                float beta2, float eps, int step, const float* inv_scale, const float* found_inf, void* arena,
                cudaStream_t stream) {
-  const std::vector<ParamSlot> slots = make_param_slots(cfg, l);
-  const std::vector<CopySlot> copies = make_copy_slots(cfg, l, slots);
-  return multi_pack_slots(slots, copies, params, grads, exp_avg, exp_avg_sq, lr, wd, beta1, beta2, eps, step, inv_scale,
-                          found_inf, arena, stream);
+  const Plan& plan = plan_of(cfg);
+  return multi_pack_slots(plan.slots, plan.copies, params, grads, exp_avg, exp_avg_sq, lr, wd, beta1, beta2, eps, step,
+                          inv_scale, found_inf, arena, stream);
 }
 
 int multi_pack_slots(const std::vector<ParamSlot>& slots, const std::vector<CopySlot>& copies, float* const* params,
@@ -109,30 +170,20 @@ int multi_pack_slots(const std::vector<ParamSlot>& slots, const std::vector<Copy
   t.inv_scale = inv_scale;
   t.found_inf = found_inf;
   t.additive = (step == 0 && grads != nullptr) ? 1 : 0;
-  int n_copy = 0;
-  int64_t max_elems = 0;
+  std::vector<const CopySlot*> second(slots.size(), nullptr);
+  for (const CopySlot& cs : copies) second[cs.param] = &cs;
+  int blocks = 0;
   auto flush = [&]() -> int {
     if (t.n_seg == 0) return BSRL_OK;
-    int64_t bx = (max_elems + 255) / 256;
-    if (bx > 64) bx = 64;
-    if (bx < 1) bx = 1;
-    multi_pack_kernel<<<dim3((unsigned)bx, (unsigned)t.n_seg), 256, 0, stream>>>(t, static_cast<uint8_t*>(arena));
+    multi_pack_kernel<<<(unsigned)blocks, 256, 0, stream>>>(t, static_cast<uint8_t*>(arena));
     BSRL_LAUNCH_OK("multi_pack_kernel");
     t.n_seg = 0;
-    n_copy = 0;
-    max_elems = 0;
+    blocks = 0;
     return BSRL_OK;
   };
   for (size_t i = 0; i < slots.size(); ++i) {
     const ParamSlot& ps = slots[i];
-    int mine = 0;
-    for (const CopySlot& cs : copies)
-      if (cs.param == (int)i) ++mine;
-    if (mine > kMaxCopies) {
-      set_error("pack: parameter %s has %d regrouped row ranges (limit %d)", ps.name.c_str(), mine, kMaxCopies);
-      return BSRL_ERR_UNSUPPORTED;
-    }
-    if (t.n_seg == kMaxSegs || n_copy + mine > kMaxCopies) {
+    if (t.n_seg == kMaxSegs) {
       int rc = flush();
       if (rc != BSRL_OK) return rc;
     }
@@ -145,19 +196,23 @@ int multi_pack_slots(const std::vector<ParamSlot>& slots, const std::vector<Copy
       set_error("adam_step_pack: parameter %s has a gradient but no optimizer state", ps.name.c_str());
       return BSRL_ERR_NULL;
     }
+    s.n = (int)(ps.rows * ps.cols);
+    s.cols = ps.half ? (int)ps.cols : s.n;
     s.dst = ps.dst;
-    s.rows = (int)ps.rows; s.cols = (int)ps.cols; s.pitch = (int)ps.dst_pitch; s.half = ps.half ? 1 : 0;
-    s.lr = lr ? lr[i] : 0.f;
+    s.pitch = ps.half ? (int)ps.dst_pitch : 0;
+    s.group = s.gstride = s.pitch2 = 0;
+    s.dst2 = 0;
+    if (const CopySlot* cs = second[i]) {
+      s.group = cs->group_rows; s.gstride = cs->group_stride;
+      s.dst2 = cs->dst; s.pitch2 = (int)cs->dst_pitch;
+    }
+    s.lr = lr ? lr[i] : (t.additive ? 1.f : 0.f);
     s.wd = wd ? wd[i] : 0.f;
-    s.copy_first = n_copy;
-    s.copy_n = mine;
-    for (const CopySlot& cs : copies)
-      if (cs.param == (int)i) {
-        Copy& c = t.copy[n_copy++];
-        c.row0 = (int)cs.src_row0; c.n_rows = (int)cs.n_rows; c.pitch = (int)cs.dst_pitch; c.half = cs.half ? 1 : 0;
-        c.dst = cs.dst;
-      }
-    if (ps.rows * ps.cols > max_elems) max_elems = ps.rows * ps.cols;
+    // 16-byte pieces: a piece must not cross a matrix row, and 8-byte fp16 stores need pitches of four elements
+    s.vec = s.n % 4 == 0 && aligned16(s.p) && (!s.g || aligned16(s.g)) && (!s.m || aligned16(s.m)) && (!s.v || aligned16(s.v)) &&
+            (!ps.half || (ps.cols % 4 == 0 && s.pitch % 4 == 0 && s.pitch2 % 4 == 0 && s.dst % 8 == 0 && s.dst2 % 8 == 0));
+    s.blk0 = blocks;
+    blocks += (s.n + kBlockElems - 1) / kBlockElems;
   }
   return flush();
 }

@@ -248,6 +248,11 @@ bool make_tmap_rows(CUtensorMap* map, const void* base, int elem_bytes, int64_t 
 bool make_tmap_env3d(CUtensorMap* map, const void* base, int64_t n_envs, int tokens_per_env, int64_t cols,
                      int64_t ld_elems, int box_cols, int box_tokens, int box_envs);
 
+// (k_rows, cols) 2-byte row-major matrix seen as {64 columns, k rows, cols / 64 blocks}: one load of a {64, box_k,
+// box_blocks} box brings box_blocks tiles of box_k x 128 bytes, each with the 128-byte swizzle (MN-major operands).
+bool make_tmap_mn(CUtensorMap* map, const void* base, int64_t k_rows, int64_t cols, int64_t ld_elems, int box_k,
+                  int box_blocks);
+
 // Address of the current device's status word (nullptr with the error message set on failure).
 int* device_status_ptr();
 // Reads and clears the current device's status word (synchronises the device); -1 on failure.

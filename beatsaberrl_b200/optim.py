@@ -12,19 +12,38 @@ dimensions only.  Parameters without a gradient (frozen, or owned by another opt
 reference's Muon half) are left alone and only re-scattered.
 
 ``PackedMuon`` is that other half (python/train_batch.py:797-968): Nesterov momentum, five quintic Newton-Schulz
-steps towards the nearest orthogonal matrix, an RMS-matched step scale, on the hidden 2-D matrices only.  The
-small matrix products run as batched fp32 ``torch.bmm`` chains, one per matrix shape; the step itself -- masters
-plus their places in the arena -- is again one call of the library (``bsrl_apply_updates_pack``).
+steps towards the nearest orthogonal matrix, an RMS-matched step scale, on the hidden 2-D matrices only.  It is
+one call of the library too (``bsrl_muon_step``): the products of all matrices run together on the tensor cores with
+fp32 accuracy, and the last kernel writes the masters and their places in the arena.
 """
 from __future__ import annotations
 
 import ctypes as C
-import math
-from collections import defaultdict
 
 import torch
 
 from . import _native as nat
+
+
+def _lr_of(opt, name: str) -> float:
+    for prefix, mult in opt.lr_scale.items():
+        if name.startswith(prefix):
+            return opt.lr * mult
+    return opt.lr
+
+
+def _lr_table(opt, names, wd=None):
+    """Per-parameter learning rates (and weight decays) as C arrays, rebuilt only when a setting they come from changed."""
+    key = (opt.lr, opt.weight_decay, tuple(opt.lr_scale.items()))
+    if opt._lr_key != key:
+        n = len(names)
+        opt._lr_arrays = ((C.c_float * n)(*[_lr_of(opt, nm) for nm in names]), (C.c_float * n)(*(wd or [0.0] * n)))
+        opt._lr_key = key
+    return opt._lr_arrays
+
+
+def _pointers(tensors):
+    return (C.c_void_p * len(tensors))(*[t.data_ptr() for t in tensors])
 
 
 class PackedAdamW:
@@ -46,14 +65,9 @@ class PackedAdamW:
                 raise ValueError("PackedAdamW needs contiguous float32 parameters")
         self.exp_avg = [torch.zeros_like(p, memory_format=torch.preserve_format) for p in self.params]
         self.exp_avg_sq = [torch.zeros_like(p, memory_format=torch.preserve_format) for p in self.params]
-        n = len(self.params)
-        self._ptr = lambda ts: (C.c_void_p * n)(*[t.data_ptr() if t is not None else None for t in ts])
-
-    def _lr_of(self, name: str) -> float:
-        for prefix, mult in self.lr_scale.items():
-            if name.startswith(prefix):
-                return self.lr * mult
-        return self.lr
+        self._lr_key = self._lr_arrays = None
+        self._moments = _pointers(self.exp_avg), _pointers(self.exp_avg_sq)     # private tensors, only written in place
+        self._owned = [(i, p) for i, (nm, p) in enumerate(zip(self.names, self.params)) if nm not in self.exclude]
 
     def zero_grad(self, set_to_none: bool = True) -> None:
         for p in self.params:
@@ -72,17 +86,24 @@ class PackedAdamW:
         pol._pack()                           # the arena exists and its padding is zero
         self.step_count += 1
         n = len(self.params)
-        grads = [p.grad.contiguous() if (p.grad is not None and p.requires_grad and nm not in self.exclude) else None
-                 for nm, p in zip(self.names, self.params)]
-        lr = (C.c_float * n)(*[self._lr_of(nm) for nm in self.names])
-        wd = (C.c_float * n)(*[self.weight_decay if p.dim() >= 2 else 0.0 for p in self.params])
+        grads, keep = (C.c_void_p * n)(), []
+        for i, p in self._owned:
+            g = p.grad
+            if g is None or not p.requires_grad:
+                continue
+            if not g.is_contiguous():
+                g = g.contiguous()
+                keep.append(g)
+            grads[i] = g.data_ptr()
+        lr, wd = _lr_table(self, self.names, [self.weight_decay if p.dim() >= 2 else 0.0 for p in self.params]
+                           if self.weight_decay else None)
         for name, s in (("inv_scale", inv_scale), ("found_inf", found_inf)):
             if s is not None and (s.numel() != 1 or s.dtype is not torch.float32 or s.device != dev):
                 raise ValueError(f"{name} must be a one-element float32 tensor on {dev}")
         with torch.cuda.device(dev):
             nat.check(nat.lib.bsrl_adam_step_pack(
-                C.byref(pol._cfg), self._ptr(self.params), self._ptr(grads), self._ptr(self.exp_avg),
-                self._ptr(self.exp_avg_sq), n, lr, wd, self.betas[0], self.betas[1], self.eps, self.step_count,
+                C.byref(pol._cfg), _pointers(self.params), grads, *self._moments, n, lr, wd, self.betas[0],
+                self.betas[1], self.eps, self.step_count,
                 inv_scale.data_ptr() if inv_scale is not None else None,
                 found_inf.data_ptr() if found_inf is not None else None,
                 pol._arena.data_ptr(), pol._arena.numel(), torch.cuda.current_stream().cuda_stream))
@@ -100,8 +121,9 @@ class PackedAdamW:
             v.copy_(sd["exp_avg_sq"][n])
 
 
-# Newton-Schulz coefficients, one (a, b, c) per step, applied as a x + b x^3 + c x^5 to the singular values of the
-# normalised update: the published five-step schedule the reference adopted (python/train_batch.py:797-816).
+# Newton-Schulz coefficients (those of bsrl_muon_step), one (a, b, c) per step, applied as a x + b x^3 + c x^5 to the
+# singular values of the normalised update: the published five-step schedule the reference adopted
+# (python/train_batch.py:797-816).
 MUON_NS_COEFS = ((4.0848, -6.8946, 2.9270),
                  (3.9505, -6.3029, 2.6377),
                  (3.7418, -5.5913, 2.3037),
@@ -127,7 +149,8 @@ def muon_param_names(policy, enc_hidden: bool = False) -> list:
 
 def orthogonalize(stack: torch.Tensor, eps: float = 1e-7) -> torch.Tensor:
     """Five Newton-Schulz steps on a stack (k, m, n) of wide (m <= n) fp32 matrices: each is scaled to unit Frobenius
-    norm and pushed towards the nearest orthogonal matrix; the iteration runs on the small (m, m) Gram matrix."""
+    norm and pushed towards the nearest orthogonal matrix; the iteration runs on the small (m, m) Gram matrix.  The
+    plain statement of what ``bsrl_muon_step`` computes."""
     x = stack / (torch.linalg.vector_norm(stack, dim=(1, 2), keepdim=True) + eps)
     for a, b, c in MUON_NS_COEFS:
         gram = torch.bmm(x, x.transpose(1, 2))
@@ -153,13 +176,13 @@ class PackedMuon:
                 raise ValueError(f"PackedMuon owns 2-D parameters only: {n}")
         self.params = [named[n] for n in self.names]
         self.bufs = [torch.zeros_like(p) for p in self.params]
-        self._slot = {n: i for i, n in enumerate(self.table)}
-
-    def _lr_of(self, name: str) -> float:
-        for prefix, mult in self.lr_scale.items():
-            if name.startswith(prefix):
-                return self.lr * mult
-        return self.lr
+        slot = {n: i for i, n in enumerate(self.table)}
+        for p in self.params:
+            if p.dtype is not torch.float32 or not p.is_contiguous():
+                raise ValueError("PackedMuon needs contiguous float32 parameters")
+        self._rows = [(slot[n], p, b) for n, p, b in zip(self.names, self.params, self.bufs)]
+        self._ws_key, self._ws_bytes = None, 0
+        self._lr_key = self._lr_arrays = None
 
     def zero_grad(self, set_to_none: bool = True) -> None:
         for p in self.params:
@@ -173,37 +196,32 @@ class PackedMuon:
         if dev.type != "cuda":
             raise RuntimeError("PackedMuon runs on a CUDA device only")
         pol._pack()
-        live = [(n, p, b) for n, p, b in zip(self.names, self.params, self.bufs) if p.grad is not None and p.requires_grad]
-        updates = [None] * len(self.table)
-        if live:
-            grads = [p.grad for _, p, _ in live]
-            bufs = [b for _, _, b in live]
-            torch._foreach_mul_(bufs, self.momentum)
-            torch._foreach_add_(bufs, grads)
-            nesterov = torch._foreach_add(grads, bufs, alpha=self.momentum)
-            by_shape = defaultdict(list)
-            for i, (_, p, _) in enumerate(live):
-                by_shape[(min(p.shape), max(p.shape))].append(i)
-            for idx in by_shape.values():                                 # one chain of batched products per shape
-                tall = [live[i][1].shape[0] > live[i][1].shape[1] for i in idx]
-                stack = torch.stack([nesterov[i].t() if t else nesterov[i] for i, t in zip(idx, tall)])
-                ortho = orthogonalize(stack)
-                for k, (i, t) in enumerate(zip(idx, tall)):
-                    name, p, _ = live[i]
-                    lr = self._lr_of(name)
-                    upd = (ortho[k].t() if t else ortho[k]) * (-lr * 0.2 * math.sqrt(max(p.shape)))
-                    if self.weight_decay:
-                        upd = upd - (lr * self.weight_decay) * p
-                    updates[self._slot[name]] = upd.contiguous()
-        n = len(self.table)
-        ptr = lambda ts: (C.c_void_p * n)(*[t.data_ptr() if t is not None else None for t in ts])
         if found_inf is not None and (found_inf.numel() != 1 or found_inf.dtype is not torch.float32 or found_inf.device != dev):
             raise ValueError(f"found_inf must be a one-element float32 tensor on {dev}")
+        n = len(self.table)
+        grads, bufs, owned = (C.c_void_p * n)(), (C.c_void_p * n)(), (C.c_int32 * n)()
+        keep = []
+        for slot, p, b in self._rows:
+            g = p.grad
+            if g is None or not p.requires_grad:
+                continue
+            if not g.is_contiguous():
+                g = g.contiguous()
+                keep.append(g)
+            grads[slot], bufs[slot], owned[slot] = g.data_ptr(), b.data_ptr(), 1
+        lrs, _ = _lr_table(self, self.table)
+        if self._ws_key != bytes(owned):
+            self._ws_bytes = nat.lib.bsrl_muon_workspace_bytes(C.byref(pol._cfg), owned, n)
+            if self._ws_bytes < 0:
+                raise nat.BsrlError(int(self._ws_bytes), nat.last_error())
+            self._ws_key = bytes(owned)
+        ws = torch.empty(self._ws_bytes, dtype=torch.uint8, device=dev)
         with torch.cuda.device(dev):
-            nat.check(nat.lib.bsrl_apply_updates_pack(
-                C.byref(pol._cfg), ptr(self.all_params), ptr(updates), n,
-                found_inf.data_ptr() if found_inf is not None else None,
-                pol._arena.data_ptr(), pol._arena.numel(), torch.cuda.current_stream().cuda_stream))
+            nat.check(nat.lib.bsrl_muon_step(
+                C.byref(pol._cfg), _pointers(self.all_params), grads, bufs, n, lrs,
+                self.weight_decay, self.momentum, found_inf.data_ptr() if found_inf is not None else None,
+                pol._arena.data_ptr(), pol._arena.numel(), ws.data_ptr(), ws.numel(),
+                torch.cuda.current_stream().cuda_stream))
 
     def state_dict(self) -> dict:
         return {"momentum": self.momentum, "bufs": {n: b.clone() for n, b in zip(self.names, self.bufs)}}

@@ -129,6 +129,19 @@ int bsrl_adam_step_pack(const bsrl_config* cfg, float* const* params, const floa
 int bsrl_apply_updates_pack(const bsrl_config* cfg, float* const* params, const float* const* updates, int32_t n_params,
                             const float* found_inf, void* arena, int64_t arena_bytes, void* stream);
 
+/* One step of the Muon half (python/train_batch.py:797-931): bufs[i] = momentum bufs[i] + grads[i]; the Nesterov
+ * direction grads[i] + momentum bufs[i] is scaled to unit Frobenius norm and taken through five Newton-Schulz steps
+ * towards the nearest orthogonal matrix O; params[i] = params[i] (1 - lr[i] weight_decay) - lr[i] 0.2 sqrt(max side) O,
+ * masters and arena together as in bsrl_apply_updates_pack.  Matrices only; grads[i] == NULL: parameter i is only
+ * re-scattered.  bufs: n_params DEVICE pointers (fp32, one per owned matrix); lr: n_params HOST floats; found_inf (device
+ * float, may be NULL): non-zero skips the update of the masters (the momentum advances all the same).  The products have
+ * fp32 accuracy.  workspace: 256-byte aligned device memory; its size for the matrices with a non-zero owned[] flag
+ * (HOST, n_params) comes from bsrl_muon_workspace_bytes (-1 on error). */
+int64_t bsrl_muon_workspace_bytes(const bsrl_config* cfg, const int32_t* owned, int32_t n_params);
+int bsrl_muon_step(const bsrl_config* cfg, float* const* params, const float* const* grads, float* const* bufs,
+                   int32_t n_params, const float* lr, float weight_decay, float momentum, const float* found_inf,
+                   void* arena, int64_t arena_bytes, void* workspace, int64_t workspace_bytes, void* stream);
+
 /* --- forward -------------------------------------------------------------------- */
 int64_t bsrl_workspace_bytes(const bsrl_config* cfg, int64_t n_envs);
 

@@ -170,3 +170,34 @@ def test_packed_muon_matches_a_per_matrix_implementation_and_a_repack():
     muon2 = PackedMuon(m, names)
     muon2.load_state_dict(sd2)
     assert torch.equal(muon2.bufs[0], muon.bufs[0])
+
+
+@pytest.mark.parametrize("embed,heads,trunk,hidden", [(64, 2, 128, None), (96, 3, 160, 224), (192, 4, 384, None), (256, 8, 512, None)])
+def test_muon_products_are_fp32_accurate(embed, heads, trunk, hidden):
+    """The Newton-Schulz chain on split bf16 planes against float64, at widths that fill the 128-wide tiles, leave
+    remainders (96, 160, 224: padding to 64) and make tall, wide and square matrices: its error is that of a plain fp32
+    chain (bound: 1.5 times the fp32 chain's own error against float64, matrix by matrix; both are rounding noise of the
+    same size, so the worst of some thirty matrices may stand out by a fraction)."""
+    import math
+    from beatsaberrl_b200.optim import PackedMuon, orthogonalize
+    from beatsaberrl_b200.policy import NotePolicy
+    torch.manual_seed(3)
+    m = NotePolicy(embed=embed, trunk_dim=trunk, n_blocks=2, n_heads=heads, n_gears=5, trunk_hidden=hidden).cuda()
+    muon = PackedMuon(m, lr=1.0, momentum=0.5)
+    named = dict(m.named_parameters())
+    g = torch.Generator(device="cuda").manual_seed(7)
+    want = {}
+    for n in muon.names:
+        p = named[n]
+        p.zero_()                                # the step leaves -0.2 sqrt(max side) O in the master
+        p.grad = torch.randn(p.shape, generator=g, device="cuda") * 0.02
+        u = p.grad * 1.5
+        u = u.t() if u.shape[0] > u.shape[1] else u
+        want[n] = (orthogonalize(u[None].double())[0], orthogonalize(u[None])[0].double())
+    muon.step()
+    m.check_device()
+    for n, (exact, fp32) in want.items():
+        o = named[n].double() / (-0.2 * math.sqrt(max(named[n].shape)))
+        o = o.t() if o.shape[0] > o.shape[1] else o
+        err, own = float((o - exact).norm()), float((fp32 - exact).norm())
+        assert err <= 1.5 * own + 1e-7 * float(exact.norm()), (n, err, own)
