@@ -231,29 +231,32 @@ int run_trunk(const Ctx& c, const __half* lead16, float* raw) {
   const int64_t B = c.B;
   const float eps = c.cfg->eps;
   const RowMap ident = identity_map();
-  float* xt = at<float>(c.ws, w.xt);
-  __half* u = at<__half>(c.ws, w.u);
-  __half* r = at<__half>(c.ws, w.r);
-  __half* z = at<__half>(c.ws, w.z);
+  const TrainPtrs* tr = c.train;
+  float* xt = tr ? tr->xt : at<float>(c.ws, w.xt);
+  float* xt2 = tr ? tr->xt2 : xt;                 // in place where nothing needs the input afterwards
+  __half* u = tr ? tr->u : at<__half>(c.ws, w.u);
+  __half* r = tr ? tr->r : at<__half>(c.ws, w.r);
+  __half* z = tr ? tr->z : at<__half>(c.ws, w.z);
   const int ldz = d + D;
   g_stage = kStTrunk;
   BSRL_TRY(linear(linear_args(lead16, kLead * d, c.W(l.trunk_proj), kLead * d, c.Bv(l.trunk_proj), xt, D, 1, 0, B, D, kLead * d), c.st));
   if (l.trunk_v2) {
     // SimBaV2 (python/policy.py:1140-1155): x = l2n(s_in W_in z); y = l2n(W2 relu(s_1 W1 x));
     // x = l2n(x + alpha (y - x)); h = sqrt(D) x.  GEMMs on fp16 operands, everything else fp32.
-    float* t32 = at<float>(c.ws, w.t32);
-    BSRL_TRY(simba2_rows(0, xt, xt, at<float>(c.arena, l.v2_s_in), 0.f, B, D, u, D, c.st));
-    BSRL_TRY(linear(linear_args(u, D, c.W(l.trunk_fc1), D, c.Bv(l.trunk_fc1), t32, l.Hh, 1, 0, B, l.Hh, D), c.st));
-    BSRL_TRY(scale_relu_rows(t32, at<float>(c.arena, l.v2_s_1), B, l.Hh, r, c.st));
-    BSRL_TRY(linear(linear_args(r, l.Hh, c.W(l.trunk_fc2), l.Hh, c.Bv(l.trunk_fc2), t32, D, 1, 0, B, D, l.Hh), c.st));
-    BSRL_TRY(simba2_rows(1, t32, xt, at<float>(c.arena, l.v2_alpha), 0.5f * sqrtf((float)D), B, D, z + d, ldz, c.st));
+    float* t1 = tr ? tr->t1 : at<float>(c.ws, w.t32);
+    float* t2 = tr ? tr->t2 : at<float>(c.ws, w.t32);
+    BSRL_TRY(simba2_rows(0, xt, xt2, at<float>(c.arena, l.v2_s_in), 0.f, B, D, u, D, c.st));
+    BSRL_TRY(linear(linear_args(u, D, c.W(l.trunk_fc1), D, c.Bv(l.trunk_fc1), t1, l.Hh, 1, 0, B, l.Hh, D), c.st));
+    BSRL_TRY(scale_relu_rows(t1, at<float>(c.arena, l.v2_s_1), B, l.Hh, r, c.st));
+    BSRL_TRY(linear(linear_args(r, l.Hh, c.W(l.trunk_fc2), l.Hh, c.Bv(l.trunk_fc2), t2, D, 1, 0, B, D, l.Hh), c.st));
+    BSRL_TRY(simba2_rows(1, t2, xt2, at<float>(c.arena, l.v2_alpha), 0.5f * sqrtf((float)D), B, D, z + d, ldz, c.st));
   } else {
     BSRL_TRY(layernorm(xt, D, ident, c.G(l.trunk_ln1), c.Be(l.trunk_ln1), eps, B, D, u, D, c.st));
     BSRL_TRY(linear(linear_args(u, D, c.W(l.trunk_fc1), D, c.Bv(l.trunk_fc1), r, l.Hh, 0, 1, B, l.Hh, D), c.st));
-    LinearArgs p2 = linear_args(r, l.Hh, c.W(l.trunk_fc2), l.Hh, c.Bv(l.trunk_fc2), xt, D, 1, 0, B, D, l.Hh);
+    LinearArgs p2 = linear_args(r, l.Hh, c.W(l.trunk_fc2), l.Hh, c.Bv(l.trunk_fc2), xt2, D, 1, 0, B, D, l.Hh);
     p2.R = xt; p2.ldr = D;
     BSRL_TRY(linear(p2, c.st));
-    BSRL_TRY(layernorm(xt, D, ident, c.G(l.trunk_ln2), c.Be(l.trunk_ln2), eps, B, D, z + d, ldz, c.st));
+    BSRL_TRY(layernorm(xt2, D, ident, c.G(l.trunk_ln2), c.Be(l.trunk_ln2), eps, B, D, z + d, ldz, c.st));
   }
   return linear(linear_args(z + d, ldz, c.W(l.heads), D, c.Bv(l.heads), raw, l.head_cols_pad, 1, 0, B, l.head_cols_pad, D), c.st);
 }
@@ -417,7 +420,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
   }
 
   // SimBa trunk on the (B, 5d) readout; its output h lands in z[:, d:]; then the packed heads
-  __half* z = at<__half>(c.ws, w.z);
+  __half* z = c.train ? c.train->z : at<__half>(c.ws, w.z);
   const int ldz = d + D;
   float* raw = c.train ? c.train->raw : at<float>(c.ws, w.raw);
   BSRL_TRY(run_trunk(c, lead16, raw));

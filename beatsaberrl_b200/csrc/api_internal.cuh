@@ -27,16 +27,23 @@ inline const T* at(const void* base, int64_t off) {
 
 constexpr int kMaxBlocks = 32;
 
-// Where a grad-mode forward keeps what the backward needs (all caller memory): the tokenizer's feature
-// rows, the key bias, the residual stream ENTERING every block (block i reads x[i] and writes x[i + 1]
-// instead of updating one buffer in place), the readout rows and the head / value-bin outputs.
+// Where a grad-mode forward keeps what the backward needs (all caller memory): the tokenizer's feature rows, the key
+// bias, the residual stream ENTERING every block (block i reads x[i] and writes x[i + 1] instead of updating one buffer
+// in place), the readout and trunk activations and the head / value-bin outputs.
 struct TrainPtrs {
-  __half* feat;          // (29 B, 64) f16
-  float* key_bias;       // (B, 29) f32
-  float* x[kMaxBlocks];  // (29 B, d) f32, x[i] = stream entering block i
-  __half* lead16;        // (B, 5 d) f16 readout
-  float* raw;            // (B, head_cols_pad) f32
-  float* vraw;           // (B, bins_pad) f32
+  __half* feat;            // (29 B, 64) f16 encoder inputs
+  float* key_bias;         // (B, 29) f32
+  float* x[kMaxBlocks];    // (29 B, d) f32, x[i] = stream entering block i
+  __half* lead16;          // (B, 5 d) f16 readout
+  float* xt;               // (B, D) f32 trunk_proj (SimBaV2: W_in) output
+  float* xt2;              // (B, D) f32 input of trunk_ln2 (SimBaV2: x0)
+  float* t1;               // SimBaV2: (B, Hh) and (B, D) f32 outputs of W1 and W2
+  float* t2;
+  __half* u;               // (B, D) f16 operand of fc1
+  __half* r;               // (B, Hh) f16 operand of fc2
+  __half* z;               // (B, d + D) f16 [critic pool | trunk h]
+  float* raw;              // (B, head_cols_pad) f32
+  float* vraw;             // (B, bins_pad) f32
 };
 
 struct Ctx {

@@ -211,22 +211,51 @@ __global__ void __launch_bounds__(256) cast_rows16_kernel(const float* __restric
   }
 }
 
-// dst[map(r), :] (+)= src[r, :] (fp32 rows)
+// dst[map(r), :] += src[r, :] (fp32 rows); dst16, if given, gets the sums as fp16 (dense rows of n columns)
 __global__ void __launch_bounds__(256) add_rows_kernel(const float* __restrict__ src, int64_t lds, float* __restrict__ dst,
-                                                       int64_t ldd, RowMap dmap, int64_t rows, int n, int accumulate) {
+                                                       int64_t ldd, RowMap dmap, int64_t rows, int n, __half* __restrict__ dst16) {
   const int nv = n >> 2;
   const int64_t total = rows * nv;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     int piece;
     const int64_t r = div_index(i, nv, &piece);
     const int c = piece * 4;
+    const int64_t row = dmap(r);
     float4 v = *reinterpret_cast<const float4*>(src + r * lds + c);
-    float4* o = reinterpret_cast<float4*>(dst + dmap(r) * ldd + c);
-    if (accumulate) {
-      const float4 w = *o;
-      v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
-    }
+    float4* o = reinterpret_cast<float4*>(dst + row * ldd + c);
+    const float4 w = *o;
+    v.x += w.x; v.y += w.y; v.z += w.z; v.w += w.w;
     *o = v;
+    if (dst16) *reinterpret_cast<uint2*>(dst16 + row * n + c) = make_uint2(pack_half2(v.x, v.y), pack_half2(v.z, v.w));
+  }
+}
+
+// out[r, :] = in[map(r), :] (fp16 rows, dense output; n % 8 == 0)
+__global__ void __launch_bounds__(256) gather_rows16_kernel(const __half* __restrict__ in, int64_t ldi, RowMap imap,
+                                                            __half* __restrict__ out, int64_t rows, int n) {
+  const int nv = n >> 3;
+  const int64_t total = rows * nv;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    int piece;
+    const int64_t r = div_index(i, nv, &piece);
+    reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(in + imap(r) * ldi + piece * 8);
+  }
+}
+
+// token rows (env-major) -> the encoders' row order: 2 saber rows per env, then torso, 2 leg, 24 slot rows per env
+__global__ void __launch_bounds__(256) gather_tokens16_kernel(const __half* __restrict__ in, int64_t n_envs, int n,
+                                                              __half* __restrict__ out) {
+  const int nv = n >> 3;
+  const int64_t total = n_envs * kT * nv;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
+    int piece, tok;
+    const int64_t r = div_index(i, nv, &piece);
+    int64_t env;
+    if (r < 2 * n_envs) { env = r >> 1; tok = (int)(r & 1); }
+    else if (r < 3 * n_envs) { env = r - 2 * n_envs; tok = 2; }
+    else if (r < 5 * n_envs) { env = (r - 3 * n_envs) >> 1; tok = 3 + (int)((r - 3 * n_envs) & 1); }
+    else { env = div_index(r - 5 * n_envs, kSlots, &tok); tok += kLead; }
+    reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(in + (env * kT + tok) * n + piece * 8);
   }
 }
 
@@ -440,11 +469,25 @@ int cast_rows16(const float* in, int64_t ldi, RowMap imap, float scale, __half* 
   return BSRL_OK;
 }
 
-int add_rows32(const float* src, int64_t lds, float* dst, int64_t ldd, RowMap dmap, int64_t rows, int n, int accumulate,
-               cudaStream_t stream) {
+int add_rows32(const float* src, int64_t lds, float* dst, int64_t ldd, RowMap dmap, int64_t rows, int n, cudaStream_t stream,
+               __half* dst16) {
   if (rows == 0) return BSRL_OK;
-  add_rows_kernel<<<(unsigned)grid_for(rows * (n >> 2), 256), 256, 0, stream>>>(src, lds, dst, ldd, dmap, rows, n, accumulate);
+  add_rows_kernel<<<(unsigned)grid_for(rows * (n >> 2), 256), 256, 0, stream>>>(src, lds, dst, ldd, dmap, rows, n, dst16);
   BSRL_LAUNCH_OK("add_rows_kernel");
+  return BSRL_OK;
+}
+
+int gather_rows16(const __half* in, int64_t ldi, RowMap imap, __half* out, int64_t rows, int n, cudaStream_t stream) {
+  if (rows == 0) return BSRL_OK;
+  gather_rows16_kernel<<<(unsigned)grid_for(rows * (n >> 3), 256), 256, 0, stream>>>(in, ldi, imap, out, rows, n);
+  BSRL_LAUNCH_OK("gather_rows16_kernel");
+  return BSRL_OK;
+}
+
+int gather_tokens16(const __half* in, int64_t n_envs, int n, __half* out, cudaStream_t stream) {
+  if (n_envs == 0) return BSRL_OK;
+  gather_tokens16_kernel<<<(unsigned)grid_for(n_envs * kT * (n >> 3), 256), 256, 0, stream>>>(in, n_envs, n, out);
+  BSRL_LAUNCH_OK("gather_tokens16_kernel");
   return BSRL_OK;
 }
 

@@ -34,6 +34,7 @@ constexpr int EPI_WARPS = 8;
 constexpr int THREADS = (2 + EPI_WARPS) * 32;
 constexpr int TMEM_COLS = 2 * BN;               // two accumulator buffers = all 512 columns
 constexpr int STG_BYTES = 32 * 128;             // per-warp transposition buffer: 32 rows x 128 bytes
+constexpr int ONES_BYTES = 16 * 128;            // B operand of the column sums: 16 rows of 64 fp16 ones
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * STG_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 
 struct Shared {
@@ -98,6 +99,12 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLS);
     tmem_relinquish();
   }
+  // the tile of ones borrows the first epilogue warp's staging block: a launch with column sums has one work item per
+  // CTA, so the block is not staged into before the MMAs have retired
+  if (p.a_sums) {
+    for (int i = threadIdx.x; i < ONES_BYTES / 4; i += THREADS) reinterpret_cast<uint32_t*>(staging)[i] = 0x3c003c00u;
+    fence_proxy_async_smem();
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -156,6 +163,9 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         if (!mbar_wait(smem_u32(&sh->tmem_empty[buf]), acc_ph ^ 1, abort)) { give_up(sh, status, 3); ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
+        const bool sums = p.a_sums != nullptr && wi.nt == 0;     // into the second accumulator buffer, which is idle then
+        const uint32_t idesc1 = idesc_f16(BM, 16, 1, 0);
+        const uint64_t ones = smem_desc_sw128(smem_u32(staging));
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -167,6 +177,11 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
             mma_f16_ss(d_tmem, a_desc + a_step * k, w_desc + w_step * k, idesc, (kb != kb0 || k) ? 1u : 0u);
+          if (sums) {
+#pragma unroll
+            for (int k = 0; k < BK / 16; ++k)
+              mma_f16_ss(tmem_base + BN, a_desc + a_step * k, ones + 2 * k, idesc1, (kb != kb0 || k) ? 1u : 0u);
+          }
           tc_commit(smem_u32(&sh->empty[s]));
         }
         if (ok) tc_commit(smem_u32(&sh->tmem_full[buf]));
@@ -214,6 +229,13 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       }
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + half * (BN / 2);
+      if (p.a_sums && wi.nt == 0 && half == 0) {     // all 16 columns hold the same sum
+        uint32_t s16[16];
+        tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + BN, s16);
+        tmem_wait_ld();
+        const int64_t row = m0 + q * 32 + lane;
+        if (row < p.M) atomicAdd(p.a_sums + row, __uint_as_float(s16[0]));
+      }
 #pragma unroll 1
       for (int c = 0; c < BN / 2; c += cw) {
         const int col = n0 + half * (BN / 2) + c;     // first column of this block
@@ -295,7 +317,8 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0 && m0 + q * 32 < p.M) {
-            tma_store_2d(&tm_c, col, (int)(m0 + q * 32), smem_u32(stg));
+            if (splits > 1) tma_reduce_add_2d(&tm_c, col, (int)(m0 + q * 32), smem_u32(stg));
+            else tma_store_2d(&tm_c, col, (int)(m0 + q * 32), smem_u32(stg));
             bulk_commit();
           }
           continue;
@@ -465,7 +488,7 @@ bool linear_tc5_ok(const LinearArgs& p) {
   if (!p.A || !p.W || !p.C || p.M < 1) return false;
   if (p.N % 16 != 0 || p.N < 16 || p.K < 1) return false;
   if (!p.a_mn && !p.w_mn && p.K % BK != 0) return false;
-  if (p.K % 8 != 0) return false;                                // columns past K of a K-major operand read as zero
+  if (p.K % 8 != 0 && !(p.a_mn && p.w_mn)) return false;          // columns past K of a K-major operand read as zero
   if (p.a_mn && (p.M % 64 != 0 || p.lda < p.M)) return false;
   if (p.w_mn && (p.N % 64 != 0 || p.ldw < p.N)) return false;
   if (p.amap.group != 0x7fffffff || p.amap.first != 0) return false;      // TMA reads A rows in order
@@ -476,6 +499,12 @@ bool linear_tc5_ok(const LinearArgs& p) {
   if (p.k_splits > 1 && (!p.out_f32 || p.relu || p.R || p.mask)) return false;   // split-K adds raw fp32 partial products
   if (p.mask && (!aligned16(p.mask) || (p.ldm % 8) || p.cmap.group != 0x7fffffff || p.cmap.first != 0)) return false;
   return true;
+}
+
+// the column sums need one work item per CTA: they use the second accumulator buffer and a staging block
+bool linear_tc5_sums_ok(const LinearArgs& p) {
+  const int64_t tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  return p.a_mn && linear_tc5_ok(p) && tiles * (p.k_splits > 1 ? p.k_splits : 1) <= sm_count();
 }
 
 int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
@@ -492,6 +521,10 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
     set_error("linear: shape m=%lld n=%d k=%d does not fit the tcgen05 engine", (long long)p.M, p.N, p.K);
     return BSRL_ERR_UNSUPPORTED;
   }
+  if (p.a_sums && !linear_tc5_sums_ok(p)) {
+    set_error("linear: column sums need row-contraction operands and at most one work item per SM");
+    return BSRL_ERR_UNSUPPORTED;
+  }
   int* status = device_status_ptr();
   if (!status) return BSRL_ERR_CUDA;
   CUtensorMap tm_a, tm_w;
@@ -499,8 +532,9 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
     return BSRL_ERR_CUDA;
   if (p.w_mn ? !make_tmap_mn(&tm_w, p.W, p.K, p.N, p.ldw, BK, BN / 64) : !make_tmap_f16(&tm_w, p.W, p.N, p.K, p.ldw, BN))
     return BSRL_ERR_CUDA;
-  // dense output rows without a residual leave as TMA stores of the epilogue's 32 x 128-byte staging blocks
-  const bool tma_c = !p.R && p.k_splits <= 1 && p.cmap.group == 0x7fffffff && p.cmap.stride == 0 && p.cmap.first == 0 &&
+  // dense output rows without a residual leave as TMA stores (split-K: TMA additions) of the epilogue's 32 x 128-byte
+  // staging blocks
+  const bool tma_c = !p.R && p.cmap.group == 0x7fffffff && p.cmap.stride == 0 && p.cmap.first == 0 &&
                      p.M <= 0x7fffff00;
   CUtensorMap tm_c = tm_a;
   if (tma_c && !make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, p.M, p.N, p.ldc, 32, 128)) return BSRL_ERR_CUDA;

@@ -36,6 +36,10 @@ struct LinearArgs {
   // pitch ldm, dense rows) is not positive are written as zero.
   const __half* mask = nullptr;
   int ldm = 0;
+  // Column sums of the (K, M) A matrix, added to M floats (a_mn products; a weight gradient's bias gradient): an
+  // MMA against a tile of ones beside each k-block's MMAs, so A is not read a second time.  Only where
+  // linear_tc5_sums_ok says so.
+  float* a_sums = nullptr;
 };
 LinearArgs linear_args(const __half* A, int lda, const __half* W, int ldw, const float* bias,
                        void* C, int ldc, int out_f32, int relu, int64_t M, int N, int K);
@@ -43,6 +47,7 @@ LinearArgs linear_args(const __half* A, int lda, const __half* W, int ldw, const
 int linear_mma(const LinearArgs& p, cudaStream_t stream);   // warp-MMA engine
 int linear_tc5(const LinearArgs& p, cudaStream_t stream);   // tcgen05 / TMEM engine
 bool linear_tc5_ok(const LinearArgs& p);                     // shape fits the tcgen05 engine
+bool linear_tc5_sums_ok(const LinearArgs& p);                // ... and its column sums can ride along (a_sums)
 
 // Projection + residual + LayerNorm in one kernel (gemm_ln_tc5.cu): x_out = R + A W^T + bias (fp32), h =
 // LayerNorm(x_out) (fp16).  N a multiple of 64 up to 512 (of 128 above 256), K a multiple of 64.  R and x_out

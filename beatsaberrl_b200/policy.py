@@ -108,19 +108,15 @@ class _RecomputeFn(torch.autograd.Function):
                 entropy.data_ptr(), ent_h.data_ptr(), value.data_ptr(), vlogits.data_ptr(), save.data_ptr(),
                 save.numel(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
         ctx.policy, ctx.save, ctx.action, ctx.B = policy, save, action, B
-        ctx.needs = [p.requires_grad for p in params]
         ctx.mark_non_differentiable(ent_h)
+        ctx.set_materialize_grads(False)        # outputs the loss does not use: no gradient instead of zeros
         return logits, logprob, entropy, value, vlogits, ent_h
 
     @staticmethod
     def backward(ctx, g_logits, g_logprob, g_entropy, g_value, g_vlogits, _g_ent_h):
         policy, B = ctx.policy, ctx.B
         cfg, dev = policy._cfg, ctx.save.device
-        n = len(policy._param_table)
-        offs = (C.c_int64 * n)()
-        total = nat.lib.bsrl_grad_floats(C.byref(cfg), offs, n)
-        if total < 0:
-            raise nat.BsrlError(int(total), nat.last_error())
+        total, pieces, order = policy._grad_pieces()
         flat = torch.empty(total, dtype=torch.float32, device=dev)
         n_ws = nat.lib.bsrl_backward_workspace_bytes(C.byref(cfg), B)
         ws = torch.empty(max(n_ws, 256), dtype=torch.uint8, device=dev)
@@ -136,14 +132,10 @@ class _RecomputeFn(torch.autograd.Function):
                 ctx.save.data_ptr(), ctx.save.numel(), ptr(ups[0]), ptr(ups[1]), ptr(ups[2]), ptr(ups[3]), ptr(ups[4]),
                 scale, flat.data_ptr(), total, ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream))
         flat.mul_(1.0 / scale)
-        grads = []
-        for i, (_, rows, cols) in enumerate(policy._param_table):
-            if not ctx.needs[i]:
-                grads.append(None)
-                continue
-            grads.append(flat[offs[i]: offs[i] + rows * cols])
+        views = torch._C._nn.unflatten_dense_tensors(flat, pieces)
+        needs = ctx.needs_input_grad[3:]
         ctx.save = None
-        return (None, None, None, *grads)
+        return (None, None, None, *[views[k] if need else None for k, need in zip(order, needs)])
 
 
 class NotePolicy(nn.Module):
@@ -260,6 +252,8 @@ class NotePolicy(nn.Module):
         self._arena_version = None
         self._workspaces = {}
         self._rng_state = None
+        self._param_places = None
+        self._grad_cut = None
 
     # ------------------------------------------------------------------ weights
     def _pack(self, force: bool = False) -> None:
@@ -375,12 +369,39 @@ class NotePolicy(nn.Module):
         """Grad-mode forward: one autograd node over all parameters (see ``_RecomputeFn``)."""
         obs = self._check_obs(obs)
         self._pack()
-        named = dict(self.named_parameters())
-        params = [named[n] for n, _, _ in self._param_table]
-        shapes = [p.shape for p in params]
-        flat_params = [p.reshape(-1) if p.dim() != 1 else p for p in params]   # the node hands back flat gradients
-        del shapes
-        return _RecomputeFn.apply(self, obs, action, *flat_params)
+        return _RecomputeFn.apply(self, obs, action, *self._table_params())
+
+    def _table_params(self) -> list:
+        """The live parameters in the library's order.  Walking the module tree for their names takes longer than a
+        small update's kernels, so the (module, attribute) places are looked up once; the parameters are read from
+        them on every call."""
+        if self._param_places is None:
+            places = {}
+            for prefix, mod in self.named_modules():
+                for name in mod._parameters:
+                    places[f"{prefix}.{name}" if prefix else name] = (mod._parameters, name)
+            self._param_places = [places[n] for n, _, _ in self._param_table]
+        return [d[k] for d, k in self._param_places]
+
+    def _grad_pieces(self):
+        """The flat gradient buffer's length, empty stand-ins whose shapes cut it into the parameters' gradients and the
+        gaps between them (in buffer order), and the index of every parameter's piece."""
+        if self._grad_cut is None:
+            n = len(self._param_table)
+            offs = (C.c_int64 * n)()
+            total = nat.lib.bsrl_grad_floats(C.byref(self._cfg), offs, n)
+            if total < 0:
+                raise nat.BsrlError(int(total), nat.last_error())
+            pieces, order, at = [], [0] * n, 0
+            for i in sorted(range(n), key=lambda i: offs[i]):
+                if offs[i] > at:
+                    pieces.append(torch.empty(offs[i] - at, device="meta"))
+                order[i] = len(pieces)
+                pieces.append(torch.empty(self._table_params()[i].shape, device="meta"))
+                at = offs[i] + pieces[-1].numel()
+            pieces.append(torch.empty(total - at, device="meta"))
+            self._grad_cut = (int(total), pieces, order)
+        return self._grad_cut
 
     def forward_stacked(self, obs: torch.Tensor):
         """obs (B, 630) -> stacked logits (B, 29, k_max) fp32 + the critic's value (B,) fp32.  In grad mode
