@@ -37,7 +37,8 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const float* __restrict__ x
   for (int i = 0; i < kMaxVec; ++i) acc_g[i] = acc_b[i] = make_float4(0.f, 0.f, 0.f, 0.f);
   for (int64_t row = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows; row += warps) {
     const float4* xr = reinterpret_cast<const float4*>(x + xmap(row) * ldx);
-    float4 v[kMaxVec], g[kMaxVec];
+    float4 v[kMaxVec], g[kMaxVec], r[kMaxVec];        // r: the residual gradient, requested with the rest of the row
+    const int64_t go = gmap(row) * ldg;
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < kMaxVec; ++i) {
@@ -53,6 +54,7 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const float* __restrict__ x
           const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
           g[i] = make_float4(a.x, a.y, b.x, b.y);
         }
+        r[i] = gres ? reinterpret_cast<const float4*>(gres + go)[c] : make_float4(0.f, 0.f, 0.f, 0.f);
       }
     }
     const float mean = warp_sum(s) / d;
@@ -80,7 +82,6 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const float* __restrict__ x
     }
     s1 = warp_sum(s1) / d;
     s2 = warp_sum(s2) / d;
-    const int64_t go = gmap(row) * ldg;
 #pragma unroll
     for (int i = 0; i < kMaxVec; ++i) {
       const int c = lane + i * 32;
@@ -88,8 +89,7 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const float* __restrict__ x
         float4 o = make_float4(rstd * (g[i].x - s1 - v[i].x * s2), rstd * (g[i].y - s1 - v[i].y * s2),
                                rstd * (g[i].z - s1 - v[i].z * s2), rstd * (g[i].w - s1 - v[i].w * s2));
         if (gres) {
-          const float4 r = reinterpret_cast<const float4*>(gres + go)[c];
-          o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w;
+          o.x += r[i].x; o.y += r[i].y; o.z += r[i].z; o.w += r[i].w;
         }
         reinterpret_cast<float4*>(gx_out + go)[c] = o;
         if (gx16)      // the same gradient as the fp16 operand of the products that follow (dense rows)

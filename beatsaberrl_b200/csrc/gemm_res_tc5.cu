@@ -1,0 +1,417 @@
+// tcgen05 linear layer with the weight tile resident in shared memory: C = act(A W^T + bias) (+ residual) for K <= 256
+// over many rows (the token-row products of the backward and of the unfused forward paths).
+//
+// gemm_tc5.cu streams A and W tiles together; with K <= 256 that draws 192 KB from L2 per 128 x 256 output tile -- 4 to
+// 5 K cycles at what an SM gets from L2 -- where the tile's HBM traffic (64 KB in, 64 KB out) needs 3 K.  Here a CTA
+// works down the row tiles of ONE column tile: its weights (<= 128 KB) are loaded once, only A streams, through a ring
+// of 16 KB stages over the rest of the 192 KB.  Roles as in gemm_tc5.cu:
+//   warp 0      TMA producer;   warp 1      MMA issuer (one thread, M = 128, N <= 256, two TMEM accumulators);
+//   warps 2..9  epilogue.
+//
+// What bounds it now is the epilogue's chain of latencies (475 K x 768 x 256: MMAs alone 156 us, loads hidden, epilogue
+// alone about 200), so the next block's accumulator is requested before this block is staged, residual rows a block
+// ahead (and the next tile's into L2), and the bias sits in shared memory.  Its loops stay rolled: unrolled they spill.
+// Other ways of writing the rows measured slower: threads storing their own row in 32-byte pieces 418 us, boxes of
+// 64 bytes per row through three buffers 278 us (a TMA store costs the same whatever its size).
+// Measured, 475 K rows, same box as gemm_tc5.cu: x 768 x 256 fp16 269 -> 227 us, x 768 x 192 302 -> 236, x 1024 x 128
+// 347 -> 268, x 192 x 192 fp32 + residual 296 -> 229, x 256 x 256 fp32 + residual 316 -> 290.
+//
+// ReLU masks as bits: a product with ReLU can leave one bit per output (1 = positive), which the product that carries
+// the gradient back reads instead of the fp16 activations: 1/16 of their bytes.  One 32-bit word holds 32 columns of
+// one row (bit i: column 2 i, bit 16 + i: column 2 i + 1); word (c / 32) * ld + row, so that a warp's 32 rows are 128
+// contiguous bytes.
+#include "kernels.cuh"
+#include "tc5.cuh"
+
+namespace bsrl {
+namespace {
+using namespace tc5;
+
+constexpr int BM = 128, BN = 256, BK = 64;
+constexpr int A_BYTES = BM * BK * 2, W_BYTES = BN * BK * 2;
+constexpr int OPERAND_BYTES = 192 * 1024;       // weights, A ring and second staging buffers
+constexpr int MAX_STAGES = 10;
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = (2 + EPI_WARPS) * 32;
+constexpr int TMEM_COLS = 2 * BN;
+constexpr int STG_BYTES = 32 * 128;             // staging buffer: 32 rows x 128 bytes
+constexpr int SMEM_BYTES = OPERAND_BYTES + EPI_WARPS * STG_BYTES + BN * 4 /*bias*/ + 1024 /*alignment*/ + 256 /*barriers*/;
+constexpr int KERNEL_ID = 10;
+
+struct Shared {
+  uint64_t full[MAX_STAGES], empty[MAX_STAGES], tmem_full[2], tmem_empty[2], mma_done, w_full;
+  uint32_t tmem_base;
+  int abort;
+};
+static_assert(sizeof(Shared) <= 256, "barrier space");
+
+__device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
+  atomicCAS(status, 0, KERNEL_ID * 16 + role);
+  sh->abort = 1;
+}
+
+// 32 fp32 values of a residual row (the first `left` of them exist, a multiple of 16; wide: 32-byte aligned)
+struct Row32 {
+  float v[32];
+  __device__ __forceinline__ void load(const float* p, int left, bool wide) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float* o = v + 8 * j;
+      if (8 * j >= left) {
+#pragma unroll
+        for (int t = 0; t < 8; ++t) o[t] = 0.f;
+      } else if (wide) {
+        asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7])
+                     : "l"(p + 8 * j)
+                     : "memory");
+      } else {
+        const float4 a = *reinterpret_cast<const float4*>(p + 8 * j), b = *reinterpret_cast<const float4*>(p + 8 * j + 4);
+        o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w; o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+      }
+    }
+  }
+};
+
+// fp16 pairs after a ReLU (non-negative): bits i and 16 + i of the word for pair i's two values
+__device__ __forceinline__ uint32_t positive_bits(const uint32_t* h) {
+  uint32_t w = 0;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) w |= ((h[i] + 0x7fff7fffu) >> (15 - i)) & (0x00010001u << i);
+  return w;
+}
+// pair i's halves of a packed gradient, zeroed where their bits are
+__device__ __forceinline__ uint32_t keep_positive(uint32_t h, uint32_t w, int i) { return h & (((w >> i) & 0x00010001u) * 0xffffu); }
+
+template <bool HAS_R>
+__global__ void __launch_bounds__(THREADS, 1)
+linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
+                  const __grid_constant__ CUtensorMap tm_c, int tma_c, int r32, LinearArgs p, int m_tiles, int n_tiles,
+                  int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  const int k_blocks = (p.K + BK - 1) / BK;
+  // a second staging buffer per epilogue warp where the weights leave the ring at least four stages
+  const int nbuf = k_blocks <= 3 ? 2 : 1;
+  const int ring_bytes = OPERAND_BYTES - (nbuf - 1) * EPI_WARPS * STG_BYTES;
+  const int n_st = min(MAX_STAGES, (ring_bytes - k_blocks * W_BYTES) / A_BYTES);
+  const uint32_t w_base = base + n_st * A_BYTES;
+  uint8_t* staging = smem_raw + (base - raw) + ring_bytes;
+  float* s_bias = reinterpret_cast<float*>(staging + EPI_WARPS * nbuf * STG_BYTES);
+  Shared* sh = reinterpret_cast<Shared*>(s_bias + BN);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // this CTA's column tile, its first row tile and the step to the next
+  const int nt = (int)(blockIdx.x % (unsigned)n_tiles), n0 = nt * BN;
+  const int t0 = (int)(blockIdx.x / (unsigned)n_tiles), t_step = ((int)gridDim.x - nt + n_tiles - 1) / n_tiles;
+  volatile int* abort = &sh->abort;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < n_st; ++s) {
+      mbar_init(smem_u32(&sh->full[s]), 1);
+      mbar_init(smem_u32(&sh->empty[s]), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&sh->tmem_full[b]), 1);
+      mbar_init(smem_u32(&sh->tmem_empty[b]), EPI_WARPS);
+    }
+    mbar_init(smem_u32(&sh->mma_done), 1);
+    mbar_init(smem_u32(&sh->w_full), 1);
+    sh->abort = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tm_a);
+    tma_prefetch_desc(&tm_w);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLS);
+    tmem_relinquish();
+  }
+  for (int i = threadIdx.x; i < BN; i += THREADS) s_bias[i] = p.bias && n0 + i < p.N ? p.bias[n0 + i] : 0.f;
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = sh->tmem_base;
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- TMA producer
+    if (lane == 0 && t0 < m_tiles) {
+      const uint32_t w_bar = smem_u32(&sh->w_full);
+      mbar_expect_tx(w_bar, (uint32_t)k_blocks * W_BYTES);
+      for (int kb = 0; kb < k_blocks; ++kb) {
+        if (p.w_mn) tma_load_3d(w_base + kb * W_BYTES, &tm_w, 0, kb * BK, n0 / 64, w_bar);
+        else tma_load_2d(w_base + kb * W_BYTES, &tm_w, kb * BK, n0, w_bar);
+      }
+      uint32_t it = 0, slot = 0, phase = 0;
+      bool ok = true;
+      for (int t = t0; t < m_tiles && ok; t += t_step) {
+        for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+          if (!mbar_wait(smem_u32(&sh->empty[slot]), phase ^ 1, abort)) { give_up(sh, status, 1); ok = false; break; }
+          const uint32_t bar = smem_u32(&sh->full[slot]);
+          mbar_expect_tx(bar, A_BYTES);
+          tma_load_2d(base + slot * A_BYTES, &tm_a, kb * BK, t * BM, bar);
+          if (++slot == (uint32_t)n_st) { slot = 0; phase ^= 1; }
+        }
+      }
+      // loads in flight must land before this CTA may exit (also when a wait above gave up): bounded, ignoring abort
+      uint32_t spins = 0;
+      for (uint32_t j = it > (uint32_t)n_st ? it - n_st : 0; j < it; ++j)
+        while (!mbar_try_wait(smem_u32(&sh->full[j % n_st]), (j / n_st) & 1) && ++spins < kSpinLimit) {}
+      while (!mbar_try_wait(w_bar, 0) && ++spins < kSpinLimit) {}
+      if (spins >= kSpinLimit) give_up(sh, status, 2);
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- MMA issuer
+    if (lane == 0) {
+      uint32_t tile_i = 0, slot = 0, phase = 0;
+      bool ok = true;
+      const uint32_t idesc = idesc_f16(BM, min(p.N - n0, BN), 0, p.w_mn);
+      const uint32_t w_step = p.w_mn ? 128u : 2u;            // 16-byte units per K step of 16
+      if (t0 < m_tiles && !mbar_wait(smem_u32(&sh->w_full), 0, abort)) { give_up(sh, status, 4); ok = false; }
+      for (int t = t0; t < m_tiles && ok; t += t_step, ++tile_i) {
+        const int buf = tile_i & 1;
+        if (!mbar_wait(smem_u32(&sh->tmem_empty[buf]), ((tile_i >> 1) & 1) ^ 1, abort)) { give_up(sh, status, 3); ok = false; break; }
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + buf * BN;
+        for (int kb = 0; kb < k_blocks; ++kb) {
+          if (!mbar_wait(smem_u32(&sh->full[slot]), phase, abort)) { give_up(sh, status, 4); ok = false; break; }
+          tc_fence_after();
+          const uint64_t a_desc = smem_desc_sw128(base + slot * A_BYTES);
+          const uint32_t w_addr = w_base + kb * W_BYTES;
+          const uint64_t w_desc = p.w_mn ? smem_desc_mn_sw128(w_addr, BK * 128) : smem_desc_sw128(w_addr);
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) mma_f16_ss(d_tmem, a_desc + 2 * k, w_desc + w_step * k, idesc, (kb || k) ? 1u : 0u);
+          tc_commit(smem_u32(&sh->empty[slot]));
+          if (++slot == (uint32_t)n_st) { slot = 0; phase ^= 1; }
+        }
+        if (ok) tc_commit(smem_u32(&sh->tmem_full[buf]));
+      }
+      // every MMA issued must have retired before TMEM is freed (bounded, ignoring abort)
+      tc_commit(smem_u32(&sh->mma_done));
+      uint32_t spins = 0;
+      while (!mbar_try_wait(smem_u32(&sh->mma_done), 0) && ++spins < kSpinLimit) {}
+      if (spins >= kSpinLimit) give_up(sh, status, 6);
+    }
+  } else {
+    // ---------------------------------------------------------------- epilogue warps
+    // 32 rows x 128 columns each, in blocks of 128 bytes per row; TMEM hands every thread one ROW.  A block leaves as one
+    // TMA store of the warp's swizzled staging buffer, or, where C's rows are scattered by a map, eight lanes per row
+    // copy it out.
+    const int q = warp & 3;                    // TMEM lane quadrant this warp may read
+    const int h0 = ((warp - 2) >> 2) * (BN / 2), c0 = n0 + h0;   // first column of this warp's half, in the tile and in C
+    uint8_t* const stg0 = staging + (warp - 2) * (nbuf * STG_BYTES);
+    uint8_t* stg = stg0;
+    const int sub = lane >> 3, piece = lane & 7;   // copying the buffer out: row sub + 4 i, 16-byte piece
+    auto wait_staging = [&]() {                // the block that used the buffer last has left it
+      if (nbuf == 2) stg = stg == stg0 ? stg0 + STG_BYTES : stg0;
+      if (tma_c && lane == 0) {
+        if (nbuf == 2) bulk_wait_read<1>();
+        else bulk_wait_read<0>();
+      }
+      __syncwarp();
+    };
+    auto put = [&](int pc, uint4 v) { *reinterpret_cast<uint4*>(stg + lane * 128 + ((pc ^ (lane & 7)) << 4)) = v; };
+    // bias and activation on 32 accumulator columns from column h0 + x of the tile on, in place
+    auto finish = [&](uint32_t (&a)[32], int x) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 bv = *reinterpret_cast<const float4*>(s_bias + h0 + x + 4 * j);
+        a[4 * j] = __float_as_uint(__uint_as_float(a[4 * j]) + bv.x);
+        a[4 * j + 1] = __float_as_uint(__uint_as_float(a[4 * j + 1]) + bv.y);
+        a[4 * j + 2] = __float_as_uint(__uint_as_float(a[4 * j + 2]) + bv.z);
+        a[4 * j + 3] = __float_as_uint(__uint_as_float(a[4 * j + 3]) + bv.w);
+      }
+      if (p.relu == 1) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(fmaxf(__uint_as_float(a[j]), 0.f));
+      } else if (p.relu == 2) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(gelu_exact(__uint_as_float(a[j])));
+      }
+    };
+    uint32_t tile_i = 0;
+    for (int t = t0; t < m_tiles; t += t_step, ++tile_i) {
+      const int64_t m0 = (int64_t)t * BM + q * 32;           // this warp's first row
+      const int buf = tile_i & 1;
+      const int64_t row = m0 + lane;
+      const bool live = row < p.M;
+      int64_t crow[8];                                       // rows this lane copies out where C's rows are scattered
+      if (!tma_c) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int64_t r = m0 + 4 * i + sub;
+          crow[i] = r < p.M ? p.cmap(r) * (int64_t)p.ldc : -1;
+        }
+      }
+      // the filled buffer (128 bytes of each of the warp's 32 rows, from column x on) -> C
+      auto emit = [&](int x, int elem) {
+        if (tma_c) {
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0 && m0 < p.M) {
+            tma_store_2d(&tm_c, x, (int)m0, smem_u32(stg));
+            bulk_commit();
+          }
+          return;
+        }
+        __syncwarp();
+        const int c = x + piece * (16 / elem);
+        if (c >= p.N) return;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          if (crow[i] < 0) continue;
+          const int rr = 4 * i + sub;
+          *reinterpret_cast<uint4*>(static_cast<uint8_t*>(p.C) + (crow[i] + c) * elem) =
+              *reinterpret_cast<const uint4*>(stg + rr * 128 + ((piece ^ (rr & 7)) << 4));
+        }
+      };
+      const float* rrow = nullptr;
+      Row32 res;
+      if (HAS_R && live) {
+        rrow = p.R + p.rmap(row) * (int64_t)p.ldr;
+        if (c0 < p.N) res.load(rrow + c0, p.N - c0, r32);
+        const int64_t rown = row + (int64_t)t_step * BM;     // the next tile's residual rows into L2
+        if (rown < p.M) {
+          const float* rn = p.R + p.rmap(rown) * (int64_t)p.ldr + c0;
+#pragma unroll
+          for (int c = 0; c < BN / 2; c += 32)
+            if (c0 + c < p.N) prefetch_l2(rn + c);
+        }
+      }
+      if (!mbar_wait_warp(smem_u32(&sh->tmem_full[buf]), (tile_i >> 1) & 1, abort)) {
+        if (lane == 0) give_up(sh, status, 5);
+        break;
+      }
+      tc_fence_after();
+      const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + h0;
+      if (HAS_R || p.out_f32) {
+        // ---- 32 columns at a time
+        uint32_t a[32];
+        if (c0 < p.N) tmem_ld32(tbase, a);
+#pragma unroll 1
+        for (int st = 0; st < BN / 64; ++st) {
+          const int col = c0 + 32 * st, left = p.N - col;    // columns from here on
+          if (left <= 0) break;                              // warp-uniform
+          tmem_wait_ld();
+          finish(a, 32 * st);
+          if (HAS_R) {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(__uint_as_float(a[j]) + res.v[j]);
+            if (rrow && left > 32 && st + 1 < BN / 64) res.load(rrow + col + 32, left - 32, r32);
+          }
+          if (p.out_f32) {
+            wait_staging();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) put(j, make_uint4(a[4 * j], a[4 * j + 1], a[4 * j + 2], a[4 * j + 3]));
+          } else {                                           // fp16 rows with a residual: half a block at a time
+            if (!(st & 1)) wait_staging();
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              put(4 * (st & 1) + j, make_uint4(pack_half2(__uint_as_float(a[8 * j]), __uint_as_float(a[8 * j + 1])),
+                                               pack_half2(__uint_as_float(a[8 * j + 2]), __uint_as_float(a[8 * j + 3])),
+                                               pack_half2(__uint_as_float(a[8 * j + 4]), __uint_as_float(a[8 * j + 5])),
+                                               pack_half2(__uint_as_float(a[8 * j + 6]), __uint_as_float(a[8 * j + 7]))));
+          }
+          if (st + 1 < BN / 64 && left > 32) tmem_ld32(tbase + 32 * (st + 1), a);
+          if (p.out_f32) emit(col, 4);
+          else if ((st & 1) || left <= 32) emit(col - 32 * (st & 1), 2);
+        }
+      } else {
+        // ---- fp16, 64 columns at a time
+        uint32_t a[32], b[32], h[32];
+        if (c0 < p.N) {
+          tmem_ld32(tbase, a);
+          tmem_ld32(tbase + 32, b);
+        }
+#pragma unroll 1
+        for (int st = 0; st < BN / 128; ++st) {
+          const int col = c0 + 64 * st;
+          if (col >= p.N) break;
+          uint32_t w0 = 0, w1 = 0;
+          if (p.bits_in && live) {
+            w0 = p.bits_in[(int64_t)(col >> 5) * p.bits_ld + row];
+            if (col + 32 < p.N) w1 = p.bits_in[(int64_t)((col >> 5) + 1) * p.bits_ld + row];
+          }
+          tmem_wait_ld();
+          finish(a, 64 * st);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) h[j] = pack_half2(__uint_as_float(a[2 * j]), __uint_as_float(a[2 * j + 1]));
+          finish(b, 64 * st + 32);
+#pragma unroll
+          for (int j = 0; j < 16; ++j) h[16 + j] = pack_half2(__uint_as_float(b[2 * j]), __uint_as_float(b[2 * j + 1]));
+          if (st + 1 < BN / 128 && col + 64 < p.N) {
+            tmem_ld32(tbase + 64 * (st + 1), a);
+            tmem_ld32(tbase + 64 * (st + 1) + 32, b);
+          }
+          if (p.bits_in) {
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              h[j] = keep_positive(h[j], w0, j);
+              h[16 + j] = keep_positive(h[16 + j], w1, j);
+            }
+          }
+          if (p.bits_out && live) {
+            p.bits_out[(int64_t)(col >> 5) * p.bits_ld + row] = positive_bits(h);
+            if (col + 32 < p.N) p.bits_out[(int64_t)((col >> 5) + 1) * p.bits_ld + row] = positive_bits(h + 16);
+          }
+          wait_staging();
+#pragma unroll
+          for (int j = 0; j < 8; ++j) put(j, make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]));
+          emit(col, 2);
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(smem_u32(&sh->tmem_empty[buf]));
+    }
+    if (tma_c && lane == 0) bulk_wait_all();      // the stores are complete before the CTA exits
+  }
+
+  // ------------------------------------------------------------------ teardown
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+}
+}  // namespace
+
+// fp32 rows without a residual stay with gemm_tc5.cu (475 K x 256 x 128: 105 us there, 120 here: four stores per half
+// tile either way, nothing to overlap them with).  K <= 256 in whole k-blocks or row-contraction weights, and at least three row tiles per CTA for the resident weights:
+// with one or two their load (128 KB before the first MMA) costs more than it saves.  fp16 masks are read by
+// gemm_tc5.cu (here only as bits).
+bool linear_res_ok(const LinearArgs& p) {
+  const int64_t tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
+  return !p.a_mn && !p.mask && (!p.out_f32 || p.R) && !p.a_sums && p.k_splits <= 1 && p.K <= 4 * BK && p.M <= 0x7fffff00 && tiles >= 3ll * sm_count() &&
+         (!(p.bits_in || p.bits_out) || (!p.out_f32 && !p.R && p.N % 32 == 0)) && linear_tc5_ok(p);
+}
+
+int linear_res(const LinearArgs& p, cudaStream_t stream) {
+  if (!linear_res_ok(p)) {
+    set_error("linear_res: shape m=%lld n=%d k=%d does not fit the resident-weight kernel", (long long)p.M, p.N, p.K);
+    return BSRL_ERR_UNSUPPORTED;
+  }
+  int* status = device_status_ptr();
+  if (!status) return BSRL_ERR_CUDA;
+  CUtensorMap tm_a, tm_w;
+  if (!make_tmap_f16(&tm_a, p.A, p.M, p.K, p.lda, BM)) return BSRL_ERR_CUDA;
+  if (p.w_mn ? !make_tmap_mn(&tm_w, p.W, p.K, p.N, p.ldw, BK, BN / 64) : !make_tmap_f16(&tm_w, p.W, p.N, p.K, p.ldw, BN))
+    return BSRL_ERR_CUDA;
+  const bool tma_c = p.cmap.group == 0x7fffffff && p.cmap.stride == 0 && p.cmap.first == 0;    // dense output rows
+  CUtensorMap tm_c = tm_a;
+  if (tma_c && !make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, p.M, p.N, p.ldc, 32, 128)) return BSRL_ERR_CUDA;
+  static DeviceOnce once;
+  int rc = once.run("linear_res_kernel set-up", [] {
+    cudaError_t e = cudaFuncSetAttribute(linear_res_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(linear_res_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+  });
+  if (rc != BSRL_OK) return rc;
+  const int m_tiles = (int)((p.M + BM - 1) / BM), n_tiles = (p.N + BN - 1) / BN;
+  const int r32 = p.R && reinterpret_cast<uintptr_t>(p.R) % 32 == 0 && p.ldr % 8 == 0;        // 32-byte residual loads
+  auto* kernel = p.R ? linear_res_kernel<true> : linear_res_kernel<false>;
+  kernel<<<sm_count(), THREADS, SMEM_BYTES, stream>>>(tm_a, tm_w, tm_c, tma_c ? 1 : 0, r32, p, m_tiles, n_tiles, status);
+  BSRL_LAUNCH_OK("linear_res_kernel");
+  return BSRL_OK;
+}
+
+}  // namespace bsrl

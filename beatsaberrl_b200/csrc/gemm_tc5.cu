@@ -62,7 +62,9 @@ __device__ __forceinline__ WorkItem work_item(int64_t w, int n_tile_work, int n_
 
 // HAS_R: a residual is added in the epilogue (its prefetch registers and address arithmetic are compiled
 // out otherwise: they cost the residual-free fp32 epilogue ~15 %).
-template <bool HAS_R>
+// SUMS: column sums of A beside the product (LinearArgs::a_sums), compiled in only where asked for: the untaken branch
+// alone cost the MMA thread 0.1 us per k-block.
+template <bool HAS_R, bool SUMS>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                   const __grid_constant__ CUtensorMap tm_c, int tma_c, LinearArgs p, int m_tiles, int n_tiles,
@@ -101,7 +103,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   }
   // the tile of ones borrows the first epilogue warp's staging block: a launch with column sums has one work item per
   // CTA, so the block is not staged into before the MMAs have retired
-  if (p.a_sums) {
+  if (SUMS) {
     for (int i = threadIdx.x; i < ONES_BYTES / 4; i += THREADS) reinterpret_cast<uint32_t*>(staging)[i] = 0x3c003c00u;
     fence_proxy_async_smem();
   }
@@ -163,9 +165,9 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         if (!mbar_wait(smem_u32(&sh->tmem_empty[buf]), acc_ph ^ 1, abort)) { give_up(sh, status, 3); ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
-        const bool sums = p.a_sums != nullptr && wi.nt == 0;     // into the second accumulator buffer, which is idle then
+        const bool sums = SUMS && wi.nt == 0;     // into the second accumulator buffer, which is idle then
         const uint32_t idesc1 = idesc_f16(BM, 16, 1, 0);
-        const uint64_t ones = smem_desc_sw128(smem_u32(staging));
+        const uint64_t ones = SUMS ? smem_desc_sw128(smem_u32(staging)) : 0;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
@@ -229,7 +231,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       }
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + buf * BN + half * (BN / 2);
-      if (p.a_sums && wi.nt == 0 && half == 0) {     // all 16 columns hold the same sum
+      if (SUMS && wi.nt == 0 && half == 0) {     // all 16 columns hold the same sum
         uint32_t s16[16];
         tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + BN, s16);
         tmem_wait_ld();
@@ -504,7 +506,7 @@ bool linear_tc5_ok(const LinearArgs& p) {
 // the column sums need one work item per CTA: they use the second accumulator buffer and a staging block
 bool linear_tc5_sums_ok(const LinearArgs& p) {
   const int64_t tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
-  return p.a_mn && linear_tc5_ok(p) && tiles * (p.k_splits > 1 ? p.k_splits : 1) <= sm_count();
+  return p.a_mn && !p.R && linear_tc5_ok(p) && tiles * (p.k_splits > 1 ? p.k_splits : 1) <= sm_count();
 }
 
 int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
@@ -525,6 +527,11 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
     set_error("linear: column sums need row-contraction operands and at most one work item per SM");
     return BSRL_ERR_UNSUPPORTED;
   }
+  if (linear_res_ok(p)) return linear_res(p, stream);
+  if (p.bits_in || p.bits_out) {
+    set_error("linear: ReLU bits need the resident-weight kernel (m=%lld n=%d k=%d)", (long long)p.M, p.N, p.K);
+    return BSRL_ERR_UNSUPPORTED;
+  }
   int* status = device_status_ptr();
   if (!status) return BSRL_ERR_CUDA;
   CUtensorMap tm_a, tm_w;
@@ -540,9 +547,10 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
   if (tma_c && !make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, p.M, p.N, p.ldc, 32, 128)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("linear_tc5_kernel set-up", [] {
-    cudaError_t e = cudaFuncSetAttribute(linear_tc5_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(linear_tc5_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaSuccess;
+    for (auto* k : {linear_tc5_kernel<false, false>, linear_tc5_kernel<true, false>, linear_tc5_kernel<false, true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    return e;
   });
   if (rc != BSRL_OK) return rc;
   const int64_t m_tiles = (p.M + BM - 1) / BM;
@@ -553,11 +561,8 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
   }
   int64_t grid = m_tiles * n_tiles * (p.k_splits > 1 ? p.k_splits : 1);
   if (grid > sm_count()) grid = sm_count();
-  if (p.R)
-    linear_tc5_kernel<true><<<(unsigned)grid, THREADS, SMEM_BYTES, stream>>>(tm_a, tm_w, tm_c, 0, p, (int)m_tiles, n_tiles, status);
-  else
-    linear_tc5_kernel<false><<<(unsigned)grid, THREADS, SMEM_BYTES, stream>>>(tm_a, tm_w, tm_c, tma_c ? 1 : 0, p, (int)m_tiles,
-                                                                             n_tiles, status);
+  auto* kernel = p.a_sums ? linear_tc5_kernel<false, true> : p.R ? linear_tc5_kernel<true, false> : linear_tc5_kernel<false, false>;
+  kernel<<<(unsigned)grid, THREADS, SMEM_BYTES, stream>>>(tm_a, tm_w, tm_c, tma_c ? 1 : 0, p, (int)m_tiles, n_tiles, status);
   BSRL_LAUNCH_OK("linear_tc5_kernel");
   return BSRL_OK;
 }

@@ -40,6 +40,11 @@ struct LinearArgs {
   // MMA against a tile of ones beside each k-block's MMAs, so A is not read a second time.  Only where
   // linear_tc5_sums_ok says so.
   float* a_sums = nullptr;
+  // ReLU masks as bits (gemm_res_tc5.cu describes the layout; only where linear_res_ok says so): bits_out of a product
+  // with ReLU, bits_in in the place of `mask`.
+  uint32_t* bits_out = nullptr;
+  const uint32_t* bits_in = nullptr;
+  int64_t bits_ld = 0;
 };
 LinearArgs linear_args(const __half* A, int lda, const __half* W, int ldw, const float* bias,
                        void* C, int ldc, int out_f32, int relu, int64_t M, int N, int K);
@@ -48,6 +53,8 @@ int linear_mma(const LinearArgs& p, cudaStream_t stream);   // warp-MMA engine
 int linear_tc5(const LinearArgs& p, cudaStream_t stream);   // tcgen05 / TMEM engine
 bool linear_tc5_ok(const LinearArgs& p);                     // shape fits the tcgen05 engine
 bool linear_tc5_sums_ok(const LinearArgs& p);                // ... and its column sums can ride along (a_sums)
+bool linear_res_ok(const LinearArgs& p);                     // linear_tc5's products with K <= 256 over many rows:
+int linear_res(const LinearArgs& p, cudaStream_t stream);    // ... weights resident in shared memory (gemm_res_tc5.cu)
 
 // Projection + residual + LayerNorm in one kernel (gemm_ln_tc5.cu): x_out = R + A W^T + bias (fp32), h =
 // LayerNorm(x_out) (fp16).  N a multiple of 64 up to 512 (of 128 above 256), K a multiple of 64.  R and x_out

@@ -169,7 +169,7 @@ const GradLayout& grad_layout(const bsrl_config& cfg) {
 
 // ---- scratch of the backward
 struct BwdLayout {
-  int64_t h16, qkv16, att16, x1, h2, hid, gx, gx16, g32, gA, gB, tA, tX, wT, hl16;
+  int64_t h16, qkv16, att16, x1, h2, hid, bits, gx, gx16, g32, gA, gB, tA, tX, wT, hl16;
   // readout-side rows (B of them)
   int64_t attc16, m1, m2, gz32, graw16, gvraw16, gsmall32, gsmall16;
   int64_t v0, vown, gv0;        // value residual: block 0's values, a block's own values, fp32 gradient of block 0's values
@@ -196,6 +196,7 @@ BwdLayout make_bwd(const Layout& l, int64_t B) {
   w.x1 = cv.take(R * d * 4);
   w.h2 = cv.take(R * d * 2);
   w.hid = cv.take(R * (int64_t)F * 2);
+  w.bits = cv.take(R * (int64_t)(round_up(F, 32) / 8));    // which hidden units were positive, one bit each
   w.gx = cv.take(R * d * 4);
   w.gx16 = cv.take(R * d * 2);     // fp16 copy of the stream gradient, written by the kernels that produce it
   w.g32 = cv.take(R * d * 4);
@@ -258,8 +259,13 @@ struct Bwd {
             const __half* relu_of = nullptr, int64_t ld_relu = 0, const RowMap* add_rows = nullptr) {
     LinearArgs r = linear_args(g, (int)ldg, W, ldw, nullptr, out, (int)ldo, out_f32 ? 1 : 0, 0, M, K, N);
     r.w_mn = 1;
-    r.mask = relu_of;
-    r.ldm = (int)ld_relu;
+    if (relu_of && relu_of == bits_of) {
+      r.bits_in = S<uint32_t>(w.bits);
+      r.bits_ld = M;
+    } else {
+      r.mask = relu_of;
+      r.ldm = (int)ld_relu;
+    }
     if (add_rows) {
       r.R = static_cast<const float*>(out);
       r.ldr = (int)ldo;
@@ -280,6 +286,21 @@ struct Bwd {
       return relu_mask16(static_cast<__half*>(out), ldo, relu_of, ld_relu, M, K, st);
     }
     return BSRL_OK;
+  }
+  // The ReLU product out = relu(a W^T + b) of M rows.  Where this product and the dgrad through it (relu_of = out, a
+  // contraction over Kb) both run on the resident-weight kernel, it leaves its mask as bits for that dgrad.
+  const __half* bits_of = nullptr;
+  int relu_fwd(const __half* a, int lda, const Mat& m, int64_t M, int N, int K, __half* out, int Kb) {
+    LinearArgs f = linear_args(a, lda, c.W(m), m.pitch, c.Bv(m), out, N, 0, 1, M, N, K);
+    LinearArgs b = linear_args(a, Kb, c.W(m), N, nullptr, out, N, 0, 0, M, N, Kb);
+    f.bits_out = S<uint32_t>(w.bits);
+    f.bits_ld = M;
+    b.w_mn = 1;
+    b.bits_in = f.bits_out;
+    const bool bits = linear_rows_ok(f) && linear_res_ok(f) && linear_res_ok(b);
+    if (!bits) f.bits_out = nullptr;
+    bits_of = bits ? out : nullptr;
+    return linear(f, st);
   }
   // One Linear, or several stacked ones: gW (N, K) f32 += g^T x over M rows, gb += column sums of g.  Both operands
   // are MN-major (the contraction index is their row); the warp-MMA cross-check engine gets transposed copies (M padded
@@ -347,7 +368,7 @@ struct Bwd {
     po.R = x_in; po.ldr = d; po.rmap = xrows;
     BSRL_TRY(linear(po, st));
     BSRL_TRY(layernorm(x1, d, identity_map(), c.G(b.ln_ffn), c.Be(b.ln_ffn), c.cfg->eps, M, d, h2, d, st));
-    return linear(linear_args(h2, d, c.W(b.up), d, c.Bv(b.up), hid, F, 0, 1, M, F, d), st);
+    return relu_fwd(h2, d, b.up, M, F, d, hid, d);
   }
 
   int run(const HeadTailArgs& tail, const float* g_logprob, const float* g_entropy, const float* g_value,
@@ -532,7 +553,7 @@ struct Bwd {
     for (const Enc& e : encs) {
       const __half* feat = sv.feat + e.row0 * 64;
       __half* g = gB + e.row0 * d;
-      BSRL_TRY(linear(linear_args(feat, 64, c.W(e.e->l0), e.e->l0.pitch, c.Bv(e.e->l0), hid, d, 0, 1, e.rows, d, 64), st));   // hidden
+      BSRL_TRY(relu_fwd(feat, 64, e.e->l0, e.rows, d, 64, hid, d));                                  // hidden
       if (c.cfg->emb_ln) {
         // tokens = emb_ln(encoder output): recompute the encoder's output rows (fp32) and take g back through the
         // LayerNorm; the fp16 copy of the result replaces g

@@ -262,3 +262,28 @@ def test_linear_bwd_stage(native, m, n, k, engine):
     torch.testing.assert_close(gw.cpu(), gy.float().t() @ x.float(), atol=2e-3 * m ** 0.5, rtol=2e-3)
     torch.testing.assert_close(gb.cpu(), gy.float().sum(0), atol=1e-3 * m ** 0.5, rtol=1e-3)
     torch.testing.assert_close(gx.cpu(), gy.float() @ w.float(), atol=2e-3, rtol=2e-3)
+
+
+@pytest.mark.parametrize("name,blocks,envs", [("cfg2", 2, 516), ("recipe", 2, 683), ("cfg1", 2, 1031)])
+def test_large_batch_gradients_equal_the_sum_of_small_batches(name, blocks, envs):
+    """Batches large enough for the resident-weight products (three 128 x 256 tiles per SM; ReLU masks as bits) and odd in
+    rows, against the same environments in small batches, which take the streaming kernel and fp16 masks: every row's
+    arithmetic is the same, so the gradients differ by the order of fp32 sums over some 15-30 thousand rows only
+    (about 2^-24 sqrt(rows) = 1e-5 of the terms' root sum of squares; the bound allows the atomics' order on top)."""
+    cfg = make_cfg(name, name == "recipe")
+    cfg.n_blocks = blocks
+    cfg.__post_init__()
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 5))
+    obs, act = po.make_obs(envs, 21, padded=True), po.make_actions(envs, cfg, 22)
+    up = po.make_upstream(envs, cfg, 23)
+    with torch.enable_grad():
+        _loss(m, obs.cuda(), act.cuda(), up).backward()
+        whole = {k: p.grad.clone() for k, p in m.named_parameters()}
+        m.zero_grad()
+        for lo in range(0, envs, 61):
+            s = slice(lo, lo + 61)
+            _loss(m, obs[s].cuda(), act[s].cuda(), {k: v[s] for k, v in up.items()}).backward()
+    m.check_device()
+    top = max(float(g.norm()) for g in whole.values())
+    for k, p in m.named_parameters():
+        assert float((p.grad - whole[k]).norm()) <= 1e-4 * float(whole[k].norm()) + 1e-6 * top, k

@@ -341,3 +341,32 @@ def test_head_tail_stage(native, case, B):
     torch.testing.assert_close(out["entropy"].cpu(), ent, atol=2e-4, rtol=1e-5)
     val = torch.softmax(vraw[:, :cfg.value_bins], -1) @ po.value_centers(cfg)
     torch.testing.assert_close(out["value"].cpu(), val, atol=1e-5, rtol=1e-5)
+
+
+@pytest.mark.parametrize("m,n,k,relu,res", [
+    (57001, 256, 256, 1, False),        # one column tile, a ragged last row tile, two A stages per ring turn
+    (19200, 784, 192, 0, False),        # four column tiles, the last 16 wide; two staging buffers
+    (28577, 512, 64, 2, False),         # one k-block, GELU
+    (57001, 208, 192, 0, True),         # fp32 rows with a residual, columns past the tile
+    (28416, 320, 128, 0, True),
+])
+def test_linear_resident_weights(native, m, n, k, relu, res):
+    """linear_tc5 sizes that take the resident-weight kernel (K <= 256, three tiles per SM) against float64 products of the
+    same fp16 operands: fp32 sums of k products of size ~1 / sqrt(k) (k 2^-24 relative at worst) and one fp16 rounding."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn(m, k, generator=g, device="cuda").half()
+    w = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).half()
+    b = torch.randn(n, generator=g, device="cuda")
+    r = torch.randn(m, n, generator=g, device="cuda") if res else None
+    out = torch.full((m, n), float("nan"), dtype=torch.float32 if res else torch.float16, device="cuda")
+    native.check(native.lib.bsrl_linear(a.data_ptr(), w.data_ptr(), b.data_ptr(), r.data_ptr() if res else None, out.data_ptr(),
+                                        int(res), relu, m, n, k, 1, torch.cuda.current_stream().cuda_stream))
+    ref = a.double() @ w.double().t() + b.double()
+    if relu == 1:
+        ref = ref.clamp_min(0)
+    elif relu == 2:
+        ref = torch.nn.functional.gelu(ref)
+    if res:
+        ref = ref + r.double()
+    tol = 2e-5 if res else 2 ** -11
+    assert bool(((out.double() - ref).abs() <= tol * ref.abs() + 2e-5).all())
