@@ -103,6 +103,9 @@ int attention(const __half* qkv, int ld, const float* kb, int64_t B, int d, int 
   return rc;
 }
 
+void begin_overlap(int64_t rows) {
+  if (!g_prof.on && rows <= 8 * 128 * (int64_t)sm_count()) pdl_enable();
+}
 void set_stage(int stage) { g_stage = stage; }
 int timed_call(cudaStream_t st, double flops, double bytes, const std::function<int()>& fn) { return timed(st, flops, bytes, fn); }
 
@@ -167,6 +170,7 @@ int run_embed(const Ctx& c, const void* obs, int obs_dtype, float* x, float* key
   BSRL_TRY(timed(c.st, 0.0, (double)B * (kObs * 4 + (2 * kSaberK + kTorsoK + 2 * kLegK + kSlots * l.note_k) * 2 + kT * 4),
                  [&] { return embed_gather(obs, obs_dtype, B, c.cfg->note_geo, c.cfg->game_flux, c.cfg->z_asinh, eb, c.st); }));
   if (have_h) *have_h = false;
+  begin_overlap(B * kT);
   if (c.paths.enc_fused) {
     EncoderArgs ea;
     ea.d = d; ea.n_envs = B; ea.feat = eb.saber;
@@ -262,6 +266,7 @@ int run_trunk(const Ctx& c, const __half* lead16, float* raw) {
 }
 
 int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs& tail_in) {
+  PdlScope pdl;
   const Layout& l = c.l;
   const Workspace& w = c.w;
   const int d = l.d, F = l.F, D = l.D;
@@ -871,6 +876,7 @@ int bsrl_embed(const bsrl_config* cfg, const void* arena, const void* obs, int32
     return BSRL_ERR_ALIGN;
   }
   if (n_envs == 0) return BSRL_OK;
+  PdlScope pdl;
   return run_embed(c, obs, obs_dtype, x, key_bias);
 }
 

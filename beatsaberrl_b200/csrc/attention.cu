@@ -24,6 +24,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
                                                            int64_t n_pairs, int tokens, int d, int n_heads,
                                                            int q_first, int n_q,
                                                            __half* __restrict__ out, int ldo) {
+  pdl_begin();
   constexpr int kWarps = WARPS, kRows = 32 * KG, NT = 4 * KG;   // NT: 8-key tiles
   constexpr int LDS = DH + 8;          // padded row (halfs): ldmatrix rows land in distinct banks
   constexpr int CH = DH / 8;           // 16-byte chunks per row
@@ -169,6 +170,7 @@ template <int DH, int NOBJ, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __restrict__ qkv, int ld,
                                                               const float* __restrict__ key_bias, int64_t n_pairs,
                                                               int d, int n_heads, int n_q, __half* __restrict__ out, int ldo) {
+  pdl_begin();
   constexpr int T = NOBJ + 1, NT = NOBJ / 8, KS = NOBJ / 16, MT = NOBJ / 16;
   constexpr int LDS = DH + 8, CH = DH / 8;
   constexpr int PER = (NOBJ + 31) / 32;              // object rows per lane in the lane-per-row passes
@@ -419,7 +421,7 @@ int launch_body(const __half* qkv, int ld, const float* key_bias, int64_t n_envs
   int64_t blocks = (pairs + kWarps - 1) / kWarps;
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  attn_body_kernel<DH, NOBJ, kWarps><<<static_cast<unsigned>(blocks), kWarps * 32, smem, stream>>>(qkv, ld, key_bias, pairs, d,
+  launch_kernel(attn_body_kernel<DH, NOBJ, kWarps>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d,
                                                                                                 n_heads, n_q, out, ldo);
   BSRL_LAUNCH_OK("attn_body_kernel");
   return BSRL_OK;
@@ -446,8 +448,7 @@ int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int
   int64_t blocks = (pairs + kWarps - 1) / kWarps;
   int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  attn29_kernel<DH, KG, kWarps><<<static_cast<unsigned>(blocks), kWarps * 32, smem, stream>>>(
-      qkv, ld, key_bias, pairs, tokens, d, n_heads, q_first, n_q, out, ldo);
+  launch_kernel(attn29_kernel<DH, KG, kWarps>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, tokens, d, n_heads, q_first, n_q, out, ldo);
   BSRL_LAUNCH_OK("attn29_kernel");
   return BSRL_OK;
 }
@@ -505,6 +506,7 @@ namespace {
 __global__ void vres_mix_kernel(__half* __restrict__ v, int ld, int64_t rows, int d,
                                 __half* __restrict__ v_out, const __half* __restrict__ v0,
                                 const float* __restrict__ vres) {
+  pdl_begin();
   const float a = vres ? vres[0] : 1.f, b = vres ? vres[1] : 0.f;
   const int per_row = d >> 3;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row;
@@ -544,7 +546,7 @@ int vres_mix(__half* v, int ld, int64_t rows, int d, __half* v_out, const __half
   int64_t blocks = (rows * (d >> 3) + 255) / 256;
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  vres_mix_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(v, ld, rows, d, v_out, v0, vres);
+  launch_kernel(vres_mix_kernel, static_cast<unsigned>(blocks), 256, 0, stream, v, ld, rows, d, v_out, v0, vres);
   BSRL_LAUNCH_OK("vres_mix_kernel");
   return BSRL_OK;
 }

@@ -301,6 +301,7 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
+  if (warp != 0) pdl_begin();    // the producer waits below, after its first weight stages
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -318,11 +319,17 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
         ++it;
         return true;
       };
+      if (STREAM) pdl_wait();
       for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, ++tile_i) {
         if (STREAM) {
           for (int g = 0; g < n_groups && ok; ++g)
             for (int kb = 0; kb < KB && ok; ++kb) ok = w_stage(g, kb, t);
           continue;
+        }
+        int early = 0;                          // first tile: weights ahead of the predecessor's last rows
+        if (tile_i == 0) {
+          for (; early < KB && early < STAGES && ok; ++early) ok = w_stage(0, early, t);
+          pdl_wait();
         }
         for (int kb = 0; kb < KB && ok; ++kb) {
           // chunk kb of the h tile is free once the previous tile's last group has used it
@@ -330,7 +337,7 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
           const uint32_t bar = smem_u32(&sh->a_full[kb]);
           mbar_expect_tx(bar, CHUNK_BYTES);
           tma_load_3d(sA + kb * CHUNK_BYTES, &tm_h, 64 * kb, BODY ? p.tok0 : 0, t * EPT, bar);
-          ok = w_stage(0, kb, t);
+          if (kb >= early) ok = w_stage(0, kb, t);
         }
         for (int g = 1; g < n_groups && ok; ++g)
           for (int kb = 0; kb < KB && ok; ++kb) ok = w_stage(g, kb, t);
@@ -674,13 +681,13 @@ int attn_block(const AttnBlockArgs& a, cudaStream_t stream) {
   p.status = status;
   const int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
   const bool vres = a.v_out || a.v0;
-  if (a.body) attn_block_kernel<32, 2, false, true><<<grid, THREADS, Shape<32, 2>::SMEM_BYTES, stream>>>(tm_h, tm_w, tm_o, p);
-  else if (dh == 32 && !vres) attn_block_kernel<32, 2, false><<<grid, THREADS, Shape<32, 2>::SMEM_BYTES, stream>>>(tm_h, tm_w, tm_o, p);
-  else if (dh == 32) attn_block_kernel<32, 2, true><<<grid, THREADS, Shape<32, 2>::SMEM_BYTES, stream>>>(tm_h, tm_w, tm_o, p);
-  else if (dh == 48 && !vres) attn_block_kernel<48, 1, false><<<grid, THREADS, Shape<48, 1>::SMEM_BYTES, stream>>>(tm_h, tm_w, tm_o, p);
-  else if (dh == 48) attn_block_kernel<48, 1, true><<<grid, THREADS, Shape<48, 1>::SMEM_BYTES, stream>>>(tm_h, tm_w, tm_o, p);
-  else if (!vres) attn_block_kernel<64, 1, false><<<grid, THREADS, Shape<64, 1>::SMEM_BYTES, stream>>>(tm_h, tm_w, tm_o, p);
-  else attn_block_kernel<64, 1, true><<<grid, THREADS, Shape<64, 1>::SMEM_BYTES, stream>>>(tm_h, tm_w, tm_o, p);
+  if (a.body) launch_kernel(attn_block_kernel<32, 2, false, true>, grid, THREADS, Shape<32, 2>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
+  else if (dh == 32 && !vres) launch_kernel(attn_block_kernel<32, 2, false>, grid, THREADS, Shape<32, 2>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
+  else if (dh == 32) launch_kernel(attn_block_kernel<32, 2, true>, grid, THREADS, Shape<32, 2>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
+  else if (dh == 48 && !vres) launch_kernel(attn_block_kernel<48, 1, false>, grid, THREADS, Shape<48, 1>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
+  else if (dh == 48) launch_kernel(attn_block_kernel<48, 1, true>, grid, THREADS, Shape<48, 1>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
+  else if (!vres) launch_kernel(attn_block_kernel<64, 1, false>, grid, THREADS, Shape<64, 1>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
+  else launch_kernel(attn_block_kernel<64, 1, true>, grid, THREADS, Shape<64, 1>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
   BSRL_LAUNCH_OK("attn_block_kernel");
   return BSRL_OK;
 }

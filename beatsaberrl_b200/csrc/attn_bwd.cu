@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
                                                                const __half* __restrict__ g_out, int ldgo, __half* __restrict__ gq,
                                                                int ldq, __half* __restrict__ gk, int ldk, __half* __restrict__ gv,
                                                                int ldv) {
+  pdl_begin();
   constexpr int LDS = DH + 8;                         // padded row (halves): ldmatrix rows land in distinct banks
   constexpr int CH = DH / 8;
   constexpr int QR = 16 * MT;                         // staged query rows
@@ -257,7 +258,7 @@ int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int
   int64_t blocks = (pairs + kWarps - 1) / kWarps;
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  attn_bwd_kernel<DH, MT><<<(unsigned)blocks, kWarps * 32, smem, stream>>>(qkv, ld, key_bias, pairs, d, n_heads, q_first, n_q, g_out,
+  launch_kernel(attn_bwd_kernel<DH, MT>, (unsigned)blocks, kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d, n_heads, q_first, n_q, g_out,
                                                                           ldgo, gq, ldq, gk, ldk, gv, ldv);
   BSRL_LAUNCH_OK("attn_bwd_kernel");
   return BSRL_OK;

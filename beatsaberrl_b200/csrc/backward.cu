@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const float* __restrict__ x
                                                      int64_t ldgy, const float* gres, float* gx_out, int64_t ldg, RowMap gmap,
                                                      __half* __restrict__ gx16, int64_t ldg16,
                                                      float* __restrict__ ggamma, float* __restrict__ gbeta, int64_t rows, int d) {
+  pdl_begin();
   extern __shared__ float s_part[];                  // [2][d]
   for (int i = threadIdx.x; i < 2 * d; i += blockDim.x) s_part[i] = 0.f;
   __syncthreads();
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(256) ln_bwd_kernel(const float* __restrict__ x
 // memory and leave as one atomic per column and block.  n % 8 == 0, ld % 8 == 0, 16-byte aligned base.
 __global__ void __launch_bounds__(256) colsum_kernel(const __half* __restrict__ in, int64_t ld, int64_t rows, int n,
                                                      int64_t chunk, float* __restrict__ out) {
+  pdl_begin();
   __shared__ float part[8][256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * 256 + lane * 8;
@@ -166,6 +168,7 @@ __global__ void __launch_bounds__(256) colsum_kernel(const __half* __restrict__ 
 // any shape: one thread per column
 __global__ void __launch_bounds__(256) colsum_slow_kernel(const __half* __restrict__ in, int64_t ld, int64_t rows, int n,
                                                           int64_t chunk, float* __restrict__ out) {
+  pdl_begin();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   const int64_t r0 = (int64_t)blockIdx.y * chunk, r1 = r0 + chunk < rows ? r0 + chunk : rows;
@@ -177,6 +180,7 @@ __global__ void __launch_bounds__(256) colsum_slow_kernel(const __half* __restri
 // g <- (act > 0) ? g : 0, fp16 rows of n columns (n % 8 == 0)
 __global__ void __launch_bounds__(256) relu_mask_kernel(__half* __restrict__ g, int64_t ldg, const __half* __restrict__ act,
                                                         int64_t lda, int64_t rows, int n) {
+  pdl_begin();
   const int nv = n >> 3;
   const int64_t total = rows * nv;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -197,6 +201,7 @@ __global__ void __launch_bounds__(256) relu_mask_kernel(__half* __restrict__ g, 
 // out16[r, :] = fp16(in32[map(r), :] * scale)
 __global__ void __launch_bounds__(256) cast_rows16_kernel(const float* __restrict__ in, int64_t ldi, RowMap imap, float scale,
                                                           __half* __restrict__ out, int64_t ldo, int64_t rows, int n) {
+  pdl_begin();
   const int nv = n >> 2;
   const int64_t total = rows * nv;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -214,6 +219,7 @@ __global__ void __launch_bounds__(256) cast_rows16_kernel(const float* __restric
 // dst[map(r), :] += src[r, :] (fp32 rows); dst16, if given, gets the sums as fp16 (dense rows of n columns)
 __global__ void __launch_bounds__(256) add_rows_kernel(const float* __restrict__ src, int64_t lds, float* __restrict__ dst,
                                                        int64_t ldd, RowMap dmap, int64_t rows, int n, __half* __restrict__ dst16) {
+  pdl_begin();
   const int nv = n >> 2;
   const int64_t total = rows * nv;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -233,6 +239,7 @@ __global__ void __launch_bounds__(256) add_rows_kernel(const float* __restrict__
 // out[r, :] = in[map(r), :] (fp16 rows, dense output; n % 8 == 0)
 __global__ void __launch_bounds__(256) gather_rows16_kernel(const __half* __restrict__ in, int64_t ldi, RowMap imap,
                                                             __half* __restrict__ out, int64_t rows, int n) {
+  pdl_begin();
   const int nv = n >> 3;
   const int64_t total = rows * nv;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -245,6 +252,7 @@ __global__ void __launch_bounds__(256) gather_rows16_kernel(const __half* __rest
 // token rows (env-major) -> the encoders' row order: 2 saber rows per env, then torso, 2 leg, 24 slot rows per env
 __global__ void __launch_bounds__(256) gather_tokens16_kernel(const __half* __restrict__ in, int64_t n_envs, int n,
                                                               __half* __restrict__ out) {
+  pdl_begin();
   const int nv = n >> 3;
   const int64_t total = n_envs * kT * nv;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
@@ -267,6 +275,7 @@ __global__ void __launch_bounds__(256) gather_tokens16_kernel(const __half* __re
 __global__ void __launch_bounds__(256) transpose16_kernel(const __half* __restrict__ in, int64_t ldi, RowMap imap, int64_t rows,
                                                           int cols, __half* __restrict__ out, int64_t ldo, int64_t rows_pad,
                                                           float* __restrict__ colsum) {
+  pdl_begin();
   __shared__ __align__(16) __half tile[64][72];      // 144-byte rows: column reads of 8 rows hit 8 bank groups
   const int64_t r0 = (int64_t)blockIdx.x * 64;
   const int c0 = blockIdx.y * 64;
@@ -302,6 +311,7 @@ __global__ void __launch_bounds__(256) transpose16_kernel(const __half* __restri
 __global__ void __launch_bounds__(256) transpose16_slow_kernel(const __half* __restrict__ in, int64_t ldi, RowMap imap, int64_t rows,
                                                                int cols, __half* __restrict__ out, int64_t ldo, int64_t rows_pad,
                                                                float* __restrict__ colsum) {
+  pdl_begin();
   __shared__ __half tile[64][66];
   const int64_t r0 = (int64_t)blockIdx.x * 64;
   const int c0 = blockIdx.y * 64;
@@ -338,6 +348,7 @@ __global__ void __launch_bounds__(256) head_tail_bwd_kernel(HeadTailArgs p, cons
                                                             const float* __restrict__ g_vlogits, const float* __restrict__ g_logits,
                                                             float scale, __half* __restrict__ g_raw, int ldg_raw,
                                                             __half* __restrict__ g_vraw, int ldg_v) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t env = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); env < p.n_envs; env += warps) {
@@ -426,7 +437,7 @@ int layernorm_bwd(const float* x, int64_t ldx, RowMap xmap, const float* gamma, 
   const int blocks = (int)grid_for(rows, 8 * 4);
   const size_t smem = 2 * d * sizeof(float);
 #define BSRL_LN_BWD(F32, NV) \
-  ln_bwd_kernel<F32, NV><<<blocks, 256, smem, stream>>>(x, ldx, xmap, gamma, eps, gy, ldgy, gres, gx_out, ldg, gmap, gx16, ldg16, ggamma, gbeta, rows, d)
+  launch_kernel(ln_bwd_kernel<F32, NV>, blocks, 256, smem, stream, x, ldx, xmap, gamma, eps, gy, ldgy, gres, gx_out, ldg, gmap, gx16, ldg16, ggamma, gbeta, rows, d)
   const int nv = (d + 127) / 128;          // float4 per lane actually needed: fewer registers, more rows in flight
   if (gy_f32) {
     if (nv <= 2) BSRL_LN_BWD(true, 2); else if (nv <= 4) BSRL_LN_BWD(true, 4); else BSRL_LN_BWD(true, 8);
@@ -448,15 +459,15 @@ int colsum16(const __half* in, int64_t ld, int64_t rows, int n, float* out, cuda
   const int64_t chunk = (rows + chunks - 1) / chunks;
   chunks = (rows + chunk - 1) / chunk;
   const dim3 grid((unsigned)col_blocks, (unsigned)chunks);
-  if (n % 8 == 0 && ld % 8 == 0 && aligned16(in)) colsum_kernel<<<grid, 256, 0, stream>>>(in, ld, rows, n, chunk, out);
-  else colsum_slow_kernel<<<grid, 256, 0, stream>>>(in, ld, rows, n, chunk, out);
+  if (n % 8 == 0 && ld % 8 == 0 && aligned16(in)) launch_kernel(colsum_kernel, grid, 256, 0, stream, in, ld, rows, n, chunk, out);
+  else launch_kernel(colsum_slow_kernel, grid, 256, 0, stream, in, ld, rows, n, chunk, out);
   BSRL_LAUNCH_OK("colsum_kernel");
   return BSRL_OK;
 }
 
 int relu_mask16(__half* g, int64_t ldg, const __half* act, int64_t lda, int64_t rows, int n, cudaStream_t stream) {
   if (rows == 0) return BSRL_OK;
-  relu_mask_kernel<<<(unsigned)grid_for(rows * (n >> 3), 256), 256, 0, stream>>>(g, ldg, act, lda, rows, n);
+  launch_kernel(relu_mask_kernel, (unsigned)grid_for(rows * (n >> 3), 256), 256, 0, stream, g, ldg, act, lda, rows, n);
   BSRL_LAUNCH_OK("relu_mask_kernel");
   return BSRL_OK;
 }
@@ -464,7 +475,7 @@ int relu_mask16(__half* g, int64_t ldg, const __half* act, int64_t lda, int64_t 
 int cast_rows16(const float* in, int64_t ldi, RowMap imap, float scale, __half* out, int64_t ldo, int64_t rows, int n,
                 cudaStream_t stream) {
   if (rows == 0) return BSRL_OK;
-  cast_rows16_kernel<<<(unsigned)grid_for(rows * (n >> 2), 256), 256, 0, stream>>>(in, ldi, imap, scale, out, ldo, rows, n);
+  launch_kernel(cast_rows16_kernel, (unsigned)grid_for(rows * (n >> 2), 256), 256, 0, stream, in, ldi, imap, scale, out, ldo, rows, n);
   BSRL_LAUNCH_OK("cast_rows16_kernel");
   return BSRL_OK;
 }
@@ -472,21 +483,21 @@ int cast_rows16(const float* in, int64_t ldi, RowMap imap, float scale, __half* 
 int add_rows32(const float* src, int64_t lds, float* dst, int64_t ldd, RowMap dmap, int64_t rows, int n, cudaStream_t stream,
                __half* dst16) {
   if (rows == 0) return BSRL_OK;
-  add_rows_kernel<<<(unsigned)grid_for(rows * (n >> 2), 256), 256, 0, stream>>>(src, lds, dst, ldd, dmap, rows, n, dst16);
+  launch_kernel(add_rows_kernel, (unsigned)grid_for(rows * (n >> 2), 256), 256, 0, stream, src, lds, dst, ldd, dmap, rows, n, dst16);
   BSRL_LAUNCH_OK("add_rows_kernel");
   return BSRL_OK;
 }
 
 int gather_rows16(const __half* in, int64_t ldi, RowMap imap, __half* out, int64_t rows, int n, cudaStream_t stream) {
   if (rows == 0) return BSRL_OK;
-  gather_rows16_kernel<<<(unsigned)grid_for(rows * (n >> 3), 256), 256, 0, stream>>>(in, ldi, imap, out, rows, n);
+  launch_kernel(gather_rows16_kernel, (unsigned)grid_for(rows * (n >> 3), 256), 256, 0, stream, in, ldi, imap, out, rows, n);
   BSRL_LAUNCH_OK("gather_rows16_kernel");
   return BSRL_OK;
 }
 
 int gather_tokens16(const __half* in, int64_t n_envs, int n, __half* out, cudaStream_t stream) {
   if (n_envs == 0) return BSRL_OK;
-  gather_tokens16_kernel<<<(unsigned)grid_for(n_envs * kT * (n >> 3), 256), 256, 0, stream>>>(in, n_envs, n, out);
+  launch_kernel(gather_tokens16_kernel, (unsigned)grid_for(n_envs * kT * (n >> 3), 256), 256, 0, stream, in, n_envs, n, out);
   BSRL_LAUNCH_OK("gather_tokens16_kernel");
   return BSRL_OK;
 }
@@ -501,8 +512,8 @@ int transpose16(const __half* in, int64_t ldi, RowMap imap, int64_t rows, int co
   }
   const dim3 grid((unsigned)bx, (cols + 63) / 64);
   const bool fast = cols % 8 == 0 && ldi % 8 == 0 && ldo % 8 == 0 && rows_pad % 8 == 0 && aligned16(in) && aligned16(out);
-  if (fast) transpose16_kernel<<<grid, 256, 0, stream>>>(in, ldi, imap, rows, cols, out, ldo, rows_pad, colsum);
-  else transpose16_slow_kernel<<<grid, 256, 0, stream>>>(in, ldi, imap, rows, cols, out, ldo, rows_pad, colsum);
+  if (fast) launch_kernel(transpose16_kernel, grid, 256, 0, stream, in, ldi, imap, rows, cols, out, ldo, rows_pad, colsum);
+  else launch_kernel(transpose16_slow_kernel, grid, 256, 0, stream, in, ldi, imap, rows, cols, out, ldo, rows_pad, colsum);
   BSRL_LAUNCH_OK("transpose16_kernel");
   return BSRL_OK;
 }
@@ -515,7 +526,7 @@ int head_tail_bwd(const HeadTailArgs& a, const float* g_logprob, const float* g_
     return BSRL_ERR_NULL;
   }
   if (a.n_envs == 0) return BSRL_OK;
-  head_tail_bwd_kernel<<<(unsigned)grid_for(a.n_envs, 8), 256, 0, stream>>>(a, g_logprob, g_entropy, g_value, g_vlogits,
+  launch_kernel(head_tail_bwd_kernel, (unsigned)grid_for(a.n_envs, 8), 256, 0, stream, a, g_logprob, g_entropy, g_value, g_vlogits,
                                                                             g_logits, scale, g_raw, ldg_raw, g_vraw, ldg_v);
   BSRL_LAUNCH_OK("head_tail_bwd_kernel");
   return BSRL_OK;

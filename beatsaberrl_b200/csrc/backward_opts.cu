@@ -23,6 +23,7 @@ __global__ void __launch_bounds__(256) vres_bwd_kernel(__half* __restrict__ g, i
                                                        const __half* __restrict__ v0, const float* __restrict__ ab,
                                                        float* __restrict__ g_v0, float* __restrict__ g_a, float* __restrict__ g_b,
                                                        int64_t rows, int d) {
+  pdl_begin();
   const float a = ab[0], b = ab[1];
   const int per_row = d >> 3;
   float sa = 0.f, sb = 0.f;
@@ -75,6 +76,7 @@ __global__ void __launch_bounds__(256) vres_bwd_kernel(__half* __restrict__ g, i
 // g16[r, c] += fp16(acc32[r, c]) (fp32 arithmetic, rounded once)
 __global__ void __launch_bounds__(256) add_f32_into_f16_kernel(__half* __restrict__ g, int64_t ldg, const float* __restrict__ acc,
                                                                int64_t rows, int d) {
+  pdl_begin();
   const int per_row = d >> 2;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += (int64_t)gridDim.x * blockDim.x) {
     int piece;
@@ -113,6 +115,7 @@ __global__ void __launch_bounds__(256) simba2_out_bwd_kernel(const float* __rest
                                                              const float* __restrict__ g_h, float* __restrict__ g_x0,
                                                              __half* __restrict__ g_t2, float* __restrict__ g_alpha,
                                                              int64_t rows, int d) {
+  pdl_begin();
   extern __shared__ float s_part[];
   for (int i = threadIdx.x; i < d; i += blockDim.x) s_part[i] = 0.f;
   __syncthreads();
@@ -192,6 +195,7 @@ __global__ void __launch_bounds__(256) simba2_out_bwd_kernel(const float* __rest
 __global__ void __launch_bounds__(256) simba2_in_bwd_kernel(const float* __restrict__ t0, const float* __restrict__ s,
                                                             const float* __restrict__ g_a, const float* __restrict__ g_b,
                                                             __half* __restrict__ g_t0, float* __restrict__ g_s, int64_t rows, int d) {
+  pdl_begin();
   extern __shared__ float s_part[];
   for (int i = threadIdx.x; i < d; i += blockDim.x) s_part[i] = 0.f;
   __syncthreads();
@@ -242,6 +246,7 @@ __global__ void __launch_bounds__(256) simba2_in_bwd_kernel(const float* __restr
 // r = relu(t s): g_t (fp16, in place on g_r) = g_r s [t s > 0]; g_s += sum g_r t [t s > 0].  One warp per row.
 __global__ void __launch_bounds__(256) scale_relu_bwd_kernel(__half* __restrict__ g, const float* __restrict__ t,
                                                              const float* __restrict__ s, float* __restrict__ g_s, int64_t rows, int n) {
+  pdl_begin();
   extern __shared__ float s_part[];
   for (int i = threadIdx.x; i < n; i += blockDim.x) s_part[i] = 0.f;
   __syncthreads();
@@ -280,7 +285,7 @@ int vres_bwd(__half* g, int64_t ldg, const __half* v_own, const __half* v0, cons
     return BSRL_ERR_SHAPE;
   }
   if (rows == 0) return BSRL_OK;
-  vres_bwd_kernel<<<(unsigned)blocks_for_rows(rows * (d >> 3), 256), 256, 0, stream>>>(g, ldg, v_own, v0, ab, g_v0, g_a, g_b, rows, d);
+  launch_kernel(vres_bwd_kernel, (unsigned)blocks_for_rows(rows * (d >> 3), 256), 256, 0, stream, g, ldg, v_own, v0, ab, g_v0, g_a, g_b, rows, d);
   BSRL_LAUNCH_OK("vres_bwd_kernel");
   return BSRL_OK;
 }
@@ -291,7 +296,7 @@ int add_f32_into_f16(__half* g, int64_t ldg, const float* acc, int64_t rows, int
     return BSRL_ERR_SHAPE;
   }
   if (rows == 0) return BSRL_OK;
-  add_f32_into_f16_kernel<<<(unsigned)blocks_for_rows(rows * (d >> 2), 256), 256, 0, stream>>>(g, ldg, acc, rows, d);
+  launch_kernel(add_f32_into_f16_kernel, (unsigned)blocks_for_rows(rows * (d >> 2), 256), 256, 0, stream, g, ldg, acc, rows, d);
   BSRL_LAUNCH_OK("add_f32_into_f16_kernel");
   return BSRL_OK;
 }
@@ -305,7 +310,7 @@ int simba2_out_bwd(const float* x0, const float* t2, const float* alpha, float c
     return BSRL_ERR_SHAPE;
   }
   if (rows == 0) return BSRL_OK;
-  simba2_out_bwd_kernel<<<(unsigned)blocks_for_rows(rows, 8), 256, d * sizeof(float), stream>>>(x0, t2, alpha, c_alpha, g_h, g_x0, g_t2,
+  launch_kernel(simba2_out_bwd_kernel, (unsigned)blocks_for_rows(rows, 8), 256, d * sizeof(float), stream, x0, t2, alpha, c_alpha, g_h, g_x0, g_t2,
                                                                                              g_alpha, rows, d);
   BSRL_LAUNCH_OK("simba2_out_bwd_kernel");
   return BSRL_OK;
@@ -318,7 +323,7 @@ int simba2_in_bwd(const float* t0, const float* s, const float* g_a, const float
     return BSRL_ERR_SHAPE;
   }
   if (rows == 0) return BSRL_OK;
-  simba2_in_bwd_kernel<<<(unsigned)blocks_for_rows(rows, 8), 256, d * sizeof(float), stream>>>(t0, s, g_a, g_b, g_t0, g_s, rows, d);
+  launch_kernel(simba2_in_bwd_kernel, (unsigned)blocks_for_rows(rows, 8), 256, d * sizeof(float), stream, t0, s, g_a, g_b, g_t0, g_s, rows, d);
   BSRL_LAUNCH_OK("simba2_in_bwd_kernel");
   return BSRL_OK;
 }
@@ -329,7 +334,7 @@ int scale_relu_bwd(__half* g, const float* t, const float* s, float* g_s, int64_
     return BSRL_ERR_SHAPE;
   }
   if (rows == 0) return BSRL_OK;
-  scale_relu_bwd_kernel<<<(unsigned)blocks_for_rows(rows, 8), 256, n * sizeof(float), stream>>>(g, t, s, g_s, rows, n);
+  launch_kernel(scale_relu_bwd_kernel, (unsigned)blocks_for_rows(rows, 8), 256, n * sizeof(float), stream, g, t, s, g_s, rows, n);
   BSRL_LAUNCH_OK("scale_relu_bwd_kernel");
   return BSRL_OK;
 }

@@ -229,6 +229,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
+  if (warp != 0) pdl_begin();    // the weight producer depends on no earlier kernel
   const int rows_d = d;          // weight rows of an N = d tile
   const int rows_h = HC;         // ... of an N = 128 tile
 
@@ -937,8 +938,8 @@ int block_tail(const BlockTailArgs& a, cudaStream_t stream) {
   p.x_tma = x_tma ? 1 : 0;
   p.status = status;
   int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
-  if (a.gelu) block_tail_kernel<true><<<grid, THREADS, SMEM_BYTES, stream>>>(tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
-  else block_tail_kernel<false><<<grid, THREADS, SMEM_BYTES, stream>>>(tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
+  if (a.gelu) launch_kernel(block_tail_kernel<true>, grid, THREADS, SMEM_BYTES, stream, tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
+  else launch_kernel(block_tail_kernel<false>, grid, THREADS, SMEM_BYTES, stream, tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
   BSRL_LAUNCH_OK("block_tail_kernel");
   return BSRL_OK;
 }

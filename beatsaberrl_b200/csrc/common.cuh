@@ -99,7 +99,42 @@ class DeviceOnce {
   cudaError_t err_[kMaxDevices] = {};
 };
 
+// Kernel launches.  Inside a sequence (PdlScope, after pdl_enable()) a launch is programmatic: the kernel may start while
+// its predecessor still runs, does what needs nothing of it (barriers, TMEM, weight loads) and waits in pdl_wait()
+// until every earlier kernel has completed and its writes are visible; outside of one it is an ordinary launch and
+// pdl_wait() returns at once.  Every kernel launched this way calls pdl_wait() before it touches anything an earlier
+// kernel of the sequence wrote or reads, and pdl_trigger() only after it: a successor's early part therefore runs when
+// at most ONE predecessor is unfinished, so reading the weights there is safe as long as no kernel of the sequence
+// writes them (the pack kernels run outside of sequences).
+extern thread_local bool g_pdl;
+inline void pdl_enable() { g_pdl = true; }
+struct PdlScope {
+  ~PdlScope() { g_pdl = false; }
+};
+template <typename... P, typename... A>
+inline void launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = g_pdl ? 1 : 0;
+  (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);     // BSRL_LAUNCH_OK follows every launch
+}
+
 // ----------------------------------------------------------------------------- device
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// the first statement of a kernel with nothing to do ahead of its predecessor
+__device__ __forceinline__ void pdl_begin() {
+  pdl_wait();
+  pdl_trigger();
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }

@@ -95,6 +95,7 @@ template <bool OBS_F16>
 __global__ void __launch_bounds__(kWarps * 32, 4) embed_gather_kernel(const void* __restrict__ obs_,
                                                                   int64_t n_envs, int note_geo,
                                                                   float z_asinh, EmbedBuffers out) {
+  pdl_begin();
   __shared__ float s_obs[kWarps][kObs + 2];
   __shared__ float s_geo[kWarps][kSlots * kGeoFeat];
   __shared__ int16_t s_lanes[5][64];
@@ -182,11 +183,9 @@ int embed_gather(const void* obs, int obs_dtype, int64_t n_envs, int note_geo, i
   int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
   if (obs_dtype == BSRL_F16)
-    embed_gather_kernel<true><<<static_cast<unsigned>(blocks), kWarps * 32, 0, stream>>>(
-        obs, n_envs, note_geo, z_asinh, out);
+    launch_kernel(embed_gather_kernel<true>, static_cast<unsigned>(blocks), kWarps * 32, 0, stream, obs, n_envs, note_geo, z_asinh, out);
   else
-    embed_gather_kernel<false><<<static_cast<unsigned>(blocks), kWarps * 32, 0, stream>>>(
-        obs, n_envs, note_geo, z_asinh, out);
+    launch_kernel(embed_gather_kernel<false>, static_cast<unsigned>(blocks), kWarps * 32, 0, stream, obs, n_envs, note_geo, z_asinh, out);
   BSRL_LAUNCH_OK("embed_gather_kernel");
   return BSRL_OK;
 }

@@ -160,6 +160,7 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
+  if (warp != 0) pdl_begin();    // the producer waits below, after its first weight stages
   const uint32_t stage_bytes = (uint32_t)d * 128u;      // a (d x 64) fp16 weight tile
 
   if (warp == 0) {
@@ -180,12 +181,19 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
       for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, ++tile_i) {
         const int e = part_of_tile(p, t);
         const int64_t row0 = p.part[e].row0 + (int64_t)(t - (int)p.part[e].tile0) * BM;
+        int early = 0;                          // first tile: weights ahead of the predecessor's last rows
+        if (tile_i == 0) {
+          ok = stage(&m.w0[e], 0);
+          for (; early < KB && early < STAGES - 1 && ok; ++early) ok = stage(&m.w1[e], 64 * early);
+          pdl_wait();
+          if (!ok) break;
+        }
         if (!mbar_wait(smem_u32(&sh->a_free), (tile_i & 1) ^ 1, abort)) { give_up(sh, p.status, 2); break; }
         const uint32_t bar = smem_u32(&sh->a_full);
         mbar_expect_tx(bar, SA_BYTES);
         tma_load_2d(sA, &m.a, 0, (int)row0, bar);
-        ok = stage(&m.w0[e], 0);
-        for (int kb = 0; kb < KB && ok; ++kb) ok = stage(&m.w1[e], 64 * kb);
+        if (tile_i != 0) ok = stage(&m.w0[e], 0);
+        for (int kb = early; kb < KB && ok; ++kb) ok = stage(&m.w1[e], 64 * kb);
       }
       // loads in flight must land before the CTA exits (bounded, ignoring abort)
       for (uint32_t j = it > STAGES ? it - STAGES : 0; j < it; ++j) {
@@ -496,7 +504,7 @@ int encoder_fused(const EncoderArgs& a, cudaStream_t stream) {
   p.h = a.h;
   p.status = status;
   const int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
-  encoder_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(mo, p);
+  launch_kernel(encoder_kernel, grid, THREADS, SMEM_BYTES, stream, mo, p);
   BSRL_LAUNCH_OK("encoder_kernel");
   return BSRL_OK;
 }

@@ -119,6 +119,7 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
+  pdl_begin();
   const uint32_t stage_tx = (uint32_t)(A_BYTES + N * BK * 2);
 
   if (warp == 0) {
@@ -363,7 +364,7 @@ int linear_ln(const LinearLnArgs& a, cudaStream_t stream) {
   p.n_tiles = (int)((a.M + BM - 1) / BM);
   p.status = status;
   const int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
-  linear_ln_kernel<<<grid, THREADS, SMEM_BYTES, stream>>>(tm_a, tm_w, tm_h, p);
+  launch_kernel(linear_ln_kernel, grid, THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_h, p);
   BSRL_LAUNCH_OK("linear_ln_kernel");
   return BSRL_OK;
 }

@@ -23,6 +23,7 @@ __device__ __forceinline__ uint32_t tile_off(int row, int kc) {
 }
 
 __global__ void __launch_bounds__(THREADS) linear_mma_kernel(LinearArgs p) {
+  pdl_begin();
   extern __shared__ __align__(128) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp >> 2, wn = warp & 3;  // 2 x 4 warps, warp tile 64 x 32
@@ -172,7 +173,7 @@ int linear_mma(const LinearArgs& p, cudaStream_t stream) {
     set_error("linear: too many tiles");
     return BSRL_ERR_SHAPE;
   }
-  linear_mma_kernel<<<static_cast<unsigned>(tiles), THREADS, STAGES * STAGE_BYTES, stream>>>(p);
+  launch_kernel(linear_mma_kernel, static_cast<unsigned>(tiles), THREADS, STAGES * STAGE_BYTES, stream, p);
   BSRL_LAUNCH_OK("linear_mma_kernel");
   return BSRL_OK;
 }

@@ -131,6 +131,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
+  pdl_begin();
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
@@ -409,7 +410,7 @@ int linear_res(const LinearArgs& p, cudaStream_t stream) {
   const int m_tiles = (int)((p.M + BM - 1) / BM), n_tiles = (p.N + BN - 1) / BN;
   const int r32 = p.R && reinterpret_cast<uintptr_t>(p.R) % 32 == 0 && p.ldr % 8 == 0;        // 32-byte residual loads
   auto* kernel = p.R ? linear_res_kernel<true> : linear_res_kernel<false>;
-  kernel<<<sm_count(), THREADS, SMEM_BYTES, stream>>>(tm_a, tm_w, tm_c, tma_c ? 1 : 0, r32, p, m_tiles, n_tiles, status);
+  launch_kernel(kernel, sm_count(), THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, tma_c ? 1 : 0, r32, p, m_tiles, n_tiles, status);
   BSRL_LAUNCH_OK("linear_res_kernel");
   return BSRL_OK;
 }

@@ -111,6 +111,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
+  pdl_begin();
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
@@ -562,7 +563,7 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
   int64_t grid = m_tiles * n_tiles * (p.k_splits > 1 ? p.k_splits : 1);
   if (grid > sm_count()) grid = sm_count();
   auto* kernel = p.a_sums ? linear_tc5_kernel<false, true> : p.R ? linear_tc5_kernel<true, false> : linear_tc5_kernel<false, false>;
-  kernel<<<(unsigned)grid, THREADS, SMEM_BYTES, stream>>>(tm_a, tm_w, tm_c, tma_c ? 1 : 0, p, (int)m_tiles, n_tiles, status);
+  launch_kernel(kernel, (unsigned)grid, THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, tma_c ? 1 : 0, p, (int)m_tiles, n_tiles, status);
   BSRL_LAUNCH_OK("linear_tc5_kernel");
   return BSRL_OK;
 }

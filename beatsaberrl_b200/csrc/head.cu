@@ -41,6 +41,7 @@ __device__ __forceinline__ float uniform01(uint32_t x) {   // in (0, 1)
 }
 
 __global__ void __launch_bounds__(256) head_tail_kernel(HeadTailArgs p) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   for (int64_t env = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); env < p.n_envs;
@@ -169,7 +170,7 @@ int head_tail(const HeadTailArgs& a, cudaStream_t stream) {
   int64_t blocks = (a.n_envs + 7) / 8;
   int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  head_tail_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(a);
+  launch_kernel(head_tail_kernel, static_cast<unsigned>(blocks), 256, 0, stream, a);
   BSRL_LAUNCH_OK("head_tail_kernel");
   return BSRL_OK;
 }

@@ -19,6 +19,7 @@ __global__ void __launch_bounds__(256, RPW > 1 ? 4 : 1) layernorm_kernel(const f
                                                        const float* __restrict__ beta, float eps,
                                                        int64_t rows, int d, __half* __restrict__ y,
                                                        int64_t ldy) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const int nvec = d >> 2;
@@ -126,9 +127,9 @@ int launch_layernorm(const float* x, int64_t ldx, RowMap xmap, const float* gamm
   int64_t blocks = (rows + 8 * rpw - 1) / (8 * rpw);
   if (blocks > cap) blocks = cap;
   const unsigned nb = static_cast<unsigned>(blocks);
-  if (rpw == 4) layernorm_kernel<4, F32><<<nb, 256, 0, stream>>>(x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy);
-  else if (rpw == 2) layernorm_kernel<2, F32><<<nb, 256, 0, stream>>>(x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy);
-  else layernorm_kernel<1, F32><<<nb, 256, 0, stream>>>(x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy);
+  if (rpw == 4) launch_kernel(layernorm_kernel<4, F32>, nb, 256, 0, stream, x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy);
+  else if (rpw == 2) launch_kernel(layernorm_kernel<2, F32>, nb, 256, 0, stream, x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy);
+  else launch_kernel(layernorm_kernel<1, F32>, nb, 256, 0, stream, x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy);
   BSRL_LAUNCH_OK("layernorm_kernel");
   return BSRL_OK;
 }
@@ -142,6 +143,7 @@ __global__ void __launch_bounds__(256) simba2_rows_kernel(int mode, const float*
                                                          const float* __restrict__ vec, float c_alpha,
                                                          int64_t rows, int d, __half* __restrict__ out16,
                                                          int64_t ld16) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const int nvec = d >> 2;
@@ -203,6 +205,7 @@ __global__ void __launch_bounds__(256) simba2_rows_kernel(int mode, const float*
 // out16 = relu(in * s), elementwise on (rows, n) fp32 -> fp16
 __global__ void scale_relu_kernel(const float* __restrict__ in, const float* __restrict__ s, int64_t rows, int n,
                                   __half* __restrict__ out16) {
+  pdl_begin();
   const int per_row = n >> 2;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row;
        i += (int64_t)gridDim.x * blockDim.x) {
@@ -230,7 +233,7 @@ int simba2_rows(int mode, const float* in, float* x, const float* vec, float c_a
   int64_t blocks = (rows + 7) / 8;
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  simba2_rows_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(mode, in, x, vec, c_alpha, rows, d, out16, ld16);
+  launch_kernel(simba2_rows_kernel, static_cast<unsigned>(blocks), 256, 0, stream, mode, in, x, vec, c_alpha, rows, d, out16, ld16);
   BSRL_LAUNCH_OK("simba2_rows_kernel");
   return BSRL_OK;
 }
@@ -244,7 +247,7 @@ int scale_relu_rows(const float* in, const float* s, int64_t rows, int n, __half
   int64_t blocks = (rows * (n >> 2) + 255) / 256;
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  scale_relu_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(in, s, rows, n, out16);
+  launch_kernel(scale_relu_kernel, static_cast<unsigned>(blocks), 256, 0, stream, in, s, rows, n, out16);
   BSRL_LAUNCH_OK("scale_relu_kernel");
   return BSRL_OK;
 }

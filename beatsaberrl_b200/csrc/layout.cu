@@ -21,6 +21,8 @@ void set_error(const char* fmt, ...) {
 }
 const char* last_error() { return g_err; }
 
+thread_local bool g_pdl = false;
+
 int cuda_fail(cudaError_t e, const char* what) {
   set_error("CUDA error %d (%s) at %s", (int)e, cudaGetErrorString(e), what);
   return BSRL_ERR_CUDA;

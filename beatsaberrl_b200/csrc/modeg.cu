@@ -210,6 +210,7 @@ bool g_tail_fused(const GLayout& l, int engine) {
 __global__ void __launch_bounds__(256) embed_g_kernel(const float* __restrict__ obs, int64_t n_envs, int obs_dim, int body_dim,
                                                       int body_k, int n_obj, int obj_dim, __half* __restrict__ f_body,
                                                       __half* __restrict__ f_obj, float* __restrict__ key_bias) {
+  pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const int T = 1 + n_obj;
@@ -263,11 +264,13 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
     int64_t blocks = (B + 7) / 8;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    embed_g_kernel<<<(unsigned)blocks, 256, 0, st>>>(obs, B, l.obs_dim, l.body_dim, l.body_k, l.n_obj, l.obj_dim, f_body, f_obj,
+    launch_kernel(embed_g_kernel, (unsigned)blocks, 256, 0, st, obs, B, l.obs_dim, l.body_dim, l.body_k, l.n_obj, l.obj_dim, f_body, f_obj,
                                                      key_bias);
     BSRL_LAUNCH_OK("embed_g_kernel");
     return BSRL_OK;
   }));
+  PdlScope pdl;
+  begin_overlap(B * l.T);
   set_stage(kStEncoder);
   {
     LinearArgs a = linear_args(f_body, l.body_k, c.W(l.body), l.body.pitch, c.Bv(l.body), x, d, 1, 0, B, d, l.body_k);

@@ -402,6 +402,8 @@ struct Bwd {
 
     // ---- head tail
     BSRL_TRY(head_tail_bwd(tail, g_logprob, g_entropy, g_value, g_vlogits, g_logits, scale, graw, w.ld_graw, gvraw, w.ld_gv, st));
+    PdlScope pdl;
+    begin_overlap(R);
 
     // ---- recompute the critic's activations (its pool lands in z beside the trunk's output)
     BSRL_TRY(layernorm(x_last, d, ident, c.G(l.critic_ln), c.Be(l.critic_ln), eps, R, d, h16, d, st));
