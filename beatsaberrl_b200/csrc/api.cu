@@ -79,6 +79,7 @@ int linear(const LinearArgs& p, cudaStream_t st) {
                 (long long)p.M, p.N, p.K);
       return (int)BSRL_ERR_UNSUPPORTED;
     }
+    if (g_call_engine == 0 && linear_small_wins(p)) return linear_small(p, st);
     if (g_call_engine == 0 && p.M >= 128 && linear_tc5_ok(p)) return linear_tc5(p, st);
     return linear_mma(p, st);
   });
@@ -992,6 +993,7 @@ int bsrl_linear(const void* a_f16, const void* w_f16, const float* bias, const f
   p.R = residual;
   p.ldr = n;
   if (engine == 0) return linear_mma(p, as_stream(stream));
+  if (engine == 2) return linear_small(p, as_stream(stream));
   if (engine == 1) {
     if (!linear_tc5_ok(p)) {
       set_error("linear: shape m=%lld n=%d k=%d does not fit the tcgen05 engine", (long long)m, n, k);
@@ -999,7 +1001,7 @@ int bsrl_linear(const void* a_f16, const void* w_f16, const float* bias, const f
     }
     return linear_tc5(p, as_stream(stream));
   }
-  set_error("linear: engine must be 0 (warp-MMA) or 1 (tcgen05)");
+  set_error("linear: engine must be 0 (warp-MMA), 1 (tcgen05) or 2 (small tiles)");
   return BSRL_ERR_UNSUPPORTED;
 }
 

@@ -50,6 +50,9 @@ LinearArgs linear_args(const __half* A, int lda, const __half* W, int ldw, const
                        void* C, int ldc, int out_f32, int relu, int64_t M, int N, int K);
 
 int linear_mma(const LinearArgs& p, cudaStream_t stream);   // warp-MMA engine
+bool linear_small_ok(const LinearArgs& p);                   // few rows: small warp-MMA tiles (gemm_small.cu)
+bool linear_small_wins(const LinearArgs& p);                 // ... and it is the faster kernel for them
+int linear_small(const LinearArgs& p, cudaStream_t stream);
 int linear_tc5(const LinearArgs& p, cudaStream_t stream);   // tcgen05 / TMEM engine
 bool linear_tc5_ok(const LinearArgs& p);                     // shape fits the tcgen05 engine
 bool linear_tc5_sums_ok(const LinearArgs& p);                // ... and its column sums can ride along (a_sums)

@@ -370,3 +370,28 @@ def test_linear_resident_weights(native, m, n, k, relu, res):
         ref = ref + r.double()
     tol = 2e-5 if res else 2 ** -11
     assert bool(((out.double() - ref).abs() <= tol * ref.abs() + 2e-5).all())
+
+
+@pytest.mark.parametrize("m,n,k,relu,resid,f32", [
+    (1, 8, 64, 0, 0, 1), (16, 32, 128, 1, 0, 0), (17, 40, 192, 0, 1, 1),      # one tile, remainders in every direction
+    (29, 160, 960, 0, 0, 1), (45, 1024, 1408, 2, 0, 0),                       # a full ring, a ring that is refilled
+    (700, 256, 640, 0, 0, 1), (1023, 256, 640, 0, 1, 0),                      # the last of the 16 x 32 tiles, 32 x 32 tiles
+])
+def test_linear_small_tiles(native, m, n, k, relu, resid, f32):
+    """The few-row kernel adds the same products in the same order as the general warp-MMA kernel: equal bits."""
+    g = torch.Generator(device="cuda").manual_seed(m * 7 + n)
+    a = torch.randn(m, k, generator=g, device="cuda").half()
+    w = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).half()
+    bias = torch.randn(n, generator=g, device="cuda")
+    r = torch.randn(m, n, generator=g, device="cuda") if resid else None
+    outs = []
+    for engine in (0, 2):
+        out = torch.full((m, n), float("nan"), dtype=torch.float32 if f32 else torch.float16, device="cuda")
+        native.check(native.lib.bsrl_linear(a.data_ptr(), w.data_ptr(), bias.data_ptr(), r.data_ptr() if resid else None,
+                                            out.data_ptr(), f32, relu, m, n, k, engine, _stream()))
+        outs.append(out)
+    assert torch.equal(*outs)
+    ref = a.float() @ w.float().t() + bias
+    ref = ref.relu() if relu == 1 else F.gelu(ref) if relu == 2 else ref
+    ref = ref + r if resid else ref
+    torch.testing.assert_close(outs[1].float(), ref, **(dict(atol=2e-4, rtol=1e-4) if f32 else dict(atol=4e-3, rtol=1e-3)))
