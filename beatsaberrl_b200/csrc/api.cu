@@ -84,6 +84,14 @@ int linear(const LinearArgs& p, cudaStream_t st) {
     return linear_mma(p, st);
   });
 }
+// two products that do not depend on each other: one launch where both are small
+int linear_two(const LinearArgs& p, const LinearArgs& q, cudaStream_t st) {
+  if (g_call_engine == 0 && linear_small_two_wins(p, q))
+    return timed(st, 2.0 * p.M * p.N * p.K + 2.0 * q.M * q.N * q.K, linear_bytes(p) + linear_bytes(q),
+                 [&] { return linear_small_two(p, q, st); });
+  int rc = linear(p, st);
+  return rc != BSRL_OK ? rc : linear(q, st);
+}
 bool linear_rows_ok(const LinearArgs& p) { return g_call_engine == 0 && linear_tc5_ok(p); }
 int layernorm(const float* x, int64_t ldx, RowMap xmap, const float* g, const float* b, float eps,
               int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t st) {
@@ -229,7 +237,8 @@ void head_shape(const bsrl_config& cfg, const Layout& l, HeadTailArgs& t) {
 
 // readout (B, 5d) f16 -> SimBa / SimBaV2 trunk -> h (f16, in z[:, d:]) -> packed head outputs raw (B, head_cols_pad) f32
 // (NotePolicy._trunk + the packed head GEMM, python/policy.py:1107-1155, :1311-1335)
-int run_trunk(const Ctx& c, const __half* lead16, float* raw) {
+// with_proj / with_heads: independent products that go along with the first and the last one
+int run_trunk(const Ctx& c, const __half* lead16, float* raw, const LinearArgs* with_proj = nullptr, const LinearArgs* with_heads = nullptr) {
   const Layout& l = c.l;
   const Workspace& w = c.w;
   const int d = l.d, D = l.D;
@@ -244,7 +253,8 @@ int run_trunk(const Ctx& c, const __half* lead16, float* raw) {
   __half* z = tr ? tr->z : at<__half>(c.ws, w.z);
   const int ldz = d + D;
   g_stage = kStTrunk;
-  BSRL_TRY(linear(linear_args(lead16, kLead * d, c.W(l.trunk_proj), kLead * d, c.Bv(l.trunk_proj), xt, D, 1, 0, B, D, kLead * d), c.st));
+  const LinearArgs proj = linear_args(lead16, kLead * d, c.W(l.trunk_proj), kLead * d, c.Bv(l.trunk_proj), xt, D, 1, 0, B, D, kLead * d);
+  BSRL_TRY(with_proj ? linear_two(proj, *with_proj, c.st) : linear(proj, c.st));
   if (l.trunk_v2) {
     // SimBaV2 (python/policy.py:1140-1155): x = l2n(s_in W_in z); y = l2n(W2 relu(s_1 W1 x));
     // x = l2n(x + alpha (y - x)); h = sqrt(D) x.  GEMMs on fp16 operands, everything else fp32.
@@ -263,7 +273,70 @@ int run_trunk(const Ctx& c, const __half* lead16, float* raw) {
     BSRL_TRY(linear(p2, c.st));
     BSRL_TRY(layernorm(xt2, D, ident, c.G(l.trunk_ln2), c.Be(l.trunk_ln2), eps, B, D, z + d, ldz, c.st));
   }
-  return linear(linear_args(z + d, ldz, c.W(l.heads), D, c.Bv(l.heads), raw, l.head_cols_pad, 1, 0, B, l.head_cols_pad, D), c.st);
+  const LinearArgs heads = linear_args(z + d, ldz, c.W(l.heads), D, c.Bv(l.heads), raw, l.head_cols_pad, 1, 0, B, l.head_cols_pad, D);
+  return with_heads ? linear_two(heads, *with_heads, c.st) : linear(heads, c.st);
+}
+
+// The blocks and the critic's attention for few environments (Paths::small): four launches per block, each spread over
+// many SMs -- attention per (env, head group), out-projection, FFN-up and FFN-down in 16-row tiles, the LayerNorms at the
+// entry of the kernels that need them -- instead of two that walk a 128-row tile through its phases on one SM.
+// x: the token stream, h: block 0's LayerNorm rows (from the encoder kernel).
+int run_blocks_small(const Ctx& c, float* x, const __half* h, const float* key_bias, __half* lead16, __half* att_c) {
+  const Layout& l = c.l;
+  const Workspace& w = c.w;
+  const int d = l.d, F = l.F;
+  const int64_t B = c.B, R = B * kT, Rl = B * kLead;
+  const RowMap ident = identity_map(), lead_rows{kLead, kT, 0};
+  __half* att = at<__half>(c.ws, w.att);
+  __half* hid = at<__half>(c.ws, w.hid);
+  __half* v0buf = l.value_residual ? at<__half>(c.ws, w.v0) : nullptr;
+  float* x_lead = at<float>(c.ws, w.x_lead);
+  auto norm_of = [&](const float* rows, const Norm& n, int quads) { return RowNorm{rows, d, ident, c.G(n), c.Be(n), c.cfg->eps, quads}; };
+  auto attn = [&](const AttnSmallArgs* a, int n) {
+    g_stage = kStAttnBlock;
+    return timed(c.st, n * (2.0 * R * 3.0 * d * d + 4.0 * R * kT * d), n * (double)R * d * 6, [&] { return attn_small(a, n, l.H, B, c.st); });
+  };
+  auto product = [&](const LinearArgs& p, int start, const RowNorm* n) {
+    g_stage = kStBlockTail;
+    return timed(c.st, 2.0 * p.M * p.N * p.K, linear_bytes(p), [&] { return linear_small_block(p, start, n, c.st); });
+  };
+  for (int i = 0; i < l.L; ++i) {
+    const BlockW& b = l.blocks[i];
+    const bool last = i + 1 == l.L;
+    float* x_next = c.train && !last ? c.train->x[i + 1] : x;
+    AttnSmallArgs a[2];
+    memset(a, 0, sizeof(a));
+    a[0].d = d;
+    if (i == 0) { a[0].h = h; a[0].ldh = d; }
+    else a[0].norm = norm_of(x, b.ln_attn, 1);
+    a[0].wg = c.W(b.qkv_g); a[0].bg = c.Bv(b.qkv_g);
+    a[0].key_bias = key_bias; a[0].q_first = 0; a[0].n_q = last ? kLead : kT;
+    a[0].out = att; a[0].ldo = d;
+    if (v0buf && i == 0) a[0].v_out = v0buf;
+    if (v0buf && i > 0) { a[0].v0 = v0buf; a[0].vres = at<float>(c.arena, b.vres); }
+    if (last) {                       // the critic's query reads the same rows: same launch
+      a[1].d = d;
+      a[1].norm = norm_of(x, l.critic_ln, 1);
+      a[1].wg = c.W(l.critic_qkv_g); a[1].bg = c.Bv(l.critic_qkv_g);
+      a[1].key_bias = key_bias; a[1].q_first = 2; a[1].n_q = 1;
+      a[1].out = att_c; a[1].ldo = d;
+    }
+    BSRL_TRY(attn(a, last ? 2 : 1));
+    const int64_t M = last ? Rl : R;
+    float* x1 = last ? x_lead : x_next;
+    LinearArgs po = linear_args(att, d, c.W(b.out), d, c.Bv(b.out), x1, d, 1, 0, M, d, d);
+    po.R = x; po.ldr = d;
+    if (last) po.rmap = lead_rows;
+    BSRL_TRY(product(po, 1, nullptr));
+    const RowNorm n = norm_of(x1, b.ln_ffn, 0);
+    BSRL_TRY(product(linear_args(nullptr, d, c.W(b.up), d, c.Bv(b.up), hid, F, 0, 1, M, F, d), 0, &n));
+    LinearArgs pd = last ? linear_args(hid, F, c.W(b.down), F, c.Bv(b.down), lead16, d, 0, 0, M, d, F)
+                         : linear_args(hid, F, c.W(b.down), F, c.Bv(b.down), x1, d, 1, 0, M, d, F);
+    pd.R = x1; pd.ldr = d;
+    BSRL_TRY(product(pd, 2, nullptr));
+    x = x_next;
+  }
+  return BSRL_OK;
 }
 
 int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs& tail_in) {
@@ -286,6 +359,10 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
 
   bool have_h = false, have_hv = false;
   BSRL_TRY(run_embed(c, obs, obs_dtype, x, key_bias, h, &have_h));
+  __half* lead16 = c.train ? c.train->lead16 : at<__half>(c.ws, w.lead16);
+  __half* att_c = at<__half>(c.ws, w.att_c);
+  const bool small = c.paths.small && have_h;
+  if (small) BSRL_TRY(run_blocks_small(c, x, h, key_bias, lead16, att_c));
 
   // Fused block tail (out-projection + LayerNorm + FFN in one tcgen05 kernel) where the widths fit;
   // it also emits the next block's LayerNorm rows (and the critic's), so the standalone LayerNorm
@@ -337,7 +414,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
                     i > 0 ? at<float>(c.arena, l.blocks[i].vres) : nullptr, c.st);
   };
 
-  for (int i = 0; i + 1 < l.L; ++i) {
+  for (int i = 0; i + 1 < l.L && !small; ++i) {
     const BlockW& b = l.blocks[i];
     float* x_next = c.train ? c.train->x[i + 1] : x;
     if (!have_h) BSRL_TRY(layernorm(x, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h, d, c.st));
@@ -379,8 +456,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
   // final block: keys/values over all 29 rows, everything else on the 5 lead rows
   float* x_lead = at<float>(c.ws, w.x_lead);
   __half* h_lead = at<__half>(c.ws, w.h_lead);
-  __half* lead16 = c.train ? c.train->lead16 : at<__half>(c.ws, w.lead16);
-  {
+  if (!small) {
     const BlockW& b = l.blocks[l.L - 1];
     if (!have_h) BSRL_TRY(layernorm(x, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h, d, c.st));
     if (fused_qkv) {
@@ -425,18 +501,10 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
     }
   }
 
-  // SimBa trunk on the (B, 5d) readout; its output h lands in z[:, d:]; then the packed heads
+  // adapool critic over the resolved stream entering the final block (still in x): its attention ...
   __half* z = c.train ? c.train->z : at<__half>(c.ws, w.z);
   const int ldz = d + D;
-  float* raw = c.train ? c.train->raw : at<float>(c.ws, w.raw);
-  BSRL_TRY(run_trunk(c, lead16, raw));
-
-  // adapool critic over the resolved stream entering the final block (still in x)
-  __half* att_c = at<__half>(c.ws, w.att_c);
-  __half* m1 = at<__half>(c.ws, w.m1);
-  __half* m2 = at<__half>(c.ws, w.m2);
-  float* vraw = c.train ? c.train->vraw : at<float>(c.ws, w.vraw);
-  {
+  if (!small) {
     const RowMap torso_rows{1, kT, 2};
     g_stage = kStCritic;
     const __half* hc = have_hv ? hv : h;
@@ -451,11 +519,19 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
       BSRL_TRY(linear(pq, c.st));
       BSRL_TRY(attention(qkv, 3 * d, key_bias, B, d, l.H, 2, 1, att_c, d, c.st));
     }
-    BSRL_TRY(linear(linear_args(att_c, d, c.W(l.critic_out), d, c.Bv(l.critic_out), z, ldz, 0, 0, B, d, d), c.st));
-    BSRL_TRY(linear(linear_args(z, ldz, c.W(l.critic_m0), ldz, c.Bv(l.critic_m0), m1, D, 0, 1, B, D, ldz), c.st));
-    BSRL_TRY(linear(linear_args(m1, D, c.W(l.critic_m1), D, c.Bv(l.critic_m1), m2, D, 0, 1, B, D, D), c.st));
-    BSRL_TRY(linear(linear_args(m2, D, c.W(l.critic_m2), D, c.Bv(l.critic_m2), vraw, l.bins_pad, 1, 0, B, l.bins_pad, D), c.st));
   }
+  // ... then the SimBa trunk on the (B, 5d) readout, its output h landing in z[:, d:], and the packed heads; the critic's
+  // output projection (z[:, :d]) and first MLP layer go along with the trunk's first product and the heads
+  __half* m1 = at<__half>(c.ws, w.m1);
+  __half* m2 = at<__half>(c.ws, w.m2);
+  float* raw = c.train ? c.train->raw : at<float>(c.ws, w.raw);
+  float* vraw = c.train ? c.train->vraw : at<float>(c.ws, w.vraw);
+  const LinearArgs c_out = linear_args(att_c, d, c.W(l.critic_out), d, c.Bv(l.critic_out), z, ldz, 0, 0, B, d, d);
+  const LinearArgs c_m0 = linear_args(z, ldz, c.W(l.critic_m0), ldz, c.Bv(l.critic_m0), m1, D, 0, 1, B, D, ldz);
+  BSRL_TRY(run_trunk(c, lead16, raw, &c_out, &c_m0));
+  g_stage = kStCritic;
+  BSRL_TRY(linear(linear_args(m1, D, c.W(l.critic_m1), D, c.Bv(l.critic_m1), m2, D, 0, 1, B, D, D), c.st));
+  BSRL_TRY(linear(linear_args(m2, D, c.W(l.critic_m2), D, c.Bv(l.critic_m2), vraw, l.bins_pad, 1, 0, B, l.bins_pad, D), c.st));
 
   HeadTailArgs t = tail_in;
   t.raw = raw; t.ld_raw = l.head_cols_pad;
@@ -485,7 +561,7 @@ int make_ctx(Ctx& c, const bsrl_config* cfg, const void* arena, int64_t n_envs, 
   c.cfg = cfg;
   c.l = make_layout(*cfg);
   use_process_engine();
-  c.paths = plan_paths(c.l, g_call_engine);
+  c.paths = plan_paths(c.l, g_call_engine, n_envs);
   c.w = make_workspace(c.l, n_envs, c.paths);
   if (ws_bytes < c.w.bytes) {
     set_error("forward: workspace %lld bytes < required %lld", (long long)ws_bytes, (long long)c.w.bytes);
@@ -656,7 +732,7 @@ int64_t bsrl_workspace_bytes(const bsrl_config* cfg, int64_t n_envs) {
   if (validate_config(cfg) != BSRL_OK) return -1;
   if (n_envs < 0) return -1;
   Layout l = make_layout(*cfg);
-  return make_workspace(l, n_envs, plan_paths(l, g_engine.load(std::memory_order_relaxed))).bytes;
+  return make_workspace(l, n_envs, plan_paths(l, g_engine.load(std::memory_order_relaxed), n_envs)).bytes;
 }
 
 int bsrl_forward(const bsrl_config* cfg, const void* arena, const void* obs, int32_t obs_dtype,
@@ -945,7 +1021,7 @@ int bsrl_workspace_region(const bsrl_config* cfg, int64_t n_envs, const char* na
     return BSRL_ERR_NULL;
   }
   Layout l = make_layout(*cfg);
-  Workspace w = make_workspace(l, n_envs, plan_paths(l, g_engine.load(std::memory_order_relaxed)));
+  Workspace w = make_workspace(l, n_envs, plan_paths(l, g_engine.load(std::memory_order_relaxed), n_envs));
   int64_t off = -1, r = 0, cc = 0, ld = 0;
   int32_t dt = BSRL_F16;
   if (!strcmp(name, "trunk_h")) { off = w.z + (int64_t)l.d * 2; r = n_envs; cc = l.D; ld = l.d + l.D; }

@@ -24,6 +24,7 @@
 // for one head of 48) is staged in shared memory and leaves as one TMA store per env.  All waits are
 // bounded (tc5.cuh).
 #include "kernels.cuh"
+#include "attend.cuh"
 #include "tc5.cuh"
 
 namespace bsrl {
@@ -91,158 +92,6 @@ struct Params {
 __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
   atomicCAS(status, 0, KERNEL_ID * 16 + role);
   sh->abort = 1;
-}
-
-__device__ __forceinline__ float ex2_approx(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-__device__ __forceinline__ float rcp_approx(float x) {
-  float y;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-
-// Attention of one (env, head) pair from the shared q|k|v tile; one warp.  q, k, v are byte
-// addresses (shared window) of the pair's first row / first column; rows are LDQ bytes apart.
-// The MT 16-row query tiles are processed side by side: two independent dependency chains per warp
-// (the kernel is latency-bound here) and each K / V fragment is fetched once for both.
-// OB: bytes per row of the staged group output (128: two heads of 32, swizzled; 96: one head of 48, dense)
-// BODY: one more key outside the tile (the body token): x_lane = q_row . k_0 for row `lane` (raw), kb0 its
-// base-2 key bias, v0 its DH values (shared memory, generic pointer); its score joins each row's softmax and its
-// probability times v_0 starts the row's output.
-template <int MT, int DH, int LDQ, int OB, bool BODY = false>
-__device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t sv, const float (&kb)[4][2],
-                                            int n_q, __half* out_env, int ldo, int lane, uint8_t* so, int so_row0, int so_piece0,
-                                            float x_lane = 0.f, float kb0 = 0.f, const __half* v0 = nullptr) {
-  const int g = lane >> 2, tig = lane & 3;
-  const float scale = rsqrtf((float)DH) * 1.4426950408889634f;   // 1/sqrt(dh) * log2(e)
-  float s[MT][4][4];
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) s[mt][nt][e] = 0.f;
-#pragma unroll
-  for (int ks = 0; ks < DH / 16; ++ks) {
-    uint32_t a[MT][4];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-      ldmatrix_x4(a[mt], sq + (mt * 16 + (lane & 15)) * LDQ + (ks * 16 + (lane >> 4) * 8) * 2);
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      uint32_t b[4];
-      const int row = j * 16 + (lane & 7) + ((lane >> 4) << 3);
-      ldmatrix_x4(b, sk + row * LDQ + (ks * 16 + ((lane >> 3) & 1) * 8) * 2);
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        mma_f16(s[mt][2 * j], a[mt], b[0], b[1]);
-        mma_f16(s[mt][2 * j + 1], a[mt], b[2], b[3]);
-      }
-    }
-  }
-  uint32_t pa[MT][2][4];
-  float p0[MT][2];                    // BODY: the body key's probability for rows g and g + 8 of each query tile
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt) {
-    float mx[2] = {-INFINITY, -INFINITY};
-    if (BODY) {
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        p0[mt][r] = fmaf(__shfl_sync(0xffffffffu, x_lane, mt * 16 + g + r * 8), scale, kb0);
-        mx[r] = p0[mt][r];
-      }
-    }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        s[mt][nt][e] = fmaf(s[mt][nt][e], scale, kb[nt][e & 1]);   // base-2 logits: scale and key bias carry log2(e)
-        mx[e >> 1] = fmaxf(mx[e >> 1], s[mt][nt][e]);
-      }
-    float sum[2] = {0.f, 0.f};
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-    }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        s[mt][nt][e] = ex2_approx(s[mt][nt][e] - mx[e >> 1]);
-        sum[e >> 1] += s[mt][nt][e];
-      }
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
-      sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
-      if (BODY) {
-        p0[mt][r] = ex2_approx(p0[mt][r] - mx[r]);
-        sum[r] = rcp_approx(sum[r] + p0[mt][r]);
-        p0[mt][r] *= sum[r];
-      } else {
-        sum[r] = rcp_approx(sum[r]);
-      }
-    }
-#pragma unroll
-    for (int ks = 0; ks < 2; ++ks) {
-      pa[mt][ks][0] = pack_half2(s[mt][2 * ks][0] * sum[0], s[mt][2 * ks][1] * sum[0]);
-      pa[mt][ks][1] = pack_half2(s[mt][2 * ks][2] * sum[1], s[mt][2 * ks][3] * sum[1]);
-      pa[mt][ks][2] = pack_half2(s[mt][2 * ks + 1][0] * sum[0], s[mt][2 * ks + 1][1] * sum[0]);
-      pa[mt][ks][3] = pack_half2(s[mt][2 * ks + 1][2] * sum[1], s[mt][2 * ks + 1][3] * sum[1]);
-    }
-  }
-  float o[MT][DH / 8][4];
-#pragma unroll
-  for (int nt = 0; nt < DH / 8; ++nt) {
-    float2 v = make_float2(0.f, 0.f);
-    if (BODY) v = __half22float2(*reinterpret_cast<const __half2*>(v0 + nt * 8 + tig * 2));
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      o[mt][nt][0] = BODY ? p0[mt][0] * v.x : 0.f;
-      o[mt][nt][1] = BODY ? p0[mt][0] * v.y : 0.f;
-      o[mt][nt][2] = BODY ? p0[mt][1] * v.x : 0.f;
-      o[mt][nt][3] = BODY ? p0[mt][1] * v.y : 0.f;
-    }
-  }
-#pragma unroll
-  for (int ks = 0; ks < 2; ++ks) {
-#pragma unroll
-    for (int j = 0; j < DH / 16; ++j) {
-      uint32_t b[4];
-      const int row = ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-      ldmatrix_x4_trans(b, sv + row * LDQ + (j * 16 + (lane >> 4) * 8) * 2);
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        mma_f16(o[mt][2 * j], pa[mt][ks], b[0], b[1]);
-        mma_f16(o[mt][2 * j + 1], pa[mt][ks], b[2], b[3]);
-      }
-    }
-  }
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int qrow = mt * 16 + g + r * 8;
-      if (qrow < n_q && so) {
-        // staged for the group's TMA store.  128-byte rows: 16-byte piece p of row r at ((p ^ (r & 7)) << 4),
-        // the 8 rows of a store instruction hit 32 different banks; 96-byte rows: dense (2-way conflicts)
-        const int row = so_row0 + qrow;
-        uint8_t* orow = so + row * OB + tig * 4;
-#pragma unroll
-        for (int nt = 0; nt < DH / 8; ++nt)
-          *reinterpret_cast<uint32_t*>(orow + (OB == 128 ? (((so_piece0 + nt) ^ (row & 7)) << 4) : ((so_piece0 + nt) << 4))) =
-              pack_half2(o[mt][nt][r * 2], o[mt][nt][r * 2 + 1]);
-      } else if (qrow < n_q) {
-        __half* orow = out_env + (int64_t)qrow * ldo + tig * 2;
-#pragma unroll
-        for (int nt = 0; nt < DH / 8; ++nt)
-          *reinterpret_cast<uint32_t*>(orow + nt * 8) = pack_half2(o[mt][nt][r * 2], o[mt][nt][r * 2 + 1]);
-      }
-    }
 }
 
 // VRES: the value-residual code of the drain is compiled in (it costs ~14 % of the kernel even when idle)
@@ -559,37 +408,8 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
             // the projection of the next head group shares, 16 warp MMAs of 32 cycles per (env, head); this is ~200
             // plain instructions (lane = key for the scores, lane = output column for the weighted sum).
             if (mt_own == 0) {
-              const uint8_t* rows_g = sQ_g + (env_l * EROWS) * LDQ;
-              const uint8_t* qrow = rows_g + p.q_first * LDQ + (hh * DH) * 2;
-              const uint8_t* krow = rows_g + (lane < NKEYS ? lane : 0) * LDQ + (GD + hh * DH) * 2;
-              float sc = 0.f;
-#pragma unroll
-              for (int ch = 0; ch < DH / 8; ++ch) {
-                const uint4 qv = *reinterpret_cast<const uint4*>(qrow + ch * 16);
-                const uint4 kv = *reinterpret_cast<const uint4*>(krow + ch * 16);
-                const __half2* qh = reinterpret_cast<const __half2*>(&qv);
-                const __half2* kh = reinterpret_cast<const __half2*>(&kv);
-#pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float2 a = __half22float2(qh[e]), b = __half22float2(kh[e]);
-                  sc = fmaf(a.x, b.x, fmaf(a.y, b.y, sc));
-                }
-              }
-              sc = fmaf(sc, rsqrtf((float)DH) * 1.4426950408889634f, kb_row);      // -inf past the last key
-              const float mx = warp_max(sc);
-              const float pj = ex2_approx(sc - mx);
-              const float inv = rcp_approx(warp_sum(pj));
-              __half* orow = p.out + env * (int64_t)p.ldo + (g * G + hh) * DH;
-#pragma unroll
-              for (int dd = 0; dd < DH; dd += 32) {
-                const int col = dd + lane;
-                const uint8_t* vcol = rows_g + (2 * GD + hh * DH) * 2 + (col < DH ? col : 0) * 2;
-                float acc = 0.f;
-#pragma unroll 8
-                for (int j = 0; j < NKEYS; ++j)
-                  acc = fmaf(__shfl_sync(0xffffffffu, pj, j), __half2float(*reinterpret_cast<const __half*>(vcol + j * LDQ)), acc);
-                if (col < DH) orow[col] = __float2half_rn(acc * inv);
-              }
+              attend_one_row<DH, LDQ, NKEYS>(sQ_g + (env_l * EROWS) * LDQ, p.q_first, hh * DH, GD, kb_row,
+                                             p.out + env * (int64_t)p.ldo + (g * G + hh) * DH, lane);
             }
           } else {
             if (G == 2 && n_q > 16) attend_pair<2, DH, LDQ, GD * 2>(sq_pair, sk_pair, sv_pair, kb, n_q, out_pair, p.ldo, lane, so_tile, env_l * EROWS + mt_own * 16, hh * (DH / 8));

@@ -12,7 +12,7 @@
 //
 // Reference call sites: fp16_linear / fp16_linear_relu / fp16_packed_linear (python/fp16_linear.py:506-517, :633-641,
 // :794-805).
-#include "kernels.cuh"
+#include "row_norm.cuh"
 
 namespace bsrl {
 
@@ -25,16 +25,29 @@ __device__ __forceinline__ uint32_t piece_off(int row, int kc) {
   return static_cast<uint32_t>(row * ROW_BYTES + ((kc ^ (row & 7)) << 4));
 }
 
+struct SmallArgs {
+  LinearArgs p[2];           // the second one is optional: blocks from tiles0 on
+  int tiles0, stages[2];
+  int start;                 // linear_small_block
+  RowNorm norm;
+};
+
 // TM x TN output tile, one warp per 16 x 8 piece of it (a dependent chain of MMAs: 25 cycles per K step of 16)
-template <int TM, int TN>
-__global__ void __launch_bounds__(TM * TN / 4) linear_small_kernel(LinearArgs p, int n_tiles, int stages) {
+// NORM: the A operand is the LayerNorm of fp32 rows, made in shared memory (every column tile's CTA makes its own; all of
+// K is resident)
+template <int TM, int TN, bool NORM>
+__global__ void __launch_bounds__(TM * TN / 4) linear_small_kernel(const __grid_constant__ SmallArgs args) {
   constexpr int THREADS = TM * TN / 4, STAGE_BYTES = (TM + TN) * ROW_BYTES;
   extern __shared__ __align__(128) uint8_t smem[];
   const uint32_t base = smem_u32(smem);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp % (TM / 16), wn = warp / (TM / 16);
-  const int nt = (int)(blockIdx.x % (unsigned)n_tiles);
-  const int64_t m0 = (int64_t)(blockIdx.x / (unsigned)n_tiles) * TM;
+  const bool second = blockIdx.x >= (unsigned)args.tiles0;
+  const LinearArgs& p = args.p[second ? 1 : 0];
+  const int stages = args.stages[second ? 1 : 0], n_tiles = (p.N + TN - 1) / TN;
+  const unsigned tile = blockIdx.x - (second ? (unsigned)args.tiles0 : 0u);
+  const int nt = (int)(tile % (unsigned)n_tiles);
+  const int64_t m0 = (int64_t)(tile / (unsigned)n_tiles) * TM;
   const int n0 = nt * TN;
   const int chunks = (p.K + KC - 1) / KC;
 
@@ -66,16 +79,50 @@ __global__ void __launch_bounds__(TM * TN / 4) linear_small_kernel(LinearArgs p,
   const int ahead = chunks < stages ? chunks : stages;
   for (int c = 0; c < ahead; ++c) load_w(c, base + c * STAGE_BYTES);          // the weights are nobody's output
   pdl_begin();
-  for (int c = 0; c < ahead; ++c) {
+  if (NORM) {
+    const RowNorm& n = args.norm;
+    const int d = p.K, pitch = d + 4;
+    float* xs = reinterpret_cast<float*>(smem + stages * STAGE_BYTES);
+    float2* part = reinterpret_cast<float2*>(xs + TM * pitch);
+    for (int i = tid; i < TM * (d >> 2); i += THREADS) {
+      const int row = i / (d >> 2), c = (i - row * (d >> 2)) * 4;
+      const bool ok = m0 + row < p.M;
+      cp_async16(smem_u32(xs + row * pitch + c), ok ? n.x + n.map(m0 + row) * n.ldx + c : n.x, ok);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    row_norm_sums(xs, pitch, TM, d, n.quads != 0, part, tid);
+    __syncthreads();
+    for (int i = tid; i < TM * (d >> 3); i += THREADS) {
+      const int row = i / (d >> 3), c = (i - row * (d >> 3)) * 8;
+      *reinterpret_cast<uint4*>(smem + (c / KC) * STAGE_BYTES + piece_off(row, (c % KC) >> 3)) =
+          row_norm_piece(xs + row * pitch, c, part[row], part[TM + row], d, n);
+    }
+  }
+  for (int c = 0; c < ahead && !NORM; ++c) {
     load_a(c, base + c * STAGE_BYTES);
     cp_async_commit();                                // group c: the weights so far and rows' chunk c
   }
 
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  const int g = lane >> 2, tig = lane & 3, col = n0 + wn * 8 + tig * 2;
+  const float2 bias = p.bias && col < p.N ? make_float2(p.bias[col], p.bias[col + 1]) : make_float2(0.f, 0.f);
+  if (args.start && col < p.N) {                      // the sums start at the residual (+ bias)
+#pragma unroll
+    for (int hh = 0; hh < 2; ++hh) {
+      const int64_t gm = m0 + wm * 16 + g + hh * 8;
+      if (gm >= p.M) continue;
+      const float2 r = *reinterpret_cast<const float2*>(p.R + p.rmap(gm) * (int64_t)p.ldr + col);
+      acc[2 * hh] = args.start == 1 ? r.x + bias.x : r.x;
+      acc[2 * hh + 1] = args.start == 1 ? r.y + bias.y : r.y;
+    }
+  }
   for (int c = 0; c < chunks; ++c) {
     // chunk c's group is complete when at most the groups issued after it are in flight
     const int later = min(c + ahead, chunks) - 1 - c;
-    if (later >= 7) cp_async_wait<7>();
+    if (NORM) {}
+    else if (later >= 7) cp_async_wait<7>();
     else if (later == 6) cp_async_wait<6>();
     else if (later == 5) cp_async_wait<5>();
     else if (later == 4) cp_async_wait<4>();
@@ -105,19 +152,17 @@ __global__ void __launch_bounds__(TM * TN / 4) linear_small_kernel(LinearArgs p,
     }
   }
 
-  const int g = lane >> 2, tig = lane & 3;
+  if (col >= p.N) return;
 #pragma unroll
   for (int hh = 0; hh < 2; ++hh) {
     const int64_t gm = m0 + wm * 16 + g + hh * 8;
     if (gm >= p.M) continue;
     const int64_t crow = p.cmap(gm) * (int64_t)p.ldc;
-    const float* rrow = p.R ? p.R + p.rmap(gm) * (int64_t)p.ldr : nullptr;
-    const int col = n0 + wn * 8 + tig * 2;
-    if (col >= p.N) continue;
+    const float* rrow = p.R && !args.start ? p.R + p.rmap(gm) * (int64_t)p.ldr : nullptr;
     float v0 = acc[hh * 2], v1 = acc[hh * 2 + 1];
-    if (p.bias) {
-      v0 += p.bias[col];
-      v1 += p.bias[col + 1];
+    if (p.bias && args.start != 1) {
+      v0 += bias.x;
+      v1 += bias.y;
     }
     if (p.relu == 1) {
       v0 = fmaxf(v0, 0.f);
@@ -145,22 +190,34 @@ struct Tile {
     return chunks < MAX_STAGES ? chunks : MAX_STAGES;
   }
   static int64_t tiles(const LinearArgs& p) { return (p.M + TM - 1) / TM * ((p.N + TN - 1) / TN); }
-  static bool one_wave(const LinearArgs& p) {         // every tile has a place on the chip at once
-    const int by_smem = 227 * 1024 / (stages(p) * STAGE_BYTES + 1024), by_threads = 2048 / THREADS;
+  static int norm_bytes(int d) { return TM * (d + 4) * 4 + 2 * TM * 8; }
+  static bool one_wave(const LinearArgs& p, bool norm = false) {      // every tile has a place on the chip at once
+    const int by_smem = 227 * 1024 / (stages(p) * STAGE_BYTES + (norm ? norm_bytes(p.K) : 0) + 1024), by_threads = 2048 / THREADS;
     return tiles(p) <= (int64_t)sm_count() * (by_smem < by_threads ? by_smem : by_threads);
   }
-  static int run(const LinearArgs& p, cudaStream_t stream) {
+  static int run(SmallArgs& a, bool two, bool norm, cudaStream_t stream) {
     static DeviceOnce once;
     int rc = once.run("linear_small_kernel set-up", [] {
-      return cudaFuncSetAttribute(linear_small_kernel<TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_STAGES * STAGE_BYTES);
+      cudaError_t e = cudaFuncSetAttribute(linear_small_kernel<TM, TN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_STAGES * STAGE_BYTES);
+      return e != cudaSuccess ? e : cudaFuncSetAttribute(linear_small_kernel<TM, TN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                         2 * STAGE_BYTES + norm_bytes(2 * KC));
     });
     if (rc != BSRL_OK) return rc;
-    launch_kernel(linear_small_kernel<TM, TN>, static_cast<unsigned>(tiles(p)), THREADS, (size_t)stages(p) * STAGE_BYTES, stream, p,
-                  (p.N + TN - 1) / TN, stages(p));
+    a.tiles0 = (int)tiles(a.p[0]);
+    a.stages[0] = stages(a.p[0]);
+    a.stages[1] = two ? stages(a.p[1]) : 0;
+    const unsigned blocks = (unsigned)(a.tiles0 + (two ? tiles(a.p[1]) : 0));
+    const size_t smem = (size_t)(a.stages[0] > a.stages[1] ? a.stages[0] : a.stages[1]) * STAGE_BYTES + (norm ? norm_bytes(a.p[0].K) : 0);
+    if (norm) launch_kernel(linear_small_kernel<TM, TN, true>, blocks, THREADS, smem, stream, a);
+    else launch_kernel(linear_small_kernel<TM, TN, false>, blocks, THREADS, smem, stream, a);
     BSRL_LAUNCH_OK("linear_small_kernel");
     return BSRL_OK;
   }
 };
+int refuse(const LinearArgs& p) {
+  set_error("linear_small: shape m=%lld n=%d k=%d or its alignment is not supported", (long long)p.M, p.N, p.K);
+  return BSRL_ERR_UNSUPPORTED;
+}
 }  // namespace
 
 bool linear_small_ok(const LinearArgs& p) {
@@ -168,7 +225,7 @@ bool linear_small_ok(const LinearArgs& p) {
   if (p.N % 8 || p.K % 8 || p.N < 8 || p.K < 8) return false;
   if (!aligned16(p.A) || !aligned16(p.W) || (p.lda % 8) || (p.ldw % 8) || (reinterpret_cast<uintptr_t>(p.C) & 7) || (p.ldc % 2)) return false;
   if (p.R && ((p.ldr % 2) || (reinterpret_cast<uintptr_t>(p.R) & 7))) return false;
-  return Tile<16, 32>::tiles(p) <= 0x7fffffff;
+  return Tile<16, 32>::tiles(p) <= 0x3fffffff;
 }
 
 // Where it is the faster one: below the tcgen05 kernel's 128 rows always, above as long as all tiles run at once (256 x
@@ -179,11 +236,43 @@ bool linear_small_wins(const LinearArgs& p) {
 }
 
 int linear_small(const LinearArgs& p, cudaStream_t stream) {
-  if (!linear_small_ok(p)) {
-    set_error("linear_small: shape m=%lld n=%d k=%d or its alignment is not supported", (long long)p.M, p.N, p.K);
-    return BSRL_ERR_UNSUPPORTED;
+  if (!linear_small_ok(p)) return refuse(p);
+  SmallArgs a{};
+  a.p[0] = p;
+  return Tile<16, 32>::one_wave(p) ? Tile<16, 32>::run(a, false, false, stream) : Tile<32, 32>::run(a, false, false, stream);
+}
+
+bool linear_small_two_wins(const LinearArgs& p, const LinearArgs& q) {       // both as one wave of the smallest tiles
+  using T = Tile<16, 32>;
+  if (!linear_small_ok(p) || !linear_small_ok(q)) return false;
+  const int stages = T::stages(p) > T::stages(q) ? T::stages(p) : T::stages(q);
+  const int by_smem = 227 * 1024 / (stages * T::STAGE_BYTES + 1024), by_threads = 2048 / T::THREADS;
+  return T::tiles(p) + T::tiles(q) <= (int64_t)sm_count() * (by_smem < by_threads ? by_smem : by_threads);
+}
+
+int linear_small_two(const LinearArgs& p, const LinearArgs& q, cudaStream_t stream) {
+  if (!linear_small_ok(p)) return refuse(p);
+  if (!linear_small_ok(q)) return refuse(q);
+  SmallArgs a{};
+  a.p[0] = p;
+  a.p[1] = q;
+  return Tile<16, 32>::run(a, true, false, stream);
+}
+
+int linear_small_block(const LinearArgs& p, int start, const RowNorm* norm, cudaStream_t stream) {
+  LinearArgs q = p;
+  if (norm) {
+    q.A = p.W;                                        // not read: the operand comes from norm->x
+    q.lda = p.ldw;
+    if (!norm->x || !norm->g || !norm->b || !aligned16(norm->x) || (norm->ldx % 4) || p.K % 64 || p.K > 2 * KC || p.K < 64) return refuse(p);
   }
-  return Tile<16, 32>::one_wave(p) ? Tile<16, 32>::run(p, stream) : Tile<32, 32>::run(p, stream);
+  if (!linear_small_ok(q) || (start && !p.R)) return refuse(p);
+  SmallArgs a{};
+  a.p[0] = q;
+  a.start = start;
+  if (norm) a.norm = *norm;
+  return Tile<16, 32>::one_wave(q, norm != nullptr) ? Tile<16, 32>::run(a, false, norm != nullptr, stream)
+                                                    : Tile<32, 32>::run(a, false, norm != nullptr, stream);
 }
 
 }  // namespace bsrl

@@ -59,6 +59,25 @@ bool linear_tc5_sums_ok(const LinearArgs& p);                // ... and its colu
 bool linear_res_ok(const LinearArgs& p);                     // linear_tc5's products with K <= 256 over many rows:
 int linear_res(const LinearArgs& p, cudaStream_t stream);    // ... weights resident in shared memory (gemm_res_tc5.cu)
 
+// LayerNorm of fp32 rows inside a kernel that takes them as its operand (row_norm.cuh): rows mapped by `map`; quads: the
+// statistics' grouping (the one of the LayerNorm rows a block hands to the next, else the one ahead of its FFN).
+struct RowNorm {
+  const float* x;
+  int64_t ldx;
+  RowMap map;
+  const float* g;
+  const float* b;
+  float eps;
+  int quads;
+};
+// Pieces of a transformer block for few rows, each with the arithmetic of the fused kernels' counterpart (bit for bit).
+// linear_small_block: start 1: the sums start at R + bias, start 2: at R, the bias comes last (0: as in linear_small);
+// with `norm` the A operand is the LayerNorm of those rows (K = d <= 256, a multiple of 64).  linear_small_two: two
+// independent products in one launch.
+int linear_small_block(const LinearArgs& p, int start, const RowNorm* norm, cudaStream_t stream);
+bool linear_small_two_wins(const LinearArgs& a, const LinearArgs& b);
+int linear_small_two(const LinearArgs& a, const LinearArgs& b, cudaStream_t stream);
+
 // Projection + residual + LayerNorm in one kernel (gemm_ln_tc5.cu): x_out = R + A W^T + bias (fp32), h =
 // LayerNorm(x_out) (fp16).  N a multiple of 64 up to 512 (of 128 above 256), K a multiple of 64.  R and x_out
 // may be the same buffer.
@@ -135,6 +154,26 @@ struct AttnBlockArgs {
   int body = 0, tokens = 29;
   const __half* qkv0 = nullptr;
 };
+// The same for few environments (attn_small.cu): one CTA per environment and head group, up to two problems over the
+// same environments in a launch.  The rows come as fp16 (h) or are LayerNormed from fp32 (norm.x set; dense rows).
+struct AttnSmallArgs {
+  int d;
+  const __half* h;
+  int ldh;
+  RowNorm norm;
+  const __half* wg;        // regrouped weight, bias, key bias, query rows and output as in AttnBlockArgs
+  const float* bg;
+  const float* key_bias;
+  int q_first, n_q;
+  __half* out;
+  int ldo;
+  __half* v_out;           // value residual, the first problem only
+  const __half* v0;
+  const float* vres;
+};
+bool attn_small_ok(const AttnSmallArgs& a, int n_heads, int64_t n_envs);
+int attn_small(const AttnSmallArgs* a, int n, int n_heads, int64_t n_envs, cudaStream_t stream);
+
 // v columns of a packed projection: copy out (v_out) and / or mix with v0 in place (value residual)
 int vres_mix(__half* v, int ld, int64_t rows, int d, __half* v_out, const __half* v0, const float* vres,
              cudaStream_t stream);

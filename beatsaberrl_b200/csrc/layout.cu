@@ -321,12 +321,17 @@ const Plan& plan_of(const bsrl_config& c) {
 }
 
 // ------------------------------------------------------------------ workspace
-Paths plan_paths(const Layout& l, int engine) {
+Paths plan_paths(const Layout& l, int engine, int64_t n_envs) {
   Paths p;
   const bool widths = engine == 0 && l.d % 64 == 0 && l.d >= 64 && l.d <= 256;
   p.attn_fused = engine == 0 && l.attn_G > 0;
   p.tail_fused = widths && l.F % 256 == 0 && l.F >= 256 && l.F <= 1024;
   p.enc_fused = widths && !l.emb_ln.width && l.note_k == 64;
+  // Few environments: the small-CTA launches, whose cost grows with the environments and the weights' size, against the
+  // fused kernels, which take the same time up to one tile per SM.  Forward behind a graph, small / fused us: d 64 at 64
+  // envs 68 / 70, at 128 74 / 70; d 128 at 64 84 / 90, at 96 98 / 90; d 192 at 1 151 / 230, at 24 223 / 239, at 48 284 /
+  // 240; d 256 at 1 124 / 204, at 16 168 / 206, at 32 229 / 209.
+  p.small = l.L >= 2 && p.attn_fused && p.tail_fused && p.enc_fused && !l.final_ln.width && n_envs <= 64 && n_envs * l.d * l.d <= 1 << 20;
   return p;
 }
 
@@ -347,7 +352,7 @@ Workspace make_workspace(const Layout& l, int64_t B, const Paths& paths) {
   w.h = cv.take(R * d * 2);
   w.qkv = paths.attn_fused ? -1 : cv.take(R * 3 * d * 2);
   w.att = cv.take(R * d * 2);
-  w.hid = paths.tail_fused ? -1 : cv.take(R * (int64_t)l.F * 2);
+  w.hid = paths.tail_fused && !paths.small ? -1 : cv.take(R * (int64_t)l.F * 2);
   w.x_lead = cv.take(Rl * d * 4);
   w.h_lead = cv.take(Rl * d * 2);
   w.lead16 = cv.take(Rl * d * 2);

@@ -94,8 +94,9 @@ struct Paths {
   bool attn_fused;   // q|k|v projection + attention in one kernel (no (rows, 3d) buffer)
   bool tail_fused;   // out-projection + LayerNorm + FFN in one kernel (no (rows, 4d) hidden buffer)
   bool enc_fused;    // both encoder layers + block 0's LayerNorm in one kernel
+  bool small;        // few environments: every block as four launches of many small CTAs
 };
-Paths plan_paths(const Layout& l, int engine);
+Paths plan_paths(const Layout& l, int engine, int64_t n_envs);
 
 // Workspace carve-up for a batch of n_envs (offsets of buffers the path does not use are -1).
 struct Workspace {

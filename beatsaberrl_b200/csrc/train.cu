@@ -787,7 +787,7 @@ int bsrl_backward(const bsrl_config* cfg, const void* arena, int64_t n_envs, con
   Ctx c;
   c.cfg = cfg;
   c.l = l;
-  c.paths = plan_paths(l, 1);       // the recomputation runs the separate GEMM / LayerNorm / attention kernels
+  c.paths = plan_paths(l, 1, n_envs);       // the recomputation runs the separate GEMM / LayerNorm / attention kernels
   use_process_engine();
   c.arena = arena;
   c.ws = workspace;

@@ -256,3 +256,18 @@ def test_full_size_properties():
     idx = torch.arange(0, B, 128, device="cuda")      # 1,024 envs spread over the batch
     ref_l, ref_v = po.forward_stacked(sd, cfg, obs[idx].cpu())
     assert_parity(logits[idx], value[idx], ref_l, ref_v, argmax_min=0.998)
+
+
+@pytest.mark.parametrize("name,geo,opts", [("cfg1", False, None), ("recipe", True, None), ("recipe", False, dict(value_residual=True)),
+                                           ("cfg2", False, None)])
+def test_few_envs_take_other_kernels_and_give_the_same_bits(name, geo, opts):
+    """Up to 16 (d 256) to 64 (d 128) environments run as many small launches, more as the fused tile kernels: an env's
+    logits and value are the same bits either way, on both sides of the line and with the value residual's extra reads."""
+    cfg = make_cfg(name, geo, opts=dict(opts or {}, n_blocks=3))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
+    obs = po.make_obs(130, 33, padded=True).cuda()
+    full_l, full_v = m.forward_stacked(obs)
+    for B in (1, 5, 16, 17, 28, 29, 64, 65):
+        l, v = m.forward_stacked(obs[:B])
+        assert torch.equal(l, full_l[:B]) and torch.equal(v, full_v[:B]), B
+    m.check_device()
