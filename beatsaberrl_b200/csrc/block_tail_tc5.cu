@@ -229,7 +229,10 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
-  if (warp != 0) pdl_begin();    // the weight producer depends on no earlier kernel
+  // The weight producer depends on no earlier kernel.  The epilogue warps' first work, the residual rows, is the output
+  // of a kernel at least two launches back (between two block tails runs at least the attention), which has completed by
+  // the time this one may start: they wait after it.
+  if (warp == 1 || warp == PROD_WARP) pdl_begin();
   const int rows_d = d;          // weight rows of an N = d tile
   const int rows_h = HC;         // ... of an N = 128 tile
 
@@ -684,6 +687,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
       ok = prestore(tile0, 0u);
       signal(&sh->x_ready);
     }
+    pdl_wait();
     for (int t = tile0; t < t_end && ok; t += tstep, ++tile_i) {
       const uint32_t par = tile_i & 1;
       const uint32_t xcol = par ? 256u : 0u, acol = par ? 0u : 256u;
