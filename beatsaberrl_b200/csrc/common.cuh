@@ -111,18 +111,27 @@ inline void pdl_enable() { g_pdl = true; }
 struct PdlScope {
   ~PdlScope() { g_pdl = false; }
 };
-template <typename... P, typename... A>
+template <int CLUSTER = 1, typename... P, typename... A>
 inline void launch_kernel(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr;
-  cfg.numAttrs = g_pdl ? 1 : 0;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (g_pdl) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (CLUSTER > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = CLUSTER;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
   (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);     // BSRL_LAUNCH_OK follows every launch
 }
 

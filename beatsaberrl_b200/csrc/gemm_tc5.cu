@@ -529,6 +529,7 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
     return BSRL_ERR_UNSUPPORTED;
   }
   if (linear_res_ok(p)) return linear_res(p, stream);
+  if (linear_pair_ok(p)) return linear_pair(p, stream);
   if (p.bits_in || p.bits_out) {
     set_error("linear: ReLU bits need the resident-weight kernel (m=%lld n=%d k=%d)", (long long)p.M, p.N, p.K);
     return BSRL_ERR_UNSUPPORTED;

@@ -56,6 +56,8 @@ int linear_small(const LinearArgs& p, cudaStream_t stream);
 int linear_tc5(const LinearArgs& p, cudaStream_t stream);   // tcgen05 / TMEM engine
 bool linear_tc5_ok(const LinearArgs& p);                     // shape fits the tcgen05 engine
 bool linear_tc5_sums_ok(const LinearArgs& p);                // ... and its column sums can ride along (a_sums)
+bool linear_pair_ok(const LinearArgs& p);                    // ... with K > 256 and whole 256-column tiles:
+int linear_pair(const LinearArgs& p, cudaStream_t stream);   // ... CTA pairs (gemm_pair_tc5.cu)
 bool linear_res_ok(const LinearArgs& p);                     // linear_tc5's products with K <= 256 over many rows:
 int linear_res(const LinearArgs& p, cudaStream_t stream);    // ... weights resident in shared memory (gemm_res_tc5.cu)
 

@@ -395,3 +395,30 @@ def test_linear_small_tiles(native, m, n, k, relu, resid, f32):
     ref = ref.relu() if relu == 1 else F.gelu(ref) if relu == 2 else ref
     ref = ref + r if resid else ref
     torch.testing.assert_close(outs[1].float(), ref, **(dict(atol=2e-4, rtol=1e-4) if f32 else dict(atol=4e-3, rtol=1e-3)))
+
+
+@pytest.mark.parametrize("m,n,k,relu,resid,f32", [
+    (18945, 512, 320, 1, 0, 0),         # the first size that takes CTA pairs; half a pair and one row in the last tile
+    (19021, 512, 576, 0, 1, 1), (37889, 256, 1024, 2, 0, 0), (12801, 768, 520, 0, 0, 1), (18999, 512, 512, 0, 1, 0),
+])
+def test_linear_cta_pairs(native, m, n, k, relu, resid, f32):
+    """Large products with K > 256 on CTA pairs, K and rows with remainders, against float64 products of the same fp16
+    operands: fp32 sums of k products of size ~1 / sqrt(k) (k 2^-24 at worst) and one fp16 rounding."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn(m, k, generator=g, device="cuda").half()
+    w = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).half()
+    b = torch.randn(n, generator=g, device="cuda")
+    r = torch.randn(m, n, generator=g, device="cuda") if resid else None
+    out = torch.full((m, n), float("nan"), dtype=torch.float32 if f32 else torch.float16, device="cuda")
+    rc = native.lib.bsrl_linear(a.data_ptr(), w.data_ptr(), b.data_ptr(), r.data_ptr() if resid else None, out.data_ptr(),
+                                f32, relu, m, n, k, 1, _stream())
+    if k % 64:
+        assert rc != 0                  # K in whole k-blocks where the rows of both operands are contiguous
+        return
+    native.check(rc)
+    native.check(native.lib.bsrl_device_status())
+    ref = a.double() @ w.double().t() + b.double()
+    ref = ref.clamp_min(0) if relu == 1 else F.gelu(ref) if relu == 2 else ref
+    ref = ref + r.double() if resid else ref
+    tol = 4e-5 if f32 else 2 ** -11
+    assert bool(((out.double() - ref).abs() <= tol * ref.abs() + 4e-5).all())
