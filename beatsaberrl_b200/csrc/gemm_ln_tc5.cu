@@ -4,22 +4,26 @@
 //   x_out = R + A W^T + b        (fp32 residual stream, N = d columns)
 //   h     = LayerNorm(x_out)     (fp16 rows: the operand of the GEMM that follows)
 //
-// A 128-row tile of a 512-wide fp32 row fills all 512 TMEM columns, so there is no second accumulator
-// buffer: the MMAs of a tile and its epilogue run one after the other, and the epilogue is what the kernel
-// is made of -- it moves 5 KB per row (residual in, stream out, LayerNorm row out) against 2 N K FLOP, i.e.
-// the kernel is HBM-bound for K = d and only worth having there.  What it saves is the separate LayerNorm
-// pass (2 KB read + 1 KB written per row again) and the slower residual epilogue of the plain GEMM.
+// Rows wider than 256 are shared by a cluster of two CTAs, each with half of the columns: a 128 x 256 accumulator
+// leaves room in TMEM for a second one, so that a tile's MMAs run beside the previous tile's epilogue.  The two swap
+// their row sums through distributed shared memory, counted in bytes on an mbarrier of the receiver (a release at
+// cluster scope costs ~3,000 cycles, the counted store none).  The kernel moves 5 KB per 512-wide row against 2 N K
+// FLOP: for K = d it is bound by HBM and by the epilogue that feeds it.  The shared memory goes there: two 48 KB operand
+// stages are enough for K = d, and every epilogue warp has three 4 KB row buffers, through which the residual arrives
+// and the sum leaves by TMA.  N = K = 512, 950 K rows: one CTA with all 512 columns, MMAs and epilogue in turn 1516 us;
+// cluster with row loads by the threads 1376; residual by TMA, two buffers and three stages 1290; this 1089 (5.4 TB/s;
+// 905 at copy speed).  N = K = 256: 921 -> 569 us.
 //
-//   warp 0      TMA producer: stages of a (128 x 64) A chunk + the (N x 64) weight chunk, 2 stages
-//   warp 1      MMA issuer: per 16-wide K step two tcgen05.mma (M = 128, N = 256) into the two column halves
-//   warps 2..9  epilogue; warp w reads TMEM lane quadrant w & 3 and owns column half (w - 2) / 4:
-//     pass 1    32 columns at a time: accumulator + bias, transposed through a 4 KB staging block so that the
-//               residual is read and the stream written with 8 lanes per 128-byte line; row sums of x and
-//               x^2 on the way; x goes back into TMEM for pass 2
-//     exchange  the two warps that share a quadrant swap their half-row sums (a 64-thread named barrier)
-//     pass 2    64 columns at a time: TMEM -> (x - mean) rstd gamma + beta -> fp16 -> staging -> one TMA store
+//   warp 0      TMA producer: stages of a (128 x 64) A chunk + this CTA's (N_cta x 64) weight chunk
+//   warp 1      MMA issuer
+//   warps 2..9  epilogue, thread = row; warp w reads TMEM lane quadrant w & 3 and owns column half (w - 2) / 4:
+//     pass 1    32 columns at a time: residual block in a row buffer + accumulator + bias -> stream rows, in place and
+//               out by TMA; row sums of x and x^2; x back into TMEM.  The block after the next is requested meanwhile
+//               and the next tile's rows are pulled into L2
+//     exchange  partial sums of the row's two (CL = 1) or four (CL = 2) column ranges
+//     pass 2    TMEM -> (x - mean) rstd gamma + beta -> fp16 -> row buffer -> TMA store
 //
-// Statistics are fp32 sums of x and x^2 over pieces of 32 values, combined pairwise (lanes, then halves).
+// Statistics are fp32 sums of x and x^2.
 // Stands in for out_proj + ln_ffn.forward_add (python/policy.py:655-668; ln_fwd_add,
 // python/beat_arena_env/csrc/layer_norm.cu) where the fused block tail does not reach.  All waits are bounded.
 #include "kernels.cuh"
@@ -30,37 +34,36 @@ namespace {
 using namespace tc5;
 
 constexpr int BM = 128, BK = 64, STAGES = 2;
-constexpr int MAX_N = 512;
+constexpr int BUFS = 3;                          // row buffers per epilogue warp
+constexpr int MAX_N = 512, MAX_NC = 256;         // columns, columns per CTA
 constexpr int A_BYTES = BM * BK * 2;             // 16 KB
-constexpr int W_BYTES = MAX_N * BK * 2;          // 64 KB
+constexpr int W_BYTES = MAX_NC * BK * 2;         // 32 KB
 constexpr int STAGE_BYTES = A_BYTES + W_BYTES;
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = (2 + EPI_WARPS) * 32;
-constexpr int STG_BYTES = 32 * 128;
-constexpr int PRM_BYTES = 3 * MAX_N * 4;         // bias | gamma | beta
-constexpr int PART_BYTES = 2 * BM * 8;           // per half and row: (sum, sum of squares)
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * STG_BYTES + PRM_BYTES + PART_BYTES + 1024 + 256;
+constexpr int STG_BYTES = 32 * 128;              // a row buffer: 32 rows x 32 fp32 or 64 fp16 columns
+constexpr int PRM_BYTES = 3 * MAX_NC * 4;        // bias | gamma | beta
+constexpr int PART_BYTES = 2 * 4 * BM * 8;       // per tile parity, column range and row: (sum, sum of squares)
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * BUFS * STG_BYTES + PRM_BYTES + PART_BYTES + 1024 + 512;
 constexpr int KERNEL_ID = 6;
 
 struct Shared {
-  uint64_t full[STAGES], empty[STAGES], acc_full, acc_empty, mma_done;
+  uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], stats[2], row_full[EPI_WARPS][BUFS], mma_done;
   uint32_t tmem_base;
   int abort;
-  int quit[4][2];   // abort as sampled by one thread of a quadrant's warp pair ahead of their barrier (per tile parity),
-                    // so that both warps leave the tile loop at the same tile
 };
+static_assert(sizeof(Shared) <= 512 && SMEM_BYTES <= 227 * 1024, "shared memory");
 
 struct Params {
-  int N, K;
+  int nc, K;          // columns per CTA
   int64_t M;
+  float inv_n;
   const float* bias;
   const float* gamma;
   const float* beta;
   float eps;
-  const float* R;     // (M, ldr) f32 residual
-  int64_t ldr;
-  float* x_out;       // (M, ldx) f32
-  int64_t ldx;
+  __half* h;
+  int64_t ldh;
   int n_tiles;
   int* status;
 };
@@ -70,25 +73,29 @@ __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
   sh->abort = 1;
 }
 
-// 16-byte global load that stays where it is written (the compiler may not sink it to its first use)
-__device__ __forceinline__ float4 ld_f4_here(const float* p) {
-  float4 v;
-  asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
-  return v;
+// eight bytes into the peer's shared memory, counted on the peer's barrier
+__device__ __forceinline__ void st_async_f2(uint32_t cluster_addr, float2 v, uint32_t cluster_bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [%0], {%1, %2}, [%3];" ::"r"(cluster_addr), "f"(v.x),
+               "f"(v.y), "r"(cluster_bar)
+               : "memory");
 }
 
+template <int CL>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
+                 const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_x,
                  const __grid_constant__ CUtensorMap tm_h, Params p) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t ring = (raw + 1023u) & ~1023u;
   uint8_t* staging = smem_raw + (ring - raw) + STAGES * STAGE_BYTES;
-  float* prm = reinterpret_cast<float*>(staging + EPI_WARPS * STG_BYTES);
-  float2* part = reinterpret_cast<float2*>(staging + EPI_WARPS * STG_BYTES + PRM_BYTES);
-  Shared* sh = reinterpret_cast<Shared*>(staging + EPI_WARPS * STG_BYTES + PRM_BYTES + PART_BYTES);
+  float* prm = reinterpret_cast<float*>(staging + EPI_WARPS * BUFS * STG_BYTES);
+  float2* part = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(prm) + PRM_BYTES);
+  Shared* sh = reinterpret_cast<Shared*>(reinterpret_cast<uint8_t*>(part) + PART_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int N = p.N, k_blocks = p.K / BK, n_halves = N > 256 ? 2 : 1, NH = N / n_halves;   // NH: columns per half
+  const uint32_t rank = CL == 2 ? cluster_rank() : 0u;
+  const int nc = p.nc, col_cta = (int)rank * nc, k_blocks = p.K / BK;
+  const int t0 = (int)(blockIdx.x / CL), t_step = (int)(gridDim.x / CL);
   volatile int* abort = &sh->abort;
 
   if (threadIdx.x == 0) {
@@ -96,38 +103,45 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       mbar_init(smem_u32(&sh->full[s]), 1);
       mbar_init(smem_u32(&sh->empty[s]), 1);
     }
-    mbar_init(smem_u32(&sh->acc_full), 1);
-    mbar_init(smem_u32(&sh->acc_empty), EPI_WARPS);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(smem_u32(&sh->acc_full[b]), 1);
+      mbar_init(smem_u32(&sh->acc_empty[b]), EPI_WARPS);
+      mbar_init(smem_u32(&sh->stats[b]), EPI_WARPS);
+    }
+    for (int w = 0; w < EPI_WARPS; ++w)
+      for (int b = 0; b < BUFS; ++b) mbar_init(smem_u32(&sh->row_full[w][b]), 1);
     mbar_init(smem_u32(&sh->mma_done), 1);
     sh->abort = 0;
-    for (int i = 0; i < 8; ++i) (&sh->quit[0][0])[i] = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tm_a);
     tma_prefetch_desc(&tm_w);
+    tma_prefetch_desc(&tm_r);
+    tma_prefetch_desc(&tm_x);
     tma_prefetch_desc(&tm_h);
   }
   if (warp == 1) {
     tmem_alloc(smem_u32(&sh->tmem_base), 512);
     tmem_relinquish();
   }
-  for (int i = threadIdx.x; i < N; i += THREADS) {
-    prm[i] = p.bias ? p.bias[i] : 0.f;
-    prm[MAX_N + i] = p.gamma[i];
-    prm[2 * MAX_N + i] = p.beta[i];
+  for (int i = threadIdx.x; i < nc; i += THREADS) {
+    prm[i] = p.bias ? p.bias[col_cta + i] : 0.f;
+    prm[MAX_NC + i] = p.gamma[col_cta + i];
+    prm[2 * MAX_NC + i] = p.beta[col_cta + i];
   }
   tc_fence_before();
   __syncthreads();
+  if (CL == 2) cluster_sync_all();          // the peer's barriers exist before anything is counted on them
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
   pdl_begin();
-  const uint32_t stage_tx = (uint32_t)(A_BYTES + N * BK * 2);
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
     if (lane == 0) {
+      const uint32_t stage_tx = (uint32_t)(A_BYTES + nc * BK * 2);
       uint32_t it = 0;
       bool ok = true;
-      for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
+      for (int t = t0; t < p.n_tiles && ok; t += t_step) {
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(smem_u32(&sh->empty[s]), ((it / STAGES) & 1) ^ 1, abort)) { give_up(sh, p.status, 1); ok = false; break; }
@@ -135,7 +149,7 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           mbar_expect_tx(bar, stage_tx);
           const uint32_t dst = ring + s * STAGE_BYTES;
           tma_load_2d(dst, &tm_a, kb * BK, t * BM, bar);
-          for (int hf = 0; hf < n_halves; ++hf) tma_load_2d(dst + A_BYTES + hf * NH * BK * 2, &tm_w, kb * BK, hf * NH, bar);
+          tma_load_2d(dst + A_BYTES, &tm_w, kb * BK, col_cta, bar);
         }
       }
       for (uint32_t j = it > STAGES ? it - STAGES : 0; j < it; ++j) {   // loads in flight land before the CTA exits
@@ -149,24 +163,22 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     if (lane == 0) {
       uint32_t it = 0, tile_i = 0;
       bool ok = true;
-      const uint32_t idesc = idesc_f16(BM, NH);
-      for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, ++tile_i) {
-        if (!mbar_wait(smem_u32(&sh->acc_empty), (tile_i & 1) ^ 1, abort)) { give_up(sh, p.status, 3); ok = false; break; }
+      const uint32_t idesc = idesc_f16(BM, nc);
+      for (int t = t0; t < p.n_tiles && ok; t += t_step, ++tile_i) {
+        const int buf = tile_i & 1;
+        if (!mbar_wait(smem_u32(&sh->acc_empty[buf]), ((tile_i >> 1) & 1) ^ 1, abort)) { give_up(sh, p.status, 3); ok = false; break; }
         tc_fence_after();
+        const uint32_t d_tmem = tmem_base + buf * MAX_NC;
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(smem_u32(&sh->full[s]), (it / STAGES) & 1, abort)) { give_up(sh, p.status, 4); ok = false; break; }
           tc_fence_after();
-          const uint32_t a_addr = ring + s * STAGE_BYTES;
-          const uint64_t ad = smem_desc_sw128(a_addr);
+          const uint64_t ad = smem_desc_sw128(ring + s * STAGE_BYTES), wd = smem_desc_sw128(ring + s * STAGE_BYTES + A_BYTES);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k)
-            for (int hf = 0; hf < n_halves; ++hf)
-              mma_f16_ss(tmem_base + hf * 256, ad + 2 * k, smem_desc_sw128(a_addr + A_BYTES + hf * NH * BK * 2) + 2 * k, idesc,
-                         (kb | k) ? 1u : 0u);
+          for (int k = 0; k < BK / 16; ++k) mma_f16_ss(d_tmem, ad + 2 * k, wd + 2 * k, idesc, (kb | k) != 0);
           tc_commit(smem_u32(&sh->empty[s]));
         }
-        if (ok) tc_commit(smem_u32(&sh->acc_full));
+        if (ok) tc_commit(smem_u32(&sh->acc_full[buf]));
       }
       tc_commit(smem_u32(&sh->mma_done));
       uint32_t spins = 0;
@@ -176,146 +188,165 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   } else {
     // ---------------------------------------------------------------- epilogue warps
     const int q = warp & 3, half = (warp - 2) >> 2;
-    const bool active = half < n_halves;                 // N <= 256: the second group of warps only keeps the barriers company
-    uint8_t* stg = staging + (warp - 2) * STG_BYTES;
-    const int sub = lane >> 3, piece = lane & 7;
-    const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + half * 256;
-    const int col0 = half * NH;
-    const float inv_n = 1.f / (float)N;
+    const int hc = nc >> 1, lo = half * hc;                  // this warp's columns [lo, lo + hc) of the CTA's
+    const int trow = q * 32 + lane;
+    uint8_t* const bufs = staging + (warp - 2) * (BUFS * STG_BYTES);
+    uint64_t* const row_full = sh->row_full[warp - 2];
+    // A tile takes nx + nh row buffers in turn: nx blocks of the stream (the residual arrives in the buffer, the sum
+    // leaves from it), then nh of h.  The residual of the block BUFS - 1 places on is requested once the buffer it
+    // takes has been stored.
+    const int nx = hc >> 5, nh = hc >> 6, n_use = nx + nh;
+    int use_b = 0, ask_b = 0, ask_pos = 0, ask_t = t0;
+    uint32_t parity = 0, pending = 0;                        // bit b: buffer b's next phase; a load is on its way to it
+    auto ask = [&]() {
+      if (ask_t < p.n_tiles && ask_pos < nx) {
+        pending |= 1u << ask_b;
+        if (lane == 0) {
+          const uint32_t bar = smem_u32(row_full + ask_b);
+          mbar_expect_tx(bar, STG_BYTES);
+          tma_load_2d(smem_u32(bufs + ask_b * STG_BYTES), &tm_r, col_cta + lo + ask_pos * 32, ask_t * BM + q * 32, bar);
+        }
+      }
+      ask_b = ask_b + 1 == BUFS ? 0 : ask_b + 1;
+      if (++ask_pos == n_use) {
+        ask_pos = 0;
+        ask_t += t_step;
+      }
+    };
+    auto free_and_ask = [&]() {                              // the store before this use has read its buffer
+      if (lane == 0) bulk_wait_read<0>();
+      __syncwarp();
+      ask();
+    };
+    auto emit = [&](const CUtensorMap* map, int x, int64_t m0, const uint8_t* buf) {
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        if (m0 < p.M) tma_store_2d(map, x, (int)m0, smem_u32(buf));
+        bulk_commit();
+      }
+    };
+    for (int i = 0; i < BUFS - 1; ++i) ask();
     uint32_t tile_i = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, ++tile_i) {
-      const int64_t m0 = (int64_t)t * BM;
-      int64_t rrow[8];                                   // rows this lane touches in the transposed phase, or -1
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int64_t row = m0 + q * 32 + i * 4 + sub;
-        rrow[i] = row < p.M ? row : -1;
+    for (int t = t0; t < p.n_tiles && ok; t += t_step, ++tile_i) {
+      const int buf = tile_i & 1;
+      const int64_t m0 = (int64_t)t * BM + q * 32, row = m0 + lane;
+      const bool live = row < p.M;
+      if (lane == 0 && t + t_step < p.n_tiles)               // the next tile's residual rows into L2
+        for (int c = 0; c < hc; c += 32) tma_prefetch_2d(&tm_r, col_cta + lo + c, (t + t_step) * BM + q * 32);
+      if (!mbar_wait_warp(smem_u32(&sh->acc_full[buf]), (tile_i >> 1) & 1, abort)) {
+        if (lane == 0) give_up(sh, p.status, 5);
+        break;
       }
-      // a failed wait does not leave the loop here: the warp goes on (on garbage) to the pair barrier, where both
-      // warps of the quadrant take the same decision
-      if (!mbar_wait_warp(smem_u32(&sh->acc_full), tile_i & 1, abort) && lane == 0) give_up(sh, p.status, 5);
       tc_fence_after();
-      float s1[8], s2[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) s1[i] = s2[i] = 0.f;
-      // ---- pass 1: x = acc + bias + R, written out and kept in TMEM; row sums
-      if (active) {
-        // the residual pieces of a block are asked for one block ahead: read on demand they arrive at DRAM
-        // latency with one block's worth of loads in flight, and this loop is most of the kernel
-        float4 rv[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-          rv[i] = rrow[i] >= 0 ? ld_f4_here(p.R + rrow[i] * p.ldr + col0 + piece * 4) : make_float4(0.f, 0.f, 0.f, 0.f);
+      const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + buf * MAX_NC + lo;
+      // ---- pass 1
+      float sum = 0.f, sq = 0.f;
+      uint32_t r[32];
+      tmem_ld32(tbase, r);
 #pragma unroll 1
-        for (int c = 0; c < NH; c += 32) {
-          const int col = col0 + c, pc = col + piece * 4;
-          float4 rn[8];
-          if (c + 32 < NH) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              rn[i] = rrow[i] >= 0 ? ld_f4_here(p.R + rrow[i] * p.ldr + pc + 32) : make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-          uint32_t r[32];
-          tmem_ld32(tbase + c, r);
-          tmem_wait_ld();
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float4 bv = *reinterpret_cast<const float4*>(prm + col + 4 * j);
-            *reinterpret_cast<float4*>(stg + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                make_float4(__uint_as_float(r[4 * j]) + bv.x, __uint_as_float(r[4 * j + 1]) + bv.y,
-                            __uint_as_float(r[4 * j + 2]) + bv.z, __uint_as_float(r[4 * j + 3]) + bv.w);
-          }
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            const int rr = i * 4 + sub;
-            float4* sp = reinterpret_cast<float4*>(stg + rr * 128 + ((piece ^ (rr & 7)) << 4));
-            float4 f = *sp;
-            f.x += rv[i].x; f.y += rv[i].y; f.z += rv[i].z; f.w += rv[i].w;
-            *sp = f;
-            s1[i] += (f.x + f.y) + (f.z + f.w);
-            s2[i] += (f.x * f.x + f.y * f.y) + (f.z * f.z + f.w * f.w);
-            if (rrow[i] >= 0) *reinterpret_cast<float4*>(p.x_out + rrow[i] * p.ldx + pc) = f;
-          }
-          __syncwarp();
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float4 f = *reinterpret_cast<const float4*>(stg + lane * 128 + ((j ^ (lane & 7)) << 4));
-            r[4 * j] = __float_as_uint(f.x); r[4 * j + 1] = __float_as_uint(f.y);
-            r[4 * j + 2] = __float_as_uint(f.z); r[4 * j + 3] = __float_as_uint(f.w);
-          }
-          tmem_st32(tbase + c, r);
-          __syncwarp();
-#pragma unroll
-          for (int i = 0; i < 8; ++i) rv[i] = rn[i];
+      for (int c = 0; c < hc; c += 32) {
+        if (!mbar_wait_warp(smem_u32(row_full + use_b), (parity >> use_b) & 1, abort)) {
+          if (lane == 0) give_up(sh, p.status, 8);
+          ok = false;
+          break;
         }
-        tmem_wait_st();
-        // the 8 lanes of a row add up their pieces; lane piece 0 publishes the half-row sums
+        parity ^= 1u << use_b;
+        pending &= ~(1u << use_b);
+        uint8_t* stg = bufs + use_b * STG_BYTES;
+        tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-#pragma unroll
-          for (int o = 1; o < 8; o <<= 1) {
-            s1[i] += __shfl_xor_sync(0xffffffffu, s1[i], o);
-            s2[i] += __shfl_xor_sync(0xffffffffu, s2[i], o);
-          }
-          if (piece == 0) part[half * BM + q * 32 + i * 4 + sub] = make_float2(s1[i], s2[i]);
+        for (int j = 0; j < 8; ++j) {
+          float4* cell = reinterpret_cast<float4*>(stg + lane * 128 + ((j ^ (lane & 7)) << 4));
+          const float4 bv = *reinterpret_cast<const float4*>(prm + lo + c + 4 * j), rv = *cell;
+          const float v0 = (__uint_as_float(r[4 * j]) + bv.x) + rv.x, v1 = (__uint_as_float(r[4 * j + 1]) + bv.y) + rv.y;
+          const float v2 = (__uint_as_float(r[4 * j + 2]) + bv.z) + rv.z, v3 = (__uint_as_float(r[4 * j + 3]) + bv.w) + rv.w;
+          sum += (v0 + v1) + (v2 + v3);
+          sq += (v0 * v0 + v1 * v1) + (v2 * v2 + v3 * v3);
+          r[4 * j] = __float_as_uint(v0); r[4 * j + 1] = __float_as_uint(v1);
+          r[4 * j + 2] = __float_as_uint(v2); r[4 * j + 3] = __float_as_uint(v3);
+          *cell = make_float4(v0, v1, v2, v3);
         }
+        tmem_st32(tbase + c, r);
+        if (c + 32 < hc) tmem_ld32(tbase + c + 32, r);
+        free_and_ask();
+        emit(&tm_x, col_cta + lo + c, m0, stg);
+        use_b = use_b + 1 == BUFS ? 0 : use_b + 1;
       }
-      if (half == 0 && lane == 0) sh->quit[q][tile_i & 1] = *abort;
-      asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory");        // the quadrant's two warps: half-row sums are in
-      const bool quit = *reinterpret_cast<volatile int*>(&sh->quit[q][tile_i & 1]) != 0;
-      // ---- pass 2: thread = row again: normalise, fp16, 64 columns per TMA store
-      if (active && !quit) {
-        const int trow = q * 32 + lane;
-        float2 a = part[trow];
-        if (n_halves == 2) {
-          const float2 b = part[BM + trow];
-          a.x += b.x; a.y += b.y;
-        }
-        const float mean = a.x * inv_n;
-        const float rstd = rsqrtf(fmaxf(a.y * inv_n - mean * mean, 0.f) + p.eps);
+      if (!ok) break;
+      tmem_wait_st();
+      // ---- exchange: the row's partial sums, in column order
+      float2* pt = part + buf * (4 * BM);
+      const int mine = (int)rank * 2 + half;
+      pt[mine * BM + trow] = make_float2(sum, sq);
+      if (CL == 2)
+        st_async_f2(map_to_cta(smem_u32(pt + mine * BM + trow), rank ^ 1), make_float2(sum, sq), map_to_cta(smem_u32(&sh->stats[buf]), rank ^ 1));
+      __syncwarp();
+      if (lane == 0) {
+        if (CL == 2) mbar_expect_tx(smem_u32(&sh->stats[buf]), 32 * 8);      // what the peer's warp of this place sends
+        else mbar_arrive(smem_u32(&sh->stats[buf]));
+      }
+      if (!mbar_wait_warp(smem_u32(&sh->stats[buf]), (tile_i >> 1) & 1, abort)) {
+        if (lane == 0) give_up(sh, p.status, 7);
+        break;
+      }
+      float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+      for (int i = 0; i < 2 * CL; ++i) {
+        const float2 o = pt[i * BM + trow];
+        s.x += o.x;
+        s.y += o.y;
+      }
+      const float mean = s.x * p.inv_n, rstd = rsqrtf(fmaxf(s.y * p.inv_n - mean * mean, 0.f) + p.eps);
+      // ---- pass 2: 64 columns (128 bytes of fp16) per store; a last block of 32 goes out directly
+      tmem_ld32(tbase, r);
 #pragma unroll 1
-        for (int c = 0; c < NH; c += 64) {
-          const int col = col0 + c;
-          uint32_t r[32];
-          if (c > 0) {                      // the previous block's TMA store has read the staging buffer
-            if (lane == 0) bulk_wait_read<0>();
-            __syncwarp();
-          }
+      for (int c = 0; c < hc; c += 32) {
+        tmem_wait_ld();
+        uint4 y[4];
 #pragma unroll
-          for (int s32 = 0; s32 < 64; s32 += 32) {
-            tmem_ld32(tbase + c + s32, r);
-            tmem_wait_ld();
-            float v[32];
+        for (int j = 0; j < 4; ++j) {
+          float v[8];
 #pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              const float4 g = *reinterpret_cast<const float4*>(prm + MAX_N + col + s32 + j);
-              const float4 b = *reinterpret_cast<const float4*>(prm + 2 * MAX_N + col + s32 + j);
-              v[j] = (__uint_as_float(r[j]) - mean) * rstd * g.x + b.x;
-              v[j + 1] = (__uint_as_float(r[j + 1]) - mean) * rstd * g.y + b.y;
-              v[j + 2] = (__uint_as_float(r[j + 2]) - mean) * rstd * g.z + b.z;
-              v[j + 3] = (__uint_as_float(r[j + 3]) - mean) * rstd * g.w + b.w;
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              *reinterpret_cast<uint4*>(stg + lane * 128 + ((((s32 >> 3) + j) ^ (lane & 7)) << 4)) =
-                  make_uint4(pack_half2(v[8 * j], v[8 * j + 1]), pack_half2(v[8 * j + 2], v[8 * j + 3]),
-                             pack_half2(v[8 * j + 4], v[8 * j + 5]), pack_half2(v[8 * j + 6], v[8 * j + 7]));
+          for (int e = 0; e < 2; ++e) {
+            const float4 g = *reinterpret_cast<const float4*>(prm + MAX_NC + lo + c + 8 * j + 4 * e);
+            const float4 b = *reinterpret_cast<const float4*>(prm + 2 * MAX_NC + lo + c + 8 * j + 4 * e);
+            const uint32_t* a = r + 8 * j + 4 * e;
+            v[4 * e] = (__uint_as_float(a[0]) - mean) * rstd * g.x + b.x;
+            v[4 * e + 1] = (__uint_as_float(a[1]) - mean) * rstd * g.y + b.y;
+            v[4 * e + 2] = (__uint_as_float(a[2]) - mean) * rstd * g.z + b.z;
+            v[4 * e + 3] = (__uint_as_float(a[3]) - mean) * rstd * g.w + b.w;
           }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0 && m0 + q * 32 < p.M) {
-            tma_store_2d(&tm_h, col, (int)(m0 + q * 32), smem_u32(stg));
-            bulk_commit();
-          }
+          y[j] = make_uint4(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
         }
-        if (lane == 0) bulk_wait_read<0>();    // pass 1 of the next tile writes the staging buffer with plain stores
+        if (c + 32 < hc) tmem_ld32(tbase + c + 32, r);
+        const int hb = (c >> 5) & 1;
+        if (!hb && c + 64 > hc) {                            // the odd last block (row widths that are not multiples of 256)
+          if (live) {
+            uint4* dst = reinterpret_cast<uint4*>(p.h + row * p.ldh + col_cta + lo + c);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) dst[j] = y[j];
+          }
+          continue;
+        }
+        if (!hb) free_and_ask();
+        uint8_t* stg = bufs + use_b * STG_BYTES;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(stg + lane * 128 + (((4 * hb + j) ^ (lane & 7)) << 4)) = y[j];
+        if (hb) {
+          emit(&tm_h, col_cta + lo + c - 32, m0, stg);
+          use_b = use_b + 1 == BUFS ? 0 : use_b + 1;
+        }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sh->acc_empty));
-      if (quit) ok = false;
+      if (lane == 0) mbar_arrive(smem_u32(&sh->acc_empty[buf]));
+    }
+    for (int b = 0; b < BUFS; ++b) {                         // after a wait that ran out: loads in flight land first
+      uint32_t spins = 0;
+      if ((pending >> b) & 1)
+        while (!mbar_try_wait(smem_u32(row_full + b), (parity >> b) & 1) && ++spins < kSpinLimit) {}
     }
     if (lane == 0) bulk_wait_all();
   }
@@ -323,6 +354,7 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
+  if (CL == 2) cluster_sync_all();          // the peer's sums land in this CTA's shared memory
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 512);
@@ -347,24 +379,28 @@ int linear_ln(const LinearLnArgs& a, cudaStream_t stream) {
   }
   int* status = device_status_ptr();
   if (!status) return BSRL_ERR_CUDA;
-  const int NH = a.N > 256 ? a.N / 2 : a.N;
-  CUtensorMap tm_a, tm_w, tm_h;
+  const int cl = a.N > MAX_NC ? 2 : 1, nc = a.N / cl;
+  CUtensorMap tm_a, tm_w, tm_r, tm_x, tm_h;
   if (!make_tmap_f16(&tm_a, a.A, a.M, a.K, a.lda, BM)) return BSRL_ERR_CUDA;
-  if (!make_tmap_f16(&tm_w, a.W, a.N, a.K, a.ldw, NH)) return BSRL_ERR_CUDA;
+  if (!make_tmap_f16(&tm_w, a.W, a.N, a.K, a.ldw, nc)) return BSRL_ERR_CUDA;
+  if (!make_tmap_rows(&tm_r, a.R, 4, a.M, a.N, a.ldr, 32, 128)) return BSRL_ERR_CUDA;
+  if (!make_tmap_rows(&tm_x, a.x_out, 4, a.M, a.N, a.ldx, 32, 128)) return BSRL_ERR_CUDA;
   if (!make_tmap_rows(&tm_h, a.h, 2, a.M, a.N, a.ldh, 32, 128)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("linear_ln_kernel set-up", [] {
-    return cudaFuncSetAttribute(linear_ln_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(linear_ln_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(linear_ln_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   });
   if (rc != BSRL_OK) return rc;
   Params p;
-  p.N = a.N; p.K = a.K; p.M = a.M;
+  p.nc = nc; p.K = a.K; p.M = a.M; p.inv_n = 1.0f / (float)a.N;
   p.bias = a.bias; p.gamma = a.gamma; p.beta = a.beta; p.eps = a.eps;
-  p.R = a.R; p.ldr = a.ldr; p.x_out = a.x_out; p.ldx = a.ldx;
+  p.h = a.h; p.ldh = a.ldh;
   p.n_tiles = (int)((a.M + BM - 1) / BM);
   p.status = status;
-  const int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
-  launch_kernel(linear_ln_kernel, grid, THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_h, p);
+  const int places = sm_count() / cl, groups = p.n_tiles < places ? p.n_tiles : places;
+  if (cl == 2) launch_kernel<2>(linear_ln_kernel<2>, (unsigned)(2 * groups), THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_r, tm_x, tm_h, p);
+  else launch_kernel(linear_ln_kernel<1>, (unsigned)groups, THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_r, tm_x, tm_h, p);
   BSRL_LAUNCH_OK("linear_ln_kernel");
   return BSRL_OK;
 }
