@@ -15,8 +15,15 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
-// Attention of one (env, head) pair from the shared q|k|v tile; one warp.  q, k, v are byte
-// addresses (shared window) of the pair's first row / first column; rows are LDQ bytes apart.
+// Byte address of 16-byte piece `piece` of row `row` of a section (q, k or v): rows LDQ bytes apart, or, for LDQ = 128, a
+// 128-byte-swizzled tile (piece p of row r at ((p ^ (r & 7)) << 4)) that starts on a 1024-byte boundary
+template <int LDQ>
+__device__ __forceinline__ uint32_t section_at(uint32_t base, int row, int piece) {
+  return LDQ == 128 ? base + row * 128 + ((piece ^ (row & 7)) << 4) : base + row * LDQ + (piece << 4);
+}
+
+// Attention of one (env, head) pair from the shared q|k|v tile; one warp.  sq, sk, sv: byte addresses (shared window) of
+// the env's first row in the three sections; query rows from q_row0, the head's columns from 16-byte piece piece0.
 // The MT 16-row query tiles are processed side by side: two independent dependency chains per warp
 // (the kernel is latency-bound here) and each K / V fragment is fetched once for both.
 // OB: bytes per row of the staged group output (128: two heads of 32, swizzled; 96: one head of 48, dense)
@@ -24,7 +31,7 @@ __device__ __forceinline__ float rcp_approx(float x) {
 // base-2 key bias, v0 its DH values (shared memory, generic pointer); its score joins each row's softmax and its
 // probability times v_0 starts the row's output.
 template <int MT, int DH, int LDQ, int OB, bool BODY = false>
-__device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t sv, const float (&kb)[4][2],
+__device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t sv, int q_row0, int piece0, const float (&kb)[4][2],
                                             int n_q, __half* out_env, int ldo, int lane, uint8_t* so, int so_row0, int so_piece0,
                                             float x_lane = 0.f, float kb0 = 0.f, const __half* v0 = nullptr) {
   const int g = lane >> 2, tig = lane & 3;
@@ -41,12 +48,12 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
     uint32_t a[MT][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
-      ldmatrix_x4(a[mt], sq + (mt * 16 + (lane & 15)) * LDQ + (ks * 16 + (lane >> 4) * 8) * 2);
+      ldmatrix_x4(a[mt], section_at<LDQ>(sq, q_row0 + mt * 16 + (lane & 15), piece0 + ks * 2 + (lane >> 4)));
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       uint32_t b[4];
       const int row = j * 16 + (lane & 7) + ((lane >> 4) << 3);
-      ldmatrix_x4(b, sk + row * LDQ + (ks * 16 + ((lane >> 3) & 1) * 8) * 2);
+      ldmatrix_x4(b, section_at<LDQ>(sk, row, piece0 + ks * 2 + ((lane >> 3) & 1)));
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         mma_f16(s[mt][2 * j], a[mt], b[0], b[1]);
@@ -125,7 +132,7 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
     for (int j = 0; j < DH / 16; ++j) {
       uint32_t b[4];
       const int row = ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-      ldmatrix_x4_trans(b, sv + row * LDQ + (j * 16 + (lane >> 4) * 8) * 2);
+      ldmatrix_x4_trans(b, section_at<LDQ>(sv, row, piece0 + j * 2 + (lane >> 4)));
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         mma_f16(o[mt][2 * j], pa[mt][ks], b[0], b[1]);
@@ -157,17 +164,17 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
 }
 
 // One query row of an env on the CUDA cores (lane = key for the scores, lane = output column for the weighted sum):
-// q row `q_row` at column `col0` of the tile (rows LDQ bytes apart), k and v GD and 2 GD columns further; kb_row: this
-// lane's key bias in base 2, -inf past the last key.
+// row q_row of section sq (as in attend_pair, generic pointers) against the NKEYS rows of sk and sv, the head's columns
+// from piece0; kb_row: this lane's key bias in base 2, -inf past the last key.
 template <int DH, int LDQ, int NKEYS>
-__device__ __forceinline__ void attend_one_row(const uint8_t* rows_g, int q_row, int col0, int GD, float kb_row, __half* orow, int lane) {
-  const uint8_t* qrow = rows_g + q_row * LDQ + col0 * 2;
-  const uint8_t* krow = rows_g + (lane < NKEYS ? lane : 0) * LDQ + (GD + col0) * 2;
+__device__ __forceinline__ void attend_one_row(const uint8_t* sq, const uint8_t* sk, const uint8_t* sv, int q_row, int piece0, float kb_row,
+                                               __half* orow, int lane) {
+  const int krow = lane < NKEYS ? lane : 0;
   float sc = 0.f;
 #pragma unroll
   for (int ch = 0; ch < DH / 8; ++ch) {
-    const uint4 qv = *reinterpret_cast<const uint4*>(qrow + ch * 16);
-    const uint4 kv = *reinterpret_cast<const uint4*>(krow + ch * 16);
+    const uint4 qv = *reinterpret_cast<const uint4*>(sq + section_at<LDQ>(0, q_row, piece0 + ch));
+    const uint4 kv = *reinterpret_cast<const uint4*>(sk + section_at<LDQ>(0, krow, piece0 + ch));
     const __half2* qh = reinterpret_cast<const __half2*>(&qv);
     const __half2* kh = reinterpret_cast<const __half2*>(&kv);
 #pragma unroll
@@ -183,11 +190,11 @@ __device__ __forceinline__ void attend_one_row(const uint8_t* rows_g, int q_row,
 #pragma unroll
   for (int dd = 0; dd < DH; dd += 32) {
     const int col = dd + lane;
-    const uint8_t* vcol = rows_g + (2 * GD + col0) * 2 + (col < DH ? col : 0) * 2;
+    const int vc = col < DH ? col : 0;
     float acc = 0.f;
 #pragma unroll 8
     for (int j = 0; j < NKEYS; ++j)
-      acc = fmaf(__shfl_sync(0xffffffffu, pj, j), __half2float(*reinterpret_cast<const __half*>(vcol + j * LDQ)), acc);
+      acc = fmaf(__shfl_sync(0xffffffffu, pj, j), __half2float(*reinterpret_cast<const __half*>(sv + section_at<LDQ>(0, j, piece0 + (vc >> 3)) + (vc & 7) * 2)), acc);
     if (col < DH) orow[col] = __float2half_rn(acc * inv);
   }
 }

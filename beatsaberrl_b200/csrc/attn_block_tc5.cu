@@ -7,22 +7,30 @@
 // One tile = 4 environments, each padded from 29 to 32 token rows (a 3-D TMA load zero-fills rows
 // 29..31), so that env e of the tile is exactly rows [32 e, 32 e + 32) = TMEM lane quadrant e of the
 // 128-row MMA.  The projection runs per HEAD GROUP (two heads: 64 q + 64 k + 64 v = 192 output
-// columns, the weight rows regrouped at pack time), so that a group's q, k, v fit in one 50 KB
+// columns, the weight rows regrouped at pack time), so that a group's q, k, v fit in one 48 KB
 // shared-memory tile.  The two warps that own a lane quadrant drain THEIR env's rows (half of the
 // columns each) and then attend that env's two heads (m16n8k16 MMAs, fp32 softmax in registers): an env
-// only ever waits for its own pair of warps (a 64-thread named barrier), never for the whole CTA, while
-// the tensor core already projects the next group into the other TMEM buffer.
+// only ever waits for its own pair of warps (a 64-thread named barrier), never for the whole CTA.  Two
+// sets of eight workers take the groups in turn, each with its own TMEM buffer and q|k|v tile: with one
+// set, two warps per scheduler, the chain drain -> barrier -> scores -> softmax -> output was most of the
+// time (head_dim 48: issue slots 33 % and tensor pipe 36 % busy).
 //
 //   warp 0      TMA producer: the h tile (d/64 swizzled chunks, loaded once per tile) and the
-//               regrouped weight tiles (192 x 64 or 144 x 64 per stage, 3- or 4-stage ring)
+//               regrouped weight tiles (192 x 64 or 144 x 64 per stage, ring of 2 to 4 stages)
 //   warp 1      MMA issuer: tcgen05.mma M = 128, N = 192, K = 16
-//   warps 2..9  drain the accumulator (+ bias, fp16) into the q|k|v tile, then attend
+//   warps 2..17 two sets of eight: drain the accumulator (+ bias, fp16) into the q|k|v tile, then attend
+//
+// Long runs sit at the power cap (990 W, 1.4 to 1.8 GHz), where time follows the energy of an env rather than
+// the length of a chain.  There a PAIR of CTAs (cta_group::2) shares the weight tile: each fetches half of its
+// rows and the leader's MMAs (M = 256) read both.  65,536 envs, us in a loop of seconds, one set of workers / two /
+// two and pairs: 192 wide 885 / 790 / 800 (not taken: N = 144 pads to 160), 256 wide 1237 / 1164 / 1121; 16,384 envs
+// of 512: 925 / 925 / 863.
 //
 // HBM traffic per token: read h (2d B), write att (2d B).  Replaces fp16_packed_linear + attn29 /
 // packed_sdpa (python/policy.py:586-600, :645-692; python/beat_arena_env/csrc/small_attn.cu).
 // With all 29 query rows, an env's output for the group (29 rows x 128 bytes for two heads of 32, x 96 bytes
-// for one head of 48) is staged in shared memory and leaves as one TMA store per env.  All waits are
-// bounded (tc5.cuh).
+// for one head of 48) is staged in shared memory (64-wide groups: in place of its q rows) and leaves as one TMA
+// store per env.  All waits are bounded (tc5.cuh).
 #include "kernels.cuh"
 #include "attend.cuh"
 #include "tc5.cuh"
@@ -33,40 +41,48 @@ using namespace tc5;
 
 constexpr int EPT = 4;                  // envs per tile
 constexpr int EROWS = 32;               // tile rows per env: 29 tokens + 3 zero rows
+constexpr int TEAM = 2, SETS = 2;       // workers: two sets, each two warps per env
 constexpr int BM = EPT * EROWS;
-constexpr int MAX_STAGES = 4;           // weight ring: 3 stages of 24 KB (head_dim 32) or 4 of 18 KB (head_dim 48), as measured
+constexpr int MAX_STAGES = 4;
 constexpr int CHUNK_BYTES = BM * 128;   // 16 KB: 128 rows x 64 k-columns
-constexpr int WORKERS = 8;
-constexpr int THREADS = (2 + WORKERS) * 32;
 // Head group of G heads of width DH: 3 G DH projection columns per group -- (32, 2): 192, two heads;
 // (48, 1): 144, one head (the reference's production shape, 4 heads of 48); (64, 1): 192, one head (the wide policy).
-template <int DH_, int G_>
+template <int DH_, int G_, bool PAIR>
 struct Shape {
   static constexpr int DH = DH_, G = G_, GD = G * DH, NG = 3 * GD;
   // STREAM (head_dim 64, d up to 512): the h tile does not stay resident (128 rows x 512 x 2 B = 128 KB); its
   // 64-column chunks travel through the ring beside the weight chunks, once per head group (from L2 after the first)
   static constexpr bool STREAM = DH == 64;
-  static constexpr int STAGES = DH == 48 ? 4 : 3;
-  static constexpr int W_BYTES = NG * 128;       // NG weight rows x 64 k-columns (24 KB / 18 KB)
+  // 24 KB (18, in a pair 12) a stage, with the h chunk 40 (28): as many as fit beside two q|k|v tiles
+  static constexpr int STAGES = PAIR || DH == 48 ? 4 : DH == 32 ? 2 : 3;
+  static constexpr int W_ROWS = PAIR ? NG / 2 : NG;    // weight rows per CTA
+  static constexpr int W_BYTES = W_ROWS * 128;         // x 64 k-columns (24 KB / 18 KB, 12 KB in a pair)
   static constexpr int STAGE_BYTES = W_BYTES + (STREAM ? CHUNK_BYTES : 0);
-  static constexpr int A_BYTES = STREAM ? 0 : 4 * CHUNK_BYTES;
-  static constexpr int MAX_D = STREAM ? 512 : 256;
-  static constexpr int LDQ = NG * 2 + 16;        // row pitch of the q|k|v tile: 400 / 304 bytes, ldmatrix conflict-free
-  static constexpr int SQ_BYTES = BM * LDQ;
-  static constexpr int SO_BYTES = BM * 128;      // attention output of one group: 128 rows x 128 B, 128-byte swizzle
+  static constexpr int WORKERS = EPT * TEAM * SETS, THREADS = (2 + WORKERS) * 32;
+  static constexpr int MAX_D = STREAM ? 512 : DH == 48 ? 192 : 256;
+  static constexpr int A_BYTES = STREAM ? 0 : MAX_D / 64 * CHUNK_BYTES;
+  // q|k|v of a group.  Head groups 64 columns wide: three swizzled 128-byte-row sections, and the output takes the place of
+  // the q rows it came from.  48 wide: rows of 304 bytes (ldmatrix conflict-free), the output beside them.
+  static constexpr bool INPLACE = GD == 64;
+  static constexpr int LDQ = INPLACE ? 128 : NG * 2 + 16;
+  static constexpr int SECTION = INPLACE ? CHUNK_BYTES : GD * 2;      // from a row's q to its k, and to its v
+  static constexpr int SQ_BYTES = INPLACE ? 3 * CHUNK_BYTES : BM * LDQ;
+  static constexpr int SO_BYTES = INPLACE ? 0 : BM * GD * 2;
   static constexpr int BIAS_BYTES = 3 * MAX_D * 4;
-  static constexpr int SB_BYTES = EPT * 2 * 3 * 64;   // body-token mode: q0 | k0 | v0 (64 B each) per env and head of the group
-  static constexpr int SMEM_BYTES = A_BYTES + STAGES * STAGE_BYTES + SO_BYTES + SQ_BYTES + BIAS_BYTES + SB_BYTES + 1024 + 256;
-  static_assert(NG % 16 == 0 && NG <= 256 && STAGE_BYTES % 1024 == 0 && W_BYTES % 1024 == 0, "group width");
+  static constexpr int SB_BYTES = DH == 32 ? SETS * EPT * 2 * 3 * 64 : 0;   // body-token mode: q0 | k0 | v0 (64 B each) per env and head of the group
+  static constexpr int SMEM_BYTES = A_BYTES + STAGES * STAGE_BYTES + SETS * (SO_BYTES + SQ_BYTES) + BIAS_BYTES + SB_BYTES + 1024 + 256;
+  static_assert((!PAIR || NG % 32 == 0) && NG <= 256 && W_ROWS % 8 == 0 && STAGES <= MAX_STAGES && STAGE_BYTES % 1024 == 0 && W_BYTES % 1024 == 0, "group width");
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 };
 constexpr int KERNEL_ID = 3;
+template <int V>
+struct Int { static constexpr int value = V; };
 
 struct Shared {
-  uint64_t w_full[MAX_STAGES], w_empty[MAX_STAGES], a_full[4], a_free[4], acc_full[2], acc_empty[2], attn_done[2], mma_done;
+  uint64_t w_full[MAX_STAGES], w_empty[MAX_STAGES], a_full[4], a_free[4], acc_full[2], acc_empty[2], mma_done;
   uint32_t tmem_base;
   int abort;
-  int quit[EPT];   // abort flag as sampled by one thread of an env's warp pair before their barrier, so both leave together
+  int quit[2 * EPT];   // abort flag as sampled by one thread of an env's warp pair before their barrier, so both leave together
 };
 
 struct Params {
@@ -96,29 +112,40 @@ __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
 
 // VRES: the value-residual code of the drain is compiled in (it costs ~14 % of the kernel even when idle)
 // BODY: the single-body-token layout (Params::tokens and below); DH = 32, G = 2 only
-template <int DH, int G, bool VRES, bool BODY = false>
-__global__ void __launch_bounds__(THREADS, 1)
+template <int DH, int G, bool PAIR, bool VRES, bool BODY = false>
+__global__ void __launch_bounds__((Shape<DH, G, PAIR>::THREADS), 1)
 attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constant__ CUtensorMap tm_w,
                   const __grid_constant__ CUtensorMap tm_o, Params p) {
-  using S = Shape<DH, G>;
+  using S = Shape<DH, G, PAIR>;
   constexpr int STAGES = S::STAGES, GD = S::GD, NG = S::NG, STAGE_BYTES = S::STAGE_BYTES, LDQ = S::LDQ, SQ_BYTES = S::SQ_BYTES;
+  constexpr int THREADS = S::THREADS, SECTION = S::SECTION;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - raw);
   constexpr bool STREAM = S::STREAM;
-  const uint32_t sA = base, ring = base + S::A_BYTES, sO = ring + STAGES * STAGE_BYTES, sQ = sO + S::SO_BYTES;
-  uint8_t* sO_g = gen + S::A_BYTES + STAGES * STAGE_BYTES;
-  uint8_t* sQ_g = sO_g + S::SO_BYTES;
-  float* s_bias = reinterpret_cast<float*>(sQ_g + SQ_BYTES);
-  uint8_t* sB_g = sQ_g + SQ_BYTES + S::BIAS_BYTES;
-  Shared* sh = reinterpret_cast<Shared*>(sB_g + S::SB_BYTES);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int set = warp >= 2 + EPT * TEAM ? 1 : 0;                   // the set of workers this warp is in
+  const uint32_t sA = base, ring = base + S::A_BYTES, sQ = ring + STAGES * STAGE_BYTES + set * SQ_BYTES;
+  const uint32_t sO = S::INPLACE ? sQ : ring + STAGES * STAGE_BYTES + SETS * SQ_BYTES + set * S::SO_BYTES;
+  uint8_t* sQ_g = gen + (sQ - base);
+  uint8_t* sO_g = S::INPLACE ? sQ_g : gen + (sO - base);
+  float* s_bias = reinterpret_cast<float*>(gen + S::A_BYTES + STAGES * STAGE_BYTES + SETS * (S::SO_BYTES + SQ_BYTES));
+  uint8_t* sB_all = reinterpret_cast<uint8_t*>(s_bias) + S::BIAS_BYTES;
+  uint8_t* sB_g = sB_all + set * (S::SB_BYTES / SETS);
+  Shared* sh = reinterpret_cast<Shared*>(sB_all + S::SB_BYTES);
   static_assert(!BODY || (DH == 32 && G == 2 && !VRES), "body-token mode: two heads of 32 per group");
   constexpr int NKEYS = BODY ? EROWS : kT;            // live keys of an env inside the tile
   const int T = BODY ? p.tokens : kT;                 // token rows per env in memory
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d = p.d, KB = d >> 6, n_groups = d / GD;
   volatile int* abort = &sh->abort;
+  const uint32_t rank = PAIR ? cluster_rank() : 0u;
+  const int t_end = PAIR ? (p.n_tiles + 1) & ~1 : p.n_tiles;       // both CTAs of a pair take the same number of tiles
+  constexpr int CTAS = PAIR ? 2 : 1;
+  auto commit = [&](uint64_t* bar) {                  // -> the barrier, in both CTAs of a pair
+    if (PAIR) tc_commit_pair(smem_u32(bar));
+    else tc_commit(smem_u32(bar));
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -131,23 +158,28 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&sh->acc_full[b]), 1);
-      mbar_init(smem_u32(&sh->acc_empty[b]), WORKERS);
-      mbar_init(smem_u32(&sh->attn_done[b]), WORKERS);
+      mbar_init(smem_u32(&sh->acc_empty[b]), CTAS * EPT * TEAM);      // a pair's leader: both CTAs' workers
     }
     mbar_init(smem_u32(&sh->mma_done), 1);
     sh->abort = 0;
-    for (int e = 0; e < EPT; ++e) sh->quit[e] = 0;
+    for (int e = 0; e < 2 * EPT; ++e) sh->quit[e] = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tm_h);
     tma_prefetch_desc(&tm_w);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&sh->tmem_base), 512);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc_pair(smem_u32(&sh->tmem_base), 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(smem_u32(&sh->tmem_base), 512);
+      tmem_relinquish();
+    }
   }
   for (int i = threadIdx.x; i < 3 * d; i += THREADS) s_bias[i] = p.bias[i];
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();          // the peer's barriers exist before anything is signalled across
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
   if (warp != 0) pdl_begin();    // the producer waits below, after its first weight stages
@@ -157,19 +189,27 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
     if (lane == 0) {
       uint32_t it = 0, tile_i = 0;
       bool ok = true;
+      auto load_w = [&](uint32_t dst, int x, int y, uint32_t bar) {
+        if (PAIR) tma_load_2d_pair(dst, &tm_w, x, y, map_to_cta(bar, 0));
+        else tma_load_2d(dst, &tm_w, x, y, bar);
+      };
+      auto load_h = [&](uint32_t dst, int kb, int t, uint32_t bar) {
+        if (PAIR) tma_load_3d_pair(dst, &tm_h, 64 * kb, BODY ? p.tok0 : 0, t * EPT, map_to_cta(bar, 0));
+        else tma_load_3d(dst, &tm_h, 64 * kb, BODY ? p.tok0 : 0, t * EPT, bar);
+      };
       auto w_stage = [&](int g, int kb, int t) -> bool {
         const int s = it % STAGES;
         const uint32_t ph = (it / STAGES) & 1;
         if (!mbar_wait(smem_u32(&sh->w_empty[s]), ph ^ 1, abort)) { give_up(sh, p.status, 1); return false; }
         const uint32_t bar = smem_u32(&sh->w_full[s]);
-        mbar_expect_tx(bar, STAGE_BYTES);
-        tma_load_2d(ring + s * STAGE_BYTES, &tm_w, 64 * kb, NG * g, bar);
-        if (STREAM) tma_load_3d(ring + s * STAGE_BYTES + S::W_BYTES, &tm_h, 64 * kb, BODY ? p.tok0 : 0, t * EPT, bar);
+        if (rank == 0) mbar_expect_tx(bar, CTAS * STAGE_BYTES);   // both CTAs' bytes
+        load_w(ring + s * STAGE_BYTES, 64 * kb, NG * g + (int)rank * S::W_ROWS, bar);
+        if (STREAM) load_h(ring + s * STAGE_BYTES + S::W_BYTES, kb, t, bar);
         ++it;
         return true;
       };
       if (STREAM) pdl_wait();
-      for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, ++tile_i) {
+      for (int t = blockIdx.x; t < t_end && ok; t += gridDim.x, ++tile_i) {
         if (STREAM) {
           for (int g = 0; g < n_groups && ok; ++g)
             for (int kb = 0; kb < KB && ok; ++kb) ok = w_stage(g, kb, t);
@@ -184,20 +224,20 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
           // chunk kb of the h tile is free once the previous tile's last group has used it
           if (!mbar_wait(smem_u32(&sh->a_free[kb]), (tile_i & 1) ^ 1, abort)) { give_up(sh, p.status, 2); ok = false; break; }
           const uint32_t bar = smem_u32(&sh->a_full[kb]);
-          mbar_expect_tx(bar, CHUNK_BYTES);
-          tma_load_3d(sA + kb * CHUNK_BYTES, &tm_h, 64 * kb, BODY ? p.tok0 : 0, t * EPT, bar);
+          if (rank == 0) mbar_expect_tx(bar, CTAS * CHUNK_BYTES);
+          load_h(sA + kb * CHUNK_BYTES, kb, t, bar);
           if (kb >= early) ok = w_stage(0, kb, t);
         }
         for (int g = 1; g < n_groups && ok; ++g)
           for (int kb = 0; kb < KB && ok; ++kb) ok = w_stage(g, kb, t);
       }
-      // loads in flight must land before the CTA exits (bounded, ignoring abort)
-      for (uint32_t j = it > STAGES ? it - STAGES : 0; j < it; ++j) {
+      // loads in flight (both CTAs' are counted on the leader's barriers) land before the pair exits; bounded, ignoring abort
+      for (uint32_t j = it > STAGES ? it - STAGES : 0; rank == 0 && j < it; ++j) {
         uint32_t spins = 0;
         while (!mbar_try_wait(smem_u32(&sh->w_full[j % STAGES]), (j / STAGES) & 1) && ++spins < kSpinLimit) {}
         if (spins >= kSpinLimit) give_up(sh, p.status, 3);
       }
-      if (!STREAM && tile_i > 0)
+      if (!STREAM && rank == 0 && tile_i > 0)
         for (int kb = 0; kb < KB; ++kb) {
           uint32_t spins = 0;
           while (!mbar_try_wait(smem_u32(&sh->a_full[kb]), (tile_i - 1) & 1) && ++spins < kSpinLimit) {}
@@ -205,20 +245,15 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
         }
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // ------------------------------------------------------------ MMA issuer (the leader's)
+    if (lane == 0 && rank == 0) {
       uint32_t it = 0, tile_i = 0, gi = 0;
       bool ok = true;
-      const uint32_t idesc = idesc_f16(BM, NG);
-      for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, ++tile_i) {
+      const uint32_t idesc = idesc_f16(CTAS * BM, NG);
+      for (int t = blockIdx.x; t < t_end && ok; t += gridDim.x, ++tile_i) {
         for (int g = 0; g < n_groups && ok; ++g, ++gi) {
           const int buf = gi & 1;
           if (!mbar_wait(smem_u32(&sh->acc_empty[buf]), ((gi >> 1) & 1) ^ 1, abort)) { give_up(sh, p.status, 5); ok = false; break; }
-          // The workers' attention runs on warp-level MMAs, which queue behind tcgen05 MMAs on the same
-          // tensor cores: this group's projection is held back until the attention of two groups ago is
-          // over, so that it runs while the workers drain the previous group instead (without the wait the
-          // kernel measured 3 % slower).
-          if (gi >= 2 && !mbar_wait(smem_u32(&sh->attn_done[buf]), ((gi - 2) >> 1) & 1, abort)) { give_up(sh, p.status, 10); ok = false; break; }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + buf * 256;
           for (int kb = 0; kb < KB; ++kb, ++it) {
@@ -229,34 +264,35 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
             const uint64_t ad = smem_desc_sw128(STREAM ? ring + s * STAGE_BYTES + S::W_BYTES : sA + kb * CHUNK_BYTES);
             const uint64_t wd = smem_desc_sw128(ring + s * STAGE_BYTES);
 #pragma unroll
-            for (int k = 0; k < 4; ++k) mma_f16_ss(d_tmem, ad + 2 * k, wd + 2 * k, idesc, (kb | k) != 0);
-            tc_commit(smem_u32(&sh->w_empty[s]));
-            if (!STREAM && g == n_groups - 1) tc_commit(smem_u32(&sh->a_free[kb]));
+            for (int k = 0; k < 4; ++k) {
+              if (PAIR) mma_f16_ss_pair(d_tmem, ad + 2 * k, wd + 2 * k, idesc, (kb | k) != 0);
+              else mma_f16_ss(d_tmem, ad + 2 * k, wd + 2 * k, idesc, (kb | k) != 0);
+            }
+            commit(&sh->w_empty[s]);
+            if (!STREAM && g == n_groups - 1) commit(&sh->a_free[kb]);
           }
-          if (ok) tc_commit(smem_u32(&sh->acc_full[buf]));
+          if (ok) commit(&sh->acc_full[buf]);
         }
       }
-      tc_commit(smem_u32(&sh->mma_done));
+      commit(&sh->mma_done);
       uint32_t spins = 0;
       while (!mbar_try_wait(smem_u32(&sh->mma_done), 0) && ++spins < kSpinLimit) {}
       if (spins >= kSpinLimit) give_up(sh, p.status, 8);
     }
   } else {
     // ------------------------------------------------------------ workers: drain, then attend
-    const int wi = warp - 2;
-    const int q = warp & 3, half = wi >> 2;           // TMEM lane quadrant = env of the tile, column half
+    const int q = warp & 3, part = ((warp - 2) >> 2) % TEAM;   // TMEM lane quadrant = env of the tile; place in the env's team
     const int trow = q * EROWS + lane;                // tile row: token `lane` of env q (29..31: zero rows)
-    // drain: the group's NG columns in 16-column units, split between the two halves (6 + 6 or 5 + 4)
-    constexpr int UNITS = NG / 16, U0 = (UNITS + 1) / 2;
-    const int u_first = half ? U0 : 0, u_count = half ? UNITS - U0 : U0;
-    // attention of the env this warp drained: G = 2: one head per warp of the pair, both 16-row query tiles;
-    // G = 1: one query tile each
-    const int env_l = q, hh = G == 2 ? half : 0, mt_own = G == 2 ? 0 : half;
-    auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + q) : "memory"); };
+    // drain: the group's NG columns in 16-column units, split over the team (3 + 3 + 3 + 3, 6 + 6 or 5 + 4)
+    constexpr int UNITS = NG / 16, U0 = (UNITS + TEAM - 1) / TEAM;
+    const int u_first = part * U0, u_count = UNITS - u_first < U0 ? UNITS - u_first : U0;
+    // attention of the env this pair drained: G = 2: one head per warp, both 16-row query tiles; G = 1: one query tile each
+    const int env_l = q, hh = G == 2 ? part : 0, mt_own = G == 2 ? 0 : part;
+    auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + q + set * EPT), "n"(TEAM * 32) : "memory"); };
     uint32_t gi = 0;
     bool ok = true;
     const float vres_a = (VRES && p.vres) ? p.vres[0] : 1.f, vres_b = (VRES && p.vres) ? p.vres[1] : 0.f;
-    for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x) {
+    for (int t = blockIdx.x; t < t_end && ok; t += gridDim.x) {
       const int64_t env = (int64_t)t * EPT + env_l;
       // this lane's key-bias values (keys nt * 8 + tig * 2 + e of the m16n8 accumulator layout, times
       // log2 e; -inf past the 29th key), fetched once per tile and long before the first softmax
@@ -266,7 +302,7 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int key = nt * 8 + (lane & 3) * 2 + e;
-          kb[nt][e] = (key < NKEYS && env < p.n_envs) ? p.key_bias[env * T + (BODY ? p.tok0 : 0) + key] * 1.4426950408889634f : -INFINITY;
+          kb[nt][e] = (key < NKEYS && env < p.n_envs) ? p.key_bias[env * T + (BODY ? p.tok0 : 0) + key] : -INFINITY;
         }
       // body-token mode: the body key's bias, and this lane's object key's (lane = key in the body row's softmax)
       float kb0 = 0.f, kbl = 0.f;
@@ -278,8 +314,10 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
       const bool one_row = !BODY && p.n_q == 1;
       float kb_row = -INFINITY;
       if (one_row && lane < NKEYS && env < p.n_envs) kb_row = p.key_bias[env * T + lane] * 1.4426950408889634f;
+      bool fresh = true;
       for (int g = 0; g < n_groups && ok; ++g, ++gi) {
         const int buf = gi & 1;
+        if (buf != set) continue;                       // the other set's group
         // body token's q0 | k0 | v0 of this warp's head: lanes 0..11 fetch one 16-byte piece each, long before use
         uint4 b0v = make_uint4(0, 0, 0, 0);
         if (BODY && lane < 12 && env < p.n_envs)
@@ -289,10 +327,13 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
         // the abort flag ahead of a barrier.
         if (!mbar_wait_warp(smem_u32(&sh->acc_full[buf]), (gi >> 1) & 1, abort) && lane == 0) give_up(sh, p.status, 9);
         tc_fence_after();
+        if (S::INPLACE && p.out_tma && part == 0) {      // the warp that writes the q rows: the store from them has read them
+          if (lane == 0) bulk_wait_read<0>();
+          __syncwarp();
+        }
         {
           const uint32_t tcol = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256 + u_first * 16;
           const float* bias_u = s_bias + g * NG + u_first * 16;
-          uint8_t* dst_u = sQ_g + trow * LDQ + (u_first * 16) * 2;
           // 16 columns -> bias, fp16, two 16-byte pieces of this thread's row
           auto put16 = [&](const uint32_t* v, int u) {
             const float4* b4 = reinterpret_cast<const float4*>(bias_u + u * 16);
@@ -321,7 +362,9 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
                   f[2 * e + 1] = fmaf(vres_a, f[2 * e + 1], vres_b * ov.y);
                 }
               }
-              *reinterpret_cast<uint4*>(dst_u + u * 32 + 16 * j) =
+              const int un = u_first + u;                              // 16-byte piece of this thread's row
+              uint8_t* dst = S::INPLACE ? sQ_g + (un >> 2) * SECTION + section_at<LDQ>(0, trow, (un & 3) * 2 + j) : sQ_g + trow * LDQ + un * 32 + 16 * j;
+              *reinterpret_cast<uint4*>(dst) =
                   make_uint4(pack_half2(f[0], f[1]), pack_half2(f[2], f[3]), pack_half2(f[4], f[5]), pack_half2(f[6], f[7]));
             }
           };
@@ -340,23 +383,30 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
             put16(r, u);
           }
         }
-        if (BODY && lane < 12) *reinterpret_cast<uint4*>(sB_g + ((env_l * 2 + hh) * 3 + (lane >> 2)) * 64 + (lane & 3) * 16) = b0v;
+        if (BODY && mt_own == 0 && lane < 12) *reinterpret_cast<uint4*>(sB_g + ((env_l * 2 + hh) * 3 + (lane >> 2)) * 64 + (lane & 3) * 16) = b0v;
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sh->acc_empty[buf]));     // the TMEM buffer may be refilled
-        if (half == 0 && lane == 0) {
-          sh->quit[q] = *abort;
-          if (p.out_tma) bulk_wait_read<0>();           // this env's previous output store has read its sO rows
+        if (lane == 0) {
+          if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->acc_empty[buf]), 0));
+          else mbar_arrive(smem_u32(&sh->acc_empty[buf]));
+        }     // the TMEM buffer may be refilled
+        if (part == 0 && lane == 0) {
+          sh->quit[set * EPT + q] = *abort;
+          if (!S::INPLACE && p.out_tma) bulk_wait_read<0>();      // this env's previous output store has read its sO rows
         }
-        pair_sync();                                    // the env's q|k|v rows are complete
-        if (*reinterpret_cast<volatile int*>(&sh->quit[q])) {
+        team_sync();                                    // the env's q|k|v rows are complete
+        if (*reinterpret_cast<volatile int*>(&sh->quit[set * EPT + q])) {
           ok = false;
           break;
         }
+        if (fresh) {                                    // to base 2, where the loads have long landed
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) kb[nt][0] *= 1.4426950408889634f, kb[nt][1] *= 1.4426950408889634f;
+          fresh = false;
+        }
         if (env < p.n_envs) {
-          const uint32_t rows = sQ + (env_l * EROWS) * LDQ;
-          const uint32_t sq_pair = rows + (p.q_first + mt_own * 16) * LDQ + (hh * DH) * 2,
-                         sk_pair = rows + (GD + hh * DH) * 2, sv_pair = rows + (2 * GD + hh * DH) * 2;
+          const uint32_t rows = sQ + (env_l * EROWS) * LDQ;             // the env's q rows; k and v at SECTION and 2 SECTION
+          const int q_row0 = p.q_first + mt_own * 16, piece0 = hh * (DH / 8);
           __half* out_pair = p.out + (env * p.n_q + mt_own * 16) * (int64_t)p.ldo + (g * G + hh) * DH;
           const int n_q = p.n_q - mt_own * 16;      // query rows left from this warp's first one
           uint8_t* so_tile = p.out_tma ? sO_g : nullptr;
@@ -370,8 +420,8 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
             for (int ch = 0; ch < DH / 8; ++ch) {
               const uint4 q0v = *reinterpret_cast<const uint4*>(sb + ch * 16);
               const uint4 k0v = *reinterpret_cast<const uint4*>(sb + 64 + ch * 16);
-              const uint4 qv = *reinterpret_cast<const uint4*>(rows_g + lane * LDQ + (hh * DH) * 2 + ch * 16);
-              const uint4 kv = *reinterpret_cast<const uint4*>(rows_g + lane * LDQ + (GD + hh * DH) * 2 + ch * 16);
+              const uint4 qv = *reinterpret_cast<const uint4*>(rows_g + section_at<LDQ>(0, lane, piece0 + ch));
+              const uint4 kv = *reinterpret_cast<const uint4*>(rows_g + SECTION + section_at<LDQ>(0, lane, piece0 + ch));
               const __half2* q0h = reinterpret_cast<const __half2*>(&q0v);
               const __half2* k0h = reinterpret_cast<const __half2*>(&k0v);
               const __half2* qh = reinterpret_cast<const __half2*>(&qv);
@@ -392,50 +442,79 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
               const float pj = ex2_approx(sc - mx), p00 = ex2_approx(s00 - mx);
               const float inv = rcp_approx(warp_sum(pj) + p00);
               const __half* v0h = reinterpret_cast<const __half*>(sb + 128);
-              const uint8_t* vcol = rows_g + (2 * GD + hh * DH) * 2 + lane * 2;      // column `lane` of the head's v rows
+              const uint8_t* v_g = rows_g + 2 * SECTION;                   // column `lane` of the head's v rows
               float acc = p00 * __half2float(v0h[lane]);
 #pragma unroll 8
               for (int j = 0; j < EROWS; ++j)
-                acc = fmaf(__shfl_sync(0xffffffffu, pj, j), __half2float(*reinterpret_cast<const __half*>(vcol + j * LDQ)), acc);
+                acc = fmaf(__shfl_sync(0xffffffffu, pj, j),
+                           __half2float(*reinterpret_cast<const __half*>(v_g + section_at<LDQ>(0, j, piece0 + (lane >> 3)) + (lane & 7) * 2)), acc);
               __half* orow = p.out + (env * (p.body_only ? 1 : T)) * (int64_t)p.ldo + (g * G + hh) * DH;
               orow[lane] = __float2half_rn(acc * inv);
             }
             if (!p.body_only)
-              attend_pair<2, DH, LDQ, GD * 2, true>(sq_pair, sk_pair, sv_pair, kb, n_q, out_pair, p.ldo, lane, so_tile,
-                                                    env_l * EROWS, hh * (DH / 8), x_lane, kb0, reinterpret_cast<const __half*>(sb + 128));
+              attend_pair<2, DH, LDQ, GD * 2, true>(rows, rows + SECTION, rows + 2 * SECTION, q_row0, piece0, kb, n_q, out_pair, p.ldo, lane,
+                                                    so_tile, env_l * EROWS, piece0, x_lane, kb0, reinterpret_cast<const __half*>(sb + 128));
           } else if (one_row) {
             // One query row per env: on the CUDA cores.  A 16-row MMA tile for one row costs the tensor pipe, which
             // the projection of the next head group shares, 16 warp MMAs of 32 cycles per (env, head); this is ~200
             // plain instructions (lane = key for the scores, lane = output column for the weighted sum).
             if (mt_own == 0) {
-              attend_one_row<DH, LDQ, NKEYS>(sQ_g + (env_l * EROWS) * LDQ, p.q_first, hh * DH, GD, kb_row,
+              const uint8_t* rows_g = sQ_g + (env_l * EROWS) * LDQ;
+              attend_one_row<DH, LDQ, NKEYS>(rows_g, rows_g + SECTION, rows_g + 2 * SECTION, p.q_first, piece0, kb_row,
                                              p.out + env * (int64_t)p.ldo + (g * G + hh) * DH, lane);
             }
           } else {
-            if (G == 2 && n_q > 16) attend_pair<2, DH, LDQ, GD * 2>(sq_pair, sk_pair, sv_pair, kb, n_q, out_pair, p.ldo, lane, so_tile, env_l * EROWS + mt_own * 16, hh * (DH / 8));
-            else if (n_q > 0) attend_pair<1, DH, LDQ, GD * 2>(sq_pair, sk_pair, sv_pair, kb, n_q, out_pair, p.ldo, lane, so_tile, env_l * EROWS + mt_own * 16, hh * (DH / 8));
+            auto attend = [&](auto mt) {
+              attend_pair<decltype(mt)::value, DH, LDQ, GD * 2>(rows, rows + SECTION, rows + 2 * SECTION, q_row0, piece0, kb, n_q, out_pair, p.ldo,
+                                                                lane, so_tile, env_l * EROWS + mt_own * 16, piece0);
+            };
+            if (G == 2 && n_q > 16) attend(Int<2>());
+            else if (n_q > 0) attend(Int<1>());
           }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&sh->attn_done[buf]));
         if (p.out_tma) fence_proxy_async_smem();                         // this thread's sO writes -> the TMA engine
-        pair_sync();                                                     // the env's rows may be overwritten
-        if (p.out_tma && half == 0 && lane == 0 && env < p.n_envs) {     // token rows 29..31 of the box are clipped
+        team_sync();                                                     // the env's rows may be overwritten
+        if (p.out_tma && part == 0 && lane == 0 && env < p.n_envs) {     // token rows 29..31 of the box are clipped
           tma_store_3d(&tm_o, g * GD, BODY ? p.tok0 : 0, (int)env, sO + (uint32_t)(q * EROWS) * (uint32_t)(GD * 2));
           bulk_commit();
         }
       }
     }
-    if (p.out_tma && half == 0 && lane == 0) bulk_wait_all();   // the output stores are complete before the CTA exits
+    if (p.out_tma && part == 0 && lane == 0) bulk_wait_all();   // the output stores are complete before the CTA exits
   }
 
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    if (PAIR) tmem_dealloc_pair(tmem_base, 512);
+    else tmem_dealloc(tmem_base, 512);
   }
+}
+
+template <int DH, int G, bool VRES, bool BODY>
+cudaError_t prepare() {
+  const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+  cudaError_t e = cudaFuncSetAttribute(attn_block_kernel<DH, G, false, VRES, BODY>, at, Shape<DH, G, false>::SMEM_BYTES);
+  if constexpr (DH != 48)
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_block_kernel<DH, G, true, VRES, BODY>, at, Shape<DH, G, true>::SMEM_BYTES);
+  return e;
+}
+template <int DH, int G, bool VRES, bool BODY>
+void launch(bool pair, const CUtensorMap& tm_h, const CUtensorMap& tm_w, const CUtensorMap& tm_o, const Params& p, cudaStream_t stream) {
+  if constexpr (DH != 48)
+    if (pair) {
+      using S = Shape<DH, G, true>;
+      const int pairs = (p.n_tiles + 1) / 2, places = sm_count() / 2;
+      launch_kernel<2>(attn_block_kernel<DH, G, true, VRES, BODY>, 2 * (pairs < places ? pairs : places), S::THREADS, S::SMEM_BYTES, stream,
+                       tm_h, tm_w, tm_o, p);
+      return;
+    }
+  using S = Shape<DH, G, false>;
+  const int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
+  launch_kernel(attn_block_kernel<DH, G, false, VRES, BODY>, grid, S::THREADS, S::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
 }
 }  // namespace
 
@@ -443,7 +522,7 @@ bool attn_block_ok(const AttnBlockArgs& a) {
   if (a.d % 64 != 0 || a.d < 64 || a.n_heads < 1 || a.d % a.n_heads != 0) return false;
   const int dh = a.d / a.n_heads;
   if (!((dh == 32 && a.n_heads % 2 == 0) || dh == 48 || dh == 64)) return false;
-  if (a.d > (dh == 64 ? Shape<64, 1>::MAX_D : Shape<32, 2>::MAX_D)) return false;
+  if (a.d > (dh == 64 ? Shape<64, 1, false>::MAX_D : dh == 48 ? Shape<48, 1, false>::MAX_D : Shape<32, 2, false>::MAX_D)) return false;
   if (a.n_envs < 1 || a.n_envs > 0x7fffffffLL / (BM * 2)) return false;
   if (!aligned16(a.h) || !aligned16(a.wg) || !aligned16(a.bg) || !aligned16(a.out) || (a.ldh % 8) || (a.ldo % 8)) return false;
   if (a.body) {      // one body token + 32 object tokens per env; all rows out, or the body row only
@@ -468,23 +547,26 @@ int attn_block(const AttnBlockArgs& a, cudaStream_t stream) {
   if (!status) return BSRL_ERR_CUDA;
   const int dh = a.d / a.n_heads;
   const int T = a.body ? a.tokens : kT;
+  // Pairs of CTAs where the run is long enough to pay for the cluster start (~2 us) and the projection's width allows it
+  // (M = 256 wants multiples of 32 columns: 144 would compute 16 for nothing, 800 us against 790 at 65,536 envs x 192).
+  const int n_tiles = (int)((a.n_envs + EPT - 1) / EPT);
+  const bool pair = dh != 48 && n_tiles >= 4 * sm_count();
   CUtensorMap tm_h, tm_w;
   if (!make_tmap_env3d(&tm_h, a.h, a.n_envs, T, a.d, a.ldh, 64, EROWS, EPT)) return BSRL_ERR_CUDA;
-  if (!make_tmap_f16(&tm_w, a.wg, 3 * a.d, a.d, a.d, dh == 48 ? Shape<48, 1>::NG : Shape<32, 2>::NG)) return BSRL_ERR_CUDA;
+  if (!make_tmap_f16(&tm_w, a.wg, 3 * a.d, a.d, a.d, dh == 48 ? 144 : pair ? 96 : 192)) return BSRL_ERR_CUDA;
   // all query rows: an env's output for a group is contiguous rows x 128 (two heads of 32) or 96 bytes (one of 48) = one TMA store
   const bool out_tma = a.q_first == 0 && a.n_q == T;
   CUtensorMap tm_o = tm_h;
   if (out_tma && !make_tmap_env3d(&tm_o, a.out, a.n_envs, T, a.d, a.ldo, dh == 48 ? 48 : 64, EROWS, 1)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("attn_block_kernel set-up", [] {
-    const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(attn_block_kernel<32, 2, false>, at, Shape<32, 2>::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_block_kernel<32, 2, true>, at, Shape<32, 2>::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_block_kernel<32, 2, false, true>, at, Shape<32, 2>::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_block_kernel<48, 1, false>, at, Shape<48, 1>::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_block_kernel<48, 1, true>, at, Shape<48, 1>::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_block_kernel<64, 1, false>, at, Shape<64, 1>::SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_block_kernel<64, 1, true>, at, Shape<64, 1>::SMEM_BYTES);
+    cudaError_t e = prepare<32, 2, false, false>();
+    if (e == cudaSuccess) e = prepare<32, 2, true, false>();
+    if (e == cudaSuccess) e = prepare<32, 2, false, true>();
+    if (e == cudaSuccess) e = prepare<48, 1, false, false>();
+    if (e == cudaSuccess) e = prepare<48, 1, true, false>();
+    if (e == cudaSuccess) e = prepare<64, 1, false, false>();
+    if (e == cudaSuccess) e = prepare<64, 1, true, false>();
     return e;
   });
   if (rc != BSRL_OK) return rc;
@@ -493,21 +575,17 @@ int attn_block(const AttnBlockArgs& a, cudaStream_t stream) {
   p.q_first = a.body ? 0 : a.q_first;
   p.n_q = a.body ? EROWS : a.n_q;                 // body-token layout: the tile's query rows are the 32 object tokens
   p.n_envs = a.n_envs;
-  p.n_tiles = (int)((a.n_envs + EPT - 1) / EPT);
+  p.n_tiles = n_tiles;
   p.bias = a.bg; p.key_bias = a.key_bias; p.out = a.out; p.ldo = a.ldo;
   p.v_out = a.v_out; p.v0 = a.v0; p.vres = a.vres;
   p.out_tma = out_tma ? 1 : 0;
   p.tokens = T; p.tok0 = a.body ? 1 : 0; p.body_only = (a.body && a.n_q == 1) ? 1 : 0; p.qkv0 = a.qkv0;
   p.status = status;
-  const int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
   const bool vres = a.v_out || a.v0;
-  if (a.body) launch_kernel(attn_block_kernel<32, 2, false, true>, grid, THREADS, Shape<32, 2>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
-  else if (dh == 32 && !vres) launch_kernel(attn_block_kernel<32, 2, false>, grid, THREADS, Shape<32, 2>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
-  else if (dh == 32) launch_kernel(attn_block_kernel<32, 2, true>, grid, THREADS, Shape<32, 2>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
-  else if (dh == 48 && !vres) launch_kernel(attn_block_kernel<48, 1, false>, grid, THREADS, Shape<48, 1>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
-  else if (dh == 48) launch_kernel(attn_block_kernel<48, 1, true>, grid, THREADS, Shape<48, 1>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
-  else if (!vres) launch_kernel(attn_block_kernel<64, 1, false>, grid, THREADS, Shape<64, 1>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
-  else launch_kernel(attn_block_kernel<64, 1, true>, grid, THREADS, Shape<64, 1>::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
+  auto* run = a.body ? launch<32, 2, false, true> : dh == 32 ? (vres ? launch<32, 2, true, false> : launch<32, 2, false, false>)
+            : dh == 48 ? (vres ? launch<48, 1, true, false> : launch<48, 1, false, false>)
+                       : (vres ? launch<64, 1, true, false> : launch<64, 1, false, false>);
+  run(pair, tm_h, tm_w, tm_o, p, stream);
   BSRL_LAUNCH_OK("attn_block_kernel");
   return BSRL_OK;
 }

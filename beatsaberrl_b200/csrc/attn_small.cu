@@ -139,7 +139,7 @@ __global__ void __launch_bounds__(THREADS) attn_small_kernel(const __grid_consta
   if (p.n_q == 1) {
     if (mt_own != 0) return;
     const float kb_row = lane < kT ? p.key_bias[env * kT + lane] * 1.4426950408889634f : -INFINITY;
-    attend_one_row<DH, LDQ, kT>(sq_g, p.q_first, hh * DH, GD, kb_row, p.out + env * (int64_t)p.ldo + (grp * G + hh) * DH, lane);
+    attend_one_row<DH, LDQ, kT>(sq_g, sq_g + GD * 2, sq_g + 2 * GD * 2, p.q_first, hh * (DH / 8), kb_row, p.out + env * (int64_t)p.ldo + (grp * G + hh) * DH, lane);
     return;
   }
   float kb[4][2];
@@ -150,12 +150,11 @@ __global__ void __launch_bounds__(THREADS) attn_small_kernel(const __grid_consta
       const int key = nt * 8 + tig * 2 + e;
       kb[nt][e] = key < kT ? p.key_bias[env * kT + key] * 1.4426950408889634f : -INFINITY;
     }
-  const uint32_t sq_pair = sq + (p.q_first + mt_own * 16) * LDQ + (hh * DH) * 2, sk_pair = sq + (GD + hh * DH) * 2,
-                 sv_pair = sq + (2 * GD + hh * DH) * 2;
+  const int q_row0 = p.q_first + mt_own * 16, piece0 = hh * (DH / 8);
   __half* out = p.out + (env * p.n_q + mt_own * 16) * (int64_t)p.ldo + (grp * G + hh) * DH;
   const int n_q = p.n_q - mt_own * 16;
-  if (G == 2 && n_q > 16) attend_pair<2, DH, LDQ, GD * 2>(sq_pair, sk_pair, sv_pair, kb, n_q, out, p.ldo, lane, nullptr, 0, 0);
-  else if (n_q > 0) attend_pair<1, DH, LDQ, GD * 2>(sq_pair, sk_pair, sv_pair, kb, n_q, out, p.ldo, lane, nullptr, 0, 0);
+  if (G == 2 && n_q > 16) attend_pair<2, DH, LDQ, GD * 2>(sq, sq + GD * 2, sq + 2 * GD * 2, q_row0, piece0, kb, n_q, out, p.ldo, lane, nullptr, 0, 0);
+  else if (n_q > 0) attend_pair<1, DH, LDQ, GD * 2>(sq, sq + GD * 2, sq + 2 * GD * 2, q_row0, piece0, kb, n_q, out, p.ldo, lane, nullptr, 0, 0);
 }
 
 template <int DH, int G>

@@ -422,3 +422,35 @@ def test_linear_cta_pairs(native, m, n, k, relu, resid, f32):
     ref = ref + r.double() if resid else ref
     tol = 4e-5 if f32 else 2 ** -11
     assert bool(((out.double() - ref).abs() <= tol * ref.abs() + 4e-5).all())
+
+
+@pytest.mark.parametrize("B,d,H,n_q,body", [(2365, 64, 2, 29, 0), (2369, 256, 8, 29, 0), (2373, 256, 8, 5, 0), (2369, 512, 8, 29, 0),
+                                            (2365, 512, 8, 1, 0), (2369, 128, 4, 33, 1), (2365, 256, 8, 1, 1)])
+def test_qkv_attention_cta_pairs(native, B, d, H, n_q, body):
+    """Long runs on CTA pairs (an even and an odd number of 4-env tiles, the last with one env): an env's rows are bit-identical
+    to those of short launches, which run on single CTAs (the same K order, and no sum crosses environments)."""
+    T = 33 if body else 29
+    g = torch.Generator(device="cuda").manual_seed(B + d)
+    h = torch.randn(B * T, d, generator=g, device="cuda").half()
+    w = (torch.randn(3 * d, d, generator=g, device="cuda") * d ** -0.5).half()
+    b = torch.randn(3 * d, generator=g, device="cuda") * 0.2
+    q0 = torch.randn(B, 3 * d, generator=g, device="cuda").half()
+    kb = torch.where(torch.rand(B, T, generator=g, device="cuda") < 0.3, -16384.0, 0.0)
+    kb[:, 0] = 0.0
+
+    def run(lo, hi):
+        out = torch.full(((hi - lo) * n_q, d), float("nan"), dtype=torch.float16, device="cuda")
+        hs, ks, qs = h[lo * T:hi * T].contiguous(), kb[lo:hi].contiguous(), q0[lo:hi].contiguous()
+        if body:
+            rc = native.lib.bsrl_qkv_attention_body(hs.data_ptr(), w.data_ptr(), b.data_ptr(), qs.data_ptr(), ks.data_ptr(),
+                                                    hi - lo, d, H, n_q, out.data_ptr(), _stream())
+        else:
+            rc = native.lib.bsrl_qkv_attention(hs.data_ptr(), w.data_ptr(), b.data_ptr(), ks.data_ptr(), hi - lo, d, H, 0, n_q,
+                                               out.data_ptr(), _stream())
+        native.check(rc)
+        native.check(native.lib.bsrl_device_status())
+        return out
+
+    parts = torch.cat([run(lo, min(lo + 1000, B)) for lo in range(0, B, 1000)])
+    whole = run(0, B)
+    assert not bool(torch.isnan(whole).any()) and torch.equal(whole, parts)
