@@ -10,8 +10,15 @@
 // as ONE kernel.  HBM traffic per token: read att (2d B) + x (4d B), write xo (4d B) + LN rows
 // (2d B each) -- against 18 d^2 FLOP, i.e. tensor-bound.
 //
+// Long runs go to PAIRS of CTAs (cta_group::2): the leader's thread issues M = 256 MMAs over both CTAs' tiles, each CTA
+// fetches half of every weight tile.  These runs sit at the power cap (990 W, 1.5 GHz), so what counts is the bytes moved
+// per row: a tile streams all 9 d^2 weights from L2, 1.2 MB at d = 256, and a pair needs that once for 256 rows.  The half
+// ring leaves room for row buffers of 128-byte rows instead of 64, half as many TMA boxes in the pre-store and the drain.
+// 1.9 M rows, in a loop of seconds, us, single CTAs / pairs / pairs with 128-byte rows: d = 256 2965 / 2823 / 2753,
+// d = 192 2015 / 1933 / 1887.
+//
 // Layout of one CTA (persistent, one per SM, 352 threads):
-//   warp 0       TMA producer of the weight tiles: a 3-stage ring of 32 KB stages, in the MMA's
+//   warp 0       TMA producer of the weight tiles: a 3-stage ring of 32 KB (pair: 16 KB) stages, in the MMA's
 //                consumption order
 //   warp 10      TMA producer of the attention tiles (att tile -> sA, d/64 chunks of [128 x 64], 128B
 //                swizzle; sA is freed before the tile ends); pulls the next tile's residual rows into L2
@@ -19,7 +26,7 @@
 //   warps 2..9   epilogue (two groups of four warps, each group owns half of the columns), thread = row:
 //                LayerNorm on TMEM rows -> h2 into sA; bias + ReLU of each 128-wide hidden chunk -> sH;
 //                final drain and LayerNorm outputs.  Global traffic moves as per-warp TMA boxes (32 rows
-//                x 64 bytes) through three 2 KB swizzled buffers per warp -- residual rows in, fp32 and
+//                x 64 or 128 bytes) through three swizzled buffers per warp -- residual rows in, fp32 and
 //                fp16 rows out; rows gathered through a row map fall back to coalesced loads through
 //                the staging buffer.  The per-column parameters live in shared memory.
 // TMEM (512 columns): region X (d columns) accumulates x1 and then xo in place -- x is
@@ -41,19 +48,27 @@ using namespace tc5;
 
 constexpr int BM = 128;          // rows per tile
 constexpr int HC = 128;          // hidden chunk width
-constexpr int STAGES = 3, STAGE_BYTES = 32768;   // weight ring
-constexpr int RING_BYTES = STAGES * STAGE_BYTES;
+constexpr int STAGES = 3;        // weight ring: stages of 32 KB (in a pair each CTA holds half of their rows)
+template <bool PAIR>
+constexpr int stage_bytes() { return PAIR ? 16384 : 32768; }
 constexpr int CHUNK_BYTES = BM * 64 * 2;   // one [128 x 64] fp16 swizzled chunk
 constexpr int SA_BYTES = 4 * CHUNK_BYTES;  // d <= 256
 constexpr int SH_BYTES = 2 * CHUNK_BYTES;  // one 128 x 128 hidden chunk
 constexpr int EPI_WARPS = 8;                     // two groups of four: each group owns half of the columns
 constexpr int PROD_WARP = 2 + EPI_WARPS;         // attention-tile producer / L2 prefetcher
 constexpr int THREADS = (3 + EPI_WARPS) * 32;
-constexpr int STG_BYTES = 32 * 64;               // per-warp transposition buffer (32 rows x 64 B)
+// row buffers: blocks of 32 rows x 64 bytes, in a pair (whose ring is half as large) x 128 bytes; three per warp, of which
+// one (two) in the staging area and the rest in sH
+template <bool PAIR>
+constexpr int io_bytes() { return PAIR ? 32 * 128 : 32 * 64; }
+template <bool PAIR>
+constexpr int stg_bytes() { return (PAIR ? 2 : 1) * io_bytes<PAIR>(); }
 constexpr int PARAM_FLOATS = 8 * 256 + 1024;     // bo, ln_g, ln_b, b2, g16[2], b16[2] (d each) + b0 (F)
 constexpr int PART_BYTES = 2 * 2 * BM * 8;       // LayerNorm partial sums exchanged between the two groups
-constexpr int SMEM_BYTES = SA_BYTES + SH_BYTES + RING_BYTES + EPI_WARPS * STG_BYTES + PARAM_FLOATS * 4 +
-                           PART_BYTES + 1024 + 256;
+template <bool PAIR>
+constexpr int smem_bytes() {
+  return SA_BYTES + SH_BYTES + STAGES * stage_bytes<PAIR>() + EPI_WARPS * stg_bytes<PAIR>() + PARAM_FLOATS * 4 + PART_BYTES + 1024 + 256;
+}
 constexpr int KERNEL_ID = 2;
 
 struct Shared {
@@ -84,6 +99,7 @@ struct TailParams {
   const float* g16[2];
   const float* b16[2];
   int n_tiles;
+  int wide16;               // 128-byte rows per fp16 output block too (d a multiple of 128; else 64)
   int x_tma;                // residual rows are read with TMA (identity row map)
   int* status;
 };
@@ -107,31 +123,43 @@ __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
     break;                                                         \
   }
 
-// four MMAs (K = 64) of one k-block: A chunk and B tile both [rows x 64] swizzled
-__device__ __forceinline__ void mma_kblock(uint32_t d_tmem, uint32_t a_addr, uint32_t b_addr, uint32_t idesc,
-                                           bool acc_first) {
+// four MMAs (K = 64) of one k-block: A chunk and B tile both [rows x 64] swizzled, from ready-made descriptors;
+// `fresh`: the first one overwrites the accumulator
+template <bool PAIR>
+__device__ __forceinline__ void mma_one(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  if (PAIR) mma_f16_ss_pair(d_tmem, a_desc, b_desc, idesc, accumulate);
+  else mma_f16_ss(d_tmem, a_desc, b_desc, idesc, accumulate);
+}
+template <bool PAIR>
+__device__ __forceinline__ void mma_acc(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
+  if (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.eq.b32 p, 0, 0;\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.eq.b32 p, 0, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
+        : "memory");
+}
+template <bool PAIR>
+__device__ __forceinline__ void mma_kblock_desc(uint32_t d_tmem, uint64_t ad, uint64_t bd, uint32_t idesc, bool fresh) {
+  if (fresh) mma_one<PAIR>(d_tmem, ad, bd, idesc, 0u);
+  else mma_acc<PAIR>(d_tmem, ad, bd, idesc);
+  mma_acc<PAIR>(d_tmem, ad + 2, bd + 2, idesc);
+  mma_acc<PAIR>(d_tmem, ad + 4, bd + 4, idesc);
+  mma_acc<PAIR>(d_tmem, ad + 6, bd + 6, idesc);
+}
+template <bool PAIR>
+__device__ __forceinline__ void mma_kblock(uint32_t d_tmem, uint32_t a_addr, uint32_t b_addr, uint32_t idesc, bool acc_first) {
   const uint64_t ad = smem_desc_sw128(a_addr), bd = smem_desc_sw128(b_addr);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    mma_f16_ss(d_tmem, ad + 2 * k, bd + 2 * k, idesc, (acc_first || k) ? 1u : 0u);
-  }
-}
-
-// the same four MMAs from ready-made descriptors; `fresh`: the first one overwrites the accumulator
-__device__ __forceinline__ void mma_acc(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.eq.b32 p, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc)
-      : "memory");
-}
-__device__ __forceinline__ void mma_kblock_desc(uint32_t d_tmem, uint64_t ad, uint64_t bd, uint32_t idesc, bool fresh) {
-  if (fresh) mma_f16_ss(d_tmem, ad, bd, idesc, 0u);
-  else mma_acc(d_tmem, ad, bd, idesc);
-  mma_acc(d_tmem, ad + 2, bd + 2, idesc);
-  mma_acc(d_tmem, ad + 4, bd + 4, idesc);
-  mma_acc(d_tmem, ad + 6, bd + 6, idesc);
+  for (int k = 0; k < 4; ++k) mma_one<PAIR>(d_tmem, ad + 2 * k, bd + 2 * k, idesc, (acc_first || k) ? 1u : 0u);
 }
 template <int N>
 using StageNo = std::integral_constant<int, N>;
@@ -150,7 +178,7 @@ __device__ __forceinline__ void store_h32(uint8_t* chunks, int row, int col, con
 
 // GELU: the FFN activation is the exact GELU instead of ReLU (a compile-time variant: the hidden-chunk
 // epilogue sits on the chunk loop's critical path)
-template <bool GELU>
+template <bool GELU, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1)
 block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_constant__ CUtensorMap tm_wo,
                   const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w2,
@@ -167,6 +195,9 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
 #define tile0 ((int)blockIdx.x)
 #define tstep (gridDim.x)
 #define t_end (p.n_tiles)
+  constexpr int CTAS = PAIR ? 2 : 1, STAGE_BYTES = stage_bytes<PAIR>(), RING_BYTES = STAGES * STAGE_BYTES;
+  constexpr int STG_BYTES = stg_bytes<PAIR>(), IO_BYTES = io_bytes<PAIR>(), CB = IO_BYTES / 128;   // CB: fp32 columns per block
+  const uint32_t rank = PAIR ? cluster_rank() : 0u;
   const uint32_t sA = base, sH = base + SA_BYTES, ring = sH + SH_BYTES;
   uint8_t* sA_g = gen;
   uint8_t* sH_g = gen + SA_BYTES;
@@ -185,14 +216,14 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
     }
     mbar_init(smem_u32(&sh->a_full), 1);
     mbar_init(smem_u32(&sh->a_free), 1);
-    mbar_init(smem_u32(&sh->x_ready), EPI_WARPS);
+    mbar_init(smem_u32(&sh->x_ready), CTAS * EPI_WARPS);     // *_ready in a pair: both CTAs', at the leader
     mbar_init(smem_u32(&sh->o_done), 1);
-    mbar_init(smem_u32(&sh->h2_ready), EPI_WARPS);
+    mbar_init(smem_u32(&sh->h2_ready), CTAS * EPI_WARPS);
     mbar_init(smem_u32(&sh->x_done), 1);
     mbar_init(smem_u32(&sh->mma_done), 1);
     for (int b = 0; b < 2; ++b) mbar_init(smem_u32(&sh->acc1_full[b]), 1);
     for (int b = 0; b < 2; ++b) {
-      mbar_init(smem_u32(&sh->hid_ready[b]), 4);
+      mbar_init(smem_u32(&sh->hid_ready[b]), CTAS * 4);
       mbar_init(smem_u32(&sh->hid_free[b]), 1);
     }
     for (int w = 0; w < EPI_WARPS; ++w)
@@ -209,8 +240,13 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
     tma_prefetch_desc(&tm_o1);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&sh->tmem_base), 512);
-    tmem_relinquish();
+    if (PAIR) {
+      tmem_alloc_pair(smem_u32(&sh->tmem_base), 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(smem_u32(&sh->tmem_base), 512);
+      tmem_relinquish();
+    }
   }
   // per-column parameters into shared memory: [bo | ln_g | ln_b | b2 | g16_0 | b16_0 | g16_1 | b16_1] (256
   // floats each) then b0 (F floats); absent vectors read as gamma = 1, beta = 0
@@ -227,14 +263,15 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
   for (int i = threadIdx.x; i < p.F; i += THREADS) prm[8 * 256 + i] = p.b0[i];
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();  // the peer's barriers exist before anything is signalled across
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
   // The weight producer depends on no earlier kernel.  The epilogue warps' first work, the residual rows, is the output
   // of a kernel at least two launches back (between two block tails runs at least the attention), which has completed by
   // the time this one may start: they wait after it.
   if (warp == 1 || warp == PROD_WARP) pdl_begin();
-  const int rows_d = d;          // weight rows of an N = d tile
-  const int rows_h = HC;         // ... of an N = 128 tile
+  const int rows_d = d / CTAS;             // this CTA's weight rows of an N = d tile
+  constexpr int rows_h = HC / CTAS;        // ... of an N = 128 tile
 
   if (warp == 0) {
     // ------------------------------------------------------------ weight producer
@@ -247,29 +284,31 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         const uint32_t ph = (it / STAGES) & 1;
         if (!mbar_wait(smem_u32(&sh->w_empty[s]), ph ^ 1, abort)) { give_up(sh, p.status, 1); return false; }
         const uint32_t bar = smem_u32(&sh->w_full[s]);
-        mbar_expect_tx(bar, bytes_each * n_loads);
-        for (int i = 0; i < n_loads; ++i)
-          tma_load_2d(ring + s * STAGE_BYTES + i * bytes_each, map, x0 + i * 64, y0, bar);
+        if (rank == 0) mbar_expect_tx(bar, CTAS * bytes_each * n_loads);     // a pair: both CTAs' bytes, at the leader
+        for (int i = 0; i < n_loads; ++i) {
+          if (PAIR) tma_load_2d_pair(ring + s * STAGE_BYTES + i * bytes_each, map, x0 + i * 64, y0, map_to_cta(bar, 0));
+          else tma_load_2d(ring + s * STAGE_BYTES + i * bytes_each, map, x0 + i * 64, y0, bar);
+        }
         ++it;
         return true;
       };
       auto g1 = [&](int j) -> bool {   // W0 rows [128 j, +128), two k-blocks per stage
         for (int i = 0; i < S1; ++i) {
           const int n = (2 * i + 1 < KB) ? 2 : 1;
-          if (!stage(&tm_w0, 128 * i, HC * j, n, rows_h * 128)) return false;
+          if (!stage(&tm_w0, 128 * i, HC * j + (int)rank * rows_h, n, rows_h * 128)) return false;
         }
         return true;
       };
       for (int t = tile0; t < t_end && ok; t += tstep) {
-        for (int kb = 0; kb < KB && ok; ++kb) ok = stage(&tm_wo, 64 * kb, 0, 1, rows_d * 128);
+        for (int kb = 0; kb < KB && ok; ++kb) ok = stage(&tm_wo, 64 * kb, (int)rank * rows_d, 1, rows_d * 128);
         ok = ok && g1(0) && g1(1);
         for (int j = 0; j < NC && ok; ++j) {
-          for (int kc = 0; kc < 2 && ok; ++kc) ok = stage(&tm_w2, HC * j + 64 * kc, 0, 1, rows_d * 128);
+          for (int kc = 0; kc < 2 && ok; ++kc) ok = stage(&tm_w2, HC * j + 64 * kc, (int)rank * rows_d, 1, rows_d * 128);
           if (ok && j + 2 < NC) ok = g1(j + 2);
         }
       }
-      // loads in flight must land before the CTA exits (bounded, ignoring abort)
-      for (uint32_t j = it > STAGES ? it - STAGES : 0; j < it; ++j) {
+      // loads in flight (a pair's are counted at the leader) must land before the CTA exits (bounded, ignoring abort)
+      for (uint32_t j = it > STAGES ? it - STAGES : 0; rank == 0 && j < it; ++j) {
         uint32_t spins = 0;
         while (!mbar_try_wait(smem_u32(&sh->w_full[j % STAGES]), (j / STAGES) & 1) && ++spins < kSpinLimit) {}
         if (spins >= kSpinLimit) give_up(sh, p.status, 2);
@@ -290,8 +329,11 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
       }
       if (lane == 0) {
         const uint32_t bar = smem_u32(&sh->a_full);
-        mbar_expect_tx(bar, KB * CHUNK_BYTES);
-        for (int c = 0; c < KB; ++c) tma_load_2d(sA + c * CHUNK_BYTES, &tm_att, 64 * c, t * BM, bar);
+        if (rank == 0) mbar_expect_tx(bar, CTAS * KB * CHUNK_BYTES);
+        for (int c = 0; c < KB; ++c) {
+          if (PAIR) tma_load_2d_pair(sA + c * CHUNK_BYTES, &tm_att, 64 * c, t * BM, map_to_cta(bar, 0));
+          else tma_load_2d(sA + c * CHUNK_BYTES, &tm_att, 64 * c, t * BM, bar);
+        }
       }
       const int tn = t + tstep;
       if (tn < t_end) {
@@ -304,19 +346,23 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         }
       }
     }
-    if (lane == 0 && tile_i > 0) {
+    if (lane == 0 && rank == 0 && tile_i > 0) {
       uint32_t spins = 0;
       while (!mbar_try_wait(smem_u32(&sh->a_full), (tile_i - 1) & 1) && ++spins < kSpinLimit) {}
       if (spins >= kSpinLimit) give_up(sh, p.status, 4);
     }
   } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    // ------------------------------------------------------------ MMA issuer (of a pair: the leader's)
+    if (lane == 0 && rank == 0) {
       uint32_t it = 0, tile_i = 0, n_hid = 0;
       bool ok = true;
-      const uint32_t idesc_d = idesc_f16(BM, d), idesc_h = idesc_f16(BM, HC);
+      const uint32_t idesc_d = idesc_f16(CTAS * BM, d), idesc_h = idesc_f16(CTAS * BM, HC);
       // completion of the MMAs issued so far -> the barrier
-      auto commit = [&](uint64_t* bar) { tc_commit(smem_u32(bar)); };
+      auto commit_at = [&](uint32_t bar) {                 // in both CTAs of a pair
+        if (PAIR) tc_commit_pair(bar);
+        else tc_commit(bar);
+      };
+      auto commit = [&](uint64_t* bar) { commit_at(smem_u32(bar)); };
       // consume one ring stage: wait, run `body(stage address)`, release the stage
       auto with_stage = [&](auto&& body) -> bool {
         const int s = it % STAGES;
@@ -336,7 +382,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
       if (KB == 4 && NC == 8) {
         const uint64_t rd0 = smem_desc_sw128(ring), ad0 = smem_desc_sw128(sA), hd0 = smem_desc_sw128(sH);
         const uint32_t wf0 = smem_u32(&sh->w_full[0]), we0 = smem_u32(&sh->w_empty[0]);
-        constexpr uint64_t kSlot = STAGE_BYTES >> 4, kChunk = CHUNK_BYTES >> 4;   // descriptor address units
+        constexpr uint64_t kSlot = STAGE_BYTES >> 4, kChunk = CHUNK_BYTES >> 4, kHalf = rows_h * 128 >> 4;   // descriptor address units
         // wait for ring stage n (tile-relative): slot n % 3, phase (n / 3) & 1
         auto wait_stage = [&](auto n_) -> bool {
           constexpr int n = decltype(n_)::value;
@@ -344,19 +390,19 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           tc_fence_after();
           return true;
         };
-        auto release_stage = [&](auto n_) { tc_commit(we0 + 8u * (decltype(n_)::value % 3)); };
+        auto release_stage = [&](auto n_) { commit_at(we0 + 8u * (decltype(n_)::value % 3)); };
         // FFN-up of one hidden chunk: two stages of two k-blocks each, N = 128
         auto up = [&](auto n_, uint32_t dst, uint64_t* acc1_bar) -> bool {
           constexpr int n = decltype(n_)::value;
           if (!wait_stage(StageNo<n>{})) return false;
-          mma_kblock_desc(dst, ad0, rd0 + kSlot * (n % 3), idesc_h, true);
-          mma_kblock_desc(dst, ad0 + kChunk, rd0 + kSlot * (n % 3) + kChunk, idesc_h, false);
+          mma_kblock_desc<PAIR>(dst, ad0, rd0 + kSlot * (n % 3), idesc_h, true);
+          mma_kblock_desc<PAIR>(dst, ad0 + kChunk, rd0 + kSlot * (n % 3) + kHalf, idesc_h, false);
           release_stage(StageNo<n>{});
           if (!wait_stage(StageNo<n + 1>{})) return false;
-          mma_kblock_desc(dst, ad0 + 2 * kChunk, rd0 + kSlot * ((n + 1) % 3), idesc_h, false);
-          mma_kblock_desc(dst, ad0 + 3 * kChunk, rd0 + kSlot * ((n + 1) % 3) + kChunk, idesc_h, false);
+          mma_kblock_desc<PAIR>(dst, ad0 + 2 * kChunk, rd0 + kSlot * ((n + 1) % 3), idesc_h, false);
+          mma_kblock_desc<PAIR>(dst, ad0 + 3 * kChunk, rd0 + kSlot * ((n + 1) % 3) + kHalf, idesc_h, false);
           release_stage(StageNo<n + 1>{});
-          tc_commit(smem_u32(acc1_bar));
+          commit(acc1_bar);
           return true;
         };
         // FFN-down of one hidden chunk: its two 64-column halves as the epilogue publishes them, N = 256
@@ -364,14 +410,14 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           constexpr int n = decltype(n_)::value;
           if (!mbar_wait(smem_u32(&sh->hid_ready[0]), hid_par, abort)) { give_up(sh, p.status, 9); return false; }
           if (!wait_stage(StageNo<n>{})) return false;
-          mma_kblock_desc(xcol, hd0, rd0 + kSlot * (n % 3), idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, hd0, rd0 + kSlot * (n % 3), idesc_d, false);
           release_stage(StageNo<n>{});
-          tc_commit(smem_u32(&sh->hid_free[0]));
+          commit(&sh->hid_free[0]);
           if (!mbar_wait(smem_u32(&sh->hid_ready[1]), hid_par, abort)) { give_up(sh, p.status, 9); return false; }
           if (!wait_stage(StageNo<n + 1>{})) return false;
-          mma_kblock_desc(xcol, hd0 + kChunk, rd0 + kSlot * ((n + 1) % 3), idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, hd0 + kChunk, rd0 + kSlot * ((n + 1) % 3), idesc_d, false);
           release_stage(StageNo<n + 1>{});
-          tc_commit(smem_u32(&sh->hid_free[1]));
+          commit(&sh->hid_free[1]);
           return true;
         };
         for (int t = tile0; t < t_end && ok; t += tstep, ++tile_i) {
@@ -384,19 +430,19 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           // x1 = x (pre-stored) + att Wo^T: stages 0..3
           ok = wait_stage(StageNo<0>{});
           if (!ok) break;
-          mma_kblock_desc(xcol, ad0, rd0, idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, ad0, rd0, idesc_d, false);
           release_stage(StageNo<0>{});
           ok = wait_stage(StageNo<1>{});
           if (!ok) break;
-          mma_kblock_desc(xcol, ad0 + kChunk, rd0 + kSlot, idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, ad0 + kChunk, rd0 + kSlot, idesc_d, false);
           release_stage(StageNo<1>{});
           ok = wait_stage(StageNo<2>{});
           if (!ok) break;
-          mma_kblock_desc(xcol, ad0 + 2 * kChunk, rd0 + 2 * kSlot, idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, ad0 + 2 * kChunk, rd0 + 2 * kSlot, idesc_d, false);
           release_stage(StageNo<2>{});
           ok = wait_stage(StageNo<3>{});
           if (!ok) break;
-          mma_kblock_desc(xcol, ad0 + 3 * kChunk, rd0, idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, ad0 + 3 * kChunk, rd0, idesc_d, false);
           release_stage(StageNo<3>{});
           commit(&sh->o_done);
           TAIL_WAIT(&sh->h2_ready, par, 8);
@@ -423,7 +469,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         // ring, an odd number: the slots repeat from tile to tile, the phases alternate with the tile's parity
         const uint64_t rd0 = smem_desc_sw128(ring), ad0 = smem_desc_sw128(sA), hd0 = smem_desc_sw128(sH);
         const uint32_t wf0 = smem_u32(&sh->w_full[0]), we0 = smem_u32(&sh->w_empty[0]);
-        constexpr uint64_t kSlot = STAGE_BYTES >> 4, kChunk = CHUNK_BYTES >> 4;   // descriptor address units
+        constexpr uint64_t kSlot = STAGE_BYTES >> 4, kChunk = CHUNK_BYTES >> 4, kHalf = rows_h * 128 >> 4;   // descriptor address units
         uint32_t flip = 0;                                          // tile parity: phase of stage n is ((n / 3) & 1) ^ flip
         auto wait_stage = [&](auto n_) -> bool {
           constexpr int n = decltype(n_)::value;
@@ -431,32 +477,32 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           tc_fence_after();
           return true;
         };
-        auto release_stage = [&](auto n_) { tc_commit(we0 + 8u * (decltype(n_)::value % 3)); };
+        auto release_stage = [&](auto n_) { commit_at(we0 + 8u * (decltype(n_)::value % 3)); };
         // FFN-up of one hidden chunk: k-blocks 0 and 1 from one stage, k-block 2 from the next, N = 128
         auto up = [&](auto n_, uint32_t dst, uint64_t* acc1_bar) -> bool {
           constexpr int n = decltype(n_)::value;
           if (!wait_stage(StageNo<n>{})) return false;
-          mma_kblock_desc(dst, ad0, rd0 + kSlot * (n % 3), idesc_h, true);
-          mma_kblock_desc(dst, ad0 + kChunk, rd0 + kSlot * (n % 3) + kChunk, idesc_h, false);
+          mma_kblock_desc<PAIR>(dst, ad0, rd0 + kSlot * (n % 3), idesc_h, true);
+          mma_kblock_desc<PAIR>(dst, ad0 + kChunk, rd0 + kSlot * (n % 3) + kHalf, idesc_h, false);
           release_stage(StageNo<n>{});
           if (!wait_stage(StageNo<n + 1>{})) return false;
-          mma_kblock_desc(dst, ad0 + 2 * kChunk, rd0 + kSlot * ((n + 1) % 3), idesc_h, false);
+          mma_kblock_desc<PAIR>(dst, ad0 + 2 * kChunk, rd0 + kSlot * ((n + 1) % 3), idesc_h, false);
           release_stage(StageNo<n + 1>{});
-          tc_commit(smem_u32(acc1_bar));
+          commit(acc1_bar);
           return true;
         };
         auto down = [&](auto n_, uint32_t xcol, uint32_t hid_par) -> bool {
           constexpr int n = decltype(n_)::value;
           if (!mbar_wait(smem_u32(&sh->hid_ready[0]), hid_par, abort)) { give_up(sh, p.status, 9); return false; }
           if (!wait_stage(StageNo<n>{})) return false;
-          mma_kblock_desc(xcol, hd0, rd0 + kSlot * (n % 3), idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, hd0, rd0 + kSlot * (n % 3), idesc_d, false);
           release_stage(StageNo<n>{});
-          tc_commit(smem_u32(&sh->hid_free[0]));
+          commit(&sh->hid_free[0]);
           if (!mbar_wait(smem_u32(&sh->hid_ready[1]), hid_par, abort)) { give_up(sh, p.status, 9); return false; }
           if (!wait_stage(StageNo<n + 1>{})) return false;
-          mma_kblock_desc(xcol, hd0 + kChunk, rd0 + kSlot * ((n + 1) % 3), idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, hd0 + kChunk, rd0 + kSlot * ((n + 1) % 3), idesc_d, false);
           release_stage(StageNo<n + 1>{});
-          tc_commit(smem_u32(&sh->hid_free[1]));
+          commit(&sh->hid_free[1]);
           return true;
         };
         for (int t = tile0; t < t_end && ok; t += tstep, ++tile_i) {
@@ -470,15 +516,15 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           // x1 = x (pre-stored) + att Wo^T: stages 0..2
           ok = wait_stage(StageNo<0>{});
           if (!ok) break;
-          mma_kblock_desc(xcol, ad0, rd0, idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, ad0, rd0, idesc_d, false);
           release_stage(StageNo<0>{});
           ok = wait_stage(StageNo<1>{});
           if (!ok) break;
-          mma_kblock_desc(xcol, ad0 + kChunk, rd0 + kSlot, idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, ad0 + kChunk, rd0 + kSlot, idesc_d, false);
           release_stage(StageNo<1>{});
           ok = wait_stage(StageNo<2>{});
           if (!ok) break;
-          mma_kblock_desc(xcol, ad0 + 2 * kChunk, rd0 + 2 * kSlot, idesc_d, false);
+          mma_kblock_desc<PAIR>(xcol, ad0 + 2 * kChunk, rd0 + 2 * kSlot, idesc_d, false);
           release_stage(StageNo<2>{});
           commit(&sh->o_done);
           TAIL_WAIT(&sh->h2_ready, par, 8);
@@ -505,8 +551,8 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           const uint32_t dst = acol + (j & 1) * HC;
           for (int i = 0; i < S1; ++i) {
             if (!with_stage([&](uint32_t st) {
-                  mma_kblock(dst, sA + (2 * i) * CHUNK_BYTES, st, idesc_h, i != 0);
-                  if (2 * i + 1 < KB) mma_kblock(dst, sA + (2 * i + 1) * CHUNK_BYTES, st + rows_h * 128, idesc_h, true);
+                  mma_kblock<PAIR>(dst, sA + (2 * i) * CHUNK_BYTES, st, idesc_h, i != 0);
+                  if (2 * i + 1 < KB) mma_kblock<PAIR>(dst, sA + (2 * i + 1) * CHUNK_BYTES, st + rows_h * 128, idesc_h, true);
                 }))
               return false;
           }
@@ -517,7 +563,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         TAIL_WAIT(&sh->x_ready, par, 7);
         tc_fence_after();
         for (int kb = 0; kb < KB && ok; ++kb)       // x1 = x (pre-stored) + att Wo^T
-          ok = with_stage([&](uint32_t st) { mma_kblock(xcol, sA + kb * CHUNK_BYTES, st, idesc_d, true); });
+          ok = with_stage([&](uint32_t st) { mma_kblock<PAIR>(xcol, sA + kb * CHUNK_BYTES, st, idesc_d, true); });
         if (!ok) break;
         commit(&sh->o_done);
         TAIL_WAIT(&sh->h2_ready, par, 8);
@@ -528,7 +574,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           for (int kc = 0; kc < 2 && ok; ++kc) {    // xo += hidden chunk j * W2[:, chunk j]^T, one 64-column half at a time
             if (!mbar_wait(smem_u32(&sh->hid_ready[kc]), n_hid & 1, abort)) { give_up(sh, p.status, 9); ok = false; break; }
             tc_fence_after();
-            ok = with_stage([&](uint32_t st) { mma_kblock(xcol, sH + kc * CHUNK_BYTES, st, idesc_d, true); });
+            ok = with_stage([&](uint32_t st) { mma_kblock<PAIR>(xcol, sH + kc * CHUNK_BYTES, st, idesc_d, true); });
             if (ok) commit(&sh->hid_free[kc]);   // this half of sH may be overwritten once retired
           }
           ++n_hid;
@@ -563,24 +609,27 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
     bool ok = true;
     const float inv_d = 1.0f / (float)d;
 
-    // Three 2 KB transposition buffers per warp (32 rows x 64 B, 64-byte swizzle -- the layout of the
-    // 64-byte-wide TMA boxes): its slice of the staging area and, while no hidden chunk is live (from
-    // the tile's last FFN-down MMA to the next tile's first hidden chunk), 4 KB of sH.
-    auto io_buf = [&](int b) -> uint8_t* { return b == 0 ? stg : sH_g + (warp - 2) * 4096 + (b - 1) * 2048; };
-    auto buf_write = [&](uint8_t* buf, int row, int pc, uint4 v) {   // 16-byte piece pc (0..3) of row
-      *reinterpret_cast<uint4*>(buf + row * 64 + ((pc ^ ((row >> 1) & 3)) << 4)) = v;
+    // Three row buffers per warp (32 rows, swizzled -- the layout of the TMA boxes): its slice of the staging area and,
+    // while no hidden chunk is live (from the tile's last FFN-down MMA to the next tile's first hidden chunk), 4 KB of sH.
+    auto io_buf = [&](int b) -> uint8_t* {
+      uint8_t* in_h = sH_g + (warp - 2) * 4096;
+      return PAIR ? (b < 2 ? stg + b * IO_BYTES : in_h) : b == 0 ? stg : in_h + (b - 1) * IO_BYTES;
     };
-    auto buf_read = [&](const uint8_t* buf, int row, int pc) -> uint4 {
-      return *reinterpret_cast<const uint4*>(buf + row * 64 + ((pc ^ ((row >> 1) & 3)) << 4));
-    };
-    auto stg_write = [&](int row, int pc, uint4 v) { buf_write(stg, row, pc, v); };
-    auto stg_read = [&](int row, int pc) -> uint4 { return buf_read(stg, row, pc); };
+    // 16-byte piece pc of row: rows of 64 bytes (pc 0..3) or 128 (pc 0..7)
+    auto at64 = [](int row, int pc) -> int { return row * 64 + ((pc ^ ((row >> 1) & 3)) << 4); };
+    auto at128 = [](int row, int pc) -> int { return row * 128 + ((pc ^ (row & 7)) << 4); };
+    auto io_at = [&](int row, int pc) -> int { return PAIR ? at128(row, pc) : at64(row, pc); };
+    auto stg_write = [&](int row, int pc, uint4 v) { *reinterpret_cast<uint4*>(stg + at64(row, pc)) = v; };
+    auto stg_read = [&](int row, int pc) -> uint4 { return *reinterpret_cast<const uint4*>(stg + at64(row, pc)); };
     uint32_t n_io = 0;                                      // residual blocks this warp has consumed so far
     auto group_sync = [&]() { asm volatile("bar.sync 2, %0;" ::"n"(EPI_WARPS * 32) : "memory"); };
     auto signal = [&](uint64_t* bar) {   // one arrival per warp, after everyone's writes
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(bar));
+      if (lane == 0) {
+        if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(bar), 0));
+        else mbar_arrive(smem_u32(bar));
+      }
     };
     // shared-memory writes of this thread -> visible to the tensor core (the all-state-space form of
     // the fence measured ~2,000 cycles per use and is not needed for this CTA's own shared memory)
@@ -634,17 +683,17 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
       }
       tmem_wait_st();
     };
-    // (b) dense rows: 16-column blocks of this warp's 32 rows arrive by TMA in the three buffers, up to
+    // (b) dense rows: CB-column blocks of this warp's 32 rows arrive by TMA in the three buffers, up to
     // three in flight; block n (counted over the whole kernel) uses buffer n % 3, phase (n / 3) & 1
     auto prestore_tma = [&](int t, uint32_t col0) -> bool {
       const int row0 = t * BM + q * 32;
-      const int nb = dh2 >> 4;
+      const int nb = dh2 / CB;
       auto issue = [&](int k) {                             // k-th block of this call
         if (lane == 0) {
           const uint32_t n = n_io + k;
           const uint32_t bar = smem_u32(&sh->io_full[warp - 2][n % 3]);
-          mbar_expect_tx(bar, STG_BYTES);
-          tma_load_2d(smem_u32(io_buf(n % 3)), &tm_x, c_lo + 16 * k, row0, bar);
+          mbar_expect_tx(bar, IO_BYTES);
+          tma_load_2d(smem_u32(io_buf(n % 3)), &tm_x, c_lo + CB * k, row0, bar);
         }
       };
       for (int k = 0; k < 3 && k < nb; ++k) issue(k);
@@ -652,7 +701,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
       for (int c = c_lo; c < c_lo + dh2; c += 32) {
         uint32_t r[32];
 #pragma unroll
-        for (int hb = 0; hb < 2; ++hb, ++k) {
+        for (int hb = 0; hb < 32 / CB; ++hb, ++k) {
           const uint32_t n = n_io + k;
           if (!mbar_wait_warp(smem_u32(&sh->io_full[warp - 2][n % 3]), (n / 3) & 1, abort)) {
             if (lane == 0) give_up(sh, p.status, 15);
@@ -660,13 +709,13 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           }
           const uint8_t* buf = io_buf(n % 3);
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const uint4 v = buf_read(buf, lane, j);
-            const float4 bo = P_bo[((c + 16 * hb) >> 2) + j];
-            r[16 * hb + 4 * j] = __float_as_uint(__uint_as_float(v.x) + bo.x);
-            r[16 * hb + 4 * j + 1] = __float_as_uint(__uint_as_float(v.y) + bo.y);
-            r[16 * hb + 4 * j + 2] = __float_as_uint(__uint_as_float(v.z) + bo.z);
-            r[16 * hb + 4 * j + 3] = __float_as_uint(__uint_as_float(v.w) + bo.w);
+          for (int j = 0; j < CB / 4; ++j) {
+            const uint4 v = *reinterpret_cast<const uint4*>(buf + io_at(lane, j));
+            const float4 bo = P_bo[((c + CB * hb) >> 2) + j];
+            r[CB * hb + 4 * j] = __float_as_uint(__uint_as_float(v.x) + bo.x);
+            r[CB * hb + 4 * j + 1] = __float_as_uint(__uint_as_float(v.y) + bo.y);
+            r[CB * hb + 4 * j + 2] = __float_as_uint(__uint_as_float(v.z) + bo.z);
+            r[CB * hb + 4 * j + 3] = __float_as_uint(__uint_as_float(v.w) + bo.w);
           }
           __syncwarp();                                     // everyone has read the buffer: refill it
           if (k + 3 < nb) issue(k + 3);
@@ -800,7 +849,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           }
           return io_buf(n_st % 3);
         };
-        // the warp's writes to the buffer -> one TMA store of 32 rows x 64 bytes (rows >= M are clipped)
+        // the warp's writes to the buffer -> one TMA store of its 32 rows (rows >= M are clipped)
         auto store_block = [&](const CUtensorMap* map, int x) {
           fence_proxy_async_smem();
           __syncwarp();
@@ -816,20 +865,19 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
             tmem_ld32(lane_base + xcol + c, r);
             tmem_wait_ld();
 #pragma unroll
-            for (int hb = 0; hb < 2; ++hb) {
+            for (int hb = 0; hb < 32 / CB; ++hb) {
               uint8_t* buf = p.x_out ? next_buf() : nullptr;
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const float4 b2 = P_b2[((c + 16 * hb) >> 2) + j];
-                float4 v = make_float4(__uint_as_float(r[16 * hb + 4 * j]) + b2.x, __uint_as_float(r[16 * hb + 4 * j + 1]) + b2.y,
-                                       __uint_as_float(r[16 * hb + 4 * j + 2]) + b2.z, __uint_as_float(r[16 * hb + 4 * j + 3]) + b2.w);
+              for (int j = 0; j < CB / 4; ++j) {
+                const uint32_t* a = r + CB * hb + 4 * j;
+                const float4 b2 = P_b2[((c + CB * hb) >> 2) + j];
+                float4 v = make_float4(__uint_as_float(a[0]) + b2.x, __uint_as_float(a[1]) + b2.y, __uint_as_float(a[2]) + b2.z,
+                                       __uint_as_float(a[3]) + b2.w);
                 sum += (v.x + v.y) + (v.z + v.w);
                 sq = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sq))));
-                if (p.x_out)
-                  buf_write(buf, lane, j, make_uint4(__float_as_uint(v.x), __float_as_uint(v.y), __float_as_uint(v.z),
-                                                     __float_as_uint(v.w)));
+                if (p.x_out) *reinterpret_cast<float4*>(buf + io_at(lane, j)) = v;
               }
-              if (p.x_out) store_block(&tm_xo, c + 16 * hb);
+              if (p.x_out) store_block(&tm_xo, c + CB * hb);
             }
           }
         }
@@ -842,11 +890,14 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           const float sc = ln ? rstd : 1.f, sh0 = ln ? -mean * rstd : 0.f;
           const float4 *P_go = prm4 + 256 + 128 * o, *P_bo16 = prm4 + 320 + 128 * o;
           const CUtensorMap* tm_o = o ? &tm_o1 : &tm_o0;
-          for (int c = c_lo; c < c_lo + dh2; c += 32) {     // 32 columns = 64 bytes of fp16 per row
+          const bool wide = PAIR && p.wide16;
+          uint8_t* buf = nullptr;
+          for (int c = c_lo; c < c_lo + dh2; c += 32) {     // 32 columns = 64 bytes of fp16 per row: a block, or half of one
             uint32_t r[32];
             tmem_ld32(lane_base + xcol + c, r);
             tmem_wait_ld();
-            uint8_t* buf = next_buf();
+            const int half = wide ? ((c - c_lo) >> 5) & 1 : 0;
+            if (half == 0) buf = next_buf();
 #pragma unroll
             for (int j = 0; j < 4; ++j) {                   // 8 columns -> one 16-byte fp16 piece
               float y[8];
@@ -859,10 +910,10 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
                 y[4 * e + 2] = fmaf(fmaf(__uint_as_float(r[8 * j + 4 * e + 2]) + b2.z, sc, sh0), g.z, bb.z);
                 y[4 * e + 3] = fmaf(fmaf(__uint_as_float(r[8 * j + 4 * e + 3]) + b2.w, sc, sh0), g.w, bb.w);
               }
-              buf_write(buf, lane, j, make_uint4(pack_half2(y[0], y[1]), pack_half2(y[2], y[3]),
-                                                 pack_half2(y[4], y[5]), pack_half2(y[6], y[7])));
+              *reinterpret_cast<uint4*>(buf + (wide ? at128(lane, 4 * half + j) : at64(lane, j))) =
+                  make_uint4(pack_half2(y[0], y[1]), pack_half2(y[2], y[3]), pack_half2(y[4], y[5]), pack_half2(y[6], y[7]));
             }
-            store_block(tm_o, c);
+            if (!wide || half == 1) store_block(tm_o, c - 32 * half);
           }
         }
         // the buffers (two of them inside sH) are reused by the next tile: all stores have read them
@@ -877,9 +928,11 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync_all();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, 512);
+    if (PAIR) tmem_dealloc_pair(tmem_base, 512);
+    else tmem_dealloc(tmem_base, 512);
   }
 }
 #undef tile0
@@ -910,24 +963,34 @@ int block_tail(const BlockTailArgs& a, cudaStream_t stream) {
   int* status = device_status_ptr();
   if (!status) return BSRL_ERR_CUDA;
   const int n_tiles = (int)((a.M + BM - 1) / BM);
+  // pairs from four waves on: below, the cluster start (~2 us) costs more than half of the weight traffic
+  const bool pair = n_tiles >= 4 * sm_count() && a.M <= 0x7ffffe00;
+  const int ctas = pair ? 2 : 1;
   CUtensorMap tm_att, tm_wo, tm_w0, tm_w2;
   if (!make_tmap_f16(&tm_att, a.att, a.M, a.d, a.ld_att, BM)) return BSRL_ERR_CUDA;
-  if (!make_tmap_f16(&tm_wo, a.wo, a.d, a.d, a.d, a.d)) return BSRL_ERR_CUDA;
-  if (!make_tmap_f16(&tm_w0, a.w0, a.F, a.d, a.d, HC)) return BSRL_ERR_CUDA;
-  if (!make_tmap_f16(&tm_w2, a.w2, a.d, a.F, a.F, a.d)) return BSRL_ERR_CUDA;
-  // residual rows in and the outputs move as 32-row x 64-byte TMA boxes; a map that is not needed
+  if (!make_tmap_f16(&tm_wo, a.wo, a.d, a.d, a.d, a.d / ctas)) return BSRL_ERR_CUDA;
+  if (!make_tmap_f16(&tm_w0, a.w0, a.F, a.d, a.d, HC / ctas)) return BSRL_ERR_CUDA;
+  if (!make_tmap_f16(&tm_w2, a.w2, a.d, a.F, a.F, a.d / ctas)) return BSRL_ERR_CUDA;
+  // residual rows in and the outputs move as 32-row TMA boxes of 64 or 128 bytes a row; a map that is not needed
   // aliases the attention tile's (the kernel only prefetches its descriptor)
   const bool x_tma = a.xmap.group == 0x7fffffff && a.xmap.stride == 0 && a.xmap.first == 0;
   CUtensorMap tm_x = tm_att, tm_xo = tm_att, tm_o[2] = {tm_att, tm_att};
-  if (x_tma && !make_tmap_rows64(&tm_x, a.x, 4, a.M, a.d, a.ldx, 32)) return BSRL_ERR_CUDA;
-  if (a.x_out && !make_tmap_rows64(&tm_xo, a.x_out, 4, a.M, a.d, a.d, 32)) return BSRL_ERR_CUDA;
+  const bool wide16 = pair && a.d % 128 == 0;
+  auto rows_map = [&](CUtensorMap* map, const void* base, int elem, int64_t ld, bool wide) {
+    return wide ? make_tmap_rows(map, base, elem, a.M, a.d, ld, 32, 128) : make_tmap_rows64(map, base, elem, a.M, a.d, ld, 32);
+  };
+  if (x_tma && !rows_map(&tm_x, a.x, 4, a.ldx, pair)) return BSRL_ERR_CUDA;
+  if (a.x_out && !rows_map(&tm_xo, a.x_out, 4, a.d, pair)) return BSRL_ERR_CUDA;
   for (int o = 0; o < 2; ++o)
-    if (a.out16[o] && !make_tmap_rows64(&tm_o[o], a.out16[o], 2, a.M, a.d, a.ld16[o], 32)) return BSRL_ERR_CUDA;
+    if (a.out16[o] && !rows_map(&tm_o[o], a.out16[o], 2, a.ld16[o], wide16)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("block_tail_kernel set-up", [] {
-    cudaError_t e = cudaFuncSetAttribute(block_tail_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(block_tail_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(block_tail_kernel<false, false>, at, smem_bytes<false>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(block_tail_kernel<true, false>, at, smem_bytes<false>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(block_tail_kernel<false, true>, at, smem_bytes<true>());
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(block_tail_kernel<true, true>, at, smem_bytes<true>());
+    return e;
   });
   if (rc != BSRL_OK) return rc;
   TailParams p;
@@ -938,12 +1001,16 @@ int block_tail(const BlockTailArgs& a, cudaStream_t stream) {
   for (int o = 0; o < 2; ++o) {
     p.out16[o] = a.out16[o]; p.ld16[o] = a.ld16[o]; p.g16[o] = a.g16[o]; p.b16[o] = a.b16[o];
   }
-  p.n_tiles = n_tiles;
+  p.n_tiles = pair ? (n_tiles + 1) & ~1 : n_tiles;     // both CTAs of a pair take the same number of tiles
+  p.wide16 = wide16 ? 1 : 0;
   p.x_tma = x_tma ? 1 : 0;
   p.status = status;
-  int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
-  if (a.gelu) launch_kernel(block_tail_kernel<true>, grid, THREADS, SMEM_BYTES, stream, tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
-  else launch_kernel(block_tail_kernel<false>, grid, THREADS, SMEM_BYTES, stream, tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
+  if (pair)
+    launch_kernel<2>(a.gelu ? block_tail_kernel<true, true> : block_tail_kernel<false, true>, sm_count() & ~1, THREADS, smem_bytes<true>(), stream,
+                     tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
+  else
+    launch_kernel(a.gelu ? block_tail_kernel<true, false> : block_tail_kernel<false, false>, p.n_tiles < sm_count() ? p.n_tiles : sm_count(), THREADS,
+                  smem_bytes<false>(), stream, tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
   BSRL_LAUNCH_OK("block_tail_kernel");
   return BSRL_OK;
 }

@@ -454,3 +454,28 @@ def test_qkv_attention_cta_pairs(native, B, d, H, n_q, body):
     parts = torch.cat([run(lo, min(lo + 1000, B)) for lo in range(0, B, 1000)])
     whole = run(0, B)
     assert not bool(torch.isnan(whole).any()) and torch.equal(whole, parts)
+
+
+@pytest.mark.parametrize("m,d,f", [(75713, 256, 1024), (75777, 192, 768), (75777, 64, 256), (75900, 128, 512)])
+def test_block_tail_cta_pairs(native, m, d, f):
+    """Long runs on CTA pairs (an even and an odd number of 128-row tiles): every row is bit-identical to short launches,
+    which run on single CTAs (the same K order, and no sum crosses rows)."""
+    g = torch.Generator(device="cuda").manual_seed(m + d)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda")  # noqa: E731
+    att, x = rnd(m, d).half(), rnd(m, d) * 2
+    wo, w0, w2 = (rnd(d, d) / d ** 0.5).half(), (rnd(f, d) / d ** 0.5).half(), (rnd(d, f) / f ** 0.5).half()
+    bo, b0, b2, lb, ob = rnd(d) * 0.1, rnd(f) * 0.1, rnd(d) * 0.1, rnd(d) * 0.1, rnd(d) * 0.1
+    lg, og = 1 + 0.1 * rnd(d), 1 + 0.1 * rnd(d)
+
+    def run(lo, hi):
+        x_out = torch.full((hi - lo, d), float("nan"), device="cuda")
+        h = torch.full((hi - lo, d), float("nan"), dtype=torch.float16, device="cuda")
+        native.check(native.lib.bsrl_block_tail(
+            att[lo:].data_ptr(), x[lo:].data_ptr(), wo.data_ptr(), bo.data_ptr(), lg.data_ptr(), lb.data_ptr(), w0.data_ptr(), b0.data_ptr(),
+            w2.data_ptr(), b2.data_ptr(), 1e-5, hi - lo, d, f, x_out.data_ptr(), h.data_ptr(), og.data_ptr(), ob.data_ptr(), _stream()))
+        native.check(native.lib.bsrl_device_status())
+        return x_out, h
+
+    parts = [torch.cat(t) for t in zip(*(run(lo, min(lo + 32768, m)) for lo in range(0, m, 32768)))]
+    for whole, part in zip(run(0, m), parts):
+        assert not bool(torch.isnan(whole).any()) and torch.equal(whole, part)
