@@ -163,6 +163,25 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
     }
 }
 
+// One row block of a warp's shared-memory tile (rows LDS halves apart, DH used) -> rows of `out`, 16 bytes per lane: a row's
+// sectors are written once and whole.  (Straight from the accumulator fragments a store covers 16 bytes of each of 8 rows.)
+// wide: out and ldo allow 16-byte stores
+template <int DH, int LDS>
+__device__ __forceinline__ void copy_rows_out(const __half* s, int n_rows, __half* out, int64_t ldo, bool wide, int lane) {
+  constexpr int CH = DH / 8;
+  for (int c = lane; c < n_rows * CH; c += 32) {
+    const int row = c / CH, ch = c % CH;
+    const uint4 v = *reinterpret_cast<const uint4*>(s + row * LDS + ch * 8);
+    __half* o = out + row * ldo + ch * 8;
+    if (wide) {
+      *reinterpret_cast<uint4*>(o) = v;
+    } else {
+      uint32_t* o32 = reinterpret_cast<uint32_t*>(o);
+      o32[0] = v.x; o32[1] = v.y; o32[2] = v.z; o32[3] = v.w;
+    }
+  }
+}
+
 // One query row of an env on the CUDA cores (lane = key for the scores, lane = output column for the weighted sum):
 // row q_row of section sq (as in attend_pair, generic pointers) against the NKEYS rows of sk and sv, the head's columns
 // from piece0; kb_row: this lane's key bias in base 2, -inf past the last key.

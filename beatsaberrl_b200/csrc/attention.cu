@@ -13,6 +13,7 @@
 // (python/policy.py:686-690).  The kernel is not tied to (T, d, H) = (29, 192, 4): head_dim
 // 32, 48 or 64, any head count.
 #include "kernels.cuh"
+#include "attend.cuh"
 
 namespace bsrl {
 namespace {
@@ -46,19 +47,15 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
     __syncwarp();
     // stage q (query rows), k, v; rows past the live range are zero
     for (int c = lane; c < kRows * CH; c += 32) {
-      int row = c / CH, ch = c % CH;
-      uint4 zq = make_uint4(0, 0, 0, 0), zk = zq, zv = zq;
-      if (row < n_q)
-        zq = *reinterpret_cast<const uint4*>(base + (int64_t)(q_first + row) * ld + ch * 8);
-      if (row < tokens) {
-        const __half* r = base + (int64_t)row * ld + ch * 8;
-        zk = *reinterpret_cast<const uint4*>(r + d);
-        zv = *reinterpret_cast<const uint4*>(r + 2 * d);
-      }
-      *reinterpret_cast<uint4*>(sq + row * LDS + ch * 8) = zq;
-      *reinterpret_cast<uint4*>(sk + row * LDS + ch * 8) = zk;
-      *reinterpret_cast<uint4*>(sv + row * LDS + ch * 8) = zv;
+      const int row = c / CH, ch = c % CH;
+      const bool live = row < tokens, asks = row < n_q;
+      const __half* r = base + (int64_t)(live ? row : 0) * ld + ch * 8;
+      const uint32_t at = (row * LDS + ch * 8) * 2;
+      cp_async16(sq_u + at, base + (int64_t)(asks ? q_first + row : 0) * ld + ch * 8, asks);
+      cp_async16(sk_u + at, r + d, live);
+      cp_async16(sv_u + at, r + 2 * d, live);
     }
+    cp_async_commit();
     // key bias of the 8 key columns this lane sees: keys nt*8 + tig*2 + {0,1}
     float kb[NT][2];
 #pragma unroll
@@ -68,6 +65,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
         int key = nt * 8 + tig * 2 + e;
         kb[nt][e] = key < tokens ? key_bias[env * tokens + key] : -INFINITY;
       }
+    cp_async_wait<0>();
     __syncwarp();
 
     for (int mt = 0; mt < m_tiles; ++mt) {
@@ -142,17 +140,16 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
           mma_f16(o[2 * j + 1], pa[ks], b[2], b[3]);
         }
       }
+      // the output takes the place of the query rows it came from
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        int qrow = mt * 16 + g + r * 8;
-        if (qrow < n_q) {
-          __half* orow = out + (env * n_q + qrow) * (int64_t)ldo + head * DH + tig * 2;
+        __half* orow = sq + (mt * 16 + g + r * 8) * LDS + tig * 2;
 #pragma unroll
-          for (int nt = 0; nt < DH / 8; ++nt)
-            *reinterpret_cast<uint32_t*>(orow + nt * 8) = pack_half2(o[nt][r * 2], o[nt][r * 2 + 1]);
-        }
+        for (int nt = 0; nt < DH / 8; ++nt) *reinterpret_cast<uint32_t*>(orow + nt * 8) = pack_half2(o[nt][r * 2], o[nt][r * 2 + 1]);
       }
     }
+    __syncwarp();
+    copy_rows_out<DH, LDS>(sq, n_q, out + env * n_q * (int64_t)ldo + head * DH, ldo, true, lane);
   }
 }
 
@@ -166,7 +163,9 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
 // n_q = tokens (every row) or 1 (the body row only: the last block's readout).  Same arithmetic as
 // attn29_kernel: fp32 scores and softmax, masked keys exactly 0, probabilities rounded to fp16 only where
 // they enter an MMA.
-template <int DH, int NOBJ, int WARPS>
+// TEAM: warps per (env, head) -- two where the pair's tile is so large (28 KB at 64 tokens x 64) that one warp each left two
+// per scheduler; each takes half of the object query rows and of the body row's output columns.
+template <int DH, int NOBJ, int WARPS, int TEAM>
 __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __restrict__ qkv, int ld,
                                                               const float* __restrict__ key_bias, int64_t n_pairs,
                                                               int d, int n_heads, int n_q, __half* __restrict__ out, int ldo) {
@@ -174,38 +173,47 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
   constexpr int T = NOBJ + 1, NT = NOBJ / 8, KS = NOBJ / 16, MT = NOBJ / 16;
   constexpr int LDS = DH + 8, CH = DH / 8;
   constexpr int PER = (NOBJ + 31) / 32;              // object rows per lane in the lane-per-row passes
+  static_assert(TEAM == 1 || (TEAM == 2 && NOBJ == 64), "a team's warps take 32 object rows each");
   extern __shared__ __align__(16) uint8_t smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // per warp: q, k, v of the object tokens (NOBJ rows each), then q0 | k0 | v0, then the extra score column
+  // per team: q, k, v of the object tokens (NOBJ rows each), then q0 | k0 | v0, then the extra score column
   constexpr int kWarpHalfs = 3 * NOBJ * LDS + 3 * LDS;
-  __half* sq = reinterpret_cast<__half*>(smem) + (size_t)warp * kWarpHalfs;
+  const int team = warp / TEAM, part = warp % TEAM, tlane = part * 32 + lane;
+  __half* sq = reinterpret_cast<__half*>(smem) + (size_t)team * kWarpHalfs;
   __half* sk = sq + NOBJ * LDS;
   __half* sv = sk + NOBJ * LDS;
   __half* s0 = sv + NOBJ * LDS;                      // q0 at [0, DH), k0 at [LDS, ..), v0 at [2 LDS, ..)
-  float* sx = reinterpret_cast<float*>(smem + (size_t)WARPS * kWarpHalfs * 2) + warp * NOBJ;
+  float* sx = reinterpret_cast<float*>(smem + (size_t)(WARPS / TEAM) * kWarpHalfs * 2) + team * NOBJ;
   const uint32_t sq_u = smem_u32(sq), sk_u = smem_u32(sk), sv_u = smem_u32(sv);
   const float scale = rsqrtf(static_cast<float>(DH));
   const int g = lane >> 2, tig = lane & 3;
   const bool all_rows = n_q == T;
+  auto team_sync = [&]() {
+    if (TEAM == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(TEAM * 32) : "memory");
+  };
 
-  for (int64_t pair = (int64_t)blockIdx.x * WARPS + warp; pair < n_pairs; pair += (int64_t)gridDim.x * WARPS) {
+  for (int64_t pair = (int64_t)blockIdx.x * (WARPS / TEAM) + team; pair < n_pairs; pair += (int64_t)gridDim.x * (WARPS / TEAM)) {
     int head;
     const int64_t env = div_index(pair, n_heads, &head);
     const __half* base = qkv + env * T * (int64_t)ld + head * DH;
-    __syncwarp();
-    for (int c = lane; c < NOBJ * CH; c += 32) {
+    team_sync();
+    for (int c = tlane; c < NOBJ * CH; c += 32 * TEAM) {
       const int row = c / CH, ch = c % CH;
       const __half* r = base + (int64_t)(row + 1) * ld + ch * 8;
-      if (all_rows) *reinterpret_cast<uint4*>(sq + row * LDS + ch * 8) = *reinterpret_cast<const uint4*>(r);
-      *reinterpret_cast<uint4*>(sk + row * LDS + ch * 8) = *reinterpret_cast<const uint4*>(r + d);
-      *reinterpret_cast<uint4*>(sv + row * LDS + ch * 8) = *reinterpret_cast<const uint4*>(r + 2 * d);
+      const uint32_t at = (row * LDS + ch * 8) * 2;
+      if (all_rows) cp_async16(sq_u + at, r, true);
+      cp_async16(sk_u + at, r + d, true);
+      cp_async16(sv_u + at, r + 2 * d, true);
     }
-    if (lane < 3 * CH) {
-      const int which = lane / CH, ch = lane % CH;
-      *reinterpret_cast<uint4*>(s0 + which * LDS + ch * 8) = *reinterpret_cast<const uint4*>(base + which * d + ch * 8);
+    if (tlane < 3 * CH) {
+      const int which = tlane / CH, ch = tlane % CH;
+      cp_async16(smem_u32(s0 + which * LDS + ch * 8), base + which * d + ch * 8, true);
     }
+    cp_async_commit();
     const float kb0 = key_bias[env * T];
-    __syncwarp();
+    cp_async_wait<0>();
+    team_sync();
 
     // ---- body query row: lane j scores object keys j, j + 32
     {
@@ -255,12 +263,12 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
       }
       sum = warp_sum(sum) + p00;
       const float inv = 1.f / sum;
-      // o0[c] = p00 v0[c] + sum_j p_j v_j[c]; lane owns columns lane, lane + 32
-      constexpr int CPL = (DH + 31) / 32;
+      // o0[c] = p00 v0[c] + sum_j p_j v_j[c]; a lane of the team owns columns tlane, tlane + 32 TEAM
+      constexpr int CPL = (DH + 32 * TEAM - 1) / (32 * TEAM);
       float o[CPL];
 #pragma unroll
       for (int u = 0; u < CPL; ++u) {
-        const int c = lane + 32 * u;
+        const int c = tlane + 32 * TEAM * u;
         o[u] = c < DH ? p00 * __half2float(s0[2 * LDS + c]) : 0.f;
       }
 #pragma unroll
@@ -272,7 +280,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
           const float pj = __shfl_sync(0xffffffffu, sc[i], jj);
 #pragma unroll
           for (int u = 0; u < CPL; ++u) {
-            const int c = lane + 32 * u;
+            const int c = tlane + 32 * TEAM * u;
             if (c < DH) o[u] = fmaf(pj, __half2float(sv[j * LDS + c]), o[u]);
           }
         }
@@ -280,7 +288,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
       __half* orow = out + env * n_q * (int64_t)ldo + head * DH;
 #pragma unroll
       for (int u = 0; u < CPL; ++u) {
-        const int c = lane + 32 * u;
+        const int c = tlane + 32 * TEAM * u;
         if (c < DH) orow[c] = __float2half_rn(o[u] * inv);
       }
     }
@@ -290,7 +298,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
       const int r = lane + 32 * i;
-      if (r < NOBJ) {
+      if (r < NOBJ && (TEAM == 1 || i == part)) {           // the rows of this warp's query tiles
         float acc = 0.f;
 #pragma unroll
         for (int ch = 0; ch < CH; ++ch) {
@@ -316,7 +324,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
 
     // ---- object query rows against the object keys on the tensor cores
 #pragma unroll 1
-    for (int mt = 0; mt < MT; ++mt) {
+    for (int mt = part * (MT / TEAM); mt < (part + 1) * (MT / TEAM); ++mt) {
       float s[NT][4];
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
@@ -395,33 +403,35 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
           mma_f16(o[2 * j + 1], pa[ks], b[2], b[3]);
         }
       }
+      // the output takes the place of the query rows it came from
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const int token = 1 + mt * 16 + g + r * 8;
-        __half* orow = out + (env * T + token) * (int64_t)ldo + head * DH + tig * 2;
+        __half* orow = sq + (mt * 16 + g + r * 8) * LDS + tig * 2;
 #pragma unroll
-        for (int nt = 0; nt < DH / 8; ++nt)
-          *reinterpret_cast<uint32_t*>(orow + nt * 8) = pack_half2(o[nt][r * 2], o[nt][r * 2 + 1]);
+        for (int nt = 0; nt < DH / 8; ++nt) *reinterpret_cast<uint32_t*>(orow + nt * 8) = pack_half2(o[nt][r * 2], o[nt][r * 2 + 1]);
       }
     }
+    __syncwarp();
+    const int row0 = part * (NOBJ / TEAM);
+    copy_rows_out<DH, LDS>(sq + row0 * LDS, NOBJ / TEAM, out + (env * T + 1 + row0) * (int64_t)ldo + head * DH, ldo, true, lane);
   }
 }
 
 template <int DH, int NOBJ>
 int launch_body(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int d, int n_heads, int n_q, __half* out,
                 int ldo, cudaStream_t stream) {
-  constexpr int kWarps = NOBJ <= 32 ? 8 : 4;
-  constexpr int smem = kWarps * ((3 * NOBJ + 3) * (DH + 8) * 2 + NOBJ * 4);
+  constexpr int kWarps = 8, kTeam = NOBJ <= 32 ? 1 : 2, kPairs = kWarps / kTeam;
+  constexpr int smem = kPairs * ((3 * NOBJ + 3) * (DH + 8) * 2 + NOBJ * 4);
   static DeviceOnce once;
   int rc = once.run("attn_body_kernel set-up", [] {
-    return cudaFuncSetAttribute(attn_body_kernel<DH, NOBJ, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    return cudaFuncSetAttribute(attn_body_kernel<DH, NOBJ, kWarps, kTeam>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   });
   if (rc != BSRL_OK) return rc;
   const int64_t pairs = n_envs * n_heads;
-  int64_t blocks = (pairs + kWarps - 1) / kWarps;
+  int64_t blocks = (pairs + kPairs - 1) / kPairs;
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  launch_kernel(attn_body_kernel<DH, NOBJ, kWarps>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d,
+  launch_kernel(attn_body_kernel<DH, NOBJ, kWarps, kTeam>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d,
                                                                                                 n_heads, n_q, out, ldo);
   BSRL_LAUNCH_OK("attn_body_kernel");
   return BSRL_OK;

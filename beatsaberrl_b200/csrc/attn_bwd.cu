@@ -9,40 +9,45 @@
 // problem of one (env, head) pair -- at most 32 x 64 values per matrix -- lives in the warp's shared-memory
 // tile; the five products run on m16n8k16 MMAs with fp32 accumulation, P and dS rounded to fp16 as operands.
 #include "kernels.cuh"
+#include "attend.cuh"
 
 namespace bsrl {
 namespace {
 
 constexpr int kWarps = 4;
 constexpr int kKeys = 32;      // 29 keys padded to four 8-key MMA tiles
-constexpr int LDP = kKeys + 8; // row pitch (halves) of the P / dS tiles
+
+// the 8 x 8 matrix of fp16 pairs that the warp holds (row lane / 4, columns 2 (lane % 4)..) -> its transpose, in the same layout
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
 
 // One warp per (env, head); MT = 16-row query tiles (2: all 29 queries, 1: the lead rows or the critic's one).
 // Five small products on m16n8k16 MMAs: S = q k^T and dP = dO v^T (A rows = queries, B rows = keys);
 // dQ = dS k (A = dS from the accumulator registers, B = k with the keys as the reduction dimension);
-// dV = P^T dO and dK = dS^T q (A = the transposed P / dS tile, fetched from shared memory with
-// ldmatrix.trans; B = dO / q with the queries as the reduction dimension).
+// dV = P^T dO and dK = dS^T q (A = P / dS transposed in registers, 8 x 8 at a time; B = dO / q with the queries as the
+// reduction dimension).  The operands arrive by cp.async, the results leave from the rows of the operands they replace, 16
+// bytes per lane.  Bound by latency: what sets its speed is the warps an SM can hold, that is the bytes of a warp's tile.
 template <int DH, int MT>
 __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __restrict__ qkv, int ld, const float* __restrict__ key_bias,
                                                                int64_t n_pairs, int d, int n_heads, int q_first, int n_q,
                                                                const __half* __restrict__ g_out, int ldgo, __half* __restrict__ gq,
                                                                int ldq, __half* __restrict__ gk, int ldk, __half* __restrict__ gv,
-                                                               int ldv) {
+                                                               int ldv, int wide) {
   pdl_begin();
   constexpr int LDS = DH + 8;                         // padded row (halves): ldmatrix rows land in distinct banks
   constexpr int CH = DH / 8;
   constexpr int QR = 16 * MT;                         // staged query rows
-  constexpr int PER_WARP = (2 * QR + 2 * kKeys) * LDS * 2 + 2 * QR * LDP * 2;
+  constexpr int PER_WARP = (2 * QR + 2 * kKeys) * LDS * 2;
   extern __shared__ __align__(16) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   __half* sq = reinterpret_cast<__half*>(smem + (size_t)warp * PER_WARP);
   __half* sg = sq + QR * LDS;
   __half* sk = sg + QR * LDS;
   __half* sv = sk + kKeys * LDS;
-  __half* sp = sv + kKeys * LDS;                      // P  [query][key]
-  __half* sd = sp + QR * LDP;                         // dS [query][key]
-  const uint32_t sq_u = smem_u32(sq), sg_u = smem_u32(sg), sk_u = smem_u32(sk), sv_u = smem_u32(sv), sp_u = smem_u32(sp),
-                 sd_u = smem_u32(sd);
+  const uint32_t sq_u = smem_u32(sq), sg_u = smem_u32(sg), sk_u = smem_u32(sk), sv_u = smem_u32(sv);
   const float scale = rsqrtf((float)DH);
   const int g = lane >> 2, tig = lane & 3;
   const int64_t warps = (int64_t)gridDim.x * kWarps;
@@ -54,23 +59,17 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
     // stage q, dO (query rows) and k, v (key rows); rows past the live range are zero
     for (int c = lane; c < kKeys * CH; c += 32) {
       const int row = c / CH, ch = c % CH;
-      uint4 zk = make_uint4(0, 0, 0, 0), zv = zk, zq = zk, zg = zk;
-      if (row < kT) {
-        const __half* r = base + (int64_t)row * ld + ch * 8;
-        zk = *reinterpret_cast<const uint4*>(r + d);
-        zv = *reinterpret_cast<const uint4*>(r + 2 * d);
-      }
-      if (row < n_q) {
-        zq = *reinterpret_cast<const uint4*>(base + (int64_t)(q_first + row) * ld + ch * 8);
-        zg = *reinterpret_cast<const uint4*>(g_out + (env * n_q + row) * (int64_t)ldgo + head * DH + ch * 8);
-      }
-      *reinterpret_cast<uint4*>(sk + row * LDS + ch * 8) = zk;
-      *reinterpret_cast<uint4*>(sv + row * LDS + ch * 8) = zv;
+      const bool live = row < kT, asks = row < n_q;
+      const __half* r = base + (int64_t)(live ? row : 0) * ld + ch * 8;
+      const uint32_t at = (row * LDS + ch * 8) * 2;
+      cp_async16(sk_u + at, r + d, live);
+      cp_async16(sv_u + at, r + 2 * d, live);
       if (row < QR) {
-        *reinterpret_cast<uint4*>(sq + row * LDS + ch * 8) = zq;
-        *reinterpret_cast<uint4*>(sg + row * LDS + ch * 8) = zg;
+        cp_async16(sq_u + at, base + (int64_t)(asks ? q_first + row : 0) * ld + ch * 8, asks);
+        cp_async16(sg_u + at, g_out + (env * n_q + (asks ? row : 0)) * (int64_t)ldgo + head * DH + ch * 8, asks);
       }
     }
+    cp_async_commit();
     float kb[4][2];
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
@@ -79,7 +78,11 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
         const int key = nt * 8 + tig * 2 + e;
         kb[nt][e] = key < kT ? key_bias[env * kT + key] : -INFINITY;
       }
+    cp_async_wait<0>();
     __syncwarp();
+
+    uint32_t tp[MT][2][4], td[MT][2][4];                // P^T and dS^T, A fragments of 16 keys x 16 queries
+    uint32_t oq16[MT][DH / 8][2];                       // dQ
 
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
@@ -153,14 +156,13 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) dp[nt][e] = s[nt][e] * (dp[nt][e] - dot[e >> 1]) * scale;   // dS
-      // P and dS tiles to shared memory ([query][key] fp16) for the two transposed products
+      // 8 x 8 blocks (8 queries x 8 keys) transposed across the warp
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const int off = (mt * 16 + g + r * 8) * LDP + nt * 8 + tig * 2;
-          *reinterpret_cast<uint32_t*>(sp + off) = pack_half2(s[nt][2 * r], s[nt][2 * r + 1]);
-          *reinterpret_cast<uint32_t*>(sd + off) = pack_half2(dp[nt][2 * r], dp[nt][2 * r + 1]);
+          tp[mt][nt >> 1][(nt & 1) + 2 * r] = transpose8x8(pack_half2(s[nt][2 * r], s[nt][2 * r + 1]));
+          td[mt][nt >> 1][(nt & 1) + 2 * r] = transpose8x8(pack_half2(dp[nt][2 * r], dp[nt][2 * r + 1]));
         }
       // ---- dQ = dS k: A = dS from the accumulator registers (as P feeds P v in the forward)
       uint32_t da[2][4];
@@ -187,16 +189,11 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
           mma_f16(oq[2 * j + 1], da[ks], b[2], b[3]);
         }
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const int qrow = mt * 16 + g + r * 8;
-        if (qrow < n_q) {
-          __half* orow = gq + (env * n_q + qrow) * (int64_t)ldq + head * DH + tig * 2;
+      for (int nt = 0; nt < DH / 8; ++nt)
 #pragma unroll
-          for (int nt = 0; nt < DH / 8; ++nt) *reinterpret_cast<uint32_t*>(orow + nt * 8) = pack_half2(oq[nt][r * 2], oq[nt][r * 2 + 1]);
-        }
-      }
+        for (int r = 0; r < 2; ++r) oq16[mt][nt][r] = pack_half2(oq[nt][r * 2], oq[nt][r * 2 + 1]);
     }
-    __syncwarp();
+    __syncwarp();                                       // k and v have been read: dK and dV take their places
     // ---- dV = P^T dO and dK = dS^T q: key tiles as rows, the queries as the reduction dimension
 #pragma unroll
     for (int kt = 0; kt < 2; ++kt) {
@@ -207,13 +204,6 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
         for (int e = 0; e < 4; ++e) ov[nt][e] = ok[nt][e] = 0.f;
 #pragma unroll
       for (int qs = 0; qs < MT; ++qs) {                 // 16 queries per step
-        // A fragment (16 keys x 16 queries) of the transposed tile: matrix m of the x4 load covers
-        // keys kt * 16 + (m & 1) * 8 .., queries qs * 16 + (m >> 1) * 8 ..; lane l supplies query row l & 7 of matrix l >> 3
-        uint32_t ap[4], ad[4];
-        const int m = lane >> 3;
-        const uint32_t toff = ((qs * 16 + (m >> 1) * 8 + (lane & 7)) * LDP + kt * 16 + (m & 1) * 8) * 2;
-        ldmatrix_x4_trans(ap, sp_u + toff);
-        ldmatrix_x4_trans(ad, sd_u + toff);
 #pragma unroll
         for (int j = 0; j < DH / 16; ++j) {
           uint32_t b[4], bq[4];
@@ -221,45 +211,52 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
           const uint32_t boff = (row * LDS + j * 16 + (lane >> 4) * 8) * 2;
           ldmatrix_x4_trans(b, sg_u + boff);
           ldmatrix_x4_trans(bq, sq_u + boff);
-          mma_f16(ov[2 * j], ap, b[0], b[1]);
-          mma_f16(ov[2 * j + 1], ap, b[2], b[3]);
-          mma_f16(ok[2 * j], ad, bq[0], bq[1]);
-          mma_f16(ok[2 * j + 1], ad, bq[2], bq[3]);
+          mma_f16(ov[2 * j], tp[qs][kt], b[0], b[1]);
+          mma_f16(ov[2 * j + 1], tp[qs][kt], b[2], b[3]);
+          mma_f16(ok[2 * j], td[qs][kt], bq[0], bq[1]);
+          mma_f16(ok[2 * j + 1], td[qs][kt], bq[2], bq[3]);
         }
       }
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const int key = kt * 16 + g + r * 8;
-        if (key < kT) {
-          const int64_t row = env * kT + key;
-          __half* vrow = gv + row * ldv + head * DH + tig * 2;
-          __half* krow = gk + row * ldk + head * DH + tig * 2;
+        const int at = (kt * 16 + g + r * 8) * LDS + tig * 2;
 #pragma unroll
-          for (int nt = 0; nt < DH / 8; ++nt) {
-            *reinterpret_cast<uint32_t*>(vrow + nt * 8) = pack_half2(ov[nt][r * 2], ov[nt][r * 2 + 1]);
-            *reinterpret_cast<uint32_t*>(krow + nt * 8) = pack_half2(ok[nt][r * 2], ok[nt][r * 2 + 1]);
-          }
+        for (int nt = 0; nt < DH / 8; ++nt) {
+          *reinterpret_cast<uint32_t*>(sv + at + nt * 8) = pack_half2(ov[nt][r * 2], ov[nt][r * 2 + 1]);
+          *reinterpret_cast<uint32_t*>(sk + at + nt * 8) = pack_half2(ok[nt][r * 2], ok[nt][r * 2 + 1]);
         }
       }
     }
+    __syncwarp();                                       // q has been read too
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int nt = 0; nt < DH / 8; ++nt) *reinterpret_cast<uint32_t*>(sq + (mt * 16 + g + r * 8) * LDS + nt * 8 + tig * 2) = oq16[mt][nt][r];
+    __syncwarp();
+    copy_rows_out<DH, LDS>(sv, kT, gv + env * kT * (int64_t)ldv + head * DH, ldv, wide, lane);
+    copy_rows_out<DH, LDS>(sk, kT, gk + env * kT * (int64_t)ldk + head * DH, ldk, wide, lane);
+    copy_rows_out<DH, LDS>(sq, n_q, gq + env * n_q * (int64_t)ldq + head * DH, ldq, wide, lane);
   }
 }
 
 template <int DH, int MT>
 int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int d, int n_heads, int q_first, int n_q,
            const __half* g_out, int ldgo, __half* gq, int ldq, __half* gk, int ldk, __half* gv, int ldv, cudaStream_t stream) {
-  constexpr int smem = kWarps * ((2 * 16 * MT + 2 * kKeys) * (DH + 8) * 2 + 2 * 16 * MT * LDP * 2);
+  constexpr int smem = kWarps * (2 * 16 * MT + 2 * kKeys) * (DH + 8) * 2;
   static DeviceOnce once;
   int rc = once.run("attn_bwd_kernel set-up", [] {
     return cudaFuncSetAttribute(attn_bwd_kernel<DH, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   });
   if (rc != BSRL_OK) return rc;
+  const int wide = aligned16(gq) && aligned16(gk) && aligned16(gv) && ldq % 8 == 0 && ldk % 8 == 0 && ldv % 8 == 0;
   const int64_t pairs = n_envs * n_heads;
   int64_t blocks = (pairs + kWarps - 1) / kWarps;
   const int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
   launch_kernel(attn_bwd_kernel<DH, MT>, (unsigned)blocks, kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d, n_heads, q_first, n_q, g_out,
-                                                                          ldgo, gq, ldq, gk, ldk, gv, ldv);
+                                                                          ldgo, gq, ldq, gk, ldk, gv, ldv, wide);
   BSRL_LAUNCH_OK("attn_bwd_kernel");
   return BSRL_OK;
 }
