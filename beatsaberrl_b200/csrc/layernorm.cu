@@ -123,7 +123,9 @@ int launch_layernorm(const float* x, int64_t ldx, RowMap xmap, const float* gamm
   }
   if (rows == 0) return BSRL_OK;
   const int64_t cap = (int64_t)sm_count() * 16;
-  const int rpw = rows < cap * 8 * 4 ? 1 : d <= 256 ? 4 : d <= 512 ? 2 : 1;   // long inputs: several rows per warp
+  // several rows per warp as soon as every SM has a block: 59,421 rows of 192 17 us against 33 with one (11 at copy speed),
+  // 11,600 rows 7.6 against 10.4; with fewer rows there is nothing to choose
+  const int rpw = rows <= 8 * (int64_t)sm_count() ? 1 : d <= 256 ? 4 : d <= 512 ? 2 : 1;
   int64_t blocks = (rows + 8 * rpw - 1) / (8 * rpw);
   if (blocks > cap) blocks = cap;
   const unsigned nb = static_cast<unsigned>(blocks);
