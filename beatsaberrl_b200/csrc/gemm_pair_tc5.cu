@@ -72,7 +72,7 @@ __device__ __forceinline__ uint32_t keep_positive(uint32_t h, uint32_t mask) {
 template <bool HAS_R>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
-                   const __grid_constant__ CUtensorMap tm_c, int r32, LinearArgs p, int m_pairs, int n_tiles, int* status) {
+                   const __grid_constant__ CUtensorMap tm_c, int box_rows, int r32, LinearArgs p, int m_pairs, int n_tiles, int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -214,7 +214,8 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && m0 < p.M) {
-          tma_store_2d(&tm_c, x, (int)m0, smem_u32(stg));
+          if (box_rows == 32) tma_store_2d(&tm_c, x, (int)m0, smem_u32(stg));
+          else store_mapped8(&tm_c, x, m0, p.M, p.cmap, smem_u32(stg));
           bulk_commit();
         }
       };
@@ -317,9 +318,8 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
 // Whole 256-column tiles, dense rows, K past the resident-weight kernel, and at least two pair tiles per CTA pair.
 bool linear_pair_ok(const LinearArgs& p) {
   const int64_t work = (p.M + 2 * BM - 1) / (2 * BM) * (p.N / BN);
-  auto dense = [](const RowMap& m) { return m.group == 0x7fffffff && m.stride == 0 && m.first == 0; };
   return !p.a_mn && !p.a_sums && !p.bits_in && !p.bits_out && p.k_splits <= 1 && p.N % BN == 0 && p.K > 4 * BK && p.M <= 0x7fffff00 &&
-         work >= sm_count() && work <= 0x7fffffff && dense(p.cmap) && (!p.R || (dense(p.rmap) && !p.mask)) && (!p.mask || !p.out_f32) &&
+         work >= sm_count() && work <= 0x7fffffff && store_box_rows(p.cmap, p.M) != 0 && (!p.R || (dense_rows(p.cmap) && dense_rows(p.rmap) && !p.mask)) && (!p.mask || !p.out_f32) &&
          linear_tc5_ok(p);
 }
 
@@ -334,7 +334,8 @@ int linear_pair(const LinearArgs& p, cudaStream_t stream) {
   if (!make_tmap_f16(&tm_a, p.A, p.M, p.K, p.lda, BM)) return BSRL_ERR_CUDA;
   if (p.w_mn ? !make_tmap_mn(&tm_w, p.W, p.K, p.N, p.ldw, BK, BN / 128) : !make_tmap_f16(&tm_w, p.W, p.N, p.K, p.ldw, BN / 2))
     return BSRL_ERR_CUDA;
-  if (!make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, p.M, p.N, p.ldc, 32, 128)) return BSRL_ERR_CUDA;
+  const int box_rows = store_box_rows(p.cmap, p.M);
+  if (!make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, box_rows == 32 ? p.M : p.cmap(p.M - 1) + 1, p.N, p.ldc, box_rows, 128)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("linear_pair_kernel set-up", [] {
     cudaError_t e = cudaFuncSetAttribute(linear_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
@@ -344,7 +345,7 @@ int linear_pair(const LinearArgs& p, cudaStream_t stream) {
   const int m_pairs = (int)((p.M + 2 * BM - 1) / (2 * BM)), n_tiles = p.N / BN;
   const int r32 = p.R && reinterpret_cast<uintptr_t>(p.R) % 32 == 0 && p.ldr % 8 == 0;        // 32-byte residual loads
   auto* kernel = p.R ? linear_pair_kernel<true> : linear_pair_kernel<false>;
-  launch_kernel<2>(kernel, (unsigned)(sm_count() & ~1), THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, r32, p, m_pairs, n_tiles, status);
+  launch_kernel<2>(kernel, (unsigned)(sm_count() & ~1), THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, box_rows, r32, p, m_pairs, n_tiles, status);
   BSRL_LAUNCH_OK("linear_pair_kernel");
   return BSRL_OK;
 }

@@ -249,7 +249,8 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0 && m0 < p.M) {
-            tma_store_2d(&tm_c, x, (int)m0, smem_u32(stg));
+            if (tma_c == 32) tma_store_2d(&tm_c, x, (int)m0, smem_u32(stg));
+            else store_mapped8(&tm_c, x, m0, p.M, p.cmap, smem_u32(stg));
             bulk_commit();
           }
           return;
@@ -377,13 +378,14 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 }
 }  // namespace
 
-// fp32 rows without a residual stay with gemm_tc5.cu (475 K x 256 x 128: 105 us there, 120 here: four stores per half
-// tile either way, nothing to overlap them with).  K <= 256 in whole k-blocks or row-contraction weights, and at least three row tiles per CTA for the resident weights:
+// Dense fp32 rows without a residual stay with gemm_tc5.cu (475 K x 256 x 128: 105 us there, 120 here: four stores per half
+// tile either way, nothing to overlap them with); rows placed by a map come here, where runs of 8 leave by TMA (2.1 M token
+// rows x 256, K = 64: 827 -> 631 us, bound by the 2.1 GB it writes).  K <= 256 in whole k-blocks or row-contraction weights, and at least three row tiles per CTA for the resident weights:
 // with one or two their load (128 KB before the first MMA) costs more than it saves.  fp16 masks are read by
 // gemm_tc5.cu (here only as bits).
 bool linear_res_ok(const LinearArgs& p) {
   const int64_t tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
-  return !p.a_mn && !p.mask && (!p.out_f32 || p.R) && !p.a_sums && p.k_splits <= 1 && p.K <= 4 * BK && p.M <= 0x7fffff00 && tiles >= 3ll * sm_count() &&
+  return !p.a_mn && !p.mask && (!p.out_f32 || p.R || !dense_rows(p.cmap)) && !p.a_sums && p.k_splits <= 1 && p.K <= 4 * BK && p.M <= 0x7fffff00 && tiles >= 3ll * sm_count() &&
          (!(p.bits_in || p.bits_out) || (!p.out_f32 && !p.R && p.N % 32 == 0)) && linear_tc5_ok(p);
 }
 
@@ -398,9 +400,9 @@ int linear_res(const LinearArgs& p, cudaStream_t stream) {
   if (!make_tmap_f16(&tm_a, p.A, p.M, p.K, p.lda, BM)) return BSRL_ERR_CUDA;
   if (p.w_mn ? !make_tmap_mn(&tm_w, p.W, p.K, p.N, p.ldw, BK, BN / 64) : !make_tmap_f16(&tm_w, p.W, p.N, p.K, p.ldw, BN))
     return BSRL_ERR_CUDA;
-  const bool tma_c = p.cmap.group == 0x7fffffff && p.cmap.stride == 0 && p.cmap.first == 0;    // dense output rows
+  const int tma_c = store_box_rows(p.cmap, p.M);
   CUtensorMap tm_c = tm_a;
-  if (tma_c && !make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, p.M, p.N, p.ldc, 32, 128)) return BSRL_ERR_CUDA;
+  if (tma_c && !make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, tma_c == 32 ? p.M : p.cmap(p.M - 1) + 1, p.N, p.ldc, tma_c, 128)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("linear_res_kernel set-up", [] {
     cudaError_t e = cudaFuncSetAttribute(linear_res_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
@@ -410,7 +412,7 @@ int linear_res(const LinearArgs& p, cudaStream_t stream) {
   const int m_tiles = (int)((p.M + BM - 1) / BM), n_tiles = (p.N + BN - 1) / BN;
   const int r32 = p.R && reinterpret_cast<uintptr_t>(p.R) % 32 == 0 && p.ldr % 8 == 0;        // 32-byte residual loads
   auto* kernel = p.R ? linear_res_kernel<true> : linear_res_kernel<false>;
-  launch_kernel(kernel, sm_count(), THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, tma_c ? 1 : 0, r32, p, m_tiles, n_tiles, status);
+  launch_kernel(kernel, sm_count(), THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, tma_c, r32, p, m_tiles, n_tiles, status);
   BSRL_LAUNCH_OK("linear_res_kernel");
   return BSRL_OK;
 }
