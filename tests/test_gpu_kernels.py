@@ -479,3 +479,34 @@ def test_block_tail_cta_pairs(native, m, d, f):
     parts = [torch.cat(t) for t in zip(*(run(lo, min(lo + 32768, m)) for lo in range(0, m, 32768)))]
     for whole, part in zip(run(0, m), parts):
         assert not bool(torch.isnan(whole).any()) and torch.equal(whole, part)
+
+
+@pytest.mark.parametrize("B,d,H,body", [(65, 256, 8, 0), (147, 192, 4, 0), (296, 192, 4, 0), (293, 512, 8, 0), (117, 128, 4, 1), (9, 256, 8, 1),
+                                        (70, 320, 5, 0)])
+def test_qkv_attention_split_groups(native, B, d, H, body):
+    """Few tiles: CTAs share a tile's head groups (two, four or eight shares, the last ones of five groups uneven).  Each env
+    is bit-identical to a launch with so many tiles that none is shared."""
+    T = 33 if body else 29
+    g = torch.Generator(device="cuda").manual_seed(B + d)
+    h = torch.randn(B * T, d, generator=g, device="cuda").half()
+    w = (torch.randn(3 * d, d, generator=g, device="cuda") * d ** -0.5).half()
+    b = torch.randn(3 * d, generator=g, device="cuda") * 0.2
+    q0 = torch.randn(B, 3 * d, generator=g, device="cuda").half()
+    kb = torch.where(torch.rand(B, T, generator=g, device="cuda") < 0.3, -16384.0, 0.0)
+    kb[:, 0] = 0.0
+
+    def run(rep):
+        hs, ks, qs = h.repeat(rep, 1), kb.repeat(rep, 1), q0.repeat(rep, 1)
+        out = torch.full((rep * B * T, d), float("nan"), dtype=torch.float16, device="cuda")
+        if body:
+            rc = native.lib.bsrl_qkv_attention_body(hs.data_ptr(), w.data_ptr(), b.data_ptr(), qs.data_ptr(), ks.data_ptr(),
+                                                    rep * B, d, H, T, out.data_ptr(), _stream())
+        else:
+            rc = native.lib.bsrl_qkv_attention(hs.data_ptr(), w.data_ptr(), b.data_ptr(), ks.data_ptr(), rep * B, d, H, 0, T,
+                                               out.data_ptr(), _stream())
+        native.check(rc)
+        native.check(native.lib.bsrl_device_status())
+        return out
+
+    few, many = run(1), run(-(-700 // B))
+    assert not bool(torch.isnan(few).any()) and torch.equal(few, many[:B * T])
