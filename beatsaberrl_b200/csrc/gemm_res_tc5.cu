@@ -2,19 +2,23 @@
 // over many rows (the token-row products of the backward and of the unfused forward paths).
 //
 // gemm_tc5.cu streams A and W tiles together; with K <= 256 that draws 192 KB from L2 per 128 x 256 output tile -- 4 to
-// 5 K cycles at what an SM gets from L2 -- where the tile's HBM traffic (64 KB in, 64 KB out) needs 3 K.  Here a CTA
-// works down the row tiles of ONE column tile: its weights (<= 128 KB) are loaded once, only A streams, through a ring
-// of 16 KB stages over the rest of the 192 KB.  Roles as in gemm_tc5.cu:
-//   warp 0      TMA producer;   warp 1      MMA issuer (one thread, M = 128, N <= 256, two TMEM accumulators);
-//   warps 2..9  epilogue.
+// 5 K cycles at what an SM gets from L2 -- where the tile's HBM traffic (64 KB in, 64 KB out) needs 3 K.  Here a PAIR of
+// CTAs (cta_group::2) works down the row tiles of ONE column tile: each holds half of its weights (<= 64 KB, loaded once)
+// and streams its own 128 rows of A through a ring of 16 KB stages over the rest of 160 KB (6 stages at K = 256, where a
+// single CTA with all the weights had 4 and one staging buffer less per warp).  Roles as in gemm_tc5.cu:
+//   warp 0      TMA producer (completion is counted on the leader's barriers);
+//   warp 1      of the leader: MMA issuer (one thread, M = 256, N <= 256, two TMEM accumulators);
+//   warps 2..9  epilogue of the CTA's own rows.
 //
-// What bounds it now is the epilogue's chain of latencies (475 K x 768 x 256: MMAs alone 156 us, loads hidden, epilogue
+// What bounds it is the epilogue's chain of latencies (475 K x 768 x 256: MMAs alone 156 us, loads hidden, epilogue
 // alone about 200), so the next block's accumulator is requested before this block is staged, residual rows a block
 // ahead (and the next tile's into L2), and the bias sits in shared memory.  Its loops stay rolled: unrolled they spill.
 // Other ways of writing the rows measured slower: threads storing their own row in 32-byte pieces 418 us, boxes of
-// 64 bytes per row through three buffers 278 us (a TMA store costs the same whatever its size).
-// Measured, 475 K rows, same box as gemm_tc5.cu: x 768 x 256 fp16 269 -> 227 us, x 768 x 192 302 -> 236, x 1024 x 128
-// 347 -> 268, x 192 x 192 fp32 + residual 296 -> 229, x 256 x 256 fp32 + residual 316 -> 290.
+// 64 bytes per row through three buffers 278 us (a TMA store costs the same whatever its size); three buffers and four
+// stages 224 us, two and two (single CTA) 285.
+// Measured, 475 K rows, us, gemm_tc5.cu / single CTAs / pairs: x 768 x 256 fp16 304 / 231 / 217, x 1024 x 256 with ReLU
+// 439 / 318 / 289, x 576 x 192 246 / 207 / 191, x 384 x 128 175 / 128 / 115, x 192 x 192 fp32 + residual 291 / 204 / 195,
+// x 256 x 256 fp32 + residual 323 / 248 / 242.
 //
 // ReLU masks as bits: a product with ReLU can leave one bit per output (1 = positive), which the product that carries
 // the gradient back reads instead of the fp16 activations: 1/16 of their bytes.  One 32-bit word holds 32 columns of
@@ -28,14 +32,15 @@ namespace {
 using namespace tc5;
 
 constexpr int BM = 128, BN = 256, BK = 64;
-constexpr int A_BYTES = BM * BK * 2, W_BYTES = BN * BK * 2;
-constexpr int OPERAND_BYTES = 192 * 1024;       // weights, A ring and second staging buffers
+constexpr int A_BYTES = BM * BK * 2, W_BYTES = BN / 2 * BK * 2;      // per CTA of the pair
+constexpr int OPERAND_BYTES = 160 * 1024;       // half of the weights, A ring
 constexpr int MAX_STAGES = 10;
 constexpr int EPI_WARPS = 8;
 constexpr int THREADS = (2 + EPI_WARPS) * 32;
 constexpr int TMEM_COLS = 2 * BN;
 constexpr int STG_BYTES = 32 * 128;             // staging buffer: 32 rows x 128 bytes
-constexpr int SMEM_BYTES = OPERAND_BYTES + EPI_WARPS * STG_BYTES + BN * 4 /*bias*/ + 1024 /*alignment*/ + 256 /*barriers*/;
+constexpr int NBUF = 2;                         // of them per epilogue warp
+constexpr int SMEM_BYTES = OPERAND_BYTES + EPI_WARPS * NBUF * STG_BYTES + BN * 4 /*bias*/ + 1024 /*alignment*/ + 256 /*barriers*/;
 constexpr int KERNEL_ID = 10;
 
 struct Shared {
@@ -86,24 +91,23 @@ __device__ __forceinline__ uint32_t keep_positive(uint32_t h, uint32_t w, int i)
 template <bool HAS_R>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
-                  const __grid_constant__ CUtensorMap tm_c, int tma_c, int r32, LinearArgs p, int m_tiles, int n_tiles,
+                  const __grid_constant__ CUtensorMap tm_c, int tma_c, int r32, LinearArgs p, int bn, int m_tiles, int n_tiles,
                   int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   const int k_blocks = (p.K + BK - 1) / BK;
-  // a second staging buffer per epilogue warp where the weights leave the ring at least four stages
-  const int nbuf = k_blocks <= 3 ? 2 : 1;
-  const int ring_bytes = OPERAND_BYTES - (nbuf - 1) * EPI_WARPS * STG_BYTES;
-  const int n_st = min(MAX_STAGES, (ring_bytes - k_blocks * W_BYTES) / A_BYTES);
+  const int n_st = min(MAX_STAGES, (OPERAND_BYTES - k_blocks * W_BYTES) / A_BYTES);
   const uint32_t w_base = base + n_st * A_BYTES;
-  uint8_t* staging = smem_raw + (base - raw) + ring_bytes;
-  float* s_bias = reinterpret_cast<float*>(staging + EPI_WARPS * nbuf * STG_BYTES);
+  uint8_t* staging = smem_raw + (base - raw) + OPERAND_BYTES;
+  float* s_bias = reinterpret_cast<float*>(staging + EPI_WARPS * NBUF * STG_BYTES);
   Shared* sh = reinterpret_cast<Shared*>(s_bias + BN);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // this CTA's column tile, its first row tile and the step to the next
-  const int nt = (int)(blockIdx.x % (unsigned)n_tiles), n0 = nt * BN;
-  const int t0 = (int)(blockIdx.x / (unsigned)n_tiles), t_step = ((int)gridDim.x - nt + n_tiles - 1) / n_tiles;
+  const uint32_t rank = cluster_rank();
+  // this pair's column tile, its first tile of 256 rows and the step to the next
+  const unsigned pair = blockIdx.x >> 1;
+  const int nt = (int)(pair % (unsigned)n_tiles), n0 = nt * bn, n_end = min(p.N, n0 + bn);
+  const int t0 = (int)(pair / (unsigned)n_tiles), t_step = ((int)(gridDim.x >> 1) - nt + n_tiles - 1) / n_tiles;
   volatile int* abort = &sh->abort;
 
   if (threadIdx.x == 0) {
@@ -113,7 +117,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&sh->tmem_full[b]), 1);
-      mbar_init(smem_u32(&sh->tmem_empty[b]), EPI_WARPS);
+      mbar_init(smem_u32(&sh->tmem_empty[b]), 2 * EPI_WARPS);     // the leader's: both CTAs' epilogue warps
     }
     mbar_init(smem_u32(&sh->mma_done), 1);
     mbar_init(smem_u32(&sh->w_full), 1);
@@ -123,12 +127,13 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     tma_prefetch_desc(&tm_w);
   }
   if (warp == 1) {
-    tmem_alloc(smem_u32(&sh->tmem_base), TMEM_COLS);
-    tmem_relinquish();
+    tmem_alloc_pair(smem_u32(&sh->tmem_base), TMEM_COLS);
+    tmem_relinquish_pair();
   }
-  for (int i = threadIdx.x; i < BN; i += THREADS) s_bias[i] = p.bias && n0 + i < p.N ? p.bias[n0 + i] : 0.f;
+  for (int i = threadIdx.x; i < BN; i += THREADS) s_bias[i] = p.bias && n0 + i < n_end ? p.bias[n0 + i] : 0.f;
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();          // the peer's barriers exist before anything is signalled across
   tc_fence_after();
   const uint32_t tmem_base = sh->tmem_base;
   pdl_begin();
@@ -137,10 +142,16 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // ---------------------------------------------------------------- TMA producer
     if (lane == 0 && t0 < m_tiles) {
       const uint32_t w_bar = smem_u32(&sh->w_full);
-      mbar_expect_tx(w_bar, (uint32_t)k_blocks * W_BYTES);
+      if (rank == 0) mbar_expect_tx(w_bar, 2u * (uint32_t)k_blocks * W_BYTES);       // both CTAs' bytes
+      const int w0 = n0 + (int)rank * ((n_end - n0) / 2);      // this CTA's half of the tile's columns (and what follows it)
       for (int kb = 0; kb < k_blocks; ++kb) {
-        if (p.w_mn) tma_load_3d(w_base + kb * W_BYTES, &tm_w, 0, kb * BK, n0 / 64, w_bar);
-        else tma_load_2d(w_base + kb * W_BYTES, &tm_w, kb * BK, n0, w_bar);
+        const uint32_t dst = w_base + kb * W_BYTES, lead = map_to_cta(w_bar, 0);
+        if (p.w_mn) {
+          tma_load_2d_pair(dst, &tm_w, w0, kb * BK, lead);
+          tma_load_2d_pair(dst + W_BYTES / 2, &tm_w, w0 + 64, kb * BK, lead);
+        } else {
+          tma_load_2d_pair(dst, &tm_w, kb * BK, w0, lead);
+        }
       }
       uint32_t it = 0, slot = 0, phase = 0;
       bool ok = true;
@@ -148,24 +159,26 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           if (!mbar_wait(smem_u32(&sh->empty[slot]), phase ^ 1, abort)) { give_up(sh, status, 1); ok = false; break; }
           const uint32_t bar = smem_u32(&sh->full[slot]);
-          mbar_expect_tx(bar, A_BYTES);
-          tma_load_2d(base + slot * A_BYTES, &tm_a, kb * BK, t * BM, bar);
+          if (rank == 0) mbar_expect_tx(bar, 2 * A_BYTES);
+          tma_load_2d_pair(base + slot * A_BYTES, &tm_a, kb * BK, (2 * t + (int)rank) * BM, map_to_cta(bar, 0));
           if (++slot == (uint32_t)n_st) { slot = 0; phase ^= 1; }
         }
       }
-      // loads in flight must land before this CTA may exit (also when a wait above gave up): bounded, ignoring abort
+      // loads in flight (both CTAs' are counted on the leader's barriers) land before the pair exits, also when a wait above
+      // gave up: bounded, ignoring abort
       uint32_t spins = 0;
+      if (rank != 0) it = 0;
       for (uint32_t j = it > (uint32_t)n_st ? it - n_st : 0; j < it; ++j)
         while (!mbar_try_wait(smem_u32(&sh->full[j % n_st]), (j / n_st) & 1) && ++spins < kSpinLimit) {}
-      while (!mbar_try_wait(w_bar, 0) && ++spins < kSpinLimit) {}
+      while (rank == 0 && !mbar_try_wait(w_bar, 0) && ++spins < kSpinLimit) {}
       if (spins >= kSpinLimit) give_up(sh, status, 2);
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    // ---------------------------------------------------------------- MMA issuer (the leader's)
+    if (lane == 0 && rank == 0) {
       uint32_t tile_i = 0, slot = 0, phase = 0;
       bool ok = true;
-      const uint32_t idesc = idesc_f16(BM, min(p.N - n0, BN), 0, p.w_mn);
+      const uint32_t idesc = idesc_f16(2 * BM, n_end - n0, 0, p.w_mn);
       const uint32_t w_step = p.w_mn ? 128u : 2u;            // 16-byte units per K step of 16
       if (t0 < m_tiles && !mbar_wait(smem_u32(&sh->w_full), 0, abort)) { give_up(sh, status, 4); ok = false; }
       for (int t = t0; t < m_tiles && ok; t += t_step, ++tile_i) {
@@ -180,14 +193,14 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           const uint32_t w_addr = w_base + kb * W_BYTES;
           const uint64_t w_desc = p.w_mn ? smem_desc_mn_sw128(w_addr, BK * 128) : smem_desc_sw128(w_addr);
 #pragma unroll
-          for (int k = 0; k < BK / 16; ++k) mma_f16_ss(d_tmem, a_desc + 2 * k, w_desc + w_step * k, idesc, (kb || k) ? 1u : 0u);
-          tc_commit(smem_u32(&sh->empty[slot]));
+          for (int k = 0; k < BK / 16; ++k) mma_f16_ss_pair(d_tmem, a_desc + 2 * k, w_desc + w_step * k, idesc, (kb || k) ? 1u : 0u);
+          tc_commit_pair(smem_u32(&sh->empty[slot]));
           if (++slot == (uint32_t)n_st) { slot = 0; phase ^= 1; }
         }
-        if (ok) tc_commit(smem_u32(&sh->tmem_full[buf]));
+        if (ok) tc_commit_pair(smem_u32(&sh->tmem_full[buf]));
       }
       // every MMA issued must have retired before TMEM is freed (bounded, ignoring abort)
-      tc_commit(smem_u32(&sh->mma_done));
+      tc_commit_pair(smem_u32(&sh->mma_done));
       uint32_t spins = 0;
       while (!mbar_try_wait(smem_u32(&sh->mma_done), 0) && ++spins < kSpinLimit) {}
       if (spins >= kSpinLimit) give_up(sh, status, 6);
@@ -199,15 +212,12 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     // copy it out.
     const int q = warp & 3;                    // TMEM lane quadrant this warp may read
     const int h0 = ((warp - 2) >> 2) * (BN / 2), c0 = n0 + h0;   // first column of this warp's half, in the tile and in C
-    uint8_t* const stg0 = staging + (warp - 2) * (nbuf * STG_BYTES);
+    uint8_t* const stg0 = staging + (warp - 2) * (NBUF * STG_BYTES);
     uint8_t* stg = stg0;
     const int sub = lane >> 3, piece = lane & 7;   // copying the buffer out: row sub + 4 i, 16-byte piece
     auto wait_staging = [&]() {                // the block that used the buffer last has left it
-      if (nbuf == 2) stg = stg == stg0 ? stg0 + STG_BYTES : stg0;
-      if (tma_c && lane == 0) {
-        if (nbuf == 2) bulk_wait_read<1>();
-        else bulk_wait_read<0>();
-      }
+      stg = stg == stg0 ? stg0 + STG_BYTES : stg0;
+      if (tma_c && lane == 0) bulk_wait_read<1>();
       __syncwarp();
     };
     auto put = [&](int pc, uint4 v) { *reinterpret_cast<uint4*>(stg + lane * 128 + ((pc ^ (lane & 7)) << 4)) = v; };
@@ -231,7 +241,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     };
     uint32_t tile_i = 0;
     for (int t = t0; t < m_tiles; t += t_step, ++tile_i) {
-      const int64_t m0 = (int64_t)t * BM + q * 32;           // this warp's first row
+      const int64_t m0 = ((int64_t)t * 2 + rank) * BM + q * 32;    // this warp's first row
       const int buf = tile_i & 1;
       const int64_t row = m0 + lane;
       const bool live = row < p.M;
@@ -257,7 +267,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         }
         __syncwarp();
         const int c = x + piece * (16 / elem);
-        if (c >= p.N) return;
+        if (c >= n_end) return;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           if (crow[i] < 0) continue;
@@ -270,13 +280,13 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       Row32 res;
       if (HAS_R && live) {
         rrow = p.R + p.rmap(row) * (int64_t)p.ldr;
-        if (c0 < p.N) res.load(rrow + c0, p.N - c0, r32);
-        const int64_t rown = row + (int64_t)t_step * BM;     // the next tile's residual rows into L2
+        if (c0 < n_end) res.load(rrow + c0, n_end - c0, r32);
+        const int64_t rown = row + (int64_t)t_step * 2 * BM; // the next tile's residual rows into L2
         if (rown < p.M) {
           const float* rn = p.R + p.rmap(rown) * (int64_t)p.ldr + c0;
 #pragma unroll
           for (int c = 0; c < BN / 2; c += 32)
-            if (c0 + c < p.N) prefetch_l2(rn + c);
+            if (c0 + c < n_end) prefetch_l2(rn + c);
         }
       }
       if (!mbar_wait_warp(smem_u32(&sh->tmem_full[buf]), (tile_i >> 1) & 1, abort)) {
@@ -288,10 +298,10 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       if (HAS_R || p.out_f32) {
         // ---- 32 columns at a time
         uint32_t a[32];
-        if (c0 < p.N) tmem_ld32(tbase, a);
+        if (c0 < n_end) tmem_ld32(tbase, a);
 #pragma unroll 1
         for (int st = 0; st < BN / 64; ++st) {
-          const int col = c0 + 32 * st, left = p.N - col;    // columns from here on
+          const int col = c0 + 32 * st, left = n_end - col;    // columns from here on
           if (left <= 0) break;                              // warp-uniform
           tmem_wait_ld();
           finish(a, 32 * st);
@@ -320,18 +330,18 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       } else {
         // ---- fp16, 64 columns at a time
         uint32_t a[32], b[32], h[32];
-        if (c0 < p.N) {
+        if (c0 < n_end) {
           tmem_ld32(tbase, a);
           tmem_ld32(tbase + 32, b);
         }
 #pragma unroll 1
         for (int st = 0; st < BN / 128; ++st) {
           const int col = c0 + 64 * st;
-          if (col >= p.N) break;
+          if (col >= n_end) break;
           uint32_t w0 = 0, w1 = 0;
           if (p.bits_in && live) {
             w0 = p.bits_in[(int64_t)(col >> 5) * p.bits_ld + row];
-            if (col + 32 < p.N) w1 = p.bits_in[(int64_t)((col >> 5) + 1) * p.bits_ld + row];
+            if (col + 32 < n_end) w1 = p.bits_in[(int64_t)((col >> 5) + 1) * p.bits_ld + row];
           }
           tmem_wait_ld();
           finish(a, 64 * st);
@@ -340,7 +350,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           finish(b, 64 * st + 32);
 #pragma unroll
           for (int j = 0; j < 16; ++j) h[16 + j] = pack_half2(__uint_as_float(b[2 * j]), __uint_as_float(b[2 * j + 1]));
-          if (st + 1 < BN / 128 && col + 64 < p.N) {
+          if (st + 1 < BN / 128 && col + 64 < n_end) {
             tmem_ld32(tbase + 64 * (st + 1), a);
             tmem_ld32(tbase + 64 * (st + 1) + 32, b);
           }
@@ -353,7 +363,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           }
           if (p.bits_out && live) {
             p.bits_out[(int64_t)(col >> 5) * p.bits_ld + row] = positive_bits(h);
-            if (col + 32 < p.N) p.bits_out[(int64_t)((col >> 5) + 1) * p.bits_ld + row] = positive_bits(h + 16);
+            if (col + 32 < n_end) p.bits_out[(int64_t)((col >> 5) + 1) * p.bits_ld + row] = positive_bits(h + 16);
           }
           wait_staging();
 #pragma unroll
@@ -363,7 +373,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(smem_u32(&sh->tmem_empty[buf]));
+      if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->tmem_empty[buf]), 0));
     }
     if (tma_c && lane == 0) bulk_wait_all();      // the stores are complete before the CTA exits
   }
@@ -371,21 +381,24 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
+  cluster_sync_all();          // the leader's MMAs read the peer's shared memory until they retire
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    tmem_dealloc_pair(tmem_base, TMEM_COLS);
   }
 }
 }  // namespace
 
 // Dense fp32 rows without a residual stay with gemm_tc5.cu (475 K x 256 x 128: 105 us there, 120 here: four stores per half
 // tile either way, nothing to overlap them with); rows placed by a map come here, where runs of 8 leave by TMA (2.1 M token
-// rows x 256, K = 64: 827 -> 631 us, bound by the 2.1 GB it writes).  K <= 256 in whole k-blocks or row-contraction weights, and at least three row tiles per CTA for the resident weights:
-// with one or two their load (128 KB before the first MMA) costs more than it saves.  fp16 masks are read by
-// gemm_tc5.cu (here only as bits).
+// rows x 256, K = 64: 827 -> 631 us, bound by the 2.1 GB it writes).
+// K <= 256 in whole k-blocks or row-contraction weights, N in the 32-column steps of a pair's MMAs, and at least three row
+// tiles per CTA for the resident weights: with one or two their load before the first MMA costs more than it saves.  fp16
+// masks are read by gemm_tc5.cu (here only as bits).
 bool linear_res_ok(const LinearArgs& p) {
   const int64_t tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
-  return !p.a_mn && !p.mask && (!p.out_f32 || p.R || !dense_rows(p.cmap)) && !p.a_sums && p.k_splits <= 1 && p.K <= 4 * BK && p.M <= 0x7fffff00 && tiles >= 3ll * sm_count() &&
+  return !p.a_mn && !p.mask && (!p.out_f32 || p.R || !dense_rows(p.cmap)) && !p.a_sums && p.k_splits <= 1 && p.K <= 4 * BK &&
+         p.N % 32 == 0 && p.M <= 0x7ffffe00 && tiles >= 3ll * sm_count() &&
          (!(p.bits_in || p.bits_out) || (!p.out_f32 && !p.R && p.N % 32 == 0)) && linear_tc5_ok(p);
 }
 
@@ -398,7 +411,7 @@ int linear_res(const LinearArgs& p, cudaStream_t stream) {
   if (!status) return BSRL_ERR_CUDA;
   CUtensorMap tm_a, tm_w;
   if (!make_tmap_f16(&tm_a, p.A, p.M, p.K, p.lda, BM)) return BSRL_ERR_CUDA;
-  if (p.w_mn ? !make_tmap_mn(&tm_w, p.W, p.K, p.N, p.ldw, BK, BN / 64) : !make_tmap_f16(&tm_w, p.W, p.N, p.K, p.ldw, BN))
+  if (p.w_mn ? !make_tmap_f16(&tm_w, p.W, p.K, p.N, p.ldw, BK) : !make_tmap_f16(&tm_w, p.W, p.N, p.K, p.ldw, BN / 2))
     return BSRL_ERR_CUDA;
   const int tma_c = store_box_rows(p.cmap, p.M);
   CUtensorMap tm_c = tm_a;
@@ -409,10 +422,11 @@ int linear_res(const LinearArgs& p, cudaStream_t stream) {
     return e != cudaSuccess ? e : cudaFuncSetAttribute(linear_res_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   });
   if (rc != BSRL_OK) return rc;
-  const int m_tiles = (int)((p.M + BM - 1) / BM), n_tiles = (p.N + BN - 1) / BN;
+  const int bn = p.N > BN && p.N % BN != 0 && p.N % 192 == 0 ? 192 : BN;       // even column tiles where the width has them
+  const int m_tiles = (int)((p.M + 2 * BM - 1) / (2 * BM)), n_tiles = (p.N + bn - 1) / bn;
   const int r32 = p.R && reinterpret_cast<uintptr_t>(p.R) % 32 == 0 && p.ldr % 8 == 0;        // 32-byte residual loads
   auto* kernel = p.R ? linear_res_kernel<true> : linear_res_kernel<false>;
-  launch_kernel(kernel, sm_count(), THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, tma_c, r32, p, m_tiles, n_tiles, status);
+  launch_kernel<2>(kernel, (unsigned)(sm_count() & ~1), THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, tma_c, r32, p, bn, m_tiles, n_tiles, status);
   BSRL_LAUNCH_OK("linear_res_kernel");
   return BSRL_OK;
 }

@@ -510,3 +510,14 @@ def test_qkv_attention_split_groups(native, B, d, H, body):
 
     few, many = run(1), run(-(-700 // B))
     assert not bool(torch.isnan(few).any()) and torch.equal(few, many[:B * T])
+
+
+@pytest.mark.parametrize("m,n,k,relu,res", [
+    (19201, 576, 192, 0, False),        # three column tiles of 192, one row in the last tile of 256
+    (19073, 544, 256, 1, False),        # 256 + 256 + 32 columns, an odd number of 128-row tiles
+    (56833, 32, 64, 2, False),          # the narrowest pair MMA
+    (56961, 160, 128, 0, True),         # fp32 rows with a residual, 80 columns per CTA
+])
+def test_linear_resident_weights_on_pairs(native, m, n, k, relu, res):
+    """The resident-weight kernel's column halves and row remainders per CTA pair; bounds as in test_linear_resident_weights."""
+    test_linear_resident_weights(native, m, n, k, relu, res)
