@@ -1,6 +1,6 @@
 """CPU oracle for the batched transformer-policy forward (TEST INFRASTRUCTURE).
 
-This file is the checker, not the product.  Only tests, the smoke check and
+This file is the oracle, not the product.  Only tests, the smoke check and
 the CPU-baseline leg of the benchmark may import it; the CUDA path never does.
 
 It restates, in plain torch fp32 on the CPU, the arithmetic of the reference's
