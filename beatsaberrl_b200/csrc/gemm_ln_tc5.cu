@@ -12,18 +12,20 @@
 // stages are enough for K = d, and every epilogue warp has three 4 KB row buffers, through which the residual arrives
 // and the sum leaves by TMA.  N = K = 512, 950 K rows: one CTA with all 512 columns, MMAs and epilogue in turn 1516 us;
 // cluster with row loads by the threads 1376; residual by TMA, two buffers and three stages 1290; this 1089 (5.4 TB/s;
-// 905 at copy speed).  N = K = 256: 921 -> 569 us.
+// 905 at copy speed).  Passing the running sums on instead of adding four column ranges: 1172 us against 1173 on one box.
 //
 //   warp 0      TMA producer: stages of a (128 x 64) A chunk + this CTA's (N_cta x 64) weight chunk
 //   warp 1      MMA issuer
 //   warps 2..9  epilogue, thread = row; warp w reads TMEM lane quadrant w & 3 and owns column half (w - 2) / 4:
 //     pass 1    32 columns at a time: residual block in a row buffer + accumulator + bias -> stream rows, in place and
-//               out by TMA; row sums of x and x^2; x back into TMEM.  The block after the next is requested meanwhile
-//               and the next tile's rows are pulled into L2
-//     exchange  partial sums of the row's two (CL = 1) or four (CL = 2) column ranges
+//               out by TMA; sums of x and x^2 of each four columns; x back into TMEM.  The block after the next is
+//               requested meanwhile and the next tile's rows are pulled into L2
+//     sums      the low columns' warp hands its eight running sums to the high columns' warp, which finishes the row's sum
+//               over the CTA's columns and sends it to the peer (CL = 2)
 //     pass 2    TMEM -> (x - mean) rstd gamma + beta -> fp16 -> row buffer -> TMA store
 //
-// Statistics are fp32 sums of x and x^2.
+// Statistics are fp32 sums of x and x^2 in one fixed order, which the LayerNorm rows' last bit depends on: per CTA eight
+// running sums (sum p over columns 4 p .. 4 p + 3 of every block of 32, blocks in order), added pairwise, then the two CTAs'.
 // Stands in for out_proj + ln_ffn.forward_add (python/policy.py:655-668; ln_fwd_add,
 // python/beat_arena_env/csrc/layer_norm.cu) where the fused block tail does not reach.  All waits are bounded.
 #include "kernels.cuh"
@@ -43,12 +45,14 @@ constexpr int EPI_WARPS = 8;
 constexpr int THREADS = (2 + EPI_WARPS) * 32;
 constexpr int STG_BYTES = 32 * 128;              // a row buffer: 32 rows x 32 fp32 or 64 fp16 columns
 constexpr int PRM_BYTES = 3 * MAX_NC * 4;        // bias | gamma | beta
-constexpr int PART_BYTES = 2 * 4 * BM * 8;       // per tile parity, column range and row: (sum, sum of squares)
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * BUFS * STG_BYTES + PRM_BYTES + PART_BYTES + 1024 + 512;
+constexpr int MAX_NX = MAX_NC / 64;              // 32-column blocks per epilogue warp
+constexpr int PART_BYTES = 2 * 2 * BM * 8;       // per tile parity, CTA and row: (sum, sum of squares)
+constexpr int CARRY_BYTES = 8 * BM * 8;          // per running sum and row: (sum, sum of squares) of the low columns
+constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * BUFS * STG_BYTES + PRM_BYTES + PART_BYTES + CARRY_BYTES + 1024 + 512;
 constexpr int KERNEL_ID = 6;
 
 struct Shared {
-  uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], stats[2], row_full[EPI_WARPS][BUFS], mma_done;
+  uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2], carry[4], stats[2], row_full[EPI_WARPS][BUFS], mma_done;
   uint32_t tmem_base;
   int abort;
 };
@@ -91,7 +95,8 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   uint8_t* staging = smem_raw + (ring - raw) + STAGES * STAGE_BYTES;
   float* prm = reinterpret_cast<float*>(staging + EPI_WARPS * BUFS * STG_BYTES);
   float2* part = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(prm) + PRM_BYTES);
-  Shared* sh = reinterpret_cast<Shared*>(reinterpret_cast<uint8_t*>(part) + PART_BYTES);
+  float2* carry = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(part) + PART_BYTES);
+  Shared* sh = reinterpret_cast<Shared*>(reinterpret_cast<uint8_t*>(carry) + CARRY_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = CL == 2 ? cluster_rank() : 0u;
   const int nc = p.nc, col_cta = (int)rank * nc, k_blocks = p.K / BK;
@@ -106,8 +111,9 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&sh->acc_full[b]), 1);
       mbar_init(smem_u32(&sh->acc_empty[b]), EPI_WARPS);
-      mbar_init(smem_u32(&sh->stats[b]), EPI_WARPS);
+      mbar_init(smem_u32(&sh->stats[b]), EPI_WARPS / 2);
     }
+    for (int i = 0; i < 4; ++i) mbar_init(smem_u32(&sh->carry[i]), 1);
     for (int w = 0; w < EPI_WARPS; ++w)
       for (int b = 0; b < BUFS; ++b) mbar_init(smem_u32(&sh->row_full[w][b]), 1);
     mbar_init(smem_u32(&sh->mma_done), 1);
@@ -242,15 +248,17 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       tc_fence_after();
       const uint32_t tbase = tmem_base + ((uint32_t)(q * 32) << 16) + buf * MAX_NC + lo;
       // ---- pass 1
-      float sum = 0.f, sq = 0.f;
+      float e1[MAX_NX][8], e2[MAX_NX][8];                    // per block: sums over four columns each
       uint32_t r[32];
       tmem_ld32(tbase, r);
-#pragma unroll 1
-      for (int c = 0; c < hc; c += 32) {
+#pragma unroll
+      for (int b = 0; b < MAX_NX; ++b) {
+        const int c = 32 * b;
+        if (!ok || c >= hc) continue;
         if (!mbar_wait_warp(smem_u32(row_full + use_b), (parity >> use_b) & 1, abort)) {
           if (lane == 0) give_up(sh, p.status, 8);
           ok = false;
-          break;
+          continue;
         }
         parity ^= 1u << use_b;
         pending &= ~(1u << use_b);
@@ -262,8 +270,8 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           const float4 bv = *reinterpret_cast<const float4*>(prm + lo + c + 4 * j), rv = *cell;
           const float v0 = (__uint_as_float(r[4 * j]) + bv.x) + rv.x, v1 = (__uint_as_float(r[4 * j + 1]) + bv.y) + rv.y;
           const float v2 = (__uint_as_float(r[4 * j + 2]) + bv.z) + rv.z, v3 = (__uint_as_float(r[4 * j + 3]) + bv.w) + rv.w;
-          sum += (v0 + v1) + (v2 + v3);
-          sq += (v0 * v0 + v1 * v1) + (v2 * v2 + v3 * v3);
+          e1[b][j] = (v0 + v1) + (v2 + v3);
+          e2[b][j] = fmaf(v0, v0, v1 * v1) + fmaf(v2, v2, v3 * v3);
           r[4 * j] = __float_as_uint(v0); r[4 * j + 1] = __float_as_uint(v1);
           r[4 * j + 2] = __float_as_uint(v2); r[4 * j + 3] = __float_as_uint(v3);
           *cell = make_float4(v0, v1, v2, v3);
@@ -276,29 +284,56 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       }
       if (!ok) break;
       tmem_wait_st();
-      // ---- exchange: the row's partial sums, in column order
-      float2* pt = part + buf * (4 * BM);
-      const int mine = (int)rank * 2 + half;
-      pt[mine * BM + trow] = make_float2(sum, sq);
-      if (CL == 2)
-        st_async_f2(map_to_cta(smem_u32(pt + mine * BM + trow), rank ^ 1), make_float2(sum, sq), map_to_cta(smem_u32(&sh->stats[buf]), rank ^ 1));
-      __syncwarp();
-      if (lane == 0) {
-        if (CL == 2) mbar_expect_tx(smem_u32(&sh->stats[buf]), 32 * 8);      // what the peer's warp of this place sends
-        else mbar_arrive(smem_u32(&sh->stats[buf]));
+      // ---- sums: the row's eight running sums pass from the low columns' warp to the high columns' warp of its quadrant
+      float2* pt = part + buf * (2 * BM);
+      if (half && !mbar_wait_warp(smem_u32(&sh->carry[q]), tile_i & 1, abort)) {
+        if (lane == 0) give_up(sh, p.status, 9);
+        break;
+      }
+      float2 run[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        run[j] = half ? carry[j * BM + trow] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int b = 0; b < MAX_NX; ++b)
+          if (b < nx) {
+            run[j].x += e1[b][j];
+            run[j].y += e2[b][j];
+          }
+      }
+      if (half == 0) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) carry[j * BM + trow] = run[j];
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&sh->carry[q]));
+      } else {
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1)
+#pragma unroll
+          for (int j = 0; j < 8; j += 2 * o) {
+            run[j].x += run[j + o].x;
+            run[j].y += run[j + o].y;
+          }
+        pt[rank * BM + trow] = run[0];
+        if (CL == 2)
+          st_async_f2(map_to_cta(smem_u32(pt + rank * BM + trow), rank ^ 1), run[0], map_to_cta(smem_u32(&sh->stats[buf]), rank ^ 1));
+        __syncwarp();
+        if (lane == 0) {
+          if (CL == 2) mbar_expect_tx(smem_u32(&sh->stats[buf]), 32 * 8);    // what the peer's warp of this place sends
+          else mbar_arrive(smem_u32(&sh->stats[buf]));
+        }
       }
       if (!mbar_wait_warp(smem_u32(&sh->stats[buf]), (tile_i >> 1) & 1, abort)) {
         if (lane == 0) give_up(sh, p.status, 7);
         break;
       }
-      float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-      for (int i = 0; i < 2 * CL; ++i) {
-        const float2 o = pt[i * BM + trow];
+      float2 s = pt[trow];
+      if (CL == 2) {
+        const float2 o = pt[BM + trow];
         s.x += o.x;
         s.y += o.y;
       }
-      const float mean = s.x * p.inv_n, rstd = rsqrtf(fmaxf(s.y * p.inv_n - mean * mean, 0.f) + p.eps);
+      const float mean = s.x * p.inv_n, rstd = rsqrtf(fmaxf(fmaf(s.y, p.inv_n, -(mean * mean)), 0.f) + p.eps);
       // ---- pass 2: 64 columns (128 bytes of fp16) per store; a last block of 32 goes out directly
       tmem_ld32(tbase, r);
 #pragma unroll 1
@@ -313,10 +348,10 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             const float4 g = *reinterpret_cast<const float4*>(prm + MAX_NC + lo + c + 8 * j + 4 * e);
             const float4 b = *reinterpret_cast<const float4*>(prm + 2 * MAX_NC + lo + c + 8 * j + 4 * e);
             const uint32_t* a = r + 8 * j + 4 * e;
-            v[4 * e] = (__uint_as_float(a[0]) - mean) * rstd * g.x + b.x;
-            v[4 * e + 1] = (__uint_as_float(a[1]) - mean) * rstd * g.y + b.y;
-            v[4 * e + 2] = (__uint_as_float(a[2]) - mean) * rstd * g.z + b.z;
-            v[4 * e + 3] = (__uint_as_float(a[3]) - mean) * rstd * g.w + b.w;
+            v[4 * e] = fmaf((__uint_as_float(a[0]) - mean) * rstd, g.x, b.x);
+            v[4 * e + 1] = fmaf((__uint_as_float(a[1]) - mean) * rstd, g.y, b.y);
+            v[4 * e + 2] = fmaf((__uint_as_float(a[2]) - mean) * rstd, g.z, b.z);
+            v[4 * e + 3] = fmaf((__uint_as_float(a[3]) - mean) * rstd, g.w, b.w);
           }
           y[j] = make_uint4(pack_half2(v[0], v[1]), pack_half2(v[2], v[3]), pack_half2(v[4], v[5]), pack_half2(v[6], v[7]));
         }

@@ -273,6 +273,44 @@ def test_linear_ln(native, m, n, k, in_place):
     torch.testing.assert_close(h.float().cpu(), ref_h, atol=4e-3, rtol=2e-3)
 
 
+def _ln_rows_in_order(x, gamma, beta, eps):
+    """LayerNorm rows of fp32 `x` with every sum in linear_ln's order, operation by operation in fp32 (a fused multiply-add as
+    float64 arithmetic rounded to fp32: the product is exact there)."""
+    m, n = x.shape
+    fma = lambda a, b, c: (a.double() * b.double() + c.double()).float()  # noqa: E731
+    inv_n = torch.tensor(1.0, device=x.device) / n
+    parts = x.view(m, 2 if n > 256 else 1, -1, 8, 4)         # CTA, block of 32 columns, four columns each
+    v = parts.unbind(-1)
+    sums = []
+    for e in ((v[0] + v[1]) + (v[2] + v[3]), fma(v[0], v[0], v[1] * v[1]) + fma(v[2], v[2], v[3] * v[3])):
+        run = torch.zeros_like(e[:, :, 0])
+        for b in range(e.shape[2]):
+            run = run + e[:, :, b]
+        for _ in range(3):                                   # pairs of neighbours
+            run = run[..., 0::2] + run[..., 1::2]
+        sums.append(run[:, 0, 0] + run[:, 1, 0] if run.shape[1] == 2 else run[:, 0, 0])
+    mean = sums[0] * inv_n
+    rstd = torch.rsqrt(fma(sums[1], inv_n, -(mean * mean)).clamp_min(0) + torch.tensor(eps, device=x.device))
+    return fma((x - mean[:, None]) * rstd[:, None], gamma.expand_as(x), beta.expand_as(x)).half()
+
+
+@pytest.mark.parametrize("m,n,k", [(4099, 512, 512), (19001, 512, 64), (1000, 384, 128), (300, 256, 256), (257, 192, 64), (513, 64, 64)])
+def test_linear_ln_sums_in_order(native, m, n, k):
+    """The LayerNorm rows depend on their sums' order in the last bit, and a policy's outputs on the rows: the order is part of
+    what the kernel computes.  Its stream rows are taken as they came out, so every bit of h follows from them."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn(m, k, generator=g, device="cuda").half()
+    w = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).half()
+    bias, res = torch.randn(n, generator=g, device="cuda") * 0.3, torch.randn(m, n, generator=g, device="cuda") * 2 + 0.5
+    gamma, beta = 1 + 0.2 * torch.randn(n, generator=g, device="cuda"), 0.1 * torch.randn(n, generator=g, device="cuda")
+    x = torch.full((m, n), float("nan"), device="cuda")
+    h = torch.full((m, n), float("nan"), dtype=torch.float16, device="cuda")
+    native.check(native.lib.bsrl_linear_ln(a.data_ptr(), w.data_ptr(), bias.data_ptr(), res.data_ptr(), gamma.data_ptr(),
+                                           beta.data_ptr(), 1e-5, m, n, k, x.data_ptr(), h.data_ptr(), _stream()))
+    native.check(native.lib.bsrl_device_status())
+    assert torch.equal(h, _ln_rows_in_order(x, gamma, beta, 1e-5))
+
+
 def _native_cfg(native, cfg):
     return native.make_config(cfg.embed, cfg.n_heads, cfg.n_blocks, cfg.ffn_mult, cfg.trunk_dim,
                               cfg.trunk_hidden, cfg.value_bins, cfg.note_geo, cfg.head_gears,
