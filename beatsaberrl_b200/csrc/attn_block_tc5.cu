@@ -260,7 +260,7 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
         const int g_lo = first_group(i), g_hi = min(g_lo + per_item, n_groups);
         for (int g = g_lo; g < g_hi && ok; ++g, ++gi) {
           const int buf = gi & 1;
-          if (!mbar_wait(smem_u32(&sh->acc_empty[buf]), ((gi >> 1) & 1) ^ 1, abort)) { give_up(sh, p.status, 5); ok = false; break; }
+          if (!mbar_wait<PAIR>(smem_u32(&sh->acc_empty[buf]), ((gi >> 1) & 1) ^ 1, abort)) { give_up(sh, p.status, 5); ok = false; break; }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + buf * 256;
           for (int kb = 0; kb < KB; ++kb, ++it) {

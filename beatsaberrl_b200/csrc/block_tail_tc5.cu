@@ -357,6 +357,10 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
       uint32_t it = 0, tile_i = 0, n_hid = 0;
       bool ok = true;
       const uint32_t idesc_d = idesc_f16(CTAS * BM, d), idesc_h = idesc_f16(CTAS * BM, HC);
+      // for the epilogue warps' operands, of a pair: both CTAs'
+      auto wait_epilogue = [&](uint32_t bar, uint32_t parity) -> bool {
+        return mbar_wait<PAIR>(bar, parity, abort);
+      };
       // completion of the MMAs issued so far -> the barrier
       auto commit_at = [&](uint32_t bar) {                 // in both CTAs of a pair
         if (PAIR) tc_commit_pair(bar);
@@ -408,12 +412,12 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         // FFN-down of one hidden chunk: its two 64-column halves as the epilogue publishes them, N = 256
         auto down = [&](auto n_, uint32_t xcol, uint32_t hid_par) -> bool {
           constexpr int n = decltype(n_)::value;
-          if (!mbar_wait(smem_u32(&sh->hid_ready[0]), hid_par, abort)) { give_up(sh, p.status, 9); return false; }
+          if (!wait_epilogue(smem_u32(&sh->hid_ready[0]), hid_par)) { give_up(sh, p.status, 9); return false; }
           if (!wait_stage(StageNo<n>{})) return false;
           mma_kblock_desc<PAIR>(xcol, hd0, rd0 + kSlot * (n % 3), idesc_d, false);
           release_stage(StageNo<n>{});
           commit(&sh->hid_free[0]);
-          if (!mbar_wait(smem_u32(&sh->hid_ready[1]), hid_par, abort)) { give_up(sh, p.status, 9); return false; }
+          if (!wait_epilogue(smem_u32(&sh->hid_ready[1]), hid_par)) { give_up(sh, p.status, 9); return false; }
           if (!wait_stage(StageNo<n + 1>{})) return false;
           mma_kblock_desc<PAIR>(xcol, hd0 + kChunk, rd0 + kSlot * ((n + 1) % 3), idesc_d, false);
           release_stage(StageNo<n + 1>{});
@@ -425,7 +429,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           const uint32_t xcol = tmem_base + (par ? 256u : 0u);     // region X of this tile
           const uint32_t acol = tmem_base + (par ? 0u : 256u);     // two hidden-chunk buffers
           TAIL_WAIT(&sh->a_full, par, 6);
-          TAIL_WAIT(&sh->x_ready, par, 7);
+          if (!wait_epilogue(smem_u32(&sh->x_ready), par)) { give_up(sh, p.status, 7); ok = false; break; }
           tc_fence_after();
           // x1 = x (pre-stored) + att Wo^T: stages 0..3
           ok = wait_stage(StageNo<0>{});
@@ -445,7 +449,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           mma_kblock_desc<PAIR>(xcol, ad0 + 3 * kChunk, rd0, idesc_d, false);
           release_stage(StageNo<3>{});
           commit(&sh->o_done);
-          TAIL_WAIT(&sh->h2_ready, par, 8);
+          if (!wait_epilogue(smem_u32(&sh->h2_ready), par)) { give_up(sh, p.status, 8); ok = false; break; }
           tc_fence_after();
           // hidden chunks 0 and 1: stages 4..7
           ok = up(StageNo<4>{}, acol, &sh->acc1_full[0]) && up(StageNo<6>{}, acol + HC, &sh->acc1_full[1]);
@@ -493,12 +497,12 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         };
         auto down = [&](auto n_, uint32_t xcol, uint32_t hid_par) -> bool {
           constexpr int n = decltype(n_)::value;
-          if (!mbar_wait(smem_u32(&sh->hid_ready[0]), hid_par, abort)) { give_up(sh, p.status, 9); return false; }
+          if (!wait_epilogue(smem_u32(&sh->hid_ready[0]), hid_par)) { give_up(sh, p.status, 9); return false; }
           if (!wait_stage(StageNo<n>{})) return false;
           mma_kblock_desc<PAIR>(xcol, hd0, rd0 + kSlot * (n % 3), idesc_d, false);
           release_stage(StageNo<n>{});
           commit(&sh->hid_free[0]);
-          if (!mbar_wait(smem_u32(&sh->hid_ready[1]), hid_par, abort)) { give_up(sh, p.status, 9); return false; }
+          if (!wait_epilogue(smem_u32(&sh->hid_ready[1]), hid_par)) { give_up(sh, p.status, 9); return false; }
           if (!wait_stage(StageNo<n + 1>{})) return false;
           mma_kblock_desc<PAIR>(xcol, hd0 + kChunk, rd0 + kSlot * ((n + 1) % 3), idesc_d, false);
           release_stage(StageNo<n + 1>{});
@@ -511,7 +515,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           const uint32_t acol = tmem_base + (par ? 0u : 256u);     // two hidden-chunk buffers
           flip = par;
           TAIL_WAIT(&sh->a_full, par, 6);
-          TAIL_WAIT(&sh->x_ready, par, 7);
+          if (!wait_epilogue(smem_u32(&sh->x_ready), par)) { give_up(sh, p.status, 7); ok = false; break; }
           tc_fence_after();
           // x1 = x (pre-stored) + att Wo^T: stages 0..2
           ok = wait_stage(StageNo<0>{});
@@ -527,7 +531,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           mma_kblock_desc<PAIR>(xcol, ad0 + 2 * kChunk, rd0 + 2 * kSlot, idesc_d, false);
           release_stage(StageNo<2>{});
           commit(&sh->o_done);
-          TAIL_WAIT(&sh->h2_ready, par, 8);
+          if (!wait_epilogue(smem_u32(&sh->h2_ready), par)) { give_up(sh, p.status, 8); ok = false; break; }
           tc_fence_after();
           // hidden chunks 0 and 1 (stages 3..6), then chunk j's FFN-down and chunk j + 2's FFN-up for j = 0..3
           // (stages 7..22), then the FFN-down of chunks 4 and 5 (stages 23..26); the hidden-chunk barriers complete
@@ -560,19 +564,19 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           return true;
         };
         TAIL_WAIT(&sh->a_full, par, 6);
-        TAIL_WAIT(&sh->x_ready, par, 7);
+        if (!wait_epilogue(smem_u32(&sh->x_ready), par)) { give_up(sh, p.status, 7); ok = false; break; }
         tc_fence_after();
         for (int kb = 0; kb < KB && ok; ++kb)       // x1 = x (pre-stored) + att Wo^T
           ok = with_stage([&](uint32_t st) { mma_kblock<PAIR>(xcol, sA + kb * CHUNK_BYTES, st, idesc_d, true); });
         if (!ok) break;
         commit(&sh->o_done);
-        TAIL_WAIT(&sh->h2_ready, par, 8);
+        if (!wait_epilogue(smem_u32(&sh->h2_ready), par)) { give_up(sh, p.status, 8); ok = false; break; }
         tc_fence_after();
         ok = g1(0) && g1(1);
         if (NC == 2 && ok) commit(&sh->a_free);
         for (int j = 0; j < NC && ok; ++j) {
           for (int kc = 0; kc < 2 && ok; ++kc) {    // xo += hidden chunk j * W2[:, chunk j]^T, one 64-column half at a time
-            if (!mbar_wait(smem_u32(&sh->hid_ready[kc]), n_hid & 1, abort)) { give_up(sh, p.status, 9); ok = false; break; }
+            if (!wait_epilogue(smem_u32(&sh->hid_ready[kc]), n_hid & 1)) { give_up(sh, p.status, 9); ok = false; break; }
             tc_fence_after();
             ok = with_stage([&](uint32_t st) { mma_kblock<PAIR>(xcol, sH + kc * CHUNK_BYTES, st, idesc_d, true); });
             if (ok) commit(&sh->hid_free[kc]);   // this half of sH may be overwritten once retired

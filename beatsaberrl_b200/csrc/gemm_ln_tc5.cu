@@ -323,7 +323,7 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           else mbar_arrive(smem_u32(&sh->stats[buf]));
         }
       }
-      if (!mbar_wait_warp(smem_u32(&sh->stats[buf]), (tile_i >> 1) & 1, abort)) {
+      if (!mbar_wait_warp<CL == 2>(smem_u32(&sh->stats[buf]), (tile_i >> 1) & 1, abort)) {
         if (lane == 0) give_up(sh, p.status, 7);
         break;
       }

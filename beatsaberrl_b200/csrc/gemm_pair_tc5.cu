@@ -147,7 +147,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       const uint32_t w_step16 = p.w_mn ? 128u : 2u;          // 16-byte units per K step of 16
       for (int w = w_first; w < n_work && ok; w += w_step, ++tile_i) {
         const int buf = tile_i & 1;
-        if (!mbar_wait(smem_u32(&sh->tmem_empty[buf]), ((tile_i >> 1) & 1) ^ 1, abort)) { give_up(sh, status, 3); ok = false; break; }
+        if (!mbar_wait<true>(smem_u32(&sh->tmem_empty[buf]), ((tile_i >> 1) & 1) ^ 1, abort)) { give_up(sh, status, 3); ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
         for (int kb = 0; kb < k_blocks; ++kb) {

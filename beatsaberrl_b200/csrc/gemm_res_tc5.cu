@@ -183,7 +183,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       if (t0 < m_tiles && !mbar_wait(smem_u32(&sh->w_full), 0, abort)) { give_up(sh, status, 4); ok = false; }
       for (int t = t0; t < m_tiles && ok; t += t_step, ++tile_i) {
         const int buf = tile_i & 1;
-        if (!mbar_wait(smem_u32(&sh->tmem_empty[buf]), ((tile_i >> 1) & 1) ^ 1, abort)) { give_up(sh, status, 3); ok = false; break; }
+        if (!mbar_wait<true>(smem_u32(&sh->tmem_empty[buf]), ((tile_i >> 1) & 1) ^ 1, abort)) { give_up(sh, status, 3); ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + buf * BN;
         for (int kb = 0; kb < k_blocks; ++kb) {

@@ -30,35 +30,49 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+// CLUSTER: the barrier is one that threads of the pair's other CTA arrive at (mbar_arrive_cluster) or store with (st.async)
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
+  if (CLUSTER)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 // Bounded wait: false when `limit` polls ran out or another role already gave up (*abort != 0).
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity, volatile int* abort, uint32_t limit) {
   for (uint32_t i = 0; i < limit; ++i) {
-    if (mbar_try_wait(bar, parity)) return true;   // the hardware parks the thread inside try_wait
+    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;   // the hardware parks the thread inside try_wait
     if ((i & 1023u) == 1023u && *abort) return false;
   }
   return false;
 }
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort) {
-  return mbar_wait_limit(bar, parity, abort, kSpinLimit);
+  return mbar_wait_limit<CLUSTER>(bar, parity, abort, kSpinLimit);
 }
 
 // Whole-warp bounded wait: only lane 0 polls the barrier (32 lanes polling the same word would
 // compete with the tensor core's operand reads for shared-memory bandwidth); the outcome is
 // broadcast.  Must be called by all 32 lanes.
+template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort) {
   int ok = 1;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort) ? 1 : 0;
+  if ((threadIdx.x & 31) == 0) ok = mbar_wait<CLUSTER>(bar, parity, abort) ? 1 : 0;
   return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
@@ -222,10 +236,16 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
-// (the form with .release.cluster costs ~3,000 cycles here: it waits for everything the thread has in flight; what this
-// arrival orders are tcgen05.ld's, which tcgen05.fence::before_thread_sync does)
+// Arrival at the leader's barrier: what this thread and those synchronised with it did to TMEM and wrote to this CTA's
+// shared memory comes before what follows a mbar_wait<true> there.  The fence releases shared memory only: 2.66 ms per
+// 1.9 M rows of the block tail, as with an arrival of CTA scope, which promises nothing across CTAs; the arrival's own
+// .release.cluster, which also waits for global transfers, costs 3.12 (on the lane with TMA stores in flight 3.22, passed on
+// by the peer's idle MMA warp 3.14).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile(
+      "fence.release.sync_restrict::shared::cta.cluster;\n\t"
+      "mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
+      : "memory");
 }
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");

@@ -1,0 +1,42 @@
+"""What the kernels on CTA pairs promise each other, read from their source: a race between two SMs shows in no run."""
+import re
+from pathlib import Path
+
+CSRC = Path(__file__).resolve().parent.parent / "beatsaberrl_b200" / "csrc"
+
+
+def _sources():
+    return {p.name: p.read_text() for p in sorted(CSRC.iterdir()) if p.suffix in (".cu", ".cuh")}
+
+
+def test_arrivals_at_the_other_cta_release_at_cluster_scope():
+    """An mbarrier arrival without a scope releases within its own CTA only.  One that hands rows to a thread of another CTA has
+    cluster scope, as a release or behind a release fence of that scope in the same statement."""
+    seen = 0
+    for name, text in _sources().items():
+        for stmt in re.findall(r"asm volatile\((.*?);\s*\n(?:\}|  asm|  return)", text, re.S):
+            for op in re.findall(r"mbarrier\.arrive[\w.:]*", stmt):
+                if "shared::cluster" not in op:
+                    continue
+                seen += 1
+                assert ".cluster.shared::cluster" in op, (name, op)
+                assert ".release." in op or re.search(r"fence\.(release|acq_rel)[\w.:]*\.cluster", stmt), (name, op)
+    assert seen >= 1
+
+
+def test_barriers_of_both_ctas_are_awaited_at_cluster_scope():
+    """Every barrier that mbar_arrive_cluster arrives at, or st.async counts on, is waited for with an acquire of cluster scope
+    by the thread that goes on from it."""
+    text = _sources()
+    waits = {"gemm_res_tc5.cu": ["tmem_empty[buf]"], "gemm_pair_tc5.cu": ["tmem_empty[buf]"], "attn_block_tc5.cu": ["acc_empty[buf]"],
+             "gemm_ln_tc5.cu": ["stats[buf]"], "block_tail_tc5.cu": ["x_ready", "h2_ready", "hid_ready["]}
+    for name, src in text.items():
+        if "mbar_arrive_cluster(map_to_cta" in src or "st_async_f2(map_to_cta" in src:
+            assert name in waits, name
+    for name, bars in waits.items():
+        for bar in bars:
+            calls = re.findall(r"(mbar_wait\w*|wait_epilogue|TAIL_WAIT\w*)(<[^>]*>)?\((?:smem_u32\()?&sh->" + re.escape(bar), text[name])
+            assert calls, (name, bar)
+            for fn, scope in calls:
+                assert fn == "wait_epilogue" or scope in ("<true>", "<PAIR>", "<CL == 2>"), (name, bar, fn, scope)
+    assert "return mbar_wait<PAIR>(bar, parity, abort);" in text["block_tail_tc5.cu"]
