@@ -394,11 +394,12 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 // rows x 256, K = 64: 827 -> 631 us, bound by the 2.1 GB it writes).
 // K <= 256 in whole k-blocks or row-contraction weights, N in the 32-column steps of a pair's MMAs, and at least three row
 // tiles per CTA for the resident weights: with one or two their load before the first MMA costs more than it saves.  fp16
-// masks are read by gemm_tc5.cu (here only as bits).
+// masks are read by gemm_tc5.cu (here only as bits).  A pair works on one column tile, so there are at most as many as pairs.
+static int res_cols(int n) { return n > BN && n % BN != 0 && n % 192 == 0 ? 192 : BN; }      // even column tiles where the width has them
 bool linear_res_ok(const LinearArgs& p) {
   const int64_t tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   return !p.a_mn && !p.mask && (!p.out_f32 || p.R || !dense_rows(p.cmap)) && !p.a_sums && p.k_splits <= 1 && p.K <= 4 * BK &&
-         p.N % 32 == 0 && p.M <= 0x7ffffe00 && tiles >= 3ll * sm_count() &&
+         p.N % 32 == 0 && p.M <= 0x7ffffe00 && tiles >= 3ll * sm_count() && (p.N + res_cols(p.N) - 1) / res_cols(p.N) <= sm_count() / 2 &&
          (!(p.bits_in || p.bits_out) || (!p.out_f32 && !p.R && p.N % 32 == 0)) && linear_tc5_ok(p);
 }
 
@@ -422,7 +423,7 @@ int linear_res(const LinearArgs& p, cudaStream_t stream) {
     return e != cudaSuccess ? e : cudaFuncSetAttribute(linear_res_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   });
   if (rc != BSRL_OK) return rc;
-  const int bn = p.N > BN && p.N % BN != 0 && p.N % 192 == 0 ? 192 : BN;       // even column tiles where the width has them
+  const int bn = res_cols(p.N);
   const int m_tiles = (int)((p.M + 2 * BM - 1) / (2 * BM)), n_tiles = (p.N + bn - 1) / bn;
   const int r32 = p.R && reinterpret_cast<uintptr_t>(p.R) % 32 == 0 && p.ldr % 8 == 0;        // 32-byte residual loads
   auto* kernel = p.R ? linear_res_kernel<true> : linear_res_kernel<false>;

@@ -559,3 +559,18 @@ def test_qkv_attention_split_groups(native, B, d, H, body):
 def test_linear_resident_weights_on_pairs(native, m, n, k, relu, res):
     """The resident-weight kernel's column halves and row remainders per CTA pair; bounds as in test_linear_resident_weights."""
     test_linear_resident_weights(native, m, n, k, relu, res)
+
+
+@pytest.mark.parametrize("n", [18944, 18976, 14400, 20480])
+def test_linear_many_column_tiles(native, n):
+    """K <= 256 and as many column tiles as the resident-weight kernel has CTA pairs (74 of 256 columns on 148 SMs), and more
+    than that (75 of 192; 256-column tiles past the last pair): every column is written."""
+    m, k = 2048, 128
+    g = torch.Generator(device="cuda").manual_seed(n)
+    a = torch.randn(m, k, generator=g, device="cuda").half()
+    w = (torch.randn(n, k, generator=g, device="cuda") * k ** -0.5).half()
+    b = torch.randn(n, generator=g, device="cuda")
+    out = torch.full((m, n), float("nan"), dtype=torch.float16, device="cuda")
+    native.check(native.lib.bsrl_linear(a.data_ptr(), w.data_ptr(), b.data_ptr(), None, out.data_ptr(), 0, 0, m, n, k, 1, _stream()))
+    ref = a.double() @ w.double().t() + b.double()
+    assert bool(((out.double() - ref).abs() <= 2 ** -11 * ref.abs() + 2e-5).all())
