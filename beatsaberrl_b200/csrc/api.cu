@@ -6,6 +6,7 @@
 // in a CUDA graph next to the simulator's step kernel (python/rollout_graph.py:45-74).
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <functional>
 #include <vector>
@@ -732,7 +733,12 @@ int64_t bsrl_workspace_bytes(const bsrl_config* cfg, int64_t n_envs) {
   if (validate_config(cfg) != BSRL_OK) return -1;
   if (n_envs < 0) return -1;
   Layout l = make_layout(*cfg);
-  return make_workspace(l, n_envs, plan_paths(l, g_engine.load(std::memory_order_relaxed), n_envs)).bytes;
+  const int engine = g_engine.load(std::memory_order_relaxed);
+  const int64_t bytes = make_workspace(l, n_envs, plan_paths(l, engine, n_envs)).bytes;
+  // a workspace serves every smaller batch too: the largest one on the few-environment path needs a buffer that the batches
+  // after it do not have
+  const int64_t few = small_envs(l);
+  return few < n_envs ? std::max(bytes, make_workspace(l, few, plan_paths(l, engine, few)).bytes) : bytes;
 }
 
 int bsrl_forward(const bsrl_config* cfg, const void* arena, const void* obs, int32_t obs_dtype,

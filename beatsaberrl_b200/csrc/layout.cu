@@ -321,6 +321,10 @@ const Plan& plan_of(const bsrl_config& c) {
 }
 
 // ------------------------------------------------------------------ workspace
+int64_t small_envs(const Layout& l) {
+  const int64_t by_width = (1 << 20) / ((int64_t)l.d * l.d);
+  return by_width < 64 ? by_width : 64;
+}
 Paths plan_paths(const Layout& l, int engine, int64_t n_envs) {
   Paths p;
   const bool widths = engine == 0 && l.d % 64 == 0 && l.d >= 64 && l.d <= 256;
@@ -331,7 +335,7 @@ Paths plan_paths(const Layout& l, int engine, int64_t n_envs) {
   // fused kernels, which take the same time up to one tile per SM.  Forward behind a graph, small / fused us: d 64 at 64
   // envs 68 / 70, at 128 74 / 70; d 128 at 64 84 / 90, at 96 98 / 90; d 192 at 1 151 / 230, at 24 223 / 239, at 48 284 /
   // 240; d 256 at 1 124 / 204, at 16 168 / 206, at 32 229 / 209.
-  p.small = l.L >= 2 && p.attn_fused && p.tail_fused && p.enc_fused && !l.final_ln.width && n_envs <= 64 && n_envs * l.d * l.d <= 1 << 20;
+  p.small = l.L >= 2 && p.attn_fused && p.tail_fused && p.enc_fused && !l.final_ln.width && n_envs <= small_envs(l);
   return p;
 }
 

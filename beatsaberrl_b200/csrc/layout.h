@@ -96,6 +96,7 @@ struct Paths {
   bool enc_fused;    // both encoder layers + block 0's LayerNorm in one kernel
   bool small;        // few environments: every block as four launches of many small CTAs
 };
+int64_t small_envs(const Layout& l);      // the largest batch that may take Paths::small
 Paths plan_paths(const Layout& l, int engine, int64_t n_envs);
 
 // Workspace carve-up for a batch of n_envs (offsets of buffers the path does not use are -1).

@@ -59,6 +59,17 @@ def test_sizes_grow_with_batch(native):
     assert native.lib.bsrl_weights_bytes(C.byref(c)) > 2 * 5_000_000  # > fp16 copy of 5.7 M params
 
 
+@pytest.mark.parametrize("name,geo,opts", [("tiny", False, None), ("cfg1", False, None), ("cfg2", False, dict(value_residual=True)),
+                                           ("recipe", True, None), ("cfg4", False, None), ("cfg2", False, dict(final_ln=True))])
+def test_a_workspace_serves_every_smaller_batch(native, name, geo, opts):
+    """Callers allocate once for their largest batch: the size never falls from one batch to the next larger one, in particular
+    not where the few-environment path and its hidden buffer end."""
+    from beatsaberrl_b200.policy import NotePolicy
+    c = NotePolicy(**make_cfg(name, geo, opts=opts).ref_kwargs())._cfg
+    sizes = [native.lib.bsrl_workspace_bytes(C.byref(c), n) for n in range(200)]
+    assert sizes[0] >= 0 and all(a <= b for a, b in zip(sizes, sizes[1:]))
+
+
 def test_config_errors_are_reported(native):
     good = make_cfg("cfg1")
     c = _cfg(native, good)
