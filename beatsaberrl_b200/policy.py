@@ -373,15 +373,22 @@ class NotePolicy(nn.Module):
 
     def _table_params(self) -> list:
         """The live parameters in the library's order.  Walking the module tree for their names takes longer than a
-        small update's kernels, so the (module, attribute) places are looked up once; the parameters are read from
-        them on every call."""
-        if self._param_places is None:
-            places = {}
-            for prefix, mod in self.named_modules():
-                for name in mod._parameters:
-                    places[f"{prefix}.{name}" if prefix else name] = (mod._parameters, name)
-            self._param_places = [places[n] for n, _, _ in self._param_table]
-        return [d[k] for d, k in self._param_places]
+        small update's kernels, so their modules are looked up once and again when one on the way to them was replaced;
+        the parameters are read from the modules on every call."""
+        root = self._modules        # the lists below name the policy itself None: it must not hold itself alive
+        if self._param_places is None or any(
+                (root if parent is None else parent._modules).get(key) is not mod for parent, key, mod in self._param_places[0]):
+            edges, owners = {}, []
+            for name, _, _ in self._param_table:
+                *path, leaf = name.split(".")
+                mod = None
+                for i, key in enumerate(path):
+                    parent, mod = mod, (root if mod is None else mod._modules)[key]
+                    edges[tuple(path[:i + 1])] = (parent, key, mod)
+                owners.append((mod, leaf))
+            self._param_places = list(edges.values()), owners
+        own = self._parameters
+        return [(own if mod is None else mod._parameters)[leaf] for mod, leaf in self._param_places[1]]
 
     def _grad_pieces(self):
         """The flat gradient buffer's length, empty stand-ins whose shapes cut it into the parameters' gradients and the

@@ -132,3 +132,24 @@ def test_policy_facade_host_side(native):
     with pytest.raises(ValueError):
         NotePolicy(z_asinh=0.0)
     bump_weights_version()
+
+
+def test_a_replaced_module_is_the_one_that_gets_gradients(native):
+    """The grad-mode forward hands the live parameters to autograd: after a module was replaced (at any depth) or a
+    parameter exchanged, the new ones."""
+    from beatsaberrl_b200.policy import NotePolicy
+    kw = dict(embed=64, trunk_dim=128, n_blocks=2, n_heads=2, n_gears=5, trunk_arch="simbav2")
+    m, other = NotePolicy(**kw), NotePolicy(**kw)
+
+    def check():
+        named = dict(m.named_parameters())
+        got = m._table_params()
+        assert len(got) == len(m._param_table) and all(p is named[n] for p, (n, _, _) in zip(got, m._param_table))
+
+    check()
+    for change in (lambda: setattr(m, "critic_q", other.critic_q), lambda: m.blocks.__setitem__(0, other.blocks[0]),
+                   lambda: setattr(m, "blocks", other.blocks), lambda: m.blocks[1].ffn.__setitem__(2, torch.nn.Linear(256, 64)),
+                   lambda: setattr(m.heads[3], "weight", torch.nn.Parameter(torch.zeros(5, 128))),
+                   lambda: setattr(m, "trunk_alpha", other.trunk_alpha)):
+        change()
+        check()
