@@ -66,7 +66,6 @@ class PackedAdamW:
         self.exp_avg = [torch.zeros_like(p, memory_format=torch.preserve_format) for p in self.params]
         self.exp_avg_sq = [torch.zeros_like(p, memory_format=torch.preserve_format) for p in self.params]
         self._lr_key = self._lr_arrays = None
-        self._moments = _pointers(self.exp_avg), _pointers(self.exp_avg_sq)     # private tensors, only written in place
         self._owned = [(i, p) for i, (nm, p) in enumerate(zip(self.names, self.params)) if nm not in self.exclude]
 
     def zero_grad(self, set_to_none: bool = True) -> None:
@@ -102,8 +101,8 @@ class PackedAdamW:
                 raise ValueError(f"{name} must be a one-element float32 tensor on {dev}")
         with torch.cuda.device(dev):
             nat.check(nat.lib.bsrl_adam_step_pack(
-                C.byref(pol._cfg), _pointers(self.params), grads, *self._moments, n, lr, wd, self.betas[0],
-                self.betas[1], self.eps, self.step_count,
+                C.byref(pol._cfg), _pointers(self.params), grads, _pointers(self.exp_avg), _pointers(self.exp_avg_sq), n,
+                lr, wd, self.betas[0], self.betas[1], self.eps, self.step_count,
                 inv_scale.data_ptr() if inv_scale is not None else None,
                 found_inf.data_ptr() if found_inf is not None else None,
                 pol._arena.data_ptr(), pol._arena.numel(), torch.cuda.current_stream().cuda_stream))

@@ -153,3 +153,17 @@ def test_a_replaced_module_is_the_one_that_gets_gradients(native):
                    lambda: setattr(m, "trunk_alpha", other.trunk_alpha)):
         change()
         check()
+
+
+def test_optimizers_can_be_copied(native):
+    """copy.deepcopy of an optimizer (with its policy) is an optimizer of the copy: its own moments, no addresses of the original."""
+    import copy
+    from beatsaberrl_b200.optim import PackedAdamW, PackedMuon
+    from beatsaberrl_b200.policy import NotePolicy
+    m = NotePolicy(embed=64, trunk_dim=128, n_blocks=2, n_heads=2, n_gears=5)
+    for opt, state in ((PackedAdamW(m), "exp_avg"), (PackedMuon(m), "bufs")):
+        twin = copy.deepcopy(opt)
+        live = dict(twin.policy.named_parameters())
+        assert twin.policy is not m and all(p is live[n] for n, p in zip(twin.names, twin.params))
+        getattr(twin, state)[0].fill_(1.0)
+        assert float(getattr(opt, state)[0].abs().max()) == 0.0

@@ -201,3 +201,26 @@ def test_muon_products_are_fp32_accurate(embed, heads, trunk, hidden):
         o = o.t() if o.shape[0] > o.shape[1] else o
         err, own = float((o - exact).norm()), float((fp32 - exact).norm())
         assert err <= 1.5 * own + 1e-7 * float(exact.norm()), (n, err, own)
+
+
+def test_adam_moments_may_be_exchanged_between_steps():
+    """The moments a step reads and writes are the lists' tensors at that time (a caller may assign loaded or moved ones)."""
+    from beatsaberrl_b200.optim import PackedAdamW
+    cfg, sd = golden_case("tiny_plain")
+    results = []
+    for exchange in (False, True):
+        m = cuda_policy(cfg, sd)
+        opt = PackedAdamW(m, lr=1e-2)
+        g = torch.Generator(device="cuda").manual_seed(2)
+        kept = []
+        for step in range(2):
+            for p in m.parameters():
+                p.grad = torch.randn(p.shape, generator=g, device="cuda")
+            opt.step()
+            if exchange and step == 0:
+                kept = opt.exp_avg + opt.exp_avg_sq          # stay allocated
+                opt.exp_avg, opt.exp_avg_sq = [t.clone() for t in opt.exp_avg], [t.clone() for t in opt.exp_avg_sq]
+                for t in kept:
+                    t.fill_(1e3)
+        results.append([p.detach().clone() for p in m.parameters()] + opt.exp_avg + opt.exp_avg_sq)
+    assert all(torch.equal(a, b) for a, b in zip(*results))
