@@ -66,7 +66,6 @@ class PackedAdamW:
         self.exp_avg = [torch.zeros_like(p, memory_format=torch.preserve_format) for p in self.params]
         self.exp_avg_sq = [torch.zeros_like(p, memory_format=torch.preserve_format) for p in self.params]
         self._lr_key = self._lr_arrays = None
-        self._owned = [(i, p) for i, (nm, p) in enumerate(zip(self.names, self.params)) if nm not in self.exclude]
 
     def zero_grad(self, set_to_none: bool = True) -> None:
         for p in self.params:
@@ -86,9 +85,9 @@ class PackedAdamW:
         self.step_count += 1
         n = len(self.params)
         grads, keep = (C.c_void_p * n)(), []
-        for i, p in self._owned:
+        for i, (name, p) in enumerate(zip(self.names, self.params)):
             g = p.grad
-            if g is None or not p.requires_grad:
+            if g is None or not p.requires_grad or name in self.exclude:
                 continue
             if not g.is_contiguous():
                 g = g.contiguous()
@@ -175,11 +174,10 @@ class PackedMuon:
                 raise ValueError(f"PackedMuon owns 2-D parameters only: {n}")
         self.params = [named[n] for n in self.names]
         self.bufs = [torch.zeros_like(p) for p in self.params]
-        slot = {n: i for i, n in enumerate(self.table)}
+        self._slot = {n: i for i, n in enumerate(self.table)}
         for p in self.params:
             if p.dtype is not torch.float32 or not p.is_contiguous():
                 raise ValueError("PackedMuon needs contiguous float32 parameters")
-        self._rows = [(slot[n], p, b) for n, p, b in zip(self.names, self.params, self.bufs)]
         self._ws_key, self._ws_bytes = None, 0
         self._lr_key = self._lr_arrays = None
 
@@ -200,10 +198,11 @@ class PackedMuon:
         n = len(self.table)
         grads, bufs, owned = (C.c_void_p * n)(), (C.c_void_p * n)(), (C.c_int32 * n)()
         keep = []
-        for slot, p, b in self._rows:
+        for name, p, b in zip(self.names, self.params, self.bufs):
             g = p.grad
             if g is None or not p.requires_grad:
                 continue
+            slot = self._slot[name]
             if not g.is_contiguous():
                 g = g.contiguous()
                 keep.append(g)

@@ -224,3 +224,29 @@ def test_adam_moments_may_be_exchanged_between_steps():
                     t.fill_(1e3)
         results.append([p.detach().clone() for p in m.parameters()] + opt.exp_avg + opt.exp_avg_sq)
     assert all(torch.equal(a, b) for a, b in zip(*results))
+
+
+def test_optimizers_read_their_lists_on_every_step():
+    """``exclude`` may change between steps (a run that hands matrices over to Muon), and so may Muon's momentum buffers."""
+    from beatsaberrl_b200.optim import PackedAdamW, PackedMuon, muon_param_names
+    cfg, sd = golden_case("tiny_plain")
+    m = cuda_policy(cfg, sd)
+    names = muon_param_names(m)
+    named = dict(m.named_parameters())
+    adam, muon = PackedAdamW(m, lr=1e-2), PackedMuon(m, names, momentum=0.5)
+
+    def grads():
+        for p in m.parameters():
+            p.grad = torch.ones_like(p)
+
+    grads()
+    adam.step()
+    adam.exclude = frozenset(names)
+    before = {n: p.detach().clone() for n, p in named.items()}
+    adam.step()
+    assert all(torch.equal(p, before[n]) == (n in adam.exclude) for n, p in named.items())
+    kept = muon.bufs
+    muon.bufs = [torch.full_like(b, 2.0) for b in muon.bufs]
+    muon.step()
+    for old, new in zip(kept, muon.bufs):
+        assert float(old.abs().max()) == 0.0 and float((new - 2.0).abs().max()) == 0.0       # 0.5 * 2 + 1
