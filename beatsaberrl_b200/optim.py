@@ -34,7 +34,7 @@ def _lr_of(opt, name: str) -> float:
 
 def _lr_table(opt, names, wd=None):
     """Per-parameter learning rates (and weight decays) as C arrays, rebuilt only when a setting they come from changed."""
-    key = (opt.lr, opt.weight_decay, tuple(opt.lr_scale.items()))
+    key = (float(opt.lr), float(opt.weight_decay), tuple((k, float(v)) for k, v in opt.lr_scale.items()))
     if opt._lr_key != key:
         n = len(names)
         opt._lr_arrays = ((C.c_float * n)(*[_lr_of(opt, nm) for nm in names]), (C.c_float * n)(*(wd or [0.0] * n)))

@@ -167,3 +167,18 @@ def test_optimizers_can_be_copied(native):
         assert twin.policy is not m and all(p is live[n] for n, p in zip(twin.names, twin.params))
         getattr(twin, state)[0].fill_(1.0)
         assert float(getattr(opt, state)[0].abs().max()) == 0.0
+
+
+def test_a_learning_rate_changed_in_place_is_seen(native):
+    """Schedules may hold the rate in a tensor or an array and change that: the per-parameter rates follow its value."""
+    import numpy as np
+    from beatsaberrl_b200.optim import PackedAdamW, _lr_table
+    from beatsaberrl_b200.policy import NotePolicy
+    opt = PackedAdamW(NotePolicy(embed=64, trunk_dim=128, n_blocks=2, n_heads=2, n_gears=5))
+    for rate, mult in ((torch.tensor(0.5), 2.0), (np.array(0.5), 2.0), (0.5, torch.tensor(2.0))):
+        opt.lr, opt.lr_scale = rate, {"critic_": mult}
+        assert set(_lr_table(opt, opt.names)[0]) == {0.5, 1.0}
+        for value in (rate, mult):
+            if not isinstance(value, float):
+                value *= 0.25
+        assert set(_lr_table(opt, opt.names)[0]) == ({0.5, 0.25} if isinstance(rate, float) else {0.125, 0.25})
