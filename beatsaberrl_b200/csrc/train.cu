@@ -277,7 +277,7 @@ struct Bwd {
     BSRL_TRY(transpose16(W, ldw, identity_map(), N, K, wT, Np, Np, st));
     LinearArgs a = linear_args(g, (int)ldg, wT, Np, nullptr, out, (int)ldo, out_f32 ? 1 : 0, 0, M, K, Np);
     a.R = r.R; a.ldr = r.ldr; a.rmap = r.rmap; a.cmap = r.cmap;
-    BSRL_TRY(linear(a, st));
+    BSRL_TRY(linear_mma(a, st));       // wT is this sequence's own: not a kernel that fetches weights ahead of its predecessor
     if (relu_of) {
       if (out_f32) {
         set_error("backward: the ReLU mask applies to fp16 gradients");
@@ -326,7 +326,7 @@ struct Bwd {
     BSRL_TRY(transpose16(x, ldx, identity_map(), M, K, tX, Mp, Mp, st));
     LinearArgs a = linear_args(tA, (int)Mp, tX, (int)Mp, nullptr, gW, ldgw, 1, 0, N, K, (int)Mp);
     a.k_splits = splits;
-    return linear(a, st);
+    return linear_mma(a, st);          // as in dgrad
   }
   int wgrad(const __half* g, int64_t ldg, int64_t M, int N, const __half* x, int64_t ldx, int K, const std::string& name) {
     return wgrad(g, ldg, M, N, x, ldx, K, G(name + ".weight"), K, G(name + ".bias"));

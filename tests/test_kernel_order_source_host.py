@@ -1,4 +1,4 @@
-"""What the kernels on CTA pairs promise each other, read from their source: a race between two SMs shows in no run."""
+"""What kernels that run at the same time promise each other, read from their source: a race between them shows in no run."""
 import re
 from pathlib import Path
 
@@ -40,3 +40,14 @@ def test_barriers_of_both_ctas_are_awaited_at_cluster_scope():
             for fn, scope in calls:
                 assert fn == "wait_epilogue" or scope in ("<true>", "<PAIR>", "<CL == 2>"), (name, bar, fn, scope)
     assert "return mbar_wait<PAIR>(bar, parity, abort);" in text["block_tail_tc5.cu"]
+
+
+def test_copied_operands_go_to_a_kernel_that_waits_for_them():
+    """Inside an overlapping sequence some kernels fetch their weight operand before their predecessor has ended, since weights
+    are nobody's output.  The backward's transposed copies are: their products run on the warp-MMA kernel, which waits first."""
+    struct = _sources()["train.cu"].split("struct Bwd {")[1].split("\n};")[0]
+    for part in struct.split("transpose16(")[1:]:
+        call = re.search(r"\b(linear\w*)\((?:a|r|f), st\)|transpose16\(", part)
+        assert call is None or call.group(1) in (None, "linear_mma"), part[:200]
+    body = _sources()["gemm_mma.cu"].split("linear_mma_kernel(LinearArgs p) {")[1]
+    assert body.lstrip().startswith("pdl_begin();")
