@@ -59,3 +59,13 @@ def assert_parity(logits, value, ref_logits, ref_value, argmax_min=ARGMAX_MIN):
     assert rep["value_within"] == 1.0, rep
     assert rep["argmax_agree"] >= argmax_min, rep
     return rep
+
+
+def kernels_of(fn):
+    """Names of the CUDA kernels that fn() launches."""
+    import torch.profiler as tp
+    torch.cuda.synchronize()
+    with tp.profile(activities=[tp.ProfilerActivity.CUDA], acc_events=True) as prof:
+        fn()
+        torch.cuda.synchronize()
+    return [e.name for e in prof.events() if e.name.endswith(")") or "kernel" in e.name]

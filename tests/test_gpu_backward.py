@@ -264,10 +264,11 @@ def test_linear_bwd_stage(native, m, n, k, engine):
     torch.testing.assert_close(gx.cpu(), gy.float() @ w.float(), atol=2e-3, rtol=2e-3)
 
 
-@pytest.mark.parametrize("name,blocks,envs", [("cfg2", 2, 516), ("recipe", 2, 683), ("cfg1", 2, 1031)])
+@pytest.mark.parametrize("name,blocks,envs", [("cfg2", 2, 516), ("recipe", 2, 683), ("cfg1", 2, 1031), ("cfg4", 2, 331)])
 def test_large_batch_gradients_equal_the_sum_of_small_batches(name, blocks, envs):
-    """Batches large enough for the resident-weight products (three 128 x 256 tiles per SM; ReLU masks as bits) and odd in
-    rows, against the same environments in small batches, which take the streaming kernel and fp16 masks: every row's
+    """Batches large enough for the resident-weight products (three 128 x 256 tiles per SM; ReLU masks as bits; at 512 columns
+    the CTA-pair products, with fp16 masks) and odd in rows, against the same environments in small batches, which take the
+    streaming kernel and fp16 masks: every row's
     arithmetic is the same, so the gradients differ by the order of fp32 sums over some 15-30 thousand rows only
     (about 2^-24 sqrt(rows) = 1e-5 of the terms' root sum of squares; the bound allows the atomics' order on top)."""
     cfg = make_cfg(name, name == "recipe")

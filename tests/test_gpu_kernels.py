@@ -5,7 +5,7 @@ import pytest
 import torch
 import torch.nn.functional as F
 
-from helpers import golden_case, make_cfg, po
+from helpers import golden_case, kernels_of, make_cfg, po
 
 pytestmark = pytest.mark.gpu
 
@@ -383,9 +383,9 @@ def test_head_tail_stage(native, case, B):
 
 @pytest.mark.parametrize("m,n,k,relu,res", [
     (57001, 256, 256, 1, False),        # one column tile, a ragged last row tile, two A stages per ring turn
-    (19200, 784, 192, 0, False),        # four column tiles, the last 16 wide; two staging buffers
+    (19200, 800, 192, 0, False),        # four column tiles, the last 32 wide
     (28577, 512, 64, 2, False),         # one k-block, GELU
-    (57001, 208, 192, 0, True),         # fp32 rows with a residual, columns past the tile
+    (57001, 224, 192, 0, True),         # fp32 rows with a residual, fewer columns than the tile
     (28416, 320, 128, 0, True),
 ])
 def test_linear_resident_weights(native, m, n, k, relu, res):
@@ -397,8 +397,9 @@ def test_linear_resident_weights(native, m, n, k, relu, res):
     b = torch.randn(n, generator=g, device="cuda")
     r = torch.randn(m, n, generator=g, device="cuda") if res else None
     out = torch.full((m, n), float("nan"), dtype=torch.float32 if res else torch.float16, device="cuda")
-    native.check(native.lib.bsrl_linear(a.data_ptr(), w.data_ptr(), b.data_ptr(), r.data_ptr() if res else None, out.data_ptr(),
-                                        int(res), relu, m, n, k, 1, torch.cuda.current_stream().cuda_stream))
+    ran = kernels_of(lambda: native.check(native.lib.bsrl_linear(
+        a.data_ptr(), w.data_ptr(), b.data_ptr(), r.data_ptr() if res else None, out.data_ptr(), int(res), relu, m, n, k, 1, _stream())))
+    assert len(ran) == 1 and "linear_res_kernel" in ran[0], ran
     ref = a.double() @ w.double().t() + b.double()
     if relu == 1:
         ref = ref.clamp_min(0)
@@ -437,10 +438,10 @@ def test_linear_small_tiles(native, m, n, k, relu, resid, f32):
 
 @pytest.mark.parametrize("m,n,k,relu,resid,f32", [
     (18945, 512, 320, 1, 0, 0),         # the first size that takes CTA pairs; half a pair and one row in the last tile
-    (19021, 512, 576, 0, 1, 1), (37889, 256, 1024, 2, 0, 0), (12801, 768, 520, 0, 0, 1), (18999, 512, 512, 0, 1, 0),
+    (19021, 512, 576, 0, 1, 1), (37889, 256, 1024, 2, 0, 0), (12801, 768, 512, 0, 0, 1), (18999, 512, 512, 0, 1, 0),
 ])
 def test_linear_cta_pairs(native, m, n, k, relu, resid, f32):
-    """Large products with K > 256 on CTA pairs, K and rows with remainders, against float64 products of the same fp16
+    """Large products with K > 256 on CTA pairs, rows with remainders, against float64 products of the same fp16
     operands: fp32 sums of k products of size ~1 / sqrt(k) (k 2^-24 at worst) and one fp16 rounding."""
     g = torch.Generator(device="cuda").manual_seed(m + n)
     a = torch.randn(m, k, generator=g, device="cuda").half()
@@ -448,16 +449,31 @@ def test_linear_cta_pairs(native, m, n, k, relu, resid, f32):
     b = torch.randn(n, generator=g, device="cuda")
     r = torch.randn(m, n, generator=g, device="cuda") if resid else None
     out = torch.full((m, n), float("nan"), dtype=torch.float32 if f32 else torch.float16, device="cuda")
-    rc = native.lib.bsrl_linear(a.data_ptr(), w.data_ptr(), b.data_ptr(), r.data_ptr() if resid else None, out.data_ptr(),
-                                f32, relu, m, n, k, 1, _stream())
-    if k % 64:
-        assert rc != 0                  # K in whole k-blocks where the rows of both operands are contiguous
-        return
-    native.check(rc)
+    ran = kernels_of(lambda: native.check(native.lib.bsrl_linear(
+        a.data_ptr(), w.data_ptr(), b.data_ptr(), r.data_ptr() if resid else None, out.data_ptr(), f32, relu, m, n, k, 1, _stream())))
+    assert len(ran) == 1 and "linear_pair_kernel" in ran[0], ran
     native.check(native.lib.bsrl_device_status())
     ref = a.double() @ w.double().t() + b.double()
     ref = ref.clamp_min(0) if relu == 1 else F.gelu(ref) if relu == 2 else ref
     ref = ref + r.double() if resid else ref
+    tol = 4e-5 if f32 else 2 ** -11
+    assert bool(((out.double() - ref).abs() <= tol * ref.abs() + 4e-5).all())
+
+
+@pytest.mark.parametrize("m,n,k,f32", [(18945, 512, 512, 0), (19021, 320, 512, 1), (12801, 2048, 768, 0)])
+def test_linear_cta_pairs_read_weights_by_rows(native, m, n, k, f32):
+    """Input gradients g W on CTA pairs: the weight's rows are the contraction index.  Bounds as in test_linear_cta_pairs."""
+    g = torch.Generator(device="cuda").manual_seed(m + n)
+    gy = torch.randn(m, n, generator=g, device="cuda").half()
+    w = (torch.randn(n, k, generator=g, device="cuda") * n ** -0.5).half()
+    out = torch.full((m, k), float("nan"), dtype=torch.float32 if f32 else torch.float16, device="cuda")
+    n_s = native.lib.bsrl_linear_bwd_scratch_bytes(m, n, k)
+    scratch = torch.empty(n_s, dtype=torch.uint8, device="cuda")
+    ran = kernels_of(lambda: native.check(native.lib.bsrl_linear_bwd(
+        gy.data_ptr(), gy.data_ptr(), w.data_ptr(), m, n, k, None, None, out.data_ptr(), f32, scratch.data_ptr(), n_s, _stream())))
+    assert len(ran) == 1 and "linear_pair_kernel" in ran[0], ran
+    native.check(native.lib.bsrl_device_status())
+    ref = gy.double() @ w.double()
     tol = 4e-5 if f32 else 2 ** -11
     assert bool(((out.double() - ref).abs() <= tol * ref.abs() + 4e-5).all())
 

@@ -250,3 +250,26 @@ def test_optimizers_read_their_lists_on_every_step():
     muon.step()
     for old, new in zip(kept, muon.bufs):
         assert float(old.abs().max()) == 0.0 and float((new - 2.0).abs().max()) == 0.0       # 0.5 * 2 + 1
+
+
+def test_apply_updates_pack_adds_and_repacks(native):
+    """The ABI's additive step: masters with an update become p + u (one fp32 addition), the others stay, the arena equals a full
+    repack, and found_inf leaves the masters alone."""
+    import ctypes as C
+    cfg, sd = golden_case("tiny_geo_mixed")
+    m = cuda_policy(cfg, sd)
+    m.flatten_fp16()
+    named = dict(m.named_parameters())
+    params = [named[n] for n, _, _ in m._param_table]
+    g = torch.Generator(device="cuda").manual_seed(4)
+    ups = [torch.randn(p.shape, generator=g, device="cuda") if i % 3 else None for i, p in enumerate(params)]
+    array = lambda ts: (C.c_void_p * len(ts))(*[None if t is None else t.data_ptr() for t in ts])  # noqa: E731
+    for skip in (1.0, 0.0):
+        want = [p.detach().clone() if u is None or skip else p.detach() + u for p, u in zip(params, ups)]
+        inf = torch.tensor(skip, device="cuda")
+        native.check(native.lib.bsrl_apply_updates_pack(C.byref(m._cfg), array(params), array(ups), len(params), inf.data_ptr(),
+                                                        m._arena.data_ptr(), m._arena.numel(), torch.cuda.current_stream().cuda_stream))
+        assert all(torch.equal(p, w) for p, w in zip(params, want))
+        arena = m._arena.clone()
+        m.refresh_fp16_caches()
+        assert torch.equal(arena, m._arena)
