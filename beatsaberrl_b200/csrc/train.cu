@@ -405,12 +405,11 @@ struct Bwd {
     PdlScope pdl;
     begin_overlap(R);
 
-    // ---- recompute the critic's activations (its pool lands in z beside the trunk's output)
+    // ---- recompute the critic's activations; its pool is in the saved z, beside the trunk's output
     BSRL_TRY(layernorm(x_last, d, ident, c.G(l.critic_ln), c.Be(l.critic_ln), eps, R, d, h16, d, st));
     BSRL_TRY(linear(linear_args(hv, d, c.W(l.critic_kv), d, c.Bv(l.critic_kv), qkv + d, 3 * d, 0, 0, R, 2 * d, d), st));
     BSRL_TRY(linear(linear_args(hv_torso, kT * d, c.W(l.critic_q), d, c.Bv(l.critic_q), qkv + 2 * 3 * d, kT * 3 * d, 0, 0, B, d, d), st));
     BSRL_TRY(attention(qkv, 3 * d, sv.key_bias, B, d, l.H, 2, 1, attc, d, st));
-    BSRL_TRY(linear(linear_args(attc, d, c.W(l.critic_out), d, c.Bv(l.critic_out), sv.z, ldz, 0, 0, B, d, d), st));
     BSRL_TRY(linear(linear_args(sv.z, ldz, c.W(l.critic_m0), ldz, c.Bv(l.critic_m0), m1, D, 0, 1, B, D, ldz), st));
     BSRL_TRY(linear(linear_args(m1, D, c.W(l.critic_m1), D, c.Bv(l.critic_m1), m2, D, 0, 1, B, D, D), st));
 

@@ -288,3 +288,19 @@ def test_large_batch_gradients_equal_the_sum_of_small_batches(name, blocks, envs
     top = max(float(g.norm()) for g in whole.values())
     for k, p in m.named_parameters():
         assert float((p.grad - whole[k]).norm()) <= 1e-4 * float(whole[k].norm()) + 1e-6 * top, k
+
+
+@pytest.mark.parametrize("name,opts,envs", [("cfg1", None, 70), ("recipe", dict(value_residual=True), 45),
+                                            ("tiny", dict(trunk_arch="simbav2", emb_ln=True, final_ln=True), 33)])
+def test_backward_only_reads_the_save_buffer(name, opts, envs):
+    """``save`` is an input of bsrl_backward: two backward calls may share one, on two streams as well."""
+    cfg = make_cfg(name, name == "recipe", opts=opts)
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 5))
+    obs, act, up = po.make_obs(envs, 21, padded=True), po.make_actions(envs, cfg, 22), po.make_upstream(envs, cfg, 23)
+    with torch.enable_grad():
+        _, lp, ent, val = m.get_action_and_value(obs.cuda(), act.cuda())
+        save = lp.grad_fn.save
+        before = save.clone()
+        ((up["logprob"].cuda() * lp).sum() + (up["entropy"].cuda() * ent).sum() + (up["value"].cuda() * val).sum()
+         + (up["value_logits"].cuda() * m._value_logits).sum()).backward()
+    assert torch.equal(save, before)
