@@ -139,19 +139,15 @@ def test_full_size_properties():
     assert_parity(logits[idx], value[idx], ref_l, ref_v, argmax_min=0.998)
 
 
-@pytest.mark.parametrize("name,B,part,exact", [("cfg2", 2375, 400, True), ("cfg1", 3601, 500, True), ("cfg4", 601, 67, False)])
-def test_many_envs_match_slices(name, B, part, exact):
+@pytest.mark.parametrize("name,B,part", [("cfg2", 2375, 400), ("cfg1", 3601, 500), ("cfg4", 601, 67)])
+def test_many_envs_match_slices(name, B, part):
     """Batches past the sizes at which the encoder's rows leave by mapped TMA boxes, the GEMMs take resident weights or CTA pairs,
-    and the block kernels take CTA pairs, against slices that take none of these: bit for bit up to 256 columns (the same order
-    of every sum), within fp16 rounding of the LayerNorm rows above."""
+    and the block kernels take CTA pairs, against slices that take none of these: bit for bit (the same order of
+    every sum)."""
     cfg = bo.named_config(name)
     m = cuda_body_policy(cfg, bo.build_state_dict(cfg, 7, xavier=True))
     obs = bo.make_obs(B, cfg, 11, padded=True).cuda()
     logits, value = m.forward_stacked(obs)
     for lo in range(0, B, part):
         l, v = m.forward_stacked(obs[lo:lo + part])
-        if exact:
-            assert torch.equal(l, logits[lo:lo + part]) and torch.equal(v, value[lo:lo + part])
-        else:
-            torch.testing.assert_close(l, logits[lo:lo + part], atol=1e-2, rtol=1e-2)
-            torch.testing.assert_close(v, value[lo:lo + part], atol=1e-2, rtol=1e-2)
+        assert torch.equal(l, logits[lo:lo + part]) and torch.equal(v, value[lo:lo + part])

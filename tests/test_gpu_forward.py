@@ -273,10 +273,10 @@ def test_few_envs_take_other_kernels_and_give_the_same_bits(name, geo, opts):
     m.check_device()
 
 
-@pytest.mark.parametrize("name,B,part,exact", [("cfg2", 2601, 300, True), ("cfg4", 1001, 90, False)])
-def test_many_envs_match_slices(name, B, part, exact):
+@pytest.mark.parametrize("name,B,part", [("cfg2", 2601, 300), ("cfg4", 1001, 90)])
+def test_many_envs_match_slices(name, B, part):
     """Batches past the sizes at which kernels take CTA pairs, resident weights or mapped TMA boxes against slices that take none
-    of these: bit for bit at 256 columns (the same order of every sum), within fp16 rounding of the LayerNorm rows at 512."""
+    of these: bit for bit (the same order of every sum)."""
     cfg = po.named_config(name)
     sd = po.build_state_dict(cfg, 5, xavier=True)
     m = cuda_policy(cfg, sd)
@@ -284,8 +284,4 @@ def test_many_envs_match_slices(name, B, part, exact):
     logits, value = m.forward_stacked(obs)
     for lo in range(0, B, part):
         l, v = m.forward_stacked(obs[lo:lo + part])
-        if exact:
-            assert torch.equal(l, logits[lo:lo + part]) and torch.equal(v, value[lo:lo + part])
-        else:
-            torch.testing.assert_close(l, logits[lo:lo + part], atol=1e-2, rtol=1e-2)
-            torch.testing.assert_close(v, value[lo:lo + part], atol=1e-2, rtol=1e-2)
+        assert torch.equal(l, logits[lo:lo + part]) and torch.equal(v, value[lo:lo + part])
