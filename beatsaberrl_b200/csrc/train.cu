@@ -171,7 +171,7 @@ const GradLayout& grad_layout(const bsrl_config& cfg) {
 struct BwdLayout {
   int64_t h16, qkv16, att16, x1, h2, hid, bits, gx, gx16, g32, gA, gB, tA, tX, wT, hl16;
   // readout-side rows (B of them)
-  int64_t attc16, m1, m2, gz32, graw16, gvraw16, gsmall32, gsmall16;
+  int64_t attc16, z16, m1, m2, gz32, graw16, gvraw16, gsmall32, gsmall16;
   int64_t v0, vown, gv0;        // value residual: block 0's values, a block's own values, fp32 gradient of block 0's values
   int64_t bytes;
   int64_t Rpad;
@@ -212,6 +212,7 @@ BwdLayout make_bwd(const Layout& l, int64_t B) {
   w.wT = cv.take(wmax * 2);
   w.hl16 = cv.take(B * kLead * (int64_t)d * 2);
   w.attc16 = cv.take(B * d * 2);
+  w.z16 = cv.take(B * (int64_t)(d + D) * 2);
   w.m1 = cv.take(B * D * 2);
   w.m2 = cv.take(B * D * 2);
   w.gz32 = cv.take(B * (int64_t)(d + D) * 4);
@@ -397,20 +398,25 @@ struct Bwd {
     // the torso rows (token 2 of every env) of a token-row matrix are a matrix of pitch 29 times its own
     const __half *hv = h16, *hv_torso = h16 + 2 * d;
     __half* attc = S<__half>(w.attc16);
+    __half* z = S<__half>(w.z16);
     __half* m1 = S<__half>(w.m1);
     __half* m2 = S<__half>(w.m2);
+
+    // ---- [critic pool | trunk h] of the recomputation: h is the saved one (the caller's buffer is only read), the pool follows
+    BSRL_CUDA_OK(cudaMemcpy2DAsync(z + d, (size_t)ldz * 2, sv.z + d, (size_t)ldz * 2, (size_t)D * 2, B, cudaMemcpyDeviceToDevice, st));
 
     // ---- head tail
     BSRL_TRY(head_tail_bwd(tail, g_logprob, g_entropy, g_value, g_vlogits, g_logits, scale, graw, w.ld_graw, gvraw, w.ld_gv, st));
     PdlScope pdl;
     begin_overlap(R);
 
-    // ---- recompute the critic's activations; its pool is in the saved z, beside the trunk's output
+    // ---- recompute the critic's activations (its pool lands in z beside the trunk's output)
     BSRL_TRY(layernorm(x_last, d, ident, c.G(l.critic_ln), c.Be(l.critic_ln), eps, R, d, h16, d, st));
     BSRL_TRY(linear(linear_args(hv, d, c.W(l.critic_kv), d, c.Bv(l.critic_kv), qkv + d, 3 * d, 0, 0, R, 2 * d, d), st));
     BSRL_TRY(linear(linear_args(hv_torso, kT * d, c.W(l.critic_q), d, c.Bv(l.critic_q), qkv + 2 * 3 * d, kT * 3 * d, 0, 0, B, d, d), st));
     BSRL_TRY(attention(qkv, 3 * d, sv.key_bias, B, d, l.H, 2, 1, attc, d, st));
-    BSRL_TRY(linear(linear_args(sv.z, ldz, c.W(l.critic_m0), ldz, c.Bv(l.critic_m0), m1, D, 0, 1, B, D, ldz), st));
+    BSRL_TRY(linear(linear_args(attc, d, c.W(l.critic_out), d, c.Bv(l.critic_out), z, ldz, 0, 0, B, d, d), st));
+    BSRL_TRY(linear(linear_args(z, ldz, c.W(l.critic_m0), ldz, c.Bv(l.critic_m0), m1, D, 0, 1, B, D, ldz), st));
     BSRL_TRY(linear(linear_args(m1, D, c.W(l.critic_m1), D, c.Bv(l.critic_m1), m2, D, 0, 1, B, D, D), st));
 
     // ---- critic MLP
@@ -418,7 +424,7 @@ struct Bwd {
     BSRL_TRY(dgrad(gvraw, w.ld_gv, B, c.W(l.critic_m2), l.critic_m2.pitch, l.bins_pad, D, gs16, D, false, m2, D));
     BSRL_TRY(wgrad(gs16, D, B, D, m1, D, D, "critic_mlp.2"));
     BSRL_TRY(dgrad(gs16, D, B, c.W(l.critic_m1), l.critic_m1.pitch, D, D, gA, D, false, m1, D));
-    BSRL_TRY(wgrad(gA, D, B, D, sv.z, ldz, ldz, "critic_mlp.0"));
+    BSRL_TRY(wgrad(gA, D, B, D, z, ldz, ldz, "critic_mlp.0"));
     BSRL_TRY(dgrad(gA, D, B, c.W(l.critic_m0), l.critic_m0.pitch, D, ldz, gz32, ldz, true));     // g_z = [g_a | g_h from the critic]
     // critic attention pool
     BSRL_TRY(cast16(gz32, ldz, ident, gs16, d, B, d));                                           // g_a
