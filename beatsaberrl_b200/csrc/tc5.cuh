@@ -30,14 +30,15 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
 __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
-// CLUSTER: the barrier is one that threads of the pair's other CTA arrive at (mbar_arrive_cluster) or store with (st.async)
+// CLUSTER: the barrier is one that threads of the pair's other CTA arrive at (mbar_arrive_cluster) or store with (st.async);
+// the acquire that goes with it is wait_acquire_cluster, once the wait is over
 template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   if (CLUSTER)
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;\n\t"
         "selp.b32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
         : "r"(bar), "r"(parity)
@@ -52,11 +53,17 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
         : "memory");
   return ok != 0;
 }
+// of shared memory only: with the wait's own .acquire.cluster the issuing thread of gemm_pair_tc5.cu stands still for so long
+// that a forward of 266 K rows through six 512-wide blocks takes 14.19 ms instead of 13.93; this costs nothing measurable
+__device__ __forceinline__ void wait_acquire_cluster() { asm volatile("fence.acquire.sync_restrict::shared::cluster.cluster;" ::: "memory"); }
 // Bounded wait: false when `limit` polls ran out or another role already gave up (*abort != 0).
 template <bool CLUSTER = false>
 __device__ __forceinline__ bool mbar_wait_limit(uint32_t bar, uint32_t parity, volatile int* abort, uint32_t limit) {
   for (uint32_t i = 0; i < limit; ++i) {
-    if (mbar_try_wait<CLUSTER>(bar, parity)) return true;   // the hardware parks the thread inside try_wait
+    if (mbar_try_wait<CLUSTER>(bar, parity)) {   // the hardware parks the thread inside try_wait
+      if (CLUSTER) wait_acquire_cluster();
+      return true;
+    }
     if ((i & 1023u) == 1023u && *abort) return false;
   }
   return false;
@@ -91,7 +98,6 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int 
                "r"(src), "r"(x), "r"(y)
                : "memory");
 }
-// the same box ADDED to the fp32 rows in global memory (split-K partial products)
 // Output rows placed by a row map, from a staged block of 32 rows x 128 bytes: as long as the map keeps runs of 8 rows
 // together, four boxes of 8 rows do what one box of 32 does for dense rows.
 inline bool dense_rows(const RowMap& m) { return m.group == 0x7fffffff && m.stride == 0 && m.first == 0; }
@@ -104,6 +110,7 @@ __device__ __forceinline__ void store_mapped8(const CUtensorMap* map, int x, int
   for (int i = 0; i < 4; ++i)
     if (m0 + 8 * i < rows) tma_store_2d(map, x, (int)cmap(m0 + 8 * i), src + i * 1024);
 }
+// a box ADDED to the fp32 rows in global memory (split-K partial products)
 __device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, int x, int y, uint32_t src) {
   asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"(
                    reinterpret_cast<uint64_t>(map)),

@@ -40,6 +40,8 @@ def test_barriers_of_both_ctas_are_awaited_at_cluster_scope():
             for fn, scope in calls:
                 assert fn == "wait_epilogue" or scope in ("<true>", "<PAIR>", "<CL == 2>"), (name, bar, fn, scope)
     assert "return mbar_wait<PAIR>(bar, parity, abort);" in text["block_tail_tc5.cu"]
+    assert "if (CLUSTER) wait_acquire_cluster();" in text["tc5.cuh"]
+    assert re.search(r"wait_acquire_cluster\(\) \{ asm volatile\(\"fence\.acquire[\w.:]*\.cluster;", text["tc5.cuh"])
 
 
 def test_copied_operands_go_to_a_kernel_that_waits_for_them():
