@@ -400,11 +400,12 @@ class NotePolicy(nn.Module):
             if total < 0:
                 raise nat.BsrlError(int(total), nat.last_error())
             pieces, order, at = [], [0] * n, 0
+            shapes = [p.shape for p in self._table_params()]
             for i in sorted(range(n), key=lambda i: offs[i]):
                 if offs[i] > at:
                     pieces.append(torch.empty(offs[i] - at, device="meta"))
                 order[i] = len(pieces)
-                pieces.append(torch.empty(self._table_params()[i].shape, device="meta"))
+                pieces.append(torch.empty(shapes[i], device="meta"))
                 at = offs[i] + pieces[-1].numel()
             pieces.append(torch.empty(total - at, device="meta"))
             self._grad_cut = (int(total), pieces, order)
