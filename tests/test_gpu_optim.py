@@ -241,7 +241,9 @@ def test_optimizers_read_their_lists_on_every_step():
 
     grads()
     adam.step()
-    adam.exclude = frozenset(names)
+    adam.exclude = set(names[1:])
+    adam.step()
+    adam.exclude.add(names[0])                               # in place, too
     before = {n: p.detach().clone() for n, p in named.items()}
     adam.step()
     assert all(torch.equal(p, before[n]) == (n in adam.exclude) for n, p in named.items())
