@@ -16,8 +16,9 @@
 // 128 x 128 output tile per CTA, longest contractions first, and S and P -- symmetric -- from their lower tiles only,
 // mirrored by the epilogue.  A k-block is 96 KB of operand tiles for 24 MMAs of N = 128 (1,536 cycles), so loads and MMAs
 // take about equally long; at these sizes (K of 4 to 20 k-blocks) a tile's fixed costs -- first loads, epilogue -- are as
-// much again.  d = 256, four blocks, 33 matrices: 0.56 ms per step; as batched fp32 torch products and element-wise
-// launches it was 2.1 ms of GPU time and 2.9 ms of host time.
+// much again.  d = 256, four blocks, 33 matrices: 0.56 ms per step, of which the 15 product stages are 0.48, momentum and
+// planes 0.04, the weights' refresh 0.02; as batched fp32 torch products and element-wise launches it was 2.1 ms of GPU time
+// and 2.9 ms of host time.
 #include <string.h>
 
 #include <algorithm>

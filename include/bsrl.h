@@ -143,6 +143,7 @@ int bsrl_muon_step(const bsrl_config* cfg, float* const* params, const float* co
                    void* arena, int64_t arena_bytes, void* workspace, int64_t workspace_bytes, void* stream);
 
 /* --- forward -------------------------------------------------------------------- */
+/* Bytes of workspace for n_envs: enough for every smaller batch too. */
 int64_t bsrl_workspace_bytes(const bsrl_config* cfg, int64_t n_envs);
 
 /* NotePolicy.forward_stacked (python/policy.py:1179-1344): obs (n_envs, 630) f32 or f16
@@ -223,12 +224,13 @@ int bsrl_forward_rollout(const bsrl_config* cfg, const void* arena, const void* 
  * grad mode, then loss.backward().  The reference gets its backward from autograd over its
  * autograd.Functions (python/fp16_linear.py:461-767, :931-1064, :1197-1251; python/fused_ln.py:58-107)
  * and their kernels (ln_bwd*, attn29_bwd, wgrad / wgrad_bgrad / dgrad_drelu / relu_bwd); here the two
- * halves are two calls.  Not built for emb_ln / final_ln / value_residual / trunk_v2 (BSRL_ERR_UNSUPPORTED).
+ * halves are two calls.
  *
  * bsrl_forward_train: same arguments and outputs as bsrl_forward_act, computed by the same kernels
  * (outputs are bit-identical to bsrl_forward_act's), plus a caller-owned `save` buffer of
  * bsrl_train_save_bytes() that receives what the backward needs: the tokenizer's feature rows, the key
- * bias, the residual stream entering every block, the readout rows, the head outputs. */
+ * bias, the residual stream entering every block, the readout rows, the trunk's activations, the critic's
+ * pool, the head outputs.  bsrl_backward only reads it. */
 int64_t bsrl_train_save_bytes(const bsrl_config* cfg, int64_t n_envs);
 int bsrl_forward_train(const bsrl_config* cfg, const void* arena, const void* obs, int32_t obs_dtype, int64_t n_envs,
                        const void* actions, int32_t act_dtype, float* logits, float* logprob, float* entropy,
