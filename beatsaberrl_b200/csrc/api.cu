@@ -879,7 +879,8 @@ int bsrl_forward_fixed(const bsrl_config* cfg, const void* arena, const void* ob
     set_error("forward_fixed: n_envs %lld is negative", (long long)n_envs);
     return BSRL_ERR_SHAPE;
   }
-  const int64_t need = bsrl_workspace_bytes(cfg, n_envs);
+  const Layout l = make_layout(*cfg);
+  const int64_t need = make_workspace(l, n_envs, plan_paths(l, g_engine.load(std::memory_order_relaxed), n_envs)).bytes;   // this batch's own
   if (need > BSRL_FIXED_SCRATCH_BYTES) {
     set_error("forward_fixed: %lld envs need %lld bytes of scratch, the built-in scratch holds %lld; "
               "use bsrl_forward with a caller workspace for larger batches",
