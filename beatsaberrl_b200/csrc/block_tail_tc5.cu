@@ -801,11 +801,13 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
 #pragma unroll
           for (int jj = 0; jj < 8; ++jj) {
             const float4 b0 = P_b0[((j * HC + grp * 64 + c) >> 2) + jj];
-            const float a0 = __uint_as_float(r[4 * jj]) + b0.x, a1 = __uint_as_float(r[4 * jj + 1]) + b0.y;
-            const float a2 = __uint_as_float(r[4 * jj + 2]) + b0.z, a3 = __uint_as_float(r[4 * jj + 3]) + b0.w;
+            float a0 = __uint_as_float(r[4 * jj]) + b0.x, a1 = __uint_as_float(r[4 * jj + 1]) + b0.y;
+            float a2 = __uint_as_float(r[4 * jj + 2]) + b0.z, a3 = __uint_as_float(r[4 * jj + 3]) + b0.w;
             if (GELU) {
-              hp[(c >> 1) + 2 * jj] = pack_half2(gelu_exact(a0), gelu_exact(a1));
-              hp[(c >> 1) + 2 * jj + 1] = pack_half2(gelu_exact(a2), gelu_exact(a3));
+              gelu_exact2(a0, a1);
+              gelu_exact2(a2, a3);
+              hp[(c >> 1) + 2 * jj] = pack_half2(a0, a1);
+              hp[(c >> 1) + 2 * jj + 1] = pack_half2(a2, a3);
             } else {
               hp[(c >> 1) + 2 * jj] = pack_half2(fmaxf(a0, 0.f), fmaxf(a1, 0.f));
               hp[(c >> 1) + 2 * jj + 1] = pack_half2(fmaxf(a2, 0.f), fmaxf(a3, 0.f));

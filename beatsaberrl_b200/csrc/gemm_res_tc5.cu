@@ -236,7 +236,12 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(fmaxf(__uint_as_float(a[j]), 0.f));
       } else if (p.relu == 2) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(gelu_exact(__uint_as_float(a[j])));
+        for (int j = 0; j < 32; j += 2) {
+          float v0 = __uint_as_float(a[j]), v1 = __uint_as_float(a[j + 1]);
+          gelu_exact2(v0, v1);
+          a[j] = __float_as_uint(v0);
+          a[j + 1] = __float_as_uint(v1);
+        }
       }
     };
     uint32_t tile_i = 0;

@@ -286,7 +286,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
           } else if (p.relu == 2) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = gelu_exact(v[j]);
+            for (int j = 0; j < 32; j += 2) gelu_exact2(v[j], v[j + 1]);
           }
           if (masked) {
 #pragma unroll

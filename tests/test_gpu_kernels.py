@@ -460,6 +460,24 @@ def test_linear_cta_pairs(native, m, n, k, relu, resid, f32):
     assert bool(((out.double() - ref).abs() <= tol * ref.abs() + 4e-5).all())
 
 
+@pytest.mark.parametrize("m,k,engine,kernel", [(992, 64, 0, "linear_mma"), (992, 64, 2, "linear_small"), (992, 64, 1, "linear_tc5"),
+                                               (992 * 60, 64, 1, "linear_res"), (124 * 160, 512, 1, "linear_pair")])
+def test_gelu_of_every_half(native, m, k, engine, kernel):
+    """GELU in the epilogues, on every finite fp16 number (the product is with an identity matrix): half an ulp of the
+    fp16 result, plus what the fit and its fp32 evaluation may be off: 1.2e-7 |x|, 2e-5 of a negative result."""
+    bits = torch.arange(65536, device="cuda").to(torch.int16).view(torch.float16)
+    x = bits[bits.isfinite()]
+    a = x.repeat(m * k // x.numel()).view(m, k).contiguous()
+    out = torch.full((m, k), float("nan"), dtype=torch.float16, device="cuda")
+    w = torch.eye(k, device="cuda").half()
+    ran = kernels_of(lambda: native.check(native.lib.bsrl_linear(
+        a.data_ptr(), w.data_ptr(), None, None, out.data_ptr(), 0, 2, m, k, k, engine, _stream())))
+    assert len(ran) == 1 and kernel in ran[0], ran
+    ref = F.gelu(a.double())
+    bound = ref.abs().clamp_min(2.0 ** -14) * 2.0 ** -11 + 1.2e-7 * a.double().abs().clamp_max(8) + 2e-5 * ref.abs()
+    assert bool(((out.double() - ref).abs() <= bound).all())
+
+
 @pytest.mark.parametrize("m,n,k,f32", [(18945, 512, 512, 0), (19021, 320, 512, 1), (12801, 2048, 768, 0)])
 def test_linear_cta_pairs_read_weights_by_rows(native, m, n, k, f32):
     """Input gradients g W on CTA pairs: the weight's rows are the contraction index.  Bounds as in test_linear_cta_pairs."""
