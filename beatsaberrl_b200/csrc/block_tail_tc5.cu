@@ -23,12 +23,19 @@
 //   warp 10      TMA producer of the attention tiles (att tile -> sA, d/64 chunks of [128 x 64], 128B
 //                swizzle; sA is freed before the tile ends); pulls the next tile's residual rows into L2
 //   warp 1       MMA issuer (one thread): tcgen05.mma, M = 128, K = 16
-//   warps 2..9   epilogue (two groups of four warps, each group owns half of the columns), thread = row:
+//   warps 2..9   epilogue (two groups of four warps, each group owns half of the columns):
 //                LayerNorm on TMEM rows -> h2 into sA; bias + ReLU of each 128-wide hidden chunk -> sH;
-//                final drain and LayerNorm outputs.  Global traffic moves as per-warp TMA boxes (32 rows
+//                final drain and LayerNorm outputs.  Row sums and fp32 rows go one row per thread; whatever only
+//                scales and shifts columns works on fragments (tc5.cuh): the MMA operands alone take 1,280 of the
+//                2,048 cycles of shared-memory bandwidth that a chunk has, and with one row per thread the parameter
+//                reads and the hidden took another 770.  Global traffic moves as per-warp TMA boxes (32 rows
 //                x 64 or 128 bytes) through three swizzled buffers per warp -- residual rows in, fp32 and
 //                fp16 rows out; rows gathered through a row map fall back to coalesced loads through
 //                the staging buffer.  The per-column parameters live in shared memory.
+// Cycles of a tile in a long run (d = 256, pairs), before -> with fragments and early residual blocks: LayerNorm 3,500 ->
+// 2,300, chunk 2,350 -> 2,190, pre-store 5,000 -> 3,900, one fp16 output 4,300 -> 3,400, fp32 rows 3,900 -> 4,100 (192 KB leave
+// an SM at ~26 B per cycle, on every SM at the same time: that is what the drain waits for).  65,536 environments: 14.64 ->
+// 13.80 ms before the power cap sets in, 16.06 -> 15.69 in a loop; d 192, 32,768 environments 8.57 -> 8.44.
 // TMEM (512 columns): region X (d columns) accumulates x1 and then xo in place -- x is
 // pre-stored there by the epilogue warps, so the out-projection and the FFN-down MMAs simply
 // accumulate onto it; the other 256 columns are two 128-column buffers for hidden chunks.  The
@@ -164,18 +171,6 @@ __device__ __forceinline__ void mma_kblock(uint32_t d_tmem, uint32_t a_addr, uin
 template <int N>
 using StageNo = std::integral_constant<int, N>;
 
-// 32 fp32 values of row `row`, columns [col, col + 32) -> fp16 into a swizzled [128 x 64] chunk set
-__device__ __forceinline__ void store_h32(uint8_t* chunks, int row, int col, const float (&v)[32]) {
-  uint8_t* base = chunks + (col >> 6) * CHUNK_BYTES + (row >> 3) * 1024 + (row & 7) * 128;
-  const int p0 = (col & 63) >> 3;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint4 w = make_uint4(pack_half2(v[8 * i], v[8 * i + 1]), pack_half2(v[8 * i + 2], v[8 * i + 3]),
-                         pack_half2(v[8 * i + 4], v[8 * i + 5]), pack_half2(v[8 * i + 6], v[8 * i + 7]));
-    *reinterpret_cast<uint4*>(base + (((p0 + i) ^ (row & 7)) << 4)) = w;
-  }
-}
-
 // GELU: the FFN activation is the exact GELU instead of ReLU (a compile-time variant: the hidden-chunk
 // epilogue sits on the chunk loop's critical path)
 template <bool GELU, bool PAIR>
@@ -199,7 +194,6 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
   constexpr int STG_BYTES = stg_bytes<PAIR>(), IO_BYTES = io_bytes<PAIR>(), CB = IO_BYTES / 128;   // CB: fp32 columns per block
   const uint32_t rank = PAIR ? cluster_rank() : 0u;
   const uint32_t sA = base, sH = base + SA_BYTES, ring = sH + SH_BYTES;
-  uint8_t* sA_g = gen;
   uint8_t* sH_g = gen + SA_BYTES;
   uint8_t* stg_all = gen + SA_BYTES + SH_BYTES + RING_BYTES;
   float* prm = reinterpret_cast<float*>(stg_all + EPI_WARPS * STG_BYTES);
@@ -608,7 +602,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
     const int sub8 = lane >> 2, piece = lane & 3;
     const int dh2 = d >> 1, c_lo = grp * dh2;               // this group's columns of the d-wide row
     const float4* prm4 = reinterpret_cast<const float4*>(prm);
-    const float4 *P_bo = prm4, *P_g = prm4 + 64, *P_b = prm4 + 128, *P_b2 = prm4 + 192, *P_b0 = prm4 + 512;
+    const float4 *P_bo = prm4, *P_b2 = prm4 + 192;
     uint32_t tile_i = 0, n_acc[2] = {0, 0}, n_free = 0;
     bool ok = true;
     const float inv_d = 1.0f / (float)d;
@@ -623,10 +617,28 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
     auto at64 = [](int row, int pc) -> int { return row * 64 + ((pc ^ ((row >> 1) & 3)) << 4); };
     auto at128 = [](int row, int pc) -> int { return row * 128 + ((pc ^ (row & 7)) << 4); };
     auto io_at = [&](int row, int pc) -> int { return PAIR ? at128(row, pc) : at64(row, pc); };
+    // Fragments (tmem_ld_frag32): this thread's rows are fr + 8 i of the warp's 32, its columns fc, fc + 1 of every 8.
+    // store_frag: 8 rows x 32 fp16 columns (r0..r3: 8 columns each) as four 16-byte pieces per row; piece 0 or 4 onwards
+    const int fr = lane >> 2, fc = 2 * (lane & 3), st_row = lane & 7, st_piece = lane >> 3;
+    const uint64_t* prm_frag = reinterpret_cast<const uint64_t*>(prm + fc);      // parameter pair of 8-column unit u of vector v: [128 v + 4 u]
+    auto load_frag = [&](uint32_t col, uint32_t (&r)[32]) {      // 32 rows x 32 columns: rows fr, fr + 8 in r[0..15], fr + 16, fr + 24 in r[16..31]
+      tmem_ld_frag32(lane_base + col, r);
+      tmem_ld_frag32(lane_base + (16u << 16) + col, r + 16);
+    };
+    // body(c, r) for the 32-column blocks of [c_lo, c_lo + d / 2): load(c, r) requests a block while the one before it is worked on
+    auto each_block = [&](auto&& load, auto&& body) {
+      for (int c = c_lo; c < c_lo + dh2; c += 32) {
+        uint32_t r[32];
+        load(c, r);
+        tmem_wait_ld();
+        body(c, r);
+      }
+    };
     auto stg_write = [&](int row, int pc, uint4 v) { *reinterpret_cast<uint4*>(stg + at64(row, pc)) = v; };
     auto stg_read = [&](int row, int pc) -> uint4 { return *reinterpret_cast<const uint4*>(stg + at64(row, pc)); };
-    uint32_t n_io = 0;                                      // residual blocks this warp has consumed so far
-    auto group_sync = [&]() { asm volatile("bar.sync 2, %0;" ::"n"(EPI_WARPS * 32) : "memory"); };
+    uint32_t io_phase = 0;                                  // bit b: phase of the next residual block in row buffer b
+    int n_early = 0;                                        // residual blocks of the next tile requested ahead of its pre-store
+    auto group_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory"); };     // the two warps that share these rows
     auto signal = [&](uint64_t* bar) {   // one arrival per warp, after everyone's writes
       tc_fence_before();
       __syncwarp();
@@ -645,6 +657,24 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
       const float2 o = part[(phase * 2 + (grp ^ 1)) * BM + trow];
       mean = (sum + o.x) * inv_d;
       rstd = rsqrtf(fmaxf((sq + o.y) * inv_d - mean * mean, 0.f) + p.eps);
+    };
+    // values of this thread's fragment rows out of the row-per-thread scale and shift, one per row of the warp
+    auto frag_scale = [&](float scale, float shift, uint64_t (&sc)[4], uint64_t (&sf)[4]) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float a = __shfl_sync(0xffffffffu, scale, fr + 8 * i), b = __shfl_sync(0xffffffffu, shift, fr + 8 * i);
+        sc[i] = f2_make(a, a);
+        sf[i] = f2_make(b, b);
+      }
+    };
+    auto frag_at = [](const uint32_t (&r)[32], int i, int u) -> uint64_t {      // row fr + 8 i, 8-column unit u of a block
+      const int at = 16 * (i >> 1) + 4 * u + 2 * (i & 1);
+      return f2_make(__uint_as_float(r[at]), __uint_as_float(r[at + 1]));
+    };
+    auto pack_f2 = [](uint64_t v) -> uint32_t {
+      float a, b;
+      f2_split(v, a, b);
+      return pack_half2(a, b);
     };
     // pre-store (x + bo) of tile t, this group's columns, into TMEM columns col0 + ...
     // (a) rows gathered through the row map: coalesced loads, transposed through the staging buffer
@@ -687,31 +717,36 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
       }
       tmem_wait_st();
     };
-    // (b) dense rows: CB-column blocks of this warp's 32 rows arrive by TMA in the three buffers, up to
-    // three in flight; block n (counted over the whole kernel) uses buffer n % 3, phase (n / 3) & 1
+    // (b) dense rows: CB-column blocks of this warp's 32 rows arrive by TMA in the three buffers, block k in buffer k % 3.
+    // The blocks whose buffers lie in the staging area are requested as soon as the previous drain has left it, a whole
+    // FFN ahead; the others once the tile's MMAs have retired.
+    const int nb = dh2 / CB;
+    auto issue_block = [&](int t, int k) {
+      if (lane == 0) {
+        const uint32_t bar = smem_u32(&sh->io_full[warp - 2][k % 3]);
+        mbar_expect_tx(bar, IO_BYTES);
+        tma_load_2d(smem_u32(io_buf(k % 3)), &tm_x, c_lo + CB * k, t * BM + q * 32, bar);
+      }
+    };
+    auto request_early = [&](int t) {
+      if (!p.x_tma) return;
+      n_early = nb < (PAIR ? 2 : 1) ? nb : PAIR ? 2 : 1;
+      for (int k = 0; k < n_early; ++k) issue_block(t, k);
+    };
     auto prestore_tma = [&](int t, uint32_t col0) -> bool {
-      const int row0 = t * BM + q * 32;
-      const int nb = dh2 / CB;
-      auto issue = [&](int k) {                             // k-th block of this call
-        if (lane == 0) {
-          const uint32_t n = n_io + k;
-          const uint32_t bar = smem_u32(&sh->io_full[warp - 2][n % 3]);
-          mbar_expect_tx(bar, IO_BYTES);
-          tma_load_2d(smem_u32(io_buf(n % 3)), &tm_x, c_lo + CB * k, row0, bar);
-        }
-      };
-      for (int k = 0; k < 3 && k < nb; ++k) issue(k);
-      int k = 0;
+      for (int k = n_early; k < 3 && k < nb; ++k) issue_block(t, k);
+      int k = 0, b = 0;
       for (int c = c_lo; c < c_lo + dh2; c += 32) {
         uint32_t r[32];
 #pragma unroll
         for (int hb = 0; hb < 32 / CB; ++hb, ++k) {
-          const uint32_t n = n_io + k;
-          if (!mbar_wait_warp(smem_u32(&sh->io_full[warp - 2][n % 3]), (n / 3) & 1, abort)) {
+          if (!mbar_wait_warp(smem_u32(&sh->io_full[warp - 2][b]), (io_phase >> b) & 1, abort)) {
             if (lane == 0) give_up(sh, p.status, 15);
+            n_early = 0;
             return false;
           }
-          const uint8_t* buf = io_buf(n % 3);
+          io_phase ^= 1u << b;
+          const uint8_t* buf = io_buf(b);
 #pragma unroll
           for (int j = 0; j < CB / 4; ++j) {
             const uint4 v = *reinterpret_cast<const uint4*>(buf + io_at(lane, j));
@@ -722,11 +757,12 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
             r[CB * hb + 4 * j + 3] = __float_as_uint(__uint_as_float(v.w) + bo.w);
           }
           __syncwarp();                                     // everyone has read the buffer: refill it
-          if (k + 3 < nb) issue(k + 3);
+          if (k + 3 < nb) issue_block(t, k + 3);
+          b = b == 2 ? 0 : b + 1;
         }
         tmem_st32(lane_base + col0 + c, r);
       }
-      n_io += nb;
+      n_early = 0;
       tmem_wait_st();
       return true;
     };
@@ -745,40 +781,38 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
       const uint32_t par = tile_i & 1;
       const uint32_t xcol = par ? 256u : 0u, acol = par ? 0u : 256u;
       const int t_next = t + tstep;
+      if (t_next < t_end) request_early(t_next);
       // ---- E1: h2 = LN_ffn(x1) -> sA   (X already holds x + bo + att Wo^T)
       TAIL_WAIT_WARP(&sh->o_done, par, 11);
       tc_fence_after();
       {
         float sum = 0.f, sq = 0.f;
-        for (int c = c_lo; c < c_lo + dh2; c += 32) {
-          uint32_t r[32];
-          tmem_ld32(lane_base + xcol + c, r);
-          tmem_wait_ld();
+        each_block([&](int c, uint32_t (&r)[32]) { tmem_ld32(lane_base + xcol + c, r); },
+                   [&](int, const uint32_t (&r)[32]) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const float v = __uint_as_float(r[j]);
-            sum += v;
-            sq = fmaf(v, v, sq);
-          }
-        }
+                     for (int j = 0; j < 32; ++j) {
+                       const float v = __uint_as_float(r[j]);
+                       sum += v;
+                       sq = fmaf(v, v, sq);
+                     }
+                   });
         float mean, rstd;
         row_stats(0, sum, sq, mean, rstd);
-        const float shift = -mean * rstd;
-        for (int c = c_lo; c < c_lo + dh2; c += 32) {
-          uint32_t r[32];
-          float v[32];
-          tmem_ld32(lane_base + xcol + c, r);
-          tmem_wait_ld();
+        uint64_t sc[4], sf[4];
+        frag_scale(rstd, -mean * rstd, sc, sf);
+        each_block([&](int c, uint32_t (&r)[32]) { load_frag(xcol + c, r); },
+                   [&](int c, const uint32_t (&r)[32]) {
+                     uint32_t h[4][4];
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float4 g = P_g[(c >> 2) + j], bb = P_b[(c >> 2) + j];
-            v[4 * j] = fmaf(fmaf(__uint_as_float(r[4 * j]), rstd, shift), g.x, bb.x);
-            v[4 * j + 1] = fmaf(fmaf(__uint_as_float(r[4 * j + 1]), rstd, shift), g.y, bb.y);
-            v[4 * j + 2] = fmaf(fmaf(__uint_as_float(r[4 * j + 2]), rstd, shift), g.z, bb.z);
-            v[4 * j + 3] = fmaf(fmaf(__uint_as_float(r[4 * j + 3]), rstd, shift), g.w, bb.w);
-          }
-          store_h32(sA_g, trow, c, v);
-        }
+                     for (int u = 0; u < 4; ++u) {
+                       const uint64_t g = prm_frag[128 + (c >> 1) + 4 * u], b = prm_frag[256 + (c >> 1) + 4 * u];
+#pragma unroll
+                       for (int i = 0; i < 4; ++i) h[i][u] = pack_f2(f2_fma(f2_fma(frag_at(r, i, u), sc[i], sf[i]), g, b));
+                     }
+                     const uint32_t at = sA + (c >> 6) * CHUNK_BYTES + q * 4096 + st_row * 128 + (((st_piece ^ st_row) << 4) ^ ((c & 32) << 1));
+#pragma unroll
+                     for (int i = 0; i < 4; ++i) stmatrix_x4(at + i * 1024, h[i][0], h[i][1], h[i][2], h[i][3]);
+                   });
       }
       publish_smem();
       signal(&sh->h2_ready);
@@ -792,27 +826,29 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         }
         ++n_acc[b];
         tc_fence_after();
-        uint32_t hp[32];                                    // 64 fp16 values of this row
+        uint32_t hp[2][4][4];                               // [32 columns][rows fr + 8 i][8-column unit]: fp16 pairs
+        {
+          uint32_t r[2][32];
 #pragma unroll
-        for (int c = 0; c < 64; c += 32) {
-          uint32_t r[32];
-          tmem_ld32(lane_base + acol + b * HC + grp * 64 + c, r);
+          for (int c = 0; c < 2; ++c) load_frag(acol + b * HC + grp * 64 + 32 * c, r[c]);
           tmem_wait_ld();
 #pragma unroll
-          for (int jj = 0; jj < 8; ++jj) {
-            const float4 b0 = P_b0[((j * HC + grp * 64 + c) >> 2) + jj];
-            float a0 = __uint_as_float(r[4 * jj]) + b0.x, a1 = __uint_as_float(r[4 * jj + 1]) + b0.y;
-            float a2 = __uint_as_float(r[4 * jj + 2]) + b0.z, a3 = __uint_as_float(r[4 * jj + 3]) + b0.w;
-            if (GELU) {
-              gelu_exact2(a0, a1);
-              gelu_exact2(a2, a3);
-              hp[(c >> 1) + 2 * jj] = pack_half2(a0, a1);
-              hp[(c >> 1) + 2 * jj + 1] = pack_half2(a2, a3);
-            } else {
-              hp[(c >> 1) + 2 * jj] = pack_half2(fmaxf(a0, 0.f), fmaxf(a1, 0.f));
-              hp[(c >> 1) + 2 * jj + 1] = pack_half2(fmaxf(a2, 0.f), fmaxf(a3, 0.f));
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const uint64_t b0 = prm_frag[1024 + ((j * HC + grp * 64 + 32 * c) >> 1) + 4 * u];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                float a0, a1;
+                f2_split(f2_add(frag_at(r[c], i, u), b0), a0, a1);
+                if (GELU) {
+                  gelu_exact2(a0, a1);
+                  hp[c][i][u] = pack_half2(a0, a1);
+                } else {
+                  hp[c][i][u] = pack_half2(fmaxf(a0, 0.f), fmaxf(a1, 0.f));
+                }
+              }
             }
-          }
         }
         // this half of sH is free once the previous chunk's FFN-down MMAs on it have retired
         if (!mbar_wait_warp(smem_u32(&sh->hid_free[grp]), (n_free & 1) ^ 1, abort)) {
@@ -822,11 +858,11 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         }
         ++n_free;
         {
-          uint8_t* rowp = sH_g + grp * CHUNK_BYTES + (trow >> 3) * 1024 + (trow & 7) * 128;
+          const uint32_t at = sH + grp * CHUNK_BYTES + q * 4096 + st_row * 128 + ((st_piece ^ st_row) << 4);
 #pragma unroll
-          for (int pc = 0; pc < 8; ++pc)
-            *reinterpret_cast<uint4*>(rowp + ((pc ^ (trow & 7)) << 4)) =
-                make_uint4(hp[4 * pc], hp[4 * pc + 1], hp[4 * pc + 2], hp[4 * pc + 3]);
+          for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) stmatrix_x4((at ^ (c << 6)) + i * 1024, hp[c][i][0], hp[c][i][1], hp[c][i][2], hp[c][i][3]);
         }
         publish_smem();
         signal(&sh->hid_ready[grp]);
@@ -865,68 +901,66 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           }
           ++n_st;
         };
-        if (p.x_out || want_stats) {
-          for (int c = c_lo; c < c_lo + dh2; c += 32) {
-            uint32_t r[32];
-            tmem_ld32(lane_base + xcol + c, r);
-            tmem_wait_ld();
+        if (p.x_out || want_stats)
+          each_block([&](int c, uint32_t (&r)[32]) { tmem_ld32(lane_base + xcol + c, r); },
+                     [&](int c, const uint32_t (&r)[32]) {
 #pragma unroll
-            for (int hb = 0; hb < 32 / CB; ++hb) {
-              uint8_t* buf = p.x_out ? next_buf() : nullptr;
+                       for (int hb = 0; hb < 32 / CB; ++hb) {
+                         uint8_t* buf = p.x_out ? next_buf() : nullptr;
 #pragma unroll
-              for (int j = 0; j < CB / 4; ++j) {
-                const uint32_t* a = r + CB * hb + 4 * j;
-                const float4 b2 = P_b2[((c + CB * hb) >> 2) + j];
-                float4 v = make_float4(__uint_as_float(a[0]) + b2.x, __uint_as_float(a[1]) + b2.y, __uint_as_float(a[2]) + b2.z,
-                                       __uint_as_float(a[3]) + b2.w);
-                sum += (v.x + v.y) + (v.z + v.w);
-                sq = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sq))));
-                if (p.x_out) *reinterpret_cast<float4*>(buf + io_at(lane, j)) = v;
-              }
-              if (p.x_out) store_block(&tm_xo, c + CB * hb);
-            }
-          }
-        }
+                         for (int j = 0; j < CB / 4; ++j) {
+                           const uint32_t* a = r + CB * hb + 4 * j;
+                           const float4 b2 = P_b2[((c + CB * hb) >> 2) + j];
+                           float4 v = make_float4(__uint_as_float(a[0]) + b2.x, __uint_as_float(a[1]) + b2.y,
+                                                  __uint_as_float(a[2]) + b2.z, __uint_as_float(a[3]) + b2.w);
+                           sum += (v.x + v.y) + (v.z + v.w);
+                           sq = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sq))));
+                           if (p.x_out) *reinterpret_cast<float4*>(buf + io_at(lane, j)) = v;
+                         }
+                         if (p.x_out) store_block(&tm_xo, c + CB * hb);
+                       }
+                     });
         float mean = 0.f, rstd = 1.f;
         if (want_stats) row_stats(1, sum, sq, mean, rstd);
 #pragma unroll 1
         for (int o = 0; o < 2; ++o) {
           if (!p.out16[o]) continue;
           const bool ln = p.g16[o] != nullptr;
-          const float sc = ln ? rstd : 1.f, sh0 = ln ? -mean * rstd : 0.f;
-          const float4 *P_go = prm4 + 256 + 128 * o, *P_bo16 = prm4 + 320 + 128 * o;
+          uint64_t sc[4], sf[4];
+          frag_scale(ln ? rstd : 1.f, ln ? -mean * rstd : 0.f, sc, sf);
+          const int vg = 128 * (4 + 2 * o), vb = vg + 128;
           const CUtensorMap* tm_o = o ? &tm_o1 : &tm_o0;
           const bool wide = PAIR && p.wide16;
-          uint8_t* buf = nullptr;
-          for (int c = c_lo; c < c_lo + dh2; c += 32) {     // 32 columns = 64 bytes of fp16 per row: a block, or half of one
-            uint32_t r[32];
-            tmem_ld32(lane_base + xcol + c, r);
-            tmem_wait_ld();
-            const int half = wide ? ((c - c_lo) >> 5) & 1 : 0;
-            if (half == 0) buf = next_buf();
+          uint32_t buf = 0;
+          each_block([&](int c, uint32_t (&r)[32]) { load_frag(xcol + c, r); },     // 32 columns = 64 bytes of fp16 per row: a block, or half of one
+                     [&](int c, const uint32_t (&r)[32]) {
+                       const int half = wide ? ((c - c_lo) >> 5) & 1 : 0;
+                       if (half == 0) buf = smem_u32(next_buf());
+                       uint32_t h[4][4];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {                   // 8 columns -> one 16-byte fp16 piece
-              float y[8];
+                       for (int u = 0; u < 4; ++u) {
+                         const int at = (c >> 1) + 4 * u;
+                         const uint64_t b2 = prm_frag[384 + at], g = prm_frag[vg + at], bb = prm_frag[vb + at];
 #pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                const int f4 = (c >> 2) + 2 * j + e;
-                const float4 b2 = P_b2[f4], g = P_go[f4], bb = P_bo16[f4];
-                y[4 * e] = fmaf(fmaf(__uint_as_float(r[8 * j + 4 * e]) + b2.x, sc, sh0), g.x, bb.x);
-                y[4 * e + 1] = fmaf(fmaf(__uint_as_float(r[8 * j + 4 * e + 1]) + b2.y, sc, sh0), g.y, bb.y);
-                y[4 * e + 2] = fmaf(fmaf(__uint_as_float(r[8 * j + 4 * e + 2]) + b2.z, sc, sh0), g.z, bb.z);
-                y[4 * e + 3] = fmaf(fmaf(__uint_as_float(r[8 * j + 4 * e + 3]) + b2.w, sc, sh0), g.w, bb.w);
-              }
-              *reinterpret_cast<uint4*>(buf + (wide ? at128(lane, 4 * half + j) : at64(lane, j))) =
-                  make_uint4(pack_half2(y[0], y[1]), pack_half2(y[2], y[3]), pack_half2(y[4], y[5]), pack_half2(y[6], y[7]));
-            }
-            if (!wide || half == 1) store_block(tm_o, c - 32 * half);
-          }
+                         for (int i = 0; i < 4; ++i) h[i][u] = pack_f2(f2_fma(f2_fma(f2_add(frag_at(r, i, u), b2), sc[i], sf[i]), g, bb));
+                       }
+#pragma unroll
+                       for (int i = 0; i < 4; ++i)
+                         stmatrix_x4(buf + (wide ? at128(8 * i + st_row, 4 * half + st_piece) : at64(8 * i + st_row, st_piece)), h[i][0], h[i][1], h[i][2], h[i][3]);
+                       if (!wide || half == 1) store_block(tm_o, c - 32 * half);
+                     });
         }
         // the buffers (two of them inside sH) are reused by the next tile: all stores have read them
         if (lane == 0) bulk_wait_read<0>();
         __syncwarp();
       }
       tc_fence_before();
+    }
+    // residual blocks requested ahead of a pre-store that a wait above kept from running land before the CTA exits (bounded, ignoring abort)
+    for (int k = 0; lane == 0 && k < n_early; ++k) {
+      uint32_t spins = 0;
+      while (!mbar_try_wait(smem_u32(&sh->io_full[warp - 2][k]), (io_phase >> k) & 1) && ++spins < kSpinLimit) {}
+      if (spins >= kSpinLimit) give_up(sh, p.status, 15);
     }
     if (lane == 0) bulk_wait_all();                         // the stores are complete before the CTA exits
   }

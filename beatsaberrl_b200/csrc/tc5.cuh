@@ -215,6 +215,23 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       : "r"(taddr)
       : "memory");
 }
+// The same in fragments: 16 lanes x 8 N columns.  Thread t gets of every 8 columns its pair 2 (t % 4), + 1 in rows t / 4 (r[4 i],
+// r[4 i + 1]) and t / 4 + 8 (r[4 i + 2], r[4 i + 3]) -- what stmatrix stores, and a quarter of the columns per thread, so
+// that per-column parameters cost a quarter of the shared-memory reads of the one-row-per-thread form (where every lane
+// reads all of them: an LDS.128 returns 512 bytes, 4 cycles of the pipe the MMA operands come through, broadcast or not).
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t* r) {          // 16 lanes x 32 columns
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// four 8 x 8 matrices of 16-bit elements (register i: matrix i) to the 16-byte rows whose addresses lanes 8 i .. 8 i + 7 give
+__device__ __forceinline__ void stmatrix_x4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
