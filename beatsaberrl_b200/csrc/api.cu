@@ -452,6 +452,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
     pd.R = x; pd.ldr = d;
     g_stage = kStFfnDown;
     BSRL_TRY(linear(pd, c.st));
+    have_h = false;        // h holds this block's FFN operand (the encoder kernel may have left block 0's rows there)
   }
 
   // final block: keys/values over all 29 rows, everything else on the 5 lead rows

@@ -58,6 +58,16 @@ def test_parity_gates(name, geo, xavier, seed, B, padded):
     torch.testing.assert_close(ent.cpu(), rent, atol=5e-2, rtol=1e-2)
 
 
+@pytest.mark.parametrize("name,mult", [("cfg1", 1), ("cfg2", 8)])
+def test_ffn_widths_outside_the_fused_tail(name, mult):
+    """Hidden widths that the fused block tail does not take, behind the fused encoder kernel: every block's attention reads
+    its own LayerNorm rows."""
+    cfg = make_cfg(name, opts=dict(n_blocks=3, ffn_mult=mult))
+    sd = po.build_state_dict(cfg, 7, xavier=True)
+    obs = po.make_obs(70, 8, padded=True)
+    assert_parity(*cuda_policy(cfg, sd).forward_stacked(obs.cuda()), *po.forward_stacked(sd, cfg, obs), argmax_min=0.99)
+
+
 @pytest.mark.parametrize("B", [1, 3, 127, 129, 1000])
 def test_ragged_batches_and_batch_invariance(B):
     cfg, sd = golden_case("tiny_geo_mixed")
