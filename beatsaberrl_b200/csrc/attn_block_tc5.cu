@@ -24,7 +24,8 @@
 // the length of a chain.  There a PAIR of CTAs (cta_group::2) shares the weight tile: each fetches half of its
 // rows and the leader's MMAs (M = 256) read both.  65,536 envs, us in a loop of seconds, one set of workers / two /
 // two and pairs: 192 wide 885 / 790 / 800 (not taken: N = 144 pads to 160), 256 wide 1237 / 1164 / 1121; 16,384 envs
-// of 512: 925 / 925 / 863.
+// of 512: 925 / 925 / 863.  The drain works on fragments (tc5.cuh): with one row per thread its bias reads were two thirds
+// of the shared-memory time that it takes from the MMAs' operands and the attention.
 //
 // HBM traffic per token: read h (2d B), write att (2d B).  Replaces fp16_packed_linear + attn29 /
 // packed_sdpa (python/policy.py:586-600, :645-692; python/beat_arena_env/csrc/small_attn.cu).
@@ -376,19 +377,60 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
                   make_uint4(pack_half2(f[0], f[1]), pack_half2(f[2], f[3]), pack_half2(f[4], f[5]), pack_half2(f[6], f[7]));
             }
           };
-          int u = 0;
-          for (; u + 2 <= u_count; u += 2) {
-            uint32_t r[32];
-            tmem_ld32(tcol + u * 16, r);
-            tmem_wait_ld();
-            put16(r, u);
-            put16(r + 16, u + 1);
-          }
-          if (u < u_count) {
-            uint32_t r[16];
-            tmem_ld16(tcol + u * 16, r);
-            tmem_wait_ld();
-            put16(r, u);
+          // the same on fragments (tc5.cuh): 32 rows x 16 columns at a time, a quarter of the bias reads
+          auto put_frag = [&](const uint32_t* v, int u) {
+            const int st_row = lane & 7, st_half = (lane >> 3) & 1, st_piece = lane >> 4;   // stmatrix: rows 0..7, 8..15 of columns 0..7, then 8..15
+            const int un = u_first + u, row = q * EROWS + st_half * 8 + st_row;
+            const uint32_t dst = S::INPLACE ? sQ + (un >> 2) * SECTION : sQ + un * 32;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {                                // 16 rows
+              uint32_t h[2][2];
+#pragma unroll
+              for (int c = 0; c < 2; ++c) {
+                const uint64_t b = *reinterpret_cast<const uint64_t*>(bias_u + u * 16 + 8 * c + 2 * (lane & 3));
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
+                  h[c][k] = pack_f2(f2_add(f2_make(__uint_as_float(v[8 * e + 4 * c + 2 * k]), __uint_as_float(v[8 * e + 4 * c + 2 * k + 1])), b));
+              }
+              const int r = row + 16 * e;
+              stmatrix_x4(S::INPLACE ? section_at<LDQ>(dst, r, (un & 3) * 2 + st_piece) : dst + r * LDQ + st_piece * 16, h[0][0], h[0][1], h[1][0], h[1][1]);
+            }
+          };
+          if (VRES) {
+            int u = 0;
+            for (; u + 2 <= u_count; u += 2) {
+              uint32_t r[32];
+              tmem_ld32(tcol + u * 16, r);
+              tmem_wait_ld();
+              put16(r, u);
+              put16(r + 16, u + 1);
+            }
+            if (u < u_count) {
+              uint32_t r[16];
+              tmem_ld16(tcol + u * 16, r);
+              tmem_wait_ld();
+              put16(r, u);
+            }
+          } else {
+            auto load = [&](int u, uint32_t* r) {
+              tmem_ld_frag16(tcol + u * 16, r);
+              tmem_ld_frag16(tcol + (16u << 16) + u * 16, r + 8);
+            };
+            int u = 0;
+            for (; u + 2 <= u_count; u += 2) {
+              uint32_t r[32];
+              load(u, r);
+              load(u + 1, r + 16);
+              tmem_wait_ld();
+              put_frag(r, u);
+              put_frag(r + 16, u + 1);
+            }
+            if (u < u_count) {
+              uint32_t r[16];
+              load(u, r);
+              tmem_wait_ld();
+              put_frag(r, u);
+            }
           }
         }
         if (BODY && mt_own == 0 && lane < 12) *reinterpret_cast<uint4*>(sB_g + ((env_l * 2 + hh) * 3 + (lane >> 2)) * 64 + (lane & 3) * 16) = b0v;

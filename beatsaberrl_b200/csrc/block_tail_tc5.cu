@@ -618,13 +618,9 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
     auto at128 = [](int row, int pc) -> int { return row * 128 + ((pc ^ (row & 7)) << 4); };
     auto io_at = [&](int row, int pc) -> int { return PAIR ? at128(row, pc) : at64(row, pc); };
     // Fragments (tmem_ld_frag32): this thread's rows are fr + 8 i of the warp's 32, its columns fc, fc + 1 of every 8.
-    // store_frag: 8 rows x 32 fp16 columns (r0..r3: 8 columns each) as four 16-byte pieces per row; piece 0 or 4 onwards
+    // A stmatrix_x4 takes 8 rows x 32 columns: lane t gives the address of piece t / 8 of row t % 8.
     const int fr = lane >> 2, fc = 2 * (lane & 3), st_row = lane & 7, st_piece = lane >> 3;
     const uint64_t* prm_frag = reinterpret_cast<const uint64_t*>(prm + fc);      // parameter pair of 8-column unit u of vector v: [128 v + 4 u]
-    auto load_frag = [&](uint32_t col, uint32_t (&r)[32]) {      // 32 rows x 32 columns: rows fr, fr + 8 in r[0..15], fr + 16, fr + 24 in r[16..31]
-      tmem_ld_frag32(lane_base + col, r);
-      tmem_ld_frag32(lane_base + (16u << 16) + col, r + 16);
-    };
     // body(c, r) for the 32-column blocks of [c_lo, c_lo + d / 2): load(c, r) requests a block while the one before it is worked on
     auto each_block = [&](auto&& load, auto&& body) {
       for (int c = c_lo; c < c_lo + dh2; c += 32) {
@@ -666,15 +662,6 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         sc[i] = f2_make(a, a);
         sf[i] = f2_make(b, b);
       }
-    };
-    auto frag_at = [](const uint32_t (&r)[32], int i, int u) -> uint64_t {      // row fr + 8 i, 8-column unit u of a block
-      const int at = 16 * (i >> 1) + 4 * u + 2 * (i & 1);
-      return f2_make(__uint_as_float(r[at]), __uint_as_float(r[at + 1]));
-    };
-    auto pack_f2 = [](uint64_t v) -> uint32_t {
-      float a, b;
-      f2_split(v, a, b);
-      return pack_half2(a, b);
     };
     // pre-store (x + bo) of tile t, this group's columns, into TMEM columns col0 + ...
     // (a) rows gathered through the row map: coalesced loads, transposed through the staging buffer
@@ -800,14 +787,14 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         row_stats(0, sum, sq, mean, rstd);
         uint64_t sc[4], sf[4];
         frag_scale(rstd, -mean * rstd, sc, sf);
-        each_block([&](int c, uint32_t (&r)[32]) { load_frag(xcol + c, r); },
+        each_block([&](int c, uint32_t (&r)[32]) { tmem_ld_frags(lane_base + xcol + c, r); },
                    [&](int c, const uint32_t (&r)[32]) {
                      uint32_t h[4][4];
 #pragma unroll
                      for (int u = 0; u < 4; ++u) {
                        const uint64_t g = prm_frag[128 + (c >> 1) + 4 * u], b = prm_frag[256 + (c >> 1) + 4 * u];
 #pragma unroll
-                       for (int i = 0; i < 4; ++i) h[i][u] = pack_f2(f2_fma(f2_fma(frag_at(r, i, u), sc[i], sf[i]), g, b));
+                       for (int i = 0; i < 4; ++i) h[i][u] = pack_f2(f2_fma(f2_fma(frag_pair(r, i, u), sc[i], sf[i]), g, b));
                      }
                      const uint32_t at = sA + (c >> 6) * CHUNK_BYTES + q * 4096 + st_row * 128 + (((st_piece ^ st_row) << 4) ^ ((c & 32) << 1));
 #pragma unroll
@@ -830,7 +817,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         {
           uint32_t r[2][32];
 #pragma unroll
-          for (int c = 0; c < 2; ++c) load_frag(acol + b * HC + grp * 64 + 32 * c, r[c]);
+          for (int c = 0; c < 2; ++c) tmem_ld_frags(lane_base + acol + b * HC + grp * 64 + 32 * c, r[c]);
           tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 2; ++c)
@@ -840,7 +827,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
                 float a0, a1;
-                f2_split(f2_add(frag_at(r[c], i, u), b0), a0, a1);
+                f2_split(f2_add(frag_pair(r[c], i, u), b0), a0, a1);
                 if (GELU) {
                   gelu_exact2(a0, a1);
                   hp[c][i][u] = pack_half2(a0, a1);
@@ -932,7 +919,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
           const CUtensorMap* tm_o = o ? &tm_o1 : &tm_o0;
           const bool wide = PAIR && p.wide16;
           uint32_t buf = 0;
-          each_block([&](int c, uint32_t (&r)[32]) { load_frag(xcol + c, r); },     // 32 columns = 64 bytes of fp16 per row: a block, or half of one
+          each_block([&](int c, uint32_t (&r)[32]) { tmem_ld_frags(lane_base + xcol + c, r); },     // 32 columns = 64 bytes of fp16 per row: a block, or half of one
                      [&](int c, const uint32_t (&r)[32]) {
                        const int half = wide ? ((c - c_lo) >> 5) & 1 : 0;
                        if (half == 0) buf = smem_u32(next_buf());
@@ -942,7 +929,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
                          const int at = (c >> 1) + 4 * u;
                          const uint64_t b2 = prm_frag[384 + at], g = prm_frag[vg + at], bb = prm_frag[vb + at];
 #pragma unroll
-                         for (int i = 0; i < 4; ++i) h[i][u] = pack_f2(f2_fma(f2_fma(f2_add(frag_at(r, i, u), b2), sc[i], sf[i]), g, bb));
+                         for (int i = 0; i < 4; ++i) h[i][u] = pack_f2(f2_fma(f2_fma(f2_add(frag_pair(r, i, u), b2), sc[i], sf[i]), g, bb));
                        }
 #pragma unroll
                        for (int i = 0; i < 4; ++i)

@@ -267,8 +267,49 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
           if (p.out_f32) emit(col);
           else if (st & 1) emit(col - 32);
         }
+      } else if (!p.mask) {
+        // ---- fp16 in fragments, 64 columns at a time: bias and activation on pairs of columns, rows leave by stmatrix
+        const int fc = 2 * (lane & 3), st_row = lane & 7, st_piece = lane >> 3;
+        uint32_t a[32], b[32];
+        tmem_ld_frags(tbase, a);
+#pragma unroll 1
+        for (int st = 0; st < BN / 128; ++st) {
+          const int col = c0 + 64 * st;
+          auto half = [&](const uint32_t (&r)[32], int hc) {   // 32 columns
+            uint32_t h[4][4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const uint64_t bv = p.bias ? *reinterpret_cast<const uint64_t*>(p.bias + col + 32 * hc + 8 * u + fc) : 0ull;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                uint64_t v = frag_pair(r, i, u);
+                if (p.bias) v = f2_add(v, bv);
+                float v0, v1;
+                f2_split(v, v0, v1);
+                if (p.relu == 1) {
+                  v0 = fmaxf(v0, 0.f);
+                  v1 = fmaxf(v1, 0.f);
+                } else if (p.relu == 2) {
+                  gelu_exact2(v0, v1);
+                }
+                h[i][u] = pack_half2(v0, v1);
+              }
+            }
+            if (hc == 0) wait_staging();
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              stmatrix_x4(smem_u32(stg) + (8 * i + st_row) * 128 + (((4 * hc + st_piece) ^ st_row) << 4), h[i][0], h[i][1], h[i][2], h[i][3]);
+          };
+          tmem_wait_ld();
+          tmem_ld_frags(tbase + 64 * st + 32, b);
+          half(a, 0);
+          tmem_wait_ld();
+          if (st + 1 < BN / 128) tmem_ld_frags(tbase + 64 * (st + 1), a);
+          half(b, 1);
+          emit(col);
+        }
       } else {
-        // ---- fp16, 64 columns at a time
+        // ---- fp16 with a mask, 64 columns at a time
         uint32_t a[32], b[32], h[32];
         tmem_ld32(tbase, a);
         tmem_ld32(tbase + 32, b);
@@ -276,7 +317,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         for (int st = 0; st < BN / 128; ++st) {
           const int col = c0 + 64 * st;
           uint4 mk[8];                                       // this row's 64 mask entries
-          if (p.mask && live) {
+          if (live) {
             const __half* mrow = p.mask + row * p.ldm + col;
 #pragma unroll
             for (int j = 0; j < 8; ++j) mk[j] = *reinterpret_cast<const uint4*>(mrow + 8 * j);
@@ -292,7 +333,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
             tmem_ld32(tbase + 64 * (st + 1), a);
             tmem_ld32(tbase + 64 * (st + 1) + 32, b);
           }
-          if (p.mask && live) {
+          if (live) {
 #pragma unroll
             for (int j = 0; j < 32; ++j) h[j] = keep_positive(h[j], reinterpret_cast<const uint32_t*>(mk)[j]);
           }

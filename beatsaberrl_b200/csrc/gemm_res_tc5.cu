@@ -18,12 +18,13 @@
 // stages 224 us, two and two (single CTA) 285.
 // Measured, 475 K rows, us, gemm_tc5.cu / single CTAs / pairs: x 768 x 256 fp16 304 / 231 / 217, x 1024 x 256 with ReLU
 // 439 / 318 / 289, x 576 x 192 246 / 207 / 191, x 384 x 128 175 / 128 / 115, x 192 x 192 fp32 + residual 291 / 204 / 195,
-// x 256 x 256 fp32 + residual 323 / 248 / 242.
+// x 256 x 256 fp32 + residual 323 / 248 / 242.  fp16 rows in fragments (tc5.cuh): a quarter of the bias reads, none where
+// there is no bias, packed adds: the twenty such products of an update of 16,384 environments at d 256 3.88 -> 3.52 ms.
 //
 // ReLU masks as bits: a product with ReLU can leave one bit per output (1 = positive), which the product that carries
-// the gradient back reads instead of the fp16 activations: 1/16 of their bytes.  One 32-bit word holds 32 columns of
-// one row (bit i: column 2 i, bit 16 + i: column 2 i + 1); word (c / 32) * ld + row, so that a warp's 32 rows are 128
-// contiguous bytes.
+// the gradient back reads instead of the fp16 activations: 1/16 of their bytes.  Two 32-bit words hold what one lane has of
+// 32 rows x 64 columns (rows t / 4 + 8 i, columns 8 u + 2 (t % 4), + 1 of either half: bits 4 i + u and 16 + 4 i + u);
+// words ((c / 64) * ld + row / 32) * 64 + 2 t, so that a warp's are 256 contiguous bytes.  ld: blocks of 32 rows.
 #include "kernels.cuh"
 #include "tc5.cuh"
 
@@ -78,7 +79,7 @@ struct Row32 {
   }
 };
 
-// fp16 pairs after a ReLU (non-negative): bits i and 16 + i of the word for pair i's two values
+// 16 fp16 pairs after a ReLU (non-negative): bits i and 16 + i of the word for pair i's two values
 __device__ __forceinline__ uint32_t positive_bits(const uint32_t* h) {
   uint32_t w = 0;
 #pragma unroll
@@ -223,6 +224,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     auto put = [&](int pc, uint4 v) { *reinterpret_cast<uint4*>(stg + lane * 128 + ((pc ^ (lane & 7)) << 4)) = v; };
     // bias and activation on 32 accumulator columns from column h0 + x of the tile on, in place
     auto finish = [&](uint32_t (&a)[32], int x) {
+      if (p.bias) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float4 bv = *reinterpret_cast<const float4*>(s_bias + h0 + x + 4 * j);
@@ -230,6 +232,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         a[4 * j + 1] = __float_as_uint(__uint_as_float(a[4 * j + 1]) + bv.y);
         a[4 * j + 2] = __float_as_uint(__uint_as_float(a[4 * j + 2]) + bv.z);
         a[4 * j + 3] = __float_as_uint(__uint_as_float(a[4 * j + 3]) + bv.w);
+      }
       }
       if (p.relu == 1) {
 #pragma unroll
@@ -333,46 +336,58 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           else if ((st & 1) || left <= 32) emit(col - 32 * (st & 1), 2);
         }
       } else {
-        // ---- fp16, 64 columns at a time
-        uint32_t a[32], b[32], h[32];
-        if (c0 < n_end) {
-          tmem_ld32(tbase, a);
-          tmem_ld32(tbase + 32, b);
-        }
+        // ---- fp16 in fragments, 64 columns at a time: bias and activation on pairs of columns, rows leave by stmatrix
+        const int fc = 2 * (lane & 3), st_row = lane & 7, st_piece = lane >> 3;
+        uint32_t a[32], b[32];
+        if (c0 < n_end) tmem_ld_frags(tbase, a);
 #pragma unroll 1
         for (int st = 0; st < BN / 128; ++st) {
           const int col = c0 + 64 * st;
           if (col >= n_end) break;
-          uint32_t w0 = 0, w1 = 0;
-          if (p.bits_in && live) {
-            w0 = p.bits_in[(int64_t)(col >> 5) * p.bits_ld + row];
-            if (col + 32 < n_end) w1 = p.bits_in[(int64_t)((col >> 5) + 1) * p.bits_ld + row];
-          }
-          tmem_wait_ld();
-          finish(a, 64 * st);
+          uint2 bits = make_uint2(0, 0);                     // of this thread's pairs in the block
+          uint2* at_bits = nullptr;
+          if ((p.bits_in || p.bits_out) && m0 < p.M)
+            at_bits = const_cast<uint2*>(reinterpret_cast<const uint2*>(p.bits_in ? p.bits_in : p.bits_out)) +
+                      ((int64_t)(col >> 6) * p.bits_ld + (m0 >> 5)) * 32 + lane;
+          if (p.bits_in && at_bits) bits = *at_bits;
+          auto half = [&](const uint32_t (&r)[32], int hc) {   // 32 columns
+            uint32_t h[16];                                    // pair 4 i + u
 #pragma unroll
-          for (int j = 0; j < 16; ++j) h[j] = pack_half2(__uint_as_float(a[2 * j]), __uint_as_float(a[2 * j + 1]));
-          finish(b, 64 * st + 32);
+            for (int u = 0; u < 4; ++u) {
+              const uint64_t bv = *reinterpret_cast<const uint64_t*>(s_bias + h0 + 64 * st + 32 * hc + 8 * u + fc);
 #pragma unroll
-          for (int j = 0; j < 16; ++j) h[16 + j] = pack_half2(__uint_as_float(b[2 * j]), __uint_as_float(b[2 * j + 1]));
-          if (st + 1 < BN / 128 && col + 64 < n_end) {
-            tmem_ld32(tbase + 64 * (st + 1), a);
-            tmem_ld32(tbase + 64 * (st + 1) + 32, b);
-          }
-          if (p.bits_in) {
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              h[j] = keep_positive(h[j], w0, j);
-              h[16 + j] = keep_positive(h[16 + j], w1, j);
+              for (int i = 0; i < 4; ++i) {
+                uint64_t v = frag_pair(r, i, u);
+                if (p.bias) v = f2_add(v, bv);
+                float v0, v1;
+                f2_split(v, v0, v1);
+                if (p.relu == 1) {
+                  v0 = fmaxf(v0, 0.f);
+                  v1 = fmaxf(v1, 0.f);
+                } else if (p.relu == 2) {
+                  gelu_exact2(v0, v1);
+                }
+                h[4 * i + u] = pack_half2(v0, v1);
+              }
             }
-          }
-          if (p.bits_out && live) {
-            p.bits_out[(int64_t)(col >> 5) * p.bits_ld + row] = positive_bits(h);
-            if (col + 32 < n_end) p.bits_out[(int64_t)((col >> 5) + 1) * p.bits_ld + row] = positive_bits(h + 16);
-          }
-          wait_staging();
+            if (p.bits_in) {
 #pragma unroll
-          for (int j = 0; j < 8; ++j) put(j, make_uint4(h[4 * j], h[4 * j + 1], h[4 * j + 2], h[4 * j + 3]));
+              for (int j = 0; j < 16; ++j) h[j] = keep_positive(h[j], hc ? bits.y : bits.x, j);
+            } else if (p.bits_out) {
+              (hc ? bits.y : bits.x) = positive_bits(h);
+            }
+            if (hc == 0) wait_staging();
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              stmatrix_x4(smem_u32(stg) + (8 * i + st_row) * 128 + (((4 * hc + st_piece) ^ st_row) << 4), h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
+          };
+          tmem_wait_ld();
+          tmem_ld_frags(tbase + 64 * st + 32, b);
+          half(a, 0);
+          tmem_wait_ld();
+          if (st + 1 < BN / 128 && col + 64 < n_end) tmem_ld_frags(tbase + 64 * (st + 1), a);
+          half(b, 1);
+          if (p.bits_out && at_bits) *at_bits = bits;
           emit(col, 2);
         }
       }
@@ -405,7 +420,7 @@ bool linear_res_ok(const LinearArgs& p) {
   const int64_t tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
   return !p.a_mn && !p.mask && (!p.out_f32 || p.R || !dense_rows(p.cmap)) && !p.a_sums && p.k_splits <= 1 && p.K <= 4 * BK &&
          p.N % 32 == 0 && p.M <= 0x7ffffe00 && tiles >= 3ll * sm_count() && (p.N + res_cols(p.N) - 1) / res_cols(p.N) <= sm_count() / 2 &&
-         (!(p.bits_in || p.bits_out) || (!p.out_f32 && !p.R && p.N % 32 == 0)) && linear_tc5_ok(p);
+         (!(p.bits_in || p.bits_out) || (!p.out_f32 && !p.R && p.N % 64 == 0)) && linear_tc5_ok(p);
 }
 
 int linear_res(const LinearArgs& p, cudaStream_t stream) {

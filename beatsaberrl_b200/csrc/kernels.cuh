@@ -44,7 +44,7 @@ struct LinearArgs {
   // with ReLU, bits_in in the place of `mask`.
   uint32_t* bits_out = nullptr;
   const uint32_t* bits_in = nullptr;
-  int64_t bits_ld = 0;
+  int64_t bits_ld = 0;               // blocks of 32 rows
 };
 LinearArgs linear_args(const __half* A, int lda, const __half* W, int ldw, const float* bias,
                        void* C, int ldc, int out_f32, int relu, int64_t M, int N, int K);

@@ -228,6 +228,28 @@ __device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, uint32_t* r) {   
       : "r"(taddr)
       : "memory");
 }
+// 32 lanes x 32 columns: thread t's rows are t / 4 + 8 i
+__device__ __forceinline__ void tmem_ld_frags(uint32_t taddr, uint32_t (&r)[32]) {
+  tmem_ld_frag32(taddr, r);
+  tmem_ld_frag32(taddr + (16u << 16), r + 16);
+}
+__device__ __forceinline__ void tmem_ld_frag16(uint32_t taddr, uint32_t* r) {          // 16 lanes x 16 columns
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "r"(taddr)
+      : "memory");
+}
+// of tmem_ld_frags: the pair of row t / 4 + 8 i in columns 8 u + 2 (t % 4), + 1
+__device__ __forceinline__ uint64_t frag_pair(const uint32_t (&r)[32], int i, int u) {
+  const int at = 16 * (i >> 1) + 4 * u + 2 * (i & 1);
+  return f2_make(__uint_as_float(r[at]), __uint_as_float(r[at + 1]));
+}
+__device__ __forceinline__ uint32_t pack_f2(uint64_t v) {
+  float a, b;
+  f2_split(v, a, b);
+  return pack_half2(a, b);
+}
 // four 8 x 8 matrices of 16-bit elements (register i: matrix i) to the 16-byte rows whose addresses lanes 8 i .. 8 i + 7 give
 __device__ __forceinline__ void stmatrix_x4(uint32_t addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
   asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");

@@ -196,7 +196,7 @@ BwdLayout make_bwd(const Layout& l, int64_t B) {
   w.x1 = cv.take(R * d * 4);
   w.h2 = cv.take(R * d * 2);
   w.hid = cv.take(R * (int64_t)F * 2);
-  w.bits = cv.take(R * (int64_t)(round_up(F, 32) / 8));    // which hidden units were positive, one bit each
+  w.bits = cv.take(round_up(R, 32) * (F / 8));             // which hidden units were positive, one bit each
   w.gx = cv.take(R * d * 4);
   w.gx16 = cv.take(R * d * 2);     // fp16 copy of the stream gradient, written by the kernels that produce it
   w.g32 = cv.take(R * d * 4);
@@ -262,7 +262,7 @@ struct Bwd {
     r.w_mn = 1;
     if (relu_of && relu_of == bits_of) {
       r.bits_in = S<uint32_t>(w.bits);
-      r.bits_ld = M;
+      r.bits_ld = (M + 31) / 32;
     } else {
       r.mask = relu_of;
       r.ldm = (int)ld_relu;
@@ -295,7 +295,7 @@ struct Bwd {
     LinearArgs f = linear_args(a, lda, c.W(m), m.pitch, c.Bv(m), out, N, 0, 1, M, N, K);
     LinearArgs b = linear_args(a, Kb, c.W(m), N, nullptr, out, N, 0, 0, M, N, Kb);
     f.bits_out = S<uint32_t>(w.bits);
-    f.bits_ld = M;
+    f.bits_ld = (M + 31) / 32;
     b.w_mn = 1;
     b.bits_in = f.bits_out;
     const bool bits = linear_rows_ok(f) && linear_res_ok(f) && linear_res_ok(b);
