@@ -9,12 +9,19 @@
 // problem of one (env, head) pair -- at most 32 x 64 values per matrix -- lives in the warp's shared-memory
 // tile; the five products run on m16n8k16 MMAs with fp32 accumulation, P and dS rounded to fp16 as operands.
 #include "kernels.cuh"
-#include "attend.cuh"
+#include "tc5.cuh"
 
 namespace bsrl {
 namespace {
 
-constexpr int kWarps = 4;
+// Warps of a block, and tiles per warp: with two, the next pair's operands are on their way while this one's are worked on.
+// Heads of 32 have the shared memory for that with 14 (16 query rows: 18) warps per SM: 378 -> 353 us and 257 -> 227 per 16,384
+// environments of 256 (4 x 3 and 2 x 6 warps: 437 and 399); wider heads are faster with more warps and one tile each
+// (2,049 environments of 4 heads of 48: 43 us against 52).
+template <int DH, int MT>
+constexpr int warps_of() { return DH == 32 ? (MT == 2 ? 7 : 6) : 4; }
+template <int DH>
+constexpr int tiles_of() { return DH == 32 ? 2 : 1; }
 constexpr int kKeys = 32;      // 29 keys padded to four 8-key MMA tiles
 
 // the 8 x 8 matrix of fp16 pairs that the warp holds (row lane / 4, columns 2 (lane % 4)..) -> its transpose, in the same layout
@@ -24,53 +31,66 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
   return r;
 }
 
+// Byte offset of 16-byte piece p of row r of a tile of dense rows: the 8 rows of an ldmatrix hit 8 different 16-byte banks,
+// and so do 8 consecutive pieces (with rows padded by 16 bytes instead, those took two turns of the pipe).
+template <int DH>
+__device__ __forceinline__ uint32_t tile_at(int r, int p) {
+  return r * (DH * 2) + ((DH == 32 ? p ^ ((r >> 1) & 3) : DH == 48 ? p ^ ((r >> 2) & 1) : p ^ (r & 7)) << 4);
+}
+
 // One warp per (env, head); MT = 16-row query tiles (2: all 29 queries, 1: the lead rows or the critic's one).
 // Five small products on m16n8k16 MMAs: S = q k^T and dP = dO v^T (A rows = queries, B rows = keys);
 // dQ = dS k (A = dS from the accumulator registers, B = k with the keys as the reduction dimension);
 // dV = P^T dO and dK = dS^T q (A = P / dS transposed in registers, 8 x 8 at a time; B = dO / q with the queries as the
 // reduction dimension).  The operands arrive by cp.async, the results leave from the rows of the operands they replace, 16
-// bytes per lane.  Bound by latency: what sets its speed is the warps an SM can hold, that is the bytes of a warp's tile.
+// bytes per lane.  Bound by the turns of the shared-memory pipe (654 of the 909 cycles per pair of 29 queries x 32 before
+// the swizzled rows; every fragment is fetched once now, for both query or both key tiles).  16,384 environments of 8 heads of
+// 32, us, before / now (at copy speed): 29 queries 407 / 350 (260), 5 queries 276 / 226 (199), 1 query 272 / 224 (152).
 template <int DH, int MT>
-__global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __restrict__ qkv, int ld, const float* __restrict__ key_bias,
+__global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(const __half* __restrict__ qkv, int ld, const float* __restrict__ key_bias,
                                                                int64_t n_pairs, int d, int n_heads, int q_first, int n_q,
                                                                const __half* __restrict__ g_out, int ldgo, __half* __restrict__ gq,
                                                                int ldq, __half* __restrict__ gk, int ldk, __half* __restrict__ gv,
                                                                int ldv, int wide) {
   pdl_begin();
-  constexpr int LDS = DH + 8;                         // padded row (halves): ldmatrix rows land in distinct banks
-  constexpr int CH = DH / 8;
+  constexpr int CH = DH / 8, ROW = DH * 2;
   constexpr int QR = 16 * MT;                         // staged query rows
-  constexpr int PER_WARP = (2 * QR + 2 * kKeys) * LDS * 2;
-  extern __shared__ __align__(16) uint8_t smem[];
+  constexpr int TILE = (2 * QR + 2 * kKeys) * ROW, TILES = tiles_of<DH>(), kWarps = warps_of<DH, MT>();
+  extern __shared__ __align__(128) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __half* sq = reinterpret_cast<__half*>(smem + (size_t)warp * PER_WARP);
-  __half* sg = sq + QR * LDS;
-  __half* sk = sg + QR * LDS;
-  __half* sv = sk + kKeys * LDS;
-  const uint32_t sq_u = smem_u32(sq), sg_u = smem_u32(sg), sk_u = smem_u32(sk), sv_u = smem_u32(sv);
+  uint8_t* tile = smem + (size_t)warp * (TILES * TILE);
   const float scale = rsqrtf((float)DH);
-  const int g = lane >> 2, tig = lane & 3;
+  const int tig = lane & 3;
+  // rows (and 8-column halves) of ldmatrix / stmatrix x4: 16 rows x 16 columns as rows 0..7, 8..15 of columns 0..7, then 8..15 ...
+  const int ra = lane & 15, ca = lane >> 4;
+  // ... and 16 keys x 16 columns as columns 0..7, 8..15 of rows 0..7, then of rows 8..15
+  const int rb = (lane & 7) + ((lane >> 4) << 3), cb = (lane >> 3) & 1;
   const int64_t warps = (int64_t)gridDim.x * kWarps;
-  for (int64_t pair = (int64_t)blockIdx.x * kWarps + warp; pair < n_pairs; pair += warps) {
-    int head;
-    const int64_t env = div_index(pair, n_heads, &head);
-    const __half* base = qkv + env * kT * (int64_t)ld + head * DH;
-    __syncwarp();
-    // stage q, dO (query rows) and k, v (key rows); rows past the live range are zero
-    for (int c = lane; c < kKeys * CH; c += 32) {
-      const int row = c / CH, ch = c % CH;
-      const bool live = row < kT, asks = row < n_q;
-      const __half* r = base + (int64_t)(live ? row : 0) * ld + ch * 8;
-      const uint32_t at = (row * LDS + ch * 8) * 2;
-      cp_async16(sk_u + at, r + d, live);
-      cp_async16(sv_u + at, r + 2 * d, live);
-      if (row < QR) {
-        cp_async16(sq_u + at, base + (int64_t)(asks ? q_first + row : 0) * ld + ch * 8, asks);
-        cp_async16(sg_u + at, g_out + (env * n_q + (asks ? row : 0)) * (int64_t)ldgo + head * DH + ch * 8, asks);
+  // q, dO (query rows) and k, v (key rows) of a pair into the tile at `at0`; rows past the live range are zero
+  auto request = [&](int64_t pair, uint32_t at0) {
+    if (pair < n_pairs) {
+      int head;
+      const int64_t env = div_index(pair, n_heads, &head);
+      const __half* base = qkv + env * kT * (int64_t)ld + head * DH;
+      for (int c = lane; c < kKeys * CH; c += 32) {
+        const int row = c / CH, ch = c % CH;
+        const bool live = row < kT, asks = row < n_q;
+        const __half* r = base + (int64_t)(live ? row : 0) * ld + ch * 8;
+        const uint32_t at = at0 + tile_at<DH>(row, ch);
+        cp_async16(at + 2 * QR * ROW, r + d, live);
+        cp_async16(at + (2 * QR + kKeys) * ROW, r + 2 * d, live);
+        if (row < QR) {
+          cp_async16(at, base + (int64_t)(asks ? q_first + row : 0) * ld + ch * 8, asks);
+          cp_async16(at + QR * ROW, g_out + (env * n_q + (asks ? row : 0)) * (int64_t)ldgo + head * DH + ch * 8, asks);
+        }
       }
     }
     cp_async_commit();
-    float kb[4][2];
+  };
+  auto bias_of = [&](int64_t pair, float (&kb)[4][2]) {
+    if (pair >= n_pairs) return;
+    int head;
+    const int64_t env = div_index(pair, n_heads, &head);
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
@@ -78,47 +98,74 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
         const int key = nt * 8 + tig * 2 + e;
         kb[nt][e] = key < kT ? key_bias[env * kT + key] : -INFINITY;
       }
-    cp_async_wait<0>();
+  };
+  const int64_t first = (int64_t)blockIdx.x * kWarps + warp;
+  float kb[4][2];
+  if (TILES == 2) request(first, smem_u32(tile));
+  int cur = 0;
+  for (int64_t pair = first; pair < n_pairs; pair += warps) {
+    int head;
+    const int64_t env = div_index(pair, n_heads, &head);
+    uint8_t* sq = tile + cur * TILE;
+    uint8_t* sk = sq + 2 * QR * ROW;
+    uint8_t* sv = sk + kKeys * ROW;
+    const uint32_t sq_u = smem_u32(sq), sg_u = sq_u + QR * ROW, sk_u = smem_u32(sk), sv_u = smem_u32(sv);
+    __syncwarp();
+    bias_of(pair, kb);
+    if (TILES == 2) {
+      cur ^= 1;
+      request(pair + warps, smem_u32(tile + cur * TILE));
+      cp_async_wait<1>();
+    } else {
+      request(pair, sq_u);
+      cp_async_wait<0>();
+    }
     __syncwarp();
 
-    uint32_t tp[MT][2][4], td[MT][2][4];                // P^T and dS^T, A fragments of 16 keys x 16 queries
-    uint32_t oq16[MT][DH / 8][2];                       // dQ
-
+    // ---- S = q k^T and dP = dO v^T
+    float s[MT][4][4], dp[MT][4][4];
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      // ---- S = q k^T and dP = dO v^T for this query tile
-      float s[4][4], dp[4][4];
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[nt][e] = dp[nt][e] = 0.f;
+        for (int e = 0; e < 4; ++e) s[mt][nt][e] = dp[mt][nt][e] = 0.f;
 #pragma unroll
-      for (int ks = 0; ks < DH / 16; ++ks) {
-        uint32_t a[4], ag[4];
-        const uint32_t aoff = ((mt * 16 + (lane & 15)) * LDS + ks * 16 + (lane >> 4) * 8) * 2;
-        ldmatrix_x4(a, sq_u + aoff);
-        ldmatrix_x4(ag, sg_u + aoff);
+    for (int ks = 0; ks < DH / 16; ++ks) {
+      uint32_t a[MT][4], ag[MT][4];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          uint32_t b[4], bv[4];
-          const int row = j * 16 + (lane & 7) + ((lane >> 4) << 3);
-          const uint32_t boff = (row * LDS + ks * 16 + ((lane >> 3) & 1) * 8) * 2;
-          ldmatrix_x4(b, sk_u + boff);
-          ldmatrix_x4(bv, sv_u + boff);
-          mma_f16(s[2 * j], a, b[0], b[1]);
-          mma_f16(s[2 * j + 1], a, b[2], b[3]);
-          mma_f16(dp[2 * j], ag, bv[0], bv[1]);
-          mma_f16(dp[2 * j + 1], ag, bv[2], bv[3]);
+      for (int mt = 0; mt < MT; ++mt) {
+        const uint32_t at = tile_at<DH>(mt * 16 + ra, ks * 2 + ca);
+        ldmatrix_x4(a[mt], sq_u + at);
+        ldmatrix_x4(ag[mt], sg_u + at);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        uint32_t b[4], bv[4];
+        const uint32_t at = tile_at<DH>(j * 16 + rb, ks * 2 + cb);
+        ldmatrix_x4(b, sk_u + at);
+        ldmatrix_x4(bv, sv_u + at);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          mma_f16(s[mt][2 * j], a[mt], b[0], b[1]);
+          mma_f16(s[mt][2 * j + 1], a[mt], b[2], b[3]);
+          mma_f16(dp[mt][2 * j], ag[mt], bv[0], bv[1]);
+          mma_f16(dp[mt][2 * j + 1], ag[mt], bv[2], bv[3]);
         }
       }
+    }
+    uint32_t tp[MT][2][4], td[MT][2][4];                // P^T and dS^T, A fragments of 16 keys x 16 queries
+    uint32_t da[MT][2][4];                              // dS, A fragments of 16 queries x 16 keys
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
       // ---- P = softmax(S / sqrt(dh) + bias), dS = P (dP - rowsum(P dP)) / sqrt(dh); rows g (e = 0, 1) and g + 8 (e = 2, 3)
       float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          s[nt][e] = s[nt][e] * scale + kb[nt][e & 1];
-          mx[e >> 1] = fmaxf(mx[e >> 1], s[nt][e]);
+          s[mt][nt][e] = s[mt][nt][e] * scale + kb[nt][e & 1];
+          mx[e >> 1] = fmaxf(mx[e >> 1], s[mt][nt][e]);
         }
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -130,8 +177,8 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          s[nt][e] = expf(s[nt][e] - mx[e >> 1]);
-          sum[e >> 1] += s[nt][e];
+          s[mt][nt][e] = expf(s[mt][nt][e] - mx[e >> 1]);
+          sum[e >> 1] += s[mt][nt][e];
         }
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -144,8 +191,8 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          s[nt][e] *= sum[e >> 1];                       // P
-          dot[e >> 1] += s[nt][e] * dp[nt][e];
+          s[mt][nt][e] *= sum[e >> 1];                   // P
+          dot[e >> 1] += s[mt][nt][e] * dp[mt][nt][e];
         }
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -155,96 +202,102 @@ __global__ void __launch_bounds__(kWarps * 32) attn_bwd_kernel(const __half* __r
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) dp[nt][e] = s[nt][e] * (dp[nt][e] - dot[e >> 1]) * scale;   // dS
-      // 8 x 8 blocks (8 queries x 8 keys) transposed across the warp
+        for (int e = 0; e < 4; ++e) dp[mt][nt][e] = s[mt][nt][e] * (dp[mt][nt][e] - dot[e >> 1]) * scale;   // dS
+      // the accumulators as A fragments (as P feeds P v in the forward), and 8 x 8 blocks (8 queries x 8 keys) transposed
 #pragma unroll
       for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          tp[mt][nt >> 1][(nt & 1) + 2 * r] = transpose8x8(pack_half2(s[nt][2 * r], s[nt][2 * r + 1]));
-          td[mt][nt >> 1][(nt & 1) + 2 * r] = transpose8x8(pack_half2(dp[nt][2 * r], dp[nt][2 * r + 1]));
+          const uint32_t ds = pack_half2(dp[mt][nt][2 * r], dp[mt][nt][2 * r + 1]);
+          da[mt][nt >> 1][2 * (nt & 1) + r] = ds;
+          td[mt][nt >> 1][(nt & 1) + 2 * r] = transpose8x8(ds);
+          tp[mt][nt >> 1][(nt & 1) + 2 * r] = transpose8x8(pack_half2(s[mt][nt][2 * r], s[mt][nt][2 * r + 1]));
         }
-      // ---- dQ = dS k: A = dS from the accumulator registers (as P feeds P v in the forward)
-      uint32_t da[2][4];
+    }
+    // ---- dQ = dS k
+    uint32_t oq16[MT][DH / 8][2];
+#pragma unroll
+    for (int j = 0; j < DH / 16; ++j) {
+      float oq[MT][2][4];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int e = 0; e < 8; ++e) oq[mt][e >> 2][e & 3] = 0.f;
 #pragma unroll
       for (int ks = 0; ks < 2; ++ks) {
-        da[ks][0] = pack_half2(dp[2 * ks][0], dp[2 * ks][1]);
-        da[ks][1] = pack_half2(dp[2 * ks][2], dp[2 * ks][3]);
-        da[ks][2] = pack_half2(dp[2 * ks + 1][0], dp[2 * ks + 1][1]);
-        da[ks][3] = pack_half2(dp[2 * ks + 1][2], dp[2 * ks + 1][3]);
-      }
-      float oq[DH / 8][4];
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, sk_u + tile_at<DH>(ks * 16 + ra, j * 2 + ca));
 #pragma unroll
-      for (int nt = 0; nt < DH / 8; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) oq[nt][e] = 0.f;
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-        for (int j = 0; j < DH / 16; ++j) {
-          uint32_t b[4];
-          const int row = ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-          ldmatrix_x4_trans(b, sk_u + (row * LDS + j * 16 + (lane >> 4) * 8) * 2);
-          mma_f16(oq[2 * j], da[ks], b[0], b[1]);
-          mma_f16(oq[2 * j + 1], da[ks], b[2], b[3]);
+        for (int mt = 0; mt < MT; ++mt) {
+          mma_f16(oq[mt][0], da[mt][ks], b[0], b[1]);
+          mma_f16(oq[mt][1], da[mt][ks], b[2], b[3]);
         }
+      }
 #pragma unroll
-      for (int nt = 0; nt < DH / 8; ++nt)
+      for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int r = 0; r < 2; ++r) oq16[mt][nt][r] = pack_half2(oq[nt][r * 2], oq[nt][r * 2 + 1]);
+        for (int e = 0; e < 4; ++e) oq16[mt][2 * j + (e >> 1)][e & 1] = pack_half2(oq[mt][e >> 1][2 * (e & 1)], oq[mt][e >> 1][2 * (e & 1) + 1]);
     }
     __syncwarp();                                       // k and v have been read: dK and dV take their places
-    // ---- dV = P^T dO and dK = dS^T q: key tiles as rows, the queries as the reduction dimension
+    // ---- dV = P^T dO and dK = dS^T q: key tiles as rows, the queries as the reduction dimension, 16 columns at a time
 #pragma unroll
-    for (int kt = 0; kt < 2; ++kt) {
-      float ov[DH / 8][4], ok[DH / 8][4];
+    for (int j = 0; j < DH / 16; ++j) {
+      float ov[2][2][4], ok[2][2][4];
 #pragma unroll
-      for (int nt = 0; nt < DH / 8; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) ov[nt][e] = ok[nt][e] = 0.f;
+      for (int e = 0; e < 16; ++e) ov[e >> 3][(e >> 2) & 1][e & 3] = ok[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
 #pragma unroll
       for (int qs = 0; qs < MT; ++qs) {                 // 16 queries per step
+        uint32_t b[4], bq[4];
+        const uint32_t at = tile_at<DH>(qs * 16 + ra, j * 2 + ca);
+        ldmatrix_x4_trans(b, sg_u + at);
+        ldmatrix_x4_trans(bq, sq_u + at);
 #pragma unroll
-        for (int j = 0; j < DH / 16; ++j) {
-          uint32_t b[4], bq[4];
-          const int row = qs * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-          const uint32_t boff = (row * LDS + j * 16 + (lane >> 4) * 8) * 2;
-          ldmatrix_x4_trans(b, sg_u + boff);
-          ldmatrix_x4_trans(bq, sq_u + boff);
-          mma_f16(ov[2 * j], tp[qs][kt], b[0], b[1]);
-          mma_f16(ov[2 * j + 1], tp[qs][kt], b[2], b[3]);
-          mma_f16(ok[2 * j], td[qs][kt], bq[0], bq[1]);
-          mma_f16(ok[2 * j + 1], td[qs][kt], bq[2], bq[3]);
+        for (int kt = 0; kt < 2; ++kt) {
+          mma_f16(ov[kt][0], tp[qs][kt], b[0], b[1]);
+          mma_f16(ov[kt][1], tp[qs][kt], b[2], b[3]);
+          mma_f16(ok[kt][0], td[qs][kt], bq[0], bq[1]);
+          mma_f16(ok[kt][1], td[qs][kt], bq[2], bq[3]);
         }
       }
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const int at = (kt * 16 + g + r * 8) * LDS + tig * 2;
-#pragma unroll
-        for (int nt = 0; nt < DH / 8; ++nt) {
-          *reinterpret_cast<uint32_t*>(sv + at + nt * 8) = pack_half2(ov[nt][r * 2], ov[nt][r * 2 + 1]);
-          *reinterpret_cast<uint32_t*>(sk + at + nt * 8) = pack_half2(ok[nt][r * 2], ok[nt][r * 2 + 1]);
-        }
+      for (int kt = 0; kt < 2; ++kt) {
+        const uint32_t at = tile_at<DH>(kt * 16 + ra, j * 2 + ca);
+        tc5::stmatrix_x4(sv_u + at, pack_half2(ov[kt][0][0], ov[kt][0][1]), pack_half2(ov[kt][0][2], ov[kt][0][3]),
+                         pack_half2(ov[kt][1][0], ov[kt][1][1]), pack_half2(ov[kt][1][2], ov[kt][1][3]));
+        tc5::stmatrix_x4(sk_u + at, pack_half2(ok[kt][0][0], ok[kt][0][1]), pack_half2(ok[kt][0][2], ok[kt][0][3]),
+                         pack_half2(ok[kt][1][0], ok[kt][1][1]), pack_half2(ok[kt][1][2], ok[kt][1][3]));
       }
     }
     __syncwarp();                                       // q has been read too
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-      for (int r = 0; r < 2; ++r)
-#pragma unroll
-        for (int nt = 0; nt < DH / 8; ++nt) *reinterpret_cast<uint32_t*>(sq + (mt * 16 + g + r * 8) * LDS + nt * 8 + tig * 2) = oq16[mt][nt][r];
+      for (int j = 0; j < DH / 16; ++j)
+        tc5::stmatrix_x4(sq_u + tile_at<DH>(mt * 16 + ra, j * 2 + ca), oq16[mt][2 * j][0], oq16[mt][2 * j][1], oq16[mt][2 * j + 1][0], oq16[mt][2 * j + 1][1]);
     __syncwarp();
-    copy_rows_out<DH, LDS>(sv, kT, gv + env * kT * (int64_t)ldv + head * DH, ldv, wide, lane);
-    copy_rows_out<DH, LDS>(sk, kT, gk + env * kT * (int64_t)ldk + head * DH, ldk, wide, lane);
-    copy_rows_out<DH, LDS>(sq, n_q, gq + env * n_q * (int64_t)ldq + head * DH, ldq, wide, lane);
+    auto out = [&](const uint8_t* from, int rows, __half* dst, int64_t ldd) {
+      for (int c = lane; c < rows * CH; c += 32) {
+        const int row = c / CH, ch = c % CH;
+        const uint4 v = *reinterpret_cast<const uint4*>(from + tile_at<DH>(row, ch));
+        __half* to = dst + row * ldd + ch * 8;
+        if (wide) {
+          *reinterpret_cast<uint4*>(to) = v;
+        } else {
+          uint32_t* w = reinterpret_cast<uint32_t*>(to);
+          w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+        }
+      }
+    };
+    out(sv, kT, gv + env * kT * (int64_t)ldv + head * DH, ldv);
+    out(sk, kT, gk + env * kT * (int64_t)ldk + head * DH, ldk);
+    out(sq, n_q, gq + env * n_q * (int64_t)ldq + head * DH, ldq);
   }
 }
 
 template <int DH, int MT>
 int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int d, int n_heads, int q_first, int n_q,
            const __half* g_out, int ldgo, __half* gq, int ldq, __half* gk, int ldk, __half* gv, int ldv, cudaStream_t stream) {
-  constexpr int smem = kWarps * (2 * 16 * MT + 2 * kKeys) * (DH + 8) * 2;
+  constexpr int kWarps = warps_of<DH, MT>(), smem = kWarps * tiles_of<DH>() * (2 * 16 * MT + 2 * kKeys) * DH * 2;
   static DeviceOnce once;
   int rc = once.run("attn_bwd_kernel set-up", [] {
     return cudaFuncSetAttribute(attn_bwd_kernel<DH, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -253,7 +306,8 @@ int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int
   const int wide = aligned16(gq) && aligned16(gk) && aligned16(gv) && ldq % 8 == 0 && ldk % 8 == 0 && ldv % 8 == 0;
   const int64_t pairs = n_envs * n_heads;
   int64_t blocks = (pairs + kWarps - 1) / kWarps;
-  const int64_t cap = (int64_t)sm_count() * 8;
+  // several short waves: blocks that stay for all of their pairs stream in step, 435 us where 8 to 24 per SM take 350
+  const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
   launch_kernel(attn_bwd_kernel<DH, MT>, (unsigned)blocks, kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d, n_heads, q_first, n_q, g_out,
                                                                           ldgo, gq, ldq, gk, ldk, gv, ldv, wide);
