@@ -15,6 +15,13 @@ __device__ __forceinline__ float rcp_approx(float x) {
   return y;
 }
 
+// Byte offset of 16-byte piece p of row r of a tile of dense rows: the 8 rows of an ldmatrix hit 8 different 16-byte banks,
+// and so do 8 consecutive pieces (with rows padded by 16 bytes instead, those took two turns of the pipe).
+template <int DH>
+__device__ __forceinline__ uint32_t tile_at(int r, int p) {
+  return r * (DH * 2) + ((DH == 32 ? p ^ ((r >> 1) & 3) : DH == 48 ? p ^ ((r >> 2) & 1) : p ^ (r & 7)) << 4);
+}
+
 // Byte address of 16-byte piece `piece` of row `row` of a section (q, k or v): rows LDQ bytes apart, or, for LDQ = 128, a
 // 128-byte-swizzled tile (piece p of row r at ((p ^ (r & 7)) << 4)) that starts on a 1024-byte boundary
 template <int LDQ>
@@ -161,25 +168,6 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
           *reinterpret_cast<uint32_t*>(orow + nt * 8) = pack_half2(o[mt][nt][r * 2], o[mt][nt][r * 2 + 1]);
       }
     }
-}
-
-// One row block of a warp's shared-memory tile (rows LDS halves apart, DH used) -> rows of `out`, 16 bytes per lane: a row's
-// sectors are written once and whole.  (Straight from the accumulator fragments a store covers 16 bytes of each of 8 rows.)
-// wide: out and ldo allow 16-byte stores
-template <int DH, int LDS>
-__device__ __forceinline__ void copy_rows_out(const __half* s, int n_rows, __half* out, int64_t ldo, bool wide, int lane) {
-  constexpr int CH = DH / 8;
-  for (int c = lane; c < n_rows * CH; c += 32) {
-    const int row = c / CH, ch = c % CH;
-    const uint4 v = *reinterpret_cast<const uint4*>(s + row * LDS + ch * 8);
-    __half* o = out + row * ldo + ch * 8;
-    if (wide) {
-      *reinterpret_cast<uint4*>(o) = v;
-    } else {
-      uint32_t* o32 = reinterpret_cast<uint32_t*>(o);
-      o32[0] = v.x; o32[1] = v.y; o32[2] = v.z; o32[3] = v.w;
-    }
-  }
 }
 
 // One query row of an env on the CUDA cores (lane = key for the scores, lane = output column for the weighted sum):

@@ -14,9 +14,13 @@
 // 32, 48 or 64, any head count.
 #include "kernels.cuh"
 #include "attend.cuh"
+#include "tc5.cuh"
 
 namespace bsrl {
 namespace {
+// Rows of the operand tile are dense and swizzled (tile_at): padded by 16 bytes they took two turns of the shared-memory pipe
+// per 16-byte pass.  16,384 environments of 8 heads of 32, us, before / now (at copy speed): 29 queries 203 / 182 (149), 5
+// queries 135 / 111, 1 query 128 / 108 (76).  Two tiles per warp, loads ahead, as in the backward: 192, 120 and 119.
 // KG: groups of 32 keys (tokens padded to 32 KG rows: two 16-row MMA tiles / four 8-key tiles per group);
 // WARPS: warps per block, fewer where the per-warp tile is large
 template <int DH, int KG, int WARPS>
@@ -27,16 +31,14 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
                                                            __half* __restrict__ out, int ldo) {
   pdl_begin();
   constexpr int kWarps = WARPS, kRows = 32 * KG, NT = 4 * KG;   // NT: 8-key tiles
-  constexpr int LDS = DH + 8;          // padded row (halfs): ldmatrix rows land in distinct banks
-  constexpr int CH = DH / 8;           // 16-byte chunks per row
-  extern __shared__ __align__(16) uint8_t smem[];
+  constexpr int CH = DH / 8, SECTION = kRows * DH * 2;          // 16-byte chunks per row; bytes of q, of k, of v
+  extern __shared__ __align__(128) uint8_t smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  __half* sq = reinterpret_cast<__half*>(smem) + (size_t)warp * 3 * kRows * LDS;
-  __half* sk = sq + kRows * LDS;
-  __half* sv = sk + kRows * LDS;
-  const uint32_t sq_u = smem_u32(sq), sk_u = smem_u32(sk), sv_u = smem_u32(sv);
+  uint8_t* sq = smem + (size_t)warp * (3 * SECTION);
+  const uint32_t sq_u = smem_u32(sq), sk_u = sq_u + SECTION, sv_u = sk_u + SECTION;
   const float scale = rsqrtf(static_cast<float>(DH));
-  const int g = lane >> 2, tig = lane & 3;
+  const int tig = lane & 3;
+  const int ra = lane & 15, ca = lane >> 4, rb = (lane & 7) + ((lane >> 4) << 3), cb = (lane >> 3) & 1;   // ldmatrix rows and halves
   const int m_tiles = (n_q + 15) >> 4;
 
   for (int64_t pair = (int64_t)blockIdx.x * kWarps + warp; pair < n_pairs;
@@ -50,7 +52,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
       const int row = c / CH, ch = c % CH;
       const bool live = row < tokens, asks = row < n_q;
       const __half* r = base + (int64_t)(live ? row : 0) * ld + ch * 8;
-      const uint32_t at = (row * LDS + ch * 8) * 2;
+      const uint32_t at = tile_at<DH>(row, ch);
       cp_async16(sq_u + at, base + (int64_t)(asks ? q_first + row : 0) * ld + ch * 8, asks);
       cp_async16(sk_u + at, r + d, live);
       cp_async16(sv_u + at, r + 2 * d, live);
@@ -77,12 +79,11 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
 #pragma unroll
       for (int ks = 0; ks < DH / 16; ++ks) {
         uint32_t a[4];
-        ldmatrix_x4(a, sq_u + ((mt * 16 + (lane & 15)) * LDS + ks * 16 + (lane >> 4) * 8) * 2);
+        ldmatrix_x4(a, sq_u + tile_at<DH>(mt * 16 + ra, ks * 2 + ca));
 #pragma unroll
         for (int j = 0; j < 2 * KG; ++j) {
           uint32_t b[4];
-          int row = j * 16 + (lane & 7) + ((lane >> 4) << 3);
-          ldmatrix_x4(b, sk_u + (row * LDS + ks * 16 + ((lane >> 3) & 1) * 8) * 2);
+          ldmatrix_x4(b, sk_u + tile_at<DH>(j * 16 + rb, ks * 2 + cb));
           mma_f16(s[2 * j], a, b[0], b[1]);
           mma_f16(s[2 * j + 1], a, b[2], b[3]);
         }
@@ -134,22 +135,23 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
 #pragma unroll
         for (int j = 0; j < DH / 16; ++j) {
           uint32_t b[4];
-          int row = ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-          ldmatrix_x4_trans(b, sv_u + (row * LDS + j * 16 + (lane >> 4) * 8) * 2);
+          ldmatrix_x4_trans(b, sv_u + tile_at<DH>(ks * 16 + ra, j * 2 + ca));
           mma_f16(o[2 * j], pa[ks], b[0], b[1]);
           mma_f16(o[2 * j + 1], pa[ks], b[2], b[3]);
         }
       }
       // the output takes the place of the query rows it came from
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        __half* orow = sq + (mt * 16 + g + r * 8) * LDS + tig * 2;
-#pragma unroll
-        for (int nt = 0; nt < DH / 8; ++nt) *reinterpret_cast<uint32_t*>(orow + nt * 8) = pack_half2(o[nt][r * 2], o[nt][r * 2 + 1]);
-      }
+      for (int j = 0; j < DH / 16; ++j)
+        tc5::stmatrix_x4(sq_u + tile_at<DH>(mt * 16 + ra, j * 2 + ca), pack_half2(o[2 * j][0], o[2 * j][1]), pack_half2(o[2 * j][2], o[2 * j][3]),
+                         pack_half2(o[2 * j + 1][0], o[2 * j + 1][1]), pack_half2(o[2 * j + 1][2], o[2 * j + 1][3]));
     }
     __syncwarp();
-    copy_rows_out<DH, LDS>(sq, n_q, out + env * n_q * (int64_t)ldo + head * DH, ldo, true, lane);
+    __half* to = out + env * n_q * (int64_t)ldo + head * DH;
+    for (int c = lane; c < n_q * CH; c += 32) {
+      const int row = c / CH, ch = c % CH;
+      *reinterpret_cast<uint4*>(to + row * (int64_t)ldo + ch * 8) = *reinterpret_cast<const uint4*>(sq + tile_at<DH>(row, ch));
+    }
   }
 }
 
@@ -163,35 +165,46 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
 // n_q = tokens (every row) or 1 (the body row only: the last block's readout).  Same arithmetic as
 // attn29_kernel: fp32 scores and softmax, masked keys exactly 0, probabilities rounded to fp16 only where
 // they enter an MMA.
-// TEAM: warps per (env, head) -- two where the pair's tile is so large (28 KB at 64 tokens x 64) that one warp each left two
-// per scheduler; each takes half of the object query rows and of the body row's output columns.
+// TEAM: warps per (env, head) -- two where the pair's tile is so large (24 KB at 64 tokens x 64) that one warp each left two
+// per scheduler; each takes half of the object query rows and, for the body row, half of the object keys.
+// Bound by the turns of the shared-memory pipe and by what is done per lane for the body token; so its scores -- q_0 k_j and
+// q_i k_0 -- are products on the tensor cores too (q_0 as all 16 rows of a tile, k_0 as one key of a tile of eight), a
+// K or V fragment serves both query tiles of a warp, and rows are dense and swizzled.
+// One B200, us, before / now (at copy speed): 4,095 environments of 65 tokens, 8 heads of 64: 295 / 244 (167), the body row only
+// 121 / 92 (84); 4,096 of 33 tokens, 8 heads of 32: 78 / 72 (42); of 17, 4 heads of 32: 25 / 19 (11).
+template <int DH, int NOBJ, int TEAM>
+struct BodyTile {
+  static constexpr int ROW = DH * 2, SECTION = NOBJ * ROW;
+  // q, k, v of the object tokens; then q0 | k0 | v0, a zero piece, and what a team's warps exchange (max, sum, DH outputs)
+  static constexpr int EXTRA = 3 * ROW + 16, SWAP = EXTRA, BYTES = 3 * SECTION + (EXTRA + (4 + DH) * 4 + 127) / 128 * 128;
+};
 template <int DH, int NOBJ, int WARPS, int TEAM>
 __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __restrict__ qkv, int ld,
                                                               const float* __restrict__ key_bias, int64_t n_pairs,
                                                               int d, int n_heads, int n_q, __half* __restrict__ out, int ldo) {
   pdl_begin();
-  constexpr int T = NOBJ + 1, NT = NOBJ / 8, KS = NOBJ / 16, MT = NOBJ / 16;
-  constexpr int LDS = DH + 8, CH = DH / 8;
-  constexpr int PER = (NOBJ + 31) / 32;              // object rows per lane in the lane-per-row passes
-  static_assert(TEAM == 1 || (TEAM == 2 && NOBJ == 64), "a team's warps take 32 object rows each");
-  extern __shared__ __align__(16) uint8_t smem[];
+  using Tile = BodyTile<DH, NOBJ, TEAM>;
+  constexpr int T = NOBJ + 1, NT = NOBJ / 8, KS = NOBJ / 16, MT = NOBJ / 16 / TEAM, CH = DH / 8, ROW = Tile::ROW;
+  constexpr int KEYS = NOBJ / TEAM, CPL = DH / 32;   // object keys of this warp for the body row; output columns per lane
+  static_assert(KEYS <= 32 && (TEAM == 1 || TEAM == 2), "one key per lane");
+  extern __shared__ __align__(128) uint8_t smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // per team: q, k, v of the object tokens (NOBJ rows each), then q0 | k0 | v0, then the extra score column
-  constexpr int kWarpHalfs = 3 * NOBJ * LDS + 3 * LDS;
   const int team = warp / TEAM, part = warp % TEAM, tlane = part * 32 + lane;
-  __half* sq = reinterpret_cast<__half*>(smem) + (size_t)team * kWarpHalfs;
-  __half* sk = sq + NOBJ * LDS;
-  __half* sv = sk + NOBJ * LDS;
-  __half* s0 = sv + NOBJ * LDS;                      // q0 at [0, DH), k0 at [LDS, ..), v0 at [2 LDS, ..)
-  float* sx = reinterpret_cast<float*>(smem + (size_t)(WARPS / TEAM) * kWarpHalfs * 2) + team * NOBJ;
-  const uint32_t sq_u = smem_u32(sq), sk_u = smem_u32(sk), sv_u = smem_u32(sv);
+  uint8_t* const tile = smem + (size_t)team * Tile::BYTES;
+  uint8_t* const extra = tile + 3 * Tile::SECTION;
+  float* const swap = reinterpret_cast<float*>(extra + Tile::SWAP);
+  const uint32_t sq_u = smem_u32(tile), sk_u = sq_u + Tile::SECTION, sv_u = sk_u + Tile::SECTION, s0_u = smem_u32(extra);
+  const uint8_t* const sv = tile + 2 * Tile::SECTION;
   const float scale = rsqrtf(static_cast<float>(DH));
   const int g = lane >> 2, tig = lane & 3;
-  const bool all_rows = n_q == T;
+  const int ra = lane & 15, ca = lane >> 4, rb = (lane & 7) + ((lane >> 4) << 3), cb = (lane >> 3) & 1;   // ldmatrix rows and halves
+  const int my_key = part * KEYS + (g >> 1) * 8 + 2 * tig + (g & 1);      // this lane's object key in the body row
+  const bool has_key = (g >> 1) * 8 < KEYS, all_rows = n_q == T;
   auto team_sync = [&]() {
     if (TEAM == 1) __syncwarp();
     else asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(TEAM * 32) : "memory");
   };
+  if (tlane == 0) *reinterpret_cast<uint4*>(extra + 3 * ROW) = make_uint4(0, 0, 0, 0);
 
   for (int64_t pair = (int64_t)blockIdx.x * (WARPS / TEAM) + team; pair < n_pairs; pair += (int64_t)gridDim.x * (WARPS / TEAM)) {
     int head;
@@ -201,160 +214,149 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
     for (int c = tlane; c < NOBJ * CH; c += 32 * TEAM) {
       const int row = c / CH, ch = c % CH;
       const __half* r = base + (int64_t)(row + 1) * ld + ch * 8;
-      const uint32_t at = (row * LDS + ch * 8) * 2;
+      const uint32_t at = tile_at<DH>(row, ch);
       if (all_rows) cp_async16(sq_u + at, r, true);
       cp_async16(sk_u + at, r + d, true);
       cp_async16(sv_u + at, r + 2 * d, true);
     }
     if (tlane < 3 * CH) {
       const int which = tlane / CH, ch = tlane % CH;
-      cp_async16(smem_u32(s0 + which * LDS + ch * 8), base + which * d + ch * 8, true);
+      cp_async16(s0_u + which * ROW + ch * 16, base + which * d + ch * 8, true);
     }
     cp_async_commit();
-    const float kb0 = key_bias[env * T];
+    const float kb0 = key_bias[env * T], kb_own = has_key ? key_bias[env * T + 1 + my_key] : 0.f;
     cp_async_wait<0>();
     team_sync();
+    // the body token's key as key 0 of a tile of eight: lanes 0 and 8 (two halves of 16 columns) its pieces, the others zeros
+    const uint32_t k0_at = (lane & 7) == 0 ? s0_u + ROW + cb * 16 : s0_u + 3 * ROW, k0_step = (lane & 7) == 0 ? 32u : 0u;
 
-    // ---- body query row: lane j scores object keys j, j + 32
+    // ---- body query row against this warp's object keys
     {
-      float sc[PER], s00 = 0.f;
+      float bs[KEYS / 8][4], bz[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int i = 0; i < PER; ++i) sc[i] = 0.f;
+      for (int nt = 0; nt < KEYS / 8; ++nt)
 #pragma unroll
-      for (int ch = 0; ch < CH; ++ch) {
-        const uint4 qv = *reinterpret_cast<const uint4*>(s0 + ch * 8);
-        const uint4 k0v = *reinterpret_cast<const uint4*>(s0 + LDS + ch * 8);
-        const __half2* qh = reinterpret_cast<const __half2*>(&qv);
-        const __half2* k0h = reinterpret_cast<const __half2*>(&k0v);
+        for (int e = 0; e < 4; ++e) bs[nt][e] = 0.f;
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 a = __half22float2(qh[e]), b = __half22float2(k0h[e]);
-          s00 = fmaf(a.x, b.x, fmaf(a.y, b.y, s00));
+      for (int ks = 0; ks < DH / 16; ++ks) {
+        uint32_t a[4], z[2];
+        a[0] = a[1] = *reinterpret_cast<const uint32_t*>(extra + (ks * 16 + 2 * tig) * 2);
+        a[2] = a[3] = *reinterpret_cast<const uint32_t*>(extra + (ks * 16 + 8 + 2 * tig) * 2);
+#pragma unroll
+        for (int j = 0; j < KEYS / 16; ++j) {
+          uint32_t b[4];
+          ldmatrix_x4(b, sk_u + tile_at<DH>(part * KEYS + j * 16 + rb, ks * 2 + cb));
+          mma_f16(bs[2 * j], a, b[0], b[1]);
+          mma_f16(bs[2 * j + 1], a, b[2], b[3]);
         }
-#pragma unroll
-        for (int i = 0; i < PER; ++i) {
-          const int j = lane + 32 * i;
-          if (j < NOBJ) {
-            const uint4 kv = *reinterpret_cast<const uint4*>(sk + j * LDS + ch * 8);
-            const __half2* kh = reinterpret_cast<const __half2*>(&kv);
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float2 a = __half22float2(qh[e]), b = __half22float2(kh[e]);
-              sc[i] = fmaf(a.x, b.x, fmaf(a.y, b.y, sc[i]));
-            }
-          }
-        }
+        ldmatrix_x2(z[0], z[1], k0_at + ks * k0_step);
+        mma_f16(bz, a, z[0], z[1]);
       }
-      s00 = s00 * scale + kb0;
-      float mx = s00;
+      float sc = -INFINITY;                          // of the lane's key: all eight rows of a quad column hold the same scores
 #pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        const int j = lane + 32 * i;
-        sc[i] = j < NOBJ ? sc[i] * scale + key_bias[env * T + 1 + j] : -INFINITY;
-        mx = fmaxf(mx, sc[i]);
-      }
-      mx = warp_max(mx);
-      const float p00 = expf(s00 - mx);
-      float sum = 0.f;
+      for (int nt = 0; nt < KEYS / 8; ++nt)
 #pragma unroll
-      for (int i = 0; i < PER; ++i) {
-        sc[i] = expf(sc[i] - mx);              // exp(-inf) = 0 for the lanes past NOBJ
-        sum += sc[i];
+        for (int e = 0; e < 2; ++e)
+          if (g == 2 * nt + e) sc = bs[nt][e] * scale + kb_own;
+      const float s00 = __shfl_sync(0xffffffffu, bz[0], 0) * scale + kb0;
+      float mx = fmaxf(warp_max(sc), s00);
+      if (TEAM == 2) {
+        if (lane == 0) swap[part] = mx;
+        team_sync();
+        mx = fmaxf(mx, swap[part ^ 1]);
       }
-      sum = warp_sum(sum) + p00;
-      const float inv = 1.f / sum;
-      // o0[c] = p00 v0[c] + sum_j p_j v_j[c]; a lane of the team owns columns tlane, tlane + 32 TEAM
-      constexpr int CPL = (DH + 32 * TEAM - 1) / (32 * TEAM);
+      const float p00 = expf(s00 - mx), p = expf(sc - mx);       // exp(-inf) = 0 for the lanes without a key
+      float sum = warp_sum(p);
+      // this warp's keys' share of the output; the lane owns columns CPL lane, ...
       float o[CPL];
 #pragma unroll
-      for (int u = 0; u < CPL; ++u) {
-        const int c = tlane + 32 * TEAM * u;
-        o[u] = c < DH ? p00 * __half2float(s0[2 * LDS + c]) : 0.f;
-      }
+      for (int u = 0; u < CPL; ++u) o[u] = 0.f;
 #pragma unroll
-      for (int i = 0; i < PER; ++i) {
-#pragma unroll 8
-        for (int jj = 0; jj < 32; ++jj) {
-          const int j = jj + 32 * i;
-          if (j >= NOBJ) break;
-          const float pj = __shfl_sync(0xffffffffu, sc[i], jj);
-#pragma unroll
-          for (int u = 0; u < CPL; ++u) {
-            const int c = tlane + 32 * TEAM * u;
-            if (c < DH) o[u] = fmaf(pj, __half2float(sv[j * LDS + c]), o[u]);
-          }
+      for (int l = 0; l < KEYS; ++l) {
+        const int key = part * KEYS + (l >> 3) * 8 + 2 * (l & 3) + ((l >> 2) & 1);
+        const float pj = __shfl_sync(0xffffffffu, p, l);
+        if (CPL == 2) {
+          const float2 v = __half22float2(*reinterpret_cast<const __half2*>(sv + tile_at<DH>(key, lane >> 2) + (lane & 3) * 4));
+          o[0] = fmaf(pj, v.x, o[0]);
+          o[CPL - 1] = fmaf(pj, v.y, o[CPL - 1]);
+        } else {
+          o[0] = fmaf(pj, __half2float(*reinterpret_cast<const __half*>(sv + tile_at<DH>(key, lane >> 3) + (lane & 7) * 2)), o[0]);
         }
       }
-      __half* orow = out + env * n_q * (int64_t)ldo + head * DH;
+      if (TEAM == 2) {
+        if (part == 1) {
+          if (lane == 0) swap[2] = sum;
 #pragma unroll
-      for (int u = 0; u < CPL; ++u) {
-        const int c = tlane + 32 * TEAM * u;
-        if (c < DH) orow[c] = __float2half_rn(o[u] * inv);
+          for (int u = 0; u < CPL; ++u) swap[4 + CPL * lane + u] = o[u];
+        }
+        team_sync();
+        if (part == 0) {
+          sum += swap[2];
+#pragma unroll
+          for (int u = 0; u < CPL; ++u) o[u] += swap[4 + CPL * lane + u];
+        }
+      }
+      if (part == 0) {
+        const float inv = 1.f / (sum + p00);
+        __half* orow = out + env * n_q * (int64_t)ldo + head * DH + CPL * lane;
+        const __half* v0 = reinterpret_cast<const __half*>(extra + 2 * ROW) + CPL * lane;
+#pragma unroll
+        for (int u = 0; u < CPL; ++u) orow[u] = __float2half_rn(fmaf(p00, __half2float(v0[u]), o[u]) * inv);
       }
     }
     if (!all_rows) continue;
 
-    // ---- extra score column of the object rows: sx[i] = q_i . k_0 (raw)
+    // ---- object query rows (16 MT of them) against the object keys and the body token's
+    const int row0 = part * (16 * MT);
+    float s[MT][NT][4], x0[MT][4];
 #pragma unroll
-    for (int i = 0; i < PER; ++i) {
-      const int r = lane + 32 * i;
-      if (r < NOBJ && (TEAM == 1 || i == part)) {           // the rows of this warp's query tiles
-        float acc = 0.f;
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int ch = 0; ch < CH; ++ch) {
-          const uint4 qv = *reinterpret_cast<const uint4*>(sq + r * LDS + ch * 8);
-          const uint4 k0v = *reinterpret_cast<const uint4*>(s0 + LDS + ch * 8);
-          const __half2* qh = reinterpret_cast<const __half2*>(&qv);
-          const __half2* k0h = reinterpret_cast<const __half2*>(&k0v);
+      for (int e = 0; e < 4; ++e) {
+        x0[mt][e] = 0.f;
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const float2 a = __half22float2(qh[e]), b = __half22float2(k0h[e]);
-            acc = fmaf(a.x, b.x, fmaf(a.y, b.y, acc));
-          }
-        }
-        sx[r] = acc;
+        for (int nt = 0; nt < NT; ++nt) s[mt][nt][e] = 0.f;
       }
+#pragma unroll
+    for (int ks = 0; ks < DH / 16; ++ks) {
+      uint32_t a[MT][4], z[2];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) ldmatrix_x4(a[mt], sq_u + tile_at<DH>(row0 + mt * 16 + ra, ks * 2 + ca));
+#pragma unroll
+      for (int j = 0; j < NT / 2; ++j) {
+        uint32_t b[4];
+        ldmatrix_x4(b, sk_u + tile_at<DH>(j * 16 + rb, ks * 2 + cb));
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          mma_f16(s[mt][2 * j], a[mt], b[0], b[1]);
+          mma_f16(s[mt][2 * j + 1], a[mt], b[2], b[3]);
+        }
+      }
+      ldmatrix_x2(z[0], z[1], k0_at + ks * k0_step);
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) mma_f16(x0[mt], a[mt], z[0], z[1]);
     }
     float kb[NT][2];
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
       for (int e = 0; e < 2; ++e) kb[nt][e] = key_bias[env * T + 1 + nt * 8 + tig * 2 + e];
-    __syncwarp();
-
-    // ---- object query rows against the object keys on the tensor cores
-#pragma unroll 1
-    for (int mt = part * (MT / TEAM); mt < (part + 1) * (MT / TEAM); ++mt) {
-      float s[NT][4];
+    uint32_t pa[MT][KS][4];
+    float p0[MT][2];                                 // the body key's probability for rows g, g + 8
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) s[nt][e] = 0.f;
-#pragma unroll
-      for (int ks = 0; ks < DH / 16; ++ks) {
-        uint32_t a[4];
-        ldmatrix_x4(a, sq_u + ((mt * 16 + (lane & 15)) * LDS + ks * 16 + (lane >> 4) * 8) * 2);
-#pragma unroll
-        for (int j = 0; j < NT / 2; ++j) {
-          uint32_t b[4];
-          const int row = j * 16 + (lane & 7) + ((lane >> 4) << 3);
-          ldmatrix_x4(b, sk_u + (row * LDS + ks * 16 + ((lane >> 3) & 1) * 8) * 2);
-          mma_f16(s[2 * j], a, b[0], b[1]);
-          mma_f16(s[2 * j + 1], a, b[2], b[3]);
-        }
-      }
-      float x0[2], mx[2];
+    for (int mt = 0; mt < MT; ++mt) {
+      float mx[2];
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        x0[r] = sx[mt * 16 + g + r * 8] * scale + kb0;
-        mx[r] = x0[r];
+        p0[mt][r] = __shfl_sync(0xffffffffu, x0[mt][2 * r], lane & ~3) * scale + kb0;
+        mx[r] = p0[mt][r];
       }
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          s[nt][e] = s[nt][e] * scale + kb[nt][e & 1];
-          mx[e >> 1] = fmaxf(mx[e >> 1], s[nt][e]);
+          s[mt][nt][e] = s[mt][nt][e] * scale + kb[nt][e & 1];
+          mx[e >> 1] = fmaxf(mx[e >> 1], s[mt][nt][e]);
         }
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
@@ -366,54 +368,58 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
       for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          s[nt][e] = expf(s[nt][e] - mx[e >> 1]);
-          sum[e >> 1] += s[nt][e];
+          s[mt][nt][e] = expf(s[mt][nt][e] - mx[e >> 1]);
+          sum[e >> 1] += s[mt][nt][e];
         }
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
         sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
-        x0[r] = expf(x0[r] - mx[r]);                 // the body key's share, the same for the four lanes of a row
-        sum[r] = 1.f / (sum[r] + x0[r]);
-        x0[r] *= sum[r];
-      }
-      uint32_t pa[KS][4];
-#pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
-        pa[ks][0] = pack_half2(s[2 * ks][0] * sum[0], s[2 * ks][1] * sum[0]);
-        pa[ks][1] = pack_half2(s[2 * ks][2] * sum[1], s[2 * ks][3] * sum[1]);
-        pa[ks][2] = pack_half2(s[2 * ks + 1][0] * sum[0], s[2 * ks + 1][1] * sum[0]);
-        pa[ks][3] = pack_half2(s[2 * ks + 1][2] * sum[1], s[2 * ks + 1][3] * sum[1]);
-      }
-      float o[DH / 8][4];
-#pragma unroll
-      for (int nt = 0; nt < DH / 8; ++nt) {           // start from the body token's contribution p0 v_0
-        const float2 v0 = __half22float2(*reinterpret_cast<const __half2*>(s0 + 2 * LDS + nt * 8 + tig * 2));
-        o[nt][0] = x0[0] * v0.x; o[nt][1] = x0[0] * v0.y;
-        o[nt][2] = x0[1] * v0.x; o[nt][3] = x0[1] * v0.y;
+        p0[mt][r] = expf(p0[mt][r] - mx[r]);          // the same for the four lanes of a row
+        sum[r] = 1.f / (sum[r] + p0[mt][r]);
+        p0[mt][r] *= sum[r];
       }
 #pragma unroll
-      for (int ks = 0; ks < KS; ++ks) {
+      for (int ks = 0; ks < KS; ++ks)
 #pragma unroll
-        for (int j = 0; j < DH / 16; ++j) {
-          uint32_t b[4];
-          const int row = ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
-          ldmatrix_x4_trans(b, sv_u + (row * LDS + j * 16 + (lane >> 4) * 8) * 2);
-          mma_f16(o[2 * j], pa[ks], b[0], b[1]);
-          mma_f16(o[2 * j + 1], pa[ks], b[2], b[3]);
+        for (int e = 0; e < 4; ++e)
+          pa[mt][ks][e] = pack_half2(s[mt][2 * ks + (e >> 1)][2 * (e & 1)] * sum[e & 1], s[mt][2 * ks + (e >> 1)][2 * (e & 1) + 1] * sum[e & 1]);
+    }
+    // P V, 16 output columns at a time, from the body token's contribution p0 v_0 on; the output takes the place of the query
+    // rows it came from
+#pragma unroll
+    for (int j = 0; j < DH / 16; ++j) {
+      float o[MT][2][4];
+#pragma unroll
+      for (int nt = 0; nt < 2; ++nt) {
+        const float2 v0 = __half22float2(*reinterpret_cast<const __half2*>(extra + 2 * ROW + (j * 16 + nt * 8 + tig * 2) * 2));
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          o[mt][nt][0] = p0[mt][0] * v0.x; o[mt][nt][1] = p0[mt][0] * v0.y;
+          o[mt][nt][2] = p0[mt][1] * v0.x; o[mt][nt][3] = p0[mt][1] * v0.y;
         }
       }
-      // the output takes the place of the query rows it came from
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        __half* orow = sq + (mt * 16 + g + r * 8) * LDS + tig * 2;
+      for (int ks = 0; ks < KS; ++ks) {
+        uint32_t b[4];
+        ldmatrix_x4_trans(b, sv_u + tile_at<DH>(ks * 16 + ra, j * 2 + ca));
 #pragma unroll
-        for (int nt = 0; nt < DH / 8; ++nt) *reinterpret_cast<uint32_t*>(orow + nt * 8) = pack_half2(o[nt][r * 2], o[nt][r * 2 + 1]);
+        for (int mt = 0; mt < MT; ++mt) {
+          mma_f16(o[mt][0], pa[mt][ks], b[0], b[1]);
+          mma_f16(o[mt][1], pa[mt][ks], b[2], b[3]);
+        }
       }
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+        tc5::stmatrix_x4(sq_u + tile_at<DH>(row0 + mt * 16 + ra, j * 2 + ca), pack_half2(o[mt][0][0], o[mt][0][1]), pack_half2(o[mt][0][2], o[mt][0][3]),
+                         pack_half2(o[mt][1][0], o[mt][1][1]), pack_half2(o[mt][1][2], o[mt][1][3]));
     }
     __syncwarp();
-    const int row0 = part * (NOBJ / TEAM);
-    copy_rows_out<DH, LDS>(sq + row0 * LDS, NOBJ / TEAM, out + (env * T + 1 + row0) * (int64_t)ldo + head * DH, ldo, true, lane);
+    __half* to = out + (env * T + 1 + row0) * (int64_t)ldo + head * DH;
+    for (int c = lane; c < 16 * MT * CH; c += 32) {
+      const int row = c / CH, ch = c % CH;
+      *reinterpret_cast<uint4*>(to + row * (int64_t)ldo + ch * 8) = *reinterpret_cast<const uint4*>(tile + tile_at<DH>(row0 + row, ch));
+    }
   }
 }
 
@@ -421,7 +427,7 @@ template <int DH, int NOBJ>
 int launch_body(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int d, int n_heads, int n_q, __half* out,
                 int ldo, cudaStream_t stream) {
   constexpr int kWarps = 8, kTeam = NOBJ <= 32 ? 1 : 2, kPairs = kWarps / kTeam;
-  constexpr int smem = kPairs * ((3 * NOBJ + 3) * (DH + 8) * 2 + NOBJ * 4);
+  constexpr int smem = kPairs * BodyTile<DH, NOBJ, kTeam>::BYTES;
   static DeviceOnce once;
   int rc = once.run("attn_body_kernel set-up", [] {
     return cudaFuncSetAttribute(attn_body_kernel<DH, NOBJ, kWarps, kTeam>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -429,7 +435,7 @@ int launch_body(const __half* qkv, int ld, const float* key_bias, int64_t n_envs
   if (rc != BSRL_OK) return rc;
   const int64_t pairs = n_envs * n_heads;
   int64_t blocks = (pairs + kPairs - 1) / kPairs;
-  const int64_t cap = (int64_t)sm_count() * 8;
+  const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
   launch_kernel(attn_body_kernel<DH, NOBJ, kWarps, kTeam>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d,
                                                                                                 n_heads, n_q, out, ldo);
@@ -448,7 +454,7 @@ template <int DH, int KG>
 int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int tokens, int d, int n_heads,
            int q_first, int n_q, __half* out, int ldo, cudaStream_t stream) {
   constexpr int kWarps = KG == 1 ? 8 : 4;
-  constexpr int smem = kWarps * 3 * (32 * KG) * (DH + 8) * 2;
+  constexpr int smem = kWarps * 3 * (32 * KG) * DH * 2;
   static DeviceOnce once;
   int rc = once.run("attn29_kernel set-up", [] {
     return cudaFuncSetAttribute(attn29_kernel<DH, KG, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -456,7 +462,7 @@ int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int
   if (rc != BSRL_OK) return rc;
   int64_t pairs = n_envs * n_heads;
   int64_t blocks = (pairs + kWarps - 1) / kWarps;
-  int64_t cap = (int64_t)sm_count() * 8;
+  int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
   launch_kernel(attn29_kernel<DH, KG, kWarps>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, tokens, d, n_heads, q_first, n_q, out, ldo);
   BSRL_LAUNCH_OK("attn29_kernel");

@@ -9,6 +9,7 @@
 // problem of one (env, head) pair -- at most 32 x 64 values per matrix -- lives in the warp's shared-memory
 // tile; the five products run on m16n8k16 MMAs with fp32 accumulation, P and dS rounded to fp16 as operands.
 #include "kernels.cuh"
+#include "attend.cuh"
 #include "tc5.cuh"
 
 namespace bsrl {
@@ -29,13 +30,6 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
   uint32_t r;
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
   return r;
-}
-
-// Byte offset of 16-byte piece p of row r of a tile of dense rows: the 8 rows of an ldmatrix hit 8 different 16-byte banks,
-// and so do 8 consecutive pieces (with rows padded by 16 bytes instead, those took two turns of the pipe).
-template <int DH>
-__device__ __forceinline__ uint32_t tile_at(int r, int p) {
-  return r * (DH * 2) + ((DH == 32 ? p ^ ((r >> 1) & 3) : DH == 48 ? p ^ ((r >> 2) & 1) : p ^ (r & 7)) << 4);
 }
 
 // One warp per (env, head); MT = 16-row query tiles (2: all 29 queries, 1: the lead rows or the critic's one).
