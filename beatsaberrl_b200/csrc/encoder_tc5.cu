@@ -39,7 +39,7 @@ constexpr int FIRST_EPI = 2 + HID_WARPS;
 constexpr int THREADS = (2 + HID_WARPS + EPI_WARPS) * 32;
 constexpr int STG_BYTES = 32 * 128;                // per-warp transposition buffer: 32 rows x 128 bytes
 constexpr int PARAM_FLOATS = (2 * 4 + 2) * 256;    // b0[4], b1[4], ln gamma, ln beta
-constexpr int PART_BYTES = 2 * BM * 8;
+constexpr int PART_BYTES = 2 * 2 * BM * 8;         // per tile parity and column half
 constexpr int SMEM_BYTES = SA_BYTES + SH_BYTES + STAGES * STAGE_BYTES + EPI_WARPS * STG_BYTES + PARAM_FLOATS * 4 +
                            PART_BYTES + 1024 + 256;
 constexpr int KERNEL_ID = 4;
@@ -84,18 +84,6 @@ __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
   sh->abort = 1;
 }
 
-// 32 fp32 values of row `row`, columns [col, col + 32) -> fp16 into a swizzled [128 x 64] chunk set
-__device__ __forceinline__ void store_h32(uint8_t* chunks, int row, int col, const float (&v)[32]) {
-  uint8_t* base = chunks + (col >> 6) * CHUNK_BYTES + (row >> 3) * 1024 + (row & 7) * 128;
-  const int p0 = (col & 63) >> 3;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    uint4 w = make_uint4(pack_half2(v[8 * i], v[8 * i + 1]), pack_half2(v[8 * i + 2], v[8 * i + 3]),
-                         pack_half2(v[8 * i + 4], v[8 * i + 5]), pack_half2(v[8 * i + 6], v[8 * i + 7]));
-    *reinterpret_cast<uint4*>(base + (((p0 + i) ^ (row & 7)) << 4)) = w;
-  }
-}
-
 __device__ __forceinline__ int part_of_tile(const EncParams& p, int t) {
   int e = 0;
 #pragma unroll
@@ -111,7 +99,6 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
   const uint32_t base = (raw + 1023u) & ~1023u;
   uint8_t* gen = smem_raw + (base - raw);
   const uint32_t sA = base, sH = base + SA_BYTES, ring = sH + SH_BYTES;
-  uint8_t* sH_g = gen + SA_BYTES;
   uint8_t* stg_all = gen + SA_BYTES + SH_BYTES + STAGES * STAGE_BYTES;
   float* prm = reinterpret_cast<float*>(stg_all + EPI_WARPS * STG_BYTES);
   float2* part = reinterpret_cast<float2*>(stg_all + EPI_WARPS * STG_BYTES + PARAM_FLOATS * 4);
@@ -247,16 +234,15 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
       if (spins >= kSpinLimit) give_up(sh, p.status, 10);
     }
   } else if (warp < FIRST_EPI) {
-    // ------------------------------------------------------------ hidden warps, thread = row
+    // ------------------------------------------------------------ hidden warps
     // layer 0: relu(acc + b0) -> the fp16 hidden tile, all d columns of this warp's 32 rows
     const int q = warp & 3;
-    const int trow = q * 32 + lane;
-    const uint32_t lane_base = tmem_base + ((uint32_t)(q * 32) << 16);
-    const float4* prm4 = reinterpret_cast<const float4*>(prm);
+    const uint32_t lane_q = tmem_base + ((uint32_t)(q * 32) << 16);
+    const int st_row = lane & 7, st_piece = lane >> 3;
     uint32_t tile_i = 0;
     for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, ++tile_i) {
       const uint32_t b = tile_i & 1, use = (tile_i >> 1) & 1;
-      const float4* P_b0 = prm4 + part_of_tile(p, t) * 64;
+      const uint64_t* prm_b0 = reinterpret_cast<const uint64_t*>(prm + part_of_tile(p, t) * 256 + 2 * (lane & 3));
       // the first GEMM of this tile was issued after the second GEMM of the tile before: its completion also
       // means that nothing reads the hidden tile any more
       if (!mbar_wait_warp(smem_u32(&sh->acc1_full[b]), use, abort)) {
@@ -264,20 +250,23 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
         break;
       }
       tc_fence_after();
-      for (int c = 0; c < d; c += 32) {
-        uint32_t r[32];
-        float v[32];
-        tmem_ld32(lane_base + 256u * b + c, r);
+      for (int c = 0; c < d; c += 32) {                     // in fragments (tc5.cuh)
+        uint32_t r[32], h[4][4];
+        tmem_ld_frags(lane_q + 256u * b + c, r);
         tmem_wait_ld();
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float4 b0 = P_b0[(c >> 2) + j];
-          v[4 * j] = fmaxf(__uint_as_float(r[4 * j]) + b0.x, 0.f);
-          v[4 * j + 1] = fmaxf(__uint_as_float(r[4 * j + 1]) + b0.y, 0.f);
-          v[4 * j + 2] = fmaxf(__uint_as_float(r[4 * j + 2]) + b0.z, 0.f);
-          v[4 * j + 3] = fmaxf(__uint_as_float(r[4 * j + 3]) + b0.w, 0.f);
+        for (int u = 0; u < 4; ++u) {
+          const uint64_t b0 = prm_b0[(c >> 1) + 4 * u];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            float v0, v1;
+            f2_split(f2_add(frag_pair(r, i, u), b0), v0, v1);
+            h[i][u] = pack_half2(fmaxf(v0, 0.f), fmaxf(v1, 0.f));
+          }
         }
-        store_h32(sH_g, trow, c, v);
+        const uint32_t at = sH + (c >> 6) * CHUNK_BYTES + q * 4096 + st_row * 128 + (((st_piece ^ st_row) << 4) ^ ((c & 32) << 1));
+#pragma unroll
+        for (int i = 0; i < 4; ++i) stmatrix_x4(at + i * 1024, h[i][0], h[i][1], h[i][2], h[i][3]);
       }
       fence_proxy_async_smem();
       tc_fence_before();
@@ -295,7 +284,8 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
     const int sub = lane >> 3, piece = lane & 7;            // transposed phase: row sub + 4 i, 16-byte piece
     const int c_lo = grp * dh2, c_hi = c_lo + dh2;
     const float4* prm4 = reinterpret_cast<const float4*>(prm);
-    const float4 *P_g = prm4 + 8 * 64, *P_b = prm4 + 9 * 64;
+    const int fr = lane >> 2, st_row = lane & 7, st_piece = lane >> 3;
+    const uint64_t* prm_frag = reinterpret_cast<const uint64_t*>(prm + 2 * (lane & 3));    // pair of 8-column unit u of vector v: [128 v + 4 u]
     const float inv_d = 1.0f / (float)d;
     uint32_t tile_i = 0;
     for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, ++tile_i) {
@@ -363,35 +353,37 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
       const float sum = (s4.x + s4.y) + (s4.z + s4.w), sq = (q4.x + q4.y) + (q4.z + q4.w);
       // ---- block 0's LayerNorm rows (fp16), second pass over the accumulator
       if (p.h) {
-        part[grp * BM + trow] = make_float2(sum, sq);
-        asm volatile("bar.sync 2, %0;" ::"n"(EPI_WARPS * 32) : "memory");
-        const float2 o = part[(grp ^ 1) * BM + trow];
+        part[(2 * b + grp) * BM + trow] = make_float2(sum, sq);
+        asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory");      // the two warps that share these rows
+        const float2 o = part[(2 * b + (grp ^ 1)) * BM + trow];
         const float mean = (sum + o.x) * inv_d;
         const float rstd = rsqrtf(fmaxf((sq + o.y) * inv_d - mean * mean, 0.f) + p.eps);
         const float shift = -mean * rstd;
+        uint64_t sc[4], sf[4];                              // of rows fr + 8 i
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float a = __shfl_sync(0xffffffffu, rstd, fr + 8 * i), o2 = __shfl_sync(0xffffffffu, shift, fr + 8 * i);
+          sc[i] = f2_make(a, a);
+          sf[i] = f2_make(o2, o2);
+        }
         for (int c = c_lo; c < c_hi; c += 64) {             // 64 columns = 128 bytes of fp16 per row
           const int nc = c_hi - c < 64 ? c_hi - c : 64;     // 32 when the half is an odd number of 32s
 #pragma unroll
           for (int s32 = 0; s32 < 64; s32 += 32) {
             if (s32 >= nc) break;
-            uint32_t r[32];
-            tmem_ld32(lane_base + c + s32, r);
+            uint32_t r[32], y[4][4];
+            tmem_ld_frags(lane_base + c + s32, r);
             tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {                   // 8 columns -> one 16-byte piece
-              float y[8];
+            for (int u = 0; u < 4; ++u) {
+              const int at = ((c + s32) >> 1) + 4 * u;
+              const uint64_t b1 = prm_frag[128 * (4 + e) + at], g = prm_frag[128 * 8 + at], bb = prm_frag[128 * 9 + at];
 #pragma unroll
-              for (int u = 0; u < 2; ++u) {
-                const int f4 = ((c + s32) >> 2) + 2 * j + u;
-                const float4 b1 = P_b1[f4], g = P_g[f4], bb = P_b[f4];
-                y[4 * u] = fmaf(fmaf(__uint_as_float(r[8 * j + 4 * u]) + b1.x, rstd, shift), g.x, bb.x);
-                y[4 * u + 1] = fmaf(fmaf(__uint_as_float(r[8 * j + 4 * u + 1]) + b1.y, rstd, shift), g.y, bb.y);
-                y[4 * u + 2] = fmaf(fmaf(__uint_as_float(r[8 * j + 4 * u + 2]) + b1.z, rstd, shift), g.z, bb.z);
-                y[4 * u + 3] = fmaf(fmaf(__uint_as_float(r[8 * j + 4 * u + 3]) + b1.w, rstd, shift), g.w, bb.w);
-              }
-              *reinterpret_cast<uint4*>(stg + lane * 128 + ((((s32 >> 3) + j) ^ (lane & 7)) << 4)) =
-                  make_uint4(pack_half2(y[0], y[1]), pack_half2(y[2], y[3]), pack_half2(y[4], y[5]), pack_half2(y[6], y[7]));
+              for (int i = 0; i < 4; ++i) y[i][u] = pack_f2(f2_fma(f2_fma(f2_add(frag_pair(r, i, u), b1), sc[i], sf[i]), g, bb));
             }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              stmatrix_x4(smem_u32(stg) + (8 * i + st_row) * 128 + ((((s32 >> 3) + st_piece) ^ st_row) << 4), y[i][0], y[i][1], y[i][2], y[i][3]);
           }
           __syncwarp();
           if (piece * 8 < nc) {
