@@ -278,8 +278,74 @@ int run_trunk(const Ctx& c, const __half* lead16, float* raw, const LinearArgs* 
   return with_heads ? linear_two(heads, *with_heads, c.st) : linear(heads, c.st);
 }
 
-// The blocks and the critic's attention for few environments (Paths::small): four launches per block, each spread over
-// many SMs -- attention per (env, head group), out-projection, FFN-up and FFN-down in 16-row tiles, the LayerNorms at the
+// Trunk, heads and critic as one launch (*done), where the batch is small enough and the widths fit.
+int run_readout(const Ctx& c, const __half* lead16, const __half* att_c, float* raw, float* vraw, bool* done) {
+  const Layout& l = c.l;
+  const Workspace& w = c.w;
+  const int d = l.d, D = l.D;
+  const int64_t B = c.B;
+  const TrainPtrs* tr = c.train;
+  *done = false;
+  if (l.trunk_v2 || g_call_engine != 0) return BSRL_OK;
+  ReadoutArgs a;
+  memset(&a, 0, sizeof(a));
+  a.rows = B;
+  a.d = d; a.D = D; a.Hh = l.Hh; a.k_lead = kLead * d;
+  a.lead = lead16; a.att = att_c;
+  auto mat = [&](const Mat& m, int n) { return ReadoutMat{c.W(m), c.Bv(m), n, m.pitch}; };
+  a.m[0] = mat(l.trunk_proj, D);
+  a.m[1] = mat(l.critic_out, d);
+  a.m[2] = mat(l.trunk_fc1, l.Hh);
+  a.m[4] = mat(l.trunk_fc2, D);
+  a.m[6] = mat(l.critic_m0, D);
+  a.m[7] = mat(l.heads, l.head_cols_pad);
+  a.m[8] = mat(l.critic_m1, D);
+  a.m[10] = mat(l.critic_m2, l.bins_pad);
+  a.ln1_g = c.G(l.trunk_ln1); a.ln1_b = c.Be(l.trunk_ln1);
+  a.ln2_g = c.G(l.trunk_ln2); a.ln2_b = c.Be(l.trunk_ln2);
+  a.eps = c.cfg->eps;
+  a.raw = raw; a.vraw = vraw;
+  a.z_out = tr ? tr->z : at<__half>(c.ws, w.z);
+  if (tr) {
+    a.xt_out = tr->xt; a.xt2_out = tr->xt2;
+    a.u_out = tr->u; a.r_out = tr->r;
+  }
+  if (!readout_ok(a)) return BSRL_OK;
+  double macs = 0;
+  for (const ReadoutMat& m : a.m) macs += (double)m.n * m.k;
+  g_stage = kStTrunk;
+  *done = true;
+  return timed(c.st, 2.0 * B * macs, 2.0 * macs, [&] { return readout(a, c.st); });
+}
+
+// All blocks as one launch (*done): one cluster per environment, up to as many environments as clusters run at once.  Beyond, a
+// second round of clusters costs the whole chain again: d 192 at 8 envs 222 us of forward against 159 of the launches below.
+int run_blocks_cluster(const Ctx& c, const float* x, const __half* h, const float* key_bias, __half* lead16, __half* att_c, bool* done) {
+  const Layout& l = c.l;
+  const int64_t B = c.B, R = B * kT, d = l.d;
+  __half* v0buf = l.value_residual ? at<__half>(c.ws, c.w.v0) : nullptr;
+  BlocksArgs a;
+  memset(&a, 0, sizeof(a));
+  a.d = l.d; a.n_heads = l.H; a.group_heads = l.attn_G; a.F = l.F; a.L = l.L; a.eps = c.cfg->eps;
+  *done = blocks_small_ok(a, B);
+  if (!*done) return BSRL_OK;
+  a.x0 = x; a.h0 = h; a.key_bias = key_bias; a.v0 = v0buf;
+  a.critic_wg = c.W(l.critic_qkv_g); a.critic_bg = c.Bv(l.critic_qkv_g);
+  a.critic_ln_g = c.G(l.critic_ln); a.critic_ln_b = c.Be(l.critic_ln);
+  a.lead16 = lead16; a.att_c = att_c;
+  for (int i = 0; i < l.L; ++i) {
+    const BlockW& b = l.blocks[i];
+    a.block[i] = BlockPtrs{c.W(b.qkv_g), c.W(b.out), c.W(b.up), c.W(b.down), c.Bv(b.qkv_g), c.Bv(b.out), c.Bv(b.up), c.Bv(b.down),
+                           c.G(b.ln_attn), c.Be(b.ln_attn), c.G(b.ln_ffn), c.Be(b.ln_ffn),
+                           v0buf && i > 0 ? at<float>(c.arena, b.vres) : nullptr, c.train && i + 1 < l.L ? c.train->x[i + 1] : nullptr};
+  }
+  g_stage = kStBlockTail;
+  const double per_row = 2.0 * d * (4.0 * d + 2.0 * l.F) + 4.0 * kT * d;
+  return timed(c.st, l.L * R * per_row, l.L * 2.0 * d * (4.0 * d + 2.0 * l.F), [&] { return blocks_small(a, B, c.st); });
+}
+
+// The blocks and the critic's attention for few environments (Paths::small), as one launch or as four per block, each spread
+// over many SMs -- attention per (env, head group), out-projection, FFN-up and FFN-down in 16-row tiles, the LayerNorms at the
 // entry of the kernels that need them -- instead of two that walk a 128-row tile through its phases on one SM.
 // x: the token stream, h: block 0's LayerNorm rows (from the encoder kernel).
 int run_blocks_small(const Ctx& c, float* x, const __half* h, const float* key_bias, __half* lead16, __half* att_c) {
@@ -292,6 +358,9 @@ int run_blocks_small(const Ctx& c, float* x, const __half* h, const float* key_b
   __half* hid = at<__half>(c.ws, w.hid);
   __half* v0buf = l.value_residual ? at<__half>(c.ws, w.v0) : nullptr;
   float* x_lead = at<float>(c.ws, w.x_lead);
+  bool done = false;
+  BSRL_TRY(run_blocks_cluster(c, x, h, key_bias, lead16, att_c, &done));
+  if (done) return BSRL_OK;
   auto norm_of = [&](const float* rows, const Norm& n, int quads) { return RowNorm{rows, d, ident, c.G(n), c.Be(n), c.cfg->eps, quads}; };
   auto attn = [&](const AttnSmallArgs* a, int n) {
     g_stage = kStAttnBlock;
@@ -528,12 +597,16 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
   __half* m2 = at<__half>(c.ws, w.m2);
   float* raw = c.train ? c.train->raw : at<float>(c.ws, w.raw);
   float* vraw = c.train ? c.train->vraw : at<float>(c.ws, w.vraw);
-  const LinearArgs c_out = linear_args(att_c, d, c.W(l.critic_out), d, c.Bv(l.critic_out), z, ldz, 0, 0, B, d, d);
-  const LinearArgs c_m0 = linear_args(z, ldz, c.W(l.critic_m0), ldz, c.Bv(l.critic_m0), m1, D, 0, 1, B, D, ldz);
-  BSRL_TRY(run_trunk(c, lead16, raw, &c_out, &c_m0));
-  g_stage = kStCritic;
-  BSRL_TRY(linear(linear_args(m1, D, c.W(l.critic_m1), D, c.Bv(l.critic_m1), m2, D, 0, 1, B, D, D), c.st));
-  BSRL_TRY(linear(linear_args(m2, D, c.W(l.critic_m2), D, c.Bv(l.critic_m2), vraw, l.bins_pad, 1, 0, B, l.bins_pad, D), c.st));
+  bool chained = false;
+  BSRL_TRY(run_readout(c, lead16, att_c, raw, vraw, &chained));
+  if (!chained) {
+    const LinearArgs c_out = linear_args(att_c, d, c.W(l.critic_out), d, c.Bv(l.critic_out), z, ldz, 0, 0, B, d, d);
+    const LinearArgs c_m0 = linear_args(z, ldz, c.W(l.critic_m0), ldz, c.Bv(l.critic_m0), m1, D, 0, 1, B, D, ldz);
+    BSRL_TRY(run_trunk(c, lead16, raw, &c_out, &c_m0));
+    g_stage = kStCritic;
+    BSRL_TRY(linear(linear_args(m1, D, c.W(l.critic_m1), D, c.Bv(l.critic_m1), m2, D, 0, 1, B, D, D), c.st));
+    BSRL_TRY(linear(linear_args(m2, D, c.W(l.critic_m2), D, c.Bv(l.critic_m2), vraw, l.bins_pad, 1, 0, B, l.bins_pad, D), c.st));
+  }
 
   HeadTailArgs t = tail_in;
   t.raw = raw; t.ld_raw = l.head_cols_pad;

@@ -80,6 +80,56 @@ int linear_small_block(const LinearArgs& p, int start, const RowNorm* norm, cuda
 bool linear_small_two_wins(const LinearArgs& a, const LinearArgs& b);
 int linear_small_two(const LinearArgs& a, const LinearArgs& b, cudaStream_t stream);
 
+// All blocks of a few environments and the critic's attention in one launch (blocks_small.cu): one cluster per environment
+constexpr int kMaxSmallBlocks = 32;
+struct BlockPtrs {
+  const __half *wg, *wo, *w0, *w2;       // regrouped q|k|v (3d, d), out (d, d), up (F, d), down (d, F)
+  const float *bg, *bo, *b0, *b2;
+  const float *ln1_g, *ln1_b, *ln2_g, *ln2_b;
+  const float* vres;                     // value residual, blocks after the first
+  float* x_next;                         // (n_envs*29, d) f32 stream after the block, or nullptr
+};
+struct BlocksArgs {
+  int d, n_heads, group_heads, F, L;     // group_heads: heads per group of the regrouped weights
+  float eps;
+  const float* x0;                       // (n_envs*29, d) f32 token stream
+  const __half* h0;                      // (n_envs*29, d) f16 block 0's LayerNorm rows
+  const float* key_bias;
+  __half* v0;                            // value residual: block 0's values, (n_envs*29, d) f16, or nullptr
+  const __half* critic_wg;
+  const float *critic_bg, *critic_ln_g, *critic_ln_b;
+  __half* lead16;                        // (n_envs*5, d) f16
+  __half* att_c;                         // (n_envs, d) f16
+  BlockPtrs block[kMaxSmallBlocks];
+};
+// widths that fit, and no more envs than the device runs clusters at once
+bool blocks_small_ok(const BlocksArgs& a, int64_t n_envs);
+int blocks_small(const BlocksArgs& a, int64_t n_envs, cudaStream_t stream);
+
+// Trunk, heads and critic of a small batch in one launch (readout.cu): weights dense (n, k), n and k padded as in the arena
+constexpr int kReadoutSteps = 6;
+struct ReadoutMat {
+  const __half* w;
+  const float* bias;
+  int n, k;                // n 0: none
+};
+struct ReadoutArgs {
+  int64_t rows;
+  int d, D, Hh, k_lead;
+  const __half* lead;      // (rows, k_lead) readout
+  const __half* att;       // (rows, d) critic attention
+  ReadoutMat m[2 * kReadoutSteps];      // {projection, critic projection}, {fc1}, {fc2}, {critic 0, heads}, {critic 1}, {critic 2}
+  const float *ln1_g, *ln1_b, *ln2_g, *ln2_b;
+  float eps;
+  float *raw, *vraw;       // heads and value bins, fp32 rows as wide as their matrices
+  __half* z_out;           // (rows, d + D): critic projection | trunk output
+  float *xt_out, *xt2_out; // kept for the backward, or nullptr
+  __half *u_out, *r_out;
+};
+// widths that fit, and no more rows than the device runs clusters at once
+bool readout_ok(const ReadoutArgs& a);
+int readout(const ReadoutArgs& a, cudaStream_t stream);
+
 // Projection + residual + LayerNorm in one kernel (gemm_ln_tc5.cu): x_out = R + A W^T + bias (fp32), h =
 // LayerNorm(x_out) (fp16).  N a multiple of 64 up to 512 (of 128 above 256), K a multiple of 64.  R and x_out
 // may be the same buffer.

@@ -94,7 +94,7 @@ struct Paths {
   bool attn_fused;   // q|k|v projection + attention in one kernel (no (rows, 3d) buffer)
   bool tail_fused;   // out-projection + LayerNorm + FFN in one kernel (no (rows, 4d) hidden buffer)
   bool enc_fused;    // both encoder layers + block 0's LayerNorm in one kernel
-  bool small;        // few environments: every block as four launches of many small CTAs
+  bool small;        // few environments: all blocks as one launch of clusters, or each as four launches of many small CTAs
 };
 int64_t small_envs(const Layout& l);      // the largest batch that may take Paths::small
 Paths plan_paths(const Layout& l, int engine, int64_t n_envs);

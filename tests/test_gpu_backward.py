@@ -290,6 +290,26 @@ def test_large_batch_gradients_equal_the_sum_of_small_batches(name, blocks, envs
         assert float((p.grad - whole[k]).norm()) <= 1e-4 * float(whole[k].norm()) + 1e-6 * top, k
 
 
+@pytest.mark.parametrize("name,opts", [("cfg2", None), ("recipe", dict(value_residual=True))])
+def test_few_env_gradients_equal_those_within_a_larger_batch(name, opts):
+    """Three environments, whose forward is one launch for all blocks and one for the readout, against the same three in a
+    batch that takes other kernels and in which the rest weighs nothing: the same rows, so the gradients differ by the order
+    of fp32 sums only (bound as above)."""
+    cfg = make_cfg(name, name == "recipe", opts=dict(opts or {}, n_blocks=3))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 5))
+    obs, act, up = po.make_obs(150, 21, padded=True), po.make_actions(150, cfg, 22), po.make_upstream(150, cfg, 23)
+    grads = []
+    for n in (3, 150):
+        with torch.enable_grad():
+            _loss(m, obs[:n].cuda(), act[:n].cuda(), {k: torch.cat([v[:3], 0 * v[3:n]]) for k, v in up.items()}).backward()
+        grads.append({k: p.grad.clone() for k, p in m.named_parameters()})
+        m.zero_grad()
+    m.check_device()
+    top = max(float(g.norm()) for g in grads[1].values())
+    for k, g in grads[0].items():
+        assert float((g - grads[1][k]).norm()) <= 1e-4 * float(grads[1][k].norm()) + 1e-6 * top, k
+
+
 @pytest.mark.parametrize("name,opts,envs", [("cfg1", None, 70), ("recipe", dict(value_residual=True), 45),
                                             ("tiny", dict(trunk_arch="simbav2", emb_ln=True, final_ln=True), 33)])
 def test_backward_only_reads_the_save_buffer(name, opts, envs):

@@ -283,6 +283,21 @@ def test_few_envs_take_other_kernels_and_give_the_same_bits(name, geo, opts):
     m.check_device()
 
 
+@pytest.mark.parametrize("name,opts,blocks", [("tiny", None, 2), ("cfg1", None, 3), ("recipe", None, 2), ("recipe", dict(value_residual=True), 4),
+                                              ("cfg2", None, 2)])
+def test_one_env_per_cluster_gives_the_same_bits(name, opts, blocks):
+    """A handful of environments (as many as clusters of 16 CTAs run at once) take all blocks in one launch, and up to 16 rows
+    for each of these the readout: the bits of the launches that more environments take, on both sides of either line."""
+    cfg = make_cfg(name, name == "recipe", opts=dict(opts or {}, n_blocks=blocks))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 9))
+    obs = po.make_obs(160, 35, padded=True).cuda()
+    full_l, full_v = m.forward_stacked(obs)
+    for B in (1, 2, 4, 7, 8, 9, 15, 16, 17, 33, 96, 97, 128, 145):
+        l, v = m.forward_stacked(obs[:B])
+        assert torch.equal(l, full_l[:B]) and torch.equal(v, full_v[:B]), B
+    m.check_device()
+
+
 @pytest.mark.parametrize("name,B,part", [("cfg2", 2601, 300), ("cfg4", 1001, 90)])
 def test_many_envs_match_slices(name, B, part):
     """Batches past the sizes at which kernels take CTA pairs, resident weights or mapped TMA boxes against slices that take none
