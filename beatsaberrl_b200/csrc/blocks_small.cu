@@ -4,13 +4,16 @@
 // gemm_small.cu) each costs 4.3 us, nearly all of it latency.  Here a cluster takes an environment through all blocks
 // (cluster_chain.cuh): x, the attention output and the hidden activations live in the shared memory of all its CTAs, and
 // a block is four steps:
-//   A  LayerNorm, q|k|v projection and attention, one head per CTA (the last block: the critic's heads on the next CTAs)
+//   A  LayerNorm, q|k|v projection and attention: a head on two CTAs, each with half of the queries (in the last block, which
+//      has five, the second one takes the critic's head)
 //   B  out-projection onto x            C  LayerNorm, FFN-up            D  FFN-down onto x
 // each with its output columns spread over the CTAs in units of 8.  The arithmetic is that of the launches (attend.cuh,
 // row_norm.cuh, the sums of linear_small_block), bit for bit: a batch size does not change a row's result.
-// One env, whole forward behind a graph, launches / this: d 64 49.2 / 45.1 us, d 128 57.4 / 53.2, d 192 (6 blocks) 141.8 /
-// 128.8, d 256 116.8 / 104.5; four at d 192 149.6 / 131.1.  Of some 10 us per block (d 192) most is latency: the copies of
-// a step's results into 16 CTAs, the loads of LayerNorm's rows, short chains of MMAs.
+// Whole forward behind a graph, launches / this (with readout.cu): one env d 64 49.1 / 41.0 us, d 128 57.4 / 47.1, d 192 (6
+// blocks) 143.4 / 106.6, d 256 117.3 / 93.2; seven at d 192 157.8 / 112.8.  Some 12 us per block remain (d 192), nearly all of it
+// latency: a step's results into 16 CTAs (0.7 us, bound by the senders' 32 B per clock), LayerNorm, short chains of MMAs.
+// What took most and went: a bulk copy per weight row (100 cycles each for its issuer), LayerNorm by units along a row
+// (8-way bank conflicts), a head's 29 rows sent to 16 CTAs by one: 124.9 -> 106.6 us together.
 #include <atomic>
 #include <type_traits>
 
@@ -23,6 +26,7 @@ namespace {
 using namespace chain;
 
 constexpr int ROWS = 32, KERNEL_ID = 13;
+constexpr int MAX_D = 256;
 constexpr int UNIT16 = ROWS * 16, UNIT32 = ROWS * 32 + 32;      // a unit's 8 columns of all rows: fp16, fp32 (padded)
 
 struct Plan {
@@ -35,8 +39,8 @@ struct Params {
 };
 struct Shared {
   uint64_t in_full[4];
-  uint64_t w_full[2][WARPS];
   float2 norm[ROWS];               // per row: 1 / deviation, -mean / deviation
+  float norm_w[2 * MAX_D];         // the next LayerNorm's gamma | beta
   BlockPtrs block[kMaxSmallBlocks];
   int abort;
 };
@@ -69,13 +73,11 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
 
   if (tid == 0) {
     for (int i = 0; i < 4; ++i) tc5::mbar_init(smem_u32(&sh.in_full[i]), 1);
-    for (int b = 0; b < 2; ++b)
-      for (int w = 0; w < WARPS; ++w) tc5::mbar_init(smem_u32(&sh.w_full[b][w]), 1);
     sh.abort = 0;
     tc5::fence_barrier_init();
   }
   __syncthreads();
-  // bytes that a step sends to every CTA; the critic's heads send a mark once they are done with x
+  // bytes that a step sends to every CTA, step D to those with a head; the critic's heads send a mark once they are done with x
   auto arm = [&](int step) {
     const bool last = step >= n_steps - 4;
     const int rows = last ? 16 : ROWS, s = step & 3;
@@ -85,9 +87,9 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
   if (tid == 0)
     for (int i = 0; i < 4; ++i) arm(i);
 
-  // this CTA's head in step A, in the last block perhaps a critic's; this warp's unit of 8 columns in steps B, C and D
-  const int head = rank < H ? rank : rank - H;
-  const bool has_head = rank < H, has_critic = !has_head && rank < 2 * H;
+  // this CTA's head and half of the queries in step A, in the last block perhaps a critic's head; this warp's unit of 8 columns in steps B, C and D
+  const int head = rank % H, half = rank / H;
+  const bool has_head = half < 2;
   const int u0 = rank + warp * CTAS, row0 = (head / G) * 3 * G * DH + (head % G) * DH;
   int head_row[S::PER];                                      // weight rows of this warp's units of the head
 #pragma unroll
@@ -95,27 +97,33 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
     const int u = warp + i * WARPS;
     head_row[i] = row0 + (u / (DH / 8)) * G * DH + (u % (DH / 8)) * 8;
   }
-  // this warp's weights of a step
+  // this warp's weights of a step and, with all warps, those of its LayerNorm: a group of copies (empty past the last step)
   auto request = [&](int step) {
-    if (*abort || step >= n_steps) return;
-    const BlockPtrs& b = sh.block[step >> 2];
-    const int s = step & 3;
-    const uint32_t bar = smem_u32(&sh.w_full[step & 1][warp]), set = base + l.w_set[step & 1];
-    if (s == 0) {
-      const bool critic = has_critic && step == n_steps - 4;
-      if (!has_head && !critic) return;
-      const __half* wg = critic ? a.critic_wg : b.wg;
-      if (lane == 0) tc5::mbar_expect_tx(bar, ((S::UNITS - warp + WARPS - 1) / WARPS) * 16 * d);
-      __syncwarp();
+    if (step < n_steps) {
+      const BlockPtrs& b = sh.block[step >> 2];
+      const int s = step & 3;
+      const uint32_t set = base + l.w_set[step & 1];
+      const bool critic = s == 0 && half == 1 && step == n_steps - 4;
+      if (s == 0 ? has_head && step > 0 : s == 2) {
+        const float *gamma = critic ? a.critic_ln_g : s == 0 ? b.ln1_g : b.ln2_g, *beta = critic ? a.critic_ln_b : s == 0 ? b.ln1_b : b.ln2_b;
+        if (tid < d >> 1) cp_async16(smem_u32(sh.norm_w + 4 * tid), tid < d >> 2 ? gamma + 4 * tid : beta + (4 * tid - d), true);
+      }
+      if (s == 0) {
+        const __half* wg = critic ? a.critic_wg : b.wg;
 #pragma unroll
-      for (int i = 0; i < S::PER; ++i)
-        if (warp + i * WARPS < S::UNITS) request_unit(set + (warp + i * WARPS) * unit_bytes(d), wg + head_row[i] * d, d, bar, lane);
-    } else if (u0 < (s == 2 ? F : d) >> 3) {
-      const int K = s == 3 ? F : d;
-      if (lane == 0) tc5::mbar_expect_tx(bar, 16 * K);
-      __syncwarp();
-      request_unit(set + warp * unit_bytes(K), (s == 1 ? b.wo : s == 2 ? b.w0 : b.w2) + u0 * 8 * K, K, bar, lane);
+        for (int i = 0; i < S::PER; ++i)
+          if (has_head && warp + i * WARPS < S::UNITS) request_unit(set + (warp + i * WARPS) * unit_bytes(d), wg + head_row[i] * d, d, lane);
+      } else if (u0 < (s == 2 ? F : d) >> 3) {
+        const int K = s == 3 ? F : d;
+        request_unit(set + warp * unit_bytes(K), (s == 1 ? b.wo : s == 2 ? b.w0 : b.w2) + u0 * 8 * K, K, lane);
+      }
     }
+    cp_async_commit();
+  };
+  // ... which were requested before the last ones
+  auto wait_weights = [&] {
+    cp_async_wait<1>();
+    __syncwarp();
   };
   __syncthreads();
   request(0);
@@ -127,9 +135,9 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
   for (int i = tid; i < ROWS * (d >> 2); i += THREADS) {
     const int row = i / (d >> 2), c = i - row * (d >> 2);
     const bool ok = row < kT;
-    cp_async16(base + l.x + (c >> 1) * UNIT32 + row * 32 + (c & 1) * 16, ok ? a.x0 + (env * kT + row) * d + c * 4 : a.x0, ok);
+    cp_async16(base + l.x + (c >> 1) * UNIT32 + row32(row, c & 1), ok ? a.x0 + (env * kT + row) * d + c * 4 : a.x0, ok);
   }
-  if (rank < H)
+  if (has_head)
     for (int i = tid; i < ROWS * U; i += THREADS) {
       const int row = i / U, c = i - row * U;
       const bool ok = row < kT;
@@ -148,25 +156,17 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
   cp_async_wait<0>();
   __syncthreads();
 
-  // LayerNorm of x's rows [0, live) into h; the other rows zero.  Two threads per row add its halves; then a thread's eight
-  // columns are the same in every row, and their weights are fetched ahead of the step's wait.
-  const int ln_rows = THREADS / U, ln_unit = tid % U, ln_row0 = tid / U;
-  float gam[8], bet[8];
-  auto fetch_norm = [&](const float* gamma, const float* beta) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      *reinterpret_cast<float4*>(gam + 4 * e) = *reinterpret_cast<const float4*>(gamma + ln_unit * 8 + 4 * e);
-      *reinterpret_cast<float4*>(bet + 4 * e) = *reinterpret_cast<const float4*>(beta + ln_unit * 8 + 4 * e);
-    }
-  };
+  // LayerNorm of x's rows [0, live) into h; the other rows zero.  Two threads per row add its halves; then a warp takes a unit of
+  // all rows.
   const float inv_d = 1.0f / (float)d;
   auto layer_norm = [&](auto quads, int live) {
-    if (tid < 2 * ROWS) {
-      const uint8_t* p = x_g + ((tid & 1) * (U >> 1)) * UNIT32 + (tid >> 1) * 32;
+    if (warp < 2) {
+      const int row = warp * 16 + (lane & 15);
+      const uint8_t* p = x_g + (lane >> 4) * (U >> 1) * UNIT32;
       float sum = 0.f, sq = 0.f;
 #pragma unroll 4
       for (int j = 0; j < U >> 1; ++j, p += UNIT32) {
-        const float4 v = *reinterpret_cast<const float4*>(p), w = *reinterpret_cast<const float4*>(p + 16);
+        const float4 v = *reinterpret_cast<const float4*>(p + row32(row, 0)), w = *reinterpret_cast<const float4*>(p + row32(row, 1));
         if (decltype(quads)::value) {
           sum += (v.x + v.y) + (v.z + v.w);
           sq = fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, fmaf(v.w, v.w, sq))));
@@ -181,65 +181,65 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
           }
         }
       }
-      const float sum2 = __shfl_xor_sync(0xffffffffu, sum, 1), sq2 = __shfl_xor_sync(0xffffffffu, sq, 1);
+      const float sum2 = __shfl_xor_sync(0xffffffffu, sum, 16), sq2 = __shfl_xor_sync(0xffffffffu, sq, 16);
       const float mean = (sum + sum2) * inv_d;
       const float rstd = rsqrtf(fmaxf((sq + sq2) * inv_d - mean * mean, 0.f) + a.eps);
-      if (!(tid & 1)) sh.norm[tid >> 1] = make_float2(rstd, -mean * rstd);
+      if (lane < 16) sh.norm[row] = make_float2(rstd, -mean * rstd);
     }
-    __syncthreads();
-    if (ln_row0 < ln_rows)
-      for (int row = ln_row0; row < ROWS; row += ln_rows) {
-        uint4 out = make_uint4(0, 0, 0, 0);
-        if (row < live) {
-          const float2 n = sh.norm[row];
-          const float4 v = *reinterpret_cast<const float4*>(x_g + ln_unit * UNIT32 + row * 32);
-          const float4 w = *reinterpret_cast<const float4*>(x_g + ln_unit * UNIT32 + row * 32 + 16);
-          const float e[8] = {v.x, v.y, v.z, v.w, w.x, w.y, w.z, w.w};
-          float y[8];
+    cp_async_wait<1>();
+    __syncthreads();                                         // also: gamma and beta are there
+    const float2 n = sh.norm[lane];
+#pragma unroll 2
+    for (int u = warp; u < U; u += WARPS) {
+      const float4 v = *reinterpret_cast<const float4*>(x_g + u * UNIT32 + row32(lane, 0));
+      const float4 w = *reinterpret_cast<const float4*>(x_g + u * UNIT32 + row32(lane, 1));
+      float gam[8], bet[8];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) y[k] = fmaf(fmaf(e[k], n.x, n.y), gam[k], bet[k]);
-          out = make_uint4(pack_half2(y[0], y[1]), pack_half2(y[2], y[3]), pack_half2(y[4], y[5]), pack_half2(y[6], y[7]));
-        }
-        *reinterpret_cast<uint4*>(h_g + ln_unit * UNIT16 + row * 16) = out;
+      for (int e = 0; e < 2; ++e) {
+        *reinterpret_cast<float4*>(gam + 4 * e) = *reinterpret_cast<const float4*>(sh.norm_w + u * 8 + 4 * e);
+        *reinterpret_cast<float4*>(bet + 4 * e) = *reinterpret_cast<const float4*>(sh.norm_w + d + u * 8 + 4 * e);
       }
+      const float e[8] = {v.x, v.y, v.z, v.w, w.x, w.y, w.z, w.w};
+      float y[8];
+#pragma unroll
+      for (int k = 0; k < 8; ++k) y[k] = lane < live ? fmaf(fmaf(e[k], n.x, n.y), gam[k], bet[k]) : 0.f;
+      *reinterpret_cast<uint4*>(h_g + u * UNIT16 + lane * 16) =
+          make_uint4(pack_half2(y[0], y[1]), pack_half2(y[2], y[3]), pack_half2(y[4], y[5]), pack_half2(y[6], y[7]));
+    }
     __syncthreads();
   };
 
-  uint32_t w_phase = 0, in_phase = 0;                        // bit s: phase of the next weights of set s, of step s's bytes
-  auto wait_weights = [&](int step) {
-    if (wait_bytes<false>(smem_u32(&sh.w_full[step & 1][warp]), (w_phase >> (step & 1)) & 1, abort, args.status, KERNEL_ID * 16 + 2))
-      w_phase ^= 1u << (step & 1);
-  };
+  uint32_t in_phase = 0;                                     // bit s: phase of step s's bytes
   auto wait_in = [&](int s) {
-    if (wait_bytes<true>(smem_u32(&sh.in_full[s]), (in_phase >> s) & 1, abort, args.status, KERNEL_ID * 16 + 1)) in_phase ^= 1u << s;
+    if (wait_bytes(smem_u32(&sh.in_full[s]), (in_phase >> s) & 1, abort, args.status, KERNEL_ID * 16 + 1)) in_phase ^= 1u << s;
   };
 
 #pragma unroll 1
   for (int ib = 0; ib < a.L; ++ib) {
     const BlockPtrs& b = sh.block[ib];
-    const bool last = ib + 1 == a.L, critic = last && has_critic;
+    const bool last = ib + 1 == a.L, critic = last && half == 1;
     const int live = last ? kLead : kT, step = 4 * ib;
     // ---------------------------------------------------------------- A: LayerNorm, q|k|v, attention
     float2 bias[S::PER];
-    if (has_head || critic) {
+    if (has_head) {
       const float* bg = critic ? a.critic_bg : b.bg;
 #pragma unroll
       for (int i = 0; i < S::PER; ++i)
         if (warp + i * WARPS < S::UNITS) bias[i] = *reinterpret_cast<const float2*>(bg + head_row[i] + tig * 2);
-      if (critic) fetch_norm(a.critic_ln_g, a.critic_ln_b);
-      else fetch_norm(b.ln1_g, b.ln1_b);
     }
     if (ib > 0) {
-      wait_in(3);
-      if (tid == 0 && !*abort && !last) arm(step + 3);
+      if (has_head) {
+        wait_in(3);
+        if (tid == 0 && !*abort && !last) arm(step + 3);
+      }
       __syncthreads();
       request(step + 1);
     }
-    if (has_head || critic) {
+    if (has_head) {
       if (ib > 0) layer_norm(std::true_type{}, kT);
       uint8_t *const q_g = smem + l.hid, *const o_g = q_g + ROWS * S::LDQ;      // in the place of the hidden activations
       const uint32_t set = base + l.w_set[0], q_u = smem_u32(q_g);
-      wait_weights(step);
+      wait_weights();
       float acc[S::PER][2][4];
       uint32_t w[S::PER];
 #pragma unroll
@@ -283,17 +283,18 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
           send128(base + l.dummy + off, smem_u32(&sh.in_full[0]) + off, make_uint4(0, 0, 0, 0));
         }
       } else {
-        if (warp < 2 && live > 16 * warp)
-          attend_pair<1, DH, S::LDQ, 128>(q_u, q_u + DH * 2, q_u + 4 * DH, 16 * warp, 0, kb, live - 16 * warp,
-                                          reinterpret_cast<__half*>(o_g) + 16 * warp * (S::LDO / 2), S::LDO / 2, lane, nullptr, 0, 0);
+        if (warp == 0)
+          attend_pair<1, DH, S::LDQ, 128>(q_u, q_u + DH * 2, q_u + 4 * DH, 16 * half, 0, kb, live - 16 * half, reinterpret_cast<__half*>(o_g),
+                                          S::LDO / 2, lane, nullptr, 0, 0);
         __syncthreads();
-        // every 16-byte piece of the output to every CTA: a warp takes 32 (in the last block 16) rows of one 8-column unit
+        // every 16-byte piece of the output to every CTA: a warp takes the rows of one 8-column unit, to two CTAs at a time
         for (int c = warp; c < DH / 8; c += WARPS) {
-          if (last && lane >= 16) break;
-          const uint4 v = lane < live ? *reinterpret_cast<const uint4*>(o_g + lane * S::LDO + c * 16) : make_uint4(0, 0, 0, 0);
-          uint32_t to = base + l.att + (head * (DH / 8) + c) * UNIT16 + lane * 16 + peers.first, bar = smem_u32(&sh.in_full[0]) + peers.first;
+          const int row = 16 * half + (lane & 15);
+          const uint4 v = row < live ? *reinterpret_cast<const uint4*>(o_g + (lane & 15) * S::LDO + c * 16) : make_uint4(0, 0, 0, 0);
+          const uint32_t off = peers.first + (lane >> 4) * peers.step;
+          uint32_t to = base + l.att + (head * (DH / 8) + c) * UNIT16 + row * 16 + off, bar = smem_u32(&sh.in_full[0]) + off;
 #pragma unroll
-          for (int p = 0; p < CTAS; ++p, to += peers.step, bar += peers.step) send128(to, bar, v);
+          for (int p = 0; p < CTAS / 2; ++p, to += 2 * peers.step, bar += 2 * peers.step) send128(to, bar, v);
         }
       }
     }
@@ -304,14 +305,13 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
       const bool mine = u0 < (s == 2 ? F : d) >> 3;          // at most 128 units: one per warp
       float2 bias = make_float2(0.f, 0.f);
       if (mine) bias = *reinterpret_cast<const float2*>((s == 1 ? b.bo : s == 2 ? b.b0 : b.b2) + u0 * 8 + tig * 2);
-      if (s == 2) fetch_norm(b.ln2_g, b.ln2_b);
       wait_in(s - 1);
       if (tid == 0 && !*abort && !last) arm(step + 4 + s - 1);      // the next block's bytes of that step
       __syncthreads();                                       // every warp is done with the step before: its weights' set is free
       request(step + s + 1);
       if (s == 2) layer_norm(std::false_type{}, live);
       if (mine) {
-        wait_weights(step + s);
+        wait_weights();
         const uint32_t bar = smem_u32(&sh.in_full[s]), op = base + (s == 1 ? l.att : s == 2 ? l.h : l.hid);
         const uint32_t w[1] = {base + l.w_set[(step + s) & 1] + warp * unit_bytes(K)};
         const int u = u0, col = u * 8 + tig * 2;
@@ -319,7 +319,7 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
           float2 v = make_float2(0.f, 0.f);
-          if (s != 2) v = *reinterpret_cast<const float2*>(x_g + u * UNIT32 + (g + 8 * r) * 32 + tig * 8);   // onto x, out-projection: + bias
+          if (s != 2) v = *reinterpret_cast<const float2*>(x_g + u * UNIT32 + row32(g + 8 * r, tig >> 1) + (tig & 1) * 8);   // onto x, out-projection: + bias
           acc[0][r >> 1][2 * (r & 1)] = s == 1 ? v.x + bias.x : v.x;
           acc[0][r >> 1][2 * (r & 1) + 1] = s == 1 ? v.y + bias.y : v.y;
         }
@@ -347,7 +347,13 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
           } else if (s == 3 && last) {                       // the readout rows
             if (g < kLead) *reinterpret_cast<uint32_t*>(a.lead16 + (env * kLead + g) * d + col) = pack_half2(v[0], v[1]);
           } else {
-            push_rows32(base + l.x + u * UNIT32 + mt * 512, bar, peers, v, lane);
+            // after the out-projection every CTA needs the rows, after the block those with a head, and this warp its own columns
+            push_rows32(base + l.x + u * UNIT32 + mt * 512, bar, peers, s == 1 ? CTAS : 2 * H, v, lane);
+            if (s == 3 && !has_head) {
+#pragma unroll
+              for (int hh = 0; hh < 2; ++hh)
+                *reinterpret_cast<float2*>(x_g + u * UNIT32 + row32(mt * 16 + g + 8 * hh, tig >> 1) + (tig & 1) * 8) = make_float2(v[2 * hh], v[2 * hh + 1]);
+            }
             if (s == 3 && b.x_next) {
 #pragma unroll
               for (int hh = 0; hh < 2; ++hh) {
@@ -362,11 +368,8 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
   }
   __syncthreads();
   if (*abort) {
-    // weights in flight land (bounded), and nobody leaves while a peer may still send to it
-    for (int i = 0; lane == 0 && i < 2; ++i)
-      for (int k = 0; k < 4096 && !tc5::mbar_try_wait(smem_u32(&sh.w_full[i][warp]), (w_phase >> i) & 1); ++k) {}
-    __syncwarp();
-    tc5::cluster_sync_all();
+    cp_async_wait<0>();
+    tc5::cluster_sync_all();                                 // nobody leaves while a peer may still send to it
   }
 }
 
@@ -438,7 +441,7 @@ int chain::resident_clusters() {
 }
 
 bool blocks_small_ok(const BlocksArgs& a, int64_t n_envs) {
-  if (a.d % 64 || a.d < 64 || a.d > 256 || a.F % 256 || a.F < 256 || a.F > 1024 || a.L < 2 || a.L > kMaxSmallBlocks) return false;
+  if (a.d % 64 || a.d < 64 || a.d > MAX_D || a.F % 256 || a.F < 256 || a.F > 1024 || a.L < 2 || a.L > kMaxSmallBlocks) return false;
   if (a.n_heads < 1 || a.n_heads > CTAS / 2 || a.d % a.n_heads || n_envs < 1 || n_envs > resident_clusters()) return false;
   const int dh = a.d / a.n_heads;
   return (dh == 32 || dh == 48 || dh == 64) && make_plan(a).bytes <= SMEM_LIMIT;

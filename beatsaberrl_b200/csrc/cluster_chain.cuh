@@ -8,10 +8,12 @@
 // (With a barrier of the cluster instead, a step pays 850 cycles for the release; exchanged through L2, another 900 for
 // the operand's loads.)
 //
-// A unit is 8 output columns of a product: one warp's work.  Its 8 weight rows come whole by bulk copies, 16 bytes apart
-// in bank, as a rule a step ahead of their use, and the warp runs down K in order: every output is the same sum in the
+// A unit is 8 output columns of a product: one warp's work.  The warp copies its 8 weight rows itself, 16 bytes apart
+// in bank, as a rule a step ahead of their use (a group of cp.async per step; a bulk copy per row costs its issuer 100
+// cycles each), and runs down K in order: every output is the same sum in the
 // same order as in the other linear kernels.  Activations lie unit-major: [K / 8][rows][8], so that a unit's results
-// leave as contiguous 128-byte (fp32: 256-byte) runs and ldmatrix reads 8 rows from 128 contiguous bytes.
+// leave as contiguous 128-byte (fp32: 256-byte) runs and ldmatrix reads 8 rows from 128 contiguous bytes.  The two halves of
+// every fp32 row of 8 are swapped in rows 4-7 of 8: 16 bytes of 8 consecutive rows are in 8 different groups of banks.
 #pragma once
 #include "tc5.cuh"
 
@@ -52,8 +54,10 @@ __device__ __forceinline__ void push_rows16(uint32_t dst, uint32_t bar, const Pe
 #pragma unroll
   for (int c = 0; c < CTAS / 2; ++c, off += 2 * p.step) send128(dst + (lane & 15) * 16 + off, bar + off, row);
 }
-// ... and its fp32 results to rows of 32 bytes: lane i gathers half i % 2 of row i / 2
-__device__ __forceinline__ void push_rows32(uint32_t dst, uint32_t bar, const Peers& p, const float (&v)[4], int lane) {
+// where 16 bytes of an fp32 row of 8 lie
+__device__ __forceinline__ int row32(int row, int half) { return row * 32 + ((half ^ (row >> 2 & 1)) << 4); }
+// ... and its fp32 results to rows of 32 bytes of the first n CTAs: lane i gathers half i % 2 of row i / 2
+__device__ __forceinline__ void push_rows32(uint32_t dst, uint32_t bar, const Peers& p, int n, const float (&v)[4], int lane) {
   const int src = 4 * ((lane >> 1) & 7) + 2 * (lane & 1);
   uint4 q;
   float t[2][4];
@@ -66,20 +70,20 @@ __device__ __forceinline__ void push_rows32(uint32_t dst, uint32_t bar, const Pe
   q.y = __float_as_uint(hi ? t[0][3] : t[0][1]);
   q.z = __float_as_uint(hi ? t[1][2] : t[1][0]);
   q.w = __float_as_uint(hi ? t[1][3] : t[1][1]);
+  dst += row32(lane >> 1, lane & 1);
   uint32_t off = p.first;
-#pragma unroll
-  for (int c = 0; c < CTAS; ++c, off += p.step) send128(dst + lane * 16 + off, bar + off, q);
+#pragma unroll 4
+  for (int c = 0; c < n; ++c, off += p.step) send128(dst + off, bar + off, q);
 }
 
 // ---- weights of a unit in shared memory: 8 rows of K halves, padded by 16 bytes (K a multiple of 32: conflict-free)
 __host__ __device__ constexpr int unit_pitch(int K) { return K * 2 + 16; }
 __host__ __device__ constexpr int unit_bytes(int K) { return 8 * unit_pitch(K); }
-// lane r < 8 requests row r
-__device__ __forceinline__ void request_unit(uint32_t dst, const __half* w, int K, uint32_t bar, int lane) {
-  if (lane < 8)
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst + lane * unit_pitch(K)),
-                 "l"(w + lane * K), "r"(K * 2), "r"(bar)
-                 : "memory");
+// a warp requests a unit, whose rows follow one another in global memory
+__device__ __forceinline__ void request_unit(uint32_t dst, const __half* w, int K, int lane) {
+  for (int c = lane; c < K >> 3; c += 32)
+#pragma unroll
+    for (int r = 0; r < 8; ++r) cp_async16(dst + r * unit_pitch(K) + c * 16, w + r * K + c * 8, true);
 }
 
 // acc[u] (16 MT rows) += A[:, 0 .. K) W_u^T for NU units with their weights at w[u], rows w_pitch apart; act: the operand's first
@@ -116,23 +120,18 @@ __device__ __forceinline__ void mma_units(float (&acc)[NU][MT][4], uint32_t act,
   if (k < K) use(0);
 }
 
-// Bounded wait for bytes, by all lanes of a warp; SENT: they come from other CTAs.  A failure is recorded and later waits
-// return at once (the chain then runs through with what is there: the results of a launch whose status word is set are
-// garbage).
-template <bool SENT>
+// Bounded wait for the bytes that other CTAs send, by all lanes of a warp.  A failure is recorded and later waits return at
+// once (the chain then runs through with what is there: the results of a launch whose status word is set are garbage).
 __device__ __forceinline__ bool wait_bytes(uint32_t bar, uint32_t parity, volatile int* abort, int* status, int code) {
   for (uint32_t i = 0; i < tc5::kSpinLimit; ++i) {
     uint32_t ok;
-    if (SENT)
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t"
-          "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-          "selp.b32 %0, 1, 0, p;\n\t}"
-          : "=r"(ok)
-          : "r"(bar), "r"(parity)
-          : "memory");
-    else
-      ok = tc5::mbar_try_wait(bar, parity);
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
     if (__all_sync(0xffffffffu, ok)) return true;
     if (*abort) return false;
   }

@@ -5,7 +5,7 @@
 // own (gemm_small.cu, layernorm.cu) they cost 4-6 us each, nearly all of it launch, first loads and drain.  But rows do
 // not mix: a cluster of CTAs takes 16 rows through the whole chain (cluster_chain.cuh).  The LayerNorms add as
 // layernorm.cu does, every CTA its own copy of all rows, so a row's result does not depend on the batch around it.
-// Whole forward behind a graph, launches / this: 1 env d 192 143.5 / 139.6 us, d 256 118.8 / 114.7, d 128 57.8 / 55.5; 64
+// Whole forward behind a graph, launches / this with the blocks as they were: 1 env d 192 143.5 / 139.6 us, d 256 118.8 / 114.7, d 128 57.8 / 55.5; 64
 // envs d 192 192.1 / 186.5.  Eager, where eight launches take the host 14 us: 1 env d 192 162.6 / 149.0, d 64 78.0 / 61.9.
 // With more groups of rows than the device runs clusters at once the launches are faster: 256 envs d 192 221 / 253.
 #include "cluster_chain.cuh"
@@ -37,7 +37,6 @@ struct Params {
 };
 struct Shared {
   uint64_t in_full[STEPS];         // step i's bytes from all CTAs
-  uint64_t w_full[2][WARPS];
   int abort;
 };
 
@@ -55,8 +54,8 @@ __device__ __forceinline__ void norm_rows(const uint8_t* x, int r0, int r1, cons
   for (int i = 0; i < NV; ++i) {
     const int c = lane + i * 32;
     if (c < nvec) {
-      v[0][i] = *reinterpret_cast<const float4*>(x + (c >> 1) * UNIT32 + r0 * 32 + (c & 1) * 16);
-      v[1][i] = *reinterpret_cast<const float4*>(x + (c >> 1) * UNIT32 + r1 * 32 + (c & 1) * 16);
+      v[0][i] = *reinterpret_cast<const float4*>(x + (c >> 1) * UNIT32 + row32(r0, c & 1));
+      v[1][i] = *reinterpret_cast<const float4*>(x + (c >> 1) * UNIT32 + row32(r1, c & 1));
     }
   }
 #pragma unroll
@@ -116,8 +115,6 @@ __global__ void __launch_bounds__(THREADS, 1) readout_kernel(const __grid_consta
 
   if (tid == 0) {
     for (int i = 0; i < STEPS; ++i) tc5::mbar_init(smem_u32(&sh.in_full[i]), 1);
-    for (int b = 0; b < 2; ++b)
-      for (int w = 0; w < WARPS; ++w) tc5::mbar_init(smem_u32(&sh.w_full[b][w]), 1);
     sh.abort = 0;
     tc5::fence_barrier_init();
     // what arrives: step 0 the fp32 projection and the critic's fp16 one, 1 fc1, 2 fp32 fc2, 3 and 4 critic layers
@@ -129,20 +126,15 @@ __global__ void __launch_bounds__(THREADS, 1) readout_kernel(const __grid_consta
   // Units of step i in this CTA: every C-th one, the first product's first; the warps take them in turn.  A warp requests
   // its own units' weights (in the CTA's order in the set).
   auto request = [&](int is) {
-    if (*abort) return;
     const ReadoutMat &m0 = a.m[2 * is], &m1 = a.m[2 * is + 1];
     const int u0 = m0.n >> 3, units = u0 + (m1.n >> 3);
     const int mine0 = l.share[is][0] + (rank < l.share[is][1]);   // units of the first product in this CTA
-    const uint32_t bar = smem_u32(&sh.w_full[is & 1][warp]), set = base + l.w_set[is & 1];
-    int bytes = 0;
-    for (int j = warp, u = rank + warp * CTAS; u < units; j += WARPS, u += WARPS * CTAS) bytes += 16 * (u < u0 ? m0.k : m1.k);
-    if (lane == 0 && bytes) tc5::mbar_expect_tx(bar, bytes);
-    __syncwarp();
+    const uint32_t set = base + l.w_set[is & 1];
     for (int j = warp, u = rank + warp * CTAS; u < units; j += WARPS, u += WARPS * CTAS) {
-      if (u < u0) request_unit(set + j * unit_bytes(m0.k), m0.w + (int64_t)u * 8 * m0.k, m0.k, bar, lane);
-      else
-        request_unit(set + mine0 * unit_bytes(m0.k) + (j - mine0) * unit_bytes(m1.k), m1.w + (int64_t)(u - u0) * 8 * m1.k, m1.k, bar, lane);
+      if (u < u0) request_unit(set + j * unit_bytes(m0.k), m0.w + (int64_t)u * 8 * m0.k, m0.k, lane);
+      else request_unit(set + mine0 * unit_bytes(m0.k) + (j - mine0) * unit_bytes(m1.k), m1.w + (int64_t)(u - u0) * 8 * m1.k, m1.k, lane);
     }
+    cp_async_commit();
   };
   request(0);                                                // the weights are nobody's output
   {
@@ -171,13 +163,13 @@ __global__ void __launch_bounds__(THREADS, 1) readout_kernel(const __grid_consta
   __syncthreads();
 
   int prm_at = 0;
-  uint32_t w_phase = 0;                                      // bit b: phase of this warp's next weights in set b
 #pragma unroll 1
   for (int is = 0; is < STEPS; ++is) {
-    if (is > 0) wait_bytes<true>(smem_u32(&sh.in_full[is - 1]), 0, abort, s_args.status, KERNEL_ID * 16 + 1);
-    if (l.early && is + 1 < STEPS) {
+    if (is > 0) wait_bytes(smem_u32(&sh.in_full[is - 1]), 0, abort, s_args.status, KERNEL_ID * 16 + 1);
+    if (l.early) {
       if (is > 0) __syncthreads();                           // all warps are done with the step before: its set is free
-      request(is + 1);
+      if (is + 1 < STEPS) request(is + 1);
+      else cp_async_commit();
     }
     // ---- LayerNorm of xt in front of fc1 (into P) and of the heads and the critic (into H)
     if (is == 1 || is == 3) {
@@ -196,8 +188,9 @@ __global__ void __launch_bounds__(THREADS, 1) readout_kernel(const __grid_consta
     const int u0 = m0.n >> 3, units = u0 + (m1.n >> 3), mine0 = l.share[is][0] + (rank < l.share[is][1]);
     const uint32_t set = base + l.w_set[is & 1], bar = smem_u32(&sh.in_full[is]);
     const uint32_t op = base + (is == 0 ? l.in : is == 3 ? l.h : (is == 1 || is == 4) ? l.p : l.q);
-    if (rank + warp * CTAS < units && wait_bytes<false>(smem_u32(&sh.w_full[is & 1][warp]), (w_phase >> (is & 1)) & 1, abort, s_args.status, KERNEL_ID * 16 + 2))
-      w_phase ^= 1u << (is & 1);
+    if (l.early) cp_async_wait<1>();                           // all but the next step's weights
+    else cp_async_wait<0>();
+    __syncwarp();
 #pragma unroll 1
     for (int j = warp, u = rank + warp * CTAS; u < units; j += WARPS, u += WARPS * CTAS) {
       const bool second = u >= u0;
@@ -223,12 +216,12 @@ __global__ void __launch_bounds__(THREADS, 1) readout_kernel(const __grid_consta
         if (is == 2) {
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
-            const float2 x = *reinterpret_cast<const float2*>(smem + l.xt + (col >> 3) * UNIT32 + (g + 8 * hh) * 32 + tig * 8);
+            const float2 x = *reinterpret_cast<const float2*>(smem + l.xt + (col >> 3) * UNIT32 + row32(g + 8 * hh, tig >> 1) + (tig & 1) * 8);
             v[2 * hh] += x.x;
             v[2 * hh + 1] += x.y;
           }
         }
-        if (f32) push_rows32(base + l.xt + (col >> 3) * UNIT32, bar, peers, v, lane);
+        if (f32) push_rows32(base + l.xt + (col >> 3) * UNIT32, bar, peers, CTAS, v, lane);
         if (keep) {
           if (live[0]) *reinterpret_cast<float2*>(keep + row * ld + col) = make_float2(v[0], v[1]);
           if (live[1]) *reinterpret_cast<float2*>(keep + (row + 8) * ld + col) = make_float2(v[2], v[3]);
@@ -256,11 +249,8 @@ __global__ void __launch_bounds__(THREADS, 1) readout_kernel(const __grid_consta
   }
   __syncthreads();
   if (*abort) {
-    // weights in flight land (bounded), and nobody leaves while a peer may still send to it
-    for (int b = 0; lane == 0 && b < 2; ++b)
-      for (int i = 0; i < 4096 && !tc5::mbar_try_wait(smem_u32(&sh.w_full[b][warp]), (w_phase >> b) & 1); ++i) {}
-    __syncwarp();
-    tc5::cluster_sync_all();
+    cp_async_wait<0>();
+    tc5::cluster_sync_all();                                 // nobody leaves while a peer may still send to it
   }
 }
 
