@@ -131,12 +131,15 @@ __global__ void __launch_bounds__(THREADS, 1) blocks_small_kernel(const __grid_c
   const Peers peers = find_peers(base);
   tc5::cluster_sync_all();                                   // every CTA runs and has its barriers before anything is sent
   pdl_begin();
-  // the token stream (fp32), and block 0's LayerNorm rows where they are needed; rows past the 29th read as zero
-  for (int i = tid; i < ROWS * (d >> 2); i += THREADS) {
-    const int row = i / (d >> 2), c = i - row * (d >> 2);
-    const bool ok = row < kT;
-    cp_async16(base + l.x + (c >> 1) * UNIT32 + row32(row, c & 1), ok ? a.x0 + (env * kT + row) * d + c * 4 : a.x0, ok);
-  }
+  // the token stream (fp32) of this warp's own columns, which nobody else writes, and block 0's LayerNorm rows where they are
+  // needed; rows past the 29th read as zero.  The other columns of x arrive with step B's results, and a CTA without a head sends
+  // nothing before them that would hold its peers back until loads of its own had ended.
+  if (u0 < U)
+    for (int i = lane; i < 2 * ROWS; i += 32) {
+      const int row = i >> 1, half32 = i & 1;
+      const bool ok = row < kT;
+      cp_async16(base + l.x + u0 * UNIT32 + row32(row, half32), ok ? a.x0 + (env * kT + row) * d + u0 * 8 + half32 * 4 : a.x0, ok);
+    }
   if (has_head)
     for (int i = tid; i < ROWS * U; i += THREADS) {
       const int row = i / U, c = i - row * U;

@@ -4,9 +4,9 @@
 // Every CTA of the cluster holds all of the rows' activations in its shared memory and computes a share of every
 // product's output columns, which it sends into ALL of the CTAs' copies (st.async); a receiving CTA counts the bytes on
 // an mbarrier and goes on when the step's are complete.  Nothing else orders the CTAs: a step's data goes to buffers
-// that no CTA can still be reading, because whoever sends it has received what those readers sent after their reads.
-// (With a barrier of the cluster instead, a step pays 850 cycles for the release; exchanged through L2, another 900 for
-// the operand's loads.)
+// that no CTA can still be reading or filling itself, because whoever sends it has received what those CTAs sent after
+// their reads and loads; what a CTA fills before it has sent anything is written by nobody else.  (With a barrier of the
+// cluster instead, a step pays 850 cycles for the release; exchanged through L2, another 900 for the operand's loads.)
 //
 // A unit is 8 output columns of a product: one warp's work.  The warp copies its 8 weight rows itself, 16 bytes apart
 // in bank, as a rule a step ahead of their use (a group of cp.async per step; a bulk copy per row costs its issuer 100

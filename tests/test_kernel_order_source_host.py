@@ -53,3 +53,17 @@ def test_copied_operands_go_to_a_kernel_that_waits_for_them():
         assert call is None or call.group(1) in (None, "linear_mma"), part[:200]
     body = _sources()["gemm_mma.cu"].split("linear_mma_kernel(LinearArgs p) {")[1]
     assert body.lstrip().startswith("pdl_begin();")
+
+
+def test_a_cluster_loads_nothing_that_a_peer_may_already_be_writing():
+    """The blocks' chain starts with loads into shared memory that peers send results into.  Step B's rows go to every CTA as soon
+    as the heads' outputs are there, and with 2 H < 16 some CTA sends nothing before: nobody knows whether its loads have ended.
+    So a warp loads only the columns of x that it sends itself (unit rank + 16 warp), after the cluster's only barrier."""
+    kernel = _sources()["blocks_small.cu"].split("blocks_small_kernel(const __grid_constant__ Params args) {")[1]
+    start = kernel.split("pdl_begin();")[1].split("cp_async_wait<0>();")[0]
+    targets = re.findall(r"cp_async16\(base \+ l\.(\w+) \+ ([^,]*),", start)
+    assert [t for t, _ in targets] == ["x", "h"], targets           # h is written by its own CTA only
+    assert targets[0][1].startswith("u0 * UNIT32 + row32(row"), targets[0]
+    assert re.search(r"if \(u0 < U\)\s*for \(int i = lane; i < 2 \* ROWS; i \+= 32\) \{[^}]*cp_async16\(base \+ l\.x", start)
+    assert "const int u0 = rank + warp * CTAS" in kernel
+    assert not re.search(r"(push_rows|send128)\w*\(base \+ l\.h\b", kernel)
