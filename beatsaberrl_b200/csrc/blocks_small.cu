@@ -15,6 +15,7 @@
 // What took most and went: a bulk copy per weight row (100 cycles each for its issuer), LayerNorm by units along a row
 // (8-way bank conflicts), a head's 29 rows sent to 16 CTAs by one: 124.9 -> 106.6 us together.
 #include <atomic>
+#include <cstddef>
 #include <type_traits>
 
 #include "attend.cuh"
@@ -40,10 +41,11 @@ struct Params {
 struct Shared {
   uint64_t in_full[4];
   float2 norm[ROWS];               // per row: 1 / deviation, -mean / deviation
-  float norm_w[2 * MAX_D];         // the next LayerNorm's gamma | beta
+  alignas(16) float norm_w[2 * MAX_D];         // the next LayerNorm's gamma | beta: copied and read 16 bytes at a time
   BlockPtrs block[kMaxSmallBlocks];
   int abort;
 };
+static_assert(alignof(Shared) % 16 == 0 && offsetof(Shared, norm_w) % 16 == 0, "16-byte copies of the LayerNorm weights");
 
 // q|k|v of one head in rows of LDQ bytes, and its output in rows of LDO
 template <int DH>
