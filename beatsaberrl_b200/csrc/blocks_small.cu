@@ -421,7 +421,7 @@ int run(const Params& p, int64_t n_envs, cudaStream_t stream) {
 }  // namespace
 
 int chain::resident_clusters() {
-  static std::atomic<int> cached[kMaxDevices];               // count + 1; 0 = not read yet: racing first readers store the same value
+  static std::atomic<int> cached[kMaxDevices];               // count + 1; 0 = not known: racing first readers store the same value
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 0;
   int n = cached[dev].load(std::memory_order_relaxed);
@@ -438,7 +438,7 @@ int chain::resident_clusters() {
     cfg.numAttrs = 1;
     if (set_up<32>() != BSRL_OK || cudaOccupancyMaxActiveClusters(&n, blocks_small_kernel<32>, &cfg) != cudaSuccess || n < 0) {
       cudaGetLastError();
-      n = 0;
+      return 0;                                              // asked again next time: a failure says nothing about the device
     }
     cached[dev].store(++n, std::memory_order_relaxed);
   }

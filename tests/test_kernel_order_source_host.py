@@ -67,3 +67,11 @@ def test_a_cluster_loads_nothing_that_a_peer_may_already_be_writing():
     assert re.search(r"if \(u0 < U\)\s*for \(int i = lane; i < 2 \* ROWS; i \+= 32\) \{[^}]*cp_async16\(base \+ l\.x", start)
     assert "const int u0 = rank + warp * CTAS" in kernel
     assert not re.search(r"(push_rows|send128)\w*\(base \+ l\.h\b", kernel)
+
+
+def test_a_failed_count_of_resident_clusters_is_not_kept():
+    """With no count the few-environment launches serve the call; one failed query must not decide that for the process."""
+    body = _sources()["blocks_small.cu"].split("int chain::resident_clusters() {")[1].split("\n}")[0]
+    failed = body.split("cudaGetLastError();")[1].split("}")[0]
+    assert failed.strip().startswith("return 0;"), failed
+    assert body.index("cudaGetLastError();") < body.index(".store(")
