@@ -729,7 +729,10 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         for (int hb = 0; hb < 32 / CB; ++hb, ++k) {
           if (!mbar_wait_warp(smem_u32(&sh->io_full[warp - 2][b]), (io_phase >> b) & 1, abort)) {
             if (lane == 0) give_up(sh, p.status, 15);
-            n_early = 0;
+            // the loop at the end awaits this block and those requested behind it; the other buffers' last phases are over
+            n_early = 3;
+            for (int i = k; i < k + 3; ++i)
+              if (i >= nb) io_phase ^= 1u << (i % 3);
             return false;
           }
           io_phase ^= 1u << b;
@@ -943,7 +946,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
       }
       tc_fence_before();
     }
-    // residual blocks requested ahead of a pre-store that a wait above kept from running land before the CTA exits (bounded, ignoring abort)
+    // residual blocks that a failed wait above left on their way land before the CTA exits (bounded, ignoring abort)
     for (int k = 0; lane == 0 && k < n_early; ++k) {
       uint32_t spins = 0;
       while (!mbar_try_wait(smem_u32(&sh->io_full[warp - 2][k]), (io_phase >> k) & 1) && ++spins < kSpinLimit) {}

@@ -75,3 +75,15 @@ def test_a_failed_count_of_resident_clusters_is_not_kept():
     failed = body.split("cudaGetLastError();")[1].split("}")[0]
     assert failed.strip().startswith("return 0;"), failed
     assert body.index("cudaGetLastError();") < body.index(".store(")
+
+
+def test_residual_blocks_on_their_way_are_awaited_before_the_block_tail_exits():
+    """A CTA that gives up a wait must not exit under copies into its shared memory: whatever a pre-store requested and did not
+    consume -- a failed wait in the middle of it included -- is awaited, with a limit, buffer by buffer at the end."""
+    src = _sources()["block_tail_tc5.cu"]
+    prestore = src.split("auto prestore_tma = [&]")[1].split("    };\n")[0]
+    assert "k = n_early; k < 3 && k < nb" in prestore and "if (k + 3 < nb) issue_block(t, k + 3);" in prestore    # three on their way
+    failed = re.sub(r"\s+", " ", prestore.split("give_up(")[1].split("return false;")[0])
+    assert "n_early = 3; for (int i = k; i < k + 3; ++i) if (i >= nb) io_phase ^= 1u << (i % 3);" in failed
+    end = src.split("bounded, ignoring abort)\n    for (int k = 0; lane == 0 && k < n_early; ++k)")[1].split("bulk_wait_all();")[0]
+    assert "io_full[warp - 2][k]), (io_phase >> k) & 1)" in end and "kSpinLimit" in end
