@@ -209,31 +209,42 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
 }
 
 // erf-based GELU, 0.5 x (1 + erf(x / sqrt 2)): torch.nn.GELU() with its default approximate='none'.
-// x Phi(x) = max(x, 0) - |x| Phi(-|x|) with Phi(-a) = 2^q(a), q a polynomial of degree 8: the minimax fit (a linear
-// programme over Chebyshev nodes of [0, 6.2], this file's own) of log2 Phi(-a), weighted so that the result's absolute
-// error is below 1e-7 x and the relative error of its negative branch below 2e-5.  Past 6.2 the leading coefficient takes
-// q to minus infinity.  One special-function instruction and nine FMAs per element, the FMAs two elements at a time.
-// Against float64 over [-12, 12], this / the rational-exponential form 7.1.26 of Abramowitz & Stegun with a reciprocal and
-// an exponential: largest error 2.4e-7 / 3.3e-7, rms 4.2e-8 / 7.6e-8, relative on [-4, 0) 1.2e-5 / 4.7e-4; of results
-// rounded to fp16, 0.3 % / 2.8 % differ from the rounded exact value.   65,536 environments of 33 tokens at d 256: 18.98 -> 17.79 ms
-// per forward; 4,095 of 65 at d 512 (the FFN-up's epilogue took longer than its MMAs): 14.08 -> 12.38 ms before the power
-// cap sets in, 14.52 -> 13.71 in a loop.
+// x Phi(x) = max(x, 0) - |x| Phi(-|x|) with Phi(-a) = 2^q(a), q a polynomial: minimax fits (linear programmes over Chebyshev
+// nodes, this file's own) of log2 Phi(-a), whose negative leading coefficients take q to minus infinity past the fit.  One
+// special-function instruction per element.
+// Results that are rounded to fp16: degree 8, fitted to [0, 6.2] for an absolute error below 1e-7 x and, down to x = -4, a
+// relative error of the negative branch below 2e-5.  Past -4 that grows (2.5e-4 at -4.5, 2e-3 at -5, 3.5e-2 at -6, all of the
+// result past -8), which is 1.2e-8 at most there: a fifth of fp16's smallest step.  FMAs two elements at a time.
+// fp32 results: degree 12, fitted to [0, 12.9], where the result itself runs out of fp32: relative error of the negative branch
+// below 6e-7 to -2, 5e-6 to -4, 4e-5 to -6, 3e-4 to -8, 1e-3 to -10, 9e-3 to -12.9.
+// In fp32 against float64 over [-12.9, 12.9], degree 8 / degree 12 / the rational-exponential form 7.1.26 of Abramowitz & Stegun
+// with a reciprocal and an exponential: largest error 2.4e-7 / 2.4e-7 / 3.3e-7, rms 4.1e-8 / 4.0e-8 / 7.3e-8, relative on [-4, 0)
+// 1.1e-5 / 5.0e-6 / 4.7e-4, on [-8, -4) 0.72 / 2.9e-4 / 1.0e-2; of results rounded to fp16, 0.3 % / - / 2.8 % differ from the
+// rounded exact value.  Degree 8 against 7.1.26: 65,536 environments of 33 tokens at d 256 18.98 -> 17.79 ms per forward; 4,095
+// of 65 at d 512 (the FFN-up's epilogue took longer than its MMAs): 14.08 -> 12.38 ms before the power cap sets in, 14.52 ->
+// 13.71 in a loop.
 __device__ constexpr float kGeluQ[9] = {-9.99999744e-01f, -1.15111655e+00f, -4.59124456e-01f, -5.27288577e-02f, 7.37600707e-03f,
                                         -3.61215035e-04f, -9.85613870e-05f, 2.18674498e-05f, -1.43885577e-06f};
+__device__ constexpr float kGeluQ32[13] = {-1.00000000e+00f, -1.15110564e+00f, -4.59209889e-01f, -5.24704345e-02f, 6.98015373e-03f,
+                                           -1.46172151e-05f, -2.82148336e-04f, 8.17496766e-05f, -1.33107760e-05f, 1.37389475e-06f,
+                                           -8.84585063e-08f, 3.23252669e-09f, -5.10666856e-11f};
 __device__ __forceinline__ float gelu_ex2(float q) {
   float e;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(q));
   return e;
 }
-__device__ __forceinline__ float gelu_exact(float x) {
+template <int N>
+__device__ __forceinline__ float gelu_of(float x, const float (&c)[N]) {
   const float a = fabsf(x);
-  float q = kGeluQ[8];
+  float q = c[N - 1];
 #pragma unroll
-  for (int i = 7; i >= 0; --i) q = fmaf(q, a, kGeluQ[i]);
+  for (int i = N - 2; i >= 0; --i) q = fmaf(q, a, c[i]);
   return fmaf(-a, gelu_ex2(q), fmaxf(x, 0.f));
 }
-// the same, two at a time (bit for bit)
-__device__ __forceinline__ void gelu_exact2(float& x0, float& x1) {
+__device__ __forceinline__ float gelu_f16(float x) { return gelu_of(x, kGeluQ); }      // rounded to fp16 by the caller
+__device__ __forceinline__ float gelu_f32(float x) { return gelu_of(x, kGeluQ32); }
+// gelu_f16, two at a time (bit for bit)
+__device__ __forceinline__ void gelu2_f16(float& x0, float& x1) {
   const uint64_t a = f2_make(fabsf(x0), fabsf(x1));
   uint64_t q = f2_make(kGeluQ[8], kGeluQ[8]);
 #pragma unroll

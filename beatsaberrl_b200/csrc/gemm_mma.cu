@@ -128,8 +128,8 @@ __global__ void __launch_bounds__(THREADS) linear_mma_kernel(LinearArgs p) {
           v0 = fmaxf(v0, 0.f);
           v1 = fmaxf(v1, 0.f);
         } else if (p.relu == 2) {
-          v0 = gelu_exact(v0);
-          v1 = gelu_exact(v1);
+          v0 = p.out_f32 ? gelu_f32(v0) : gelu_f16(v0);
+          v1 = p.out_f32 ? gelu_f32(v1) : gelu_f16(v1);
         }
         if (rrow) {
           float2 r = *reinterpret_cast<const float2*>(rrow + col);

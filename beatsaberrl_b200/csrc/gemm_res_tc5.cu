@@ -239,12 +239,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(fmaxf(__uint_as_float(a[j]), 0.f));
       } else if (p.relu == 2) {
 #pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-          float v0 = __uint_as_float(a[j]), v1 = __uint_as_float(a[j + 1]);
-          gelu_exact2(v0, v1);
-          a[j] = __float_as_uint(v0);
-          a[j + 1] = __float_as_uint(v1);
-        }
+        for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(p.out_f32 ? gelu_f32(__uint_as_float(a[j])) : gelu_f16(__uint_as_float(a[j])));
       }
     };
     uint32_t tile_i = 0;
@@ -365,7 +360,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                   v0 = fmaxf(v0, 0.f);
                   v1 = fmaxf(v1, 0.f);
                 } else if (p.relu == 2) {
-                  gelu_exact2(v0, v1);
+                  gelu2_f16(v0, v1);
                 }
                 h[4 * i + u] = pack_half2(v0, v1);
               }

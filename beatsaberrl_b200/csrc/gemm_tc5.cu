@@ -286,7 +286,10 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
           } else if (p.relu == 2) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) gelu_exact2(v[j], v[j + 1]);
+            for (int j = 0; j < 32; j += 2) {
+              if (p.out_f32) v[j] = gelu_f32(v[j]), v[j + 1] = gelu_f32(v[j + 1]);
+              else gelu2_f16(v[j], v[j + 1]);
+            }
           }
           if (masked) {
 #pragma unroll
