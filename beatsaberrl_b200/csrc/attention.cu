@@ -158,18 +158,19 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
 // Token counts of the form 1 + 16 k (the single-body-token layouts: 17 / 33 / 65): the object tokens fill
 // whole 16-row MMA tiles, and only the body token (row 0 of the env) would force a padded tile on both the
 // query and the key side -- at 33 tokens the padded problem is 48 x 64 against 32 x 32, three times the MMAs.
-// So the MMAs run over the object tokens alone and the body token is folded in on the CUDA cores:
-//   * its key: one extra score column s0[i] = q_i . k_0 (a dot product per query row) joins the row's softmax,
-//     and its probability adds p0[i] v_0 to the row's output;
-//   * its query row: 1 x tokens scores, a warp-wide softmax and a tokens-long weighted sum of the v rows.
+// So the MMAs run over whole tiles of object tokens and the body token joins them:
+//   * its key: the scores q_i . k_0 are one more MMA per 16 columns and query tile (k_0 as one key of a tile of eight); on the
+//     CUDA cores they join the row's softmax, and p_0 v_0 is where the row's P V accumulators start;
+//   * its query row: its scores are MMAs too (q_0 as all 16 rows of a tile); the softmax across the warp, one key per lane, and
+//     the weighted sum of the v rows are done on the CUDA cores.
 // n_q = tokens (every row) or 1 (the body row only: the last block's readout).  Same arithmetic as
 // attn29_kernel: fp32 scores and softmax, masked keys exactly 0, probabilities rounded to fp16 only where
 // they enter an MMA.
 // TEAM: warps per (env, head) -- two where the pair's tile is so large (24 KB at 64 tokens x 64) that one warp each left two
 // per scheduler; each takes half of the object query rows and, for the body row, half of the object keys.
-// Bound by the turns of the shared-memory pipe and by what is done per lane for the body token; so its scores -- q_0 k_j and
-// q_i k_0 -- are products on the tensor cores too (q_0 as all 16 rows of a tile, k_0 as one key of a tile of eight), a
-// K or V fragment serves both query tiles of a warp, and rows are dense and swizzled.
+// Bound by the turns of the shared-memory pipe and by what is done per lane for the body token; so its scores went to the
+// tensor cores (before: dot products on the CUDA cores; error against float64 the same to six digits), a K or V fragment serves
+// both query tiles of a warp, and rows are dense and swizzled.
 // One B200, us, before / now (at copy speed): 4,095 environments of 65 tokens, 8 heads of 64: 295 / 244 (167), the body row only
 // 121 / 92 (84); 4,096 of 33 tokens, 8 heads of 32: 78 / 72 (42); of 17, 4 heads of 32: 25 / 19 (11).
 template <int DH, int NOBJ, int TEAM>

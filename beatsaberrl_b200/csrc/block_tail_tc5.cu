@@ -621,7 +621,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
     // A stmatrix_x4 takes 8 rows x 32 columns: lane t gives the address of piece t / 8 of row t % 8.
     const int fr = lane >> 2, fc = 2 * (lane & 3), st_row = lane & 7, st_piece = lane >> 3;
     const uint64_t* prm_frag = reinterpret_cast<const uint64_t*>(prm + fc);      // parameter pair of 8-column unit u of vector v: [128 v + 4 u]
-    // body(c, r) for the 32-column blocks of [c_lo, c_lo + d / 2): load(c, r) requests a block while the one before it is worked on
+    // the 32-column blocks of [c_lo, c_lo + d / 2), one after another: load(c, r), then body(c, r) on what has arrived
     auto each_block = [&](auto&& load, auto&& body) {
       for (int c = c_lo; c < c_lo + dh2; c += 32) {
         uint32_t r[32];

@@ -10,10 +10,11 @@
 // each with its output columns spread over the CTAs in units of 8.  The arithmetic is that of the launches (attend.cuh,
 // row_norm.cuh, the sums of linear_small_block), bit for bit: a batch size does not change a row's result.
 // Whole forward behind a graph, launches / this (with readout.cu): one env d 64 49.1 / 41.0 us, d 128 57.4 / 47.1, d 192 (6
-// blocks) 143.4 / 106.6, d 256 117.3 / 93.2; seven at d 192 157.8 / 112.8.  Some 12 us per block remain (d 192), nearly all of it
+// blocks) 143.4 / 105.4, d 256 117.3 / 92.2; seven at d 192 157.8 / 112.4.  Some 12 us per block remain (d 192), nearly all of it
 // latency: a step's results into 16 CTAs (0.7 us, bound by the senders' 32 B per clock), LayerNorm, short chains of MMAs.
 // What took most and went: a bulk copy per weight row (100 cycles each for its issuer), LayerNorm by units along a row
-// (8-way bank conflicts), a head's 29 rows sent to 16 CTAs by one: 124.9 -> 106.6 us together.
+// (8-way bank conflicts), a head's 29 rows sent to 16 CTAs by one: 124.9 -> 106.6 us together.  (Only a warp's own columns
+// of x loaded: 106.6 -> 105.4.)
 #include <atomic>
 #include <cstddef>
 #include <type_traits>

@@ -186,13 +186,13 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
     auto finish = [&](uint32_t (&a)[32], int col) {
       if (p.bias) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float4 bv = *reinterpret_cast<const float4*>(p.bias + col + 4 * j);
-        a[4 * j] = __float_as_uint(__uint_as_float(a[4 * j]) + bv.x);
-        a[4 * j + 1] = __float_as_uint(__uint_as_float(a[4 * j + 1]) + bv.y);
-        a[4 * j + 2] = __float_as_uint(__uint_as_float(a[4 * j + 2]) + bv.z);
-        a[4 * j + 3] = __float_as_uint(__uint_as_float(a[4 * j + 3]) + bv.w);
-      }
+        for (int j = 0; j < 8; ++j) {
+          const float4 bv = *reinterpret_cast<const float4*>(p.bias + col + 4 * j);
+          a[4 * j] = __float_as_uint(__uint_as_float(a[4 * j]) + bv.x);
+          a[4 * j + 1] = __float_as_uint(__uint_as_float(a[4 * j + 1]) + bv.y);
+          a[4 * j + 2] = __float_as_uint(__uint_as_float(a[4 * j + 2]) + bv.z);
+          a[4 * j + 3] = __float_as_uint(__uint_as_float(a[4 * j + 3]) + bv.w);
+        }
       }
       if (p.relu == 1) {
 #pragma unroll

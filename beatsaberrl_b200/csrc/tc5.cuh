@@ -1,6 +1,6 @@
 // Blackwell (sm_100a) primitives used by the tcgen05 kernels: mbarrier with bounded waits,
-// TMA tile loads (each CTA fetches its own tiles, no multicast; clusters only as CTA pairs), TMEM allocation, tcgen05.mma / ld / commit,
-// shared-memory and instruction descriptors.
+// TMA tile loads (each CTA fetches its own tiles, no multicast), clusters (CTA pairs here; 16 CTAs in cluster_chain.cuh), TMEM
+// allocation, tcgen05.mma / ld / commit, shared-memory and instruction descriptors.
 #pragma once
 #include <cuda.h>
 
