@@ -832,7 +832,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
                 float a0, a1;
                 f2_split(f2_add(frag_pair(r[c], i, u), b0), a0, a1);
                 if (GELU) {
-                  gelu2_f16(a0, a1);
+                  gelu2<false>(a0, a1);
                   hp[c][i][u] = pack_half2(a0, a1);
                 } else {
                   hp[c][i][u] = pack_half2(fmaxf(a0, 0.f), fmaxf(a1, 0.f));

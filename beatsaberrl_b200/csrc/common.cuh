@@ -243,12 +243,15 @@ __device__ __forceinline__ float gelu_of(float x, const float (&c)[N]) {
 }
 __device__ __forceinline__ float gelu_f16(float x) { return gelu_of(x, kGeluQ); }      // rounded to fp16 by the caller
 __device__ __forceinline__ float gelu_f32(float x) { return gelu_of(x, kGeluQ32); }
-// gelu_f16, two at a time (bit for bit)
-__device__ __forceinline__ void gelu2_f16(float& x0, float& x1) {
+// the same, two at a time (bit for bit)
+template <bool F32>
+__device__ __forceinline__ void gelu2(float& x0, float& x1) {
+  constexpr int N = F32 ? 13 : 9;
   const uint64_t a = f2_make(fabsf(x0), fabsf(x1));
-  uint64_t q = f2_make(kGeluQ[8], kGeluQ[8]);
+  auto c = [](int i) { return F32 ? kGeluQ32[i] : kGeluQ[i]; };
+  uint64_t q = f2_make(c(N - 1), c(N - 1));
 #pragma unroll
-  for (int i = 7; i >= 0; --i) q = f2_fma(q, a, f2_make(kGeluQ[i], kGeluQ[i]));
+  for (int i = N - 2; i >= 0; --i) q = f2_fma(q, a, f2_make(c(i), c(i)));
   float q0, q1;
   f2_split(q, q0, q1);
   f2_split(f2_fma(f2_make(-fabsf(x0), -fabsf(x1)), f2_make(gelu_ex2(q0), gelu_ex2(q1)), f2_make(fmaxf(x0, 0.f), fmaxf(x1, 0.f))), x0, x1);

@@ -22,6 +22,8 @@ __device__ __forceinline__ uint32_t tile_off(int row, int kc) {
   return static_cast<uint32_t>((row * 4 + (kc ^ ((row >> 1) & 3))) * 16);
 }
 
+// GELU32: a kernel of its own for GELU of fp32 results (see gemm_tc5.cu)
+template <bool GELU32>
 __global__ void __launch_bounds__(THREADS) linear_mma_kernel(LinearArgs p) {
   pdl_begin();
   extern __shared__ __align__(128) uint8_t smem[];
@@ -128,8 +130,8 @@ __global__ void __launch_bounds__(THREADS) linear_mma_kernel(LinearArgs p) {
           v0 = fmaxf(v0, 0.f);
           v1 = fmaxf(v1, 0.f);
         } else if (p.relu == 2) {
-          v0 = p.out_f32 ? gelu_f32(v0) : gelu_f16(v0);
-          v1 = p.out_f32 ? gelu_f32(v1) : gelu_f16(v1);
+          v0 = GELU32 ? gelu_f32(v0) : gelu_f16(v0);
+          v1 = GELU32 ? gelu_f32(v1) : gelu_f16(v1);
         }
         if (rrow) {
           float2 r = *reinterpret_cast<const float2*>(rrow + col);
@@ -165,7 +167,10 @@ int linear_mma(const LinearArgs& p, cudaStream_t stream) {
   if (p.M == 0) return BSRL_OK;
   static DeviceOnce once;
   int rc = once.run("linear_mma_kernel set-up", [] {
-    return cudaFuncSetAttribute(linear_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGES * STAGE_BYTES);
+    cudaError_t e = cudaSuccess;
+    for (auto* k : {linear_mma_kernel<false>, linear_mma_kernel<true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGES * STAGE_BYTES);
+    return e;
   });
   if (rc != BSRL_OK) return rc;
   int64_t tiles = ((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN);
@@ -173,7 +178,7 @@ int linear_mma(const LinearArgs& p, cudaStream_t stream) {
     set_error("linear: too many tiles");
     return BSRL_ERR_SHAPE;
   }
-  launch_kernel(linear_mma_kernel, static_cast<unsigned>(tiles), THREADS, STAGES * STAGE_BYTES, stream, p);
+  launch_kernel(p.relu == 2 && p.out_f32 ? linear_mma_kernel<true> : linear_mma_kernel<false>, static_cast<unsigned>(tiles), THREADS, STAGES * STAGE_BYTES, stream, p);
   BSRL_LAUNCH_OK("linear_mma_kernel");
   return BSRL_OK;
 }

@@ -69,7 +69,8 @@ __device__ __forceinline__ uint32_t keep_positive(uint32_t h, uint32_t mask) {
   return h;
 }
 
-template <bool HAS_R>
+// GELU32: GELU of an fp32 result (gelu_f32), a kernel of its own: compiled into the others it cost updates 1 % by its size alone
+template <bool HAS_R, bool GELU32 = false>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                    const __grid_constant__ CUtensorMap tm_c, int box_rows, int r32, LinearArgs p, int m_pairs, int n_tiles, int* status) {
@@ -199,7 +200,12 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
         for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(fmaxf(__uint_as_float(a[j]), 0.f));
       } else if (p.relu == 2) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(p.out_f32 ? gelu_f32(__uint_as_float(a[j])) : gelu_f16(__uint_as_float(a[j])));
+        for (int j = 0; j < 32; j += 2) {
+          float v0 = __uint_as_float(a[j]), v1 = __uint_as_float(a[j + 1]);
+          gelu2<GELU32>(v0, v1);
+          a[j] = __float_as_uint(v0);
+          a[j + 1] = __float_as_uint(v1);
+        }
       }
     };
     uint32_t tile_i = 0;
@@ -285,7 +291,7 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
                   v0 = fmaxf(v0, 0.f);
                   v1 = fmaxf(v1, 0.f);
                 } else if (p.relu == 2) {
-                  gelu2_f16(v0, v1);
+                  gelu2<false>(v0, v1);
                 }
                 h[i][u] = pack_half2(v0, v1);
               }
@@ -379,13 +385,16 @@ int linear_pair(const LinearArgs& p, cudaStream_t stream) {
   if (!make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, box_rows == 32 ? p.M : p.cmap(p.M - 1) + 1, p.N, p.ldc, box_rows, 128)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("linear_pair_kernel set-up", [] {
-    cudaError_t e = cudaFuncSetAttribute(linear_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(linear_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaSuccess;
+    for (auto* k : {linear_pair_kernel<false>, linear_pair_kernel<true>, linear_pair_kernel<false, true>, linear_pair_kernel<true, true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    return e;
   });
   if (rc != BSRL_OK) return rc;
   const int m_pairs = (int)((p.M + 2 * BM - 1) / (2 * BM)), n_tiles = p.N / BN;
   const int r32 = p.R && reinterpret_cast<uintptr_t>(p.R) % 32 == 0 && p.ldr % 8 == 0;        // 32-byte residual loads
-  auto* kernel = p.R ? linear_pair_kernel<true> : linear_pair_kernel<false>;
+  const bool gelu32 = p.relu == 2 && p.out_f32;
+  auto* kernel = gelu32 ? (p.R ? linear_pair_kernel<true, true> : linear_pair_kernel<false, true>) : p.R ? linear_pair_kernel<true> : linear_pair_kernel<false>;
   launch_kernel<2>(kernel, (unsigned)(sm_count() & ~1), THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, box_rows, r32, p, m_pairs, n_tiles, status);
   BSRL_LAUNCH_OK("linear_pair_kernel");
   return BSRL_OK;

@@ -89,7 +89,8 @@ __device__ __forceinline__ uint32_t positive_bits(const uint32_t* h) {
 // pair i's halves of a packed gradient, zeroed where their bits are
 __device__ __forceinline__ uint32_t keep_positive(uint32_t h, uint32_t w, int i) { return h & (((w >> i) & 0x00010001u) * 0xffffu); }
 
-template <bool HAS_R>
+// GELU32: GELU of an fp32 result (gelu_f32), a kernel of its own: compiled into the others it cost updates 1 % by its size alone
+template <bool HAS_R, bool GELU32 = false>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                   const __grid_constant__ CUtensorMap tm_c, int tma_c, int r32, LinearArgs p, int bn, int m_tiles, int n_tiles,
@@ -239,7 +240,12 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(fmaxf(__uint_as_float(a[j]), 0.f));
       } else if (p.relu == 2) {
 #pragma unroll
-        for (int j = 0; j < 32; ++j) a[j] = __float_as_uint(p.out_f32 ? gelu_f32(__uint_as_float(a[j])) : gelu_f16(__uint_as_float(a[j])));
+        for (int j = 0; j < 32; j += 2) {
+          float v0 = __uint_as_float(a[j]), v1 = __uint_as_float(a[j + 1]);
+          gelu2<GELU32>(v0, v1);
+          a[j] = __float_as_uint(v0);
+          a[j + 1] = __float_as_uint(v1);
+        }
       }
     };
     uint32_t tile_i = 0;
@@ -360,7 +366,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
                   v0 = fmaxf(v0, 0.f);
                   v1 = fmaxf(v1, 0.f);
                 } else if (p.relu == 2) {
-                  gelu2_f16(v0, v1);
+                  gelu2<false>(v0, v1);
                 }
                 h[4 * i + u] = pack_half2(v0, v1);
               }
@@ -434,14 +440,17 @@ int linear_res(const LinearArgs& p, cudaStream_t stream) {
   if (tma_c && !make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, tma_c == 32 ? p.M : p.cmap(p.M - 1) + 1, p.N, p.ldc, tma_c, 128)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("linear_res_kernel set-up", [] {
-    cudaError_t e = cudaFuncSetAttribute(linear_res_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    return e != cudaSuccess ? e : cudaFuncSetAttribute(linear_res_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaSuccess;
+    for (auto* k : {linear_res_kernel<false>, linear_res_kernel<true>, linear_res_kernel<false, true>, linear_res_kernel<true, true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    return e;
   });
   if (rc != BSRL_OK) return rc;
   const int bn = res_cols(p.N);
   const int m_tiles = (int)((p.M + 2 * BM - 1) / (2 * BM)), n_tiles = (p.N + bn - 1) / bn;
   const int r32 = p.R && reinterpret_cast<uintptr_t>(p.R) % 32 == 0 && p.ldr % 8 == 0;        // 32-byte residual loads
-  auto* kernel = p.R ? linear_res_kernel<true> : linear_res_kernel<false>;
+  const bool gelu32 = p.relu == 2 && p.out_f32;
+  auto* kernel = gelu32 ? (p.R ? linear_res_kernel<true, true> : linear_res_kernel<false, true>) : p.R ? linear_res_kernel<true> : linear_res_kernel<false>;
   launch_kernel<2>(kernel, (unsigned)(sm_count() & ~1), THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, tma_c, r32, p, bn, m_tiles, n_tiles, status);
   BSRL_LAUNCH_OK("linear_res_kernel");
   return BSRL_OK;

@@ -35,7 +35,8 @@ struct SmallArgs {
 // TM x TN output tile, one warp per 16 x 8 piece of it (a dependent chain of MMAs: 25 cycles per K step of 16)
 // NORM: the A operand is the LayerNorm of fp32 rows, made in shared memory (every column tile's CTA makes its own; all of
 // K is resident)
-template <int TM, int TN, bool NORM>
+// GELU32: a kernel of its own for GELU of fp32 results (see gemm_tc5.cu); no block product stores these
+template <int TM, int TN, bool NORM, bool GELU32 = false>
 __global__ void __launch_bounds__(TM * TN / 4) linear_small_kernel(const __grid_constant__ SmallArgs args) {
   constexpr int THREADS = TM * TN / 4, STAGE_BYTES = (TM + TN) * ROW_BYTES;
   extern __shared__ __align__(128) uint8_t smem[];
@@ -168,8 +169,8 @@ __global__ void __launch_bounds__(TM * TN / 4) linear_small_kernel(const __grid_
       v0 = fmaxf(v0, 0.f);
       v1 = fmaxf(v1, 0.f);
     } else if (p.relu == 2) {
-      v0 = p.out_f32 ? gelu_f32(v0) : gelu_f16(v0);
-      v1 = p.out_f32 ? gelu_f32(v1) : gelu_f16(v1);
+      v0 = GELU32 && p.out_f32 ? gelu_f32(v0) : gelu_f16(v0);
+      v1 = GELU32 && p.out_f32 ? gelu_f32(v1) : gelu_f16(v1);
     }
     if (rrow) {
       const float2 r = *reinterpret_cast<const float2*>(rrow + col);
@@ -190,6 +191,7 @@ struct Tile {
     return chunks < MAX_STAGES ? chunks : MAX_STAGES;
   }
   static int64_t tiles(const LinearArgs& p) { return (p.M + TM - 1) / TM * ((p.N + TN - 1) / TN); }
+  static bool gelu32(const LinearArgs& p) { return p.relu == 2 && p.out_f32; }
   static int norm_bytes(int d) { return TM * (d + 4) * 4 + 2 * TM * 8; }
   static bool one_wave(const LinearArgs& p, bool norm = false) {      // every tile has a place on the chip at once
     const int by_smem = 227 * 1024 / (stages(p) * STAGE_BYTES + (norm ? norm_bytes(p.K) : 0) + 1024), by_threads = 2048 / THREADS;
@@ -199,6 +201,7 @@ struct Tile {
     static DeviceOnce once;
     int rc = once.run("linear_small_kernel set-up", [] {
       cudaError_t e = cudaFuncSetAttribute(linear_small_kernel<TM, TN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_STAGES * STAGE_BYTES);
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(linear_small_kernel<TM, TN, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_STAGES * STAGE_BYTES);
       return e != cudaSuccess ? e : cudaFuncSetAttribute(linear_small_kernel<TM, TN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                          2 * STAGE_BYTES + norm_bytes(2 * KC));
     });
@@ -209,6 +212,7 @@ struct Tile {
     const unsigned blocks = (unsigned)(a.tiles0 + (two ? tiles(a.p[1]) : 0));
     const size_t smem = (size_t)(a.stages[0] > a.stages[1] ? a.stages[0] : a.stages[1]) * STAGE_BYTES + (norm ? norm_bytes(a.p[0].K) : 0);
     if (norm) launch_kernel(linear_small_kernel<TM, TN, true>, blocks, THREADS, smem, stream, a);
+    else if (gelu32(a.p[0]) || (two && gelu32(a.p[1]))) launch_kernel(linear_small_kernel<TM, TN, false, true>, blocks, THREADS, smem, stream, a);
     else launch_kernel(linear_small_kernel<TM, TN, false>, blocks, THREADS, smem, stream, a);
     BSRL_LAUNCH_OK("linear_small_kernel");
     return BSRL_OK;

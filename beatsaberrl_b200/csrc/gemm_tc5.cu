@@ -64,7 +64,8 @@ __device__ __forceinline__ WorkItem work_item(int64_t w, int n_tile_work, int n_
 // out otherwise: they cost the residual-free fp32 epilogue ~15 %).
 // SUMS: column sums of A beside the product (LinearArgs::a_sums), compiled in only where asked for: the untaken branch
 // alone cost the MMA thread 0.1 us per k-block.
-template <bool HAS_R, bool SUMS>
+// GELU32: GELU of an fp32 result (gelu_f32), a kernel of its own: compiled into the others it cost updates 1 % by its size alone
+template <bool HAS_R, bool SUMS, bool GELU32 = false>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                   const __grid_constant__ CUtensorMap tm_c, int tma_c, LinearArgs p, int m_tiles, int n_tiles,
@@ -286,10 +287,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
             for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.f);
           } else if (p.relu == 2) {
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              if (p.out_f32) v[j] = gelu_f32(v[j]), v[j + 1] = gelu_f32(v[j + 1]);
-              else gelu2_f16(v[j], v[j + 1]);
-            }
+            for (int j = 0; j < 32; j += 2) gelu2<GELU32>(v[j], v[j + 1]);
           }
           if (masked) {
 #pragma unroll
@@ -553,7 +551,8 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
   static DeviceOnce once;
   int rc = once.run("linear_tc5_kernel set-up", [] {
     cudaError_t e = cudaSuccess;
-    for (auto* k : {linear_tc5_kernel<false, false>, linear_tc5_kernel<true, false>, linear_tc5_kernel<false, true>})
+    for (auto* k : {linear_tc5_kernel<false, false>, linear_tc5_kernel<true, false>, linear_tc5_kernel<false, true>,
+                    linear_tc5_kernel<false, false, true>, linear_tc5_kernel<true, false, true>})
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     return e;
   });
@@ -566,7 +565,9 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
   }
   int64_t grid = m_tiles * n_tiles * (p.k_splits > 1 ? p.k_splits : 1);
   if (grid > sm_count()) grid = sm_count();
-  auto* kernel = p.a_sums ? linear_tc5_kernel<false, true> : p.R ? linear_tc5_kernel<true, false> : linear_tc5_kernel<false, false>;
+  const bool gelu32 = p.relu == 2 && p.out_f32;
+  auto* kernel = p.a_sums ? linear_tc5_kernel<false, true> : gelu32 ? (p.R ? linear_tc5_kernel<true, false, true> : linear_tc5_kernel<false, false, true>)
+                                                           : p.R ? linear_tc5_kernel<true, false> : linear_tc5_kernel<false, false>;
   launch_kernel(kernel, (unsigned)grid, THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, tma_c ? 1 : 0, p, (int)m_tiles, n_tiles, status);
   BSRL_LAUNCH_OK("linear_tc5_kernel");
   return BSRL_OK;
