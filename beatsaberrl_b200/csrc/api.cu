@@ -74,9 +74,9 @@ void use_process_engine() { g_call_engine = g_engine.load(std::memory_order_rela
 int process_engine() { return g_engine.load(std::memory_order_relaxed); }
 int linear(const LinearArgs& p, cudaStream_t st) {
   return timed(st, 2.0 * p.M * p.N * p.K, linear_bytes(p), [&] {
-    if (p.a_mn || p.w_mn || p.mask) {      // row-contraction operands and the epilogue mask: the tcgen05 engine only
+    if (p.a_mn || p.w_mn || p.mask || p.n_rows || p.rmap.start || p.cmap.start) {      // row-contraction operands, the epilogue mask, counted rows: the tcgen05 engine only
       if (g_call_engine == 0 && linear_tc5_ok(p)) return linear_tc5(p, st);
-      set_error("linear: row-contraction operands need the tcgen05 engine and M, N multiples of 64 (m=%lld n=%d k=%d)",
+      set_error("linear: row-contraction operands and counted rows need the tcgen05 engine and M, N multiples of 64 (m=%lld n=%d k=%d)",
                 (long long)p.M, p.N, p.K);
       return (int)BSRL_ERR_UNSUPPORTED;
     }
@@ -95,20 +95,20 @@ int linear_two(const LinearArgs& p, const LinearArgs& q, cudaStream_t st) {
 }
 bool linear_rows_ok(const LinearArgs& p) { return g_call_engine == 0 && linear_tc5_ok(p); }
 int layernorm(const float* x, int64_t ldx, RowMap xmap, const float* g, const float* b, float eps,
-              int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t st) {
+              int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t st, const int* n_rows) {
   int keep = g_stage;
   if (g_stage != kStTrunk && g_stage != kStCritic) g_stage = kStLayerNorm;
-  int rc = timed(st, 0.0, (double)rows * d * 6, [&] { return layernorm_rows(x, ldx, xmap, g, b, eps, rows, d, y, ldy, st); });
+  int rc = timed(st, 0.0, (double)rows * d * 6, [&] { return layernorm_rows(x, ldx, xmap, g, b, eps, rows, d, y, ldy, st, n_rows); });
   g_stage = keep;
   return rc;
 }
 int attention(const __half* qkv, int ld, const float* kb, int64_t B, int d, int H, int q0, int nq,
-              __half* out, int ldo, cudaStream_t st) {
+              __half* out, int ldo, cudaStream_t st, const int* start) {
   int keep = g_stage;
   if (g_stage != kStCritic) g_stage = kStAttention;
   double fl = 4.0 * B * nq * kT * d;
   double by = (double)B * (kT * 2 * d + nq * d * 2) * 2 + (double)B * kT * 4;
-  int rc = timed(st, fl, by, [&] { return attention29(qkv, ld, kb, B, d, H, q0, nq, out, ldo, st); });
+  int rc = timed(st, fl, by, [&] { return attention29(qkv, ld, kb, B, d, H, q0, nq, out, ldo, st, start); });
   g_stage = keep;
   return rc;
 }
@@ -140,8 +140,9 @@ int out_proj_ln(const LinearLnArgs& a, cudaStream_t st) {
   } else {
     LinearArgs po = linear_args(a.A, a.lda, a.W, a.ldw, a.bias, a.x_out, (int)a.ldx, 1, 0, a.M, a.N, a.K);
     po.R = a.R; po.ldr = (int)a.ldr;
+    po.n_rows = a.n_rows;
     rc = linear(po, st);
-    if (rc == BSRL_OK) rc = layernorm(a.x_out, a.ldx, identity_map(), a.gamma, a.beta, a.eps, a.M, a.N, a.h, a.ldh, st);
+    if (rc == BSRL_OK) rc = layernorm(a.x_out, a.ldx, identity_map(), a.gamma, a.beta, a.eps, a.M, a.N, a.h, a.ldh, st, a.n_rows);
   }
   g_stage = keep;
   return rc;
@@ -176,7 +177,13 @@ int run_embed(const Ctx& c, const void* obs, int obs_dtype, float* x, float* key
   eb.key_bias = key_bias;
   eb.obs16 = c.obs16;
   eb.ks = kSaberK; eb.kt = kTorsoK; eb.kl = kLegK; eb.kn = l.note_k;
+  eb.rows = c.rows;
   g_stage = kStGather;
+  if (c.rows.start && (obs_dtype == BSRL_F32 || obs_dtype == BSRL_F16)) {      // (embed_gather refuses the others)
+    const RowSource src{obs, obs_dtype == BSRL_F16, kObs, kOffMask, kSlots, kLead, kRowTileEnvs, 0};
+    BSRL_TRY(timed(c.st, 0.0, (double)B * (kSlots + 1) * 4, [&] { return token_rows(src, B, c.rows, c.st); }));
+    begin_overlap(B * kT);       // the tokenizer's launch under the count
+  }
   BSRL_TRY(timed(c.st, 0.0, (double)B * (kObs * 4 + (2 * kSaberK + kTorsoK + 2 * kLegK + kSlots * l.note_k) * 2 + kT * 4),
                  [&] { return embed_gather(obs, obs_dtype, B, c.cfg->note_geo, c.cfg->game_flux, c.cfg->z_asinh, eb, c.st); }));
   if (have_h) *have_h = false;
@@ -193,6 +200,7 @@ int run_embed(const Ctx& c, const void* obs, int obs_dtype, float* x, float* key
     const BlockW& b0 = l.blocks[0];
     ea.ln_g = c.G(b0.ln_attn); ea.ln_b = c.Be(b0.ln_attn); ea.eps = c.cfg->eps;
     ea.x = x; ea.h = h_out;
+    if (c.rows.start) { ea.dst = c.rows.dst; ea.n_rows = c.n_rows(); }
     g_stage = kStEncoderFused;
     const double rows = (double)B * kT;
     BSRL_TRY(timed(c.st, 2.0 * rows * d * (64 + d), rows * (128 + 4.0 * d + (h_out ? 2.0 * d : 0.0)),
@@ -213,15 +221,21 @@ int run_embed(const Ctx& c, const void* obs, int obs_dtype, float* x, float* key
     __half* hp = hid + p.row0 * d;
     LinearArgs a0 = linear_args(p.f, p.kpad, c.W(p.e->l0), p.e->l0.pitch, c.Bv(p.e->l0), hp, d, 0, 1,
                                 p.rows, d, p.kpad);
+    // packed token rows: the slots' rows that there are, placed one by one
+    const bool slots = p.group == kSlots;
+    a0.n_rows = slots ? c.n_rows() : nullptr;
+    a0.n_less = kLead * B;
     BSRL_TRY(linear(a0, c.st));
     LinearArgs a1 = linear_args(hp, d, c.W(p.e->l1), p.e->l1.pitch, c.Bv(p.e->l1), x, d, 1, 0, p.rows, d, d);
-    a1.cmap = RowMap{p.group, kT, p.first};
+    a1.cmap = c.rows.start ? RowMap{1, 0, 0, c.rows.dst + p.row0} : RowMap{p.group, kT, p.first};
+    a1.n_rows = a0.n_rows;
+    a1.n_less = a0.n_less;
     BSRL_TRY(linear(a1, c.st));
   }
   if (c.cfg->emb_ln) {   // tokens = emb_ln(tokens), in place on the fp32 stream (python/policy.py:1261-1262)
     g_stage = kStLayerNorm;
     BSRL_TRY(timed(c.st, 0.0, (double)B * kT * d * 8, [&] {
-      return layernorm_rows_f32(x, d, c.G(l.emb_ln), c.Be(l.emb_ln), c.cfg->eps, B * kT, d, x, d, c.st);
+      return layernorm_rows_f32(x, d, c.G(l.emb_ln), c.Be(l.emb_ln), c.cfg->eps, B * kT, d, x, d, c.st, c.n_rows());
     }));
   }
   return BSRL_OK;
@@ -409,8 +423,10 @@ int run_blocks_small(const Ctx& c, float* x, const __half* h, const float* key_b
   return BSRL_OK;
 }
 
-int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs& tail_in) {
+int run_forward(const Ctx& ctx, const void* obs, int obs_dtype, const HeadTailArgs& tail_in) {
   PdlScope pdl;
+  Ctx c = ctx;
+  if (c.paths.packed) c.rows = carve_rows(c.train ? c.train->rows : at<void>(c.ws, c.w.rows), c.B, kT);
   const Layout& l = c.l;
   const Workspace& w = c.w;
   const int d = l.d, F = l.F, D = l.D;
@@ -424,7 +440,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
   __half* qkv = w.qkv >= 0 ? at<__half>(c.ws, w.qkv) : nullptr;   // unfused attention path only
   __half* att = at<__half>(c.ws, w.att);
   __half* hid = w.hid >= 0 ? at<__half>(c.ws, w.hid) : nullptr;   // unfused FFN path only
-  const RowMap lead_rows{kLead, kT, 0};
+  const RowMap lead_rows = c.lead_rows();
   const RowMap ident = identity_map();
 
   bool have_h = false, have_hv = false;
@@ -448,6 +464,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
     a.w0 = c.W(b.up); a.b0 = c.Bv(b.up);
     a.w2 = c.W(b.down); a.b2 = c.Bv(b.down);
     a.eps = eps;
+    a.n_rows = c.n_rows();
     return a;
   };
   const bool fused = c.paths.tail_fused;
@@ -463,6 +480,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
     a.wg = c.W(wg); a.bg = c.Bv(wg);
     a.key_bias = key_bias; a.q_first = q_first; a.n_q = n_q;
     a.out = out; a.ldo = d;
+    a.rows = c.rows;
     return a;
   };
   const bool fused_qkv = c.paths.attn_fused;
@@ -487,7 +505,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
   for (int i = 0; i + 1 < l.L && !small; ++i) {
     const BlockW& b = l.blocks[i];
     float* x_next = c.train ? c.train->x[i + 1] : x;
-    if (!have_h) BSRL_TRY(layernorm(x, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h, d, c.st));
+    if (!have_h) BSRL_TRY(layernorm(x, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h, d, c.st, c.n_rows()));
     if (fused_qkv) {
       BSRL_TRY(fused_attn(vres_fused(attn_args(h, b.qkv_g, 0, kT, att), i), c.st));
     } else {
@@ -511,14 +529,17 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
       continue;
     }
     {
-      LinearLnArgs po{att, d, c.W(b.out), d, c.Bv(b.out), x, d, x_next, d, c.G(b.ln_ffn), c.Be(b.ln_ffn), eps, h, d, R, d, d};
+      LinearLnArgs po{att, d, c.W(b.out), d, c.Bv(b.out), x, d, x_next, d, c.G(b.ln_ffn), c.Be(b.ln_ffn), eps, h, d, R, d, d, c.n_rows()};
       BSRL_TRY(out_proj_ln(po, c.st));
     }
     x = x_next;
     g_stage = kStFfnUp;
-    BSRL_TRY(linear(linear_args(h, d, c.W(b.up), d, c.Bv(b.up), hid, F, 0, 1, R, F, d), c.st));
+    LinearArgs pu = linear_args(h, d, c.W(b.up), d, c.Bv(b.up), hid, F, 0, 1, R, F, d);
+    pu.n_rows = c.n_rows();
+    BSRL_TRY(linear(pu, c.st));
     LinearArgs pd = linear_args(hid, F, c.W(b.down), F, c.Bv(b.down), x, d, 1, 0, R, d, F);
     pd.R = x; pd.ldr = d;
+    pd.n_rows = c.n_rows();
     g_stage = kStFfnDown;
     BSRL_TRY(linear(pd, c.st));
     have_h = false;        // h holds this block's FFN operand (the encoder kernel may have left block 0's rows there)
@@ -529,7 +550,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
   __half* h_lead = at<__half>(c.ws, w.h_lead);
   if (!small) {
     const BlockW& b = l.blocks[l.L - 1];
-    if (!have_h) BSRL_TRY(layernorm(x, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h, d, c.st));
+    if (!have_h) BSRL_TRY(layernorm(x, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h, d, c.st, c.n_rows()));
     if (fused_qkv) {
       // q is projected for all 29 rows (a third of this kernel's MMAs, no extra HBM traffic);
       // only the 5 lead rows are attended and written
@@ -547,6 +568,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
     if (fused) {
       BlockTailArgs a = tail_args(b, Rl);
       a.xmap = lead_rows;
+      a.n_rows = nullptr;
       a.out16[0] = lead16; a.ld16[0] = d;     // plain fp16 rows: the trunk's GEMM operand
       if (c.cfg->final_ln) {                  // ... or final_ln of them (python/policy.py:1306-1307)
         a.g16[0] = c.G(l.final_ln); a.b16[0] = c.Be(l.final_ln);
@@ -579,7 +601,7 @@ int run_forward(const Ctx& c, const void* obs, int obs_dtype, const HeadTailArgs
     const RowMap torso_rows{1, kT, 2};
     g_stage = kStCritic;
     const __half* hc = have_hv ? hv : h;
-    if (!have_hv) BSRL_TRY(layernorm(x, d, ident, c.G(l.critic_ln), c.Be(l.critic_ln), eps, R, d, h, d, c.st));
+    if (!have_hv) BSRL_TRY(layernorm(x, d, ident, c.G(l.critic_ln), c.Be(l.critic_ln), eps, R, d, h, d, c.st, c.n_rows()));
     if (fused_qkv) {
       BSRL_TRY(fused_attn(attn_args(hc, l.critic_qkv_g, 2, 1, att_c), c.st));
     } else {
@@ -1102,16 +1124,23 @@ int bsrl_workspace_region(const bsrl_config* cfg, int64_t n_envs, const char* na
     return BSRL_ERR_NULL;
   }
   Layout l = make_layout(*cfg);
-  Workspace w = make_workspace(l, n_envs, plan_paths(l, g_engine.load(std::memory_order_relaxed), n_envs));
+  const Paths paths = plan_paths(l, g_engine.load(std::memory_order_relaxed), n_envs);
+  Workspace w = make_workspace(l, n_envs, paths);
   int64_t off = -1, r = 0, cc = 0, ld = 0;
   int32_t dt = BSRL_F16;
   if (!strcmp(name, "trunk_h")) { off = w.z + (int64_t)l.d * 2; r = n_envs; cc = l.D; ld = l.d + l.D; }
+  else if (!strcmp(name, "x_resolved") && paths.packed) {
+    set_error("workspace_region: a batch of %lld environments keeps rows of live slots only: ask for 'x_packed' and 'row_start'", (long long)n_envs);
+    return BSRL_ERR_UNSUPPORTED;
+  }
+  else if (paths.packed && !strcmp(name, "x_packed")) { off = w.x; r = n_envs * kT; cc = l.d; ld = l.d; dt = BSRL_F32; }
+  else if (paths.packed && !strcmp(name, "row_start")) { off = w.rows; r = n_envs + 1; cc = ld = 1; dt = BSRL_I32; }
   else if (!strcmp(name, "x_resolved")) { off = w.x; r = n_envs * kT; cc = l.d; ld = l.d; dt = BSRL_F32; }
   else if (!strcmp(name, "key_bias")) { off = w.key_bias; r = n_envs; cc = kT; ld = kT; dt = BSRL_F32; }
   else if (!strcmp(name, "readout")) { off = w.lead16; r = n_envs; cc = kLead * l.d; ld = kLead * l.d; }
   else if (!strcmp(name, "head_out")) { off = w.raw; r = n_envs; cc = l.head_cols_pad; ld = l.head_cols_pad; dt = BSRL_F32; }
   else {
-    set_error("workspace_region: unknown region '%s' (trunk_h, x_resolved, key_bias, readout, head_out)", name);
+    set_error("workspace_region: unknown region '%s' (trunk_h, x_resolved or x_packed and row_start, key_bias, readout, head_out)", name);
     return BSRL_ERR_UNSUPPORTED;
   }
   if (byte_offset) *byte_offset = off;

@@ -25,6 +25,27 @@ inline const T* at(const void* base, int64_t off) {
     if (rc__ != BSRL_OK) return rc__; \
   } while (0)
 
+// TokenRows' arrays in token_rows_bytes(n_envs, tokens, dst) bytes of memory (256-byte aligned)
+inline TokenRows carve_rows(void* base, int64_t B, int tokens, bool dst = true) {
+  const int64_t groups = (B + kRowGroup - 1) / kRowGroup, tiles = groups * kRowGroupTiles;
+  int64_t off = 0;
+  auto take = [&](int64_t bytes) {
+    const int64_t o = off;
+    off += round_up(bytes, 256);
+    return o;
+  };
+  TokenRows r;
+  r.start = at<int>(base, take((B + 1) * 4));
+  r.tiles = at<int2>(base, take((tiles + 1) * 8));
+  r.n_tiles = at<int>(base, take(8));
+  r.dst = dst ? at<int>(base, take(B * tokens * 4)) : nullptr;
+  r.kb = at<float>(base, take(B * tokens * 4));
+  r.group_rows = at<int>(base, take(groups * 4));
+  r.group_tiles = at<int>(base, take(groups * 4));
+  r.tile_env = at<int>(base, take(tiles * 4));
+  return r;
+}
+
 constexpr int kMaxBlocks = 32;
 
 // Where a grad-mode forward keeps what the backward needs (all caller memory): the tokenizer's feature rows, the key
@@ -44,6 +65,7 @@ struct TrainPtrs {
   __half* z;               // (B, d + D) f16 [critic pool | trunk h]
   float* raw;              // (B, head_cols_pad) f32
   float* vraw;             // (B, bins_pad) f32
+  void* rows;              // packed token rows: TokenRows' arrays
 };
 
 struct Ctx {
@@ -57,6 +79,9 @@ struct Ctx {
   cudaStream_t st;
   __half* obs16 = nullptr;          // optional fp16 copy of the obs rows, written by the tokenizer kernel
   const TrainPtrs* train = nullptr; // grad-mode forward: intermediates the backward needs go here
+  TokenRows rows;                   // packed token rows (start: nullptr: 29 rows per environment)
+  const int* n_rows() const { return rows.n_rows(); }
+  RowMap lead_rows() const { return RowMap{kLead, kT, 0, rows.start}; }
   const __half* W(const Mat& m, int row0 = 0) const { return at<__half>(arena, m.w) + (int64_t)row0 * m.pitch; }
   const float* Bv(const Mat& m, int row0 = 0) const { return at<float>(arena, m.b) + row0; }
   const float* G(const Norm& n) const { return at<float>(arena, n.g); }
@@ -92,9 +117,9 @@ int linear(const LinearArgs& p, cudaStream_t st);
 // a product with row-contraction operands (a_mn / w_mn) can run as asked (engine and shape)
 bool linear_rows_ok(const LinearArgs& p);
 int layernorm(const float* x, int64_t ldx, RowMap xmap, const float* g, const float* b, float eps, int64_t rows, int d,
-              __half* y, int64_t ldy, cudaStream_t st);
+              __half* y, int64_t ldy, cudaStream_t st, const int* n_rows = nullptr);
 int attention(const __half* qkv, int ld, const float* kb, int64_t B, int d, int H, int q0, int nq, __half* out, int ldo,
-              cudaStream_t st);
+              cudaStream_t st, const int* start = nullptr);
 
 }  // namespace fwd
 }  // namespace bsrl

@@ -37,17 +37,21 @@ __device__ __forceinline__ uint32_t section_at(uint32_t base, int row, int piece
 // BODY: one more key outside the tile (the body token): x_lane = q_row . k_0 for row `lane` (raw), kb0 its
 // base-2 key bias, v0 its DH values (shared memory, generic pointer); its score joins each row's softmax and its
 // probability times v_0 starts the row's output.
-template <int MT, int DH, int LDQ, int OB, bool BODY = false>
+// PACK: the env's keys are the n_keys rows from k_row0 of a tile of 128, in KT tiles of 16; what the last one holds beyond them
+// belongs to other environments and must not show, whatever it is: its scores are replaced, its v rows cleared.  Chunks
+// of keys that are left out would have added exact zeros.
+template <int MT, int DH, int LDQ, int OB, bool BODY = false, bool PACK = false, int KT = 2>
 __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t sv, int q_row0, int piece0, const float (&kb)[4][2],
                                             int n_q, __half* out_env, int ldo, int lane, uint8_t* so, int so_row0, int so_piece0,
-                                            float x_lane = 0.f, float kb0 = 0.f, const __half* v0 = nullptr) {
+                                            float x_lane = 0.f, float kb0 = 0.f, const __half* v0 = nullptr, int k_row0 = 0, int n_keys = 32) {
   const int g = lane >> 2, tig = lane & 3;
+  auto in_tile = [](int row) { return PACK ? min(row, 127) : row; };
   const float scale = rsqrtf((float)DH) * 1.4426950408889634f;   // 1/sqrt(dh) * log2(e)
-  float s[MT][4][4];
+  float s[MT][2 * KT][4];
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+    for (int nt = 0; nt < 2 * KT; ++nt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) s[mt][nt][e] = 0.f;
 #pragma unroll
@@ -55,11 +59,11 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
     uint32_t a[MT][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
-      ldmatrix_x4(a[mt], section_at<LDQ>(sq, q_row0 + mt * 16 + (lane & 15), piece0 + ks * 2 + (lane >> 4)));
+      ldmatrix_x4(a[mt], section_at<LDQ>(sq, in_tile(q_row0 + mt * 16 + (lane & 15)), piece0 + ks * 2 + (lane >> 4)));
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
+    for (int j = 0; j < KT; ++j) {
       uint32_t b[4];
-      const int row = j * 16 + (lane & 7) + ((lane >> 4) << 3);
+      const int row = in_tile(k_row0 + j * 16 + (lane & 7) + ((lane >> 4) << 3));
       ldmatrix_x4(b, section_at<LDQ>(sk, row, piece0 + ks * 2 + ((lane >> 3) & 1)));
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
@@ -68,7 +72,7 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
       }
     }
   }
-  uint32_t pa[MT][2][4];
+  uint32_t pa[MT][KT][4];
   float p0[MT][2];                    // BODY: the body key's probability for rows g and g + 8 of each query tile
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) {
@@ -81,10 +85,11 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
       }
     }
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+    for (int nt = 0; nt < 2 * KT; ++nt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         s[mt][nt][e] = fmaf(s[mt][nt][e], scale, kb[nt][e & 1]);   // base-2 logits: scale and key bias carry log2(e)
+        if (PACK && kb[nt][e & 1] == -INFINITY) s[mt][nt][e] = -INFINITY;
         mx[e >> 1] = fmaxf(mx[e >> 1], s[mt][nt][e]);
       }
     float sum[2] = {0.f, 0.f};
@@ -94,7 +99,7 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
       mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
     }
 #pragma unroll
-    for (int nt = 0; nt < 4; ++nt)
+    for (int nt = 0; nt < 2 * KT; ++nt)
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         s[mt][nt][e] = ex2_approx(s[mt][nt][e] - mx[e >> 1]);
@@ -113,12 +118,18 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
       }
     }
 #pragma unroll
-    for (int ks = 0; ks < 2; ++ks) {
+    for (int ks = 0; ks < KT; ++ks) {
       pa[mt][ks][0] = pack_half2(s[mt][2 * ks][0] * sum[0], s[mt][2 * ks][1] * sum[0]);
       pa[mt][ks][1] = pack_half2(s[mt][2 * ks][2] * sum[1], s[mt][2 * ks][3] * sum[1]);
       pa[mt][ks][2] = pack_half2(s[mt][2 * ks + 1][0] * sum[0], s[mt][2 * ks + 1][1] * sum[0]);
       pa[mt][ks][3] = pack_half2(s[mt][2 * ks + 1][2] * sum[1], s[mt][2 * ks + 1][3] * sum[1]);
     }
+  }
+  uint32_t live[2];                   // PACK: which of this lane's v rows of the last 16 (tig * 2, + 1; 8 further) are the env's
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int left = n_keys - (KT - 1) * 16 - tig * 2 - 8 * e;
+    live[e] = left > 1 ? 0xffffffffu : left == 1 ? 0xffffu : 0u;
   }
   float o[MT][DH / 8][4];
 #pragma unroll
@@ -134,12 +145,16 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
     }
   }
 #pragma unroll
-  for (int ks = 0; ks < 2; ++ks) {
+  for (int ks = 0; ks < KT; ++ks) {
 #pragma unroll
     for (int j = 0; j < DH / 16; ++j) {
       uint32_t b[4];
-      const int row = ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8;
+      const int row = in_tile(k_row0 + ks * 16 + (lane & 7) + ((lane >> 3) & 1) * 8);
       ldmatrix_x4_trans(b, section_at<LDQ>(sv, row, piece0 + j * 2 + (lane >> 4)));
+      if (PACK && ks == KT - 1) {
+        b[0] &= live[0]; b[2] &= live[0];
+        b[1] &= live[1]; b[3] &= live[1];
+      }
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         mma_f16(o[mt][2 * j], pa[mt][ks], b[0], b[1]);
@@ -172,11 +187,11 @@ __device__ __forceinline__ void attend_pair(uint32_t sq, uint32_t sk, uint32_t s
 
 // One query row of an env on the CUDA cores (lane = key for the scores, lane = output column for the weighted sum):
 // row q_row of section sq (as in attend_pair, generic pointers) against the NKEYS rows of sk and sv, the head's columns
-// from piece0; kb_row: this lane's key bias in base 2, -inf past the last key.
+// from piece0; kb_row: this lane's key bias in base 2, -inf past the last key.  The keys are the n_keys rows from k_row0.
 template <int DH, int LDQ, int NKEYS>
 __device__ __forceinline__ void attend_one_row(const uint8_t* sq, const uint8_t* sk, const uint8_t* sv, int q_row, int piece0, float kb_row,
-                                               __half* orow, int lane) {
-  const int krow = lane < NKEYS ? lane : 0;
+                                               __half* orow, int lane, int k_row0 = 0, int n_keys = NKEYS) {
+  const int krow = k_row0 + (lane < n_keys ? lane : 0);
   float sc = 0.f;
 #pragma unroll
   for (int ch = 0; ch < DH / 8; ++ch) {
@@ -200,8 +215,8 @@ __device__ __forceinline__ void attend_one_row(const uint8_t* sq, const uint8_t*
     const int vc = col < DH ? col : 0;
     float acc = 0.f;
 #pragma unroll 8
-    for (int j = 0; j < NKEYS; ++j)
-      acc = fmaf(__shfl_sync(0xffffffffu, pj, j), __half2float(*reinterpret_cast<const __half*>(sv + section_at<LDQ>(0, j, piece0 + (vc >> 3)) + (vc & 7) * 2)), acc);
+    for (int j = 0; j < n_keys; ++j)
+      acc = fmaf(__shfl_sync(0xffffffffu, pj, j), __half2float(*reinterpret_cast<const __half*>(sv + section_at<LDQ>(0, k_row0 + j, piece0 + (vc >> 3)) + (vc & 7) * 2)), acc);
     if (col < DH) orow[col] = __float2half_rn(acc * inv);
   }
 }

@@ -12,6 +12,8 @@
 // fp32 arithmetic it is checked against, softmax(q k^T / sqrt(dh) + bias) v
 // (python/policy.py:686-690).  The kernel is not tied to (T, d, H) = (29, 192, 4): head_dim
 // 32, 48 or 64, any head count.
+#include <type_traits>
+
 #include "kernels.cuh"
 #include "attend.cuh"
 #include "tc5.cuh"
@@ -27,8 +29,8 @@ template <int DH, int KG, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __restrict__ qkv, int ld,
                                                            const float* __restrict__ key_bias,
                                                            int64_t n_pairs, int tokens, int d, int n_heads,
-                                                           int q_first, int n_q,
-                                                           __half* __restrict__ out, int ldo) {
+                                                           int q_first, int n_queries,
+                                                           __half* __restrict__ out, int ldo, const int* __restrict__ start) {
   pdl_begin();
   constexpr int kWarps = WARPS, kRows = 32 * KG, NT = 4 * KG;   // NT: 8-key tiles
   constexpr int CH = DH / 8, SECTION = kRows * DH * 2;          // 16-byte chunks per row; bytes of q, of k, of v
@@ -39,18 +41,22 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
   const float scale = rsqrtf(static_cast<float>(DH));
   const int tig = lane & 3;
   const int ra = lane & 15, ca = lane >> 4, rb = (lane & 7) + ((lane >> 4) << 3), cb = (lane >> 3) & 1;   // ldmatrix rows and halves
-  const int m_tiles = (n_q + 15) >> 4;
 
   for (int64_t pair = (int64_t)blockIdx.x * kWarps + warp; pair < n_pairs;
        pair += (int64_t)gridDim.x * kWarps) {
     int head;
     const int64_t env = div_index(pair, n_heads, &head);
-    const __half* base = qkv + env * tokens * (int64_t)ld + head * DH;
+    // packed token rows: the environment's own, and as many queries where all are asked for
+    const int64_t row0 = start ? start[env] : env * tokens;
+    const int T = start ? (int)(start[env + 1] - row0) : tokens;
+    const bool all = start && n_queries == tokens;
+    const int n_q = all ? T : n_queries, m_tiles = (n_q + 15) >> 4;
+    const __half* base = qkv + row0 * ld + head * DH;
     __syncwarp();
     // stage q (query rows), k, v; rows past the live range are zero
-    for (int c = lane; c < kRows * CH; c += 32) {
+    for (int c = lane; c < (T <= 16 ? 16 : kRows) * CH; c += 32) {
       const int row = c / CH, ch = c % CH;
-      const bool live = row < tokens, asks = row < n_q;
+      const bool live = row < T, asks = row < n_q;
       const __half* r = base + (int64_t)(live ? row : 0) * ld + ch * 8;
       const uint32_t at = tile_at<DH>(row, ch);
       cp_async16(sq_u + at, base + (int64_t)(asks ? q_first + row : 0) * ld + ch * 8, asks);
@@ -65,89 +71,95 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         int key = nt * 8 + tig * 2 + e;
-        kb[nt][e] = key < tokens ? key_bias[env * tokens + key] : -INFINITY;
+        kb[nt][e] = key < T ? key_bias[env * tokens + key] : -INFINITY;
       }
     cp_async_wait<0>();
     __syncwarp();
 
-    for (int mt = 0; mt < m_tiles; ++mt) {
-      float s[NT][4];
+    // K tiles of 16 keys: short environments leave out those that hold exact zeros
+    auto attend = [&](auto k_tiles) {
+      constexpr int K = decltype(k_tiles)::value;
+      for (int mt = 0; mt < m_tiles; ++mt) {
+        float s[2 * K][4];
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
+        for (int nt = 0; nt < 2 * K; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[nt][e] = 0.f;
+          for (int e = 0; e < 4; ++e) s[nt][e] = 0.f;
 #pragma unroll
-      for (int ks = 0; ks < DH / 16; ++ks) {
-        uint32_t a[4];
-        ldmatrix_x4(a, sq_u + tile_at<DH>(mt * 16 + ra, ks * 2 + ca));
+        for (int ks = 0; ks < DH / 16; ++ks) {
+          uint32_t a[4];
+          ldmatrix_x4(a, sq_u + tile_at<DH>(mt * 16 + ra, ks * 2 + ca));
 #pragma unroll
-        for (int j = 0; j < 2 * KG; ++j) {
-          uint32_t b[4];
-          ldmatrix_x4(b, sk_u + tile_at<DH>(j * 16 + rb, ks * 2 + cb));
-          mma_f16(s[2 * j], a, b[0], b[1]);
-          mma_f16(s[2 * j + 1], a, b[2], b[3]);
+          for (int j = 0; j < K; ++j) {
+            uint32_t b[4];
+            ldmatrix_x4(b, sk_u + tile_at<DH>(j * 16 + rb, ks * 2 + cb));
+            mma_f16(s[2 * j], a, b[0], b[1]);
+            mma_f16(s[2 * j + 1], a, b[2], b[3]);
+          }
         }
-      }
-      // softmax over keys for rows g (e = 0,1) and g + 8 (e = 2,3)
-      float mx[2] = {-INFINITY, -INFINITY};
+        // softmax over keys for rows g (e = 0,1) and g + 8 (e = 2,3)
+        float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
+        for (int nt = 0; nt < 2 * K; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          s[nt][e] = s[nt][e] * scale + kb[nt][e & 1];
-          mx[e >> 1] = fmaxf(mx[e >> 1], s[nt][e]);
-        }
-      float sum[2] = {0.f, 0.f};
+          for (int e = 0; e < 4; ++e) {
+            s[nt][e] = s[nt][e] * scale + kb[nt][e & 1];
+            mx[e >> 1] = fmaxf(mx[e >> 1], s[nt][e]);
+          }
+        float sum[2] = {0.f, 0.f};
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-      }
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          s[nt][e] = expf(s[nt][e] - mx[e >> 1]);
-          sum[e >> 1] += s[nt][e];
+        for (int r = 0; r < 2; ++r) {
+          mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+          mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
         }
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
-        sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
-        sum[r] = 1.f / sum[r];
-      }
-      // P (normalised, fp16) as the A operand of P V
-      uint32_t pa[2 * KG][4];
+        for (int nt = 0; nt < 2 * K; ++nt)
 #pragma unroll
-      for (int ks = 0; ks < 2 * KG; ++ks) {
-        pa[ks][0] = pack_half2(s[2 * ks][0] * sum[0], s[2 * ks][1] * sum[0]);
-        pa[ks][1] = pack_half2(s[2 * ks][2] * sum[1], s[2 * ks][3] * sum[1]);
-        pa[ks][2] = pack_half2(s[2 * ks + 1][0] * sum[0], s[2 * ks + 1][1] * sum[0]);
-        pa[ks][3] = pack_half2(s[2 * ks + 1][2] * sum[1], s[2 * ks + 1][3] * sum[1]);
-      }
-      float o[DH / 8][4];
+          for (int e = 0; e < 4; ++e) {
+            s[nt][e] = expf(s[nt][e] - mx[e >> 1]);
+            sum[e >> 1] += s[nt][e];
+          }
 #pragma unroll
-      for (int nt = 0; nt < DH / 8; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[nt][e] = 0.f;
-#pragma unroll
-      for (int ks = 0; ks < 2 * KG; ++ks) {
-#pragma unroll
-        for (int j = 0; j < DH / 16; ++j) {
-          uint32_t b[4];
-          ldmatrix_x4_trans(b, sv_u + tile_at<DH>(ks * 16 + ra, j * 2 + ca));
-          mma_f16(o[2 * j], pa[ks], b[0], b[1]);
-          mma_f16(o[2 * j + 1], pa[ks], b[2], b[3]);
+        for (int r = 0; r < 2; ++r) {
+          sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
+          sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
+          sum[r] = 1.f / sum[r];
         }
-      }
-      // the output takes the place of the query rows it came from
+        // P (normalised, fp16) as the A operand of P V
+        uint32_t pa[K][4];
 #pragma unroll
-      for (int j = 0; j < DH / 16; ++j)
-        tc5::stmatrix_x4(sq_u + tile_at<DH>(mt * 16 + ra, j * 2 + ca), pack_half2(o[2 * j][0], o[2 * j][1]), pack_half2(o[2 * j][2], o[2 * j][3]),
-                         pack_half2(o[2 * j + 1][0], o[2 * j + 1][1]), pack_half2(o[2 * j + 1][2], o[2 * j + 1][3]));
-    }
+        for (int ks = 0; ks < K; ++ks) {
+          pa[ks][0] = pack_half2(s[2 * ks][0] * sum[0], s[2 * ks][1] * sum[0]);
+          pa[ks][1] = pack_half2(s[2 * ks][2] * sum[1], s[2 * ks][3] * sum[1]);
+          pa[ks][2] = pack_half2(s[2 * ks + 1][0] * sum[0], s[2 * ks + 1][1] * sum[0]);
+          pa[ks][3] = pack_half2(s[2 * ks + 1][2] * sum[1], s[2 * ks + 1][3] * sum[1]);
+        }
+        float o[DH / 8][4];
+#pragma unroll
+        for (int nt = 0; nt < DH / 8; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) o[nt][e] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < K; ++ks) {
+#pragma unroll
+          for (int j = 0; j < DH / 16; ++j) {
+            uint32_t b[4];
+            ldmatrix_x4_trans(b, sv_u + tile_at<DH>(ks * 16 + ra, j * 2 + ca));
+            mma_f16(o[2 * j], pa[ks], b[0], b[1]);
+            mma_f16(o[2 * j + 1], pa[ks], b[2], b[3]);
+          }
+        }
+        // the output takes the place of the query rows it came from
+#pragma unroll
+        for (int j = 0; j < DH / 16; ++j)
+          tc5::stmatrix_x4(sq_u + tile_at<DH>(mt * 16 + ra, j * 2 + ca), pack_half2(o[2 * j][0], o[2 * j][1]), pack_half2(o[2 * j][2], o[2 * j][3]),
+                           pack_half2(o[2 * j + 1][0], o[2 * j + 1][1]), pack_half2(o[2 * j + 1][2], o[2 * j + 1][3]));
+      }
+    };
+    if (T <= 16) attend(std::integral_constant<int, 1>());
+    else attend(std::integral_constant<int, 2 * KG>());
     __syncwarp();
-    __half* to = out + env * n_q * (int64_t)ldo + head * DH;
+    __half* to = out + (all ? row0 : env * n_q) * ldo + head * DH;
     for (int c = lane; c < n_q * CH; c += 32) {
       const int row = c / CH, ch = c % CH;
       *reinterpret_cast<uint4*>(to + row * (int64_t)ldo + ch * 8) = *reinterpret_cast<const uint4*>(sq + tile_at<DH>(row, ch));
@@ -179,10 +191,13 @@ struct BodyTile {
   // q, k, v of the object tokens; then q0 | k0 | v0, a zero piece, and what a team's warps exchange (max, sum, DH outputs)
   static constexpr int EXTRA = 3 * ROW + 16, SWAP = EXTRA, BYTES = 3 * SECTION + (EXTRA + (4 + DH) * 4 + 127) / 128 * 128;
 };
-template <int DH, int NOBJ, int WARPS, int TEAM>
-__global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __restrict__ qkv, int ld,
+// PACK: packed token rows -- the body rows first, then the object rows that there are, an environment's from start[env] on.
+// What is missing reads as zero and is masked; whole 16-row tiles of it are left out.
+template <int DH, int NOBJ, int WARPS, int TEAM, bool PACK>
+__global__ void __launch_bounds__(WARPS * 32, PACK && NOBJ == 64 ? 2 : 0) attn_body_kernel(const __half* __restrict__ qkv, int ld,
                                                               const float* __restrict__ key_bias, int64_t n_pairs,
-                                                              int d, int n_heads, int n_q, __half* __restrict__ out, int ldo) {
+                                                              int d, int n_heads, int n_q, __half* __restrict__ out, int ldo,
+                                                              const int* __restrict__ start, int64_t n_envs) {
   pdl_begin();
   using Tile = BodyTile<DH, NOBJ, TEAM>;
   constexpr int T = NOBJ + 1, NT = NOBJ / 8, KS = NOBJ / 16, MT = NOBJ / 16 / TEAM, CH = DH / 8, ROW = Tile::ROW;
@@ -210,15 +225,19 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
   for (int64_t pair = (int64_t)blockIdx.x * (WARPS / TEAM) + team; pair < n_pairs; pair += (int64_t)gridDim.x * (WARPS / TEAM)) {
     int head;
     const int64_t env = div_index(pair, n_heads, &head);
-    const __half* base = qkv + env * T * (int64_t)ld + head * DH;
+    const int64_t body = PACK ? env : env * T, obj = PACK ? n_envs + start[env] : body + 1;      // the body row, the first object row
+    const int n_obj = PACK ? (int)(n_envs + start[env + 1] - obj) : NOBJ;
+    const __half* base = qkv + body * ld + head * DH;
+    const __half* obase = qkv + obj * ld + head * DH;
     team_sync();
     for (int c = tlane; c < NOBJ * CH; c += 32 * TEAM) {
       const int row = c / CH, ch = c % CH;
-      const __half* r = base + (int64_t)(row + 1) * ld + ch * 8;
+      const bool there = !PACK || row < n_obj;
+      const __half* r = PACK && !there ? base : obase + (int64_t)row * ld + ch * 8;
       const uint32_t at = tile_at<DH>(row, ch);
-      if (all_rows) cp_async16(sq_u + at, r, true);
-      cp_async16(sk_u + at, r + d, true);
-      cp_async16(sv_u + at, r + 2 * d, true);
+      if (all_rows) cp_async16(sq_u + at, r, there);
+      cp_async16(sk_u + at, r + d, there);
+      cp_async16(sv_u + at, r + 2 * d, there);
     }
     if (tlane < 3 * CH) {
       const int which = tlane / CH, ch = tlane % CH;
@@ -299,7 +318,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
       }
       if (part == 0) {
         const float inv = 1.f / (sum + p00);
-        __half* orow = out + env * n_q * (int64_t)ldo + head * DH + CPL * lane;
+        __half* orow = out + (PACK ? env : env * n_q) * (int64_t)ldo + head * DH + CPL * lane;
         const __half* v0 = reinterpret_cast<const __half*>(extra + 2 * ROW) + CPL * lane;
 #pragma unroll
         for (int u = 0; u < CPL; ++u) orow[u] = __float2half_rn(fmaf(p00, __half2float(v0[u]), o[u]) * inv);
@@ -309,6 +328,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
 
     // ---- object query rows (16 MT of them) against the object keys and the body token's
     const int row0 = part * (16 * MT);
+    if (PACK && row0 >= n_obj) continue;
     float s[MT][NT][4], x0[MT][4];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt)
@@ -325,6 +345,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
       for (int mt = 0; mt < MT; ++mt) ldmatrix_x4(a[mt], sq_u + tile_at<DH>(row0 + mt * 16 + ra, ks * 2 + ca));
 #pragma unroll
       for (int j = 0; j < NT / 2; ++j) {
+        if (PACK && j * 16 >= n_obj) break;
         uint32_t b[4];
         ldmatrix_x4(b, sk_u + tile_at<DH>(j * 16 + rb, ks * 2 + cb));
 #pragma unroll
@@ -402,6 +423,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
       }
 #pragma unroll
       for (int ks = 0; ks < KS; ++ks) {
+        if (PACK && ks * 16 >= n_obj) break;
         uint32_t b[4];
         ldmatrix_x4_trans(b, sv_u + tile_at<DH>(ks * 16 + ra, j * 2 + ca));
 #pragma unroll
@@ -416,8 +438,9 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
                          pack_half2(o[mt][1][0], o[mt][1][1]), pack_half2(o[mt][1][2], o[mt][1][3]));
     }
     __syncwarp();
-    __half* to = out + (env * T + 1 + row0) * (int64_t)ldo + head * DH;
-    for (int c = lane; c < 16 * MT * CH; c += 32) {
+    __half* to = out + (obj + row0) * (int64_t)ldo + head * DH;
+    const int live = PACK && n_obj - row0 < 16 * MT ? n_obj - row0 : 16 * MT;
+    for (int c = lane; c < live * CH; c += 32) {
       const int row = c / CH, ch = c % CH;
       *reinterpret_cast<uint4*>(to + row * (int64_t)ldo + ch * 8) = *reinterpret_cast<const uint4*>(tile + tile_at<DH>(row0 + row, ch));
     }
@@ -426,34 +449,36 @@ __global__ void __launch_bounds__(WARPS * 32) attn_body_kernel(const __half* __r
 
 template <int DH, int NOBJ>
 int launch_body(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int d, int n_heads, int n_q, __half* out,
-                int ldo, cudaStream_t stream) {
+                int ldo, cudaStream_t stream, const int* start) {
   constexpr int kWarps = 8, kTeam = NOBJ <= 32 ? 1 : 2, kPairs = kWarps / kTeam;
   constexpr int smem = kPairs * BodyTile<DH, NOBJ, kTeam>::BYTES;
   static DeviceOnce once;
   int rc = once.run("attn_body_kernel set-up", [] {
-    return cudaFuncSetAttribute(attn_body_kernel<DH, NOBJ, kWarps, kTeam>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    cudaError_t e = cudaFuncSetAttribute(attn_body_kernel<DH, NOBJ, kWarps, kTeam, false>, at, smem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(attn_body_kernel<DH, NOBJ, kWarps, kTeam, true>, at, smem);
   });
   if (rc != BSRL_OK) return rc;
   const int64_t pairs = n_envs * n_heads;
   int64_t blocks = (pairs + kPairs - 1) / kPairs;
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  launch_kernel(attn_body_kernel<DH, NOBJ, kWarps, kTeam>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d,
-                                                                                                n_heads, n_q, out, ldo);
+  launch_kernel(start ? attn_body_kernel<DH, NOBJ, kWarps, kTeam, true> : attn_body_kernel<DH, NOBJ, kWarps, kTeam, false>, static_cast<unsigned>(blocks),
+                kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d, n_heads, n_q, out, ldo, start, n_envs);
   BSRL_LAUNCH_OK("attn_body_kernel");
   return BSRL_OK;
 }
 template <int DH>
 int launch_body_n(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int tokens, int d, int n_heads, int n_q,
-                  __half* out, int ldo, cudaStream_t stream) {
-  if (tokens == 17) return launch_body<DH, 16>(qkv, ld, key_bias, n_envs, d, n_heads, n_q, out, ldo, stream);
-  if (tokens == 33) return launch_body<DH, 32>(qkv, ld, key_bias, n_envs, d, n_heads, n_q, out, ldo, stream);
-  return launch_body<DH, 64>(qkv, ld, key_bias, n_envs, d, n_heads, n_q, out, ldo, stream);
+                  __half* out, int ldo, cudaStream_t stream, const int* start) {
+  if (tokens == 17) return launch_body<DH, 16>(qkv, ld, key_bias, n_envs, d, n_heads, n_q, out, ldo, stream, start);
+  if (tokens == 33) return launch_body<DH, 32>(qkv, ld, key_bias, n_envs, d, n_heads, n_q, out, ldo, stream, start);
+  return launch_body<DH, 64>(qkv, ld, key_bias, n_envs, d, n_heads, n_q, out, ldo, stream, start);
 }
 
 template <int DH, int KG>
 int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int tokens, int d, int n_heads,
-           int q_first, int n_q, __half* out, int ldo, cudaStream_t stream) {
+           int q_first, int n_q, __half* out, int ldo, cudaStream_t stream, const int* start) {
   constexpr int kWarps = KG == 1 ? 8 : 4;
   constexpr int smem = kWarps * 3 * (32 * KG) * DH * 2;
   static DeviceOnce once;
@@ -465,26 +490,26 @@ int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int
   int64_t blocks = (pairs + kWarps - 1) / kWarps;
   int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  launch_kernel(attn29_kernel<DH, KG, kWarps>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, tokens, d, n_heads, q_first, n_q, out, ldo);
+  launch_kernel(attn29_kernel<DH, KG, kWarps>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, tokens, d, n_heads, q_first, n_q, out, ldo, start);
   BSRL_LAUNCH_OK("attn29_kernel");
   return BSRL_OK;
 }
 template <int DH>
 int launch_kg(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int tokens, int d, int n_heads,
-              int q_first, int n_q, __half* out, int ldo, cudaStream_t stream) {
-  if (tokens <= 32) return launch<DH, 1>(qkv, ld, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream);
-  if (tokens <= 64) return launch<DH, 2>(qkv, ld, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream);
-  return launch<DH, 3>(qkv, ld, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream);
+              int q_first, int n_q, __half* out, int ldo, cudaStream_t stream, const int* start) {
+  if (tokens <= 32) return launch<DH, 1>(qkv, ld, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream, start);
+  if (tokens <= 64) return launch<DH, 2>(qkv, ld, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream, start);
+  return launch<DH, 3>(qkv, ld, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream, start);
 }
 }  // namespace
 
 int attention29(const __half* qkv, int ld_qkv, const float* key_bias, int64_t n_envs, int d,
-                int n_heads, int q_first, int n_q, __half* out, int ldo, cudaStream_t stream) {
-  return attention_tokens(qkv, ld_qkv, key_bias, n_envs, kT, d, n_heads, q_first, n_q, out, ldo, stream);
+                int n_heads, int q_first, int n_q, __half* out, int ldo, cudaStream_t stream, const int* start) {
+  return attention_tokens(qkv, ld_qkv, key_bias, n_envs, kT, d, n_heads, q_first, n_q, out, ldo, stream, start);
 }
 
 int attention_tokens(const __half* qkv, int ld_qkv, const float* key_bias, int64_t n_envs, int tokens, int d,
-                     int n_heads, int q_first, int n_q, __half* out, int ldo, cudaStream_t stream) {
+                     int n_heads, int q_first, int n_q, __half* out, int ldo, cudaStream_t stream, const int* start) {
   if (!qkv || !key_bias || !out) {
     set_error("attention: NULL operand");
     return BSRL_ERR_NULL;
@@ -506,12 +531,12 @@ int attention_tokens(const __half* qkv, int ld_qkv, const float* key_bias, int64
   const int dh = d / n_heads;
   // one body token + 16 / 32 / 64 object tokens, all rows or the body row only: the body token off the MMA tiles
   if ((tokens == 17 || tokens == 33 || tokens == 65) && q_first == 0 && (n_q == tokens || n_q == 1)) {
-    if (dh == 32) return launch_body_n<32>(qkv, ld_qkv, key_bias, n_envs, tokens, d, n_heads, n_q, out, ldo, stream);
-    if (dh == 64) return launch_body_n<64>(qkv, ld_qkv, key_bias, n_envs, tokens, d, n_heads, n_q, out, ldo, stream);
+    if (dh == 32) return launch_body_n<32>(qkv, ld_qkv, key_bias, n_envs, tokens, d, n_heads, n_q, out, ldo, stream, start);
+    if (dh == 64) return launch_body_n<64>(qkv, ld_qkv, key_bias, n_envs, tokens, d, n_heads, n_q, out, ldo, stream, start);
   }
-  if (dh == 32) return launch_kg<32>(qkv, ld_qkv, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream);
-  if (dh == 48) return launch_kg<48>(qkv, ld_qkv, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream);
-  if (dh == 64) return launch_kg<64>(qkv, ld_qkv, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream);
+  if (dh == 32) return launch_kg<32>(qkv, ld_qkv, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream, start);
+  if (dh == 48) return launch_kg<48>(qkv, ld_qkv, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream, start);
+  if (dh == 64) return launch_kg<64>(qkv, ld_qkv, key_bias, n_envs, tokens, d, n_heads, q_first, n_q, out, ldo, stream, start);
   set_error("attention: head_dim %d unsupported (32, 48 or 64)", dh);
   return BSRL_ERR_UNSUPPORTED;
 }
@@ -520,10 +545,11 @@ int attention_tokens(const __half* qkv, int ld_qkv, const float* key_bias, int64
 // projection are copied out as the block's own values (v_out) and / or replaced by
 // vres[0] * v + vres[1] * v0 (fp32 arithmetic, rounded once).  8 columns per thread.
 namespace {
-__global__ void vres_mix_kernel(__half* __restrict__ v, int ld, int64_t rows, int d,
+__global__ void vres_mix_kernel(__half* __restrict__ v, int ld, int64_t row_bound, int d,
                                 __half* __restrict__ v_out, const __half* __restrict__ v0,
-                                const float* __restrict__ vres) {
+                                const float* __restrict__ vres, const int* n_rows) {
   pdl_begin();
+  const int64_t rows = n_rows ? n_rows[0] : row_bound;
   const float a = vres ? vres[0] : 1.f, b = vres ? vres[1] : 0.f;
   const int per_row = d >> 3;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row;
@@ -550,7 +576,7 @@ __global__ void vres_mix_kernel(__half* __restrict__ v, int ld, int64_t rows, in
 }  // namespace
 
 int vres_mix(__half* v, int ld, int64_t rows, int d, __half* v_out, const __half* v0, const float* vres,
-             cudaStream_t stream) {
+             cudaStream_t stream, const int* n_rows) {
   if (!v || (v0 && !vres)) {
     set_error("vres_mix: NULL operand");
     return BSRL_ERR_NULL;
@@ -563,7 +589,7 @@ int vres_mix(__half* v, int ld, int64_t rows, int d, __half* v_out, const __half
   int64_t blocks = (rows * (d >> 3) + 255) / 256;
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  launch_kernel(vres_mix_kernel, static_cast<unsigned>(blocks), 256, 0, stream, v, ld, rows, d, v_out, v0, vres);
+  launch_kernel(vres_mix_kernel, static_cast<unsigned>(blocks), 256, 0, stream, v, ld, rows, d, v_out, v0, vres, n_rows);
   BSRL_LAUNCH_OK("vres_mix_kernel");
   return BSRL_OK;
 }

@@ -48,7 +48,7 @@ constexpr int MAX_STAGES = 4;
 constexpr int CHUNK_BYTES = BM * 128;   // 16 KB: 128 rows x 64 k-columns
 // Head group of G heads of width DH: 3 G DH projection columns per group -- (32, 2): 192, two heads;
 // (48, 1): 144, one head (the reference's production shape, 4 heads of 48); (64, 1): 192, one head (the wide policy).
-template <int DH_, int G_, bool PAIR>
+template <int DH_, int G_, bool PAIR, bool PACK>
 struct Shape {
   static constexpr int DH = DH_, G = G_, GD = G * DH, NG = 3 * GD;
   // STREAM (head_dim 64, d up to 512): the h tile does not stay resident (128 rows x 512 x 2 B = 128 KB); its
@@ -70,8 +70,10 @@ struct Shape {
   static constexpr int SQ_BYTES = INPLACE ? 3 * CHUNK_BYTES : BM * LDQ;
   static constexpr int SO_BYTES = INPLACE ? 0 : BM * GD * 2;
   static constexpr int BIAS_BYTES = 3 * MAX_D * 4;
-  static constexpr int SB_BYTES = DH == 32 ? SETS * EPT * 2 * 3 * 64 : 0;   // body-token mode: q0 | k0 | v0 (64 B each) per env and head of the group
-  static constexpr int SMEM_BYTES = A_BYTES + STAGES * STAGE_BYTES + SETS * (SO_BYTES + SQ_BYTES) + BIAS_BYTES + SB_BYTES + 1024 + 256;
+  // body-token mode: q0 | k0 | v0 (64 B each) per head of the group and env
+  static constexpr int SB_BYTES = DH == 32 ? SETS * (PACK ? kBodyTileEnvs : EPT) * 2 * 3 * 64 : 0;
+  static constexpr int SP_BYTES = PACK ? SETS * (BM + 32) * 4 : 0;      // packed rows: key bias by tile row, first rows of the tile's environments
+  static constexpr int SMEM_BYTES = A_BYTES + STAGES * STAGE_BYTES + SETS * (SO_BYTES + SQ_BYTES) + BIAS_BYTES + SB_BYTES + SP_BYTES + 1024 + 256;
   static_assert((!PAIR || NG % 32 == 0) && NG <= 256 && W_ROWS % 8 == 0 && STAGES <= MAX_STAGES && STAGE_BYTES % 1024 == 0 && W_BYTES % 1024 == 0, "group width");
   static_assert(SMEM_BYTES <= 227 * 1024, "shared memory");
 };
@@ -105,6 +107,9 @@ struct Params {
   int tokens, tok0, body_only;
   const __half* qkv0;
   int* status;
+  TokenRows rows;          // packed token rows (PACK kernels)
+  int64_t rows_ahead;      // rows of out ahead of theirs (body-token layout: the body rows)
+  int full_rows;           // not 0: the number of rows that has all slots live, where the kernel of the full layout does the work
 };
 
 __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
@@ -114,13 +119,20 @@ __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
 
 // VRES: the value-residual code of the drain is compiled in (it costs ~14 % of the kernel even when idle)
 // BODY: the single-body-token layout (Params::tokens and below); DH = 32, G = 2 only
-template <int DH, int G, bool PAIR, bool VRES, bool BODY = false>
-__global__ void __launch_bounds__((Shape<DH, G, PAIR>::THREADS), 1)
+// PACK: packed token rows (rows.cu).  A tile is as many whole environments as fit 128 rows, from any row on; a set's eight
+// warps drain it, then take its (environment, head) pairs in turn, of 16 or 32 rows and keys as the environment has.
+template <int DH, int G, bool PAIR, bool VRES, bool BODY = false, bool PACK = false>
+__global__ void __launch_bounds__((Shape<DH, G, PAIR, PACK>::THREADS), 1)
 attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constant__ CUtensorMap tm_w,
                   const __grid_constant__ CUtensorMap tm_o, Params p) {
-  using S = Shape<DH, G, PAIR>;
+  using S = Shape<DH, G, PAIR, PACK>;
   constexpr int STAGES = S::STAGES, GD = S::GD, NG = S::NG, STAGE_BYTES = S::STAGE_BYTES, LDQ = S::LDQ, SQ_BYTES = S::SQ_BYTES;
   constexpr int THREADS = S::THREADS, SECTION = S::SECTION;
+  // which of the two launches the rows are for (counted at least two launches back)
+  if (!BODY && p.full_rows && (p.rows.n_tiles[1] == p.full_rows) == PACK) {
+    pdl_wait();
+    return;
+  }
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -135,15 +147,19 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
   float* s_bias = reinterpret_cast<float*>(gen + S::A_BYTES + STAGES * STAGE_BYTES + SETS * (S::SO_BYTES + SQ_BYTES));
   uint8_t* sB_all = reinterpret_cast<uint8_t*>(s_bias) + S::BIAS_BYTES;
   uint8_t* sB_g = sB_all + set * (S::SB_BYTES / SETS);
-  Shared* sh = reinterpret_cast<Shared*>(sB_all + S::SB_BYTES);
+  float* sP_kb = reinterpret_cast<float*>(sB_all + S::SB_BYTES) + set * (S::SP_BYTES / SETS / 4);      // PACK: key bias (base 2) by tile row ...
+  int* sP_row = reinterpret_cast<int*>(sP_kb + BM);                                     // ... and the environments' first rows
+  Shared* sh = reinterpret_cast<Shared*>(sB_all + S::SB_BYTES + S::SP_BYTES);
   static_assert(!BODY || (DH == 32 && G == 2 && !VRES), "body-token mode: two heads of 32 per group");
+  static_assert(!PACK || kBodyTileEnvs * 2 * 12 <= 2 * EPT * TEAM * 32, "two pieces of the body rows per thread of a set");
   constexpr int NKEYS = BODY ? EROWS : kT;            // live keys of an env inside the tile
   const int T = BODY ? p.tokens : kT;                 // token rows per env in memory
   const int d = p.d, KB = d >> 6, n_groups = d / GD;
   volatile int* abort = &sh->abort;
   const uint32_t rank = PAIR ? cluster_rank() : 0u;
   // work item: (tile, share of its head groups); both CTAs of a pair take the same number of tiles
-  const int t_end = PAIR ? (p.n_tiles + 1) & ~1 : p.n_tiles * p.split;
+  const int n_tiles = PACK ? p.rows.n_tiles[0] : p.n_tiles;      // (PACK: counted at least two launches back)
+  const int t_end = PAIR ? (n_tiles + 1) & ~1 : PACK ? n_tiles : n_tiles * p.split;
   const int per_item = PAIR ? n_groups : (n_groups + p.split - 1) / p.split, log_split = PAIR ? 0 : __ffs(p.split) - 1;
   auto tile_of = [&](int i) { return i >> log_split; };
   auto first_group = [&](int i) { return (i & ((1 << log_split) - 1)) * per_item; };
@@ -200,7 +216,10 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
         else tma_load_2d(dst, &tm_w, x, y, bar);
       };
       auto load_h = [&](uint32_t dst, int kb, int t, uint32_t bar) {
-        if (PAIR) tma_load_3d_pair(dst, &tm_h, 64 * kb, BODY ? p.tok0 : 0, t * EPT, map_to_cta(bar, 0));
+        if (PACK) {                              // t: the tile's first row
+          if (PAIR) tma_load_2d_pair(dst, &tm_h, 64 * kb, t, map_to_cta(bar, 0));
+          else tma_load_2d(dst, &tm_h, 64 * kb, t, bar);
+        } else if (PAIR) tma_load_3d_pair(dst, &tm_h, 64 * kb, BODY ? p.tok0 : 0, t * EPT, map_to_cta(bar, 0));
         else tma_load_3d(dst, &tm_h, 64 * kb, BODY ? p.tok0 : 0, t * EPT, bar);
       };
       auto w_stage = [&](int g, int kb, int t) -> bool {
@@ -216,7 +235,7 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
       };
       if (STREAM) pdl_wait();
       for (int i = blockIdx.x; i < t_end && ok; i += gridDim.x, ++tile_i) {
-        const int t = tile_of(i), g_lo = first_group(i), g_hi = min(g_lo + per_item, n_groups);
+        const int t = PACK ? p.rows.tiles[i].y : tile_of(i), g_lo = first_group(i), g_hi = min(g_lo + per_item, n_groups);
         if (STREAM) {
           for (int g = g_lo; g < g_hi && ok; ++g)
             for (int kb = 0; kb < KB && ok; ++kb) ok = w_stage(g, kb, t);
@@ -296,13 +315,26 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
     const int u_first = part * U0, u_count = UNITS - u_first < U0 ? UNITS - u_first : U0;
     // attention of the env this pair drained: G = 2: one head per warp, both 16-row query tiles; G = 1: one query tile each
     const int env_l = q, hh = G == 2 ? part : 0, mt_own = G == 2 ? 0 : part;
-    auto team_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + q + set * EPT), "n"(TEAM * 32) : "memory"); };
+    auto team_sync = [&]() {
+      if (PACK) asm volatile("bar.sync %0, %1;" ::"r"(1 + set), "n"(EPT * TEAM * 32) : "memory");
+      else asm volatile("bar.sync %0, %1;" ::"r"(1 + q + set * EPT), "n"(TEAM * 32) : "memory");
+    };
+    const int set_thread = threadIdx.x - 64 - set * EPT * TEAM * 32, quit_at = PACK ? set * EPT : set * EPT + q;
     uint32_t gi = 0;
     bool ok = true;
     const float vres_a = (VRES && p.vres) ? p.vres[0] : 1.f, vres_b = (VRES && p.vres) ? p.vres[1] : 0.f;
     for (int i = blockIdx.x; i < t_end && ok; i += gridDim.x) {
       const int t = tile_of(i), g_lo = first_group(i), g_hi = min(g_lo + per_item, n_groups);
       const int64_t env = (int64_t)t * EPT + env_l;
+      // PACK: the tile's environments and rows; this thread's share of their places and key bias, fetched long before use
+      const int2 tile_lo = PACK && t < n_tiles ? p.rows.tiles[t] : make_int2(0, 0), tile_hi = PACK && t < n_tiles ? p.rows.tiles[t + 1] : make_int2(0, 0);
+      const int n_tile_envs = tile_hi.x - tile_lo.x, used = tile_hi.y - tile_lo.y;
+      const int64_t row0 = tile_lo.y;
+      int sP_value = 0;
+      if (PACK) {
+        if (set_thread < BM) sP_value = set_thread < used ? __float_as_int(p.rows.kb[row0 + set_thread]) : 0;
+        else if (set_thread - BM <= n_tile_envs) sP_value = p.rows.start[tile_lo.x + set_thread - BM] - tile_lo.y;
+      }
       // this lane's key-bias values (keys nt * 8 + tig * 2 + e of the m16n8 accumulator layout, times
       // log2 e; -inf past the 29th key), fetched once per tile and long before the first softmax
       float kb[4][2];
@@ -311,25 +343,33 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
           const int key = nt * 8 + (lane & 3) * 2 + e;
-          kb[nt][e] = (key < NKEYS && env < p.n_envs) ? p.key_bias[env * T + (BODY ? p.tok0 : 0) + key] : -INFINITY;
+          kb[nt][e] = (!PACK && key < NKEYS && env < p.n_envs) ? p.key_bias[env * T + (BODY ? p.tok0 : 0) + key] : -INFINITY;
         }
       // body-token mode: the body key's bias, and this lane's object key's (lane = key in the body row's softmax)
       float kb0 = 0.f, kbl = 0.f;
-      if (BODY && env < p.n_envs) {
+      if (BODY && !PACK && env < p.n_envs) {
         kb0 = p.key_bias[env * T] * 1.4426950408889634f;
         kbl = p.key_bias[env * T + 1 + lane] * 1.4426950408889634f;
       }
       // single-query launches (the critic): lane = key in that row's softmax
       const bool one_row = !BODY && p.n_q == 1;
       float kb_row = -INFINITY;
-      if (one_row && lane < NKEYS && env < p.n_envs) kb_row = p.key_bias[env * T + lane] * 1.4426950408889634f;
+      if (!PACK && one_row && lane < NKEYS && env < p.n_envs) kb_row = p.key_bias[env * T + lane] * 1.4426950408889634f;
       bool fresh = true;
       for (int g = g_lo; g < g_hi && ok; ++g, ++gi) {
         const int buf = gi & 1;
         if (buf != set) continue;                       // the other set's group
         // body token's q0 | k0 | v0 of this warp's head: lanes 0..11 fetch one 16-byte piece each, long before use
         uint4 b0v = make_uint4(0, 0, 0, 0);
-        if (BODY && lane < 12 && env < p.n_envs)
+        uint4 b1v = b0v;
+        if (BODY && PACK) {                             // of all the tile's environments and both heads: 24 pieces each
+          auto piece = [&](int k) {
+            const int e = k / 24, m = k % 24;           // head m / 12, then q0, k0, v0 of four pieces
+            return *reinterpret_cast<const uint4*>(p.qkv0 + (tile_lo.x + e) * 3 * (int64_t)d + ((m % 12) >> 2) * d + (g * G + m / 12) * DH + (m & 3) * 8);
+          };
+          if (set_thread < 24 * n_tile_envs) b0v = piece(set_thread);
+          if (set_thread + EPT * TEAM * 32 < 24 * n_tile_envs) b1v = piece(set_thread + EPT * TEAM * 32);
+        } else if (BODY && lane < 12 && env < p.n_envs)
           b0v = *reinterpret_cast<const uint4*>(p.qkv0 + env * 3 * (int64_t)d + (lane >> 2) * d + (g * G + hh) * DH + (lane & 3) * 8);
         // A failed wait must not leave other workers stuck at the CTA-level barriers below: the
         // warp keeps going (on garbage) and everyone leaves together once one thread has sampled
@@ -349,8 +389,8 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
             // value residual (python/policy.py:604-615): the group's v columns are written out as
             // this block's own values and / or mixed with block 0's before the attention reads them
             const int vcol = (u_first + u) * 16 - 2 * GD;           // column inside the group's v section
-            const bool vres_rows = VRES && vcol >= 0 && lane < kT && env < p.n_envs;
-            const int64_t goff = (env * kT + lane) * d + g * GD + vcol;
+            const bool vres_rows = VRES && vcol >= 0 && (PACK ? trow < used : lane < kT && env < p.n_envs);
+            const int64_t goff = (PACK ? row0 + trow : env * kT + lane) * d + g * GD + vcol;
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
               const float4 b0 = b4[2 * j], b1 = b4[2 * j + 1];
@@ -433,74 +473,119 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
             }
           }
         }
-        if (BODY && mt_own == 0 && lane < 12) *reinterpret_cast<uint4*>(sB_g + ((env_l * 2 + hh) * 3 + (lane >> 2)) * 64 + (lane & 3) * 16) = b0v;
+        if (BODY && PACK) {
+          if (set_thread < 24 * n_tile_envs) *reinterpret_cast<uint4*>(sB_g + set_thread * 16) = b0v;
+          if (set_thread + EPT * TEAM * 32 < 24 * n_tile_envs) *reinterpret_cast<uint4*>(sB_g + (set_thread + EPT * TEAM * 32) * 16) = b1v;
+        } else if (BODY && mt_own == 0 && lane < 12) *reinterpret_cast<uint4*>(sB_g + ((env_l * 2 + hh) * 3 + (lane >> 2)) * 64 + (lane & 3) * 16) = b0v;
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
           if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&sh->acc_empty[buf]), 0));
           else mbar_arrive(smem_u32(&sh->acc_empty[buf]));
         }     // the TMEM buffer may be refilled
+        if (PACK && fresh && set_thread < BM + 32)
+          reinterpret_cast<int*>(sP_kb)[set_thread] = set_thread < BM ? __float_as_int(__int_as_float(sP_value) * 1.4426950408889634f) : sP_value;
         if (part == 0 && lane == 0) {
-          sh->quit[set * EPT + q] = *abort;
+          if (!PACK || q == 0) sh->quit[quit_at] = *abort;
           if (!S::INPLACE && p.out_tma) bulk_wait_read<0>();      // this env's previous output store has read its sO rows
         }
-        team_sync();                                    // the env's q|k|v rows are complete
-        if (*reinterpret_cast<volatile int*>(&sh->quit[set * EPT + q])) {
+        team_sync();                                    // the env's (PACK: the tile's) q|k|v rows are complete
+        if (*reinterpret_cast<volatile int*>(&sh->quit[quit_at])) {
           ok = false;
           break;
         }
-        if (fresh) {                                    // to base 2, where the loads have long landed
+        if (!PACK && fresh) {                           // to base 2, where the loads have long landed
 #pragma unroll
           for (int nt = 0; nt < 4; ++nt) kb[nt][0] *= 1.4426950408889634f, kb[nt][1] *= 1.4426950408889634f;
-          fresh = false;
         }
-        if (env < p.n_envs) {
+        fresh = false;
+        // ---- the body token beside the tile (one warp = one head of an env): its own output row, over the len object rows from
+        // r0 on; returns object row `lane` against the body key.  sb: q0 at +0, k0 at +64, v0 at +128
+        auto body_row = [&](const uint8_t* sb, int r0, int len, int piece0, float kbl, float kb0, __half* orow) -> float {
+          float x_lane = 0.f;
+          const float scale = rsqrtf((float)DH) * 1.4426950408889634f;
+          float sc = 0.f, s00 = 0.f;
+          const int own_row = PACK ? min(r0 + lane, BM - 1) : r0 + lane;
+#pragma unroll
+          for (int ch = 0; ch < DH / 8; ++ch) {
+            const uint4 q0v = *reinterpret_cast<const uint4*>(sb + ch * 16);
+            const uint4 k0v = *reinterpret_cast<const uint4*>(sb + 64 + ch * 16);
+            const uint4 qv = *reinterpret_cast<const uint4*>(sQ_g + section_at<LDQ>(0, own_row, piece0 + ch));
+            const uint4 kv = *reinterpret_cast<const uint4*>(sQ_g + SECTION + section_at<LDQ>(0, own_row, piece0 + ch));
+            const __half2* q0h = reinterpret_cast<const __half2*>(&q0v);
+            const __half2* k0h = reinterpret_cast<const __half2*>(&k0v);
+            const __half2* qh = reinterpret_cast<const __half2*>(&qv);
+            const __half2* kh = reinterpret_cast<const __half2*>(&kv);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const float2 a0 = __half22float2(q0h[e]), b0 = __half22float2(k0h[e]);
+              const float2 a = __half22float2(qh[e]), b = __half22float2(kh[e]);
+              x_lane = fmaf(a.x, b0.x, fmaf(a.y, b0.y, x_lane));       // object row `lane` against the body key
+              sc = fmaf(a0.x, b.x, fmaf(a0.y, b.y, sc));               // body row against object key `lane`
+              s00 = fmaf(a0.x, b0.x, fmaf(a0.y, b0.y, s00));           // body row against the body key
+            }
+          }
+          {   // the body token's own output row: softmax over the 32 object keys (one per lane) and the body key
+            sc = PACK && lane >= len ? -INFINITY : fmaf(sc, scale, kbl);
+            s00 = fmaf(s00, scale, kb0);
+            const float mx = fmaxf(warp_max(sc), s00);
+            const float pj = ex2_approx(sc - mx), p00 = ex2_approx(s00 - mx);
+            const float inv = rcp_approx(warp_sum(pj) + p00);
+            const __half* v0h = reinterpret_cast<const __half*>(sb + 128);
+            const uint8_t* v_g = sQ_g + 2 * SECTION;                   // column `lane` of the head's v rows
+            float acc = p00 * __half2float(v0h[lane]);
+#pragma unroll 8
+            for (int j = 0; j < len; ++j)
+              acc = fmaf(__shfl_sync(0xffffffffu, pj, j),
+                         __half2float(*reinterpret_cast<const __half*>(v_g + section_at<LDQ>(0, r0 + j, piece0 + (lane >> 3)) + (lane & 7) * 2)), acc);
+            orow[lane] = __float2half_rn(acc * inv);
+          }
+          return x_lane;
+        };
+        if (PACK) {
+          // (environment, head) pairs, or with one head a group (environment, 16 query rows): the first rows of all, then the others
+          const bool two = !one_row && (p.out_tma || p.n_q > 16);        // more than 16 query rows possible
+          const int n_items = G == 2 || two ? 2 * n_tile_envs : n_tile_envs;
+          for (int it = (warp - 2) % (EPT * TEAM); it < n_items; it += EPT * TEAM) {
+            const int mt0 = G == 2 ? 0 : it >= n_tile_envs, j = G == 2 ? it >> 1 : it - mt0 * n_tile_envs, hd = G == 2 ? it & 1 : 0;
+            const int r0 = sP_row[j], len = sP_row[j + 1] - r0, n_q = (p.out_tma ? len : p.n_q) - mt0 * 16, piece0 = hd * (DH / 8);
+            const int64_t e = tile_lo.x + j;
+            float x_lane = 0.f;
+            const uint8_t* sb = sB_g + (j * 2 + hd) * 192;
+            if constexpr (BODY)                          // (the body token's key bias is 0)
+              x_lane = body_row(sb, r0, len, piece0, lane < len ? sP_kb[r0 + lane] : -INFINITY, 0.f, p.out + e * (int64_t)p.ldo + (g * G + hd) * DH);
+            if (n_q <= 0 || (BODY && p.body_only)) continue;
+            if (one_row) {
+              attend_one_row<DH, LDQ, kT>(sQ_g, sQ_g + SECTION, sQ_g + 2 * SECTION, r0 + p.q_first, piece0, lane < len ? sP_kb[r0 + lane] : -INFINITY,
+                                          p.out + e * (int64_t)p.ldo + (g * G + hd) * DH, lane, r0, len);
+              continue;
+            }
+#pragma unroll
+            for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+              for (int c = 0; c < 2; ++c) {
+                const int key = nt * 8 + (lane & 3) * 2 + c;
+                kb[nt][c] = key < len ? sP_kb[r0 + key] : -INFINITY;
+              }
+            __half* out_rows = p.out + (e * p.n_q + mt0 * 16) * (int64_t)p.ldo + (g * G + hd) * DH;
+            auto attend = [&](auto mt, auto kt) {
+              attend_pair<decltype(mt)::value, DH, LDQ, GD * 2, BODY, true, decltype(kt)::value>(
+                  sQ, sQ + SECTION, sQ + 2 * SECTION, r0 + p.q_first + mt0 * 16, piece0, kb, n_q, out_rows, p.ldo, lane,
+                  p.out_tma ? sO_g : nullptr, r0 + mt0 * 16, piece0, x_lane, 0.f, reinterpret_cast<const __half*>(sb + 128), r0, len);
+            };
+            if (len <= 16) attend(Int<1>(), Int<1>());
+            else if (G == 2 && n_q > 16) attend(Int<2>(), Int<2>());
+            else attend(Int<1>(), Int<2>());
+          }
+        } else if (env < p.n_envs) {
           const uint32_t rows = sQ + (env_l * EROWS) * LDQ;             // the env's q rows; k and v at SECTION and 2 SECTION
           const int q_row0 = p.q_first + mt_own * 16, piece0 = hh * (DH / 8);
           __half* out_pair = p.out + (env * p.n_q + mt_own * 16) * (int64_t)p.ldo + (g * G + hh) * DH;
           const int n_q = p.n_q - mt_own * 16;      // query rows left from this warp's first one
           uint8_t* so_tile = p.out_tma ? sO_g : nullptr;
           if constexpr (BODY) {
-            // ---- the body token beside the tile (one warp = one head of the env's group)
-            const uint8_t* rows_g = sQ_g + (env_l * EROWS) * LDQ;
-            const uint8_t* sb = sB_g + (env_l * 2 + hh) * 192;           // q0 at +0, k0 at +64, v0 at +128
-            const float scale = rsqrtf((float)DH) * 1.4426950408889634f;
-            float x_lane = 0.f, sc = 0.f, s00 = 0.f;
-#pragma unroll
-            for (int ch = 0; ch < DH / 8; ++ch) {
-              const uint4 q0v = *reinterpret_cast<const uint4*>(sb + ch * 16);
-              const uint4 k0v = *reinterpret_cast<const uint4*>(sb + 64 + ch * 16);
-              const uint4 qv = *reinterpret_cast<const uint4*>(rows_g + section_at<LDQ>(0, lane, piece0 + ch));
-              const uint4 kv = *reinterpret_cast<const uint4*>(rows_g + SECTION + section_at<LDQ>(0, lane, piece0 + ch));
-              const __half2* q0h = reinterpret_cast<const __half2*>(&q0v);
-              const __half2* k0h = reinterpret_cast<const __half2*>(&k0v);
-              const __half2* qh = reinterpret_cast<const __half2*>(&qv);
-              const __half2* kh = reinterpret_cast<const __half2*>(&kv);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const float2 a0 = __half22float2(q0h[e]), b0 = __half22float2(k0h[e]);
-                const float2 a = __half22float2(qh[e]), b = __half22float2(kh[e]);
-                x_lane = fmaf(a.x, b0.x, fmaf(a.y, b0.y, x_lane));       // object row `lane` against the body key
-                sc = fmaf(a0.x, b.x, fmaf(a0.y, b.y, sc));               // body row against object key `lane`
-                s00 = fmaf(a0.x, b0.x, fmaf(a0.y, b0.y, s00));           // body row against the body key
-              }
-            }
-            {   // the body token's own output row: softmax over the 32 object keys (one per lane) and the body key
-              sc = fmaf(sc, scale, kbl);
-              s00 = fmaf(s00, scale, kb0);
-              const float mx = fmaxf(warp_max(sc), s00);
-              const float pj = ex2_approx(sc - mx), p00 = ex2_approx(s00 - mx);
-              const float inv = rcp_approx(warp_sum(pj) + p00);
-              const __half* v0h = reinterpret_cast<const __half*>(sb + 128);
-              const uint8_t* v_g = rows_g + 2 * SECTION;                   // column `lane` of the head's v rows
-              float acc = p00 * __half2float(v0h[lane]);
-#pragma unroll 8
-              for (int j = 0; j < EROWS; ++j)
-                acc = fmaf(__shfl_sync(0xffffffffu, pj, j),
-                           __half2float(*reinterpret_cast<const __half*>(v_g + section_at<LDQ>(0, j, piece0 + (lane >> 3)) + (lane & 7) * 2)), acc);
-              __half* orow = p.out + (env * (p.body_only ? 1 : T)) * (int64_t)p.ldo + (g * G + hh) * DH;
-              orow[lane] = __float2half_rn(acc * inv);
-            }
+            const uint8_t* sb = sB_g + (env_l * 2 + hh) * 192;
+            const float x_lane = body_row(sb, env_l * EROWS, EROWS, piece0, kbl, kb0, p.out + (env * (p.body_only ? 1 : T)) * (int64_t)p.ldo + (g * G + hh) * DH);
             if (!p.body_only)
               attend_pair<2, DH, LDQ, GD * 2, true>(rows, rows + SECTION, rows + 2 * SECTION, q_row0, piece0, kb, n_q, out_pair, p.ldo, lane,
                                                     so_tile, env_l * EROWS, piece0, x_lane, kb0, reinterpret_cast<const __half*>(sb + 128));
@@ -524,7 +609,23 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
         }
         if (p.out_tma) fence_proxy_async_smem();                         // this thread's sO writes -> the TMA engine
         team_sync();                                                     // the env's rows may be overwritten
-        if (p.out_tma && part == 0 && lane == 0 && env < p.n_envs) {     // token rows 29..31 of the box are clipped
+        if (PACK) {
+          // 32 rows as one box; what is left of the last ones row by row, for the rows behind them are another tile's
+          if (p.out_tma && part == 0 && used - q * 32 >= 32) {
+            if (lane == 0) {
+              tma_store_2d(&tm_o, g * GD, (int)row0 + q * 32, sO + (uint32_t)(q * 32) * (uint32_t)(GD * 2));
+              bulk_commit();
+            }
+          } else if (p.out_tma && part == 0) {
+            constexpr int PIECES = GD / 8;
+            for (int k = lane; k < (used - q * 32) * PIECES; k += 32) {
+              const int row = q * 32 + k / PIECES, piece = k % PIECES;
+              *reinterpret_cast<uint4*>(p.out + (p.rows_ahead + row0 + row) * (int64_t)p.ldo + g * GD + piece * 8) =
+                  *reinterpret_cast<const uint4*>(sO_g + row * (GD * 2) + (GD == 64 ? (piece ^ (row & 7)) << 4 : piece << 4));
+            }
+            __syncwarp();
+          }
+        } else if (p.out_tma && part == 0 && lane == 0 && env < p.n_envs) {     // token rows 29..31 of the box are clipped
           tma_store_3d(&tm_o, g * GD, BODY ? p.tok0 : 0, (int)env, sO + (uint32_t)(q * EROWS) * (uint32_t)(GD * 2));
           bulk_commit();
         }
@@ -544,27 +645,27 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
   }
 }
 
-template <int DH, int G, bool VRES, bool BODY>
+template <int DH, int G, bool VRES, bool BODY, bool PACK = false>
 cudaError_t prepare() {
   const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  cudaError_t e = cudaFuncSetAttribute(attn_block_kernel<DH, G, false, VRES, BODY>, at, Shape<DH, G, false>::SMEM_BYTES);
+  cudaError_t e = cudaFuncSetAttribute(attn_block_kernel<DH, G, false, VRES, BODY, PACK>, at, Shape<DH, G, false, PACK>::SMEM_BYTES);
   if constexpr (DH != 48)
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_block_kernel<DH, G, true, VRES, BODY>, at, Shape<DH, G, true>::SMEM_BYTES);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_block_kernel<DH, G, true, VRES, BODY, PACK>, at, Shape<DH, G, true, PACK>::SMEM_BYTES);
   return e;
 }
-template <int DH, int G, bool VRES, bool BODY>
+template <int DH, int G, bool VRES, bool BODY, bool PACK = false>
 void launch(bool pair, const CUtensorMap& tm_h, const CUtensorMap& tm_w, const CUtensorMap& tm_o, const Params& p, cudaStream_t stream) {
   if constexpr (DH != 48)
     if (pair) {
-      using S = Shape<DH, G, true>;
+      using S = Shape<DH, G, true, PACK>;
       const int pairs = (p.n_tiles + 1) / 2, places = sm_count() / 2;
-      launch_kernel<2>(attn_block_kernel<DH, G, true, VRES, BODY>, 2 * (pairs < places ? pairs : places), S::THREADS, S::SMEM_BYTES, stream,
+      launch_kernel<2>(attn_block_kernel<DH, G, true, VRES, BODY, PACK>, 2 * (pairs < places ? pairs : places), S::THREADS, S::SMEM_BYTES, stream,
                        tm_h, tm_w, tm_o, p);
       return;
     }
-  using S = Shape<DH, G, false>;
+  using S = Shape<DH, G, false, PACK>;
   const int items = p.n_tiles * p.split, grid = items < sm_count() ? items : sm_count();
-  launch_kernel(attn_block_kernel<DH, G, false, VRES, BODY>, grid, S::THREADS, S::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
+  launch_kernel(attn_block_kernel<DH, G, false, VRES, BODY, PACK>, grid, S::THREADS, S::SMEM_BYTES, stream, tm_h, tm_w, tm_o, p);
 }
 }  // namespace
 
@@ -572,7 +673,7 @@ bool attn_block_ok(const AttnBlockArgs& a) {
   if (a.d % 64 != 0 || a.d < 64 || a.n_heads < 1 || a.d % a.n_heads != 0) return false;
   const int dh = a.d / a.n_heads;
   if (!((dh == 32 && a.n_heads % 2 == 0) || dh == 48 || dh == 64)) return false;
-  if (a.d > (dh == 64 ? Shape<64, 1, false>::MAX_D : dh == 48 ? Shape<48, 1, false>::MAX_D : Shape<32, 2, false>::MAX_D)) return false;
+  if (a.d > (dh == 64 ? Shape<64, 1, false, false>::MAX_D : dh == 48 ? Shape<48, 1, false, false>::MAX_D : Shape<32, 2, false, false>::MAX_D)) return false;
   if (a.n_envs < 1 || a.n_envs > 0x7fffffffLL / (BM * 2)) return false;
   if (!aligned16(a.h) || !aligned16(a.wg) || !aligned16(a.bg) || !aligned16(a.out) || (a.ldh % 8) || (a.ldo % 8)) return false;
   if (a.body) {      // one body token + 32 object tokens per env; all rows out, or the body row only
@@ -601,13 +702,27 @@ int attn_block(const AttnBlockArgs& a, cudaStream_t stream) {
   // (M = 256 wants multiples of 32 columns: 144 would compute 16 for nothing, 800 us against 790 at 65,536 envs x 192).
   const int n_tiles = (int)((a.n_envs + EPT - 1) / EPT);
   const bool pair = dh != 48 && n_tiles >= 4 * sm_count();
-  CUtensorMap tm_h, tm_w;
-  if (!make_tmap_env3d(&tm_h, a.h, a.n_envs, T, a.d, a.ldh, 64, EROWS, EPT)) return BSRL_ERR_CUDA;
-  if (!make_tmap_f16(&tm_w, a.wg, 3 * a.d, a.d, a.d, dh == 48 ? 144 : pair ? 96 : 192)) return BSRL_ERR_CUDA;
-  // all query rows: an env's output for a group is contiguous rows x 128 (two heads of 32) or 96 bytes (one of 48) = one TMA store
+  CUtensorMap tm_h, tm_w, tm_o;
+  // packed rows of the body-token layout: the body rows come first, the tiles are of what follows
+  const bool pack = a.rows.start != nullptr;
+  const int64_t ahead = pack && a.body ? a.n_envs : 0, bound = a.n_envs * T - ahead;
+  // Where all slots are live the packed rows ARE the full layout, and its kernel, whose warps wait for one another by pairs only, is
+  // the faster one: 65,536 environments at d 256, all slots live, take 1.037 times as long as in the full layout with the
+  // packed kernel alone and 1.008 times with both.  The host cannot tell, so long runs launch both, and the one that the rows are
+  // not for returns (2 us).
+  const bool full = pack && !a.body && n_tiles >= 4 * sm_count();
   const bool out_tma = a.q_first == 0 && a.n_q == T;
-  CUtensorMap tm_o = tm_h;
-  if (out_tma && !make_tmap_env3d(&tm_o, a.out, a.n_envs, T, a.d, a.ldo, dh == 48 ? 48 : 64, EROWS, 1)) return BSRL_ERR_CUDA;
+  const int cols = dh == 48 ? 48 : 64;
+  // all query rows: a group's output of 32 tile rows x 128 bytes (two heads of 32) or 96 (one of 48) is one TMA store, or without
+  // packed rows an env's
+  auto maps = [&](bool packed) {
+    if (packed ? !make_tmap_f16(&tm_h, a.h + ahead * a.ldh, bound, a.d, a.ldh, BM) : !make_tmap_env3d(&tm_h, a.h, a.n_envs, T, a.d, a.ldh, 64, EROWS, EPT))
+      return false;
+    tm_o = tm_h;
+    return !out_tma || (packed ? make_tmap_rows(&tm_o, a.out + ahead * a.ldo, 2, bound, a.d, a.ldo, 32, cols * 2)
+                               : make_tmap_env3d(&tm_o, a.out, a.n_envs, T, a.d, a.ldo, cols, EROWS, 1));
+  };
+  if (!make_tmap_f16(&tm_w, a.wg, 3 * a.d, a.d, a.d, dh == 48 ? 144 : pair ? 96 : 192)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("attn_block_kernel set-up", [] {
     cudaError_t e = prepare<32, 2, false, false>();
@@ -617,6 +732,13 @@ int attn_block(const AttnBlockArgs& a, cudaStream_t stream) {
     if (e == cudaSuccess) e = prepare<48, 1, true, false>();
     if (e == cudaSuccess) e = prepare<64, 1, false, false>();
     if (e == cudaSuccess) e = prepare<64, 1, true, false>();
+    if (e == cudaSuccess) e = prepare<32, 2, false, false, true>();
+    if (e == cudaSuccess) e = prepare<32, 2, true, false, true>();
+    if (e == cudaSuccess) e = prepare<32, 2, false, true, true>();
+    if (e == cudaSuccess) e = prepare<48, 1, false, false, true>();
+    if (e == cudaSuccess) e = prepare<48, 1, true, false, true>();
+    if (e == cudaSuccess) e = prepare<64, 1, false, false, true>();
+    if (e == cudaSuccess) e = prepare<64, 1, true, false, true>();
     return e;
   });
   if (rc != BSRL_OK) return rc;
@@ -631,17 +753,32 @@ int attn_block(const AttnBlockArgs& a, cudaStream_t stream) {
   // envs x 256 columns 214 -> 208 us, 128 envs 205 -> 186, 100 envs of 512 613 -> 501.
   const int groups = a.d / (dh == 32 ? 64 : dh);
   p.split = 1;
-  for (int s = 2; s <= groups && n_tiles * s <= sm_count() && (n_tiles * (s + 1) <= sm_count() || 2 * s <= groups); s *= 2) p.split = s;
+  for (int s = 2; !pack && s <= groups && n_tiles * s <= sm_count() && (n_tiles * (s + 1) <= sm_count() || 2 * s <= groups); s *= 2) p.split = s;
   p.bias = a.bg; p.key_bias = a.key_bias; p.out = a.out; p.ldo = a.ldo;
   p.v_out = a.v_out; p.v0 = a.v0; p.vres = a.vres;
   p.out_tma = out_tma ? 1 : 0;
   p.tokens = T; p.tok0 = a.body ? 1 : 0; p.body_only = (a.body && a.n_q == 1) ? 1 : 0; p.qkv0 = a.qkv0;
+  p.rows = a.rows;
+  p.rows_ahead = ahead;
+  p.full_rows = 0;
   p.status = status;
   const bool vres = a.v_out || a.v0;
-  auto* run = a.body ? launch<32, 2, false, true> : dh == 32 ? (vres ? launch<32, 2, true, false> : launch<32, 2, false, false>)
-            : dh == 48 ? (vres ? launch<48, 1, true, false> : launch<48, 1, false, false>)
-                       : (vres ? launch<64, 1, true, false> : launch<64, 1, false, false>);
-  run(pair, tm_h, tm_w, tm_o, p, stream);
+  if (!pack || full) {
+    p.full_rows = full ? (int)(a.n_envs * T) : 0;
+    if (!maps(false)) return BSRL_ERR_CUDA;
+    auto* run = a.body ? launch<32, 2, false, true> : dh == 32 ? (vres ? launch<32, 2, true, false> : launch<32, 2, false, false>)
+              : dh == 48 ? (vres ? launch<48, 1, true, false> : launch<48, 1, false, false>)
+                         : (vres ? launch<64, 1, true, false> : launch<64, 1, false, false>);
+    run(pair, tm_h, tm_w, tm_o, p, stream);
+    BSRL_LAUNCH_OK("attn_block_kernel");
+  }
+  if (pack) {
+    if (!maps(true)) return BSRL_ERR_CUDA;
+    auto* run = a.body ? launch<32, 2, false, true, true> : dh == 32 ? (vres ? launch<32, 2, true, false, true> : launch<32, 2, false, false, true>)
+              : dh == 48 ? (vres ? launch<48, 1, true, false, true> : launch<48, 1, false, false, true>)
+                         : (vres ? launch<64, 1, true, false, true> : launch<64, 1, false, false, true>);
+    run(pair, tm_h, tm_w, tm_o, p, stream);
+  }
   BSRL_LAUNCH_OK("attn_block_kernel");
   return BSRL_OK;
 }

@@ -8,6 +8,8 @@
 // attn29_bwd_kernel of the reference does (python/beat_arena_env/csrc/small_attn.cu:345-463).  The whole
 // problem of one (env, head) pair -- at most 32 x 64 values per matrix -- lives in the warp's shared-memory
 // tile; the five products run on m16n8k16 MMAs with fp32 accumulation, P and dS rounded to fp16 as operands.
+#include <type_traits>
+
 #include "kernels.cuh"
 #include "attend.cuh"
 #include "tc5.cuh"
@@ -42,11 +44,22 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
 // 32, us, before / now (at copy speed): 29 queries 407 / 350 (260), 5 queries 276 / 226 (199), 1 query 272 / 224 (152).
 template <int DH, int MT>
 __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(const __half* __restrict__ qkv, int ld, const float* __restrict__ key_bias,
-                                                               int64_t n_pairs, int d, int n_heads, int q_first, int n_q,
+                                                               int64_t n_pairs, int d, int n_heads, int q_first, int n_queries,
                                                                const __half* __restrict__ g_out, int ldgo, __half* __restrict__ gq,
                                                                int ldq, __half* __restrict__ gk, int ldk, __half* __restrict__ gv,
-                                                               int ldv, int wide) {
+                                                               int ldv, int wide, const int* __restrict__ start) {
   pdl_begin();
+  // packed token rows: an environment's first row, its rows and its queries (as many where all are asked for)
+  struct Rows {
+    int64_t row0, q0;
+    int tokens, n_q;
+  };
+  auto rows_of = [&](int64_t env) {
+    const int64_t row0 = start ? start[env] : env * kT;
+    const int tokens = start ? (int)(start[env + 1] - row0) : kT;
+    const bool all = n_queries == kT;
+    return Rows{row0, all ? row0 : env * n_queries, tokens, all ? tokens : n_queries};
+  };
   constexpr int CH = DH / 8, ROW = DH * 2;
   constexpr int QR = 16 * MT;                         // staged query rows
   constexpr int TILE = (2 * QR + 2 * kKeys) * ROW, TILES = tiles_of<DH>(), kWarps = warps_of<DH, MT>();
@@ -65,17 +78,18 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
     if (pair < n_pairs) {
       int head;
       const int64_t env = div_index(pair, n_heads, &head);
-      const __half* base = qkv + env * kT * (int64_t)ld + head * DH;
-      for (int c = lane; c < kKeys * CH; c += 32) {
+      const Rows e = rows_of(env);
+      const __half* base = qkv + e.row0 * ld + head * DH;
+      for (int c = lane; c < (e.tokens <= 16 ? 16 : kKeys) * CH; c += 32) {
         const int row = c / CH, ch = c % CH;
-        const bool live = row < kT, asks = row < n_q;
+        const bool live = row < e.tokens, asks = row < e.n_q;
         const __half* r = base + (int64_t)(live ? row : 0) * ld + ch * 8;
         const uint32_t at = at0 + tile_at<DH>(row, ch);
         cp_async16(at + 2 * QR * ROW, r + d, live);
         cp_async16(at + (2 * QR + kKeys) * ROW, r + 2 * d, live);
         if (row < QR) {
           cp_async16(at, base + (int64_t)(asks ? q_first + row : 0) * ld + ch * 8, asks);
-          cp_async16(at + QR * ROW, g_out + (env * n_q + (asks ? row : 0)) * (int64_t)ldgo + head * DH + ch * 8, asks);
+          cp_async16(at + QR * ROW, g_out + (e.q0 + (asks ? row : 0)) * (int64_t)ldgo + head * DH + ch * 8, asks);
         }
       }
     }
@@ -85,12 +99,13 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
     if (pair >= n_pairs) return;
     int head;
     const int64_t env = div_index(pair, n_heads, &head);
+    const int tokens = rows_of(env).tokens;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         const int key = nt * 8 + tig * 2 + e;
-        kb[nt][e] = key < kT ? key_bias[env * kT + key] : -INFINITY;
+        kb[nt][e] = key < tokens ? key_bias[env * kT + key] : -INFINITY;
       }
   };
   const int64_t first = (int64_t)blockIdx.x * kWarps + warp;
@@ -116,159 +131,166 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
     }
     __syncwarp();
 
-    // ---- S = q k^T and dP = dO v^T
-    float s[MT][4][4], dp[MT][4][4];
+    // M tiles of 16 queries, K of 16 keys: short environments (packed rows) leave the second ones out, which hold exact zeros
+    auto products = [&](auto m_tiles, auto k_tiles) {
+      constexpr int M = decltype(m_tiles)::value, K = decltype(k_tiles)::value;
+      // ---- S = q k^T and dP = dO v^T
+      float s[M][2 * K][4], dp[M][2 * K][4];
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
+      for (int mt = 0; mt < M; ++mt)
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < 2 * K; ++nt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) s[mt][nt][e] = dp[mt][nt][e] = 0.f;
+          for (int e = 0; e < 4; ++e) s[mt][nt][e] = dp[mt][nt][e] = 0.f;
 #pragma unroll
-    for (int ks = 0; ks < DH / 16; ++ks) {
-      uint32_t a[MT][4], ag[MT][4];
+      for (int ks = 0; ks < DH / 16; ++ks) {
+        uint32_t a[M][4], ag[M][4];
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        const uint32_t at = tile_at<DH>(mt * 16 + ra, ks * 2 + ca);
-        ldmatrix_x4(a[mt], sq_u + at);
-        ldmatrix_x4(ag[mt], sg_u + at);
-      }
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        uint32_t b[4], bv[4];
-        const uint32_t at = tile_at<DH>(j * 16 + rb, ks * 2 + cb);
-        ldmatrix_x4(b, sk_u + at);
-        ldmatrix_x4(bv, sv_u + at);
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          mma_f16(s[mt][2 * j], a[mt], b[0], b[1]);
-          mma_f16(s[mt][2 * j + 1], a[mt], b[2], b[3]);
-          mma_f16(dp[mt][2 * j], ag[mt], bv[0], bv[1]);
-          mma_f16(dp[mt][2 * j + 1], ag[mt], bv[2], bv[3]);
-        }
-      }
-    }
-    uint32_t tp[MT][2][4], td[MT][2][4];                // P^T and dS^T, A fragments of 16 keys x 16 queries
-    uint32_t da[MT][2][4];                              // dS, A fragments of 16 queries x 16 keys
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt) {
-      // ---- P = softmax(S / sqrt(dh) + bias), dS = P (dP - rowsum(P dP)) / sqrt(dh); rows g (e = 0, 1) and g + 8 (e = 2, 3)
-      float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          s[mt][nt][e] = s[mt][nt][e] * scale + kb[nt][e & 1];
-          mx[e >> 1] = fmaxf(mx[e >> 1], s[mt][nt][e]);
+        for (int mt = 0; mt < M; ++mt) {
+          const uint32_t at = tile_at<DH>(mt * 16 + ra, ks * 2 + ca);
+          ldmatrix_x4(a[mt], sq_u + at);
+          ldmatrix_x4(ag[mt], sg_u + at);
         }
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-      }
-      float sum[2] = {0.f, 0.f};
+        for (int j = 0; j < K; ++j) {
+          uint32_t b[4], bv[4];
+          const uint32_t at = tile_at<DH>(j * 16 + rb, ks * 2 + cb);
+          ldmatrix_x4(b, sk_u + at);
+          ldmatrix_x4(bv, sv_u + at);
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          s[mt][nt][e] = expf(s[mt][nt][e] - mx[e >> 1]);
-          sum[e >> 1] += s[mt][nt][e];
+          for (int mt = 0; mt < M; ++mt) {
+            mma_f16(s[mt][2 * j], a[mt], b[0], b[1]);
+            mma_f16(s[mt][2 * j + 1], a[mt], b[2], b[3]);
+            mma_f16(dp[mt][2 * j], ag[mt], bv[0], bv[1]);
+            mma_f16(dp[mt][2 * j + 1], ag[mt], bv[2], bv[3]);
+          }
         }
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
-        sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
-        sum[r] = 1.f / sum[r];
       }
-      float dot[2] = {0.f, 0.f};
+      uint32_t tp[M][K][4], td[M][K][4];                // P^T and dS^T, A fragments of 16 keys x 16 queries
+      uint32_t da[M][K][4];                              // dS, A fragments of 16 queries x 16 keys
 #pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
+      for (int mt = 0; mt < M; ++mt) {
+        // ---- P = softmax(S / sqrt(dh) + bias), dS = P (dP - rowsum(P dP)) / sqrt(dh); rows g (e = 0, 1) and g + 8 (e = 2, 3)
+        float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          s[mt][nt][e] *= sum[e >> 1];                   // P
-          dot[e >> 1] += s[mt][nt][e] * dp[mt][nt][e];
-        }
+        for (int nt = 0; nt < 2 * K; ++nt)
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], 1);
-        dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], 2);
-      }
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) dp[mt][nt][e] = s[mt][nt][e] * (dp[mt][nt][e] - dot[e >> 1]) * scale;   // dS
-      // the accumulators as A fragments (as P feeds P v in the forward), and 8 x 8 blocks (8 queries x 8 keys) transposed
-#pragma unroll
-      for (int nt = 0; nt < 4; ++nt)
+          for (int e = 0; e < 4; ++e) {
+            s[mt][nt][e] = s[mt][nt][e] * scale + kb[nt][e & 1];
+            mx[e >> 1] = fmaxf(mx[e >> 1], s[mt][nt][e]);
+          }
 #pragma unroll
         for (int r = 0; r < 2; ++r) {
-          const uint32_t ds = pack_half2(dp[mt][nt][2 * r], dp[mt][nt][2 * r + 1]);
-          da[mt][nt >> 1][2 * (nt & 1) + r] = ds;
-          td[mt][nt >> 1][(nt & 1) + 2 * r] = transpose8x8(ds);
-          tp[mt][nt >> 1][(nt & 1) + 2 * r] = transpose8x8(pack_half2(s[mt][nt][2 * r], s[mt][nt][2 * r + 1]));
+          mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+          mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
         }
-    }
-    // ---- dQ = dS k
-    uint32_t oq16[MT][DH / 8][2];
+        float sum[2] = {0.f, 0.f};
 #pragma unroll
-    for (int j = 0; j < DH / 16; ++j) {
-      float oq[MT][2][4];
+        for (int nt = 0; nt < 2 * K; ++nt)
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
+          for (int e = 0; e < 4; ++e) {
+            s[mt][nt][e] = expf(s[mt][nt][e] - mx[e >> 1]);
+            sum[e >> 1] += s[mt][nt][e];
+          }
 #pragma unroll
-        for (int e = 0; e < 8; ++e) oq[mt][e >> 2][e & 3] = 0.f;
+        for (int r = 0; r < 2; ++r) {
+          sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 1);
+          sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], 2);
+          sum[r] = 1.f / sum[r];
+        }
+        float dot[2] = {0.f, 0.f};
 #pragma unroll
-      for (int ks = 0; ks < 2; ++ks) {
-        uint32_t b[4];
-        ldmatrix_x4_trans(b, sk_u + tile_at<DH>(ks * 16 + ra, j * 2 + ca));
+        for (int nt = 0; nt < 2 * K; ++nt)
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt) {
-          mma_f16(oq[mt][0], da[mt][ks], b[0], b[1]);
-          mma_f16(oq[mt][1], da[mt][ks], b[2], b[3]);
+          for (int e = 0; e < 4; ++e) {
+            s[mt][nt][e] *= sum[e >> 1];                   // P
+            dot[e >> 1] += s[mt][nt][e] * dp[mt][nt][e];
+          }
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], 1);
+          dot[r] += __shfl_xor_sync(0xffffffffu, dot[r], 2);
+        }
+#pragma unroll
+        for (int nt = 0; nt < 2 * K; ++nt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) dp[mt][nt][e] = s[mt][nt][e] * (dp[mt][nt][e] - dot[e >> 1]) * scale;   // dS
+        // the accumulators as A fragments (as P feeds P v in the forward), and 8 x 8 blocks (8 queries x 8 keys) transposed
+#pragma unroll
+        for (int nt = 0; nt < 2 * K; ++nt)
+#pragma unroll
+          for (int r = 0; r < 2; ++r) {
+            const uint32_t ds = pack_half2(dp[mt][nt][2 * r], dp[mt][nt][2 * r + 1]);
+            da[mt][nt >> 1][2 * (nt & 1) + r] = ds;
+            td[mt][nt >> 1][(nt & 1) + 2 * r] = transpose8x8(ds);
+            tp[mt][nt >> 1][(nt & 1) + 2 * r] = transpose8x8(pack_half2(s[mt][nt][2 * r], s[mt][nt][2 * r + 1]));
+          }
+      }
+      // ---- dQ = dS k
+      uint32_t oq16[M][DH / 8][2];
+#pragma unroll
+      for (int j = 0; j < DH / 16; ++j) {
+        float oq[M][2][4];
+#pragma unroll
+        for (int mt = 0; mt < M; ++mt)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) oq[mt][e >> 2][e & 3] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < K; ++ks) {
+          uint32_t b[4];
+          ldmatrix_x4_trans(b, sk_u + tile_at<DH>(ks * 16 + ra, j * 2 + ca));
+#pragma unroll
+          for (int mt = 0; mt < M; ++mt) {
+            mma_f16(oq[mt][0], da[mt][ks], b[0], b[1]);
+            mma_f16(oq[mt][1], da[mt][ks], b[2], b[3]);
+          }
+        }
+#pragma unroll
+        for (int mt = 0; mt < M; ++mt)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) oq16[mt][2 * j + (e >> 1)][e & 1] = pack_half2(oq[mt][e >> 1][2 * (e & 1)], oq[mt][e >> 1][2 * (e & 1) + 1]);
+      }
+      __syncwarp();                                       // k and v have been read: dK and dV take their places
+      // ---- dV = P^T dO and dK = dS^T q: key tiles as rows, the queries as the reduction dimension, 16 columns at a time
+#pragma unroll
+      for (int j = 0; j < DH / 16; ++j) {
+        float ov[K][2][4], ok[K][2][4];
+#pragma unroll
+        for (int e = 0; e < 8 * K; ++e) ov[e >> 3][(e >> 2) & 1][e & 3] = ok[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
+#pragma unroll
+        for (int qs = 0; qs < M; ++qs) {                 // 16 queries per step
+          uint32_t b[4], bq[4];
+          const uint32_t at = tile_at<DH>(qs * 16 + ra, j * 2 + ca);
+          ldmatrix_x4_trans(b, sg_u + at);
+          ldmatrix_x4_trans(bq, sq_u + at);
+#pragma unroll
+          for (int kt = 0; kt < K; ++kt) {
+            mma_f16(ov[kt][0], tp[qs][kt], b[0], b[1]);
+            mma_f16(ov[kt][1], tp[qs][kt], b[2], b[3]);
+            mma_f16(ok[kt][0], td[qs][kt], bq[0], bq[1]);
+            mma_f16(ok[kt][1], td[qs][kt], bq[2], bq[3]);
+          }
+        }
+#pragma unroll
+        for (int kt = 0; kt < K; ++kt) {
+          const uint32_t at = tile_at<DH>(kt * 16 + ra, j * 2 + ca);
+          tc5::stmatrix_x4(sv_u + at, pack_half2(ov[kt][0][0], ov[kt][0][1]), pack_half2(ov[kt][0][2], ov[kt][0][3]),
+                           pack_half2(ov[kt][1][0], ov[kt][1][1]), pack_half2(ov[kt][1][2], ov[kt][1][3]));
+          tc5::stmatrix_x4(sk_u + at, pack_half2(ok[kt][0][0], ok[kt][0][1]), pack_half2(ok[kt][0][2], ok[kt][0][3]),
+                           pack_half2(ok[kt][1][0], ok[kt][1][1]), pack_half2(ok[kt][1][2], ok[kt][1][3]));
         }
       }
+      __syncwarp();                                       // q has been read too
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
+      for (int mt = 0; mt < M; ++mt)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) oq16[mt][2 * j + (e >> 1)][e & 1] = pack_half2(oq[mt][e >> 1][2 * (e & 1)], oq[mt][e >> 1][2 * (e & 1) + 1]);
-    }
-    __syncwarp();                                       // k and v have been read: dK and dV take their places
-    // ---- dV = P^T dO and dK = dS^T q: key tiles as rows, the queries as the reduction dimension, 16 columns at a time
-#pragma unroll
-    for (int j = 0; j < DH / 16; ++j) {
-      float ov[2][2][4], ok[2][2][4];
-#pragma unroll
-      for (int e = 0; e < 16; ++e) ov[e >> 3][(e >> 2) & 1][e & 3] = ok[e >> 3][(e >> 2) & 1][e & 3] = 0.f;
-#pragma unroll
-      for (int qs = 0; qs < MT; ++qs) {                 // 16 queries per step
-        uint32_t b[4], bq[4];
-        const uint32_t at = tile_at<DH>(qs * 16 + ra, j * 2 + ca);
-        ldmatrix_x4_trans(b, sg_u + at);
-        ldmatrix_x4_trans(bq, sq_u + at);
-#pragma unroll
-        for (int kt = 0; kt < 2; ++kt) {
-          mma_f16(ov[kt][0], tp[qs][kt], b[0], b[1]);
-          mma_f16(ov[kt][1], tp[qs][kt], b[2], b[3]);
-          mma_f16(ok[kt][0], td[qs][kt], bq[0], bq[1]);
-          mma_f16(ok[kt][1], td[qs][kt], bq[2], bq[3]);
-        }
-      }
-#pragma unroll
-      for (int kt = 0; kt < 2; ++kt) {
-        const uint32_t at = tile_at<DH>(kt * 16 + ra, j * 2 + ca);
-        tc5::stmatrix_x4(sv_u + at, pack_half2(ov[kt][0][0], ov[kt][0][1]), pack_half2(ov[kt][0][2], ov[kt][0][3]),
-                         pack_half2(ov[kt][1][0], ov[kt][1][1]), pack_half2(ov[kt][1][2], ov[kt][1][3]));
-        tc5::stmatrix_x4(sk_u + at, pack_half2(ok[kt][0][0], ok[kt][0][1]), pack_half2(ok[kt][0][2], ok[kt][0][3]),
-                         pack_half2(ok[kt][1][0], ok[kt][1][1]), pack_half2(ok[kt][1][2], ok[kt][1][3]));
-      }
-    }
-    __syncwarp();                                       // q has been read too
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int j = 0; j < DH / 16; ++j)
-        tc5::stmatrix_x4(sq_u + tile_at<DH>(mt * 16 + ra, j * 2 + ca), oq16[mt][2 * j][0], oq16[mt][2 * j][1], oq16[mt][2 * j + 1][0], oq16[mt][2 * j + 1][1]);
-    __syncwarp();
+        for (int j = 0; j < DH / 16; ++j)
+          tc5::stmatrix_x4(sq_u + tile_at<DH>(mt * 16 + ra, j * 2 + ca), oq16[mt][2 * j][0], oq16[mt][2 * j][1], oq16[mt][2 * j + 1][0], oq16[mt][2 * j + 1][1]);
+      __syncwarp();
+    };
+    const Rows e = rows_of(env);
+    if (e.tokens <= 16) products(std::integral_constant<int, 1>(), std::integral_constant<int, 1>());
+    else products(std::integral_constant<int, MT>(), std::integral_constant<int, 2>());
     auto out = [&](const uint8_t* from, int rows, __half* dst, int64_t ldd) {
       for (int c = lane; c < rows * CH; c += 32) {
         const int row = c / CH, ch = c % CH;
@@ -282,15 +304,15 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
         }
       }
     };
-    out(sv, kT, gv + env * kT * (int64_t)ldv + head * DH, ldv);
-    out(sk, kT, gk + env * kT * (int64_t)ldk + head * DH, ldk);
-    out(sq, n_q, gq + env * n_q * (int64_t)ldq + head * DH, ldq);
+    out(sv, e.tokens, gv + e.row0 * ldv + head * DH, ldv);
+    out(sk, e.tokens, gk + e.row0 * ldk + head * DH, ldk);
+    out(sq, e.n_q, gq + e.q0 * ldq + head * DH, ldq);
   }
 }
 
 template <int DH, int MT>
 int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int d, int n_heads, int q_first, int n_q,
-           const __half* g_out, int ldgo, __half* gq, int ldq, __half* gk, int ldk, __half* gv, int ldv, cudaStream_t stream) {
+           const __half* g_out, int ldgo, __half* gq, int ldq, __half* gk, int ldk, __half* gv, int ldv, cudaStream_t stream, const int* start) {
   constexpr int kWarps = warps_of<DH, MT>(), smem = kWarps * tiles_of<DH>() * (2 * 16 * MT + 2 * kKeys) * DH * 2;
   static DeviceOnce once;
   int rc = once.run("attn_bwd_kernel set-up", [] {
@@ -304,21 +326,21 @@ int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
   launch_kernel(attn_bwd_kernel<DH, MT>, (unsigned)blocks, kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d, n_heads, q_first, n_q, g_out,
-                                                                          ldgo, gq, ldq, gk, ldk, gv, ldv, wide);
+                                                                          ldgo, gq, ldq, gk, ldk, gv, ldv, wide, start);
   BSRL_LAUNCH_OK("attn_bwd_kernel");
   return BSRL_OK;
 }
 template <int DH>
 int launch_mt(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int d, int n_heads, int q_first, int n_q,
-              const __half* g_out, int ldgo, __half* gq, int ldq, __half* gk, int ldk, __half* gv, int ldv, cudaStream_t stream) {
-  if (n_q > 16) return launch<DH, 2>(qkv, ld, key_bias, n_envs, d, n_heads, q_first, n_q, g_out, ldgo, gq, ldq, gk, ldk, gv, ldv, stream);
-  return launch<DH, 1>(qkv, ld, key_bias, n_envs, d, n_heads, q_first, n_q, g_out, ldgo, gq, ldq, gk, ldk, gv, ldv, stream);
+              const __half* g_out, int ldgo, __half* gq, int ldq, __half* gk, int ldk, __half* gv, int ldv, cudaStream_t stream, const int* start) {
+  if (n_q > 16) return launch<DH, 2>(qkv, ld, key_bias, n_envs, d, n_heads, q_first, n_q, g_out, ldgo, gq, ldq, gk, ldk, gv, ldv, stream, start);
+  return launch<DH, 1>(qkv, ld, key_bias, n_envs, d, n_heads, q_first, n_q, g_out, ldgo, gq, ldq, gk, ldk, gv, ldv, stream, start);
 }
 }  // namespace
 
 int attention29_bwd(const __half* qkv, int ld_qkv, const float* key_bias, int64_t n_envs, int d, int n_heads, int q_first,
                     int n_q, const __half* g_out, int ldgo, __half* gq, int ldq, __half* gk, int ldk, __half* gv, int ldv,
-                    cudaStream_t stream) {
+                    cudaStream_t stream, const int* start) {
   if (!qkv || !key_bias || !g_out || !gq || !gk || !gv) {
     set_error("attention_bwd: NULL operand");
     return BSRL_ERR_NULL;
@@ -330,9 +352,9 @@ int attention29_bwd(const __half* qkv, int ld_qkv, const float* key_bias, int64_
   }
   if (n_envs == 0) return BSRL_OK;
   switch (d / n_heads) {
-    case 32: return launch_mt<32>(qkv, ld_qkv, key_bias, n_envs, d, n_heads, q_first, n_q, g_out, ldgo, gq, ldq, gk, ldk, gv, ldv, stream);
-    case 48: return launch_mt<48>(qkv, ld_qkv, key_bias, n_envs, d, n_heads, q_first, n_q, g_out, ldgo, gq, ldq, gk, ldk, gv, ldv, stream);
-    case 64: return launch_mt<64>(qkv, ld_qkv, key_bias, n_envs, d, n_heads, q_first, n_q, g_out, ldgo, gq, ldq, gk, ldk, gv, ldv, stream);
+    case 32: return launch_mt<32>(qkv, ld_qkv, key_bias, n_envs, d, n_heads, q_first, n_q, g_out, ldgo, gq, ldq, gk, ldk, gv, ldv, stream, start);
+    case 48: return launch_mt<48>(qkv, ld_qkv, key_bias, n_envs, d, n_heads, q_first, n_q, g_out, ldgo, gq, ldq, gk, ldk, gv, ldv, stream, start);
+    case 64: return launch_mt<64>(qkv, ld_qkv, key_bias, n_envs, d, n_heads, q_first, n_q, g_out, ldgo, gq, ldq, gk, ldk, gv, ldv, stream, start);
     default:
       set_error("attention_bwd: head_dim %d unsupported (32, 48 or 64)", d / n_heads);
       return BSRL_ERR_UNSUPPORTED;

@@ -29,8 +29,10 @@ __global__ void __launch_bounds__(256, ln_bwd_resident<kMaxVec>()) ln_bwd_kernel
                                                      const float* __restrict__ gamma, float eps, const void* __restrict__ gy,
                                                      int64_t ldgy, const float* gres, float* gx_out, int64_t ldg, RowMap gmap,
                                                      __half* __restrict__ gx16, int64_t ldg16,
-                                                     float* __restrict__ ggamma, float* __restrict__ gbeta, int64_t rows, int d) {
+                                                     float* __restrict__ ggamma, float* __restrict__ gbeta, int64_t row_bound, int d,
+                                                     const int* n_rows, int64_t n_less) {
   pdl_begin();
+  const int64_t rows = n_rows ? n_rows[0] - n_less : row_bound;
   extern __shared__ float s_part[];                  // [2][d]
   for (int i = threadIdx.x; i < 2 * d; i += blockDim.x) s_part[i] = 0.f;
   __syncthreads();
@@ -122,9 +124,10 @@ __global__ void __launch_bounds__(256, ln_bwd_resident<kMaxVec>()) ln_bwd_kernel
 // out[c] += sum_r in[r, c] (fp16 rows): bias gradients.  A warp covers 256 consecutive columns of a row with
 // 16-byte loads, the 8 warps of a block take rows in turn (four in flight each); partial sums meet in shared
 // memory and leave as one atomic per column and block.  n % 8 == 0, ld % 8 == 0, 16-byte aligned base.
-__global__ void __launch_bounds__(256) colsum_kernel(const __half* __restrict__ in, int64_t ld, int64_t rows, int n,
-                                                     int64_t chunk, float* __restrict__ out) {
+__global__ void __launch_bounds__(256) colsum_kernel(const __half* __restrict__ in, int64_t ld, int64_t row_bound, int n,
+                                                     int64_t chunk, float* __restrict__ out, const int* n_rows, int64_t n_less) {
   pdl_begin();
+  const int64_t rows = n_rows ? n_rows[0] - n_less : row_bound;
   __shared__ float part[8][256];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int c = blockIdx.x * 256 + lane * 8;
@@ -170,9 +173,10 @@ __global__ void __launch_bounds__(256) colsum_kernel(const __half* __restrict__ 
   }
 }
 // any shape: one thread per column
-__global__ void __launch_bounds__(256) colsum_slow_kernel(const __half* __restrict__ in, int64_t ld, int64_t rows, int n,
-                                                          int64_t chunk, float* __restrict__ out) {
+__global__ void __launch_bounds__(256) colsum_slow_kernel(const __half* __restrict__ in, int64_t ld, int64_t row_bound, int n,
+                                                          int64_t chunk, float* __restrict__ out, const int* n_rows, int64_t n_less) {
   pdl_begin();
+  const int64_t rows = n_rows ? n_rows[0] - n_less : row_bound;
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= n) return;
   const int64_t r0 = (int64_t)blockIdx.y * chunk, r1 = r0 + chunk < rows ? r0 + chunk : rows;
@@ -254,14 +258,19 @@ __global__ void __launch_bounds__(256) gather_rows16_kernel(const __half* __rest
 }
 
 // token rows (env-major) -> the encoders' row order: 2 saber rows per env, then torso, 2 leg, 24 slot rows per env
+// (packed token rows: the slots that have rows, at dst)
 __global__ void __launch_bounds__(256) gather_tokens16_kernel(const __half* __restrict__ in, int64_t n_envs, int n,
-                                                              __half* __restrict__ out) {
+                                                              __half* __restrict__ out, const int* __restrict__ dst, const int* n_rows) {
   pdl_begin();
   const int nv = n >> 3;
-  const int64_t total = n_envs * kT * nv;
+  const int64_t total = (n_rows ? n_rows[0] : n_envs * kT) * nv;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
     int piece, tok;
     const int64_t r = div_index(i, nv, &piece);
+    if (dst) {
+      reinterpret_cast<uint4*>(out)[i] = *reinterpret_cast<const uint4*>(in + dst[r] * (int64_t)n + piece * 8);
+      continue;
+    }
     int64_t env;
     if (r < 2 * n_envs) { env = r >> 1; tok = (int)(r & 1); }
     else if (r < 3 * n_envs) { env = r - 2 * n_envs; tok = 2; }
@@ -428,7 +437,7 @@ int64_t grid_for(int64_t work_items, int per_block) {
 
 int layernorm_bwd(const float* x, int64_t ldx, RowMap xmap, const float* gamma, float eps, const void* gy, int gy_f32,
                   int64_t ldgy, const float* gres, float* gx_out, int64_t ldg, RowMap gmap, float* ggamma, float* gbeta,
-                  int64_t rows, int d, cudaStream_t stream, __half* gx16, int64_t ldg16) {
+                  int64_t rows, int d, cudaStream_t stream, __half* gx16, int64_t ldg16, const int* n_rows, int64_t n_less) {
   if (!x || !gamma || !gy || !gx_out) {
     set_error("layernorm_bwd: NULL operand");
     return BSRL_ERR_NULL;
@@ -442,7 +451,7 @@ int layernorm_bwd(const float* x, int64_t ldx, RowMap xmap, const float* gamma, 
   const size_t smem = 2 * d * sizeof(float);
   auto wave = [&](int resident) { return blocks < resident * sm_count() ? blocks : resident * sm_count(); };
 #define BSRL_LN_BWD(F32, NV) \
-  launch_kernel(ln_bwd_kernel<F32, NV>, wave(ln_bwd_resident<NV>()), 256, smem, stream, x, ldx, xmap, gamma, eps, gy, ldgy, gres, gx_out, ldg, gmap, gx16, ldg16, ggamma, gbeta, rows, d)
+  launch_kernel(ln_bwd_kernel<F32, NV>, wave(ln_bwd_resident<NV>()), 256, smem, stream, x, ldx, xmap, gamma, eps, gy, ldgy, gres, gx_out, ldg, gmap, gx16, ldg16, ggamma, gbeta, rows, d, n_rows, n_less)
   const int nv = (d + 127) / 128;          // float4 per lane actually needed: fewer registers, more rows in flight
   if (gy_f32) {
     if (nv <= 2) BSRL_LN_BWD(true, 2); else if (nv <= 4) BSRL_LN_BWD(true, 4); else BSRL_LN_BWD(true, 8);
@@ -454,7 +463,7 @@ int layernorm_bwd(const float* x, int64_t ldx, RowMap xmap, const float* gamma, 
   return BSRL_OK;
 }
 
-int colsum16(const __half* in, int64_t ld, int64_t rows, int n, float* out, cudaStream_t stream) {
+int colsum16(const __half* in, int64_t ld, int64_t rows, int n, float* out, cudaStream_t stream, const int* n_rows, int64_t n_less) {
   if (rows == 0 || n == 0 || !out) return BSRL_OK;
   const int col_blocks = (n + 255) / 256;
   // enough row chunks to fill the machine a few times over, at least 64 rows each
@@ -464,8 +473,8 @@ int colsum16(const __half* in, int64_t ld, int64_t rows, int n, float* out, cuda
   const int64_t chunk = (rows + chunks - 1) / chunks;
   chunks = (rows + chunk - 1) / chunk;
   const dim3 grid((unsigned)col_blocks, (unsigned)chunks);
-  if (n % 8 == 0 && ld % 8 == 0 && aligned16(in)) launch_kernel(colsum_kernel, grid, 256, 0, stream, in, ld, rows, n, chunk, out);
-  else launch_kernel(colsum_slow_kernel, grid, 256, 0, stream, in, ld, rows, n, chunk, out);
+  if (n % 8 == 0 && ld % 8 == 0 && aligned16(in)) launch_kernel(colsum_kernel, grid, 256, 0, stream, in, ld, rows, n, chunk, out, n_rows, n_less);
+  else launch_kernel(colsum_slow_kernel, grid, 256, 0, stream, in, ld, rows, n, chunk, out, n_rows, n_less);
   BSRL_LAUNCH_OK("colsum_kernel");
   return BSRL_OK;
 }
@@ -500,9 +509,9 @@ int gather_rows16(const __half* in, int64_t ldi, RowMap imap, __half* out, int64
   return BSRL_OK;
 }
 
-int gather_tokens16(const __half* in, int64_t n_envs, int n, __half* out, cudaStream_t stream) {
+int gather_tokens16(const __half* in, int64_t n_envs, int n, __half* out, cudaStream_t stream, const int* dst, const int* n_rows) {
   if (n_envs == 0) return BSRL_OK;
-  launch_kernel(gather_tokens16_kernel, (unsigned)grid_for(n_envs * kT * (n >> 3), 256), 256, 0, stream, in, n_envs, n, out);
+  launch_kernel(gather_tokens16_kernel, (unsigned)grid_for(n_envs * kT * (n >> 3), 256), 256, 0, stream, in, n_envs, n, out, dst, n_rows);
   BSRL_LAUNCH_OK("gather_tokens16_kernel");
   return BSRL_OK;
 }

@@ -22,8 +22,9 @@ int64_t blocks_for_rows(int64_t rows, int rows_per_block) {
 __global__ void __launch_bounds__(256) vres_bwd_kernel(__half* __restrict__ g, int64_t ldg, const __half* __restrict__ v_own,
                                                        const __half* __restrict__ v0, const float* __restrict__ ab,
                                                        float* __restrict__ g_v0, float* __restrict__ g_a, float* __restrict__ g_b,
-                                                       int64_t rows, int d) {
+                                                       int64_t row_bound, int d, const int* n_rows) {
   pdl_begin();
+  const int64_t rows = n_rows ? n_rows[0] : row_bound;
   const float a = ab[0], b = ab[1];
   const int per_row = d >> 3;
   float sa = 0.f, sb = 0.f;
@@ -75,8 +76,9 @@ __global__ void __launch_bounds__(256) vres_bwd_kernel(__half* __restrict__ g, i
 
 // g16[r, c] += fp16(acc32[r, c]) (fp32 arithmetic, rounded once)
 __global__ void __launch_bounds__(256) add_f32_into_f16_kernel(__half* __restrict__ g, int64_t ldg, const float* __restrict__ acc,
-                                                               int64_t rows, int d) {
+                                                               int64_t row_bound, int d, const int* n_rows) {
   pdl_begin();
+  const int64_t rows = n_rows ? n_rows[0] : row_bound;
   const int per_row = d >> 2;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * per_row; i += (int64_t)gridDim.x * blockDim.x) {
     int piece;
@@ -278,25 +280,25 @@ __global__ void __launch_bounds__(256) scale_relu_bwd_kernel(__half* __restrict_
 }  // namespace
 
 int vres_bwd(__half* g, int64_t ldg, const __half* v_own, const __half* v0, const float* ab, float* g_v0, float* g_a, float* g_b,
-             int64_t rows, int d, cudaStream_t stream) {
+             int64_t rows, int d, cudaStream_t stream, const int* n_rows) {
   if (!g || !v_own || !v0 || !ab || !g_v0 || (d % 8) || (ldg % 8) || !aligned16(g) || !aligned16(v_own) || !aligned16(v0) ||
       !aligned16(g_v0)) {
     set_error("vres_bwd: bad operand");
     return BSRL_ERR_SHAPE;
   }
   if (rows == 0) return BSRL_OK;
-  launch_kernel(vres_bwd_kernel, (unsigned)blocks_for_rows(rows * (d >> 3), 256), 256, 0, stream, g, ldg, v_own, v0, ab, g_v0, g_a, g_b, rows, d);
+  launch_kernel(vres_bwd_kernel, (unsigned)blocks_for_rows(rows * (d >> 3), 256), 256, 0, stream, g, ldg, v_own, v0, ab, g_v0, g_a, g_b, rows, d, n_rows);
   BSRL_LAUNCH_OK("vres_bwd_kernel");
   return BSRL_OK;
 }
 
-int add_f32_into_f16(__half* g, int64_t ldg, const float* acc, int64_t rows, int d, cudaStream_t stream) {
+int add_f32_into_f16(__half* g, int64_t ldg, const float* acc, int64_t rows, int d, cudaStream_t stream, const int* n_rows) {
   if (!g || !acc || (d % 4) || (ldg % 4) || !aligned16(acc) || (reinterpret_cast<uintptr_t>(g) & 7)) {
     set_error("add_f32_into_f16: bad operand");
     return BSRL_ERR_SHAPE;
   }
   if (rows == 0) return BSRL_OK;
-  launch_kernel(add_f32_into_f16_kernel, (unsigned)blocks_for_rows(rows * (d >> 2), 256), 256, 0, stream, g, ldg, acc, rows, d);
+  launch_kernel(add_f32_into_f16_kernel, (unsigned)blocks_for_rows(rows * (d >> 2), 256), 256, 0, stream, g, ldg, acc, rows, d, n_rows);
   BSRL_LAUNCH_OK("add_f32_into_f16_kernel");
   return BSRL_OK;
 }

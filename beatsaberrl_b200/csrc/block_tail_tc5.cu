@@ -85,6 +85,7 @@ struct Shared {
   uint64_t io_full[EPI_WARPS][3];                     // per epilogue warp: residual blocks landed in its buffers
   uint32_t tmem_base;
   int abort;
+  int n_tiles;
 };
 
 struct TailParams {
@@ -92,7 +93,7 @@ struct TailParams {
   int64_t M;                // rows
   const float* x;           // residual in (fp32), rows mapped by xmap
   int64_t ldx;
-  RowMap xmap;
+  PlainMap xmap;
   const float* bo;          // (d)
   const float* ln_g;        // ln_ffn gamma / beta (d)
   const float* ln_b;
@@ -109,6 +110,9 @@ struct TailParams {
   int wide16;               // 128-byte rows per fp16 output block too (d a multiple of 128; else 64)
   int x_tma;                // residual rows are read with TMA (identity row map)
   int* status;
+  const int* n_rows;        // packed token rows: the device's row count (at most M) ...
+  const int* x_start;       // ... and the first rows of xmap's groups, or nullptr
+  __device__ __forceinline__ int64_t x_row(int64_t r) const { return x_start ? (int64_t)x_start[r / xmap.group] + xmap.first + r % xmap.group : xmap.plain(r); }
 };
 
 __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
@@ -173,7 +177,9 @@ using StageNo = std::integral_constant<int, N>;
 
 // GELU: the FFN activation is the exact GELU instead of ReLU (a compile-time variant: the hidden-chunk
 // epilogue sits on the chunk loop's critical path)
-template <bool GELU, bool PAIR>
+// PACK: the number of tiles follows from the device's row count; rows past it are read (they are in the buffers) and their results
+// land past the counted rows
+template <bool GELU, bool PAIR, bool PACK>
 __global__ void __launch_bounds__(THREADS, 1)
 block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_constant__ CUtensorMap tm_wo,
                   const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_w2,
@@ -189,7 +195,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
   // kernel measured 11 % slower with them held in signed locals)
 #define tile0 ((int)blockIdx.x)
 #define tstep (gridDim.x)
-#define t_end (p.n_tiles)
+#define t_end (PACK ? sh->n_tiles : p.n_tiles)
   constexpr int CTAS = PAIR ? 2 : 1, STAGE_BYTES = stage_bytes<PAIR>(), RING_BYTES = STAGES * STAGE_BYTES;
   constexpr int STG_BYTES = stg_bytes<PAIR>(), IO_BYTES = io_bytes<PAIR>(), CB = IO_BYTES / 128;   // CB: fp32 columns per block
   const uint32_t rank = PAIR ? cluster_rank() : 0u;
@@ -223,6 +229,9 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
     for (int w = 0; w < EPI_WARPS; ++w)
       for (int b = 0; b < 3; ++b) mbar_init(smem_u32(&sh->io_full[w][b]), 1);
     sh->abort = 0;
+    // packed token rows: counted at least two launches back; both CTAs of a pair take the same number of tiles.  (Kept in a
+    // register, the count costs 3 % of the kernel.)
+    if (PACK) sh->n_tiles = (p.n_rows[0] + CTAS * BM - 1) / (CTAS * BM) * CTAS;
     fence_barrier_init();
     tma_prefetch_desc(&tm_att);
     tma_prefetch_desc(&tm_wo);
@@ -334,7 +343,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         for (int r = lane; r < BM; r += 32) {
           const int64_t row = (int64_t)tn * BM + r;
           if (row < p.M) {
-            const float* xr = p.x + p.xmap.plain(row) * p.ldx;
+            const float* xr = p.x + p.x_row(row) * p.ldx;
             for (int c = 0; c < d; c += 32) prefetch_l2(xr + c);
           }
         }
@@ -670,7 +679,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int64_t row = (int64_t)t * BM + q * 32 + i * 8 + sub8;
-        src[i] = row < p.M ? p.x + p.xmap.plain(row) * p.ldx + piece * 4 : nullptr;
+        src[i] = row < p.M ? p.x + p.x_row(row) * p.ldx + piece * 4 : nullptr;
       }
       uint4 nxt[4];
 #pragma unroll
@@ -1003,7 +1012,7 @@ int block_tail(const BlockTailArgs& a, cudaStream_t stream) {
   if (!make_tmap_f16(&tm_w2, a.w2, a.d, a.F, a.F, a.d / ctas)) return BSRL_ERR_CUDA;
   // residual rows in and the outputs move as 32-row TMA boxes of 64 or 128 bytes a row; a map that is not needed
   // aliases the attention tile's (the kernel only prefetches its descriptor)
-  const bool x_tma = a.xmap.group == 0x7fffffff && a.xmap.stride == 0 && a.xmap.first == 0;
+  const bool x_tma = a.xmap.dense();
   CUtensorMap tm_x = tm_att, tm_xo = tm_att, tm_o[2] = {tm_att, tm_att};
   const bool wide16 = pair && a.d % 128 == 0;
   auto rows_map = [&](CUtensorMap* map, const void* base, int elem, int64_t ld, bool wide) {
@@ -1016,16 +1025,17 @@ int block_tail(const BlockTailArgs& a, cudaStream_t stream) {
   static DeviceOnce once;
   int rc = once.run("block_tail_kernel set-up", [] {
     const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaError_t e = cudaFuncSetAttribute(block_tail_kernel<false, false>, at, smem_bytes<false>());
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(block_tail_kernel<true, false>, at, smem_bytes<false>());
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(block_tail_kernel<false, true>, at, smem_bytes<true>());
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(block_tail_kernel<true, true>, at, smem_bytes<true>());
+    cudaError_t e = cudaSuccess;
+    for (auto* k : {block_tail_kernel<false, false, false>, block_tail_kernel<true, false, false>, block_tail_kernel<false, false, true>, block_tail_kernel<true, false, true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, at, smem_bytes<false>());
+    for (auto* k : {block_tail_kernel<false, true, false>, block_tail_kernel<true, true, false>, block_tail_kernel<false, true, true>, block_tail_kernel<true, true, true>})
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(k, at, smem_bytes<true>());
     return e;
   });
   if (rc != BSRL_OK) return rc;
   TailParams p;
-  p.d = a.d; p.F = a.F; p.M = a.M;
-  p.x = a.x; p.ldx = a.ldx; p.xmap = a.xmap;
+  p.d = a.d; p.F = a.F; p.M = a.M; p.n_rows = a.n_rows;
+  p.x = a.x; p.ldx = a.ldx; p.xmap = a.xmap; p.x_start = a.xmap.start;
   p.bo = a.bo; p.ln_g = a.ln_g; p.ln_b = a.ln_b; p.b0 = a.b0; p.b2 = a.b2; p.eps = a.eps;
   p.x_out = a.x_out;
   for (int o = 0; o < 2; ++o) {
@@ -1035,12 +1045,17 @@ int block_tail(const BlockTailArgs& a, cudaStream_t stream) {
   p.wide16 = wide16 ? 1 : 0;
   p.x_tma = x_tma ? 1 : 0;
   p.status = status;
-  if (pair)
-    launch_kernel<2>(a.gelu ? block_tail_kernel<true, true> : block_tail_kernel<false, true>, sm_count() & ~1, THREADS, smem_bytes<true>(), stream,
-                     tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
-  else
-    launch_kernel(a.gelu ? block_tail_kernel<true, false> : block_tail_kernel<false, false>, p.n_tiles < sm_count() ? p.n_tiles : sm_count(), THREADS,
-                  smem_bytes<false>(), stream, tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
+  const bool pack = a.n_rows != nullptr;
+  if (pair) {
+    auto* kernel = pack ? (a.gelu ? block_tail_kernel<true, true, true> : block_tail_kernel<false, true, true>)
+                        : (a.gelu ? block_tail_kernel<true, true, false> : block_tail_kernel<false, true, false>);
+    launch_kernel<2>(kernel, sm_count() & ~1, THREADS, smem_bytes<true>(), stream, tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo, tm_o[0], tm_o[1], p);
+  } else {
+    auto* kernel = pack ? (a.gelu ? block_tail_kernel<true, false, true> : block_tail_kernel<false, false, true>)
+                        : (a.gelu ? block_tail_kernel<true, false, false> : block_tail_kernel<false, false, false>);
+    launch_kernel(kernel, p.n_tiles < sm_count() ? p.n_tiles : sm_count(), THREADS, smem_bytes<false>(), stream, tm_att, tm_wo, tm_w0, tm_w2, tm_x, tm_xo,
+                  tm_o[0], tm_o[1], p);
+  }
   BSRL_LAUNCH_OK("block_tail_kernel");
   return BSRL_OK;
 }

@@ -35,7 +35,7 @@ __host__ __device__ __forceinline__ int64_t div_index(int64_t i, int d, int* rem
 
 // Row remapping of a (rows, ld) matrix: logical row r lives at physical row
 // (r / group) * stride + first + (r % group).  Identity: group = INT_MAX, stride = 0, first = 0.
-struct RowMap {
+struct PlainMap {
   int group;
   int stride;
   int first;
@@ -49,6 +49,21 @@ struct RowMap {
   __host__ __device__ inline int64_t plain(int64_t r) const {
     return (r / group) * (int64_t)stride + first + (r % group);
   }
+  bool dense() const { return group == 0x7fffffff && stride == 0 && first == 0; }
+};
+// Packed token rows (rows.cu): the groups start at start[r / group] instead of at multiples of stride.  Kernels that never
+// see these take the plain part: their parameters' place is latency of small launches.
+struct RowMap : PlainMap {
+  const int* start = nullptr;
+  RowMap() = default;
+  __host__ __device__ RowMap(int g, int s, int f, const int* t = nullptr) : PlainMap{g, s, f}, start(t) {}
+  __device__ inline int64_t operator()(int64_t r) const {
+    if (!start) return PlainMap::operator()(r);
+    int rem;
+    const int64_t q = div_index(r, group, &rem);
+    return (int64_t)start[q] + first + rem;
+  }
+  bool dense() const { return PlainMap::dense() && !start; }
 };
 inline RowMap identity_map() { return RowMap{0x7fffffff, 0, 0}; }
 

@@ -91,7 +91,8 @@ __device__ void slot_geometry(const float* o, int slot, float z_asinh, bool flux
   }
 }
 
-template <bool OBS_F16>
+// PACK: packed token rows (EmbedBuffers::rows)
+template <bool OBS_F16, bool PACK>
 __global__ void __launch_bounds__(kWarps * 32, 4) embed_gather_kernel(const void* __restrict__ obs_,
                                                                   int64_t n_envs, int note_geo,
                                                                   float z_asinh, EmbedBuffers out) {
@@ -121,7 +122,10 @@ __global__ void __launch_bounds__(kWarps * 32, 4) embed_gather_kernel(const void
       uint32_t* d16 = reinterpret_cast<uint32_t*>(out.obs16 + env * kObs);
       for (int i = lane; i < kObs / 2; i += 32) d16[i] = pack_half2(o[2 * i], o[2 * i + 1]);
     }
-    if (note_geo && lane < kSlots) slot_geometry(o, lane, z_asinh, (note_geo & 2) != 0, geo + lane * kGeoFeat);
+    const int row0 = PACK ? out.rows.start[env] : 0;
+    const int n_slots = PACK ? out.rows.start[env + 1] - row0 - kLead : kSlots;
+    const int64_t slot0 = PACK ? row0 - kLead * env : env * kSlots;      // the first slot's row among the slot rows
+    if (note_geo && lane < n_slots) slot_geometry(o, lane, z_asinh, (note_geo & 2) != 0, geo + lane * kGeoFeat);
     // lead tokens: lane writes features 2*lane, 2*lane + 1
     {
       const int k = lane * 2;
@@ -143,17 +147,25 @@ __global__ void __launch_bounds__(kWarps * 32, 4) embed_gather_kernel(const void
       // every slot row is 64 features = one lane per pair: obs lanes, then the geometry lanes, then zeros
       // (the feature counts are even, so a pair never straddles two sources)
       static_assert(kNoteFeat % 2 == 0 && kGeoFeat % 2 == 0, "feature pairs");
-      uint32_t* d = reinterpret_cast<uint32_t*>(out.note + env * kSlots * 64);
+      uint32_t* d = reinterpret_cast<uint32_t*>(out.note + slot0 * 64);
       const int k = lane * 2;
       const float* src = k < kNoteFeat ? o + kOffNotes + k
                          : (note_geo && k < kNoteFeat + kGeoFeat) ? geo + (k - kNoteFeat) : nullptr;
       const int step = k < kNoteFeat ? kNoteFeat : kGeoFeat;
 #pragma unroll 8
-      for (int slot = 0; slot < kSlots; ++slot)
+      for (int slot = 0; slot < n_slots; ++slot)
         d[slot * 32 + lane] = src ? pack_half2(src[slot * step], src[slot * step + 1]) : 0u;
     }
-    if (lane < kT)
-      out.key_bias[env * kT + lane] = lane < kLead ? 0.f : (o[kOffMask + lane - kLead] - 1.0f) * kMaskBias;
+    if (lane < kT) {
+      const float bias = lane < kLead ? 0.f : (o[kOffMask + lane - kLead] - 1.0f) * kMaskBias;
+      out.key_bias[env * kT + lane] = bias;
+      if (PACK && lane < kLead + n_slots) {
+        const int64_t in = lane < 2 ? 2 * env + lane : lane < 3 ? 2 * n_envs + env : lane < kLead ? 3 * n_envs + 2 * env + lane - 3
+                                                                                                  : kLead * n_envs + slot0 + lane - kLead;
+        out.rows.dst[in] = row0 + lane;
+        out.rows.kb[row0 + lane] = bias;
+      }
+    }
   }
 }
 }  // namespace
@@ -182,10 +194,10 @@ int embed_gather(const void* obs, int obs_dtype, int64_t n_envs, int note_geo, i
   int64_t blocks = (n_envs + kWarps - 1) / kWarps;
   int64_t cap = (int64_t)sm_count() * 8;
   if (blocks > cap) blocks = cap;
-  if (obs_dtype == BSRL_F16)
-    launch_kernel(embed_gather_kernel<true>, static_cast<unsigned>(blocks), kWarps * 32, 0, stream, obs, n_envs, note_geo, z_asinh, out);
-  else
-    launch_kernel(embed_gather_kernel<false>, static_cast<unsigned>(blocks), kWarps * 32, 0, stream, obs, n_envs, note_geo, z_asinh, out);
+  const bool pack = out.rows.start != nullptr;
+  auto* kernel = obs_dtype == BSRL_F16 ? (pack ? embed_gather_kernel<true, true> : embed_gather_kernel<true, false>)
+                                       : (pack ? embed_gather_kernel<false, true> : embed_gather_kernel<false, false>);
+  launch_kernel(kernel, static_cast<unsigned>(blocks), kWarps * 32, 0, stream, obs, n_envs, note_geo, z_asinh, out);
   BSRL_LAUNCH_OK("embed_gather_kernel");
   return BSRL_OK;
 }

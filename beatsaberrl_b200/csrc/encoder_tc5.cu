@@ -77,6 +77,9 @@ struct EncParams {
   float* x;               // (n_envs * 29, d) f32
   __half* h;              // (n_envs * 29, d) f16 or nullptr
   int* status;
+  const int* dst;         // packed token rows: x row of every feature row, and the number of rows
+  const int* n_rows;
+  int64_t lead_rows;      // feature rows ahead of the slots'
 };
 
 __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
@@ -92,6 +95,8 @@ __device__ __forceinline__ int part_of_tile(const EncParams& p, int t) {
   return e;
 }
 
+// PACK: packed token rows (EncParams::dst)
+template <bool PACK>
 __global__ void __launch_bounds__(THREADS, 1)
 encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -106,6 +111,8 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int d = p.d, KB = d >> 6, dh2 = d >> 1;
   volatile int* abort = &sh->abort;
+  // packed token rows: written at least two launches back
+  const int n_tiles = PACK ? (int)(p.part[3].tile0 + (p.n_rows[0] - p.lead_rows + BM - 1) / BM) : p.n_tiles;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -165,7 +172,7 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
         ++it;
         return true;
       };
-      for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, ++tile_i) {
+      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++tile_i) {
         const int e = part_of_tile(p, t);
         const int64_t row0 = p.part[e].row0 + (int64_t)(t - (int)p.part[e].tile0) * BM;
         int early = 0;                          // first tile: weights ahead of the predecessor's last rows
@@ -212,7 +219,7 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
         ++it;
         return true;
       };
-      for (int t = blockIdx.x; t < p.n_tiles && ok; t += gridDim.x, ++tile_i) {
+      for (int t = blockIdx.x; t < n_tiles && ok; t += gridDim.x, ++tile_i) {
         const uint32_t par = tile_i & 1, b = tile_i & 1, use = (tile_i >> 1) & 1;
         const uint32_t acc = tmem_base + 256u * b;
         if (!mbar_wait(smem_u32(&sh->a_full), par, abort)) { give_up(sh, p.status, 6); break; }
@@ -240,7 +247,7 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
     const uint32_t lane_q = tmem_base + ((uint32_t)(q * 32) << 16);
     const int st_row = lane & 7, st_piece = lane >> 3;
     uint32_t tile_i = 0;
-    for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, ++tile_i) {
+    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++tile_i) {
       const uint32_t b = tile_i & 1, use = (tile_i >> 1) & 1;
       const uint64_t* prm_b0 = reinterpret_cast<const uint64_t*>(prm + part_of_tile(p, t) * 256 + 2 * (lane & 3));
       // the first GEMM of this tile was issued after the second GEMM of the tile before: its completion also
@@ -288,7 +295,7 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
     const uint64_t* prm_frag = reinterpret_cast<const uint64_t*>(prm + 2 * (lane & 3));    // pair of 8-column unit u of vector v: [128 v + 4 u]
     const float inv_d = 1.0f / (float)d;
     uint32_t tile_i = 0;
-    for (int t = blockIdx.x; t < p.n_tiles; t += gridDim.x, ++tile_i) {
+    for (int t = blockIdx.x; t < n_tiles; t += gridDim.x, ++tile_i) {
       const uint32_t b = tile_i & 1, use = (tile_i >> 1) & 1;
       const uint32_t lane_base = lane_q + 256u * b;
       const int e = part_of_tile(p, t);
@@ -299,7 +306,14 @@ encoder_kernel(const __grid_constant__ Maps m, EncParams p) {
       // boundary: eight 64-bit divisions here cost the epilogue ~2 K cycles per tile)
       int64_t orow[8];
       const int64_t r_tile = (int64_t)(t - (int)pe.tile0) * BM;
-      {
+      if (PACK) {
+        const int64_t rows = e == 3 ? p.n_rows[0] - p.lead_rows : pe.rows;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int64_t r = r_tile + q * 32 + sub + 4 * i;
+          orow[i] = r < rows ? p.dst[pe.row0 + r] * (int64_t)d : -1;
+        }
+      } else {
         int slot;
         const int64_t env = div_index(r_tile + q * 32 + sub, pe.group, &slot);      // rows < 2^31 (checked on the host)
         int64_t off = (env * kT + pe.first + slot) * (int64_t)d;
@@ -448,13 +462,14 @@ int encoder_fused(const EncoderArgs& a, cudaStream_t stream) {
   }
   static DeviceOnce once;
   int rc = once.run("encoder_kernel set-up", [] {
-    return cudaFuncSetAttribute(encoder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    cudaError_t e = cudaFuncSetAttribute(encoder_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(encoder_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
   });
   if (rc != BSRL_OK) return rc;
   EncParams p;
   p.d = a.d;
   // encoders in the order of the feature matrix and of EncoderArgs: saber (2 rows per env, slots 0-1),
-  // torso (1, slot 2), leg (2, slots 3-4), note (24, slots 5-28); tiles: the note tiles first
+  // torso (1, slot 2), leg (2, slots 3-4), note (24, slots 5-28)
   const int64_t rows[4] = {2 * B, B, 2 * B, (int64_t)kSlots * B};
   const int group[4] = {2, 1, 2, kSlots}, first[4] = {0, 2, 3, kLead};
   int64_t row0 = 0;
@@ -467,22 +482,11 @@ int encoder_fused(const EncoderArgs& a, cudaStream_t stream) {
     p.b0[e] = a.b0[e];
     p.b1[e] = a.b1[e];
   }
-  // tile numbering must be monotone in the part index for part_of_tile: parts are numbered 0..3 in tile order
-  // note, saber, torso, leg -> remap so that part[0] is the note encoder
-  EncPart ordered[4] = {p.part[3], p.part[0], p.part[1], p.part[2]};
-  const float* b0o[4] = {a.b0[3], a.b0[0], a.b0[1], a.b0[2]};
-  const float* b1o[4] = {a.b1[3], a.b1[0], a.b1[1], a.b1[2]};
-  Maps mo = m;
-  const int src[4] = {3, 0, 1, 2};
+  // the slots' tiles come last: their number may be the device's to say
   int64_t tile0 = 0;
-  for (int i = 0; i < 4; ++i) {
-    p.part[i] = ordered[i];
-    p.part[i].tile0 = tile0;
-    tile0 += (ordered[i].rows + BM - 1) / BM;
-    p.b0[i] = b0o[i];
-    p.b1[i] = b1o[i];
-    mo.w0[i] = m.w0[src[i]];
-    mo.w1[i] = m.w1[src[i]];
+  for (int e = 0; e < 4; ++e) {
+    p.part[e].tile0 = tile0;
+    tile0 += (rows[e] + BM - 1) / BM;
   }
   if (tile0 > 0x7fffffff) {
     set_error("encoder: too many tiles");
@@ -494,9 +498,12 @@ int encoder_fused(const EncoderArgs& a, cudaStream_t stream) {
   p.eps = a.eps;
   p.x = a.x;
   p.h = a.h;
+  p.dst = a.dst;
+  p.n_rows = a.n_rows;
+  p.lead_rows = row0 - rows[3];
   p.status = status;
   const int grid = p.n_tiles < sm_count() ? p.n_tiles : sm_count();
-  launch_kernel(encoder_kernel, grid, THREADS, SMEM_BYTES, stream, mo, p);
+  launch_kernel(a.dst ? encoder_kernel<true> : encoder_kernel<false>, grid, THREADS, SMEM_BYTES, stream, m, p);
   BSRL_LAUNCH_OK("encoder_kernel");
   return BSRL_OK;
 }

@@ -71,6 +71,7 @@ struct Params {
   int64_t ldh;
   int n_tiles;
   int* status;
+  const int* n_rows;  // the device's row count (at most M) or nullptr
 };
 
 __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
@@ -101,6 +102,8 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = CL == 2 ? cluster_rank() : 0u;
   const int nc = p.nc, col_cta = (int)rank * nc, k_blocks = p.K / BK;
+  const int64_t M = p.n_rows ? p.n_rows[0] : p.M;
+  const int n_tiles = p.n_rows ? (int)((M + BM - 1) / BM) : p.n_tiles;
   const int t0 = (int)(blockIdx.x / CL), t_step = (int)(gridDim.x / CL);
   volatile int* abort = &sh->abort;
 
@@ -148,7 +151,7 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       const uint32_t stage_tx = (uint32_t)(A_BYTES + nc * BK * 2);
       uint32_t it = 0;
       bool ok = true;
-      for (int t = t0; t < p.n_tiles && ok; t += t_step) {
+      for (int t = t0; t < n_tiles && ok; t += t_step) {
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           if (!mbar_wait(smem_u32(&sh->empty[s]), ((it / STAGES) & 1) ^ 1, abort)) { give_up(sh, p.status, 1); ok = false; break; }
@@ -171,7 +174,7 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       uint32_t it = 0, tile_i = 0;
       bool ok = true;
       const uint32_t idesc = idesc_f16(BM, nc);
-      for (int t = t0; t < p.n_tiles && ok; t += t_step, ++tile_i) {
+      for (int t = t0; t < n_tiles && ok; t += t_step, ++tile_i) {
         const int buf = tile_i & 1;
         if (!mbar_wait(smem_u32(&sh->acc_empty[buf]), ((tile_i >> 1) & 1) ^ 1, abort)) { give_up(sh, p.status, 3); ok = false; break; }
         tc_fence_after();
@@ -206,7 +209,7 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     int use_b = 0, ask_b = 0, ask_pos = 0, ask_t = t0;
     uint32_t parity = 0, pending = 0;                        // bit b: buffer b's next phase; a load is on its way to it
     auto ask = [&]() {
-      if (ask_t < p.n_tiles && ask_pos < nx) {
+      if (ask_t < n_tiles && ask_pos < nx) {
         pending |= 1u << ask_b;
         if (lane == 0) {
           const uint32_t bar = smem_u32(row_full + ask_b);
@@ -229,18 +232,18 @@ linear_ln_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
-        if (m0 < p.M) tma_store_2d(map, x, (int)m0, smem_u32(buf));
+        if (m0 < M) tma_store_2d(map, x, (int)m0, smem_u32(buf));
         bulk_commit();
       }
     };
     for (int i = 0; i < BUFS - 1; ++i) ask();
     uint32_t tile_i = 0;
     bool ok = true;
-    for (int t = t0; t < p.n_tiles && ok; t += t_step, ++tile_i) {
+    for (int t = t0; t < n_tiles && ok; t += t_step, ++tile_i) {
       const int buf = tile_i & 1;
       const int64_t m0 = (int64_t)t * BM + q * 32, row = m0 + lane;
-      const bool live = row < p.M;
-      if (lane == 0 && t + t_step < p.n_tiles)               // the next tile's residual rows into L2
+      const bool live = row < M;
+      if (lane == 0 && t + t_step < n_tiles)               // the next tile's residual rows into L2
         for (int c = 0; c < hc; c += 32) tma_prefetch_2d(&tm_r, col_cta + lo + c, (t + t_step) * BM + q * 32);
       if (!mbar_wait_warp(smem_u32(&sh->acc_full[buf]), (tile_i >> 1) & 1, abort)) {
         if (lane == 0) give_up(sh, p.status, 5);
@@ -429,7 +432,7 @@ int linear_ln(const LinearLnArgs& a, cudaStream_t stream) {
   });
   if (rc != BSRL_OK) return rc;
   Params p;
-  p.nc = nc; p.K = a.K; p.M = a.M; p.inv_n = 1.0f / (float)a.N;
+  p.nc = nc; p.K = a.K; p.M = a.M; p.n_rows = a.n_rows; p.inv_n = 1.0f / (float)a.N;
   p.bias = a.bias; p.gamma = a.gamma; p.beta = a.beta; p.eps = a.eps;
   p.h = a.h; p.ldh = a.ldh;
   p.n_tiles = (int)((a.M + BM - 1) / BM);

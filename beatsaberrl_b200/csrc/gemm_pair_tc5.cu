@@ -73,7 +73,7 @@ __device__ __forceinline__ uint32_t keep_positive(uint32_t h, uint32_t mask) {
 template <bool HAS_R, bool GELU32 = false>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
-                   const __grid_constant__ CUtensorMap tm_c, int box_rows, int r32, LinearArgs p, int m_pairs, int n_tiles, int* status) {
+                   const __grid_constant__ CUtensorMap tm_c, int box_rows, int r32, LinearArgs p, int m_bound, int n_tiles, int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -82,6 +82,8 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const int k_blocks = (p.K + BK - 1) / BK;
+  const int64_t M = p.live(p.M);
+  const int m_pairs = p.n_rows ? (int)((M + 2 * BM - 1) / (2 * BM)) : m_bound;
   const int n_work = m_pairs * n_tiles;                      // work item: (row pair, column tile), column tile fastest
   const int w_first = (int)(blockIdx.x >> 1), w_step = (int)(gridDim.x >> 1);
   volatile int* abort = &sh->abort;
@@ -214,14 +216,14 @@ linear_pair_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_consta
       const int64_t m0 = (int64_t)mt * (2 * BM) + (int64_t)rank * BM + q * 32;     // this warp's first row
       const int buf = tile_i & 1;
       const int64_t row = m0 + lane;
-      const bool live = row < p.M;
+      const bool live = row < M;
       // the filled buffer (128 bytes of each of the warp's 32 rows, from column x on) -> C
       auto emit = [&](int x) {
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0 && m0 < p.M) {
+        if (lane == 0 && m0 < M) {
           if (box_rows == 32) tma_store_2d(&tm_c, x, (int)m0, smem_u32(stg));
-          else store_mapped8(&tm_c, x, m0, p.M, p.cmap, smem_u32(stg));
+          else store_mapped8(&tm_c, x, m0, M, p.cmap, smem_u32(stg));
           bulk_commit();
         }
       };
@@ -382,7 +384,7 @@ int linear_pair(const LinearArgs& p, cudaStream_t stream) {
   if (p.w_mn ? !make_tmap_mn(&tm_w, p.W, p.K, p.N, p.ldw, BK, BN / 128) : !make_tmap_f16(&tm_w, p.W, p.N, p.K, p.ldw, BN / 2))
     return BSRL_ERR_CUDA;
   const int box_rows = store_box_rows(p.cmap, p.M);
-  if (!make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, box_rows == 32 ? p.M : p.cmap(p.M - 1) + 1, p.N, p.ldc, box_rows, 128)) return BSRL_ERR_CUDA;
+  if (!make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, box_rows == 32 ? p.M : p.cmap.plain(p.M - 1) + 1, p.N, p.ldc, box_rows, 128)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("linear_pair_kernel set-up", [] {
     cudaError_t e = cudaSuccess;

@@ -93,12 +93,14 @@ __device__ __forceinline__ uint32_t keep_positive(uint32_t h, uint32_t w, int i)
 template <bool HAS_R, bool GELU32 = false>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
-                  const __grid_constant__ CUtensorMap tm_c, int tma_c, int r32, LinearArgs p, int bn, int m_tiles, int n_tiles,
+                  const __grid_constant__ CUtensorMap tm_c, int tma_c, int r32, LinearArgs p, int bn, int m_bound, int n_tiles,
                   int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
   const int k_blocks = (p.K + BK - 1) / BK;
+  const int64_t M = p.live(p.M);
+  const int m_tiles = p.n_rows ? (int)((M + 2 * BM - 1) / (2 * BM)) : m_bound;
   const int n_st = min(MAX_STAGES, (OPERAND_BYTES - k_blocks * W_BYTES) / A_BYTES);
   const uint32_t w_base = base + n_st * A_BYTES;
   uint8_t* staging = smem_raw + (base - raw) + OPERAND_BYTES;
@@ -253,13 +255,13 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       const int64_t m0 = ((int64_t)t * 2 + rank) * BM + q * 32;    // this warp's first row
       const int buf = tile_i & 1;
       const int64_t row = m0 + lane;
-      const bool live = row < p.M;
+      const bool live = row < M;
       int64_t crow[8];                                       // rows this lane copies out where C's rows are scattered
       if (!tma_c) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int64_t r = m0 + 4 * i + sub;
-          crow[i] = r < p.M ? p.cmap(r) * (int64_t)p.ldc : -1;
+          crow[i] = r < M ? p.cmap(r) * (int64_t)p.ldc : -1;
         }
       }
       // the filled buffer (128 bytes of each of the warp's 32 rows, from column x on) -> C
@@ -267,9 +269,9 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         if (tma_c) {
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0 && m0 < p.M) {
+          if (lane == 0 && m0 < M) {
             if (tma_c == 32) tma_store_2d(&tm_c, x, (int)m0, smem_u32(stg));
-            else store_mapped8(&tm_c, x, m0, p.M, p.cmap, smem_u32(stg));
+            else store_mapped8(&tm_c, x, m0, M, p.cmap, smem_u32(stg));
             bulk_commit();
           }
           return;
@@ -291,7 +293,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         rrow = p.R + p.rmap(row) * (int64_t)p.ldr;
         if (c0 < n_end) res.load(rrow + c0, n_end - c0, r32);
         const int64_t rown = row + (int64_t)t_step * 2 * BM; // the next tile's residual rows into L2
-        if (rown < p.M) {
+        if (rown < M) {
           const float* rn = p.R + p.rmap(rown) * (int64_t)p.ldr + c0;
 #pragma unroll
           for (int c = 0; c < BN / 2; c += 32)
@@ -347,7 +349,7 @@ linear_res_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           if (col >= n_end) break;
           uint2 bits = make_uint2(0, 0);                     // of this thread's pairs in the block
           uint2* at_bits = nullptr;
-          if ((p.bits_in || p.bits_out) && m0 < p.M)
+          if ((p.bits_in || p.bits_out) && m0 < M)
             at_bits = const_cast<uint2*>(reinterpret_cast<const uint2*>(p.bits_in ? p.bits_in : p.bits_out)) +
                       ((int64_t)(col >> 6) * p.bits_ld + (m0 >> 5)) * 32 + lane;
           if (p.bits_in && at_bits) bits = *at_bits;
@@ -437,7 +439,7 @@ int linear_res(const LinearArgs& p, cudaStream_t stream) {
     return BSRL_ERR_CUDA;
   const int tma_c = store_box_rows(p.cmap, p.M);
   CUtensorMap tm_c = tm_a;
-  if (tma_c && !make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, tma_c == 32 ? p.M : p.cmap(p.M - 1) + 1, p.N, p.ldc, tma_c, 128)) return BSRL_ERR_CUDA;
+  if (tma_c && !make_tmap_rows(&tm_c, p.C, p.out_f32 ? 4 : 2, tma_c == 32 ? p.M : p.cmap.plain(p.M - 1) + 1, p.N, p.ldc, tma_c, 128)) return BSRL_ERR_CUDA;
   static DeviceOnce once;
   int rc = once.run("linear_res_kernel set-up", [] {
     cudaError_t e = cudaSuccess;

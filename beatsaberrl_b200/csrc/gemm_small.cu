@@ -25,8 +25,23 @@ __device__ __forceinline__ uint32_t piece_off(int row, int kc) {
   return static_cast<uint32_t>(row * ROW_BYTES + ((kc ^ (row & 7)) << 4));
 }
 
+struct Problem {             // of LinearArgs
+  const __half *A, *W;
+  int lda, ldw;
+  PlainMap amap, rmap, cmap;
+  const float *bias, *R;
+  int ldr, ldc;
+  void* C;
+  int out_f32, relu;
+  int64_t M;
+  int N, K;
+  Problem() = default;
+  Problem(const LinearArgs& a)
+      : A(a.A), W(a.W), lda(a.lda), ldw(a.ldw), amap(a.amap), rmap(a.rmap), cmap(a.cmap), bias(a.bias), R(a.R), ldr(a.ldr), ldc(a.ldc), C(a.C),
+        out_f32(a.out_f32), relu(a.relu), M(a.M), N(a.N), K(a.K) {}
+};
 struct SmallArgs {
-  LinearArgs p[2];           // the second one is optional: blocks from tiles0 on
+  Problem p[2];              // the second one is optional: blocks from tiles0 on
   int tiles0, stages[2];
   int start;                 // linear_small_block
   RowNorm norm;
@@ -44,7 +59,7 @@ __global__ void __launch_bounds__(TM * TN / 4) linear_small_kernel(const __grid_
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp % (TM / 16), wn = warp / (TM / 16);
   const bool second = blockIdx.x >= (unsigned)args.tiles0;
-  const LinearArgs& p = args.p[second ? 1 : 0];
+  const Problem& p = args.p[second ? 1 : 0];
   const int stages = args.stages[second ? 1 : 0], n_tiles = (p.N + TN - 1) / TN;
   const unsigned tile = blockIdx.x - (second ? (unsigned)args.tiles0 : 0u);
   const int nt = (int)(tile % (unsigned)n_tiles);
@@ -186,14 +201,14 @@ constexpr int MAX_STAGES = 8;
 template <int TM, int TN>
 struct Tile {
   static constexpr int THREADS = TM * TN / 4, STAGE_BYTES = (TM + TN) * ROW_BYTES;
-  static int stages(const LinearArgs& p) {
+  static int stages(const Problem& p) {
     const int chunks = (p.K + KC - 1) / KC;
     return chunks < MAX_STAGES ? chunks : MAX_STAGES;
   }
-  static int64_t tiles(const LinearArgs& p) { return (p.M + TM - 1) / TM * ((p.N + TN - 1) / TN); }
-  static bool gelu32(const LinearArgs& p) { return p.relu == 2 && p.out_f32; }
+  static int64_t tiles(const Problem& p) { return (p.M + TM - 1) / TM * ((p.N + TN - 1) / TN); }
+  static bool gelu32(const Problem& p) { return p.relu == 2 && p.out_f32; }
   static int norm_bytes(int d) { return TM * (d + 4) * 4 + 2 * TM * 8; }
-  static bool one_wave(const LinearArgs& p, bool norm = false) {      // every tile has a place on the chip at once
+  static bool one_wave(const Problem& p, bool norm = false) {      // every tile has a place on the chip at once
     const int by_smem = 227 * 1024 / (stages(p) * STAGE_BYTES + (norm ? norm_bytes(p.K) : 0) + 1024), by_threads = 2048 / THREADS;
     return tiles(p) <= (int64_t)sm_count() * (by_smem < by_threads ? by_smem : by_threads);
   }
@@ -226,6 +241,7 @@ int refuse(const LinearArgs& p) {
 
 bool linear_small_ok(const LinearArgs& p) {
   if (!p.A || !p.W || !p.C || p.M < 1 || p.a_mn || p.w_mn || p.mask || p.a_sums || p.bits_in || p.bits_out || p.k_splits > 1) return false;
+  if (p.n_rows || p.amap.start || p.rmap.start || p.cmap.start) return false;      // packed token rows
   if (p.N % 8 || p.K % 8 || p.N < 8 || p.K < 8) return false;
   if (!aligned16(p.A) || !aligned16(p.W) || (p.lda % 8) || (p.ldw % 8) || (reinterpret_cast<uintptr_t>(p.C) & 7) || (p.ldc % 2)) return false;
   if (p.R && ((p.ldr % 2) || (reinterpret_cast<uintptr_t>(p.R) & 7))) return false;

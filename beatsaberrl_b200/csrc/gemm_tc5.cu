@@ -38,7 +38,7 @@ constexpr int ONES_BYTES = 16 * 128;            // B operand of the column sums:
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_WARPS * STG_BYTES + 1024 /*alignment slack*/ + 256 /*barriers*/;
 
 struct Shared {
-  uint64_t full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], mma_done;
+  uint64_t full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2], mma_done, tail_there, tail_clear;
   uint32_t tmem_base;
   int abort;
 };
@@ -68,7 +68,7 @@ __device__ __forceinline__ WorkItem work_item(int64_t w, int n_tile_work, int n_
 template <bool HAS_R, bool SUMS, bool GELU32 = false>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
-                  const __grid_constant__ CUtensorMap tm_c, int tma_c, LinearArgs p, int m_tiles, int n_tiles,
+                  const __grid_constant__ CUtensorMap tm_c, int tma_c, LinearArgs p, int m_bound, int n_tiles,
                   int* status) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -76,9 +76,14 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   uint8_t* staging = smem_raw + (tiles_base - raw) + STAGES * STAGE_BYTES;
   Shared* sh = reinterpret_cast<Shared*>(staging + EPI_WARPS * STG_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int k_blocks = (p.K + BK - 1) / BK;
-  const int splits = p.k_splits > 1 ? p.k_splits : 1;
-  const int kps = (k_blocks + splits - 1) / splits;          // k-blocks per split
+  const int64_t M = p.a_mn ? p.M : p.live(p.M);
+  const int K = p.a_mn ? (int)p.live(p.K) : p.K;
+  const int m_tiles = p.n_rows && !p.a_mn ? (int)((M + BM - 1) / BM) : m_bound;
+  const int k_blocks = (K + BK - 1) / BK;
+  const int kps = max((k_blocks + max(p.k_splits, 1) - 1) / max(p.k_splits, 1), 1);  // k-blocks per split
+  const int splits = p.n_rows && p.a_mn ? (k_blocks + kps - 1) / kps : max(p.k_splits, 1);      // none of them empty (no rows: no work)
+  // Rows past the device's count in the contraction's last k-block are anything: an epilogue warp, idle by then, clears them
+  const int tail = p.n_rows && p.a_mn ? K % BK : 0;
   const int64_t n_tile_work = (int64_t)m_tiles * n_tiles;
   const int64_t n_work = n_tile_work * splits;                // work item = (split, tile): split-major
   volatile int* abort = &sh->abort;
@@ -93,6 +98,8 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       mbar_init(smem_u32(&sh->tmem_empty[b]), EPI_WARPS);
     }
     mbar_init(smem_u32(&sh->mma_done), 1);
+    mbar_init(smem_u32(&sh->tail_there), 1);
+    mbar_init(smem_u32(&sh->tail_clear), 1);
     sh->abort = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tm_a);
@@ -150,7 +157,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
     if (lane == 0) {
-      uint32_t it = 0, tile_i = 0;
+      uint32_t it = 0, tile_i = 0, tails = 0;
       bool ok = true;
       for (int64_t w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++tile_i) {
         const WorkItem wi = work_item(w, (int)n_tile_work, n_tiles);
@@ -174,6 +181,10 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(smem_u32(&sh->full[s]), ph, abort)) { give_up(sh, status, 4); ok = false; break; }
+          if (tail && kb == k_blocks - 1) {
+            mbar_arrive(smem_u32(&sh->tail_there));
+            if (!mbar_wait(smem_u32(&sh->tail_clear), tails++ & 1, abort)) { give_up(sh, status, 4); ok = false; break; }
+          }
           tc_fence_after();
           const uint32_t a_addr = tiles_base + s * STAGE_BYTES;
           const uint64_t a_desc = p.a_mn ? smem_desc_mn_sw128(a_addr, BK * 128) : smem_desc_sw128(a_addr);
@@ -209,10 +220,28 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     const bool wide = p.out_f32 || HAS_R;        // stage fp32 (32 columns per block) instead of fp16 (64)
     const int cw = wide ? 32 : 64;
     const int sub = lane >> 3, piece = lane & 7;   // transposed phase: row sub + 4 i, 16-byte piece
-    uint32_t tile_i = 0;
+    uint32_t tile_i = 0, it = 0, tails = 0;
     bool ok = true;
     for (int64_t w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++tile_i) {
       const WorkItem wi = work_item(w, (int)n_tile_work, n_tiles);
+      if (tail && warp == 2) {
+        const int kb0 = wi.split * kps, kb1 = min(k_blocks, kb0 + kps);
+        it += kb1 - kb0;
+        if (kb1 == k_blocks) {
+          const int s = (it - 1) % STAGES;
+          // (the issuing thread says when the k-block is there: a parity of its own wait names two phases)
+          if (!mbar_wait_warp(smem_u32(&sh->tail_there), tails++ & 1, abort) && lane == 0) give_up(sh, status, 7);
+          // a k row is 128 bytes of each 64-column block, in place whatever the swizzle: two blocks of A, four of W
+          uint8_t* tile = smem_raw + (tiles_base - raw) + s * STAGE_BYTES;
+          for (int i = lane; i < (BK - tail) * 8 * (BM + BN) / 64; i += 32) {
+            const int piece = i & 7, row = (i >> 3) % (BK - tail), blk = (i >> 3) / (BK - tail);
+            *reinterpret_cast<uint4*>(tile + blk * (BK * 128) + (tail + row) * 128 + piece * 16) = make_uint4(0, 0, 0, 0);
+          }
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(smem_u32(&sh->tail_clear));
+        }
+      }
       const bool first_split = w < n_tile_work;              // the piece that carries the bias
       const int64_t m0 = (int64_t)wi.mt * BM;
       const int n0 = wi.nt * BN;
@@ -223,8 +252,8 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int64_t row = m0 + q * 32 + i * 4 + sub;
-        crow[i] = row < p.M ? p.cmap(row) * (int64_t)p.ldc : -1;
-        rrow[i] = (HAS_R && row < p.M) ? p.rmap(row) * (int64_t)p.ldr : 0;
+        crow[i] = row < M ? p.cmap(row) * (int64_t)p.ldc : -1;
+        rrow[i] = (HAS_R && row < M) ? p.rmap(row) * (int64_t)p.ldr : 0;
       }
       if (!mbar_wait_warp(smem_u32(&sh->tmem_full[buf]), acc_ph, abort)) {
         if (lane == 0) give_up(sh, status, 5);
@@ -238,7 +267,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
         tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + BN, s16);
         tmem_wait_ld();
         const int64_t row = m0 + q * 32 + lane;
-        if (row < p.M) atomicAdd(p.a_sums + row, __uint_as_float(s16[0]));
+        if (row < M) atomicAdd(p.a_sums + row, __uint_as_float(s16[0]));
       }
 #pragma unroll 1
       for (int c = 0; c < BN / 2; c += cw) {
@@ -261,7 +290,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           if (col + s32 >= p.N) break;
           uint4 mk[4];                                   // this row's 32 mask entries, requested ahead of the accumulator
           const int64_t mrow = m0 + q * 32 + lane;
-          const bool masked = p.mask != nullptr && mrow < p.M;
+          const bool masked = p.mask != nullptr && mrow < M;
           if (masked) {
 #pragma unroll
             for (int j = 0; j < 4; ++j)
@@ -320,7 +349,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           // store; rows past M and columns past N are clipped by the tensor map
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0 && m0 + q * 32 < p.M) {
+          if (lane == 0 && m0 + q * 32 < M) {
             if (splits > 1) tma_reduce_add_2d(&tm_c, col, (int)(m0 + q * 32), smem_u32(stg));
             else tma_store_2d(&tm_c, col, (int)(m0 + q * 32), smem_u32(stg));
             bulk_commit();

@@ -4,6 +4,32 @@
 
 namespace bsrl {
 
+// Packed token rows (rows.cu): what the device knows of a batch's row layout.  Device arrays.
+constexpr int kRowGroup = 512;             // environments counted by one block
+constexpr int kRowTileEnvs = 31;           // environments of an attention tile, at most
+constexpr int kBodyTileEnvs = 16;          // ... in the single-body-token layout, whose body rows lie beside the tile
+constexpr int kRowGroupTiles = 640;        // a group's tiles, at most
+struct TokenRows {
+  int* start = nullptr;      // (n_envs + 1): an environment's first token row; the last entry: all of theirs
+  int2* tiles = nullptr;     // attention tiles {first environment, first row}, one entry past the last
+  int* n_tiles = nullptr;    // (2): their number; all token rows, with those ahead of the environments' own
+  int* dst = nullptr;        // (29 n_envs): token row of every encoder input row (saber | torso | leg | slots)
+  float* kb = nullptr;       // key bias by token row
+  int *group_rows = nullptr, *group_tiles = nullptr, *tile_env = nullptr;      // between the two launches
+  int* n_rows() const { return start ? n_tiles + 1 : nullptr; }
+};
+// Where the live flags are: obs rows of `pitch` elements (fp32 or fp16), n_slots flags from mask0 on.  lead: rows of an
+// environment ahead of its slots'; rows_ahead: rows ahead of all of theirs.
+struct RowSource {
+  const void* obs;
+  int f16;
+  int64_t pitch;
+  int mask0, n_slots, lead;
+  int tile_envs;             // environments an attention tile takes at most
+  int64_t rows_ahead;
+};
+int token_rows(const RowSource& src, int64_t n_envs, const TokenRows& out, cudaStream_t stream);
+
 // C = act(A W^T + bias) (+ R).  A (M, K) f16 and W (N, K) f16, both K-contiguous.
 struct LinearArgs {
   const __half* A;
@@ -45,6 +71,11 @@ struct LinearArgs {
   uint32_t* bits_out = nullptr;
   const uint32_t* bits_in = nullptr;
   int64_t bits_ld = 0;               // blocks of 32 rows
+  // Packed token rows: the device's count of the rows (with a_mn of the contraction, K), less n_less; M (K) is its bound.  The
+  // tcgen05 engine only.
+  const int* n_rows = nullptr;
+  int64_t n_less = 0;
+  __device__ __forceinline__ int64_t live(int64_t bound) const { return n_rows ? n_rows[0] - n_less : bound; }
 };
 LinearArgs linear_args(const __half* A, int lda, const __half* W, int ldw, const float* bias,
                        void* C, int ldc, int out_f32, int relu, int64_t M, int N, int K);
@@ -66,7 +97,7 @@ int linear_res(const LinearArgs& p, cudaStream_t stream);    // ... weights resi
 struct RowNorm {
   const float* x;
   int64_t ldx;
-  RowMap map;
+  PlainMap map;
   const float* g;
   const float* b;
   float eps;
@@ -150,6 +181,7 @@ struct LinearLnArgs {
   int64_t ldh;
   int64_t M;
   int N, K;
+  const int* n_rows = nullptr;      // device row count, at most M
 };
 bool linear_ln_ok(const LinearLnArgs& a);
 int linear_ln(const LinearLnArgs& a, cudaStream_t stream);
@@ -178,6 +210,7 @@ struct BlockTailArgs {
   const float* g16[2];
   const float* b16[2];
   int gelu;            // 1: the FFN activation is the exact GELU instead of ReLU
+  const int* n_rows = nullptr;   // device row count, at most M
 };
 bool block_tail_ok(const BlockTailArgs& a);
 int block_tail(const BlockTailArgs& a, cudaStream_t stream);
@@ -205,6 +238,7 @@ struct AttnBlockArgs {
   // n_q = 1: the body row only, out (n_envs, ldo).
   int body = 0, tokens = 29;
   const __half* qkv0 = nullptr;
+  TokenRows rows;            // packed token rows (start: nullptr: 29 per environment); key_bias then goes unread
 };
 // The same for few environments (attn_small.cu): one CTA per environment and head group, up to two problems over the
 // same environments in a launch.  The rows come as fp16 (h) or are LayerNormed from fp32 (norm.x set; dense rows).
@@ -228,16 +262,16 @@ int attn_small(const AttnSmallArgs* a, int n, int n_heads, int64_t n_envs, cudaS
 
 // v columns of a packed projection: copy out (v_out) and / or mix with v0 in place (value residual)
 int vres_mix(__half* v, int ld, int64_t rows, int d, __half* v_out, const __half* v0, const float* vres,
-             cudaStream_t stream);
+             cudaStream_t stream, const int* n_rows = nullptr);
 bool attn_block_ok(const AttnBlockArgs& a);
 int attn_block(const AttnBlockArgs& a, cudaStream_t stream);
 
 // y(f16, ldy) = LayerNorm(x(f32, ldx)) per row, fp32 statistics; layernorm_rows_f32 writes fp32 rows
-// (in place allowed).
+// (in place allowed).  n_rows: the device's row count, at most rows.
 int layernorm_rows(const float* x, int64_t ldx, RowMap xmap, const float* gamma, const float* beta,
-                   float eps, int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t stream);
+                   float eps, int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t stream, const int* n_rows = nullptr);
 int layernorm_rows_f32(const float* x, int64_t ldx, const float* gamma, const float* beta, float eps,
-                       int64_t rows, int d, float* y, int64_t ldy, cudaStream_t stream);
+                       int64_t rows, int d, float* y, int64_t ldy, cudaStream_t stream, const int* n_rows = nullptr);
 
 // SimBaV2 trunk rows (python/policy.py:1140-1155).  mode 0: x = l2n(in * vec) -> x (fp32) and out16;
 // mode 1: y = l2n(in), x' = l2n(x + vec c_alpha (y - x)), out16 = sqrt(d) x'.  scale_relu_rows: relu(in * s).
@@ -254,6 +288,7 @@ struct EmbedBuffers {
   float* key_bias;  // (B, 29)
   int ks, kt, kl, kn;
   __half* obs16 = nullptr;   // optional (B, 630) fp16 copy of the observation rows (rollout buffer row)
+  TokenRows rows;            // packed token rows: live slots' rows only, their places and key bias (start: nullptr: all rows)
 };
 int embed_gather(const void* obs, int obs_dtype, int64_t n_envs, int note_geo, int flux, float z_asinh,
                  const EmbedBuffers& out, cudaStream_t stream);
@@ -275,16 +310,19 @@ struct EncoderArgs {
   float eps;
   float* x;              // (29 n_envs, d) f32 token stream out
   __half* h;             // (29 n_envs, d) f16 LayerNorm rows out, or nullptr
+  const int* dst = nullptr;       // packed token rows: the rows' places in x and h ...
+  const int* n_rows = nullptr;    // ... and their number
 };
 bool encoder_fused_ok(const EncoderArgs& a);
 int encoder_fused(const EncoderArgs& a, cudaStream_t stream);
 
 // Masked MHA over the `tokens` keys of each env (1..96); attention29 is the 29-token case.
 int attention_tokens(const __half* qkv, int ld_qkv, const float* key_bias, int64_t n_envs, int tokens, int d,
-                     int n_heads, int q_first, int n_q, __half* out, int ldo, cudaStream_t stream);
-// Masked MHA over the 29 keys of each env.
+                     int n_heads, int q_first, int n_q, __half* out, int ldo, cudaStream_t stream, const int* start = nullptr);
+// (17, 33 and 65 tokens with start: the first rows are the environments' body tokens, the packed object rows follow)
+// Masked MHA over the 29 keys of each env.  start: packed token rows; key_bias stays one row of 29 per env.
 int attention29(const __half* qkv, int ld_qkv, const float* key_bias, int64_t n_envs, int d,
-                int n_heads, int q_first, int n_q, __half* out, int ldo, cudaStream_t stream);
+                int n_heads, int q_first, int n_q, __half* out, int ldo, cudaStream_t stream, const int* start = nullptr);
 
 // Head tail: masked-lane fill, log-softmax, log-prob of given actions, entropy; HL-Gauss value.
 struct HeadTailArgs {

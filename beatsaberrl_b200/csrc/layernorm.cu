@@ -15,11 +15,12 @@ constexpr int kMaxVec = 8;  // float4 per lane => rows up to 1024 wide
 // F32: the output rows are fp32 (y points at floats) instead of fp16.
 template <int RPW, bool F32>
 __global__ void __launch_bounds__(256, RPW > 1 ? 4 : 1) layernorm_kernel(const float* __restrict__ x, int64_t ldx,
-                                                       RowMap xmap, const float* __restrict__ gamma,
+                                                       PlainMap xmap, const float* __restrict__ gamma,
                                                        const float* __restrict__ beta, float eps,
-                                                       int64_t rows, int d, __half* __restrict__ y,
-                                                       int64_t ldy) {
+                                                       int64_t row_bound, int d, __half* __restrict__ y,
+                                                       int64_t ldy, const int* n_rows) {
   pdl_begin();
+  const int64_t rows = n_rows ? n_rows[0] : row_bound;
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const int nvec = d >> 2;
@@ -28,12 +29,12 @@ __global__ void __launch_bounds__(256, RPW > 1 ? 4 : 1) layernorm_kernel(const f
        row0 += warps * RPW) {
     float4 v[RPW][NV];
     float s[RPW];
+    const int live = rows - row0 < RPW ? (int)(rows - row0) : RPW;      // of these rows
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
       s[r] = 0.f;
-      const int64_t row = row0 + r;
-      if (row < rows) {
-        const float4* xr = reinterpret_cast<const float4*>(x + xmap(row) * ldx);
+      if (r < live) {
+        const float4* xr = reinterpret_cast<const float4*>(x + xmap(row0 + r) * ldx);
 #pragma unroll
         for (int i = 0; i < NV; ++i) {
           const int c = lane + i * 32;
@@ -45,7 +46,7 @@ __global__ void __launch_bounds__(256, RPW > 1 ? 4 : 1) layernorm_kernel(const f
     for (int r = 0; r < RPW; ++r)
 #pragma unroll
       for (int i = 0; i < NV; ++i)
-        if (lane + i * 32 < nvec && row0 + r < rows) s[r] += (v[r][i].x + v[r][i].y) + (v[r][i].z + v[r][i].w);
+        if (lane + i * 32 < nvec && r < live) s[r] += (v[r][i].x + v[r][i].y) + (v[r][i].z + v[r][i].w);
     float mean[RPW], rstd[RPW];
 #pragma unroll
     for (int r = 0; r < RPW; ++r) mean[r] = warp_sum(s[r]) / d;
@@ -54,7 +55,7 @@ __global__ void __launch_bounds__(256, RPW > 1 ? 4 : 1) layernorm_kernel(const f
       float q = 0.f;
 #pragma unroll
       for (int i = 0; i < NV; ++i)
-        if (lane + i * 32 < nvec && row0 + r < rows) {
+        if (lane + i * 32 < nvec && r < live) {
           const float a = v[r][i].x - mean[r], b = v[r][i].y - mean[r], e = v[r][i].z - mean[r], f = v[r][i].w - mean[r];
           q += (a * a + b * b) + (e * e + f * f);
         }
@@ -68,7 +69,7 @@ __global__ void __launch_bounds__(256, RPW > 1 ? 4 : 1) layernorm_kernel(const f
         const float4 b = reinterpret_cast<const float4*>(beta)[c];
 #pragma unroll
         for (int r = 0; r < RPW; ++r)
-          if (row0 + r < rows) {
+          if (r < live) {
             const float o0 = (v[r][i].x - mean[r]) * rstd[r] * g.x + b.x, o1 = (v[r][i].y - mean[r]) * rstd[r] * g.y + b.y;
             const float o2 = (v[r][i].z - mean[r]) * rstd[r] * g.z + b.z, o3 = (v[r][i].w - mean[r]) * rstd[r] * g.w + b.w;
             if (F32) {
@@ -89,25 +90,25 @@ __global__ void __launch_bounds__(256, RPW > 1 ? 4 : 1) layernorm_kernel(const f
 namespace {
 template <bool F32>
 int launch_layernorm(const float* x, int64_t ldx, RowMap xmap, const float* gamma, const float* beta,
-                     float eps, int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t stream);
+                     float eps, int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t stream, const int* n_rows);
 }
 int layernorm_rows(const float* x, int64_t ldx, RowMap xmap, const float* gamma, const float* beta,
-                   float eps, int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t stream) {
-  return launch_layernorm<false>(x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy, stream);
+                   float eps, int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t stream, const int* n_rows) {
+  return launch_layernorm<false>(x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy, stream, n_rows);
 }
 // fp32 rows out (may be in place: every row is read completely before it is written)
 int layernorm_rows_f32(const float* x, int64_t ldx, const float* gamma, const float* beta, float eps,
-                       int64_t rows, int d, float* y, int64_t ldy, cudaStream_t stream) {
+                       int64_t rows, int d, float* y, int64_t ldy, cudaStream_t stream, const int* n_rows) {
   if ((reinterpret_cast<uintptr_t>(y) & 15) || (ldy % 4)) {
     set_error("layernorm: fp32 output rows must be 16-byte aligned");
     return BSRL_ERR_ALIGN;
   }
-  return launch_layernorm<true>(x, ldx, identity_map(), gamma, beta, eps, rows, d, reinterpret_cast<__half*>(y), ldy, stream);
+  return launch_layernorm<true>(x, ldx, identity_map(), gamma, beta, eps, rows, d, reinterpret_cast<__half*>(y), ldy, stream, n_rows);
 }
 namespace {
 template <bool F32>
 int launch_layernorm(const float* x, int64_t ldx, RowMap xmap, const float* gamma, const float* beta,
-                     float eps, int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t stream) {
+                     float eps, int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t stream, const int* n_rows) {
   if (!x || !gamma || !beta || !y) {
     set_error("layernorm: NULL operand");
     return BSRL_ERR_NULL;
@@ -115,6 +116,10 @@ int launch_layernorm(const float* x, int64_t ldx, RowMap xmap, const float* gamm
   if (d <= 0 || d % 4 != 0 || d > kMaxVec * 128 || rows < 0) {
     set_error("layernorm: width %d unsupported (need d %% 4 == 0, d <= 1024)", d);
     return BSRL_ERR_SHAPE;
+  }
+  if (xmap.start) {
+    set_error("layernorm: rows by a table of first rows are not supported");
+    return BSRL_ERR_UNSUPPORTED;
   }
   if (!aligned16(x) || !aligned16(gamma) || !aligned16(beta) || (ldx % 4) || (ldy % 4) ||
       (reinterpret_cast<uintptr_t>(y) & 7)) {
@@ -129,9 +134,9 @@ int launch_layernorm(const float* x, int64_t ldx, RowMap xmap, const float* gamm
   int64_t blocks = (rows + 8 * rpw - 1) / (8 * rpw);
   if (blocks > cap) blocks = cap;
   const unsigned nb = static_cast<unsigned>(blocks);
-  if (rpw == 4) launch_kernel(layernorm_kernel<4, F32>, nb, 256, 0, stream, x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy);
-  else if (rpw == 2) launch_kernel(layernorm_kernel<2, F32>, nb, 256, 0, stream, x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy);
-  else launch_kernel(layernorm_kernel<1, F32>, nb, 256, 0, stream, x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy);
+  if (rpw == 4) launch_kernel(layernorm_kernel<4, F32>, nb, 256, 0, stream, x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy, n_rows);
+  else if (rpw == 2) launch_kernel(layernorm_kernel<2, F32>, nb, 256, 0, stream, x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy, n_rows);
+  else launch_kernel(layernorm_kernel<1, F32>, nb, 256, 0, stream, x, ldx, xmap, gamma, beta, eps, rows, d, y, ldy, n_rows);
   BSRL_LAUNCH_OK("layernorm_kernel");
   return BSRL_OK;
 }

@@ -336,6 +336,9 @@ Paths plan_paths(const Layout& l, int engine, int64_t n_envs) {
   // envs 68 / 70, at 128 74 / 70; d 128 at 64 84 / 90, at 96 98 / 90; d 192 at 1 151 / 230, at 24 223 / 239, at 48 284 /
   // 240; d 256 at 1 124 / 204, at 16 168 / 206, at 32 229 / 209.
   p.small = l.L >= 2 && p.attn_fused && p.tail_fused && p.enc_fused && !l.final_ln.width && n_envs <= small_envs(l);
+  // Packed token rows from the first batch on whose full rows take more than one 128-row tile per SM: below, every kernel has
+  // one wave either way and the two launches that lay the rows out (5 us) come on top.
+  p.packed = !p.small && p.attn_fused && (p.tail_fused || l.d > 256) && n_envs * kT > 148 * 128;
   return p;
 }
 
@@ -371,6 +374,8 @@ Workspace make_workspace(const Layout& l, int64_t B, const Paths& paths) {
   w.att_c = cv.take(B * d * 2);
   w.v0 = cv.take(l.value_residual ? R * d * 2 : 0);
   w.t32 = cv.take(l.trunk_v2 ? B * (int64_t)(l.D > l.Hh ? l.D : l.Hh) * 4 : 0);
+  // the fused block tail leaves x_lead (at least 1,280 bytes per environment, against 250) unused
+  w.rows = !paths.packed ? -1 : paths.tail_fused ? w.x_lead : cv.take(token_rows_bytes(B, kT));
   w.bytes = cv.off;
   return w;
 }

@@ -9,7 +9,7 @@
 #include <string>
 #include <vector>
 
-#include "common.cuh"
+#include "kernels.cuh"
 #include "obs_layout.h"
 
 namespace bsrl {
@@ -95,6 +95,7 @@ struct Paths {
   bool tail_fused;   // out-projection + LayerNorm + FFN in one kernel (no (rows, 4d) hidden buffer)
   bool enc_fused;    // both encoder layers + block 0's LayerNorm in one kernel
   bool small;        // few environments: all blocks as one launch of clusters, or each as four launches of many small CTAs
+  bool packed;       // token rows of live slots only (rows.cu)
 };
 int64_t small_envs(const Layout& l);      // the largest batch that may take Paths::small
 Paths plan_paths(const Layout& l, int engine, int64_t n_envs);
@@ -105,8 +106,14 @@ struct Workspace {
   int64_t x_lead, h_lead, lead16, xt, u, r, z, m1, m2, raw, vraw, att_c;
   int64_t v0;   // block 0's attention values (B*29, d) fp16 (value residual only)
   int64_t t32;  // SimBaV2 trunk: fp32 GEMM outputs (B, max(D, Hh))
+  int64_t rows; // packed token rows: TokenRows' arrays
   int64_t bytes;
 };
+inline int64_t token_rows_bytes(int64_t B, int tokens, bool dst = true) {      // of TokenRows' arrays
+  const int64_t groups = (B + kRowGroup - 1) / kRowGroup, tiles = groups * kRowGroupTiles;
+  return round_up((B + 1) * 4, 256) + round_up((tiles + 1) * 8, 256) + 256 + (dst ? 2 : 1) * round_up(B * tokens * 4, 256) +
+         2 * round_up(groups * 4, 256) + round_up(tiles * 4, 256);
+}
 Workspace make_workspace(const Layout& l, int64_t n_envs, const Paths& paths);
 
 }  // namespace bsrl

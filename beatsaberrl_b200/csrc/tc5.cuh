@@ -100,10 +100,10 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int 
 }
 // Output rows placed by a row map, from a staged block of 32 rows x 128 bytes: as long as the map keeps runs of 8 rows
 // together, four boxes of 8 rows do what one box of 32 does for dense rows.
-inline bool dense_rows(const RowMap& m) { return m.group == 0x7fffffff && m.stride == 0 && m.first == 0; }
+inline bool dense_rows(const RowMap& m) { return m.dense(); }
 // rows per box: 32 dense, 8 mapped, 0: the rows cannot be stored by TMA
 inline int store_box_rows(const RowMap& m, int64_t rows) {
-  return dense_rows(m) ? 32 : m.group % 8 == 0 && rows % 8 == 0 && m.plain(rows - 1) < 0x7fffff00 ? 8 : 0;      // 32-bit coordinates
+  return dense_rows(m) ? 32 : m.start ? 0 : m.group % 8 == 0 && rows % 8 == 0 && m.plain(rows - 1) < 0x7fffff00 ? 8 : 0;      // 32-bit coordinates
 }
 __device__ __forceinline__ void store_mapped8(const CUtensorMap* map, int x, int64_t m0, int64_t rows, const RowMap& cmap, uint32_t src) {
 #pragma unroll

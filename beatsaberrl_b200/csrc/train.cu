@@ -28,15 +28,18 @@
 namespace bsrl {
 int layernorm_bwd(const float* x, int64_t ldx, RowMap xmap, const float* gamma, float eps, const void* gy, int gy_f32,
                   int64_t ldgy, const float* gres, float* gx_out, int64_t ldg, RowMap gmap, float* ggamma, float* gbeta,
-                  int64_t rows, int d, cudaStream_t stream, __half* gx16 = nullptr, int64_t ldg16 = 0);
-int colsum16(const __half* in, int64_t ld, int64_t rows, int n, float* out, cudaStream_t stream);
+                  int64_t rows, int d, cudaStream_t stream, __half* gx16 = nullptr, int64_t ldg16 = 0, const int* n_rows = nullptr,
+                  int64_t n_less = 0);
+int colsum16(const __half* in, int64_t ld, int64_t rows, int n, float* out, cudaStream_t stream, const int* n_rows = nullptr,
+             int64_t n_less = 0);
 int relu_mask16(__half* g, int64_t ldg, const __half* act, int64_t lda, int64_t rows, int n, cudaStream_t stream);
 int cast_rows16(const float* in, int64_t ldi, RowMap imap, float scale, __half* out, int64_t ldo, int64_t rows, int n,
                 cudaStream_t stream);
 int add_rows32(const float* src, int64_t lds, float* dst, int64_t ldd, RowMap dmap, int64_t rows, int n, cudaStream_t stream,
                __half* dst16 = nullptr);
 int gather_rows16(const __half* in, int64_t ldi, RowMap imap, __half* out, int64_t rows, int n, cudaStream_t stream);
-int gather_tokens16(const __half* in, int64_t n_envs, int n, __half* out, cudaStream_t stream);
+int gather_tokens16(const __half* in, int64_t n_envs, int n, __half* out, cudaStream_t stream, const int* dst = nullptr,
+                    const int* n_rows = nullptr);
 int transpose16(const __half* in, int64_t ldi, RowMap imap, int64_t rows, int cols, __half* out, int64_t ldo,
                 int64_t rows_pad, cudaStream_t stream, float* colsum = nullptr);
 int head_tail_bwd(const HeadTailArgs& a, const float* g_logprob, const float* g_entropy, const float* g_value,
@@ -44,12 +47,11 @@ int head_tail_bwd(const HeadTailArgs& a, const float* g_logprob, const float* g_
                   int ldg_v, cudaStream_t stream);
 int attention29_bwd(const __half* qkv, int ld_qkv, const float* key_bias, int64_t n_envs, int d, int n_heads, int q_first,
                     int n_q, const __half* g_out, int ldgo, __half* gq, int ldq, __half* gk, int ldk, __half* gv, int ldv,
-                    cudaStream_t stream);
+                    cudaStream_t stream, const int* start = nullptr);
 
-int vres_mix(__half* v, int ld, int64_t rows, int d, __half* v_out, const __half* v0, const float* vres, cudaStream_t stream);
 int vres_bwd(__half* g, int64_t ldg, const __half* v_own, const __half* v0, const float* ab, float* g_v0, float* g_a, float* g_b,
-             int64_t rows, int d, cudaStream_t stream);
-int add_f32_into_f16(__half* g, int64_t ldg, const float* acc, int64_t rows, int d, cudaStream_t stream);
+             int64_t rows, int d, cudaStream_t stream, const int* n_rows = nullptr);
+int add_f32_into_f16(__half* g, int64_t ldg, const float* acc, int64_t rows, int d, cudaStream_t stream, const int* n_rows = nullptr);
 int simba2_rows(int mode, const float* in, float* x, const float* vec, float c_alpha, int64_t rows, int d, __half* out16, int64_t ld16,
                 cudaStream_t stream);
 int scale_relu_rows(const float* in, const float* s, int64_t rows, int n, __half* out16, cudaStream_t stream);
@@ -94,6 +96,7 @@ TrainPtrs carve_save(const Layout& l, int64_t B, void* save, int64_t* bytes) {
   t.z = f16(B * (d + D));
   t.raw = f32(B * l.head_cols_pad);
   t.vraw = f32(B * l.bins_pad);
+  t.rows = at<void>(save, cv.take(token_rows_bytes(B, kT)));
   *bytes = cv.off;
   return t;
 }
@@ -230,6 +233,13 @@ BwdLayout make_bwd(const Layout& l, int64_t B) {
   return w;
 }
 
+// Rows of a product or row kernel as the device counted them (packed token rows; nothing: the host's number): all token
+// rows, or the slots' among the encoders' input rows.
+struct Count {
+  const int* n_rows = nullptr;
+  int64_t less = 0;
+};
+
 struct Bwd {
   const Ctx& c;
   const Layout& l;
@@ -249,6 +259,13 @@ struct Bwd {
   }
   template <typename T>
   T* S(int64_t off) const { return at<T>(ws, off); }
+  Count all_rows() const { return Count{c.n_rows(), 0}; }
+  Count slot_rows() const { return Count{c.n_rows(), kLead * B}; }
+  LinearArgs counted(LinearArgs a, Count n) const {
+    a.n_rows = n.n_rows;
+    a.n_less = n.less;
+    return a;
+  }
 
   // out (M, K) = g (M, N) . W, W = rows [0, N) of a (N, K) fp16 matrix with pitch ldw; g has pad64(N) columns.
   // The contraction runs over W's ROWS: the tensor cores take W as it lies (an MN-major operand); only shapes
@@ -257,9 +274,11 @@ struct Bwd {
   // whose activation was not positive come out as zero.  With add_rows (fp32 out), the product is ADDED to the rows
   // of out that the map names.
   int dgrad(const __half* g, int64_t ldg, int64_t M, const __half* W, int ldw, int N, int K, void* out, int64_t ldo, bool out_f32,
-            const __half* relu_of = nullptr, int64_t ld_relu = 0, const RowMap* add_rows = nullptr) {
+            const __half* relu_of = nullptr, int64_t ld_relu = 0, const RowMap* add_rows = nullptr, Count count = Count()) {
     LinearArgs r = linear_args(g, (int)ldg, W, ldw, nullptr, out, (int)ldo, out_f32 ? 1 : 0, 0, M, K, N);
     r.w_mn = 1;
+    r.n_rows = count.n_rows;
+    r.n_less = count.less;
     if (relu_of && relu_of == bits_of) {
       r.bits_in = S<uint32_t>(w.bits);
       r.bits_ld = (M + 31) / 32;
@@ -291,8 +310,8 @@ struct Bwd {
   // The ReLU product out = relu(a W^T + b) of M rows.  Where this product and the dgrad through it (relu_of = out, a
   // contraction over Kb) both run on the resident-weight kernel, it leaves its mask as bits for that dgrad.
   const __half* bits_of = nullptr;
-  int relu_fwd(const __half* a, int lda, const Mat& m, int64_t M, int N, int K, __half* out, int Kb) {
-    LinearArgs f = linear_args(a, lda, c.W(m), m.pitch, c.Bv(m), out, N, 0, 1, M, N, K);
+  int relu_fwd(const __half* a, int lda, const Mat& m, int64_t M, int N, int K, __half* out, int Kb, Count count = Count()) {
+    LinearArgs f = counted(linear_args(a, lda, c.W(m), m.pitch, c.Bv(m), out, N, 0, 1, M, N, K), count);
     LinearArgs b = linear_args(a, Kb, c.W(m), N, nullptr, out, N, 0, 0, M, N, Kb);
     f.bits_out = S<uint32_t>(w.bits);
     f.bits_ld = (M + 31) / 32;
@@ -306,7 +325,7 @@ struct Bwd {
   // One Linear, or several stacked ones: gW (N, K) f32 += g^T x over M rows, gb += column sums of g.  Both operands
   // are MN-major (the contraction index is their row); the warp-MMA cross-check engine gets transposed copies (M padded
   // to 64).  gW and gb are zero on entry.
-  int wgrad(const __half* g, int64_t ldg, int64_t M, int N, const __half* x, int64_t ldx, int K, float* gW, int ldgw, float* gb) {
+  int wgrad(const __half* g, int64_t ldg, int64_t M, int N, const __half* x, int64_t ldx, int K, float* gW, int ldgw, float* gb, Count count) {
     const int64_t Mp = pad64(M);
     if (Mp > 0x7fffffff) {
       set_error("backward: too many rows for one weight-gradient product");
@@ -317,10 +336,16 @@ struct Bwd {
     LinearArgs r = linear_args(g, (int)ldg, x, (int)ldx, nullptr, gW, ldgw, 1, 0, N, K, (int)M);
     r.a_mn = r.w_mn = 1;
     r.k_splits = splits;
+    r.n_rows = count.n_rows;
+    r.n_less = count.less;
     if (linear_rows_ok(r)) {
       if (linear_tc5_sums_ok(r)) r.a_sums = gb;
-      else BSRL_TRY(colsum16(g, ldg, M, N, gb, st));
+      else BSRL_TRY(colsum16(g, ldg, M, N, gb, st, count.n_rows, count.less));
       return linear(r, st);
+    }
+    if (count.n_rows) {
+      set_error("backward: a weight gradient over packed token rows needs the tcgen05 engine");
+      return BSRL_ERR_UNSUPPORTED;
     }
     __half *tA = S<__half>(w.tA), *tX = S<__half>(w.tX);
     BSRL_TRY(transpose16(g, ldg, identity_map(), M, N, tA, Mp, Mp, st, gb));
@@ -329,53 +354,55 @@ struct Bwd {
     a.k_splits = splits;
     return linear_mma(a, st);          // as in dgrad
   }
-  int wgrad(const __half* g, int64_t ldg, int64_t M, int N, const __half* x, int64_t ldx, int K, const std::string& name) {
-    return wgrad(g, ldg, M, N, x, ldx, K, G(name + ".weight"), K, G(name + ".bias"));
+  int wgrad(const __half* g, int64_t ldg, int64_t M, int N, const __half* x, int64_t ldx, int K, const std::string& name, Count count = Count()) {
+    return wgrad(g, ldg, M, N, x, ldx, K, G(name + ".weight"), K, G(name + ".bias"), count);
   }
   int cast16(const float* in, int64_t ldi, RowMap map, __half* out, int64_t ldo, int64_t rows, int n) {
     return cast_rows16(in, ldi, map, 1.f, out, ldo, rows, n, st);
   }
   int ln_bwd(const float* x, int64_t ldx, RowMap xmap, const Norm& n, const std::string& name, const void* gy, bool gy_f32,
              int64_t ldgy, const float* gres, float* gx_out, int64_t ldg, RowMap gmap, int64_t rows, int width,
-             __half* gx16 = nullptr) {
+             __half* gx16 = nullptr, Count count = Count()) {
     return layernorm_bwd(x, ldx, xmap, c.G(n), c.cfg->eps, gy, gy_f32 ? 1 : 0, ldgy, gres, gx_out, ldg, gmap, G(name + ".weight"),
-                         G(name + ".bias"), rows, width, st, gx16, width);
+                         G(name + ".bias"), rows, width, st, gx16, width, count.n_rows, count.less);
   }
 
   // FFN + out-projection half of a block on M rows, given the gradient g_out (fp32, and as the fp16 operand g_out16) of
   // the block's output: leaves the gradient of x1 (the stream after the attention residual) in g_x1 and the fp16
   // gradient of the attention output in gatt16.  x1 / h2 / hid / att are the activations of those M rows.
   int tail_bwd(int i, int64_t M, const float* g_out, const __half* g_out16, float* g_x1, const float* x1, const __half* h2,
-               const __half* hid, const __half* att, __half* gatt16) {
+               const __half* hid, const __half* att, __half* gatt16, Count n = Count()) {
     const BlockW& b = l.blocks[i];
     const std::string p = "blocks." + std::to_string(i);
     __half* gA = S<__half>(w.gA);
     __half* gB = S<__half>(w.gB);
     float* g32 = S<float>(w.g32);
-    BSRL_TRY(wgrad(g_out16, d, M, d, hid, F, F, p + ".ffn.2"));
-    BSRL_TRY(dgrad(g_out16, d, M, c.W(b.down), b.down.pitch, d, F, gA, F, false, hid, F));      // g_hid, through the ReLU
-    BSRL_TRY(wgrad(gA, F, M, F, h2, d, d, p + ".ffn.0"));
-    BSRL_TRY(dgrad(gA, F, M, c.W(b.up), b.up.pitch, F, d, g32, d, true));                        // g_h2
-    BSRL_TRY(ln_bwd(x1, d, identity_map(), b.ln_ffn, p + ".ln_ffn", g32, true, d, g_out, g_x1, d, identity_map(), M, d, gB));
-    BSRL_TRY(wgrad(gB, d, M, d, att, d, d, p + ".out_proj"));
-    BSRL_TRY(dgrad(gB, d, M, c.W(b.out), b.out.pitch, d, d, gatt16, d, false));
+    BSRL_TRY(wgrad(g_out16, d, M, d, hid, F, F, p + ".ffn.2", n));
+    BSRL_TRY(dgrad(g_out16, d, M, c.W(b.down), b.down.pitch, d, F, gA, F, false, hid, F, nullptr, n));      // g_hid, through the ReLU
+    BSRL_TRY(wgrad(gA, F, M, F, h2, d, d, p + ".ffn.0", n));
+    BSRL_TRY(dgrad(gA, F, M, c.W(b.up), b.up.pitch, F, d, g32, d, true, nullptr, 0, nullptr, n));      // g_h2
+    BSRL_TRY(ln_bwd(x1, d, identity_map(), b.ln_ffn, p + ".ln_ffn", g32, true, d, g_out, g_x1, d, identity_map(), M, d, gB, n));
+    BSRL_TRY(wgrad(gB, d, M, d, att, d, d, p + ".out_proj", n));
+    BSRL_TRY(dgrad(gB, d, M, c.W(b.out), b.out.pitch, d, d, gatt16, d, false, nullptr, 0, nullptr, n));
     return BSRL_OK;
   }
 
   // recompute x1 = x[rows] + att Wo^T + bo, h2 = LN_ffn(x1), hid = relu(h2 W0^T + b0) on M rows
-  int tail_fwd(int i, int64_t M, const float* x_in, RowMap xrows, const __half* att, float* x1, __half* h2, __half* hid) {
+  int tail_fwd(int i, int64_t M, const float* x_in, RowMap xrows, const __half* att, float* x1, __half* h2, __half* hid, Count n = Count()) {
     const BlockW& b = l.blocks[i];
-    LinearArgs po = linear_args(att, d, c.W(b.out), d, c.Bv(b.out), x1, d, 1, 0, M, d, d);
+    LinearArgs po = counted(linear_args(att, d, c.W(b.out), d, c.Bv(b.out), x1, d, 1, 0, M, d, d), n);
     po.R = x_in; po.ldr = d; po.rmap = xrows;
     BSRL_TRY(linear(po, st));
-    BSRL_TRY(layernorm(x1, d, identity_map(), c.G(b.ln_ffn), c.Be(b.ln_ffn), c.cfg->eps, M, d, h2, d, st));
-    return relu_fwd(h2, d, b.up, M, F, d, hid, d);
+    BSRL_TRY(layernorm(x1, d, identity_map(), c.G(b.ln_ffn), c.Be(b.ln_ffn), c.cfg->eps, M, d, h2, d, st, n.n_rows));
+    return relu_fwd(h2, d, b.up, M, F, d, hid, d, n);
   }
 
   int run(const HeadTailArgs& tail, const float* g_logprob, const float* g_entropy, const float* g_value,
           const float* g_vlogits, const float* g_logits) {
     const float eps = c.cfg->eps;
-    const RowMap ident = identity_map(), lead_rows{kLead, kT, 0}, torso_rows{1, kT, 2};
+    const RowMap ident = identity_map(), lead_rows = c.lead_rows(), torso_rows{1, kT, 2, c.rows.start};
+    const Count all = all_rows();
+    const int *nr = all.n_rows, *start = c.rows.start;
     const int ldz = d + D, Hh = l.Hh;
     __half* h16 = S<__half>(w.h16);
     __half* qkv = S<__half>(w.qkv16);
@@ -395,8 +422,9 @@ struct Bwd {
     float* gs32 = S<float>(w.gsmall32);
     __half* gs16 = S<__half>(w.gsmall16);
     const float* x_last = sv.x[l.L - 1];            // the stream entering the last block = the critic's input
-    // the torso rows (token 2 of every env) of a token-row matrix are a matrix of pitch 29 times its own
-    const __half *hv = h16, *hv_torso = h16 + 2 * d;
+    // the torso rows (token 2 of every env) of a token-row matrix are a matrix of pitch 29 times its own, or, of packed rows, copied
+    const __half *hv = h16, *hv_torso = start ? hl : h16 + 2 * d;
+    const int ld_torso = start ? d : kT * d;
     __half* attc = S<__half>(w.attc16);
     __half* z = S<__half>(w.z16);
     __half* m1 = S<__half>(w.m1);
@@ -411,10 +439,17 @@ struct Bwd {
     begin_overlap(R);
 
     // ---- recompute the critic's activations (its pool lands in z beside the trunk's output)
-    BSRL_TRY(layernorm(x_last, d, ident, c.G(l.critic_ln), c.Be(l.critic_ln), eps, R, d, h16, d, st));
-    BSRL_TRY(linear(linear_args(hv, d, c.W(l.critic_kv), d, c.Bv(l.critic_kv), qkv + d, 3 * d, 0, 0, R, 2 * d, d), st));
-    BSRL_TRY(linear(linear_args(hv_torso, kT * d, c.W(l.critic_q), d, c.Bv(l.critic_q), qkv + 2 * 3 * d, kT * 3 * d, 0, 0, B, d, d), st));
-    BSRL_TRY(attention(qkv, 3 * d, sv.key_bias, B, d, l.H, 2, 1, attc, d, st));
+    BSRL_TRY(layernorm(x_last, d, ident, c.G(l.critic_ln), c.Be(l.critic_ln), eps, R, d, h16, d, st, nr));
+    BSRL_TRY(linear(counted(linear_args(hv, d, c.W(l.critic_kv), d, c.Bv(l.critic_kv), qkv + d, 3 * d, 0, 0, R, 2 * d, d), all), st));
+    if (start) {
+      BSRL_TRY(gather_rows16(h16, d, torso_rows, hl, B, d, st));
+      LinearArgs pq = linear_args(hl, d, c.W(l.critic_q), d, c.Bv(l.critic_q), qkv, 3 * d, 0, 0, B, d, d);
+      pq.cmap = torso_rows;
+      BSRL_TRY(linear(pq, st));
+    } else {
+      BSRL_TRY(linear(linear_args(hv_torso, ld_torso, c.W(l.critic_q), d, c.Bv(l.critic_q), qkv + 2 * 3 * d, kT * 3 * d, 0, 0, B, d, d), st));
+    }
+    BSRL_TRY(attention(qkv, 3 * d, sv.key_bias, B, d, l.H, 2, 1, attc, d, st, start));
     BSRL_TRY(linear(linear_args(attc, d, c.W(l.critic_out), d, c.Bv(l.critic_out), z, ldz, 0, 0, B, d, d), st));
     BSRL_TRY(linear(linear_args(z, ldz, c.W(l.critic_m0), ldz, c.Bv(l.critic_m0), m1, D, 0, 1, B, D, ldz), st));
     BSRL_TRY(linear(linear_args(m1, D, c.W(l.critic_m1), D, c.Bv(l.critic_m1), m2, D, 0, 1, B, D, D), st));
@@ -431,12 +466,12 @@ struct Bwd {
     BSRL_TRY(wgrad(gs16, d, B, d, attc, d, d, "critic_out"));
     BSRL_TRY(dgrad(gs16, d, B, c.W(l.critic_out), l.critic_out.pitch, d, d, gA, d, false));       // g_attc (B, d)
     __half* gq_c = gs16;                                                                          // (B, d)
-    BSRL_TRY(attention29_bwd(qkv, 3 * d, sv.key_bias, B, d, l.H, 2, 1, gA, d, gq_c, d, gB, 2 * d, gB + d, 2 * d, st));
-    BSRL_TRY(wgrad(gB, 2 * d, R, 2 * d, hv, d, d, "critic_k"));                                // k and v stacked
-    BSRL_TRY(wgrad(gq_c, d, B, d, hv_torso, kT * d, d, "critic_q"));
-    BSRL_TRY(dgrad(gB, 2 * d, R, c.W(l.critic_kv), l.critic_kv.pitch, 2 * d, d, g32, d, true));    // g_hv from k, v
+    BSRL_TRY(attention29_bwd(qkv, 3 * d, sv.key_bias, B, d, l.H, 2, 1, gA, d, gq_c, d, gB, 2 * d, gB + d, 2 * d, st, start));
+    BSRL_TRY(wgrad(gB, 2 * d, R, 2 * d, hv, d, d, "critic_k", all));                           // k and v stacked
+    BSRL_TRY(wgrad(gq_c, d, B, d, hv_torso, ld_torso, d, "critic_q"));
+    BSRL_TRY(dgrad(gB, 2 * d, R, c.W(l.critic_kv), l.critic_kv.pitch, 2 * d, d, g32, d, true, nullptr, 0, nullptr, all));    // g_hv from k, v
     BSRL_TRY(dgrad(gq_c, d, B, c.W(l.critic_q), l.critic_q.pitch, d, d, g32, d, true, nullptr, 0, &torso_rows));   // ... and q
-    BSRL_TRY(ln_bwd(x_last, d, ident, l.critic_ln, "critic_ln", g32, true, d, nullptr, gx, d, ident, R, d));   // gx = critic's share
+    BSRL_TRY(ln_bwd(x_last, d, ident, l.critic_ln, "critic_ln", g32, true, d, nullptr, gx, d, ident, R, d, nullptr, all));   // gx = critic's share
 
     // ---- action heads (one stacked product) and trunk
     BSRL_TRY(wgrad(graw, w.ld_graw, B, w.ld_graw, sv.z + d, ldz, D, "heads.0"));
@@ -473,22 +508,22 @@ struct Bwd {
     float* gv0 = vres ? S<float>(w.gv0) : nullptr;
     if (vres) {
       const BlockW& b0 = l.blocks[0];
-      BSRL_TRY(layernorm(sv.x[0], d, ident, c.G(b0.ln_attn), c.Be(b0.ln_attn), eps, R, d, h16, d, st));
-      BSRL_TRY(linear(linear_args(h16, d, c.W(b0.qkv, 2 * d), d, c.Bv(b0.qkv, 2 * d), v0, d, 0, 0, R, d, d), st));
+      BSRL_TRY(layernorm(sv.x[0], d, ident, c.G(b0.ln_attn), c.Be(b0.ln_attn), eps, R, d, h16, d, st, nr));
+      BSRL_TRY(linear(counted(linear_args(h16, d, c.W(b0.qkv, 2 * d), d, c.Bv(b0.qkv, 2 * d), v0, d, 0, 0, R, d, d), all), st));
       BSRL_CUDA_OK(cudaMemsetAsync(gv0, 0, (size_t)R * d * 4, st));
     }
     // after the projection of block i > 0: keep the block's own values, mix block 0's in (the forward's arithmetic)
     auto mix_values = [&](int i, __half* vcols, int ld) -> int {
       if (!vres || i == 0) return BSRL_OK;
-      return vres_mix(vcols, ld, R, d, vown, v0, at<float>(c.arena, l.blocks[i].vres), st);
+      return vres_mix(vcols, ld, R, d, vown, v0, at<float>(c.arena, l.blocks[i].vres), st, nr);
     };
     // after the attention backward of block i: the gradient of the mixed values becomes that of the block's own values
     // (i > 0; block 0's share collects in gv0), or block 0's own gradient takes the collected share in
     auto unmix_grads = [&](int i, __half* gvcols, int64_t ld) -> int {
       if (!vres) return BSRL_OK;
-      if (i == 0) return add_f32_into_f16(gvcols, ld, gv0, R, d, st);
+      if (i == 0) return add_f32_into_f16(gvcols, ld, gv0, R, d, st, nr);
       const std::string pn = "blocks." + std::to_string(i);
-      return vres_bwd(gvcols, ld, vown, v0, at<float>(c.arena, l.blocks[i].vres), gv0, G(pn + ".vres_a"), G(pn + ".vres_b"), R, d, st);
+      return vres_bwd(gvcols, ld, vown, v0, at<float>(c.arena, l.blocks[i].vres), gv0, G(pn + ".vres_a"), G(pn + ".vres_b"), R, d, st, nr);
     };
 
     // ---- last block, on the lead rows
@@ -496,16 +531,16 @@ struct Bwd {
       const int i = l.L - 1;
       const BlockW& b = l.blocks[i];
       const std::string p = "blocks." + std::to_string(i);
-      BSRL_TRY(layernorm(x_last, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h16, d, st));
+      BSRL_TRY(layernorm(x_last, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h16, d, st, nr));
       BSRL_TRY(gather_rows16(h16, d, lead_rows, hl, Rl, d, st));
-      BSRL_TRY(linear(linear_args(h16, d, c.W(b.qkv, d), d, c.Bv(b.qkv, d), qkv + d, 3 * d, 0, 0, R, 2 * d, d), st));
+      BSRL_TRY(linear(counted(linear_args(h16, d, c.W(b.qkv, d), d, c.Bv(b.qkv, d), qkv + d, 3 * d, 0, 0, R, 2 * d, d), all), st));
       {
         LinearArgs pq = linear_args(hl, d, c.W(b.qkv), d, c.Bv(b.qkv), qkv, 3 * d, 0, 0, Rl, d, d);
         pq.cmap = lead_rows;
         BSRL_TRY(linear(pq, st));
       }
       BSRL_TRY(mix_values(i, qkv + 2 * d, 3 * d));
-      BSRL_TRY(attention(qkv, 3 * d, sv.key_bias, B, d, l.H, 0, kLead, att, d, st));
+      BSRL_TRY(attention(qkv, 3 * d, sv.key_bias, B, d, l.H, 0, kLead, att, d, st, start));
       BSRL_TRY(tail_fwd(i, Rl, x_last, lead_rows, att, x1, h2, hid));
       float* g_x1 = x1 + Rl * d;                       // (Rl, d) f32: the unused upper part of the x1 buffer
       __half* g_lead16 = gx16;                         // (Rl, d): free until this block's last LayerNorm backward
@@ -522,13 +557,13 @@ struct Bwd {
       }
       BSRL_TRY(tail_bwd(i, Rl, g_lead, g_lead16, g_x1, x1, h2, hid, att, gA));   // gA: fp16 gradient of the attention output
       __half* gq = gs16;                               // (Rl, d)
-      BSRL_TRY(attention29_bwd(qkv, 3 * d, sv.key_bias, B, d, l.H, 0, kLead, gA, d, gq, d, gB, 2 * d, gB + d, 2 * d, st));
+      BSRL_TRY(attention29_bwd(qkv, 3 * d, sv.key_bias, B, d, l.H, 0, kLead, gA, d, gq, d, gB, 2 * d, gB + d, 2 * d, st, start));
       BSRL_TRY(unmix_grads(i, gB + d, 2 * d));
-      BSRL_TRY(wgrad(gB, 2 * d, R, 2 * d, h16, d, d, p + ".k_proj"));                               // k and v stacked
+      BSRL_TRY(wgrad(gB, 2 * d, R, 2 * d, h16, d, d, p + ".k_proj", all));                          // k and v stacked
       BSRL_TRY(wgrad(gq, d, Rl, d, hl, d, d, p + ".q_proj"));
-      BSRL_TRY(dgrad(gB, 2 * d, R, c.W(b.qkv, d), b.qkv.pitch, 2 * d, d, g32, d, true));           // g_h from k, v
+      BSRL_TRY(dgrad(gB, 2 * d, R, c.W(b.qkv, d), b.qkv.pitch, 2 * d, d, g32, d, true, nullptr, 0, nullptr, all));           // g_h from k, v
       BSRL_TRY(dgrad(gq, d, Rl, c.W(b.qkv), b.qkv.pitch, d, d, g32, d, true, nullptr, 0, &lead_rows));   // ... and from q
-      BSRL_TRY(ln_bwd(x_last, d, ident, b.ln_attn, p + ".ln_attn", g32, true, d, gx, gx, d, ident, R, d, gx16));
+      BSRL_TRY(ln_bwd(x_last, d, ident, b.ln_attn, p + ".ln_attn", g32, true, d, gx, gx, d, ident, R, d, gx16, all));
       BSRL_TRY(add_rows32(g_x1, d, gx, d, lead_rows, Rl, d, st, gx16));                            // the residual path of the lead rows
     }
 
@@ -537,21 +572,21 @@ struct Bwd {
       const BlockW& b = l.blocks[i];
       const std::string p = "blocks." + std::to_string(i);
       const float* x_in = sv.x[i];
-      BSRL_TRY(layernorm(x_in, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h16, d, st));
-      BSRL_TRY(linear(linear_args(h16, d, c.W(b.qkv), d, c.Bv(b.qkv), qkv, 3 * d, 0, 0, R, 3 * d, d), st));
+      BSRL_TRY(layernorm(x_in, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h16, d, st, nr));
+      BSRL_TRY(linear(counted(linear_args(h16, d, c.W(b.qkv), d, c.Bv(b.qkv), qkv, 3 * d, 0, 0, R, 3 * d, d), all), st));
       BSRL_TRY(mix_values(i, qkv + 2 * d, 3 * d));
-      BSRL_TRY(attention(qkv, 3 * d, sv.key_bias, B, d, l.H, 0, kT, att, d, st));
-      BSRL_TRY(tail_fwd(i, R, x_in, ident, att, x1, h2, hid));
-      BSRL_TRY(tail_bwd(i, R, gx, gx16, gx, x1, h2, hid, att, gA));                           // gx: g(x_{i+1}) -> g(x1)
-      BSRL_TRY(attention29_bwd(qkv, 3 * d, sv.key_bias, B, d, l.H, 0, kT, gA, d, gB, 3 * d, gB + d, 3 * d, gB + 2 * d, 3 * d, st));
+      BSRL_TRY(attention(qkv, 3 * d, sv.key_bias, B, d, l.H, 0, kT, att, d, st, start));
+      BSRL_TRY(tail_fwd(i, R, x_in, ident, att, x1, h2, hid, all));
+      BSRL_TRY(tail_bwd(i, R, gx, gx16, gx, x1, h2, hid, att, gA, all));                           // gx: g(x_{i+1}) -> g(x1)
+      BSRL_TRY(attention29_bwd(qkv, 3 * d, sv.key_bias, B, d, l.H, 0, kT, gA, d, gB, 3 * d, gB + d, 3 * d, gB + 2 * d, 3 * d, st, start));
       BSRL_TRY(unmix_grads(i, gB + 2 * d, 3 * d));
-      BSRL_TRY(wgrad(gB, 3 * d, R, 3 * d, h16, d, d, p + ".q_proj"));                           // q, k and v stacked
-      BSRL_TRY(dgrad(gB, 3 * d, R, c.W(b.qkv), b.qkv.pitch, 3 * d, d, g32, d, true));
-      BSRL_TRY(ln_bwd(x_in, d, ident, b.ln_attn, p + ".ln_attn", g32, true, d, gx, gx, d, ident, R, d, gx16));   // gx: g(x_i)
+      BSRL_TRY(wgrad(gB, 3 * d, R, 3 * d, h16, d, d, p + ".q_proj", all));                      // q, k and v stacked
+      BSRL_TRY(dgrad(gB, 3 * d, R, c.W(b.qkv), b.qkv.pitch, 3 * d, d, g32, d, true, nullptr, 0, nullptr, all));
+      BSRL_TRY(ln_bwd(x_in, d, ident, b.ln_attn, p + ".ln_attn", g32, true, d, gx, gx, d, ident, R, d, gx16, all));   // gx: g(x_i)
     }
 
     // ---- token encoders (no gradient flows to the observation): the tokens' gradients in the feature matrix's row order
-    BSRL_TRY(gather_tokens16(gx16, B, d, gB, st));
+    BSRL_TRY(gather_tokens16(gx16, B, d, gB, st, c.rows.dst, nr));
     struct Enc { const Encoder* e; const char* name; int64_t rows, row0; int in; float* gw; };
     const Enc encs[4] = {{&l.note, "note_mlp", (int64_t)kSlots * B, 5 * B, l.note_in, grads + gl.enc0[0]},
                          {&l.saber, "saber_mlp", 2 * B, 0, kSaberFeat + 2, grads + gl.enc0[1]},
@@ -560,18 +595,19 @@ struct Bwd {
     for (const Enc& e : encs) {
       const __half* feat = sv.feat + e.row0 * 64;
       __half* g = gB + e.row0 * d;
-      BSRL_TRY(relu_fwd(feat, 64, e.e->l0, e.rows, d, 64, hid, d));                                  // hidden
+      const Count n = e.e == &l.note ? slot_rows() : Count();
+      BSRL_TRY(relu_fwd(feat, 64, e.e->l0, e.rows, d, 64, hid, d, n));                               // hidden
       if (c.cfg->emb_ln) {
         // tokens = emb_ln(encoder output): recompute the encoder's output rows (fp32) and take g back through the
         // LayerNorm; the fp16 copy of the result replaces g
         float* pre = x1;                                  // (e.rows, d) f32: the block scratch is free by now
-        BSRL_TRY(linear(linear_args(hid, d, c.W(e.e->l1), e.e->l1.pitch, c.Bv(e.e->l1), pre, d, 1, 0, e.rows, d, d), st));
-        BSRL_TRY(ln_bwd(pre, d, ident, l.emb_ln, "emb_ln", g, false, d, nullptr, g32, d, ident, e.rows, d, g));
+        BSRL_TRY(linear(counted(linear_args(hid, d, c.W(e.e->l1), e.e->l1.pitch, c.Bv(e.e->l1), pre, d, 1, 0, e.rows, d, d), n), st));
+        BSRL_TRY(ln_bwd(pre, d, ident, l.emb_ln, "emb_ln", g, false, d, nullptr, g32, d, ident, e.rows, d, g, n));
       }
-      BSRL_TRY(wgrad(g, d, e.rows, d, hid, d, d, std::string(e.name) + ".2"));
-      BSRL_TRY(dgrad(g, d, e.rows, c.W(e.e->l1), e.e->l1.pitch, d, d, gA, d, false, hid, d));       // through the hidden ReLU
+      BSRL_TRY(wgrad(g, d, e.rows, d, hid, d, d, std::string(e.name) + ".2", n));
+      BSRL_TRY(dgrad(g, d, e.rows, c.W(e.e->l1), e.e->l1.pitch, d, d, gA, d, false, hid, d, nullptr, n));       // through the hidden ReLU
       // first layer: the K-padded (d, 64) product's first `in` columns are the gradient
-      BSRL_TRY(wgrad(gA, d, e.rows, d, feat, 64, 64, e.gw, 64, G(std::string(e.name) + ".0.bias")));
+      BSRL_TRY(wgrad(gA, d, e.rows, d, feat, 64, 64, e.gw, 64, G(std::string(e.name) + ".0.bias"), n));
       BSRL_CUDA_OK(cudaMemcpy2DAsync(G(std::string(e.name) + ".0.weight"), (size_t)e.in * 4, e.gw, 64 * 4, (size_t)e.in * 4, d,
                                      cudaMemcpyDeviceToDevice, st));
     }
@@ -798,6 +834,7 @@ int bsrl_backward(const bsrl_config* cfg, const void* arena, int64_t n_envs, con
   c.ws = workspace;
   c.B = n_envs;
   c.st = st;
+  if (plan_paths(l, process_engine(), n_envs).packed) c.rows = carve_rows(t.rows, n_envs, kT);       // as the forward laid them out
   Bwd b{c, c.l, t, w, workspace, grads, gl, loss_scale, st, n_envs, n_envs * kT, n_envs * kLead, l.d, l.F, l.D};
   HeadTailArgs h;
   memset(&h, 0, sizeof(h));

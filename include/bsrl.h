@@ -410,7 +410,9 @@ int bsrl_head_layout(const bsrl_config* cfg, int32_t* head_cols_pad, int32_t* bi
 /* Where a named intermediate of the last forward sits in the caller's workspace (valid until the next
  * call on that workspace): "trunk_h" (the reference's _diag_h), "x_resolved" (the residual stream
  * entering the last block, the critic's input; python/policy.py:1302-1305), "key_bias", "readout",
- * "head_out".  dtype is a bsrl_dtype; ld_elems the row pitch in elements. */
+ * "head_out".  dtype is a bsrl_dtype; ld_elems the row pitch in elements.  Batches of more than 18,944 token rows keep
+ * rows only for an environment's lead tokens and its slots up to the last live one, environment after environment; there
+ * the stream is "x_packed", and "row_start" (n_envs + 1, int32) says where an environment's rows begin. */
 int bsrl_workspace_region(const bsrl_config* cfg, int64_t n_envs, const char* name, int64_t* byte_offset,
                           int64_t* rows, int64_t* cols, int64_t* ld_elems, int32_t* dtype);
 

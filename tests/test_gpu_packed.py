@@ -1,0 +1,123 @@
+"""Packed token rows: batches past 18,944 token rows give rows only to each environment's slots up to its last live one.  The same
+environments in slices of a few hundred take the full layout: forwards must agree bit for bit, gradients up to the order of fp32
+sums, whatever the masks are."""
+import pytest
+import torch
+
+from helpers import make_cfg, cuda_policy
+from oracle import policy_oracle as po
+
+pytestmark = pytest.mark.gpu
+
+
+def _masks(kind, envs, slots, gen):
+    if kind == "none":
+        return torch.zeros(envs, slots)
+    if kind == "all":
+        return torch.ones(envs, slots)
+    if kind == "holes":                       # any subset: the last live slot decides
+        return (torch.rand(envs, slots, generator=gen) < 0.3).float()
+    if kind == "last":                        # one live slot, anywhere
+        return torch.eye(slots)[torch.randint(0, slots, (envs,), generator=gen)]
+    assert kind == "runs"                     # long runs of empty and of full environments
+    return (torch.arange(envs)[:, None] // 700 % 2 * torch.ones(1, slots)).float()
+
+
+def _obs(kind, envs, seed):
+    gen = torch.Generator().manual_seed(seed)
+    obs = po.make_obs(envs, seed)
+    obs[:, po.OFF_MASK:po.OFF_MASK + 24] = _masks(kind, envs, 24, gen)
+    return obs
+
+
+SHAPES = [("cfg1", {}), ("recipe", {}), ("recipe", dict(value_residual=True)), ("cfg1", dict(n_heads=2, value_residual=True)), ("cfg1", dict(n_heads=2)),
+          ("cfg4", {}), ("cfg4", dict(value_residual=True)), ("cfg1", dict(emb_ln=True, final_ln=True)), ("tiny", dict(trunk_arch="simbav2")),
+          ("cfg2", dict(value_residual=True))]
+
+
+@pytest.mark.parametrize("kind", ["none", "all", "holes", "last", "runs"])
+@pytest.mark.parametrize("name,opts", SHAPES)
+def test_forward_gives_the_bits_of_the_full_layout(name, opts, kind):
+    cfg = make_cfg(name, name == "recipe", opts=dict(opts, n_blocks=2))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
+    envs = 2600 if kind == "runs" else 1037
+    obs = _obs(kind, envs, 41).cuda()
+    for o in (obs, obs.half()):
+        logits, value = m.forward_stacked(o)
+        for lo in range(0, envs, 500):
+            l, v = m.forward_stacked(o[lo:lo + 500])
+            assert torch.equal(l, logits[lo:lo + 500]) and torch.equal(v, value[lo:lo + 500]), lo
+    m.check_device()
+
+
+@pytest.mark.parametrize("envs", [653, 654, 1024, 1025, 2357, 4736, 8193])
+def test_sizes_around_the_line_and_pairs_of_ctas(envs):
+    cfg = make_cfg("cfg1", opts=dict(n_blocks=2))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
+    obs = po.make_obs(envs, 42, padded=True).cuda()
+    logits, value = m.forward_stacked(obs)
+    for lo in range(0, envs, 600):
+        l, v = m.forward_stacked(obs[lo:lo + 600])
+        assert torch.equal(l, logits[lo:lo + 600]) and torch.equal(v, value[lo:lo + 600]), lo
+
+
+@pytest.mark.parametrize("name,opts", [("cfg1", {}), ("recipe", dict(value_residual=True)), ("cfg4", {})])
+def test_all_live_in_long_runs(name, opts):
+    """Long runs launch the attention kernels of both layouts: the full one's works where every slot is live, the other one where a
+    single one is not."""
+    cfg = make_cfg(name, opts=dict(opts, n_blocks=2))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
+    obs = po.make_obs(2401, 47).cuda()
+    for dead in (0, 1):
+        obs[1700:1700 + dead, po.OFF_MASK + 23] = 0.0
+        logits, value = m.forward_stacked(obs)
+        for lo in range(0, 2401, 600):
+            l, v = m.forward_stacked(obs[lo:lo + 600])
+            assert torch.equal(l, logits[lo:lo + 600]) and torch.equal(v, value[lo:lo + 600]), (dead, lo)
+
+
+@pytest.mark.parametrize("name", ["cfg1", "recipe", "cfg4"])
+def test_not_a_number_stays_in_its_environment(name):
+    cfg = make_cfg(name, opts=dict(n_blocks=2))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
+    obs = _obs("holes", 1200, 43).cuda()
+    clean_l, clean_v = m.forward_stacked(obs)
+    bad = torch.arange(3, 1200, 7, device="cuda")
+    obs[bad, po.OFF_MASK + 2] = float("nan")      # into the key bias, and through the attention into every row of the environment
+    obs[bad[::2], po.OFF_NOTES:po.OFF_MASK] = float("inf")
+    logits, value = m.forward_stacked(obs)
+    good = torch.ones(1200, dtype=torch.bool, device="cuda")
+    good[bad] = False
+    assert torch.equal(logits[good], clean_l[good]) and torch.equal(value[good], clean_v[good])
+    assert torch.isnan(logits[bad]).any(-1).any(-1).all()
+
+
+@pytest.mark.parametrize("kind", ["none", "all", "holes"])
+@pytest.mark.parametrize("name,opts", [("cfg1", {}), ("recipe", dict(value_residual=True)), ("cfg4", {}), ("cfg1", dict(emb_ln=True, final_ln=True)),
+                                       ("tiny", dict(trunk_arch="simbav2"))])
+def test_gradients_equal_the_sum_over_slices(name, opts, kind):
+    """Per row the same arithmetic, so the difference is the order of fp32 sums over some 20 thousand rows (about 2^-24 sqrt(rows) =
+    1e-5 of the terms' root sum of squares; the bound allows the atomics' order on top)."""
+    envs = 701
+    cfg = make_cfg(name, name == "recipe", opts=dict(opts, n_blocks=2))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 5))
+    obs, act, up = _obs(kind, envs, 44).cuda(), po.make_actions(envs, cfg, 22).cuda(), po.make_upstream(envs, cfg, 23)
+
+    def loss(s):
+        _, lp, ent, val = m.get_action_and_value(obs[s], act[s])
+        return ((up["logprob"][s].cuda() * lp).sum() + (up["entropy"][s].cuda() * ent).sum() + (up["value"][s].cuda() * val).sum()
+                + (up["value_logits"][s].cuda() * m._value_logits).sum())
+
+    with torch.enable_grad():
+        # whatever the buffers held before must not show: rows of other environments, and not a number
+        m.get_action_and_value(torch.full_like(obs, float("nan")), act)[1].sum().backward()
+        m.zero_grad()
+        loss(slice(0, envs)).backward()
+        whole = {k: p.grad.clone() for k, p in m.named_parameters() if p.grad is not None}
+        m.zero_grad()
+        for lo in range(0, envs, 351):
+            loss(slice(lo, lo + 351)).backward()
+    m.check_device()
+    top = max(float(g.norm()) for g in whole.values())
+    for k, g in whole.items():
+        assert float((m.get_parameter(k).grad - g).norm()) <= 1e-4 * float(g.norm()) + 1e-6 * top, k
