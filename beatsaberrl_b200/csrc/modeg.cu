@@ -29,7 +29,7 @@ struct GLayout {
   int64_t bytes;
 };
 struct GWorkspace {
-  int64_t key_bias, f_body, f_obj, x, h, qkv, att, hid, x_lead, h_lead, lead16, raw, bytes;
+  int64_t key_bias, f_body, f_obj, x, h, qkv, att, hid, x_lead, h_lead, lead16, raw, rows, bytes;
 };
 
 struct Carve {
@@ -179,7 +179,14 @@ std::vector<CopySlot> g_copy_slots(const GLayout& l, const std::vector<ParamSlot
   return out;
 }
 
-GWorkspace make_gws(const GLayout& l, int64_t B, bool tail_fused, bool attn_fused) {
+// Packed token rows (rows.cu): the body rows first, then the environments' object rows up to their last live one.  Where the
+// attention kernels that know the body token run, and from more than one 128-row tile per SM on.
+bool g_packed(const GLayout& l, int engine, int64_t n_envs) {
+  const int dh = l.d / l.H;
+  return engine == 0 && l.d % 64 == 0 && (l.T == 17 || l.T == 33 || l.T == 65) && (dh == 32 || dh == 64) && n_envs * l.T > 148 * 128;
+}
+
+GWorkspace make_gws(const GLayout& l, int64_t B, bool tail_fused, bool attn_fused, bool packed) {
   GWorkspace w;
   Carve cv;
   const int64_t R = B * l.T;
@@ -196,6 +203,7 @@ GWorkspace make_gws(const GLayout& l, int64_t B, bool tail_fused, bool attn_fuse
   w.h_lead = cv.take(B * d * 2);
   w.lead16 = cv.take(B * d * 2);
   w.raw = cv.take(B * (int64_t)l.cols_pad * 4);
+  w.rows = packed ? cv.take(token_rows_bytes(B, l.n_obj, false)) : -1;
   w.bytes = cv.off;
   return w;
 }
@@ -209,7 +217,7 @@ bool g_tail_fused(const GLayout& l, int engine) {
 // (token 0 always attendable, object j by its live flag: 0 or -16384, python/policy.py:422-428)
 __global__ void __launch_bounds__(256) embed_g_kernel(const float* __restrict__ obs, int64_t n_envs, int obs_dim, int body_dim,
                                                       int body_k, int n_obj, int obj_dim, __half* __restrict__ f_body,
-                                                      __half* __restrict__ f_obj, float* __restrict__ key_bias) {
+                                                      __half* __restrict__ f_obj, float* __restrict__ key_bias, TokenRows rows) {
   pdl_begin();
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
@@ -218,12 +226,18 @@ __global__ void __launch_bounds__(256) embed_g_kernel(const float* __restrict__ 
     const float* o = obs + env * obs_dim;
     for (int c = lane; c < body_k; c += 32) f_body[env * body_k + c] = __float2half_rn(c < body_dim ? o[c] : 0.f);
     const float* ob = o + body_dim;
-    for (int i = lane; i < n_obj * 64; i += 32) {
+    const int64_t obj0 = rows.start ? rows.start[env] : env * n_obj;
+    const int n_rows = rows.start ? (int)(rows.start[env + 1] - obj0) : n_obj;
+    for (int i = lane; i < n_rows * 64; i += 32) {
       const int j = i >> 6, c = i & 63;
-      f_obj[(env * n_obj + j) * 64 + c] = __float2half_rn(c < obj_dim ? ob[j * obj_dim + c] : 0.f);
+      f_obj[(obj0 + j) * 64 + c] = __float2half_rn(c < obj_dim ? ob[j * obj_dim + c] : 0.f);
     }
     const float* live = ob + n_obj * obj_dim;
-    for (int t = lane; t < T; t += 32) key_bias[env * T + t] = t == 0 ? 0.f : (live[t - 1] - 1.f) * kMaskBias;
+    for (int t = lane; t < T; t += 32) {
+      const float bias = t == 0 ? 0.f : (live[t - 1] - 1.f) * kMaskBias;
+      key_bias[env * T + t] = bias;
+      if (rows.start && t > 0 && t <= n_rows) rows.kb[obj0 + t - 1] = bias;
+    }
   }
 }
 
@@ -235,6 +249,7 @@ struct GCtx {
   void* ws;
   int64_t B;
   bool fused, attn_fused;
+  TokenRows rows;          // packed token rows (start: nullptr: T per environment, the body row first)
   cudaStream_t st;
   const __half* W(const Mat& m, int row0 = 0) const { return at<__half>(arena, m.w) + (int64_t)row0 * m.pitch; }
   const float* Bv(const Mat& m, int row0 = 0) const { return at<float>(arena, m.b) + row0; }
@@ -257,27 +272,39 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
   __half* hid = w.hid >= 0 ? at<__half>(c.ws, w.hid) : nullptr;
   __half* f_body = at<__half>(c.ws, w.f_body);
   __half* f_obj = at<__half>(c.ws, w.f_obj);
-  const RowMap ident = identity_map(), body_rows{1, T, 0}, obj_rows{l.n_obj, T, 1};
+  const TokenRows& rows = c.rows;
+  const bool packed = rows.start != nullptr;
+  const RowMap ident = identity_map(), body_rows = packed ? ident : RowMap{1, T, 0}, obj_rows = packed ? ident : RowMap{l.n_obj, T, 1};
+  auto counted = [&](LinearArgs a) {       // a product over all token rows
+    a.n_rows = rows.n_rows();
+    return a;
+  };
 
+  PdlScope pdl;
   set_stage(kStGather);
   BSRL_TRY(timed_call(st, 0.0, (double)B * (l.obs_dim * 4 + (l.body_k + l.n_obj * l.obj_k) * 2 + T * 4), [&]() -> int {
+    if (packed) {
+      BSRL_TRY(token_rows(RowSource{obs, 0, l.obs_dim, l.body_dim + l.n_obj * l.obj_dim, l.n_obj, 0, kBodyTileEnvs, B}, B, rows, st));
+      begin_overlap(B * l.T);
+    }
     int64_t blocks = (B + 7) / 8;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
     launch_kernel(embed_g_kernel, (unsigned)blocks, 256, 0, st, obs, B, l.obs_dim, l.body_dim, l.body_k, l.n_obj, l.obj_dim, f_body, f_obj,
-                                                     key_bias);
+                                                     key_bias, rows);
     BSRL_LAUNCH_OK("embed_g_kernel");
     return BSRL_OK;
   }));
-  PdlScope pdl;
   begin_overlap(B * l.T);
   set_stage(kStEncoder);
   {
     LinearArgs a = linear_args(f_body, l.body_k, c.W(l.body), l.body.pitch, c.Bv(l.body), x, d, 1, 0, B, d, l.body_k);
     a.cmap = body_rows;
     BSRL_TRY(linear(a, st));
-    LinearArgs o = linear_args(f_obj, l.obj_k, c.W(l.obj), l.obj.pitch, c.Bv(l.obj), x, d, 1, 0, B * l.n_obj, d, l.obj_k);
+    LinearArgs o = linear_args(f_obj, l.obj_k, c.W(l.obj), l.obj.pitch, c.Bv(l.obj), packed ? x + B * d : x, d, 1, 0, B * l.n_obj, d, l.obj_k);
     o.cmap = obj_rows;
+    o.n_rows = rows.n_rows();
+    o.n_less = B;
     BSRL_TRY(linear(o, st));
   }
   auto tail_args = [&](const BlockW& b, int64_t M) {
@@ -292,14 +319,15 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
     a.w2 = c.W(b.down); a.b2 = c.Bv(b.down);
     a.eps = eps;
     a.gelu = 1;
+    a.n_rows = rows.n_rows();
     return a;
   };
   // q|k|v projection + attention of block b for n_q = T (all rows) or 1 (the body row) query rows per env
   auto project_attend = [&](const BlockW& b, int n_q) -> int {
     // the body rows' own projection (B x 3d), then one kernel for the object rows' projection and all the attention
     set_stage(kStQkv);
-    // (the body rows of h are every T-th row: a dense matrix of pitch T d)
-    BSRL_TRY(linear(linear_args(h, T * d, c.W(b.qkv), d, c.Bv(b.qkv), qkv, 3 * d, 0, 0, B, 3 * d, d), st));
+    // (the body rows of h are every T-th row, a dense matrix of pitch T d, or the first)
+    BSRL_TRY(linear(linear_args(h, packed ? d : T * d, c.W(b.qkv), d, c.Bv(b.qkv), qkv, 3 * d, 0, 0, B, 3 * d, d), st));
     AttnBlockArgs a;
     a.d = d; a.n_heads = l.H; a.n_envs = B;
     a.h = h; a.ldh = d;
@@ -307,22 +335,23 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
     a.key_bias = key_bias; a.q_first = 0; a.n_q = n_q;
     a.out = att; a.ldo = d;
     a.body = 1; a.tokens = T; a.qkv0 = qkv;
+    a.rows = rows;
     return fused_attn(a, st);
   };
   auto attend = [&](int n_q) -> int {        // masked attention of n_q query rows per env over its T tokens
     set_stage(kStAttention);
     return timed_call(st, 4.0 * B * n_q * T * d, (double)B * (T * 2 * d + n_q * d * 2) * 2 + (double)B * T * 4,
-                      [&]() -> int { return attention_tokens(qkv, 3 * d, key_bias, B, T, d, l.H, 0, n_q, att, d, st); });
+                      [&]() -> int { return attention_tokens(qkv, 3 * d, key_bias, B, T, d, l.H, 0, n_q, att, d, st, rows.start); });
   };
   bool have_h = false;
   for (int i = 0; i + 1 < l.L; ++i) {
     const BlockW& b = l.blocks[i];
-    if (!have_h) BSRL_TRY(layernorm(x, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h, d, st));
+    if (!have_h) BSRL_TRY(layernorm(x, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h, d, st, rows.n_rows()));
     if (c.attn_fused) {
       BSRL_TRY(project_attend(b, T));
     } else {
       set_stage(kStQkv);
-      BSRL_TRY(linear(linear_args(h, d, c.W(b.qkv), d, c.Bv(b.qkv), qkv, 3 * d, 0, 0, R, 3 * d, d), st));
+      BSRL_TRY(linear(counted(linear_args(h, d, c.W(b.qkv), d, c.Bv(b.qkv), qkv, 3 * d, 0, 0, R, 3 * d, d)), st));
       BSRL_TRY(attend(T));
     }
     if (c.fused) {
@@ -335,13 +364,13 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
       continue;
     }
     {
-      LinearLnArgs po{att, d, c.W(b.out), d, c.Bv(b.out), x, d, x, d, c.G(b.ln_ffn), c.Be(b.ln_ffn), eps, h, d, R, d, d};
+      LinearLnArgs po{att, d, c.W(b.out), d, c.Bv(b.out), x, d, x, d, c.G(b.ln_ffn), c.Be(b.ln_ffn), eps, h, d, R, d, d, rows.n_rows()};
       BSRL_TRY(out_proj_ln(po, st));
     }
     set_stage(kStFfnUp);
-    BSRL_TRY(linear(linear_args(h, d, c.W(b.up), d, c.Bv(b.up), hid, F, 0, 2, R, F, d), st));
+    BSRL_TRY(linear(counted(linear_args(h, d, c.W(b.up), d, c.Bv(b.up), hid, F, 0, 2, R, F, d)), st));
     set_stage(kStFfnDown);
-    LinearArgs pd = linear_args(hid, F, c.W(b.down), F, c.Bv(b.down), x, d, 1, 0, R, d, F);
+    LinearArgs pd = counted(linear_args(hid, F, c.W(b.down), F, c.Bv(b.down), x, d, 1, 0, R, d, F));
     pd.R = x; pd.ldr = d;
     BSRL_TRY(linear(pd, st));
   }
@@ -351,12 +380,12 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
   __half* lead16 = at<__half>(c.ws, w.lead16);
   {
     const BlockW& b = l.blocks[l.L - 1];
-    if (!have_h) BSRL_TRY(layernorm(x, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h, d, st));
+    if (!have_h) BSRL_TRY(layernorm(x, d, ident, c.G(b.ln_attn), c.Be(b.ln_attn), eps, R, d, h, d, st, rows.n_rows()));
     if (c.attn_fused) {
       BSRL_TRY(project_attend(b, 1));
     } else {
       set_stage(kStQkv);
-      BSRL_TRY(linear(linear_args(h, d, c.W(b.qkv, d), d, c.Bv(b.qkv, d), qkv + d, 3 * d, 0, 0, R, 2 * d, d), st));
+      BSRL_TRY(linear(counted(linear_args(h, d, c.W(b.qkv, d), d, c.Bv(b.qkv, d), qkv + d, 3 * d, 0, 0, R, 2 * d, d)), st));
       LinearArgs pq = linear_args(h, d, c.W(b.qkv), d, c.Bv(b.qkv), qkv, 3 * d, 0, 0, B, d, d);
       pq.amap = body_rows; pq.cmap = body_rows;
       BSRL_TRY(linear(pq, st));
@@ -365,6 +394,7 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
     if (c.fused) {
       BlockTailArgs a = tail_args(b, B);
       a.xmap = body_rows;
+      a.n_rows = nullptr;
       a.out16[0] = lead16; a.ld16[0] = d;
       BSRL_TRY(fused_tail(a, st));
     } else {
@@ -414,12 +444,14 @@ int make_gctx(GCtx& c, const bsrl_gconfig* cfg, const void* arena, int64_t n_env
   c.l = make_glayout(*cfg);
   c.fused = g_tail_fused(c.l, process_engine());
   c.attn_fused = g_attn_fused(c.l, process_engine());
-  c.w = make_gws(c.l, n_envs, c.fused, c.attn_fused);
+  const bool packed = g_packed(c.l, process_engine(), n_envs);
+  c.w = make_gws(c.l, n_envs, c.fused, c.attn_fused, packed);
   if (ws_bytes < c.w.bytes) {
     set_error("g_forward: workspace %lld bytes < required %lld", (long long)ws_bytes, (long long)c.w.bytes);
     return BSRL_ERR_WORKSPACE;
   }
   c.arena = arena; c.ws = ws; c.B = n_envs; c.st = as_stream(stream);
+  if (packed) c.rows = carve_rows(at<void>(ws, c.w.rows), n_envs, c.l.n_obj, false);
   return BSRL_OK;
 }
 
@@ -505,7 +537,7 @@ int bsrl_g_pack_weights(const bsrl_gconfig* cfg, const float* const* params, int
 int64_t bsrl_g_workspace_bytes(const bsrl_gconfig* cfg, int64_t n_envs) {
   if (validate_g(cfg) != BSRL_OK || n_envs < 0) return -1;
   const GLayout l = make_glayout(*cfg);
-  return make_gws(l, n_envs, g_tail_fused(l, process_engine()), g_attn_fused(l, process_engine())).bytes;
+  return make_gws(l, n_envs, g_tail_fused(l, process_engine()), g_attn_fused(l, process_engine()), g_packed(l, process_engine(), n_envs)).bytes;
 }
 
 int bsrl_g_forward(const bsrl_gconfig* cfg, const void* arena, const float* obs, int64_t n_envs, const void* actions,

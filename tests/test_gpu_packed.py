@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from helpers import make_cfg, cuda_policy
+from oracle import body_policy_oracle as bo
 from oracle import policy_oracle as po
 
 pytestmark = pytest.mark.gpu
@@ -121,3 +122,26 @@ def test_gradients_equal_the_sum_over_slices(name, opts, kind):
     top = max(float(g.norm()) for g in whole.values())
     for k, g in whole.items():
         assert float((m.get_parameter(k).grad - g).norm()) <= 1e-4 * float(g.norm()) + 1e-6 * top, k
+
+
+@pytest.mark.parametrize("kind", ["none", "all", "holes", "last", "runs"])
+@pytest.mark.parametrize("name,heads", [("cfg1", 4), ("cfg2", 8), ("cfg4", 8), ("cfg2", 4), ("cfg1", 2)])
+def test_body_token_layout(native, name, heads, kind):
+    cfg = bo.named_config(name)
+    cfg.n_blocks, cfg.n_heads = 2, heads
+    from test_gpu_body_policy import cuda_body_policy
+    m = cuda_body_policy(cfg, bo.build_state_dict(cfg, 7))
+    envs = 1503 if kind != "runs" else 2600
+    obs = bo.make_obs(envs, cfg, 45)
+    obs[:, -cfg.n_obj:] = _masks(kind, envs, cfg.n_obj, torch.Generator().manual_seed(46))
+    obs = obs.cuda()
+    logits, value = m.forward_stacked(obs)
+    part = 18944 // (1 + cfg.n_obj)
+    for lo in range(0, envs, part):
+        l, v = m.forward_stacked(obs[lo:lo + part])
+        assert torch.equal(l, logits[lo:lo + part]) and torch.equal(v, value[lo:lo + part]), lo
+    obs[::5, 3] = float("nan")
+    l2, v2 = m.forward_stacked(obs)
+    good = torch.arange(envs, device="cuda") % 5 != 0
+    assert torch.equal(l2[good], logits[good]) and torch.equal(v2[good], value[good])
+    assert native.lib.bsrl_device_status() == 0
