@@ -111,8 +111,11 @@ struct TailParams {
   int x_tma;                // residual rows are read with TMA (identity row map)
   int* status;
   const int* n_rows;        // packed token rows: the device's row count (at most M) ...
-  const int* x_start;       // ... and the first rows of xmap's groups, or nullptr
-  __device__ __forceinline__ int64_t x_row(int64_t r) const { return x_start ? (int64_t)x_start[r / xmap.group] + xmap.first + r % xmap.group : xmap.plain(r); }
+  const int* x_start;       // ... and the first rows of xmap's groups; either may be nullptr
+  template <bool PACK>
+  __device__ __forceinline__ int64_t x_row(int64_t r) const {
+    return PACK && x_start ? (int64_t)x_start[r / xmap.group] + xmap.first + r % xmap.group : xmap.plain(r);
+  }
 };
 
 __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
@@ -177,8 +180,9 @@ using StageNo = std::integral_constant<int, N>;
 
 // GELU: the FFN activation is the exact GELU instead of ReLU (a compile-time variant: the hidden-chunk
 // epilogue sits on the chunk loop's critical path)
-// PACK: the number of tiles follows from the device's row count; rows past it are read (they are in the buffers) and their results
-// land past the counted rows
+// PACK: the number of tiles follows from the device's row count, where there is one; rows past it are read (they are in the buffers)
+// and their results land past the counted rows.  The other kernels have nothing of it: one tile of theirs is 6 % longer with the table
+// of first rows beside the plain map (GELU, d 128: 28.3 -> 30.0 us).
 template <bool GELU, bool PAIR, bool PACK>
 __global__ void __launch_bounds__(THREADS, 1)
 block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_constant__ CUtensorMap tm_wo,
@@ -231,7 +235,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
     sh->abort = 0;
     // packed token rows: counted at least two launches back; both CTAs of a pair take the same number of tiles.  (Kept in a
     // register, the count costs 3 % of the kernel.)
-    if (PACK) sh->n_tiles = (p.n_rows[0] + CTAS * BM - 1) / (CTAS * BM) * CTAS;
+    if (PACK) sh->n_tiles = p.n_rows ? (p.n_rows[0] + CTAS * BM - 1) / (CTAS * BM) * CTAS : p.n_tiles;
     fence_barrier_init();
     tma_prefetch_desc(&tm_att);
     tma_prefetch_desc(&tm_wo);
@@ -343,7 +347,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
         for (int r = lane; r < BM; r += 32) {
           const int64_t row = (int64_t)tn * BM + r;
           if (row < p.M) {
-            const float* xr = p.x + p.x_row(row) * p.ldx;
+            const float* xr = p.x + p.x_row<PACK>(row) * p.ldx;
             for (int c = 0; c < d; c += 32) prefetch_l2(xr + c);
           }
         }
@@ -679,7 +683,7 @@ block_tail_kernel(const __grid_constant__ CUtensorMap tm_att, const __grid_const
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int64_t row = (int64_t)t * BM + q * 32 + i * 8 + sub8;
-        src[i] = row < p.M ? p.x + p.x_row(row) * p.ldx + piece * 4 : nullptr;
+        src[i] = row < p.M ? p.x + p.x_row<PACK>(row) * p.ldx + piece * 4 : nullptr;
       }
       uint4 nxt[4];
 #pragma unroll
@@ -1045,7 +1049,7 @@ int block_tail(const BlockTailArgs& a, cudaStream_t stream) {
   p.wide16 = wide16 ? 1 : 0;
   p.x_tma = x_tma ? 1 : 0;
   p.status = status;
-  const bool pack = a.n_rows != nullptr;
+  const bool pack = a.n_rows || a.xmap.start;
   if (pair) {
     auto* kernel = pack ? (a.gelu ? block_tail_kernel<true, true, true> : block_tail_kernel<false, true, true>)
                         : (a.gelu ? block_tail_kernel<true, true, false> : block_tail_kernel<false, true, false>);

@@ -16,6 +16,8 @@
 // Stands in for the reference's cuBLAS / cuBLASLt calls on the fp16 stream (torch.addmm and the
 // RELU_BIAS epilogue, python/fp16_linear.py:134-181; linear_relu_aux,
 // python/beat_arena_env/csrc/fp16_gemm.cu:402-497).
+#include <type_traits>
+
 #include "kernels.cuh"
 #include "tc5.cuh"
 
@@ -65,7 +67,9 @@ __device__ __forceinline__ WorkItem work_item(int64_t w, int n_tile_work, int n_
 // SUMS: column sums of A beside the product (LinearArgs::a_sums), compiled in only where asked for: the untaken branch
 // alone cost the MMA thread 0.1 us per k-block.
 // GELU32: GELU of an fp32 result (gelu_f32), a kernel of its own: compiled into the others it cost updates 1 % by its size alone
-template <bool HAS_R, bool SUMS, bool GELU32 = false>
+// COUNT: packed token rows -- a row count of the device's, or maps with a table of first rows.  Kernels of their own: a launch on one
+// 128-row tile is as long as its serial phases, and the count's branches made it 13 % longer (15.9 -> 18.0 us at 910 rows, N = K = 512).
+template <bool HAS_R, bool SUMS, bool GELU32 = false, bool COUNT = false>
 __global__ void __launch_bounds__(THREADS, 1)
 linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                   const __grid_constant__ CUtensorMap tm_c, int tma_c, LinearArgs p, int m_bound, int n_tiles,
@@ -76,14 +80,16 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   uint8_t* staging = smem_raw + (tiles_base - raw) + STAGES * STAGE_BYTES;
   Shared* sh = reinterpret_cast<Shared*>(staging + EPI_WARPS * STG_BYTES);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t M = p.a_mn ? p.M : p.live(p.M);
-  const int K = p.a_mn ? (int)p.live(p.K) : p.K;
-  const int m_tiles = p.n_rows && !p.a_mn ? (int)((M + BM - 1) / BM) : m_bound;
+  const int64_t M = COUNT && !p.a_mn ? p.live(p.M) : p.M;
+  const int K = COUNT && p.a_mn ? (int)p.live(p.K) : p.K;
+  const int m_tiles = COUNT && p.n_rows && !p.a_mn ? (int)((M + BM - 1) / BM) : m_bound;
   const int k_blocks = (K + BK - 1) / BK;
-  const int kps = max((k_blocks + max(p.k_splits, 1) - 1) / max(p.k_splits, 1), 1);  // k-blocks per split
-  const int splits = p.n_rows && p.a_mn ? (k_blocks + kps - 1) / kps : max(p.k_splits, 1);      // none of them empty (no rows: no work)
+  const int max_splits = p.k_splits > 1 ? p.k_splits : 1;
+  const int kps = COUNT ? max((k_blocks + max_splits - 1) / max_splits, 1) : (k_blocks + max_splits - 1) / max_splits;  // k-blocks per split
+  const int splits = COUNT && p.n_rows && p.a_mn ? (k_blocks + kps - 1) / kps : max_splits;     // none of them empty (no rows: no work)
   // Rows past the device's count in the contraction's last k-block are anything: an epilogue warp, idle by then, clears them
-  const int tail = p.n_rows && p.a_mn ? K % BK : 0;
+  const int tail = COUNT && p.n_rows && p.a_mn ? K % BK : 0;
+  auto at_row = [](const RowMap& map, int64_t row) { return COUNT ? map(row) : static_cast<const PlainMap&>(map)(row); };
   const int64_t n_tile_work = (int64_t)m_tiles * n_tiles;
   const int64_t n_work = n_tile_work * splits;                // work item = (split, tile): split-major
   volatile int* abort = &sh->abort;
@@ -98,8 +104,10 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       mbar_init(smem_u32(&sh->tmem_empty[b]), EPI_WARPS);
     }
     mbar_init(smem_u32(&sh->mma_done), 1);
-    mbar_init(smem_u32(&sh->tail_there), 1);
-    mbar_init(smem_u32(&sh->tail_clear), 1);
+    if (COUNT) {
+      mbar_init(smem_u32(&sh->tail_there), 1);
+      mbar_init(smem_u32(&sh->tail_clear), 1);
+    }
     sh->abort = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tm_a);
@@ -181,7 +189,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!mbar_wait(smem_u32(&sh->full[s]), ph, abort)) { give_up(sh, status, 4); ok = false; break; }
-          if (tail && kb == k_blocks - 1) {
+          if (COUNT && tail && kb == k_blocks - 1) {
             mbar_arrive(smem_u32(&sh->tail_there));
             if (!mbar_wait(smem_u32(&sh->tail_clear), tails++ & 1, abort)) { give_up(sh, status, 4); ok = false; break; }
           }
@@ -224,7 +232,7 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
     bool ok = true;
     for (int64_t w = blockIdx.x; w < n_work && ok; w += gridDim.x, ++tile_i) {
       const WorkItem wi = work_item(w, (int)n_tile_work, n_tiles);
-      if (tail && warp == 2) {
+      if (COUNT && tail && warp == 2) {
         const int kb0 = wi.split * kps, kb1 = min(k_blocks, kb0 + kps);
         it += kb1 - kb0;
         if (kb1 == k_blocks) {
@@ -252,8 +260,8 @@ linear_tc5_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const int64_t row = m0 + q * 32 + i * 4 + sub;
-        crow[i] = row < M ? p.cmap(row) * (int64_t)p.ldc : -1;
-        rrow[i] = (HAS_R && row < M) ? p.rmap(row) * (int64_t)p.ldr : 0;
+        crow[i] = row < M ? at_row(p.cmap, row) * (int64_t)p.ldc : -1;
+        rrow[i] = (HAS_R && row < M) ? at_row(p.rmap, row) * (int64_t)p.ldr : 0;
       }
       if (!mbar_wait_warp(smem_u32(&sh->tmem_full[buf]), acc_ph, abort)) {
         if (lane == 0) give_up(sh, status, 5);
@@ -581,7 +589,9 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
   int rc = once.run("linear_tc5_kernel set-up", [] {
     cudaError_t e = cudaSuccess;
     for (auto* k : {linear_tc5_kernel<false, false>, linear_tc5_kernel<true, false>, linear_tc5_kernel<false, true>,
-                    linear_tc5_kernel<false, false, true>, linear_tc5_kernel<true, false, true>})
+                    linear_tc5_kernel<false, false, true>, linear_tc5_kernel<true, false, true>,
+                    linear_tc5_kernel<false, false, false, true>, linear_tc5_kernel<true, false, false, true>, linear_tc5_kernel<false, true, false, true>,
+                    linear_tc5_kernel<false, false, true, true>, linear_tc5_kernel<true, false, true, true>})
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     return e;
   });
@@ -595,8 +605,14 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
   int64_t grid = m_tiles * n_tiles * (p.k_splits > 1 ? p.k_splits : 1);
   if (grid > sm_count()) grid = sm_count();
   const bool gelu32 = p.relu == 2 && p.out_f32;
-  auto* kernel = p.a_sums ? linear_tc5_kernel<false, true> : gelu32 ? (p.R ? linear_tc5_kernel<true, false, true> : linear_tc5_kernel<false, false, true>)
-                                                           : p.R ? linear_tc5_kernel<true, false> : linear_tc5_kernel<false, false>;
+  auto pick = [&](auto count) {
+    constexpr bool COUNT = decltype(count)::value;
+    return p.a_sums ? linear_tc5_kernel<false, true, false, COUNT>
+           : gelu32 ? (p.R ? linear_tc5_kernel<true, false, true, COUNT> : linear_tc5_kernel<false, false, true, COUNT>)
+           : p.R    ? linear_tc5_kernel<true, false, false, COUNT>
+                    : linear_tc5_kernel<false, false, false, COUNT>;
+  };
+  auto* kernel = p.n_rows || p.cmap.start || p.rmap.start ? pick(std::true_type()) : pick(std::false_type());
   launch_kernel(kernel, (unsigned)grid, THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, tma_c ? 1 : 0, p, (int)m_tiles, n_tiles, status);
   BSRL_LAUNCH_OK("linear_tc5_kernel");
   return BSRL_OK;

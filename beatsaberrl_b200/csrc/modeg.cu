@@ -215,6 +215,7 @@ bool g_tail_fused(const GLayout& l, int engine) {
 
 // One warp per env: body lanes -> K-padded fp16 row, each object's lanes -> its 64-wide row, key bias
 // (token 0 always attendable, object j by its live flag: 0 or -16384, python/policy.py:422-428)
+template <bool PACK>
 __global__ void __launch_bounds__(256) embed_g_kernel(const float* __restrict__ obs, int64_t n_envs, int obs_dim, int body_dim,
                                                       int body_k, int n_obj, int obj_dim, __half* __restrict__ f_body,
                                                       __half* __restrict__ f_obj, float* __restrict__ key_bias, TokenRows rows) {
@@ -226,8 +227,8 @@ __global__ void __launch_bounds__(256) embed_g_kernel(const float* __restrict__ 
     const float* o = obs + env * obs_dim;
     for (int c = lane; c < body_k; c += 32) f_body[env * body_k + c] = __float2half_rn(c < body_dim ? o[c] : 0.f);
     const float* ob = o + body_dim;
-    const int64_t obj0 = rows.start ? rows.start[env] : env * n_obj;
-    const int n_rows = rows.start ? (int)(rows.start[env + 1] - obj0) : n_obj;
+    const int64_t obj0 = PACK ? rows.start[env] : env * n_obj;
+    const int n_rows = PACK ? (int)(rows.start[env + 1] - obj0) : n_obj;
     for (int i = lane; i < n_rows * 64; i += 32) {
       const int j = i >> 6, c = i & 63;
       f_obj[(obj0 + j) * 64 + c] = __float2half_rn(c < obj_dim ? ob[j * obj_dim + c] : 0.f);
@@ -236,7 +237,7 @@ __global__ void __launch_bounds__(256) embed_g_kernel(const float* __restrict__ 
     for (int t = lane; t < T; t += 32) {
       const float bias = t == 0 ? 0.f : (live[t - 1] - 1.f) * kMaskBias;
       key_bias[env * T + t] = bias;
-      if (rows.start && t > 0 && t <= n_rows) rows.kb[obj0 + t - 1] = bias;
+      if (PACK && t > 0 && t <= n_rows) rows.kb[obj0 + t - 1] = bias;
     }
   }
 }
@@ -290,7 +291,7 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
     int64_t blocks = (B + 7) / 8;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    launch_kernel(embed_g_kernel, (unsigned)blocks, 256, 0, st, obs, B, l.obs_dim, l.body_dim, l.body_k, l.n_obj, l.obj_dim, f_body, f_obj,
+    launch_kernel(packed ? embed_g_kernel<true> : embed_g_kernel<false>, (unsigned)blocks, 256, 0, st, obs, B, l.obs_dim, l.body_dim, l.body_k, l.n_obj, l.obj_dim, f_body, f_obj,
                                                      key_bias, rows);
     BSRL_LAUNCH_OK("embed_g_kernel");
     return BSRL_OK;
