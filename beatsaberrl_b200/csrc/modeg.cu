@@ -213,28 +213,41 @@ bool g_tail_fused(const GLayout& l, int engine) {
   return engine == 0 && l.d % 64 == 0 && l.d <= 256 && l.F % 256 == 0 && l.F >= 256 && l.F <= 1024;
 }
 
-// One warp per env: body lanes -> K-padded fp16 row, each object's lanes -> its 64-wide row, key bias
-// (token 0 always attendable, object j by its live flag: 0 or -16384, python/policy.py:422-428)
+// Per env: body lanes -> K-padded fp16 row, each object's lanes -> its 64-wide row, key bias
+// (token 0 always attendable, object j by its live flag: 0 or -16384, python/policy.py:422-428).
+// `parts` warps (a power of two) share an environment: one where the batch fills the chip, which is bound by the bytes then, and up to
+// 16 below, where the time is a warp's chain of loads and stores.
 template <bool PACK>
 __global__ void __launch_bounds__(256) embed_g_kernel(const float* __restrict__ obs, int64_t n_envs, int obs_dim, int body_dim,
                                                       int body_k, int n_obj, int obj_dim, __half* __restrict__ f_body,
-                                                      __half* __restrict__ f_obj, float* __restrict__ key_bias, TokenRows rows) {
+                                                      __half* __restrict__ f_obj, float* __restrict__ key_bias, TokenRows rows, int parts) {
   pdl_begin();
-  const int lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31, shift = __ffs(parts) - 1;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-  const int T = 1 + n_obj;
-  for (int64_t env = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); env < n_envs; env += warps) {
+  const int T = 1 + n_obj, step = 32 * parts;
+  for (int64_t w = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); w < n_envs << shift; w += warps) {
+    const int64_t env = w >> shift;
+    const int at = (int)(w & (parts - 1)) * 32 + lane;
     const float* o = obs + env * obs_dim;
-    for (int c = lane; c < body_k; c += 32) f_body[env * body_k + c] = __float2half_rn(c < body_dim ? o[c] : 0.f);
     const float* ob = o + body_dim;
+    const float* live = ob + n_obj * obj_dim;
+    __half* fb = f_body + env * body_k;
+#pragma unroll 4
+    for (int c = 2 * at; c < body_k; c += 2 * step)
+      *reinterpret_cast<uint32_t*>(fb + c) = pack_half2(c < body_dim ? o[c] : 0.f, c + 1 < body_dim ? o[c + 1] : 0.f);
     const int64_t obj0 = PACK ? rows.start[env] : env * n_obj;
     const int n_rows = PACK ? (int)(rows.start[env + 1] - obj0) : n_obj;
-    for (int i = lane; i < n_rows * 64; i += 32) {
-      const int j = i >> 6, c = i & 63;
-      f_obj[(obj0 + j) * 64 + c] = __float2half_rn(c < obj_dim ? ob[j * obj_dim + c] : 0.f);
+    uint2* fo = reinterpret_cast<uint2*>(f_obj + obj0 * 64);
+#pragma unroll 4
+    for (int i = at; i < n_rows * 16; i += step) {
+      const int c = (i & 15) * 4;
+      const float* from = ob + (i >> 4) * obj_dim + c;
+      float f[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) f[e] = c + e < obj_dim ? from[e] : 0.f;
+      fo[i] = make_uint2(pack_half2(f[0], f[1]), pack_half2(f[2], f[3]));
     }
-    const float* live = ob + n_obj * obj_dim;
-    for (int t = lane; t < T; t += 32) {
+    for (int t = at; t < T; t += step) {
       const float bias = t == 0 ? 0.f : (live[t - 1] - 1.f) * kMaskBias;
       key_bias[env * T + t] = bias;
       if (PACK && t > 0 && t <= n_rows) rows.kb[obj0 + t - 1] = bias;
@@ -288,11 +301,13 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
       BSRL_TRY(token_rows(RowSource{obs, 0, l.obs_dim, l.body_dim + l.n_obj * l.obj_dim, l.n_obj, 0, kBodyTileEnvs, B}, B, rows, st));
       begin_overlap(B * l.T);
     }
-    int64_t blocks = (B + 7) / 8;
+    int parts = 1;
+    while (parts < 16 && B * parts < (int64_t)sm_count() * 16) parts *= 2;
+    int64_t blocks = (B * parts + 7) / 8;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    launch_kernel(packed ? embed_g_kernel<true> : embed_g_kernel<false>, (unsigned)blocks, 256, 0, st, obs, B, l.obs_dim, l.body_dim, l.body_k, l.n_obj, l.obj_dim, f_body, f_obj,
-                                                     key_bias, rows);
+    launch_kernel(packed ? embed_g_kernel<true> : embed_g_kernel<false>, (unsigned)blocks, 256, 0, st, obs, B, l.obs_dim, l.body_dim, l.body_k, l.n_obj, l.obj_dim, f_body,
+                  f_obj, key_bias, rows, parts);
     BSRL_LAUNCH_OK("embed_g_kernel");
     return BSRL_OK;
   }));

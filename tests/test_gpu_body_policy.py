@@ -151,3 +151,18 @@ def test_many_envs_match_slices(name, B, part):
     for lo in range(0, B, part):
         l, v = m.forward_stacked(obs[lo:lo + part])
         assert torch.equal(l, logits[lo:lo + part]) and torch.equal(v, value[lo:lo + part])
+
+
+@pytest.mark.parametrize("body_dim,obj_dim,n_obj", [(1, 1, 16), (341, 13, 32), (64, 64, 64)])
+def test_widths_whatever_the_number_of_warps_per_env(body_dim, obj_dim, n_obj):
+    cfg = bo.named_config("cfg1")
+    cfg.body_dim, cfg.obj_dim, cfg.n_obj = body_dim, obj_dim, n_obj
+    sd = bo.build_state_dict(cfg, 5)
+    m = cuda_body_policy(cfg, sd)
+    obs = bo.make_obs(2500, cfg, 6, padded=True)
+    logits, value = m.forward_stacked(obs.cuda())
+    for B in (1, 296, 592, 1184):            # 16, 8, 4 and 2 warps per environment; the whole batch has one
+        l, v = m.forward_stacked(obs[:B].cuda())
+        assert torch.equal(l, logits[:B]) and torch.equal(v, value[:B]), B
+    ref_l, ref_v = bo.forward(sd, cfg, obs[:600])
+    assert_parity(logits[:600], value[:600], ref_l, ref_v, argmax_min=0.995)
