@@ -32,6 +32,8 @@
 // With all 29 query rows, an env's output for the group (29 rows x 128 bytes for two heads of 32, x 96 bytes
 // for one head of 48) is staged in shared memory (64-wide groups: in place of its q rows) and leaves as one TMA
 // store per env.  All waits are bounded (tc5.cuh).
+#include <type_traits>
+
 #include "kernels.cuh"
 #include "attend.cuh"
 #include "tc5.cuh"
@@ -107,10 +109,17 @@ struct Params {
   int tokens, tok0, body_only;
   const __half* qkv0;
   int* status;
-  TokenRows rows;          // packed token rows (PACK kernels)
-  int64_t rows_ahead;      // rows of out ahead of theirs (body-token layout: the body rows)
-  int full_rows;           // not 0: the number of rows that has all slots live, where the kernel of the full layout does the work
+  const int* counted;      // not nullptr: the packed layout's number of rows; where all slots are live, the full layout's kernel does the work
 };
+// Apart, for the plain kernels' launches wait for their parameters
+struct PackParams : Params {
+  TokenRows rows;          // packed token rows
+  int64_t rows_ahead;      // rows of out ahead of theirs (body-token layout: the body rows)
+};
+__device__ __forceinline__ TokenRows rows_in(const Params&) { return TokenRows(); }
+__device__ __forceinline__ const TokenRows& rows_in(const PackParams& p) { return p.rows; }
+__device__ __forceinline__ int64_t ahead_in(const Params&) { return 0; }
+__device__ __forceinline__ int64_t ahead_in(const PackParams& p) { return p.rows_ahead; }
 
 __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
   atomicCAS(status, 0, KERNEL_ID * 16 + role);
@@ -120,19 +129,22 @@ __device__ __forceinline__ void give_up(Shared* sh, int* status, int role) {
 // VRES: the value-residual code of the drain is compiled in (it costs ~14 % of the kernel even when idle)
 // BODY: the single-body-token layout (Params::tokens and below); DH = 32, G = 2 only
 // PACK: packed token rows (rows.cu).  A tile is as many whole environments as fit 128 rows, from any row on; a set's eight
-// warps drain it, then take its (environment, head) pairs in turn, of 16 or 32 rows and keys as the environment has.
+// warps drain it, then take its (environment, head) pairs in turn, of 16 or 32 rows and keys as the environment has.  Bound by the
+// softmax of those pairs, of which there are as many as before: 65,536 environments at d 256, 17 of 29 rows left, 722 us against 940;
+// 32,768 at d 512, 1,104 against 1,420 (both cold, under the profiler).
 template <int DH, int G, bool PAIR, bool VRES, bool BODY = false, bool PACK = false>
 __global__ void __launch_bounds__((Shape<DH, G, PAIR, PACK>::THREADS), 1)
 attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constant__ CUtensorMap tm_w,
-                  const __grid_constant__ CUtensorMap tm_o, Params p) {
+                  const __grid_constant__ CUtensorMap tm_o, std::conditional_t<PACK, PackParams, Params> p) {
   using S = Shape<DH, G, PAIR, PACK>;
   constexpr int STAGES = S::STAGES, GD = S::GD, NG = S::NG, STAGE_BYTES = S::STAGE_BYTES, LDQ = S::LDQ, SQ_BYTES = S::SQ_BYTES;
   constexpr int THREADS = S::THREADS, SECTION = S::SECTION;
   // which of the two launches the rows are for (counted at least two launches back)
-  if (!BODY && p.full_rows && (p.rows.n_tiles[1] == p.full_rows) == PACK) {
+  if (!BODY && p.counted && (p.counted[0] == p.n_envs * kT) == PACK) {
     pdl_wait();
     return;
   }
+  const auto& packed = rows_in(p);
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -158,7 +170,7 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
   volatile int* abort = &sh->abort;
   const uint32_t rank = PAIR ? cluster_rank() : 0u;
   // work item: (tile, share of its head groups); both CTAs of a pair take the same number of tiles
-  const int n_tiles = PACK ? p.rows.n_tiles[0] : p.n_tiles;      // (PACK: counted at least two launches back)
+  const int n_tiles = PACK ? packed.n_tiles[0] : p.n_tiles;      // (PACK: counted at least two launches back)
   const int t_end = PAIR ? (n_tiles + 1) & ~1 : PACK ? n_tiles : n_tiles * p.split;
   const int per_item = PAIR ? n_groups : (n_groups + p.split - 1) / p.split, log_split = PAIR ? 0 : __ffs(p.split) - 1;
   auto tile_of = [&](int i) { return i >> log_split; };
@@ -235,7 +247,7 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
       };
       if (STREAM) pdl_wait();
       for (int i = blockIdx.x; i < t_end && ok; i += gridDim.x, ++tile_i) {
-        const int t = PACK ? p.rows.tiles[i].y : tile_of(i), g_lo = first_group(i), g_hi = min(g_lo + per_item, n_groups);
+        const int t = PACK ? packed.tiles[i].y : tile_of(i), g_lo = first_group(i), g_hi = min(g_lo + per_item, n_groups);
         if (STREAM) {
           for (int g = g_lo; g < g_hi && ok; ++g)
             for (int kb = 0; kb < KB && ok; ++kb) ok = w_stage(g, kb, t);
@@ -327,13 +339,13 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
       const int t = tile_of(i), g_lo = first_group(i), g_hi = min(g_lo + per_item, n_groups);
       const int64_t env = (int64_t)t * EPT + env_l;
       // PACK: the tile's environments and rows; this thread's share of their places and key bias, fetched long before use
-      const int2 tile_lo = PACK && t < n_tiles ? p.rows.tiles[t] : make_int2(0, 0), tile_hi = PACK && t < n_tiles ? p.rows.tiles[t + 1] : make_int2(0, 0);
+      const int2 tile_lo = PACK && t < n_tiles ? packed.tiles[t] : make_int2(0, 0), tile_hi = PACK && t < n_tiles ? packed.tiles[t + 1] : make_int2(0, 0);
       const int n_tile_envs = tile_hi.x - tile_lo.x, used = tile_hi.y - tile_lo.y;
       const int64_t row0 = tile_lo.y;
       int sP_value = 0;
       if (PACK) {
-        if (set_thread < BM) sP_value = set_thread < used ? __float_as_int(p.rows.kb[row0 + set_thread]) : 0;
-        else if (set_thread - BM <= n_tile_envs) sP_value = p.rows.start[tile_lo.x + set_thread - BM] - tile_lo.y;
+        if (set_thread < BM) sP_value = set_thread < used ? __float_as_int(packed.kb[row0 + set_thread]) : 0;
+        else if (set_thread - BM <= n_tile_envs) sP_value = packed.start[tile_lo.x + set_thread - BM] - tile_lo.y;
       }
       // this lane's key-bias values (keys nt * 8 + tig * 2 + e of the m16n8 accumulator layout, times
       // log2 e; -inf past the 29th key), fetched once per tile and long before the first softmax
@@ -620,7 +632,7 @@ attn_block_kernel(const __grid_constant__ CUtensorMap tm_h, const __grid_constan
             constexpr int PIECES = GD / 8;
             for (int k = lane; k < (used - q * 32) * PIECES; k += 32) {
               const int row = q * 32 + k / PIECES, piece = k % PIECES;
-              *reinterpret_cast<uint4*>(p.out + (p.rows_ahead + row0 + row) * (int64_t)p.ldo + g * GD + piece * 8) =
+              *reinterpret_cast<uint4*>(p.out + (ahead_in(p) + row0 + row) * (int64_t)p.ldo + g * GD + piece * 8) =
                   *reinterpret_cast<const uint4*>(sO_g + row * (GD * 2) + (GD == 64 ? (piece ^ (row & 7)) << 4 : piece << 4));
             }
             __syncwarp();
@@ -654,7 +666,8 @@ cudaError_t prepare() {
   return e;
 }
 template <int DH, int G, bool VRES, bool BODY, bool PACK = false>
-void launch(bool pair, const CUtensorMap& tm_h, const CUtensorMap& tm_w, const CUtensorMap& tm_o, const Params& p, cudaStream_t stream) {
+void launch(bool pair, const CUtensorMap& tm_h, const CUtensorMap& tm_w, const CUtensorMap& tm_o, const PackParams& all, cudaStream_t stream) {
+  const std::conditional_t<PACK, PackParams, Params>& p = all;
   if constexpr (DH != 48)
     if (pair) {
       using S = Shape<DH, G, true, PACK>;
@@ -742,7 +755,7 @@ int attn_block(const AttnBlockArgs& a, cudaStream_t stream) {
     return e;
   });
   if (rc != BSRL_OK) return rc;
-  Params p;
+  PackParams p;
   p.d = a.d; p.n_heads = a.n_heads;
   p.q_first = a.body ? 0 : a.q_first;
   p.n_q = a.body ? EROWS : a.n_q;                 // body-token layout: the tile's query rows are the 32 object tokens
@@ -760,11 +773,10 @@ int attn_block(const AttnBlockArgs& a, cudaStream_t stream) {
   p.tokens = T; p.tok0 = a.body ? 1 : 0; p.body_only = (a.body && a.n_q == 1) ? 1 : 0; p.qkv0 = a.qkv0;
   p.rows = a.rows;
   p.rows_ahead = ahead;
-  p.full_rows = 0;
+  p.counted = full ? a.rows.n_rows() : nullptr;
   p.status = status;
   const bool vres = a.v_out || a.v0;
   if (!pack || full) {
-    p.full_rows = full ? (int)(a.n_envs * T) : 0;
     if (!maps(false)) return BSRL_ERR_CUDA;
     auto* run = a.body ? launch<32, 2, false, true> : dh == 32 ? (vres ? launch<32, 2, true, false> : launch<32, 2, false, false>)
               : dh == 48 ? (vres ? launch<48, 1, true, false> : launch<48, 1, false, false>)

@@ -42,6 +42,8 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
 // bytes per lane.  Bound by the turns of the shared-memory pipe (654 of the 909 cycles per pair of 29 queries x 32 before
 // the swizzled rows; every fragment is fetched once now, for both query or both key tiles).  16,384 environments of 8 heads of
 // 32, us, before / now (at copy speed): 29 queries 407 / 350 (260), 5 queries 276 / 226 (199), 1 query 272 / 224 (152).
+// Packed token rows (start: an environment's first row; up to 16 of them are one tile of queries and keys): 29 queries 363 / 282
+// with 17 of 29 rows left, 1 query 233 / 223.
 template <int DH, int MT>
 __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(const __half* __restrict__ qkv, int ld, const float* __restrict__ key_bias,
                                                                int64_t n_pairs, int d, int n_heads, int q_first, int n_queries,
