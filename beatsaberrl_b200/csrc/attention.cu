@@ -26,7 +26,7 @@ namespace {
 // Packed token rows with 17 of 29 left: the five launches of an update 157 / 129 on average.
 // KG: groups of 32 keys (tokens padded to 32 KG rows: two 16-row MMA tiles / four 8-key tiles per group);
 // WARPS: warps per block, fewer where the per-warp tile is large
-template <int DH, int KG, int WARPS>
+template <int DH, int KG, int WARPS, bool PACK>
 __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __restrict__ qkv, int ld,
                                                            const float* __restrict__ key_bias,
                                                            int64_t n_pairs, int tokens, int d, int n_heads,
@@ -43,19 +43,29 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
   const int tig = lane & 3;
   const int ra = lane & 15, ca = lane >> 4, rb = (lane & 7) + ((lane >> 4) << 3), cb = (lane >> 3) & 1;   // ldmatrix rows and halves
 
-  for (int64_t pair = (int64_t)blockIdx.x * kWarps + warp; pair < n_pairs;
-       pair += (int64_t)gridDim.x * kWarps) {
+  const int64_t warps = (int64_t)gridDim.x * kWarps;
+  // packed token rows: a pair's part of `start`, loaded one pair ahead
+  auto part_of = [&](int64_t pair) {
+    if (!PACK || pair >= n_pairs) return make_int2(0, 0);
     int head;
     const int64_t env = div_index(pair, n_heads, &head);
-    // packed token rows: the environment's own, and as many queries where all are asked for
-    const int64_t row0 = start ? start[env] : env * tokens;
-    const int T = start ? (int)(start[env + 1] - row0) : tokens;
-    const bool all = start && n_queries == tokens;
+    return make_int2(start[env], start[env + 1]);
+  };
+  int2 from, next = part_of((int64_t)blockIdx.x * kWarps + warp);
+  for (int64_t pair = (int64_t)blockIdx.x * kWarps + warp; pair < n_pairs; pair += warps) {
+    int head;
+    const int64_t env = div_index(pair, n_heads, &head);
+    from = next;
+    next = part_of(pair + warps);
+    // the environment's own rows, and as many queries where all are asked for
+    const int64_t row0 = PACK ? from.x : env * tokens;
+    const int T = PACK ? from.y - from.x : tokens;
+    const bool all = PACK && n_queries == tokens;
     const int n_q = all ? T : n_queries, m_tiles = (n_q + 15) >> 4;
     const __half* base = qkv + row0 * ld + head * DH;
     __syncwarp();
     // stage q (query rows), k, v; rows past the live range are zero
-    for (int c = lane; c < (T <= 16 ? 16 : kRows) * CH; c += 32) {
+    for (int c = lane; c < (PACK && T <= 16 ? 16 : kRows) * CH; c += 32) {
       const int row = c / CH, ch = c % CH;
       const bool live = row < T, asks = row < n_q;
       const __half* r = base + (int64_t)(live ? row : 0) * ld + ch * 8;
@@ -157,7 +167,7 @@ __global__ void __launch_bounds__(WARPS * 32) attn29_kernel(const __half* __rest
                            pack_half2(o[2 * j + 1][0], o[2 * j + 1][1]), pack_half2(o[2 * j + 1][2], o[2 * j + 1][3]));
       }
     };
-    if (T <= 16) attend(std::integral_constant<int, 1>());
+    if (PACK && T <= 16) attend(std::integral_constant<int, 1>());
     else attend(std::integral_constant<int, 2 * KG>());
     __syncwarp();
     __half* to = out + (all ? row0 : env * n_q) * ldo + head * DH;
@@ -484,15 +494,23 @@ int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int
   constexpr int kWarps = KG == 1 ? 8 : 4;
   constexpr int smem = kWarps * 3 * (32 * KG) * DH * 2;
   static DeviceOnce once;
+  constexpr bool kPacks = KG == 1;
   int rc = once.run("attn29_kernel set-up", [] {
-    return cudaFuncSetAttribute(attn29_kernel<DH, KG, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const cudaError_t e = cudaFuncSetAttribute(attn29_kernel<DH, KG, kWarps, false>, at, smem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(attn29_kernel<DH, KG, kWarps, kPacks>, at, smem);
   });
+  if (!kPacks && start) {
+    set_error("attention: packed token rows of %d tokens", tokens);
+    return BSRL_ERR_UNSUPPORTED;
+  }
   if (rc != BSRL_OK) return rc;
   int64_t pairs = n_envs * n_heads;
   int64_t blocks = (pairs + kWarps - 1) / kWarps;
   int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  launch_kernel(attn29_kernel<DH, KG, kWarps>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, tokens, d, n_heads, q_first, n_q, out, ldo, start);
+  launch_kernel(start ? attn29_kernel<DH, KG, kWarps, kPacks> : attn29_kernel<DH, KG, kWarps, false>, static_cast<unsigned>(blocks), kWarps * 32, smem, stream,
+                qkv, ld, key_bias, pairs, tokens, d, n_heads, q_first, n_q, out, ldo, start);
   BSRL_LAUNCH_OK("attn29_kernel");
   return BSRL_OK;
 }

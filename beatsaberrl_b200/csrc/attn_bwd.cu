@@ -43,8 +43,8 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
 // the swizzled rows; every fragment is fetched once now, for both query or both key tiles).  16,384 environments of 8 heads of
 // 32, us, before / now (at copy speed): 29 queries 407 / 350 (260), 5 queries 276 / 226 (199), 1 query 272 / 224 (152).
 // Packed token rows (start: an environment's first row; up to 16 of them are one tile of queries and keys): 29 queries 363 / 282
-// with 17 of 29 rows left, 1 query 233 / 223.
-template <int DH, int MT>
+// with 17 of 29 rows left, 1 query 233 / 201.
+template <int DH, int MT, bool PACK>
 __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(const __half* __restrict__ qkv, int ld, const float* __restrict__ key_bias,
                                                                int64_t n_pairs, int d, int n_heads, int q_first, int n_queries,
                                                                const __half* __restrict__ g_out, int ldgo, __half* __restrict__ gq,
@@ -56,11 +56,20 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
     int64_t row0, q0;
     int tokens, n_q;
   };
-  auto rows_of = [&](int64_t env) {
-    const int64_t row0 = start ? start[env] : env * kT;
-    const int tokens = start ? (int)(start[env + 1] - row0) : kT;
-    const bool all = n_queries == kT;
+  auto rows_of = [&](int64_t env, int2 from) {
+    const int64_t row0 = PACK ? from.x : env * kT;
+    const int tokens = PACK ? from.y - from.x : kT;
+    const bool all = PACK && n_queries == kT;
     return Rows{row0, all ? row0 : env * n_queries, tokens, all ? tokens : n_queries};
+  };
+  // A pair's part of `start`.  With one query tile it is loaded a pair ahead of the requests (2 launches of 16,384 environments, 17 of
+  // 29 rows left: 223 -> 201 us); with two the registers for that cost more (282 -> 302).
+  constexpr bool AHEAD = PACK && MT == 1;
+  auto part_of = [&](int64_t pair) {
+    if (!PACK || pair >= n_pairs) return make_int2(0, 0);
+    int head;
+    const int64_t env = div_index(pair, n_heads, &head);
+    return make_int2(start[env], start[env + 1]);
   };
   constexpr int CH = DH / 8, ROW = DH * 2;
   constexpr int QR = 16 * MT;                         // staged query rows
@@ -76,13 +85,13 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
   const int rb = (lane & 7) + ((lane >> 4) << 3), cb = (lane >> 3) & 1;
   const int64_t warps = (int64_t)gridDim.x * kWarps;
   // q, dO (query rows) and k, v (key rows) of a pair into the tile at `at0`; rows past the live range are zero
-  auto request = [&](int64_t pair, uint32_t at0) {
+  auto request = [&](int64_t pair, uint32_t at0, int2 from) {
     if (pair < n_pairs) {
       int head;
       const int64_t env = div_index(pair, n_heads, &head);
-      const Rows e = rows_of(env);
+      const Rows e = rows_of(env, from);
       const __half* base = qkv + e.row0 * ld + head * DH;
-      for (int c = lane; c < (e.tokens <= 16 ? 16 : kKeys) * CH; c += 32) {
+      for (int c = lane; c < (PACK && e.tokens <= 16 ? 16 : kKeys) * CH; c += 32) {
         const int row = c / CH, ch = c % CH;
         const bool live = row < e.tokens, asks = row < e.n_q;
         const __half* r = base + (int64_t)(live ? row : 0) * ld + ch * 8;
@@ -97,11 +106,11 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
     }
     cp_async_commit();
   };
-  auto bias_of = [&](int64_t pair, float (&kb)[4][2]) {
+  auto bias_of = [&](int64_t pair, float (&kb)[4][2], int2 from) {
     if (pair >= n_pairs) return;
     int head;
     const int64_t env = div_index(pair, n_heads, &head);
-    const int tokens = rows_of(env).tokens;
+    const int tokens = rows_of(env, from).tokens;
 #pragma unroll
     for (int nt = 0; nt < 4; ++nt)
 #pragma unroll
@@ -112,7 +121,8 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
   };
   const int64_t first = (int64_t)blockIdx.x * kWarps + warp;
   float kb[4][2];
-  if (TILES == 2) request(first, smem_u32(tile));
+  int2 now = AHEAD ? part_of(first) : make_int2(0, 0), next = AHEAD ? part_of(first + warps) : make_int2(0, 0);
+  if (TILES == 2) request(first, smem_u32(tile), AHEAD ? now : part_of(first));
   int cur = 0;
   for (int64_t pair = first; pair < n_pairs; pair += warps) {
     int head;
@@ -122,13 +132,14 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
     uint8_t* sv = sk + kKeys * ROW;
     const uint32_t sq_u = smem_u32(sq), sg_u = sq_u + QR * ROW, sk_u = smem_u32(sk), sv_u = smem_u32(sv);
     __syncwarp();
-    bias_of(pair, kb);
+    bias_of(pair, kb, AHEAD ? now : part_of(pair));
+    const int2 later = AHEAD ? part_of(pair + 2 * warps) : make_int2(0, 0);
     if (TILES == 2) {
       cur ^= 1;
-      request(pair + warps, smem_u32(tile + cur * TILE));
+      request(pair + warps, smem_u32(tile + cur * TILE), AHEAD ? next : part_of(pair + warps));
       cp_async_wait<1>();
     } else {
-      request(pair, sq_u);
+      request(pair, sq_u, AHEAD ? now : part_of(pair));
       cp_async_wait<0>();
     }
     __syncwarp();
@@ -290,8 +301,8 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
           tc5::stmatrix_x4(sq_u + tile_at<DH>(mt * 16 + ra, j * 2 + ca), oq16[mt][2 * j][0], oq16[mt][2 * j][1], oq16[mt][2 * j + 1][0], oq16[mt][2 * j + 1][1]);
       __syncwarp();
     };
-    const Rows e = rows_of(env);
-    if (e.tokens <= 16) products(std::integral_constant<int, 1>(), std::integral_constant<int, 1>());
+    const Rows e = rows_of(env, AHEAD ? now : part_of(pair));
+    if (PACK && e.tokens <= 16) products(std::integral_constant<int, 1>(), std::integral_constant<int, 1>());
     else products(std::integral_constant<int, MT>(), std::integral_constant<int, 2>());
     auto out = [&](const uint8_t* from, int rows, __half* dst, int64_t ldd) {
       for (int c = lane; c < rows * CH; c += 32) {
@@ -309,6 +320,8 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
     out(sv, e.tokens, gv + e.row0 * ldv + head * DH, ldv);
     out(sk, e.tokens, gk + e.row0 * ldk + head * DH, ldk);
     out(sq, e.n_q, gq + e.q0 * ldq + head * DH, ldq);
+    now = next;
+    next = later;
   }
 }
 
@@ -318,7 +331,9 @@ int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int
   constexpr int kWarps = warps_of<DH, MT>(), smem = kWarps * tiles_of<DH>() * (2 * 16 * MT + 2 * kKeys) * DH * 2;
   static DeviceOnce once;
   int rc = once.run("attn_bwd_kernel set-up", [] {
-    return cudaFuncSetAttribute(attn_bwd_kernel<DH, MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    const cudaFuncAttribute at = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    const cudaError_t e = cudaFuncSetAttribute(attn_bwd_kernel<DH, MT, false>, at, smem);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(attn_bwd_kernel<DH, MT, true>, at, smem);
   });
   if (rc != BSRL_OK) return rc;
   const int wide = aligned16(gq) && aligned16(gk) && aligned16(gv) && ldq % 8 == 0 && ldk % 8 == 0 && ldv % 8 == 0;
@@ -327,7 +342,7 @@ int launch(const __half* qkv, int ld, const float* key_bias, int64_t n_envs, int
   // several short waves: blocks that stay for all of their pairs stream in step, 435 us where 8 to 24 per SM take 350
   const int64_t cap = (int64_t)sm_count() * 16;
   if (blocks > cap) blocks = cap;
-  launch_kernel(attn_bwd_kernel<DH, MT>, (unsigned)blocks, kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d, n_heads, q_first, n_q, g_out,
+  launch_kernel(start ? attn_bwd_kernel<DH, MT, true> : attn_bwd_kernel<DH, MT, false>, (unsigned)blocks, kWarps * 32, smem, stream, qkv, ld, key_bias, pairs, d, n_heads, q_first, n_q, g_out,
                                                                           ldgo, gq, ldq, gk, ldk, gv, ldv, wide, start);
   BSRL_LAUNCH_OK("attn_bwd_kernel");
   return BSRL_OK;
