@@ -42,8 +42,8 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
 // bytes per lane.  Bound by the turns of the shared-memory pipe (654 of the 909 cycles per pair of 29 queries x 32 before
 // the swizzled rows; every fragment is fetched once now, for both query or both key tiles).  16,384 environments of 8 heads of
 // 32, us, before / now (at copy speed): 29 queries 407 / 350 (260), 5 queries 276 / 226 (199), 1 query 272 / 224 (152).
-// Packed token rows (start: an environment's first row; up to 16 of them are one tile of queries and keys): 29 queries 363 / 282
-// with 17 of 29 rows left, 1 query 233 / 201.
+// Packed token rows (start: an environment's first row; up to 16 of them are one tile of queries and keys): 29 queries 363 / 300
+// with 17 of 29 rows left, 1 query 233 / 195.
 template <int DH, int MT, bool PACK>
 __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(const __half* __restrict__ qkv, int ld, const float* __restrict__ key_bias,
                                                                int64_t n_pairs, int d, int n_heads, int q_first, int n_queries,
@@ -51,22 +51,23 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
                                                                int ldq, __half* __restrict__ gk, int ldk, __half* __restrict__ gv,
                                                                int ldv, int wide, const int* __restrict__ start) {
   pdl_begin();
+  // A pair's part of `start`.  With one query tile it is loaded a pair ahead of the requests (16,384 environments, 17 of
+  // 29 rows left: 223 -> 195 us); with two it takes registers and gives nothing (302 us against 300).
+  constexpr bool AHEAD = PACK && MT == 1;
   // packed token rows: an environment's first row, its rows and its queries (as many where all are asked for)
   struct Rows {
     int64_t row0, q0;
     int tokens, n_q;
   };
   auto rows_of = [&](int64_t env, int2 from) {
+    if (PACK && !AHEAD) from = make_int2(start[env], start[env + 1]);
     const int64_t row0 = PACK ? from.x : env * kT;
     const int tokens = PACK ? from.y - from.x : kT;
     const bool all = PACK && n_queries == kT;
     return Rows{row0, all ? row0 : env * n_queries, tokens, all ? tokens : n_queries};
   };
-  // A pair's part of `start`.  With one query tile it is loaded a pair ahead of the requests (2 launches of 16,384 environments, 17 of
-  // 29 rows left: 223 -> 201 us); with two the registers for that cost more (282 -> 302).
-  constexpr bool AHEAD = PACK && MT == 1;
   auto part_of = [&](int64_t pair) {
-    if (!PACK || pair >= n_pairs) return make_int2(0, 0);
+    if (!AHEAD || pair >= n_pairs) return make_int2(0, 0);
     int head;
     const int64_t env = div_index(pair, n_heads, &head);
     return make_int2(start[env], start[env + 1]);
@@ -121,8 +122,8 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
   };
   const int64_t first = (int64_t)blockIdx.x * kWarps + warp;
   float kb[4][2];
-  int2 now = AHEAD ? part_of(first) : make_int2(0, 0), next = AHEAD ? part_of(first + warps) : make_int2(0, 0);
-  if (TILES == 2) request(first, smem_u32(tile), AHEAD ? now : part_of(first));
+  int2 now = part_of(first), next = part_of(first + warps);
+  if (TILES == 2) request(first, smem_u32(tile), now);
   int cur = 0;
   for (int64_t pair = first; pair < n_pairs; pair += warps) {
     int head;
@@ -132,14 +133,14 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
     uint8_t* sv = sk + kKeys * ROW;
     const uint32_t sq_u = smem_u32(sq), sg_u = sq_u + QR * ROW, sk_u = smem_u32(sk), sv_u = smem_u32(sv);
     __syncwarp();
-    bias_of(pair, kb, AHEAD ? now : part_of(pair));
-    const int2 later = AHEAD ? part_of(pair + 2 * warps) : make_int2(0, 0);
+    bias_of(pair, kb, now);
+    const int2 later = part_of(pair + 2 * warps);
     if (TILES == 2) {
       cur ^= 1;
-      request(pair + warps, smem_u32(tile + cur * TILE), AHEAD ? next : part_of(pair + warps));
+      request(pair + warps, smem_u32(tile + cur * TILE), next);
       cp_async_wait<1>();
     } else {
-      request(pair, sq_u, AHEAD ? now : part_of(pair));
+      request(pair, sq_u, now);
       cp_async_wait<0>();
     }
     __syncwarp();
@@ -301,7 +302,7 @@ __global__ void __launch_bounds__((warps_of<DH, MT>()) * 32) attn_bwd_kernel(con
           tc5::stmatrix_x4(sq_u + tile_at<DH>(mt * 16 + ra, j * 2 + ca), oq16[mt][2 * j][0], oq16[mt][2 * j][1], oq16[mt][2 * j + 1][0], oq16[mt][2 * j + 1][1]);
       __syncwarp();
     };
-    const Rows e = rows_of(env, AHEAD ? now : part_of(pair));
+    const Rows e = rows_of(env, now);
     if (PACK && e.tokens <= 16) products(std::integral_constant<int, 1>(), std::integral_constant<int, 1>());
     else products(std::integral_constant<int, MT>(), std::integral_constant<int, 2>());
     auto out = [&](const uint8_t* from, int rows, __half* dst, int64_t ldd) {
