@@ -74,9 +74,13 @@ void use_process_engine() { g_call_engine = g_engine.load(std::memory_order_rela
 int process_engine() { return g_engine.load(std::memory_order_relaxed); }
 int linear(const LinearArgs& p, cudaStream_t st) {
   return timed(st, 2.0 * p.M * p.N * p.K, linear_bytes(p), [&] {
-    if (p.a_mn || p.w_mn || p.mask || p.n_rows || p.rmap.start || p.cmap.start) {      // row-contraction operands, the epilogue mask, counted rows: the tcgen05 engine only
+    const bool by_table = p.amap.start || p.rmap.start || p.cmap.start;
+    if (p.a_mn || p.w_mn || p.mask || p.n_rows || by_table) {
       if (g_call_engine == 0 && linear_tc5_ok(p)) return linear_tc5(p, st);
-      set_error("linear: row-contraction operands and counted rows need the tcgen05 engine and M, N multiples of 64 (m=%lld n=%d k=%d)",
+      // The warp-MMA kernel follows tables of first rows, and computes up to a count's bound (rows past the count are in the
+      // buffers, and so are their results).  Not both: a table's entries past the count are anything.
+      if (!p.a_mn && !p.w_mn && !p.mask && !(p.n_rows && by_table)) return linear_mma(p, st);
+      set_error("linear: row-contraction operands and mapped counted rows need the tcgen05 engine and M, N multiples of 64 (m=%lld n=%d k=%d)",
                 (long long)p.M, p.N, p.K);
       return (int)BSRL_ERR_UNSUPPORTED;
     }
@@ -427,6 +431,8 @@ int run_forward(const Ctx& ctx, const void* obs, int obs_dtype, const HeadTailAr
   PdlScope pdl;
   Ctx c = ctx;
   if (c.paths.packed) c.rows = carve_rows(c.train ? c.train->rows : at<void>(c.ws, c.w.rows), c.B, kT);
+  // the save buffer of a batch this large comes with a row table, whichever engine fills it
+  else if (c.train && train_packed(c.l, c.B)) BSRL_TRY(full_rows(c.B, carve_rows(c.train->rows, c.B, kT), c.st));
   const Layout& l = c.l;
   const Workspace& w = c.w;
   const int d = l.d, F = l.F, D = l.D;

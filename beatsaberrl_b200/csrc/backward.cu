@@ -281,14 +281,15 @@ __global__ void __launch_bounds__(256) gather_tokens16_kernel(const __half* __re
 }
 
 // out (cols, ldo) = in (rows, ldi)^T, fp16, 64 x 64 tiles through shared memory, 16-byte accesses on both
-// sides; rows [rows, rows_pad) of the input read as zero, so the padded K range of the following GEMM
-// contributes nothing.  With colsum, the column sums of the input (a Linear's bias gradient, when the input is
+// sides; rows [rows, rows_pad) of the input (rows: the device's count, where there is one) read as zero, so the padded
+// K range of the following GEMM contributes nothing.  With colsum, the column sums of the input (a Linear's bias gradient, when the input is
 // dL/dy) are accumulated on the way: per-tile partial sums, one atomic per column and tile.
 // Requires cols % 8 == 0, ldi % 8 == 0, ldo % 8 == 0 and 16-byte aligned bases.
-__global__ void __launch_bounds__(256) transpose16_kernel(const __half* __restrict__ in, int64_t ldi, RowMap imap, int64_t rows,
+__global__ void __launch_bounds__(256) transpose16_kernel(const __half* __restrict__ in, int64_t ldi, RowMap imap, int64_t row_bound,
                                                           int cols, __half* __restrict__ out, int64_t ldo, int64_t rows_pad,
-                                                          float* __restrict__ colsum) {
+                                                          float* __restrict__ colsum, const int* n_rows, int64_t n_less) {
   pdl_begin();
+  const int64_t rows = n_rows ? n_rows[0] - n_less : row_bound;
   __shared__ __align__(16) __half tile[64][72];      // 144-byte rows: column reads of 8 rows hit 8 bank groups
   const int64_t r0 = (int64_t)blockIdx.x * 64;
   const int c0 = blockIdx.y * 64;
@@ -321,10 +322,11 @@ __global__ void __launch_bounds__(256) transpose16_kernel(const __half* __restri
 }
 
 // small-shape fallback of the transpose (any cols / alignment), element-wise
-__global__ void __launch_bounds__(256) transpose16_slow_kernel(const __half* __restrict__ in, int64_t ldi, RowMap imap, int64_t rows,
+__global__ void __launch_bounds__(256) transpose16_slow_kernel(const __half* __restrict__ in, int64_t ldi, RowMap imap, int64_t row_bound,
                                                                int cols, __half* __restrict__ out, int64_t ldo, int64_t rows_pad,
-                                                               float* __restrict__ colsum) {
+                                                               float* __restrict__ colsum, const int* n_rows, int64_t n_less) {
   pdl_begin();
+  const int64_t rows = n_rows ? n_rows[0] - n_less : row_bound;
   __shared__ __half tile[64][66];
   const int64_t r0 = (int64_t)blockIdx.x * 64;
   const int c0 = blockIdx.y * 64;
@@ -517,7 +519,7 @@ int gather_tokens16(const __half* in, int64_t n_envs, int n, __half* out, cudaSt
 }
 
 int transpose16(const __half* in, int64_t ldi, RowMap imap, int64_t rows, int cols, __half* out, int64_t ldo,
-                int64_t rows_pad, cudaStream_t stream, float* colsum) {
+                int64_t rows_pad, cudaStream_t stream, float* colsum, const int* n_rows, int64_t n_less) {
   if (rows_pad == 0 || cols == 0) return BSRL_OK;
   const int64_t bx = (rows_pad + 63) / 64;
   if (bx > 0x7fffffff) {
@@ -526,8 +528,8 @@ int transpose16(const __half* in, int64_t ldi, RowMap imap, int64_t rows, int co
   }
   const dim3 grid((unsigned)bx, (cols + 63) / 64);
   const bool fast = cols % 8 == 0 && ldi % 8 == 0 && ldo % 8 == 0 && rows_pad % 8 == 0 && aligned16(in) && aligned16(out);
-  if (fast) launch_kernel(transpose16_kernel, grid, 256, 0, stream, in, ldi, imap, rows, cols, out, ldo, rows_pad, colsum);
-  else launch_kernel(transpose16_slow_kernel, grid, 256, 0, stream, in, ldi, imap, rows, cols, out, ldo, rows_pad, colsum);
+  if (fast) launch_kernel(transpose16_kernel, grid, 256, 0, stream, in, ldi, imap, rows, cols, out, ldo, rows_pad, colsum, n_rows, n_less);
+  else launch_kernel(transpose16_slow_kernel, grid, 256, 0, stream, in, ldi, imap, rows, cols, out, ldo, rows_pad, colsum, n_rows, n_less);
   BSRL_LAUNCH_OK("transpose16_kernel");
   return BSRL_OK;
 }

@@ -29,6 +29,9 @@ struct RowSource {
   int64_t rows_ahead;
 };
 int token_rows(const RowSource& src, int64_t n_envs, const TokenRows& out, cudaStream_t stream);
+// start, dst and the row count of 29 rows for every environment (no tiles, no key bias): the full layout, as a reader of packed
+// rows takes it
+int full_rows(int64_t n_envs, const TokenRows& out, cudaStream_t stream);
 
 // C = act(A W^T + bias) (+ R).  A (M, K) f16 and W (N, K) f16, both K-contiguous.
 struct LinearArgs {
@@ -72,7 +75,7 @@ struct LinearArgs {
   const uint32_t* bits_in = nullptr;
   int64_t bits_ld = 0;               // blocks of 32 rows
   // Packed token rows: the device's count of the rows (with a_mn of the contraction, K), less n_less; M (K) is its bound.  The
-  // tcgen05 engine only.
+  // tcgen05 engine; linear_mma computes up to the bound.
   const int* n_rows = nullptr;
   int64_t n_less = 0;
   __device__ __forceinline__ int64_t live(int64_t bound) const { return n_rows ? n_rows[0] - n_less : bound; }

@@ -99,6 +99,9 @@ struct Paths {
 };
 int64_t small_envs(const Layout& l);      // the largest batch that may take Paths::small
 Paths plan_paths(const Layout& l, int engine, int64_t n_envs);
+// whether a save buffer is read through its row table: by the shape and the batch alone, for the forward that fills it and the
+// backward may run on different engines
+inline bool train_packed(const Layout& l, int64_t n_envs) { return plan_paths(l, 0, n_envs).packed; }
 
 // Workspace carve-up for a batch of n_envs (offsets of buffers the path does not use are -1).
 struct Workspace {

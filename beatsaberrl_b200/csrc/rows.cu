@@ -164,7 +164,38 @@ __global__ void __launch_bounds__(kIndexGroup) row_index_kernel(int64_t n_envs, 
     out.n_tiles[1] = (int)rows_ahead + all;
   }
 }
+
+__global__ void __launch_bounds__(256) full_rows_kernel(int64_t n_envs, TokenRows out) {
+  pdl_begin();
+  const int64_t total = n_envs * kT;
+  for (int64_t in = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; in < total; in += (int64_t)gridDim.x * blockDim.x) {
+    int64_t env;
+    int tok;
+    if (in < 2 * n_envs) env = div_index(in, 2, &tok);
+    else if (in < 3 * n_envs) env = in - 2 * n_envs, tok = 2;
+    else if (in < kLead * n_envs) env = div_index(in - 3 * n_envs, 2, &tok), tok += 3;
+    else env = div_index(in - kLead * n_envs, kSlots, &tok), tok += kLead;
+    out.dst[in] = (int)(env * kT) + tok;
+    if (in <= n_envs) out.start[in] = (int)in * kT;
+    if (in == 0) out.n_tiles[0] = 0, out.n_tiles[1] = (int)total;
+  }
+}
 }  // namespace
+
+int full_rows(int64_t n_envs, const TokenRows& out, cudaStream_t stream) {
+  if (!out.start || !out.dst) {
+    set_error("full_rows: NULL operand");
+    return BSRL_ERR_NULL;
+  }
+  if (n_envs < 1 || n_envs > (int64_t)1 << 26) {
+    set_error("full_rows: %lld environments", (long long)n_envs);
+    return BSRL_ERR_UNSUPPORTED;
+  }
+  const int64_t blocks = (n_envs * kT + 255) / 256, cap = (int64_t)sm_count() * 8;
+  launch_kernel(full_rows_kernel, (unsigned)(blocks < cap ? blocks : cap), 256, 0, stream, n_envs, out);
+  BSRL_LAUNCH_OK("full_rows_kernel");
+  return BSRL_OK;
+}
 
 int token_rows(const RowSource& src, int64_t n_envs, const TokenRows& out, cudaStream_t stream) {
   if (!src.obs || !out.start) {

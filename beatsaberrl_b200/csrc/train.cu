@@ -41,7 +41,7 @@ int gather_rows16(const __half* in, int64_t ldi, RowMap imap, __half* out, int64
 int gather_tokens16(const __half* in, int64_t n_envs, int n, __half* out, cudaStream_t stream, const int* dst = nullptr,
                     const int* n_rows = nullptr);
 int transpose16(const __half* in, int64_t ldi, RowMap imap, int64_t rows, int cols, __half* out, int64_t ldo,
-                int64_t rows_pad, cudaStream_t stream, float* colsum = nullptr);
+                int64_t rows_pad, cudaStream_t stream, float* colsum = nullptr, const int* n_rows = nullptr, int64_t n_less = 0);
 int head_tail_bwd(const HeadTailArgs& a, const float* g_logprob, const float* g_entropy, const float* g_value,
                   const float* g_vlogits, const float* g_logits, float scale, __half* g_raw, int ldg_raw, __half* g_vraw,
                   int ldg_v, cudaStream_t stream);
@@ -343,13 +343,9 @@ struct Bwd {
       else BSRL_TRY(colsum16(g, ldg, M, N, gb, st, count.n_rows, count.less));
       return linear(r, st);
     }
-    if (count.n_rows) {
-      set_error("backward: a weight gradient over packed token rows needs the tcgen05 engine");
-      return BSRL_ERR_UNSUPPORTED;
-    }
     __half *tA = S<__half>(w.tA), *tX = S<__half>(w.tX);
-    BSRL_TRY(transpose16(g, ldg, identity_map(), M, N, tA, Mp, Mp, st, gb));
-    BSRL_TRY(transpose16(x, ldx, identity_map(), M, K, tX, Mp, Mp, st));
+    BSRL_TRY(transpose16(g, ldg, identity_map(), M, N, tA, Mp, Mp, st, gb, count.n_rows, count.less));
+    BSRL_TRY(transpose16(x, ldx, identity_map(), M, K, tX, Mp, Mp, st, nullptr, count.n_rows, count.less));
     LinearArgs a = linear_args(tA, (int)Mp, tX, (int)Mp, nullptr, gW, ldgw, 1, 0, N, K, (int)Mp);
     a.k_splits = splits;
     return linear_mma(a, st);          // as in dgrad
@@ -834,7 +830,7 @@ int bsrl_backward(const bsrl_config* cfg, const void* arena, int64_t n_envs, con
   c.ws = workspace;
   c.B = n_envs;
   c.st = st;
-  if (plan_paths(l, process_engine(), n_envs).packed) c.rows = carve_rows(t.rows, n_envs, kT);       // as the forward laid them out
+  if (train_packed(l, n_envs)) c.rows = carve_rows(t.rows, n_envs, kT);       // as the forward laid them out
   Bwd b{c, c.l, t, w, workspace, grads, gl, loss_scale, st, n_envs, n_envs * kT, n_envs * kLead, l.d, l.F, l.D};
   HeadTailArgs h;
   memset(&h, 0, sizeof(h));

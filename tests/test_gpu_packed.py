@@ -124,6 +124,42 @@ def test_gradients_equal_the_sum_over_slices(name, opts, kind):
         assert float((m.get_parameter(k).grad - g).norm()) <= 1e-4 * float(g.norm()) + 1e-6 * top, k
 
 
+@pytest.mark.parametrize("forward,backward", [(0, 1), (1, 0), (1, 1)])
+@pytest.mark.parametrize("name,opts", [("cfg1", {}), ("recipe", dict(value_residual=True)), ("cfg4", {}), ("cfg1", dict(emb_ln=True, final_ln=True))])
+def test_forward_and_backward_on_different_engines(native, name, opts, forward, backward):
+    """Whichever engine fills a save buffer and whichever reads it: the gradients are those of the default engine, up to the two engines'
+    fp16 roundings (the bound that the engines are compared by elsewhere)."""
+    envs = 701
+    cfg = make_cfg(name, name == "recipe", opts=dict(opts, n_blocks=2))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 5))
+    obs, act, up = _obs("holes", envs, 44).cuda(), po.make_actions(envs, cfg, 22).cuda(), po.make_upstream(envs, cfg, 23)
+
+    def grads(fwd, bwd):
+        m.zero_grad()
+        m._workspaces.clear()                 # their size is the engine's
+        try:
+            with torch.enable_grad():
+                native.lib.bsrl_set_engine(fwd)
+                _, lp, ent, val = m.get_action_and_value(obs, act)
+                loss = (up["logprob"].cuda() * lp).sum() + (up["entropy"].cuda() * ent).sum() + (up["value"].cuda() * val).sum()
+                native.lib.bsrl_set_engine(bwd)
+                loss.backward()
+            torch.cuda.synchronize()
+        finally:
+            native.lib.bsrl_set_engine(0)
+            m._workspaces.clear()
+        return {k: p.grad.clone() for k, p in m.named_parameters() if p.grad is not None}
+
+    grads(0, 0)
+    want = grads(0, 0)
+    got = grads(forward, backward)
+    m.check_device()
+    top = max(float(g.norm()) for g in want.values())
+    assert want.keys() == got.keys()
+    for k, g in want.items():
+        assert float((got[k] - g).norm()) <= 2e-2 * float(g.norm()) + 2e-3 * top, k
+
+
 @pytest.mark.parametrize("kind", ["none", "all", "holes", "last", "runs"])
 @pytest.mark.parametrize("name,heads", [("cfg1", 4), ("cfg2", 8), ("cfg4", 8), ("cfg2", 4), ("cfg1", 2)])
 def test_body_token_layout(native, name, heads, kind):
