@@ -91,7 +91,10 @@ __device__ void slot_geometry(const float* o, int slot, float z_asinh, bool flux
   }
 }
 
-// PACK: packed token rows (EmbedBuffers::rows)
+// PACK: packed token rows (EmbedBuffers::rows).  A slot without a row must not change what its environment's outputs are: with an
+// infinite feature (in fp16) its encoding is not a number, and through the attention neither is any row of the environment
+// (0 times not a number); the key bias says so in its place.  A feature that is not a number itself leaves zeros behind the encoder's
+// ReLU, and no trace.  Looked at only where an observation holds anything above a thousand (they are clipped to 5).
 template <bool OBS_F16, bool PACK>
 __global__ void __launch_bounds__(kWarps * 32, 4) embed_gather_kernel(const void* __restrict__ obs_,
                                                                   int64_t n_envs, int note_geo,
@@ -110,12 +113,17 @@ __global__ void __launch_bounds__(kWarps * 32, 4) embed_gather_kernel(const void
   for (int64_t env = (int64_t)blockIdx.x * kWarps + warp; env < n_envs;
        env += (int64_t)gridDim.x * kWarps) {
     __syncwarp();
+    float largest = 0.f;
+    auto take = [&](int i, float v) {
+      o[i] = v;
+      if (PACK) largest = fmaxf(largest, fabsf(v));
+    };
     if (OBS_F16) {
       const __half* src = static_cast<const __half*>(obs_) + env * kObs;
-      for (int i = lane; i < kObs; i += 32) o[i] = __half2float(src[i]);
+      for (int i = lane; i < kObs; i += 32) take(i, __half2float(src[i]));
     } else {
       const float* src = static_cast<const float*>(obs_) + env * kObs;
-      for (int i = lane; i < kObs; i += 32) o[i] = src[i];
+      for (int i = lane; i < kObs; i += 32) take(i, src[i]);
     }
     __syncwarp();
     if (out.obs16) {   // fp16 copy of the row (b_obs[t] of the rollout buffer, python/train_batch.py:2299)
@@ -143,6 +151,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4) embed_gather_kernel(const void
     }
     __syncwarp();
     // slot rows
+    bool infinite = false;             // a slot without a row holds an infinite feature
     {
       // every slot row is 64 features = one lane per pair: obs lanes, then the geometry lanes, then zeros
       // (the feature counts are even, so a pair never straddles two sources)
@@ -155,9 +164,19 @@ __global__ void __launch_bounds__(kWarps * 32, 4) embed_gather_kernel(const void
 #pragma unroll 8
       for (int slot = 0; slot < n_slots; ++slot)
         d[slot * 32 + lane] = src ? pack_half2(src[slot * step], src[slot * step + 1]) : 0u;
+      if (PACK && __any_sync(0xffffffffu, largest > 1000.f)) {
+        if (note_geo && lane >= n_slots && lane < kSlots) slot_geometry(o, lane, z_asinh, (note_geo & 2) != 0, geo + lane * kGeoFeat);
+        __syncwarp();
+        for (int slot = n_slots; slot < kSlots; ++slot) {
+          const uint32_t v = src ? pack_half2(src[slot * step], src[slot * step + 1]) : 0u;
+          const uint32_t lo = v & 0x7fffu, hi = (v >> 16) & 0x7fffu;
+          infinite |= __any_sync(0xffffffffu, lo == 0x7c00u || hi == 0x7c00u) && !__any_sync(0xffffffffu, lo > 0x7c00u || hi > 0x7c00u);
+        }
+      }
     }
     if (lane < kT) {
-      const float bias = lane < kLead ? 0.f : (o[kOffMask + lane - kLead] - 1.0f) * kMaskBias;
+      float bias = lane < kLead ? 0.f : (o[kOffMask + lane - kLead] - 1.0f) * kMaskBias;
+      if (PACK && lane == 0 && infinite) bias = __int_as_float(0x7fffffff);
       out.key_bias[env * kT + lane] = bias;
       if (PACK && lane < kLead + n_slots) {
         const int64_t in = lane < 2 ? 2 * env + lane : lane < 3 ? 2 * n_envs + env : lane < kLead ? 3 * n_envs + 2 * env + lane - 3

@@ -217,8 +217,11 @@ bool g_tail_fused(const GLayout& l, int engine) {
 // (token 0 always attendable, object j by its live flag: 0 or -16384, python/policy.py:422-428).
 // `parts` warps (a power of two) share an environment: one where the batch fills the chip, which is bound by the bytes then, and up to
 // 16 below, where the time is a warp's chain of loads and stores.
-template <bool PACK>
-__global__ void __launch_bounds__(256) embed_g_kernel(const float* __restrict__ obs, int64_t n_envs, int obs_dim, int body_dim,
+// PACK: objects without a row are read all the same, for what they hold must show as it does in the full layout: 84 -> 101 us at 65,536
+// environments of 32, 16 live (10 us of it the bytes; with scalar loads 136 to 144).  WIDE: for that, every row of obs and every
+// object in it starts at 16 bytes.
+template <bool PACK, bool WIDE>
+__global__ void __launch_bounds__(256, PACK ? 6 : 1) embed_g_kernel(const float* __restrict__ obs, int64_t n_envs, int obs_dim, int body_dim,
                                                       int body_k, int n_obj, int obj_dim, __half* __restrict__ f_body,
                                                       __half* __restrict__ f_obj, float* __restrict__ key_bias, TokenRows rows, int parts) {
   pdl_begin();
@@ -232,12 +235,25 @@ __global__ void __launch_bounds__(256) embed_g_kernel(const float* __restrict__ 
     const float* ob = o + body_dim;
     const float* live = ob + n_obj * obj_dim;
     __half* fb = f_body + env * body_k;
-#pragma unroll 4
-    for (int c = 2 * at; c < body_k; c += 2 * step)
-      *reinterpret_cast<uint32_t*>(fb + c) = pack_half2(c < body_dim ? o[c] : 0.f, c + 1 < body_dim ? o[c + 1] : 0.f);
     const int64_t obj0 = PACK ? rows.start[env] : env * n_obj;
     const int n_rows = PACK ? (int)(rows.start[env + 1] - obj0) : n_obj;
     uint2* fo = reinterpret_cast<uint2*>(f_obj + obj0 * 64);
+    // the objects without a row, their first lanes requested ahead of everything else
+    const float* dead = ob + n_rows * obj_dim;
+    const int n_dead = (n_obj - n_rows) * obj_dim;
+    float4 first[2];
+    bool bad = false;
+    auto look = [&](float v) { bad |= !(fabsf(v) < 65520.f); };       // fp16 holds it as infinite or not a number
+    if (PACK && WIDE) {
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const int i = at + u * step;
+        first[u] = i < n_dead >> 2 ? reinterpret_cast<const float4*>(dead)[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+    }
+#pragma unroll 4
+    for (int c = 2 * at; c < body_k; c += 2 * step)
+      *reinterpret_cast<uint32_t*>(fb + c) = pack_half2(c < body_dim ? o[c] : 0.f, c + 1 < body_dim ? o[c + 1] : 0.f);
 #pragma unroll 4
     for (int i = at; i < n_rows * 16; i += step) {
       const int c = (i & 15) * 4;
@@ -252,6 +268,17 @@ __global__ void __launch_bounds__(256) embed_g_kernel(const float* __restrict__ 
       key_bias[env * T + t] = bias;
       if (PACK && t > 0 && t <= n_rows) rows.kb[obj0 + t - 1] = bias;
     }
+    if (PACK) {
+      if (WIDE) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) look(first[u].x), look(first[u].y), look(first[u].z), look(first[u].w);
+      }
+#pragma unroll (WIDE ? 2 : 8)
+      for (int i = at + (WIDE ? 8 * step : 0); i < n_dead; i += step) look(dead[i]);
+    }
+    // Such an object must not change what its environment's outputs are: its row would not be a number, and through the attention
+    // neither would any of the environment (0 times not a number).  The warp's piece of the body row is made so.
+    if (PACK && __any_sync(0xffffffffu, bad) && lane == 0) *reinterpret_cast<uint32_t*>(fb + 2 * at) = 0x7fff7fffu;
   }
 }
 
@@ -302,11 +329,13 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
       begin_overlap(B * l.T);
     }
     int parts = 1;
-    while (parts < 16 && B * parts < (int64_t)sm_count() * 16) parts *= 2;
+    while (parts < 16 && B * parts < (int64_t)sm_count() * 16 && (!packed || 128 * parts <= l.body_k)) parts *= 2;      // packed: a piece of the body row each
     int64_t blocks = (B * parts + 7) / 8;
     const int64_t cap = (int64_t)sm_count() * 16;
     if (blocks > cap) blocks = cap;
-    launch_kernel(packed ? embed_g_kernel<true> : embed_g_kernel<false>, (unsigned)blocks, 256, 0, st, obs, B, l.obs_dim, l.body_dim, l.body_k, l.n_obj, l.obj_dim, f_body,
+    const bool wide = aligned16(obs) && l.obs_dim % 4 == 0 && l.body_dim % 4 == 0 && l.obj_dim % 4 == 0;
+    auto* kernel = !packed ? embed_g_kernel<false, false> : wide ? embed_g_kernel<true, true> : embed_g_kernel<true, false>;
+    launch_kernel(kernel, (unsigned)blocks, 256, 0, st, obs, B, l.obs_dim, l.body_dim, l.body_k, l.n_obj, l.obj_dim, f_body,
                   f_obj, key_bias, rows, parts);
     BSRL_LAUNCH_OK("embed_g_kernel");
     return BSRL_OK;

@@ -4,8 +4,10 @@
 // (the readout takes the lead tokens, the critic pools over the live keys), so its row is work for padding.  An
 // environment therefore owns only the rows up to its last live slot -- a prefix, so that every row keeps its place among
 // the keys and every sum its order: results have the bits of the full layout -- and environments follow one another
-// without gaps.  With n of 24 slots live, n uniform, 17 of 29 rows remain, and the time of everything that works on token
-// rows with them (65,536 environments at d 256: 15.6 -> 10.4 ms).
+// without gaps.  (Exactly 0 as long as no score of a live key lies 16,000 below the dead one's, which no finite weights in use come
+// near; and 0 times not a number is not a number: the tokenizers see to dead slots with lanes that fp16 cannot hold.)  With n of
+// 24 slots live, n uniform, 17 of 29 rows remain, and the time of everything that works on token rows with them (65,536 environments
+// at d 256: 15.6 -> 10.4 ms).
 //
 // The counts are known on the device only.  Per group of environments a block counts the rows, adds them up and forms the
 // attention kernel's tiles: as many whole environments as fit 128 rows, one after the other.  Up to eight groups are a

@@ -93,6 +93,35 @@ def test_not_a_number_stays_in_its_environment(name):
     assert torch.isnan(logits[bad]).any(-1).any(-1).all()
 
 
+def _same(a, b):
+    """The same bits, and not a number in the same places."""
+    return torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a.nan_to_num(nan=0.0), b.nan_to_num(nan=0.0))
+
+
+@pytest.mark.parametrize("bad,shows", [([float("inf")], True), ([float("-inf"), float("inf")], True), ([7e4], True), ([float("nan")], False),
+                                       ([float("nan"), float("inf")], False), ([6e4], False)])
+@pytest.mark.parametrize("name,opts", [("cfg1", {}), ("recipe", {}), ("recipe", dict(game="flux")), ("cfg4", {}), ("cfg1", dict(emb_ln=True, final_ln=True)),
+                                       ("cfg1", dict(n_blocks=1))])
+def test_dead_slots_that_fp16_cannot_hold(name, opts, bad, shows):
+    """What a dead slot holds shows in its environment's outputs in the full layout as soon as its encoding is not a number; without a
+    row it shows all the same."""
+    cfg = make_cfg(name, name == "recipe", opts=dict(dict(n_blocks=2), **opts))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
+    envs = 1203
+    obs = po.make_obs(envs, 48, padded=True).cuda()
+    obs[:, po.OFF_MASK + 22:po.OFF_MASK + 24] = 0.0
+    for i, v in enumerate(bad):
+        obs[2::3, po.OFF_NOTES + 18 * 23 + 5 * i] = v
+        obs[3::7, po.OFF_NOTES + 18 * 22 + 1 + 4 * i] = v
+    logits, value = m.forward_stacked(obs)
+    for lo in range(0, envs, 401):
+        l, v = m.forward_stacked(obs[lo:lo + 401])
+        assert _same(l, logits[lo:lo + 401]) and _same(v, value[lo:lo + 401]), lo
+    if name != "recipe":                         # (the geometry of such a slot may be not a number, which the encoder's ReLU drops)
+        assert bool(torch.isnan(logits[2]).any()) == shows
+    m.check_device()
+
+
 @pytest.mark.parametrize("kind", ["none", "all", "holes"])
 @pytest.mark.parametrize("name,opts", [("cfg1", {}), ("recipe", dict(value_residual=True)), ("cfg4", {}), ("cfg1", dict(emb_ln=True, final_ln=True)),
                                        ("tiny", dict(trunk_arch="simbav2"))])
@@ -158,6 +187,28 @@ def test_forward_and_backward_on_different_engines(native, name, opts, forward, 
     assert want.keys() == got.keys()
     for k, g in want.items():
         assert float((got[k] - g).norm()) <= 2e-2 * float(g.norm()) + 2e-3 * top, k
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("-inf"), 7e4, 6e4])
+@pytest.mark.parametrize("name,heads,envs", [("cfg1", 4, 1503), ("cfg2", 8, 1203), ("cfg4", 8, 803), ("cfg2", 8, 19000)])
+def test_dead_objects_that_fp16_cannot_hold(native, name, heads, envs, bad):
+    cfg = bo.named_config(name)
+    cfg.n_blocks, cfg.n_heads = 2, heads
+    from test_gpu_body_policy import cuda_body_policy
+    m = cuda_body_policy(cfg, bo.build_state_dict(cfg, 7))
+    obs = bo.make_obs(envs, cfg, 49, padded=True)
+    obs[4::7, -cfg.n_obj:] = 0.0                 # environments without a live object
+    obs[:, -1] = 0.0
+    obs[2::3, cfg.body_dim + cfg.n_obj * cfg.obj_dim - 1] = bad
+    obs = obs.cuda()
+    logits, value = m.forward_stacked(obs)
+    part = 18944 // (1 + cfg.n_obj)
+    for lo in range(0, min(envs, 4 * part), part):
+        l, v = m.forward_stacked(obs[lo:lo + part])
+        n = l.shape[0]
+        assert _same(l, logits[lo:lo + n]) and _same(v, value[lo:lo + n]), lo
+    assert bool(torch.isnan(logits[2]).any()) == (bad != 6e4)
+    assert native.lib.bsrl_device_status() == 0
 
 
 @pytest.mark.parametrize("kind", ["none", "all", "holes", "last", "runs"])
