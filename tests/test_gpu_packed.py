@@ -64,8 +64,8 @@ def test_sizes_around_the_line_and_pairs_of_ctas(envs):
 
 @pytest.mark.parametrize("name,opts", [("cfg1", {}), ("recipe", dict(value_residual=True)), ("cfg4", {})])
 def test_all_live_in_long_runs(name, opts):
-    """Long runs launch the attention kernels of both layouts: the full one's works where every slot is live, the other one where a
-    single one is not."""
+    """The attention kernel of packed rows works by tiles of four environments where every slot is live, and by rows where a single one
+    is not."""
     cfg = make_cfg(name, opts=dict(opts, n_blocks=2))
     m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
     obs = po.make_obs(2401, 47).cuda()
@@ -75,6 +75,22 @@ def test_all_live_in_long_runs(name, opts):
         for lo in range(0, 2401, 600):
             l, v = m.forward_stacked(obs[lo:lo + 600])
             assert torch.equal(l, logits[lo:lo + 600]) and torch.equal(v, value[lo:lo + 600]), (dead, lo)
+
+
+@pytest.mark.parametrize("envs", [575, 1001, 2401])
+def test_all_live_objects(native, envs):
+    cfg = bo.named_config("cfg2")
+    cfg.n_blocks = 2
+    from test_gpu_body_policy import cuda_body_policy
+    m = cuda_body_policy(cfg, bo.build_state_dict(cfg, 7))
+    obs = bo.make_obs(envs, cfg, 50).cuda()
+    for dead in (0, 1):
+        obs[400:400 + dead, -1] = 0.0
+        logits, value = m.forward_stacked(obs)
+        for lo in range(0, envs, 500):
+            l, v = m.forward_stacked(obs[lo:lo + 500])
+            assert torch.equal(l, logits[lo:lo + 500]) and torch.equal(v, value[lo:lo + 500]), (dead, lo)
+    assert native.lib.bsrl_device_status() == 0
 
 
 @pytest.mark.parametrize("name", ["cfg1", "recipe", "cfg4"])
