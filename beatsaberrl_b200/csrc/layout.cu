@@ -337,9 +337,16 @@ Paths plan_paths(const Layout& l, int engine, int64_t n_envs) {
   // 240; d 256 at 1 124 / 204, at 16 168 / 206, at 32 229 / 209.
   p.small = l.L >= 2 && p.attn_fused && p.tail_fused && p.enc_fused && !l.final_ln.width && n_envs <= small_envs(l);
   // Packed token rows from the first batch on whose full rows take more than one 128-row tile per SM: below, every kernel has
-  // one wave either way and the launches that lay the rows out come on top.  Packed / full, us, from the line on: rollouts of 696
-  // environments at d 64 131 / 141, of 1,024 at d 128 139 / 141, of 1,416 at d 64 251 / 259; evaluations of 5,003 at d 256 971 / 1,331.
-  p.packed = !p.small && p.attn_fused && (p.tail_fused || l.d > 256) && n_envs * kT > 148 * 128;
+  // one wave either way and the launches that lay the rows out come on top.  Narrow policies' kernels are as short as those launches:
+  // at d 64 from the third wave on, and at d 128 not where 17 of 29 rows (slots live in equal shares) are as many waves as all.
+  // Full / packed, us, evaluations behind a graph with 17 of 29 rows live, and with all:
+  //   d 64    900: 90 / 90, 90 / 99   1,200: 97 / 104, 97 / 108   1,400: 106 / 106, 107 / 118   2,048: 125 / 114, 126 / 139   8,192: 357 / 315, 358 / 372
+  //   d 128   654: 117 / 109, 117 / 127   1,050: 131 / 129, 131 / 145   1,200: 146 / 154, 146 / 161   2,048: 209 / 174, 209 / 228   8,192: 548 / 481, 548 / 577
+  //   d 192   654: 363 / 283, 363 / 384   1,200: 455 / 432, 455 / 476   2,048: 765 / 486, 765 / 844   8,192: 2,191 / 1,568, 2,198 / 2,198
+  //   d 256   654: 350 / 266, 350 / 369   1,200: 468 / 422, 468 / 491   2,048: 706 / 486, 707 / 755   8,192: 2,063 / 1,438, 2,070 / 2,080
+  const int64_t rows = n_envs * kT;
+  const bool no_wave_less = l.d <= 128 && rows <= 2 * kRowWave && (l.d < 128 || rows * 17 > kRowWave * 29);
+  p.packed = !p.small && p.attn_fused && (p.tail_fused || l.d > 256) && rows > kRowWave && !no_wave_less;
   return p;
 }
 

@@ -87,6 +87,10 @@ Layout make_layout(const bsrl_config& c);
 std::vector<ParamSlot> make_param_slots(const bsrl_config& c, const Layout& l);
 std::vector<CopySlot> make_copy_slots(const bsrl_config& c, const Layout& l, const std::vector<ParamSlot>& params);
 
+// Rows of one 128-row tile on each of the B200's 148 SMs.  A number and not sm_count(): layouts of save buffers and workspaces go by it,
+// and must not go by the device that is current.
+constexpr int64_t kRowWave = 148 * 128;
+
 // Which kernels a forward of this shape runs: the fused tcgen05 kernels where the widths fit them
 // (and the engine override allows), separate GEMM / LayerNorm / attention kernels otherwise.  The
 // workspace only holds the intermediates of the path taken.

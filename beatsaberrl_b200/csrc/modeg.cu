@@ -183,7 +183,7 @@ std::vector<CopySlot> g_copy_slots(const GLayout& l, const std::vector<ParamSlot
 // attention kernels that know the body token run, and from more than one 128-row tile per SM on.
 bool g_packed(const GLayout& l, int engine, int64_t n_envs) {
   const int dh = l.d / l.H;
-  return engine == 0 && l.d % 64 == 0 && (l.T == 17 || l.T == 33 || l.T == 65) && (dh == 32 || dh == 64) && n_envs * l.T > 148 * 128;
+  return engine == 0 && l.d % 64 == 0 && (l.T == 17 || l.T == 33 || l.T == 65) && (dh == 32 || dh == 64) && n_envs * l.T > kRowWave;
 }
 
 GWorkspace make_gws(const GLayout& l, int64_t B, bool tail_fused, bool attn_fused, bool packed) {

@@ -62,6 +62,17 @@ def test_sizes_around_the_line_and_pairs_of_ctas(envs):
         assert torch.equal(l, logits[lo:lo + 600]) and torch.equal(v, value[lo:lo + 600]), lo
 
 
+@pytest.mark.parametrize("name,envs", [("tiny", 1306), ("tiny", 1307), ("tiny", 2600), ("cfg1", 1114), ("cfg1", 1115), ("cfg1", 1306), ("cfg1", 1307)])
+def test_narrow_policies_around_their_lines(name, envs):
+    cfg = make_cfg(name, opts=dict(n_blocks=2))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
+    obs = po.make_obs(envs, 42, padded=True).cuda()
+    logits, value = m.forward_stacked(obs)
+    for lo in range(0, envs, 600):
+        l, v = m.forward_stacked(obs[lo:lo + 600])
+        assert torch.equal(l, logits[lo:lo + 600]) and torch.equal(v, value[lo:lo + 600]), lo
+
+
 @pytest.mark.parametrize("name,opts", [("cfg1", {}), ("recipe", dict(value_residual=True)), ("cfg4", {})])
 def test_all_live_in_long_runs(name, opts):
     """The attention kernel of packed rows works by tiles of four environments where every slot is live, and by rows where a single one
@@ -123,7 +134,7 @@ def test_dead_slots_that_fp16_cannot_hold(name, opts, bad, shows):
     row it shows all the same."""
     cfg = make_cfg(name, name == "recipe", opts=dict(dict(n_blocks=2), **opts))
     m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
-    envs = 1203
+    envs = 1403
     obs = po.make_obs(envs, 48, padded=True).cuda()
     obs[:, po.OFF_MASK + 22:po.OFF_MASK + 24] = 0.0
     for i, v in enumerate(bad):
