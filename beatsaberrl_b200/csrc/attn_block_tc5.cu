@@ -168,6 +168,13 @@ __device__ __forceinline__ void attend_tiles(const CUtensorMap& tm_h_, const CUt
   const int d = p.d, KB = d >> 6, n_groups = d / GD;
   volatile int* abort = &sh->abort;
   const uint32_t rank = PAIR ? cluster_rank() : 0u;
+  // work item: (tile, share of its head groups); both CTAs of a pair take the same number of tiles
+  const bool full = PACK && BOTH && counts.y == full_rows_in(p);      // every slot is live
+  const int n_tiles = PACK && !full ? counts.x : p.n_tiles;
+  const int t_end = PAIR ? (n_tiles + 1) & ~1 : (PACK && !full) ? n_tiles : n_tiles * p.split;
+  const int per_item = PAIR ? n_groups : (n_groups + p.split - 1) / p.split, log_split = PAIR ? 0 : __ffs(p.split) - 1;
+  auto tile_of = [&](int i) { return i >> log_split; };
+  auto first_group = [&](int i) { return (i & ((1 << log_split) - 1)) * per_item; };
   constexpr int CTAS = PAIR ? 2 : 1;
   auto commit = [&](uint64_t* bar) {                  // -> the barrier, in both CTAs of a pair
     if (PAIR) tc_commit_pair(smem_u32(bar));
@@ -214,13 +221,6 @@ __device__ __forceinline__ void attend_tiles(const CUtensorMap& tm_h_, const CUt
   // BY_ROW: packed rows with slots missing
   auto work = [&](auto by_row, const CUtensorMap& tm_h, const CUtensorMap& tm_o) {
     constexpr bool BY_ROW = decltype(by_row)::value;
-    // work item: (tile, share of its head groups); both CTAs of a pair take the same number of tiles
-    const int n_tiles = BY_ROW ? counts.x : p.n_tiles;
-    const int t_end = PAIR ? (n_tiles + 1) & ~1 : BY_ROW ? n_tiles : n_tiles * p.split;
-    const int per_item = PAIR ? n_groups : (n_groups + p.split - 1) / p.split, log_split = PAIR ? 0 : __ffs(p.split) - 1;
-    auto tile_of = [&](int i) { return i >> log_split; };
-    auto first_group = [&](int i) { return (i & ((1 << log_split) - 1)) * per_item; };
-
     if (warp == 0) {
       // ------------------------------------------------------------ TMA producer
       if (lane == 0) {
@@ -650,7 +650,7 @@ __device__ __forceinline__ void attend_tiles(const CUtensorMap& tm_h_, const CUt
     }
   };
   if constexpr (PACK && BOTH) {
-    if (counts.y == full_rows_in(p)) work(std::false_type(), full_h, full_o);
+    if (full) work(std::false_type(), full_h, full_o);
     else work(std::true_type(), tm_h_, tm_o_);
   } else {
     work(std::bool_constant<PACK>(), tm_h_, tm_o_);
