@@ -525,6 +525,7 @@ bool make_tmap_mn(CUtensorMap* map, const void* base, int64_t k_rows, int64_t co
   return true;
 }
 
+static bool counted(const LinearArgs& p) { return p.n_rows || p.cmap.start || p.rmap.start; }
 bool linear_tc5_ok(const LinearArgs& p) {
   if (!p.A || !p.W || !p.C || p.M < 1) return false;
   if (p.N % 16 != 0 || p.N < 16 || p.K < 1) return false;
@@ -537,6 +538,7 @@ bool linear_tc5_ok(const LinearArgs& p) {
   if (p.ldc % (p.out_f32 ? 4 : 8)) return false;
   if (p.bias && !aligned16(p.bias)) return false;
   if (p.R && (!aligned16(p.R) || (p.ldr % 4))) return false;
+  if (p.relu == 2 && p.out_f32 && counted(p)) return false;      // GELU of fp32 results: kernels without a count
   if (p.k_splits > 1 && (!p.out_f32 || p.relu || p.R || p.mask)) return false;   // split-K adds raw fp32 partial products
   if (p.mask && (!aligned16(p.mask) || (p.ldm % 8) || p.cmap.group != 0x7fffffff || p.cmap.first != 0)) return false;
   return true;
@@ -590,8 +592,7 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
     cudaError_t e = cudaSuccess;
     for (auto* k : {linear_tc5_kernel<false, false>, linear_tc5_kernel<true, false>, linear_tc5_kernel<false, true>,
                     linear_tc5_kernel<false, false, true>, linear_tc5_kernel<true, false, true>,
-                    linear_tc5_kernel<false, false, false, true>, linear_tc5_kernel<true, false, false, true>, linear_tc5_kernel<false, true, false, true>,
-                    linear_tc5_kernel<false, false, true, true>, linear_tc5_kernel<true, false, true, true>})
+                    linear_tc5_kernel<false, false, false, true>, linear_tc5_kernel<true, false, false, true>, linear_tc5_kernel<false, true, false, true>})
       if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
     return e;
   });
@@ -604,15 +605,14 @@ int linear_tc5(const LinearArgs& p_in, cudaStream_t stream) {
   }
   int64_t grid = m_tiles * n_tiles * (p.k_splits > 1 ? p.k_splits : 1);
   if (grid > sm_count()) grid = sm_count();
-  const bool gelu32 = p.relu == 2 && p.out_f32;
   auto pick = [&](auto count) {
     constexpr bool COUNT = decltype(count)::value;
-    return p.a_sums ? linear_tc5_kernel<false, true, false, COUNT>
-           : gelu32 ? (p.R ? linear_tc5_kernel<true, false, true, COUNT> : linear_tc5_kernel<false, false, true, COUNT>)
-           : p.R    ? linear_tc5_kernel<true, false, false, COUNT>
-                    : linear_tc5_kernel<false, false, false, COUNT>;
+    return p.a_sums ? linear_tc5_kernel<false, true, false, COUNT> : p.R ? linear_tc5_kernel<true, false, false, COUNT> : linear_tc5_kernel<false, false, false, COUNT>;
   };
-  auto* kernel = p.n_rows || p.cmap.start || p.rmap.start ? pick(std::true_type()) : pick(std::false_type());
+  const bool gelu32 = p.relu == 2 && p.out_f32;            // (not of counted rows: linear_tc5_ok)
+  auto* kernel = gelu32      ? (p.R ? linear_tc5_kernel<true, false, true> : linear_tc5_kernel<false, false, true>)
+                 : counted(p) ? pick(std::true_type())
+                              : pick(std::false_type());
   launch_kernel(kernel, (unsigned)grid, THREADS, SMEM_BYTES, stream, tm_a, tm_w, tm_c, tma_c ? 1 : 0, p, (int)m_tiles, n_tiles, status);
   BSRL_LAUNCH_OK("linear_tc5_kernel");
   return BSRL_OK;
