@@ -28,10 +28,18 @@ const char* const kStageNames[kStCount] = {"embed_gather", "encoder_gemm", "enco
                                            "trunk", "critic", "head_tail"};
 struct Profiler {
   bool on = false;
-  struct Rec { int stage; cudaEvent_t e0, e1; double flops, bytes; };
+  struct Rec {
+    int stage;
+    cudaEvent_t e0, e1;
+    double flops, bytes;
+    Counted rows;
+    const int* count;        // rows.n_rows' value behind the launch, or nullptr
+  };
+  static constexpr size_t kBlock = 4096;
   std::vector<Rec> recs;
   std::vector<cudaEvent_t> pool;
-  size_t used = 0;
+  std::vector<int*> slots;   // page-locked, kBlock each: where the counts land
+  size_t used = 0, used_slots = 0;
   cudaEvent_t get() {
     if (used == pool.size()) {
       cudaEvent_t e;
@@ -40,7 +48,16 @@ struct Profiler {
     }
     return pool[used++];
   }
-  void reset() { recs.clear(); used = 0; }
+  int* slot() {
+    if (used_slots == slots.size() * kBlock) {
+      void* p;
+      if (cudaHostAlloc(&p, kBlock * sizeof(int), cudaHostAllocPortable) != cudaSuccess) return nullptr;
+      slots.push_back(static_cast<int*>(p));
+    }
+    const size_t i = used_slots++;
+    return slots[i / kBlock] + i % kBlock;
+  }
+  void reset() { recs.clear(); used = used_slots = 0; }
 };
 // Per host thread: each thread that enables the profiler times its own forwards, and forwards
 // running on other threads are not affected.
@@ -53,15 +70,18 @@ double linear_bytes(const LinearArgs& p) {
   return b;
 }
 
+// flops, bytes: of the host's number of rows; rows: how many of them the device counts
 template <typename Fn>
-int timed(cudaStream_t st, double flops, double bytes, Fn&& fn) {
+int timed(cudaStream_t st, double flops, double bytes, Fn&& fn, const Counted& rows = Counted()) {
   if (!g_prof.on) return fn();
   cudaEvent_t e0 = g_prof.get(), e1 = g_prof.get();
   if (!e0 || !e1) return fn();
   cudaEventRecord(e0, st);
   int rc = fn();
   cudaEventRecord(e1, st);
-  g_prof.recs.push_back({g_stage, e0, e1, flops, bytes});
+  int* count = rows.n_rows ? g_prof.slot() : nullptr;
+  if (count && cudaMemcpyAsync(count, rows.n_rows, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess) count = nullptr;
+  g_prof.recs.push_back({g_stage, e0, e1, flops, bytes, rows, count});
   return rc;
 }
 
@@ -87,7 +107,7 @@ int linear(const LinearArgs& p, cudaStream_t st) {
     if (g_call_engine == 0 && linear_small_wins(p)) return linear_small(p, st);
     if (g_call_engine == 0 && p.M >= 128 && linear_tc5_ok(p)) return linear_tc5(p, st);
     return linear_mma(p, st);
-  });
+  }, Counted{p.n_rows, p.n_less, p.a_mn ? (int64_t)p.K : p.M, p.a_mn ? (double)p.M * p.N * 4 : (double)p.N * p.K * 2});
 }
 // two products that do not depend on each other: one launch where both are small
 int linear_two(const LinearArgs& p, const LinearArgs& q, cudaStream_t st) {
@@ -102,7 +122,7 @@ int layernorm(const float* x, int64_t ldx, RowMap xmap, const float* g, const fl
               int64_t rows, int d, __half* y, int64_t ldy, cudaStream_t st, const int* n_rows) {
   int keep = g_stage;
   if (g_stage != kStTrunk && g_stage != kStCritic) g_stage = kStLayerNorm;
-  int rc = timed(st, 0.0, (double)rows * d * 6, [&] { return layernorm_rows(x, ldx, xmap, g, b, eps, rows, d, y, ldy, st, n_rows); });
+  int rc = timed(st, 0.0, (double)rows * d * 6, [&] { return layernorm_rows(x, ldx, xmap, g, b, eps, rows, d, y, ldy, st, n_rows); }, Counted{n_rows, 0, rows});
   g_stage = keep;
   return rc;
 }
@@ -112,7 +132,8 @@ int attention(const __half* qkv, int ld, const float* kb, int64_t B, int d, int 
   if (g_stage != kStCritic) g_stage = kStAttention;
   double fl = 4.0 * B * nq * kT * d;
   double by = (double)B * (kT * 2 * d + nq * d * 2) * 2 + (double)B * kT * 4;
-  int rc = timed(st, fl, by, [&] { return attention29(qkv, ld, kb, B, d, H, q0, nq, out, ldo, st, start); });
+  int rc = timed(st, fl, by, [&] { return attention29(qkv, ld, kb, B, d, H, q0, nq, out, ldo, st, start); },
+                 Counted{start ? start + B : nullptr, 0, B * kT, 0.0, nq == kT ? fl : 0.0});
   g_stage = keep;
   return rc;
 }
@@ -121,14 +142,16 @@ void begin_overlap(int64_t rows) {
   if (!g_prof.on && rows <= 8 * 128 * (int64_t)sm_count()) pdl_enable();
 }
 void set_stage(int stage) { g_stage = stage; }
-int timed_call(cudaStream_t st, double flops, double bytes, const std::function<int()>& fn) { return timed(st, flops, bytes, fn); }
+int timed_call(cudaStream_t st, double flops, double bytes, const std::function<int()>& fn, const Counted& rows) {
+  return timed(st, flops, bytes, fn, rows);
+}
 
 int fused_tail(const BlockTailArgs& a, cudaStream_t st) {
   int keep = g_stage;
   g_stage = kStBlockTail;
   double fl = 2.0 * a.M * ((double)a.d * a.d + 2.0 * a.d * a.F);
   double by = (double)a.M * a.d * (2 + 4 + (a.x_out ? 4 : 0) + (a.out16[0] ? 2 : 0) + (a.out16[1] ? 2 : 0));
-  int rc = timed(st, fl, by, [&] { return block_tail(a, st); });
+  int rc = timed(st, fl, by, [&] { return block_tail(a, st); }, Counted{a.n_rows, 0, a.M});
   g_stage = keep;
   return rc;
 }
@@ -140,7 +163,7 @@ int out_proj_ln(const LinearLnArgs& a, cudaStream_t st) {
   g_stage = kStOutProj;
   int rc;
   if (g_call_engine == 0 && a.N > 256 && a.M >= 128 && linear_ln_ok(a)) {
-    rc = timed(st, 2.0 * a.M * a.N * a.K, (double)a.M * (a.K * 2 + a.N * 10.0), [&] { return linear_ln(a, st); });
+    rc = timed(st, 2.0 * a.M * a.N * a.K, (double)a.M * (a.K * 2 + a.N * 10.0), [&] { return linear_ln(a, st); }, Counted{a.n_rows, 0, a.M});
   } else {
     LinearArgs po = linear_args(a.A, a.lda, a.W, a.ldw, a.bias, a.x_out, (int)a.ldx, 1, 0, a.M, a.N, a.K);
     po.R = a.R; po.ldr = (int)a.ldr;
@@ -157,9 +180,10 @@ int fused_attn(const AttnBlockArgs& a, cudaStream_t st) {
   g_stage = kStAttnBlock;
   const int tokens = a.body ? a.tokens : kT;
   const double rows = (double)a.n_envs * tokens;
-  double fl = 2.0 * rows * 3.0 * a.d * a.d + 4.0 * a.n_envs * a.n_q * tokens * a.d;
+  const double scores = 4.0 * a.n_envs * a.n_q * tokens * a.d;
+  double fl = 2.0 * rows * 3.0 * a.d * a.d + scores;
   double by = rows * a.d * 2 + (double)a.n_envs * a.n_q * a.d * 2 + (double)a.n_envs * tokens * 4;
-  int rc = timed(st, fl, by, [&] { return attn_block(a, st); });
+  int rc = timed(st, fl, by, [&] { return attn_block(a, st); }, Counted{a.rows.n_rows(), 0, (int64_t)rows, 0.0, a.n_q == tokens ? scores : 0.0});
   g_stage = keep;
   return rc;
 }
@@ -188,8 +212,10 @@ int run_embed(const Ctx& c, const void* obs, int obs_dtype, float* x, float* key
     BSRL_TRY(timed(c.st, 0.0, (double)B * (kSlots + 1) * 4, [&] { return token_rows(src, B, c.rows, c.st); }));
     begin_overlap(B * kT);       // the tokenizer's launch under the count
   }
-  BSRL_TRY(timed(c.st, 0.0, (double)B * (kObs * 4 + (2 * kSaberK + kTorsoK + 2 * kLegK + kSlots * l.note_k) * 2 + kT * 4),
-                 [&] { return embed_gather(obs, obs_dtype, B, c.cfg->note_geo, c.cfg->game_flux, c.cfg->z_asinh, eb, c.st); }));
+  const double lead_bytes = (double)B * (kObs * 4 + (2 * kSaberK + kTorsoK + 2 * kLegK) * 2 + kT * 4);
+  BSRL_TRY(timed(c.st, 0.0, lead_bytes + (double)B * kSlots * l.note_k * 2,
+                 [&] { return embed_gather(obs, obs_dtype, B, c.cfg->note_geo, c.cfg->game_flux, c.cfg->z_asinh, eb, c.st); },
+                 Counted{c.n_rows(), kLead * B, kSlots * B, lead_bytes}));
   if (have_h) *have_h = false;
   begin_overlap(B * kT);
   if (c.paths.enc_fused) {
@@ -208,7 +234,7 @@ int run_embed(const Ctx& c, const void* obs, int obs_dtype, float* x, float* key
     g_stage = kStEncoderFused;
     const double rows = (double)B * kT;
     BSRL_TRY(timed(c.st, 2.0 * rows * d * (64 + d), rows * (128 + 4.0 * d + (h_out ? 2.0 * d : 0.0)),
-                   [&] { return encoder_fused(ea, c.st); }));
+                   [&] { return encoder_fused(ea, c.st); }, Counted{c.n_rows(), 0, B * kT}));
     if (have_h) *have_h = h_out != nullptr;
     return BSRL_OK;
   }
@@ -240,7 +266,7 @@ int run_embed(const Ctx& c, const void* obs, int obs_dtype, float* x, float* key
     g_stage = kStLayerNorm;
     BSRL_TRY(timed(c.st, 0.0, (double)B * kT * d * 8, [&] {
       return layernorm_rows_f32(x, d, c.G(l.emb_ln), c.Be(l.emb_ln), c.cfg->eps, B * kT, d, x, d, c.st, c.n_rows());
-    }));
+    }, Counted{c.n_rows(), 0, B * kT}));
   }
   return BSRL_OK;
 }
@@ -1039,7 +1065,11 @@ int bsrl_profile_stage(int32_t i, double* ms_total, int64_t* launches, double* f
     float t = 0.f;
     cudaError_t e = cudaEventElapsedTime(&t, r.e0, r.e1);
     if (e != cudaSuccess) return cuda_fail(e, "cudaEventElapsedTime (synchronise the stream before reading the profile)");
-    ms += t; fl += r.flops; by += r.bytes; ++n;
+    // what the device's count left of the host's rows
+    const double share = r.count ? (double)(*r.count - r.rows.less) / (double)r.rows.bound : 1.0;
+    fl += (r.flops - r.rows.square_flops) * share + r.rows.square_flops * share * share;
+    by += r.rows.fixed_bytes + (r.bytes - r.rows.fixed_bytes) * share;
+    ms += t; ++n;
   }
   if (ms_total) *ms_total = ms;
   if (launches) *launches = n;

@@ -107,7 +107,15 @@ enum Stage { kStGather = 0, kStEncoder, kStEncoderFused, kStLayerNorm, kStQkv, k
 // update (the waiting successors take the SMs' memory pipes and cache lines from a predecessor that still needs them).
 void begin_overlap(int64_t rows);
 void set_stage(int stage);            // label of the launches that follow on this thread
-int timed_call(cudaStream_t st, double flops, double bytes, const std::function<int()>& fn);
+// The stage profiler's view of packed token rows: a launch's rows by the device's count (less `less`) of the host's `bound`.  Its FLOPs and
+// bytes go with them, fixed_bytes apart; square_flops, the scores of all rows against all, with their square (as if every
+// environment had the average number).
+struct Counted {
+  const int* n_rows = nullptr;
+  int64_t less = 0, bound = 1;
+  double fixed_bytes = 0.0, square_flops = 0.0;
+};
+int timed_call(cudaStream_t st, double flops, double bytes, const std::function<int()>& fn, const Counted& rows = Counted());
 int fused_tail(const BlockTailArgs& a, cudaStream_t st);
 int fused_attn(const AttnBlockArgs& a, cudaStream_t st);
 int out_proj_ln(const LinearLnArgs& a, cudaStream_t st);

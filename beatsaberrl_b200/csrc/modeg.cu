@@ -339,7 +339,7 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
                   f_obj, key_bias, rows, parts);
     BSRL_LAUNCH_OK("embed_g_kernel");
     return BSRL_OK;
-  }));
+  }, Counted{rows.n_rows(), B, B * l.n_obj, (double)B * (l.obs_dim * 4 + l.body_k * 2 + T * 4)}));
   begin_overlap(B * l.T);
   set_stage(kStEncoder);
   {
@@ -386,7 +386,8 @@ int g_forward(const GCtx& c, const float* obs, const HeadTailArgs& tail_in) {
   auto attend = [&](int n_q) -> int {        // masked attention of n_q query rows per env over its T tokens
     set_stage(kStAttention);
     return timed_call(st, 4.0 * B * n_q * T * d, (double)B * (T * 2 * d + n_q * d * 2) * 2 + (double)B * T * 4,
-                      [&]() -> int { return attention_tokens(qkv, 3 * d, key_bias, B, T, d, l.H, 0, n_q, att, d, st, rows.start); });
+                      [&]() -> int { return attention_tokens(qkv, 3 * d, key_bias, B, T, d, l.H, 0, n_q, att, d, st, rows.start); },
+                      Counted{rows.n_rows(), 0, B * T, 0.0, n_q == T ? 4.0 * B * n_q * T * d : 0.0});
   };
   bool have_h = false;
   for (int i = 0; i + 1 < l.L; ++i) {

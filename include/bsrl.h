@@ -448,7 +448,8 @@ int bsrl_device_status(void);
 
 /* --- stage timing (benchmarks) ------------------------------------------------------- *
  * When enabled, every launch of a forward is bracketed by CUDA events on the caller's stream
- * and accounted to a stage ("ffn_down_gemm", "attention", ...).  Enabling clears earlier
+ * and accounted to a stage ("ffn_down_gemm", "attention", ...).  flops_total and bytes_total are of the rows that were
+ * computed: in batches that keep rows of live slots only, of as many as the device counted.  Enabling clears earlier
  * records.  Read the totals after synchronising the stream.  Leave it off while capturing a
  * CUDA graph.  Counterpart in the reference: the per-tick CUDA-event timers of its --bench
  * mode (python/train_batch.py:2120-2124, :2309-2352). */

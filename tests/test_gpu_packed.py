@@ -120,6 +120,29 @@ def test_not_a_number_stays_in_its_environment(name):
     assert torch.isnan(logits[bad]).any(-1).any(-1).all()
 
 
+@pytest.mark.parametrize("name,envs", [("cfg1", 1403), ("cfg4", 701), ("cfg1", 300)])
+def test_stage_profile_counts_the_rows_that_there_are(native, name, envs):
+    cfg = make_cfg(name, opts=dict(n_blocks=2))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
+    obs = po.make_obs(envs, 51, padded=True).cuda()
+    m.forward_stacked(obs)
+    native.check(native.lib.bsrl_profile_enable(1))
+    m.forward_stacked(obs)
+    torch.cuda.synchronize()
+    stages = native.profile_read()
+    native.check(native.lib.bsrl_profile_enable(0))
+    d, F = cfg.embed, cfg.embed * cfg.ffn_mult
+    # (the full layout's kernels compute the dead slots' rows too)
+    rows = envs * 29 if envs < 654 else 5 * envs + int(obs[:, po.OFF_MASK:po.OFF_MASK + 24].sum())
+    close = lambda a, b: abs(a - b) <= 1e-9 * b
+    if name == "cfg4":
+        assert close(stages["ffn_up_gemm"]["flops"], 2 * (rows + 5 * envs) * d * F)
+        assert close(stages["ffn_down_gemm"]["bytes"], (rows + 5 * envs) * F * 2 + 2 * d * F * 2 + rows * d * 8 + 5 * envs * d * 6)
+    else:
+        assert close(stages["block_tail"]["flops"], 2 * (rows + 5 * envs) * (d * d + 2 * d * F))
+        assert close(stages["encoder_fused"]["flops"], 2 * rows * d * (64 + d))
+
+
 def _same(a, b):
     """The same bits, and not a number in the same places."""
     return torch.equal(torch.isnan(a), torch.isnan(b)) and torch.equal(a.nan_to_num(nan=0.0), b.nan_to_num(nan=0.0))
