@@ -1166,7 +1166,8 @@ int bsrl_workspace_region(const bsrl_config* cfg, int64_t n_envs, const char* na
   int32_t dt = BSRL_F16;
   if (!strcmp(name, "trunk_h")) { off = w.z + (int64_t)l.d * 2; r = n_envs; cc = l.D; ld = l.d + l.D; }
   else if (!strcmp(name, "x_resolved") && paths.packed) {
-    set_error("workspace_region: a batch of %lld environments keeps rows of live slots only: ask for 'x_packed' and 'row_start'", (long long)n_envs);
+    set_error("workspace_region: a batch of %lld environments keeps rows of live slots only: ask for 'x_packed' and 'row_start', or run it in slices "
+              "of fewer", (long long)n_envs);
     return BSRL_ERR_UNSUPPORTED;
   }
   else if (paths.packed && !strcmp(name, "x_packed")) { off = w.x; r = n_envs * kT; cc = l.d; ld = l.d; dt = BSRL_F32; }

@@ -410,9 +410,13 @@ int bsrl_head_layout(const bsrl_config* cfg, int32_t* head_cols_pad, int32_t* bi
 /* Where a named intermediate of the last forward sits in the caller's workspace (valid until the next
  * call on that workspace): "trunk_h" (the reference's _diag_h), "x_resolved" (the residual stream
  * entering the last block, the critic's input; python/policy.py:1302-1305), "key_bias", "readout",
- * "head_out".  dtype is a bsrl_dtype; ld_elems the row pitch in elements.  Batches of more than 18,944 token rows keep
- * rows only for an environment's lead tokens and its slots up to the last live one, environment after environment; there
- * the stream is "x_packed", and "row_start" (n_envs + 1, int32) says where an environment's rows begin. */
+ * "head_out".  dtype is a bsrl_dtype; ld_elems the row pitch in elements.
+ *
+ * Large batches on the default engine keep rows only for an environment's lead tokens and its slots up to the last live
+ * one, environment after environment.  Which do follows from the shape and the batch (the size from which it pays); ask for
+ * "row_start" (n_envs + 1, int32): where an environment's rows begin in "x_packed", the stream of such a batch.  Where that
+ * is refused (BSRL_ERR_UNSUPPORTED) the stream is "x_resolved", 29 rows for every environment, and the other way round.
+ * Rows of slots behind the last live one do not exist then; batches below 18,944 / 29 environments compute them. */
 int bsrl_workspace_region(const bsrl_config* cfg, int64_t n_envs, const char* name, int64_t* byte_offset,
                           int64_t* rows, int64_t* cols, int64_t* ld_elems, int32_t* dtype);
 
@@ -437,7 +441,8 @@ int bsrl_selftest_wait_timeout(int32_t polls, void* stream);
  * 1 = the warp-MMA kernel and separate LayerNorm kernels everywhere.
  * Both are CUDA kernels of this library; 1 exists so tests can cross-check one against the
  * other.  The choice is process-wide: set it before the first forward and before asking for
- * bsrl_workspace_bytes (the unfused kernels need more workspace).  No counterpart in the reference. */
+ * bsrl_workspace_bytes (the unfused kernels need more workspace).  A save buffer of bsrl_forward_train reads the same on
+ * either.  No counterpart in the reference. */
 int bsrl_set_engine(int32_t engine);
 
 /* Synchronises the current device, then reads and clears its status word: BSRL_OK, or

@@ -1,6 +1,8 @@
 """Packed token rows: batches past 18,944 token rows give rows only to each environment's slots up to its last live one.  The same
 environments in slices of a few hundred take the full layout: forwards must agree bit for bit, gradients up to the order of fp32
 sums, whatever the masks are."""
+import ctypes as C
+
 import pytest
 import torch
 
@@ -118,6 +120,41 @@ def test_not_a_number_stays_in_its_environment(name):
     good[bad] = False
     assert torch.equal(logits[good], clean_l[good]) and torch.equal(value[good], clean_v[good])
     assert torch.isnan(logits[bad]).any(-1).any(-1).all()
+
+
+def _region(native, m, envs, name):
+    """A named intermediate of the last forward, or None where the batch has none of that name."""
+    off, rows, cols, ld, dt = C.c_int64(), C.c_int64(), C.c_int64(), C.c_int64(), C.c_int32()
+    rc = native.lib.bsrl_workspace_region(C.byref(m._cfg), envs, name, C.byref(off), C.byref(rows), C.byref(cols), C.byref(ld), C.byref(dt))
+    if rc:
+        return None
+    ws = m._workspaces[(envs, m.critic_q.weight.device)][0]
+    kind = {native.F32: torch.float32, native.I32: torch.int32}[dt.value]
+    assert cols.value == ld.value
+    return ws[off.value:off.value + rows.value * cols.value * 4].view(kind).view(rows.value, cols.value).clone()
+
+
+@pytest.mark.parametrize("kind", ["none", "holes"])
+@pytest.mark.parametrize("name,envs", [("cfg1", 1403), ("recipe", 701), ("cfg4", 701), ("recipe", 4700)])
+def test_stream_regions(native, name, envs, kind):
+    """x_packed laid out by row_start is x_resolved of the same environments below the line; each batch has one of the two."""
+    cfg = make_cfg(name, name == "recipe", opts=dict(n_blocks=3))
+    m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
+    obs = _obs(kind, envs, 52).cuda()
+    m.forward_stacked(obs)
+    x, start = _region(native, m, envs, b"x_packed"), _region(native, m, envs, b"row_start")
+    assert _region(native, m, envs, b"x_resolved") is None
+    mask = obs[:, po.OFF_MASK:po.OFF_MASK + 24] > 0
+    rows = 5 + torch.where(mask.any(1), 24 - mask.flip(1).float().argmax(1), 0)
+    assert torch.equal(start.view(-1).long(), torch.cat([rows.new_zeros(1), rows.cumsum(0)]))
+    for lo in range(0, envs, 500):
+        part = obs[lo:lo + 500]
+        m.forward_stacked(part)
+        n = part.shape[0]
+        assert _region(native, m, n, b"x_packed") is None and _region(native, m, n, b"row_start") is None
+        full = _region(native, m, n, b"x_resolved").view(n, 29, -1)
+        there = torch.arange(29, device="cuda")[None, :] < rows[lo:lo + n, None]
+        assert torch.equal(full[there], x[int(start[lo]):int(start[lo + n])]), lo
 
 
 @pytest.mark.parametrize("name,envs", [("cfg1", 1403), ("cfg4", 701), ("cfg1", 300)])
