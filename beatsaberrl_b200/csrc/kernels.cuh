@@ -241,7 +241,8 @@ struct AttnBlockArgs {
   // n_q = 1: the body row only, out (n_envs, ldo).
   int body = 0, tokens = 29;
   const __half* qkv0 = nullptr;
-  TokenRows rows;            // packed token rows (start: nullptr: 29 per environment); key_bias then goes unread
+  TokenRows rows;            // packed token rows (start: nullptr: 29 per environment); rows.kb then is the key bias, and key_bias
+                             // where every slot is live
 };
 // The same for few environments (attn_small.cu): one CTA per environment and head group, up to two problems over the
 // same environments in a launch.  The rows come as fp16 (h) or are LayerNormed from fp32 (norm.x set; dense rows).
