@@ -772,7 +772,10 @@ int attn_block(const AttnBlockArgs& a, cudaStream_t stream) {
     return !out_tma || make_tmap_rows(&m.o, a.out + ahead * a.ldo, 2, bound, a.d, a.ldo, 32, cols * 2);
   };
   if (!make_tmap_f16(&m.w, a.wg, 3 * a.d, a.d, a.d, dh == 48 ? 144 : pair ? 96 : 192)) return BSRL_ERR_CUDA;
-  if (pack ? !packed_maps() || !full_maps(&m.full_h, &m.full_o) : !full_maps(&m.h, &m.o)) return BSRL_ERR_CUDA;
+  if (pack ? !packed_maps() : !full_maps(&m.h, &m.o)) return BSRL_ERR_CUDA;
+  m.full_h = m.h;
+  m.full_o = m.o;
+  if (pack && longer && !full_maps(&m.full_h, &m.full_o)) return BSRL_ERR_CUDA;      // (an encoding is 0.3 us of the host's time)
   static DeviceOnce once;
   int rc = once.run("attn_block_kernel set-up", [] {
     cudaError_t e = prepare<32, 2, false, false>();
