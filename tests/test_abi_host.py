@@ -70,6 +70,35 @@ def test_a_workspace_serves_every_smaller_batch(native, name, geo, opts):
     assert sizes[0] >= 0 and all(a <= b for a, b in zip(sizes, sizes[1:]))
 
 
+@pytest.mark.parametrize("name,lines", [("tiny", [1306]), ("cfg1", [653, 1114, 1306]), ("recipe", [653]), ("cfg2", [653]), ("cfg4", [653])])
+def test_every_batch_has_one_form_of_the_stream(native, name, lines):
+    """29 rows per environment below each line and packed rows above it, or the other way round: one of the two, inside the workspace, the
+    row table beside the rows; the warp-MMA engine packs nothing."""
+    c = _cfg(native, make_cfg(name, name == "recipe"))
+
+    def region(n, what):
+        off, rows, cols, ld, dt = C.c_int64(), C.c_int64(), C.c_int64(), C.c_int64(), C.c_int32()
+        rc = native.lib.bsrl_workspace_region(C.byref(c), n, what, C.byref(off), C.byref(rows), C.byref(cols), C.byref(ld), C.byref(dt))
+        assert rc in (0, -5), rc
+        if rc:
+            return None
+        end = off.value + rows.value * ld.value * 4
+        assert end <= native.lib.bsrl_workspace_bytes(C.byref(c), n)
+        return off.value, end
+
+    packed = False
+    for n in [1, 100] + [n for line in lines for n in (line, line + 1)] + [4096, 4097, 65536]:
+        packed ^= n - 1 in lines
+        full, x, start = (region(n, what) for what in (b"x_resolved", b"x_packed", b"row_start"))
+        if packed:
+            assert full is None and (start[1] <= x[0] or x[1] <= start[0]), n
+        else:
+            assert x is None and start is None and full is not None, n
+        native.lib.bsrl_set_engine(1)
+        assert region(n, b"x_resolved") is not None and region(n, b"x_packed") is None
+        native.lib.bsrl_set_engine(0)
+
+
 def test_config_errors_are_reported(native):
     good = make_cfg("cfg1")
     c = _cfg(native, good)
