@@ -337,16 +337,20 @@ Paths plan_paths(const Layout& l, int engine, int64_t n_envs) {
   // 240; d 256 at 1 124 / 204, at 16 168 / 206, at 32 229 / 209.
   p.small = l.L >= 2 && p.attn_fused && p.tail_fused && p.enc_fused && !l.final_ln.width && n_envs <= small_envs(l);
   // Packed token rows from the first batch on whose full rows take more than one 128-row tile per SM: below, every kernel has
-  // one wave either way and the launches that lay the rows out come on top.  Narrow policies' kernels are as short as those launches:
-  // at d 64 from the third wave on, and at d 128 not where 17 of 29 rows (slots live in equal shares) are as many waves as all.
-  // Full / packed, us, evaluations behind a graph with 17 of 29 rows live, and with all:
-  //   d 64    900: 90 / 90, 90 / 99   1,200: 97 / 104, 97 / 108   1,400: 106 / 106, 107 / 118   2,048: 125 / 114, 126 / 139   8,192: 357 / 315, 358 / 372
-  //   d 128   654: 117 / 109, 117 / 127   1,050: 131 / 129, 131 / 145   1,200: 146 / 154, 146 / 161   2,048: 209 / 174, 209 / 228   8,192: 548 / 481, 548 / 577
-  //   d 192   654: 363 / 283, 363 / 384   1,200: 455 / 432, 455 / 476   2,048: 765 / 486, 765 / 844   8,192: 2,191 / 1,568, 2,198 / 2,198
-  //   d 256   654: 350 / 266, 350 / 369   1,200: 468 / 422, 468 / 491   2,048: 706 / 486, 707 / 755   8,192: 2,063 / 1,438, 2,070 / 2,080
+  // one wave either way and the launches that lay the rows out come on top.  Up to d 128 the kernels are short enough for that to show
+  // in the second wave too: not where 17 of 29 rows (slots live in equal shares) are as many waves as all, and not for so few blocks
+  // that the wave they save is no longer than the count.  Full / packed, us, evaluations behind a graph with 17 of 29 rows live, and with all:
+  //   d 64, 2 blocks    900: 88 / 90, 88 / 98   1,200: 97 / 104, 97 / 107   1,400: 106 / 105, 107 / 118   2,048: 125 / 114, 126 / 139
+  //         3 blocks    900: 111 / 107, 111 / 122   1,200: 121 / 127, 121 / 133   1,400: 136 / 129, 136 / 150
+  //         6 blocks    660: 168 / 149, 167 / 181   1,100: 186 / 166, 186 / 202   1,200: 192 / 197, 192 / 210   1,400: 227 / 201, 227 / 246
+  //   d 128, 2 blocks   654: 117 / 109, 117 / 127   1,100: 135 / 132, 135 / 148   1,200: 146 / 153, 147 / 160   2,048: 209 / 174, 209 / 228
+  //          6 blocks   660: 254 / 204, 255 / 275   1,200: 303 / 310, 303 / 331   1,400: 368 / 315, 368 / 397
+  //   d 192, 6 blocks   654: 363 / 283, 363 / 384   1,200: 455 / 432, 455 / 476   2,048: 765 / 486, 765 / 844   8,192: 2,191 / 1,568, 2,198 / 2,198
+  //   d 256, 4 blocks   654: 350 / 266, 350 / 369   1,200: 468 / 422, 468 / 491   2,048: 706 / 486, 707 / 755   8,192: 2,063 / 1,438, 2,070 / 2,080
   const int64_t rows = n_envs * kT;
-  const bool no_wave_less = l.d <= 128 && rows <= 2 * kRowWave && (l.d < 128 || rows * 17 > kRowWave * 29);
-  p.packed = !p.small && p.attn_fused && (p.tail_fused || l.d > 256) && rows > kRowWave && !no_wave_less;
+  const bool second_wave = rows <= 2 * kRowWave, no_wave_less = rows * 17 > kRowWave * 29;
+  const bool too_short = second_wave && (l.d * l.L <= 128 || (l.d <= 128 && no_wave_less));
+  p.packed = !p.small && p.attn_fused && (p.tail_fused || l.d > 256) && rows > kRowWave && !too_short;
   return p;
 }
 

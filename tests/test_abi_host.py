@@ -70,11 +70,12 @@ def test_a_workspace_serves_every_smaller_batch(native, name, geo, opts):
     assert sizes[0] >= 0 and all(a <= b for a, b in zip(sizes, sizes[1:]))
 
 
-@pytest.mark.parametrize("name,lines", [("tiny", [1306]), ("cfg1", [653, 1114, 1306]), ("recipe", [653]), ("cfg2", [653]), ("cfg4", [653])])
-def test_every_batch_has_one_form_of_the_stream(native, name, lines):
+@pytest.mark.parametrize("name,blocks,lines", [("tiny", 2, [1306]), ("tiny", 3, [653, 1114, 1306]), ("cfg1", 1, [1306]), ("cfg1", 2, [653, 1114, 1306]),
+                                               ("recipe", 6, [653]), ("cfg2", 1, [653]), ("cfg4", 6, [653])])
+def test_every_batch_has_one_form_of_the_stream(native, name, blocks, lines):
     """29 rows per environment below each line and packed rows above it, or the other way round: one of the two, inside the workspace, the
     row table beside the rows; the warp-MMA engine packs nothing."""
-    c = _cfg(native, make_cfg(name, name == "recipe"))
+    c = _cfg(native, make_cfg(name, name == "recipe", opts=dict(n_blocks=blocks)))
 
     def region(n, what):
         off, rows, cols, ld, dt = C.c_int64(), C.c_int64(), C.c_int64(), C.c_int64(), C.c_int32()

@@ -100,9 +100,10 @@ def test_a_captured_graph_counts_anew(name, envs):
     m.check_device()
 
 
-@pytest.mark.parametrize("name,envs", [("tiny", 1306), ("tiny", 1307), ("tiny", 2600), ("cfg1", 1114), ("cfg1", 1115), ("cfg1", 1306), ("cfg1", 1307)])
-def test_narrow_policies_around_their_lines(name, envs):
-    cfg = make_cfg(name, opts=dict(n_blocks=2))
+@pytest.mark.parametrize("name,blocks,envs", [("tiny", 2, 1306), ("tiny", 2, 1307), ("tiny", 2, 2600), ("tiny", 3, 654), ("tiny", 3, 1114), ("tiny", 3, 1115),
+                                              ("cfg1", 2, 1114), ("cfg1", 2, 1115), ("cfg1", 2, 1306), ("cfg1", 2, 1307)])
+def test_narrow_policies_around_their_lines(name, blocks, envs):
+    cfg = make_cfg(name, opts=dict(n_blocks=blocks))
     m = cuda_policy(cfg, po.build_state_dict(cfg, 6))
     obs = po.make_obs(envs, 42, padded=True).cuda()
     logits, value = m.forward_stacked(obs)
